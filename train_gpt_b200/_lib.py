@@ -83,6 +83,24 @@ def load() -> C.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native host path (`_host.so`, csrc/host.cpp) bound to the library `load()` returns; raises if it is missing."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise RuntimeError(f"the native host path is not built or does not load ({e}). "
+                               "Run `python -m train_gpt_b200.build`; there is no other path.") from e
+        mod.bind(LIB_PATH)
+        _host = mod
+    return _host
+
+
 _NAMES = {TG_ERR_SHAPE: "TG_ERR_SHAPE", TG_ERR_ALIGN: "TG_ERR_ALIGN", TG_ERR_ARCH: "TG_ERR_ARCH",
           TG_ERR_CUDA: "TG_ERR_CUDA", TG_ERR_TOO_LARGE: "TG_ERR_TOO_LARGE"}
 

@@ -1,9 +1,10 @@
-"""Build `libtrain_gpt_b200.so` (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Build `libtrain_gpt_b200.so` (the C-ABI library, nvcc for sm_100a) and `_host.so` (the torch-facing host path,
+g++ against torch's headers) in-tree.
 
     python -m train_gpt_b200.build [--force] [--verbose]
 
-nvcc cross-compiles without a GPU.  Objects and the library are written next to the
-sources; a source newer than the library triggers a rebuild.
+nvcc cross-compiles without a GPU.  Objects and libraries are written next to the
+sources; a source newer than its library triggers a rebuild.
 """
 from __future__ import annotations
 
@@ -16,6 +17,7 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 INCLUDE = os.path.join(os.path.dirname(PKG_DIR), "include")
 LIB_PATH = os.path.join(PKG_DIR, "libtrain_gpt_b200.so")
+HOST_PATH = os.path.join(PKG_DIR, "_host.so")
 
 SOURCES = ["runtime.cu", "quantize.cu", "rmsnorm.cu", "gemm_fp8.cu", "selftest.cu", "loss.cu", "optim.cu"]
 
@@ -35,18 +37,46 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found; set NVCC")
 
 
-def _stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+def _stale(target: str, suffixes) -> bool:
+    if not os.path.exists(target):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)]
+    t = os.path.getmtime(target)
+    deps = [os.path.join(d, f) for d in (CSRC, INCLUDE) for f in os.listdir(d) if f.endswith(suffixes)]
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _start_host():
+    """Start compiling the host extension (it needs torch's headers and no GPU); None if it is up to date."""
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    inc = [*cpp_extension.include_paths(), os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include"),
+           sysconfig.get_paths()["include"]]
+    # (built under another name and renamed when complete: another process never loads half a file)
+    cmd = ["g++", "-shared", "-fPIC", "-O2", "-std=c++17", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_host",
+           "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           *[a for i in inc for a in ("-isystem", i)], os.path.join(CSRC, "host.cpp"), "-o", HOST_PATH + ".new",
+           "-L" + lib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda", "-ldl", f"-Wl,-rpath,{lib}"]
+    return subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the library if it is missing or older than its sources; return its path."""
-    if not force and not _stale():
-        return LIB_PATH
+    """Compile what is missing or older than its sources; return the library's path."""
+    host = _start_host() if force or _stale(HOST_PATH, (".cpp", ".h")) else None
+    try:
+        if force or _stale(LIB_PATH, (".cu", ".cuh", ".h")):
+            _build_lib(verbose)
+    finally:
+        out, rc = ("", 0) if host is None else (host.communicate()[0], host.returncode)
+    if rc != 0:
+        raise RuntimeError(f"g++ failed on host.cpp:\n{out}")
+    if host is not None:
+        os.replace(HOST_PATH + ".new", HOST_PATH)
+    return LIB_PATH
+
+
+def _build_lib(verbose: bool) -> None:
     nvcc = _nvcc()
     objs = []
     procs = []
@@ -69,7 +99,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
         f.write("\n".join(log))
     if verbose:
         print("\n".join(log))
-    return LIB_PATH
 
 
 if __name__ == "__main__":

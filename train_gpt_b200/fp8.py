@@ -38,11 +38,6 @@ def _as_bf16(t: torch.Tensor, name: str) -> torch.Tensor:
     return n
 
 
-def _check_block(block_k: int):
-    if block_k != DEFAULT_BLOCK_K:
-        raise ValueError(f"block_k={block_k} is not supported by the sm_100a kernels (only {DEFAULT_BLOCK_K})")
-
-
 def _quantize_to_fp8(x_f32: torch.Tensor, block_k: int = DEFAULT_BLOCK_K):
     """fp8.py:39-47.  The reference only ever passes an upcast bf16 tensor (fp8.py:66,68), and the
     kernels read bf16: a float32 argument is accepted only if it holds bf16 values exactly (it is then
@@ -50,7 +45,8 @@ def _quantize_to_fp8(x_f32: torch.Tensor, block_k: int = DEFAULT_BLOCK_K):
     K = x_f32.shape[-1]
     if K % block_k != 0:
         raise ValueError(f"K={K} not divisible by block_k={block_k}")
-    _check_block(block_k)
+    if block_k != DEFAULT_BLOCK_K:
+        raise ValueError(f"block_k={block_k} is not supported by the sm_100a kernels (only {DEFAULT_BLOCK_K})")
     return ops.quantize_rowwise(_as_bf16(x_f32, "x"))
 
 
@@ -96,40 +92,27 @@ def quantize_weight(b: torch.Tensor, weight_tile=(128, 1)):
     raise ValueError(f"unsupported weight_tile {weight_tile}")
 
 
-def _validate(a, b, block_k):
-    K = a.shape[-1]
-    K_b, N = b.shape
-    if K != K_b:                                                    # fp8.py:53-54
-        raise ValueError(f"contracted-dim mismatch: a K={K}, b K={K_b}")
-    if K % block_k != 0:                                            # fp8.py:55-56
-        raise ValueError(f"K={K} not divisible by block_k={block_k}")
-    _check_block(block_k)
-    return K, N
+_MODES = {"bf16_ste": 0, "fp8": 1, "fp8_blockgrad": 2}
+
+
+def _per_column(weight_tile) -> bool:
+    tile = tuple(weight_tile)
+    if tile not in ((128, 1), (128, 128)):
+        raise ValueError(f"unsupported weight_tile {weight_tile}")
+    return tile == (128, 1)
+
+
+def _row_form(a_quantized):
+    if a_quantized is None:
+        return None, None
+    return a_quantized.rowwise() if isinstance(a_quantized, QuantizedActivation) else (a_quantized[0], a_quantized[1])
 
 
 def _fp8_forward(a, b, block_k=DEFAULT_BLOCK_K, weight_tile=(128, 1), a_quantized=None, return_weight=False):
     """fp8.py:50-78.  `a_quantized` = (q, scales) of `a` made earlier (e.g. by the fused
     norm+quantise kernel) skips the activation quantiser.  return_weight=True also returns the
     quantised weight pair (128x128 tiles serve the backward's dgrad unchanged)."""
-    K, N = _validate(a, b, block_k)
-    leading = a.shape[:-1]
-    if a_quantized is None:
-        a_q, a_s = ops.quantize_rowwise(_as_bf16(a.reshape(-1, K), "a"))
-    elif isinstance(a_quantized, QuantizedActivation):
-        a_q, a_s = a_quantized.rowwise()
-    else:
-        a_q, a_s = a_quantized[0].reshape(-1, K), a_quantized[1].reshape(-1, K // block_k)
-    b = _as_bf16(b, "b")
-    pad = (-N) % 16 if tuple(weight_tile) == (128, 1) else 0
-    if pad:
-        # the TMA row pitch of the (K, N) weight must be a multiple of 16 bytes: widen with
-        # zero columns (their tiles quantise to zeros) and drop them from the result
-        b = torch.nn.functional.pad(b, (0, pad))
-    w_q, w_s = quantize_weight(b, weight_tile)
-    y = ops.gemm_fwd(a_q, a_s, w_q, w_s, weight_tile)
-    if pad:
-        y = y[:, :N]
-    y = y.reshape(*leading, N)
+    y, w_q, w_s = ops._host().fp8_forward(a, b, block_k, _per_column(weight_tile), *_row_form(a_quantized))
     return (y, (w_q, w_s)) if return_weight else y
 
 
@@ -137,76 +120,15 @@ def _fp8_backward(block_k, residuals, g, weight_tile=(128, 1), mode="bf16_ste", 
                   b_slot=None):
     """fp8.py:85-98 (mode "bf16_ste"), or the same two GEMMs in block-scaled e4m3.
     `w_quantized`: the forward's 128x128-tile weight pair, reused instead of quantising again.
-    `b_slot`: a gradient slot of the weight (see `_BlockScaledMatmul.backward`); the FP8 modes then write the
+    `b_slot`: a gradient slot of the weight (see `block_scaled_matmul`); the FP8 modes then write the
     weight gradient there and return None for it."""
     a, b = residuals
-    K = a.shape[-1]
-    N = b.shape[1]
-    leading = a.shape[:-1]
-    a_2d = a.reshape(-1, K).to(torch.bfloat16)
-    g_2d = g.reshape(-1, N).to(torch.bfloat16)
-    b_bf = b.to(torch.bfloat16)
-    if mode == "bf16_ste":
-        da = g_2d @ b_bf.T                                          # fp8.py:96 (cuBLAS bf16)
-        db = a_2d.T @ g_2d                                          # fp8.py:97
-    elif mode in ("fp8", "fp8_blockgrad"):
-        if N % block_k != 0:
-            raise ValueError(f"N={N} not divisible by block_k={block_k} (needed by the FP8 dgrad)")
-        if mode == "fp8":
-            g_q, g_s, g_qc, g_sc = ops.quantize_rowcol(g_2d)        # one read of g for both contractions
-            grad_tile = (128, 1)
-        else:
-            g_q, g_s = ops.quantize_rowwise(g_2d)
-            g_qc, g_sc = ops.quantize_block128(g_2d)
-            grad_tile = (128, 128)
-        if tuple(weight_tile) == (128, 1):
-            w_q, w_s = ops.quantize_rowwise(b_bf)                   # tiles along N, the dgrad contraction
-        elif w_quantized is not None:
-            w_q, w_s = w_quantized
-        else:
-            w_q, w_s = ops.quantize_block128(b_bf)
-        da = ops.gemm_dgrad(g_q, g_s, w_q, w_s, weight_tile)
-        if isinstance(a_quantized, QuantizedActivation):
-            x_qc, x_sc = a_quantized.colwise()                        # shared by every GEMM fed from this activation
-        else:
-            x_qc, x_sc = ops.quantize_colwise(a_2d)
-        if b_slot is not None and b.dtype == torch.bfloat16:
-            ops.gemm_wgrad(x_qc, x_sc, g_qc, g_sc, grad_tile=grad_tile, out=b_slot.take())
-            b_slot.ready()
-            return da.reshape(*leading, K).to(a.dtype), None
-        db = ops.gemm_wgrad(x_qc, x_sc, g_qc, g_sc, grad_tile=grad_tile)
-    else:
+    if mode not in _MODES:
         raise ValueError(f"unknown backward mode {mode!r}; use 'bf16_ste', 'fp8' or 'fp8_blockgrad'")
-    return da.reshape(*leading, K).to(a.dtype), db.to(b.dtype)
-
-
-def _plain_2d(b) -> bool:
-    # the direct weight-gradient write needs no padding of N (see _fp8_forward) and a weight as stored
-    return b.dim() == 2 and b.shape[1] % 16 == 0
-
-
-class _BlockScaledMatmul(torch.autograd.Function):
-    """The custom VJP of fp8.py:30,101 as a torch.autograd.Function."""
-
-    @staticmethod
-    def forward(ctx, a, b, block_k, weight_tile, backward, a_quantized):
-        ctx.save_for_backward(a, b)                                 # fp8.py:81-82: unquantised residuals
-        ctx.cfg = (block_k, tuple(weight_tile), backward)
-        ctx.aq = a_quantized if isinstance(a_quantized, QuantizedActivation) else None
-        y, wq = _fp8_forward(a, b, block_k, weight_tile, a_quantized, return_weight=True)
-        ctx.wq = wq if (tuple(weight_tile) == (128, 128) and backward != "bf16_ste") else None
-        ctx.b_param = b if (isinstance(b, torch.nn.Parameter) and a.dim() >= 2 and _plain_2d(b)) else None
-        return y
-
-    @staticmethod
-    def backward(ctx, g):
-        block_k, weight_tile, mode = ctx.cfg
-        # A weight may carry `grad_slot` (an object with take() -> the tensor its gradient belongs in, and
-        # ready(); train_gpt_b200.dp.GradSlot): the weight-gradient GEMM then writes straight into the flat
-        # gradient bucket and autograd gets None, instead of a fresh tensor that is added into a zeroed bucket.
-        slot = getattr(ctx.b_param, "grad_slot", None) if ctx.b_param is not None else None
-        da, db = _fp8_backward(block_k, ctx.saved_tensors, g, weight_tile, mode, ctx.aq, ctx.wq, b_slot=slot)
-        return da, db, None, None, None, None
+    w_q, w_s = w_quantized if w_quantized is not None else (None, None)
+    return ops._host().fp8_backward(a, b, g, _per_column(weight_tile), _MODES[mode],
+                                    a_quantized if isinstance(a_quantized, QuantizedActivation) else None, w_q, w_s,
+                                    b_slot if b.dtype == torch.bfloat16 else None)
 
 
 def block_scaled_matmul(a: torch.Tensor, b: torch.Tensor, block_k: int = DEFAULT_BLOCK_K, *,
@@ -214,8 +136,18 @@ def block_scaled_matmul(a: torch.Tensor, b: torch.Tensor, block_k: int = DEFAULT
     """Per-K-tile block-scaled FP8 matmul.
 
     a: (..., K), b: (K, N) -> (..., N) bf16.  Requires K % block_k == 0.
-    """
-    _validate(a, b, block_k)
-    if backward not in ("bf16_ste", "fp8", "fp8_blockgrad"):
+
+    A weight may carry `grad_slot` (an object with take() -> the tensor its gradient belongs in, and
+    ready(); train_gpt_b200.dp.GradSlot): in the FP8 backward modes the weight-gradient GEMM then writes
+    straight into the flat gradient bucket and autograd gets None, instead of a fresh tensor that is added
+    into a zeroed bucket."""
+    mode = _MODES.get(backward)
+    if mode is None:
         raise ValueError(f"unknown backward mode {backward!r}; use 'bf16_ste', 'fp8' or 'fp8_blockgrad'")
-    return _BlockScaledMatmul.apply(a, b, block_k, tuple(weight_tile), backward, a_quantized)
+    row_q, row_s = _row_form(a_quantized)
+    slot = getattr(b, "grad_slot", None)
+    if slot is not None and not (a.dim() >= 2 and b.dim() == 2 and b.shape[1] % 16 == 0 and b.dtype == torch.bfloat16):
+        slot = None                              # the direct write takes a bf16 weight as stored, without padding
+    return ops._host().block_scaled_matmul(a, b, block_k, _per_column(weight_tile), mode,
+                                           a_quantized if isinstance(a_quantized, QuantizedActivation) else None,
+                                           row_q, row_s, slot)

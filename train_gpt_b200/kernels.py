@@ -13,26 +13,12 @@ import torch
 from . import ops
 
 
-class _RmsNorm(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, scale, eps, pure):
-        ctx.save_for_backward(x, scale)                             # kernels.py:101-102
-        ctx.eps = eps
-        return ops.rmsnorm_fwd(x, scale, eps, pure=pure)
-
-    @staticmethod
-    def backward(ctx, g):
-        x, scale = ctx.saved_tensors
-        dx, dscale = ops.rmsnorm_bwd(x, scale, g.to(torch.bfloat16), ctx.eps)   # kernels.py:104-118
-        return dx, dscale, None, None
-
-
 def rms_norm(x: torch.Tensor, scale: torch.Tensor, eps: float) -> torch.Tensor:
-    return _RmsNorm.apply(x, scale, float(eps), False)
+    return ops._host().rms_norm(x, scale, eps, False)
 
 
 def _rms_norm_pure(x: torch.Tensor, scale: torch.Tensor, eps: float) -> torch.Tensor:
-    return _RmsNorm.apply(x, scale, float(eps), True)
+    return ops._host().rms_norm(x, scale, eps, True)
 
 
 class NormedQuantized:
