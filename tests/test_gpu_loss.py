@@ -123,3 +123,40 @@ def test_reference_default_vocabulary_through_autograd():
     assert ga.shape == gb.shape
     rms = gb.pow(2).mean().sqrt()
     assert bool(((ga - gb).abs() <= 2e-2 * gb.abs() + 1e-2 * rms).all())
+
+
+@pytest.mark.parametrize("rows,vocab,cap", [(1, 1, 15.0), (3, 7, 15.0), (9, 256, 15.0), (17, 2047, 2.5), (5, 2048, 30.0),
+                                            (5, 2049, 15.0), (40, 5119, 15.0), (301, 5121, 64.0), (3, 50257, 15.0), (2, 110000, 15.0),
+                                            (2, 130000, 15.0), (4, 300, 80.0)])
+def test_one_pass_loss_and_gradient(rows, vocab, cap):
+    """The one-pass kernel at the edges of its shapes (one warp or one block per row, rows that start at every alignment,
+    ragged last pieces; past its limits in width and cap the two-kernel path), with an upstream gradient of 1 and another."""
+    from train_gpt_b200 import losses
+    x, t = _case(rows, vocab, rows + vocab, 0.4 * cap)
+    x.reshape(-1)[:: 97] = 0
+    a = to_torch_bf16(x).requires_grad_(True)
+    tt = torch.from_numpy(t.astype(np.int64)).cuda()
+    loss = losses.capped_cross_entropy(a, tt, cap)
+    loss.backward(retain_graph=True)
+    z_ref, _ = lo.softcap(x, cap)
+    _, nll_ref, _ = lo.cross_entropy(z_ref, t)
+    assert abs(float(loss.detach()) - nll_ref.mean()) <= 1e-5 * abs(nll_ref.mean()) + 1e-6
+    for scale in (1.0, 0.75):
+        if scale != 1.0:
+            a.grad = None
+            (loss * scale).backward()
+        ref = lo.softcap_cross_entropy_grad(x, t, cap, gscale=scale)
+        got = from_torch_bf16(a.grad).astype(np.float64)
+        rms = np.sqrt((ref ** 2).mean())
+        assert np.all(np.abs(got - ref) <= 2e-2 * np.abs(ref) + 1e-2 * rms)
+        assert np.allclose(got[np.arange(rows), t], ref[np.arange(rows), t], rtol=1e-2, atol=1e-12)
+
+
+def test_one_pass_loss_of_a_nan_row():
+    from train_gpt_b200 import losses
+    x = torch.zeros(3, 3000, dtype=torch.bfloat16, device="cuda")
+    x[1, 1234] = float("nan")
+    x.requires_grad_(True)
+    loss = losses.capped_cross_entropy(x, torch.zeros(3, dtype=torch.int64, device="cuda"), 15.0)
+    loss.backward()
+    assert bool(torch.isnan(loss)) and bool(torch.isnan(x.grad[1]).all()) and not bool(torch.isnan(x.grad[::2]).any())

@@ -11,6 +11,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <dlfcn.h>
+#include <torch/csrc/autograd/engine.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -29,6 +30,7 @@
 #include <vector>
 
 #include "../../include/train_gpt_b200.h"
+#include "host_api.h"
 
 namespace py = pybind11;
 using at::Tensor;
@@ -49,7 +51,7 @@ const auto kF8 = at::kFloat8_e4m3fn;
   X(tg_act_quantize_rowcol) X(tg_quantize_block128) X(tg_rmsnorm_fwd) X(tg_rmsnorm_quant_fwd)                       \
   X(tg_add_rmsnorm_quant_fwd) X(tg_rmsnorm_bwd_scratch_bytes) X(tg_rmsnorm_bwd) X(tg_rmsnorm_bwd_add)               \
   X(tg_softcap_ce_fwd) X(tg_softcap_ce_bwd) X(tg_sumsq_scratch_bytes) X(tg_sumsq_bf16) X(tg_adamw_bf16)             \
-  X(tg_gemm_workspace_bytes) X(tg_gemm_fp8_blockscaled)
+  X(tg_gemm_workspace_bytes) X(tg_gemm_fp8_blockscaled) X(tgh_softcap_ce_fits) X(tgh_softcap_ce)
 
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;
@@ -112,7 +114,7 @@ Tensor empty(at::IntArrayRef shape, at::ScalarType dt, const Tensor& like) {
   return at::empty(shape, at::TensorOptions().dtype(dt).device(like.device()));
 }
 
-void* stream() { return at::cuda::getCurrentCUDAStream().stream(); }
+void* cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
 float* fptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
 void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
@@ -137,7 +139,7 @@ Pair quantize_rowwise(const Tensor& x_) {
   need_tiles(k);
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor q = empty(x.sizes(), kF8, x), s = empty(with_last(x, k / kTile), at::kFloat, x);
-  check(api.tg_quantize_rowwise(ptr(x), ptr(q), fptr(s), k ? x.numel() / k : 0, k, stream()), "tg_quantize_rowwise");
+  check(api.tg_quantize_rowwise(ptr(x), ptr(q), fptr(s), k ? x.numel() / k : 0, k, cur_stream()), "tg_quantize_rowwise");
   return {q, s};
 }
 
@@ -147,7 +149,7 @@ Pair quantize_colwise(const Tensor& x_) {
   const int64_t r = x.size(0), c = x.size(1);
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor q = empty({r, c}, kF8, x), s = empty({cdiv(r, kTile), c}, at::kFloat, x);
-  check(api.tg_quantize_colwise(ptr(x), ptr(q), fptr(s), r, c, stream()), "tg_quantize_colwise");
+  check(api.tg_quantize_colwise(ptr(x), ptr(q), fptr(s), r, c, cur_stream()), "tg_quantize_colwise");
   return {q, s};
 }
 
@@ -158,7 +160,7 @@ Pair quantize_block128(const Tensor& x_) {
   if (c % kTile) throw py::value_error(cat("C=", c, " not divisible by ", kTile));
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor q = empty({r, c}, kF8, x), s = empty({cdiv(r, kTile), c / kTile}, at::kFloat, x);
-  check(api.tg_quantize_block128(ptr(x), ptr(q), fptr(s), r, c, stream()), "tg_quantize_block128");
+  check(api.tg_quantize_block128(ptr(x), ptr(q), fptr(s), r, c, cur_stream()), "tg_quantize_block128");
   return {q, s};
 }
 
@@ -178,7 +180,7 @@ RowCol quantize_rowcol(const Tensor& x_) {
   need_tiles(x.size(1));
   const c10::cuda::CUDAGuard guard(x.device());
   RowCol o = rowcol_like(x);
-  check(api.tg_quantize_rowcol(ptr(x), ptr(o.q_row), fptr(o.s_row), ptr(o.q_col), fptr(o.s_col), x.size(0), x.size(1), stream()),
+  check(api.tg_quantize_rowcol(ptr(x), ptr(o.q_row), fptr(o.s_row), ptr(o.q_col), fptr(o.s_col), x.size(0), x.size(1), cur_stream()),
         "tg_quantize_rowcol");
   return o;
 }
@@ -205,7 +207,7 @@ RowCol quantize_rowcol_into(const Tensor& x_, const std::optional<Pair>& row_out
   };
   check(api.tg_quantize_rowcol_ld(ptr(x), ptr(row.first), ld(row.first, std::max<int64_t>(c, 16)), fptr(row.second),
                                   ld(row.second, c / kTile), ptr(col.first), ld(col.first, std::max<int64_t>(c, 16)),
-                                  fptr(col.second), ld(col.second, c), r, c, stream()),
+                                  fptr(col.second), ld(col.second, c), r, c, cur_stream()),
         "tg_quantize_rowcol_ld");
   return {row.first, row.second, col.first, col.second};
 }
@@ -224,7 +226,7 @@ RowCol act_quantize_rowcol(const Tensor& x_, int act, const std::string& act_nam
   const c10::cuda::CUDAGuard guard(x.device());
   RowCol o = rowcol_like(x);
   check(api.tg_act_quantize_rowcol(ptr(x), ptr(gate), act, ptr(o.q_row), fptr(o.s_row), ptr(o.q_col), fptr(o.s_col), x.size(0),
-                                   x.size(1), stream()),
+                                   x.size(1), cur_stream()),
         "tg_act_quantize_rowcol");
   return o;
 }
@@ -244,7 +246,7 @@ Pair rmsnorm_fwd(const Tensor& x_, const Tensor& gamma_, double eps, bool pure, 
   Tensor y = at::empty_like(x), rn;
   if (want_rnorm) rn = empty(x.sizes().slice(0, x.dim() - 1), at::kFloat, x);
   check(api.tg_rmsnorm_fwd(ptr(x), ptr(gamma), float(eps), ptr(y), fptr(rn), x.numel() / d, d, pure ? TG_NORM_PURE : TG_NORM_FUSED,
-                           stream()),
+                           cur_stream()),
         "tg_rmsnorm_fwd");
   return {y, rn};
 }
@@ -265,7 +267,7 @@ NormQuant rmsnorm_quant_fwd(const Tensor& x_, const Tensor& gamma_, double eps, 
   if (want_y) o.y = at::empty_like(x);
   if (want_rnorm) o.rn = empty(x.sizes().slice(0, x.dim() - 1), at::kFloat, x);
   check(api.tg_rmsnorm_quant_fwd(ptr(x), ptr(gamma), float(eps), ptr(o.q), fptr(o.s), ptr(o.y), fptr(o.rn), x.numel() / d, d,
-                                 pure ? TG_NORM_PURE : TG_NORM_FUSED, stream()),
+                                 pure ? TG_NORM_PURE : TG_NORM_FUSED, cur_stream()),
         "tg_rmsnorm_quant_fwd");
   return o;
 }
@@ -292,7 +294,7 @@ AddNorm add_rmsnorm_quant_fwd(const Tensor& x_, const Tensor& res_, const Tensor
   }
   if (want_y) o.y = at::empty_like(x);
   check(api.tg_add_rmsnorm_quant_fwd(ptr(x), ptr(res), ptr(gamma), float(eps), ptr(o.sum), ptr(o.q), fptr(o.s), ptr(o.y), nullptr,
-                                     x.numel() / d, d, pure ? TG_NORM_PURE : TG_NORM_FUSED, stream()),
+                                     x.numel() / d, d, pure ? TG_NORM_PURE : TG_NORM_FUSED, cur_stream()),
         "tg_add_rmsnorm_quant_fwd");
   return o;
 }
@@ -313,10 +315,10 @@ Pair rmsnorm_bwd(const Tensor& x_, const Tensor& gamma_, const Tensor& g_, doubl
   Tensor scratch = empty({bytes}, at::kByte, x);
   if (addend.defined())
     check(api.tg_rmsnorm_bwd_add(ptr(x), ptr(gamma), ptr(g), ptr(addend), float(eps), ptr(dx), ptr(dgamma), ptr(scratch), rows, d,
-                                 stream()),
+                                 cur_stream()),
           "tg_rmsnorm_bwd_add");
   else
-    check(api.tg_rmsnorm_bwd(ptr(x), ptr(gamma), ptr(g), float(eps), ptr(dx), ptr(dgamma), ptr(scratch), rows, d, stream()),
+    check(api.tg_rmsnorm_bwd(ptr(x), ptr(gamma), ptr(g), float(eps), ptr(dx), ptr(dgamma), ptr(scratch), rows, d, cur_stream()),
           "tg_rmsnorm_bwd");
   return {dx, dgamma};
 }
@@ -341,7 +343,7 @@ std::tuple<Tensor, Tensor, Tensor> softcap_ce_fwd(const Tensor& logits_, const T
   Tensor nll = empty({rows}, at::kFloat, logits), lse = empty({rows}, at::kFloat, logits), th;
   if (want_tanh) th = empty({rows, pitch}, at::kBFloat16, logits);
   check(api.tg_softcap_ce_fwd(ptr(logits), static_cast<const int32_t*>(ptr(targets)), float(cap), ptr(th), fptr(lse), fptr(nll), rows,
-                              vocab, pitch, pitch, stream()),
+                              vocab, pitch, pitch, cur_stream()),
         "tg_softcap_ce_fwd");
   if (th.defined() && pitch != vocab) th = th.narrow(1, 0, vocab);     // a view: the row pitch stays `pitch`
   return {nll, lse, th};
@@ -362,7 +364,7 @@ Tensor softcap_ce_bwd(const Tensor& th, const Tensor& targets, const Tensor& lse
   Tensor gscale;
   if (gscale_) gscale = need(gscale_->reshape({1}), at::kFloat, "gscale");
   check(api.tg_softcap_ce_bwd(ptr(th), static_cast<const int32_t*>(ptr(targets)), fptr(lse), fptr(gscale), float(cap), ptr(d), rows,
-                              vocab, pitch, d_pitch, stream()),
+                              vocab, pitch, d_pitch, cur_stream()),
         "tg_softcap_ce_bwd");
   return d;
 }
@@ -374,7 +376,7 @@ Tensor sumsq(const Tensor& x_, const std::optional<Tensor>& out_, const std::opt
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor out = out_ ? *out_ : empty({1}, at::kFloat, x);
   Tensor scratch = scratch_ ? *scratch_ : empty({api.tg_sumsq_scratch_bytes()}, at::kByte, x);
-  check(api.tg_sumsq_bf16(ptr(x), x.numel(), fptr(out), ptr(scratch), stream()), "tg_sumsq_bf16");
+  check(api.tg_sumsq_bf16(ptr(x), x.numel(), fptr(out), ptr(scratch), cur_stream()), "tg_sumsq_bf16");
   return out;
 }
 
@@ -388,7 +390,7 @@ void adamw_step(const Tensor& p, const Tensor& g, const Tensor& m, const Tensor&
   if (step.scalar_type() != at::kInt || !step.is_cuda()) throw py::type_error("step must be an int32 CUDA scalar");
   const c10::cuda::CUDAGuard guard(p.device());
   check(api.tg_adamw_bf16(ptr(p), ptr(g), ptr(m), ptr(v), p.numel(), float(lr), float(b1), float(b2), float(eps), float(weight_decay),
-                          static_cast<const int32_t*>(ptr(step)), gscale ? fptr(*gscale) : nullptr, stream()),
+                          static_cast<const int32_t*>(ptr(step)), gscale ? fptr(*gscale) : nullptr, cur_stream()),
         "tg_adamw_bf16");
 }
 
@@ -440,7 +442,7 @@ Tensor gemm(const Tensor& a, const Tensor& b, const Tensor& sa, const Tensor& sb
       args.workspace_bytes = bytes;
     }
   }
-  check(api.tg_gemm_fp8_blockscaled(&args, stream()), "tg_gemm_fp8_blockscaled");
+  check(api.tg_gemm_fp8_blockscaled(&args, cur_stream()), "tg_gemm_fp8_blockscaled");
   last_gemm_launches.store(ws.defined() ? 2 : 1, std::memory_order_relaxed);
   return out;
 }
@@ -745,6 +747,43 @@ Tensor rms_norm(const Tensor& x, const Tensor& gamma, double eps, bool pure) {
   return y;
 }
 
+// The loss of rows the one-pass kernel takes: forward makes the gradient too, for an upstream gradient of 1 -- what
+// `loss.backward()` brings.  Another one is seen on the device (no synchronisation) and the gradient is made again
+// from the logits with it, so that it is rounded once all the same.  (Logits that were overwritten in between are no
+// error, as they never were for this function: the gradient at hand is then scaled.)
+struct CappedCEBackward : public Node {
+  Tensor logits, targets, d;
+  uint32_t version = 0;
+  double cap = 0;
+  bool given = false;                        // `d` has been handed out: it is no longer this node's own
+  std::string name() const override { return "CappedCEBackward"; }
+  void release_variables() override {
+    logits = targets = d = Tensor();
+  }
+  variable_list apply(variable_list&& grads) override {
+    variable_list out(1);
+    if (!grads[0].defined()) return out;
+    if (!targets.defined()) backward_twice();
+    const Tensor& x = logits;
+    if (x._version() != version) {
+      out[0] = (d * grads[0].to(at::kFloat)).to(at::kBFloat16);
+      return out;
+    }
+    const int64_t vocab = x.size(-1), rows = x.numel() / vocab;
+    const Tensor g = grads[0].to(at::kFloat).contiguous();
+    const bool again = given;
+    if (again) d = at::empty_like(d);
+    const c10::cuda::CUDAGuard guard(x.device());
+    check(api.tgh_softcap_ce(ptr(x), ptr(targets), targets.scalar_type() == at::kLong, float(cap), ptr(d), fptr(g), !again, nullptr,
+                             nullptr, rows, vocab, vocab, cur_stream()),
+          "tgh_softcap_ce");
+    given = true;
+    out[0] = d;
+    return out;
+  }
+};
+
+// ... and of any others: the tanh values go from the forward kernel to the backward one through memory
 struct SoftcapCEBackward : public Node {
   Tensor th, targets, lse;
   std::vector<int64_t> shape;
@@ -755,32 +794,59 @@ struct SoftcapCEBackward : public Node {
     variable_list out(1);
     if (!grads[0].defined()) return out;
     if (!th.defined()) backward_twice();
-    // the tanh buffer is this node's own: the gradient replaces it in place
-    out[0] = softcap_ce_bwd(th, targets, lse, grads[0].to(at::kFloat), cap, true).reshape(shape);
+    // the tanh buffer is this node's own: the gradient replaces it in place, unless it will be wanted again
+    const bool last = !torch::autograd::get_current_graph_task_keep_graph();
+    out[0] = softcap_ce_bwd(th, targets, lse, grads[0].to(at::kFloat), cap, last).reshape(shape);
     return out;
   }
 };
 
-Tensor capped_cross_entropy(const Tensor& logits, const Tensor& target_ids, double cap) {
-  if (logits.sizes().slice(0, logits.dim() - 1) != target_ids.sizes())
-    throw py::value_error(cat("logits ", logits.sizes(), " and target_ids ", target_ids.sizes(), " do not match"));
-  const bool track = at::GradMode::is_enabled() && logits.requires_grad();
-  Tensor th, t, lse, loss;
+Tensor capped_cross_entropy(const Tensor& logits_, const Tensor& target_ids, double cap) {
+  if (logits_.dim() == 0 || logits_.sizes().slice(0, logits_.dim() - 1) != target_ids.sizes())
+    throw py::value_error(cat("logits ", logits_.sizes(), " and target_ids ", target_ids.sizes(), " do not match"));
+  const bool track = at::GradMode::is_enabled() && logits_.requires_grad();
+  const int64_t vocab = logits_.size(-1), rows = target_ids.numel();
+  Tensor logits = need(logits_, at::kBFloat16, "logits"), t = target_ids.contiguous(), loss;
+  if (t.scalar_type() != at::kLong) t = t.to(at::kInt);
+  const c10::cuda::CUDAGuard guard(logits.device());
+  if (rows > 0 && t.is_cuda() && api.tgh_softcap_ce_fits(float(cap), rows, vocab)) {
+    Tensor d;
+    {
+      at::AutoDispatchBelowADInplaceOrView below;
+      if (reinterpret_cast<uintptr_t>(ptr(logits)) & 15u) logits = logits.clone();
+      if (track) d = at::empty_like(logits);
+      Tensor nll = empty({rows}, at::kFloat, logits);
+      loss = empty({}, at::kFloat, logits);
+      check(api.tgh_softcap_ce(ptr(logits), ptr(t), t.scalar_type() == at::kLong, float(cap), ptr(d), nullptr, 0, fptr(nll), fptr(loss),
+                               rows, vocab, vocab, cur_stream()),
+            "tgh_softcap_ce");
+    }
+    if (!track) return loss;
+    std::shared_ptr<CappedCEBackward> node(new CappedCEBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(logits_));
+    node->logits = logits.detach();
+    node->version = logits._version();
+    node->targets = t;
+    node->d = d;
+    node->cap = cap;
+    torch::autograd::set_history(loss, node);
+    return loss;
+  }
+  Tensor th, lse, nll;
   {
     at::AutoDispatchBelowADInplaceOrView below;
-    Tensor nll;
-    t = target_ids.reshape({-1}).to(at::kInt);
-    std::tie(nll, lse, th) = softcap_ce_fwd(logits.reshape({-1, logits.size(-1)}), t, cap, true);
+    t = t.reshape({-1}).to(at::kInt);
+    std::tie(nll, lse, th) = softcap_ce_fwd(logits.reshape({-1, vocab}), t, cap, true);
     loss = nll.mean();                                                               // losses.py:12
   }
   if (!track) return loss;
   std::shared_ptr<SoftcapCEBackward> node(new SoftcapCEBackward(), torch::autograd::deleteNode);
-  node->set_next_edges(torch::autograd::collect_next_edges(logits));
+  node->set_next_edges(torch::autograd::collect_next_edges(logits_));
   node->th = th;
   node->targets = t;
   node->lse = lse;
   node->cap = cap;
-  node->shape.assign(logits.sizes().begin(), logits.sizes().end());
+  node->shape.assign(logits_.sizes().begin(), logits_.sizes().end());
   torch::autograd::set_history(loss, node);
   return loss;
 }

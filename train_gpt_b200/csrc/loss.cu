@@ -11,8 +11,10 @@
 // Layout: one thread block per token row; each thread walks the row in 16-byte pieces (8 bf16)
 // and keeps a running (max, sum of exp) pair; the block combines the pairs.
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
+#include "host_api.h"
 
 namespace tg {
 
@@ -205,9 +207,305 @@ softcap_ce_bwd_kernel(const __nv_bfloat16* tanh_in, const int32_t* __restrict__ 
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// Loss and gradient from ONE read of the logits.  The pair of kernels above moves 8 bytes per logit (read, tanh
+// out; tanh in, gradient out) and wants rows of a 16-byte pitch, which costs a vocabulary like 50257 a padding copy
+// in and a compacting one out: 1.8 of 2.5 ms at 8192 x 50257.  Here a row's tanh values stay in shared memory
+// between the softmax sum and the gradient, so a logit is read once (2 bytes) and its gradient written once (2).
+//
+// Rows of any alignment: a row is cut at the 16-byte boundaries of MEMORY, not of the row (its first and last
+// piece may belong to two rows and go element by element), and the gradient, laid out like the logits, is cut alike.
+//
+// bf16(tanh(bf16(x / c))) by table over the bits of x.  From 4 c on it is +-1.  Below `lo`, a power of two at most
+// c / 128, the quotient is below 2^-6 and tanh is the identity after rounding, so t(x) is the rounded quotient and the
+// quotients of one binade are those of the next with another exponent: bits(t(x)) = bits(t(x')) + bits(x) - bits(x')
+// for the x' of the `lo` binade with x's mantissa.  In between: at most 11 binades x 128 mantissas, 2.8 KB.
+// (The 64 KB table of the forward kernel leaves no room for a row; with this one two blocks fit on an SM even
+// at 50304 columns, so that one block's stores overlap the other's loads.)  Magnitudes below 2^-111 are taken as 2^-111:
+// their capped value is far below half an ulp of anything it meets.  A NaN would look up 1: a row's largest
+// magnitude is tracked and a NaN in it makes the row's sum, and with it the loss and the gradient, NaN.
+//
+// No running maximum: |z| <= c <= 64, so the sum of exp(z) neither overflows nor loses its terms.
+//
+// One thread block per row (one warp for rows up to 2048 columns); a thread meets the same pieces in both passes,
+// so the only synchronisation is the reduction of the sum: one barrier per row.
+// Bound by instruction issue and the ALU pipe (49 warp instructions per 64 logits, two of them ex2 in each pass), no longer by
+// memory.  8192 x 50257: 699 us for the two kernels, 2507 with the copies -> 415 us (DRAM floor 251); 8192 x 50304: 697 -> 414.
+// ---------------------------------------------------------------------------------------
+constexpr int kCeMaxThreads = 640;
+constexpr int kCeWarpCols = 2048;                 // rows up to this wide take one warp
+constexpr int kCeTableMax = 11 * 128 + 2;
+constexpr int kCeTableBytes = (kCeTableMax * 2 + 15) / 16 * 16;
+constexpr uint32_t kCeFloor2 = 0x08000800u;
+constexpr float kLog2e = 1.4426950408889634f;
+
+struct CeArgs {
+  const __nv_bfloat16* logits;
+  const void* targets;
+  int targets_64;
+  float cap;
+  __nv_bfloat16* d;
+  const float* gscale;
+  int only_if_scaled;
+  float* nll;
+  int rows, vocab;
+  int64_t ld;
+};
+
+__device__ __forceinline__ float ex2(float v) {
+  float e;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(v));
+  return e;
+}
+__device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+  return v;
+}
+
+template <bool WARP>
+__global__ void __launch_bounds__(WARP ? 256 : kCeMaxThreads, WARP ? 4 : 2) softcap_ce_kernel(const CeArgs p) {
+  if (p.only_if_scaled && *p.gscale == 1.0f) return;
+  extern __shared__ __align__(16) uint8_t s_ce[];
+  __shared__ float s_sum[2][kCeMaxThreads / 32];
+  const Softcap sc(p.cap);
+  // the power-of-two edges of the table as bf16 bits: 2^floor(log2 c) is c with its mantissa cleared
+  const uint32_t c_pow = (__float_as_uint(sc.c) >> 16) & 0x7f80u;
+  const uint32_t lo = c_pow - (7u << 7), hi = c_pow + (3u << 7);      // c / 256 < lo <= c / 128; 4 c < hi <= 8 c
+  uint16_t* table = reinterpret_cast<uint16_t*>(s_ce);
+  for (uint32_t i = threadIdx.x; i <= hi - lo; i += blockDim.x)
+    table[i] = uint16_t(__float_as_uint(tanh_bf16(sc.quotient(__uint_as_float((lo + i) << 16)))) >> 16);
+  __syncthreads();
+
+  const uint32_t lo2 = lo * 0x10001u, hi2 = hi * 0x10001u;
+  // (address of entry 0) - 2 lo, once per half: the sum with a pair of doubled indexes is two 16-bit addresses
+  // (shared addresses of the table are far below 2^16, and a 32-bit sum of the two halves is exact)
+  const uint32_t tab = uint32_t(__cvta_generic_to_shared(s_ce)) - 2u * lo, tab2 = tab + (tab << 16);
+  const int nt = WARP ? 32 : int(blockDim.x), tid = WARP ? int(threadIdx.x & 31) : int(threadIdx.x);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int slots = (p.vocab + 14) / 8;                               // 16-byte pieces a row can touch
+  uint4* row_t = reinterpret_cast<uint4*>(s_ce + kCeTableBytes) + (WARP ? warp * slots : 0);
+  const float gs = (p.gscale != nullptr ? *p.gscale : 1.0f) * (1.0f / float(p.rows));
+  const float2 l2e = make_float2(kLog2e, kLog2e), gs2 = make_float2(gs, gs);
+  const float2 one = make_float2(1.f, 1.f), minus1 = make_float2(-1.f, -1.f);
+  const __nv_bfloat162 c2 = __float2bfloat162_rn(sc.c);
+  const int step = WARP ? int(gridDim.x) * 8 : int(gridDim.x);
+  int row = WARP ? int(blockIdx.x) * 8 + warp : int(blockIdx.x);
+
+  struct Row {
+    const __nv_bfloat16* base;     // the row's first 16-byte boundary at or below its start
+    int off;                       // elements of that piece which belong to the row before
+    int first, last;               // the whole pieces [first, last): at most one ragged piece before and one after
+  };
+  auto row_of = [&](int r) {
+    Row q;
+    const __nv_bfloat16* s = p.logits + int64_t(r) * p.ld;
+    q.off = int((reinterpret_cast<uintptr_t>(s) & 15u) >> 1);
+    q.base = s - q.off;
+    q.first = q.off != 0;
+    q.last = (q.off + p.vocab) >> 3;
+    return q;
+  };
+  auto load = [&](const Row& q, int i) -> uint4 { return i < q.last ? ld_nc_v4(q.base + i * 8) : make_uint4(0u, 0u, 0u, 0u); };
+  // the tanh values of a pair of logits
+  auto tanh_pair = [&](uint32_t w, uint32_t mag) {
+    const uint32_t m = __vmaxu2(mag, kCeFloor2);
+    const uint32_t at = __vmaxu2(mag, (mag & 0x007f007fu) + lo2);
+    const uint32_t addr = (__vminu2(at, hi2) << 1) + tab2;
+    const uint32_t t_lo = lds_u16(addr & 0xffffu), t_hi = lds_u16(addr >> 16);
+    // (no carry crosses the halves: t + m <= 0xffff, and t + m >= at by construction)
+    return (__byte_perm(t_lo, t_hi, 0x5410) + m - at) | (w & 0x80008000u);
+  };
+  // bf16(c t) of a pair: the product of two bf16 values rounded once, as the float product rounded to bf16 is
+  auto capped = [&](uint32_t t2) {
+    const __nv_bfloat162 z = __hmul2(c2, *reinterpret_cast<const __nv_bfloat162*>(&t2));
+    return bf16x2_unpack(*reinterpret_cast<const uint32_t*>(&z));
+  };
+  // the ragged pieces of a row, an element per lane of the last warp: lanes 0..7 the piece before the whole ones, lanes
+  // 8..15 the piece after them.  (One thread per piece, element after element, held every row up by 8 %.)
+  auto edge_of = [&](const Row& q) {
+    const int end = q.off + p.vocab;
+    if (!WARP && warp != nt / 32 - 1) return -1;
+    if (lane < 8) return q.off != 0 && lane >= q.off && lane < end ? lane : -1;
+    const int e = q.last * 8 + lane - 8;
+    return lane < 16 && q.last >= q.first && e < end ? e : -1;
+  };
+  auto grad1 = [&](float t, float z, float lse, bool hit) {
+    const float pr = ex2(__fmul_rn(z - lse, kLog2e)) - (hit ? 1.0f : 0.0f);
+    return __float2bfloat16_rn(__fmul_rn(__fmul_rn(pr, gs), __fmaf_rn(__fmul_rn(t, t), -1.0f, 1.0f)));
+  };
+
+  if (row >= p.rows) return;
+  Row q = row_of(row);
+  uint4 w0 = load(q, q.first + tid), w1 = load(q, q.first + tid + nt);
+  for (int it = 0; row < p.rows; row += step, ++it) {
+    // ---- tanh values and the sum of exp(z)
+    float2 acc = make_float2(0.f, 0.f);
+    uint32_t top = 0u;
+    for (int i = q.first + tid; i < q.last; i += nt) {
+      const uint4 w = w0;
+      w0 = w1;
+      w1 = load(q, i + 2 * nt);
+      const uint32_t wi[4] = {w.x, w.y, w.z, w.w};
+      uint4 to;
+      uint32_t* tp = &to.x;
+      float2 e[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t mag = wi[j] & 0x7fff7fffu;
+        top = __vmaxu2(top, mag);
+        tp[j] = tanh_pair(wi[j], mag);
+        const float2 zl = __fmul2_rn(capped(tp[j]), l2e);
+        e[j] = make_float2(ex2(zl.x), ex2(zl.y));
+      }
+      row_t[i] = to;
+      acc = __fadd2_rn(acc, __fadd2_rn(__fadd2_rn(e[0], e[1]), __fadd2_rn(e[2], e[3])));
+    }
+    const uint16_t* row_e = reinterpret_cast<const uint16_t*>(row_t);
+    const int e_mine = edge_of(q);
+    uint32_t t_edge = 0u;
+    if (e_mine >= 0) {
+      const uint32_t w = reinterpret_cast<const unsigned short*>(q.base)[e_mine];
+      t_edge = tanh_pair(w, w & 0x7fffu) & 0xffffu;
+      top = __vmaxu2(top, w & 0x7fffu);
+      acc.x += ex2(__fmul_rn(capped(t_edge).x, kLog2e));
+    }
+    // the next row's first pieces are on their way while this one is finished
+    const Row now = q;
+    if (row + step < p.rows) {
+      q = row_of(row + step);
+      w0 = load(q, q.first + tid);
+      w1 = load(q, q.first + tid + nt);
+    }
+    float s = acc.x + acc.y;
+    if ((top & 0xffffu) > 0x7f80u || (top >> 16) > 0x7f80u) s = __int_as_float(0x7fffffff);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (!WARP) {
+      if (lane == 0) s_sum[it & 1][warp] = s;
+      __syncthreads();
+      s = lane < nt / 32 ? s_sum[it & 1][lane] : 0.f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    }
+    const float lse = logf(s);
+    const float2 nl2 = make_float2(-lse, -lse);
+    int64_t t = p.targets_64 ? static_cast<const int64_t*>(p.targets)[row] : static_cast<const int32_t*>(p.targets)[row];
+    t = t < 0 ? 0 : (t >= p.vocab ? p.vocab - 1 : t);                 // clamped, as jnp.take_along_axis does
+    const int at = int(t) + now.off, piece = at >> 3;                 // the target's place in the row's pieces
+    const bool own = piece >= now.first && piece < now.last && (piece - now.first) % nt == tid;
+    // ---- the gradient: gscale / rows * (exp(z - lse) - [target]) * (1 - t^2)
+    if (p.d != nullptr) {
+      __nv_bfloat16* dp = p.d + (now.base - p.logits);
+      for (int i = now.first + tid; i < now.last; i += nt) {
+        const uint4 tw = row_t[i];
+        const uint32_t ti[4] = {tw.x, tw.y, tw.z, tw.w};
+        uint4 o;
+        uint32_t* op = &o.x;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 tf = bf16x2_unpack(ti[j]);
+          const float2 zl = __fmul2_rn(__fadd2_rn(capped(ti[j]), nl2), l2e);
+          const float2 pr = __fmul2_rn(make_float2(ex2(zl.x), ex2(zl.y)), gs2);
+          const float2 r = __fmul2_rn(pr, __ffma2_rn(__fmul2_rn(tf, tf), minus1, one));   // t^2 is exact
+          op[j] = pack_bf16x2(r.x, r.y);
+        }
+        *reinterpret_cast<uint4*>(dp + i * 8) = o;
+      }
+      if (e_mine >= 0) dp[e_mine] = grad1(bf16lo(t_edge), capped(t_edge).x, lse, e_mine == at);
+      if (own) {                                                      // the target's own element again, now with its -1
+        const uint32_t t2 = row_e[at];
+        dp[at] = grad1(bf16lo(t2), capped(t2).x, lse, true);
+      }
+    }
+    // ---- the target's log-probability, by the thread that holds it
+    if (p.nll != nullptr) {
+      if (own) p.nll[row] = lse - capped(row_e[at]).x;
+      if (e_mine == at) p.nll[row] = lse - capped(t_edge).x;
+    }
+  }
+}
+
+// mean of n floats, in a fixed order
+__global__ void __launch_bounds__(1024) mean_kernel(const float* __restrict__ v, int n, float* __restrict__ out) {
+  __shared__ float s_part[32];
+  float a = 0.f, b = 0.f;
+  for (int i = threadIdx.x; i < n; i += 2048) {
+    a += v[i];
+    if (i + 1024 < n) b += v[i + 1024];
+  }
+  a += b;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = a;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    a = s_part[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (threadIdx.x == 0) *out = a / float(n);
+  }
+}
+
+constexpr int kCeSmemMax = 226 * 1024;
+static int64_t ce_smem(int64_t vocab) {
+  const int64_t row = (vocab + 14) / 8 * 16;
+  return kCeTableBytes + (vocab <= kCeWarpCols ? 8 * row : row);
+}
+
 }  // namespace tg
 
 using namespace tg;
+
+extern "C" int tgh_softcap_ce_fits(float cap, int64_t rows, int64_t vocab) {
+  // the cap: exp(cap) and the table's exponents stay in range (see softcap_ce_kernel)
+  return cap >= 0x1p-10f && cap <= 64.0f && rows <= INT32_MAX && vocab > 0 && vocab < (1 << 24) && ce_smem(vocab) <= kCeSmemMax;
+}
+
+extern "C" int tgh_softcap_ce(const void* logits, const void* targets, int targets_64, float cap, void* dlogits, const float* gscale,
+                              int only_if_scaled, float* nll, float* loss, int64_t rows, int64_t vocab, int64_t ld, void* stream) {
+  if (rows < 0 || vocab <= 0 || ld < vocab || (loss != nullptr && nll == nullptr) || (only_if_scaled && gscale == nullptr))
+    return TG_ERR_SHAPE;
+  if (!tgh_softcap_ce_fits(cap, rows, vocab)) return TG_ERR_TOO_LARGE;
+  if (!aligned16(logits) || !aligned16(dlogits)) return TG_ERR_ALIGN;
+  if (int rc = check_arch()) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  CeArgs a = {static_cast<const __nv_bfloat16*>(logits), targets, targets_64, cap, static_cast<__nv_bfloat16*>(dlogits), gscale,
+              only_if_scaled, nll, int(rows), int(vocab), ld};
+  if (rows > 0) {
+    static std::atomic<bool> attr_set[64];
+    int dev = 0;
+    TG_CUDA_CHECK(cudaGetDevice(&dev));
+    if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
+      TG_CUDA_CHECK(cudaFuncSetAttribute(softcap_ce_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeSmemMax));
+      TG_CUDA_CHECK(cudaFuncSetAttribute(softcap_ce_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeSmemMax));
+      attr_set[dev & 63].store(true, std::memory_order_release);
+    }
+    const size_t smem = size_t(ce_smem(vocab));
+    const int64_t per_sm_smem = std::max<int64_t>(1, (227 * 1024) / int64_t(smem + 1024));
+    if (vocab <= kCeWarpCols) {
+      const int64_t cap_blocks = int64_t(sm_count()) * std::min<int64_t>(per_sm_smem, 4);
+      softcap_ce_kernel<true><<<int(std::min<int64_t>((rows + 7) / 8, cap_blocks)), 256, smem, st>>>(a);
+    } else {
+      // as many threads as make the last pass over the row nearly full (of at most 640: two blocks an SM at 48 registers)
+      const int64_t pieces = (vocab + 7) / 8;
+      int nt = kCeMaxThreads;
+      double best = 0.0;
+      for (int n = kCeMaxThreads; n >= 256; n -= 32) {
+        const double full = double(pieces) / double((pieces + n - 1) / n * n);
+        if (full > best + 0.02) { best = full; nt = n; }
+      }
+      const int64_t cap_blocks = int64_t(sm_count()) * std::min<int64_t>(per_sm_smem, 1280 / nt);
+      softcap_ce_kernel<false><<<int(std::min<int64_t>(rows, cap_blocks)), nt, smem, st>>>(a);
+    }
+    TG_CUDA_CHECK(cudaGetLastError());
+  }
+  if (loss != nullptr) {
+    mean_kernel<<<1, 1024, 0, st>>>(nll, int(rows), loss);
+    TG_CUDA_CHECK(cudaGetLastError());
+  }
+  return TG_OK;
+}
 
 extern "C" int tg_softcap_ce_fwd(const void* logits, const int32_t* targets, float cap, void* tanh_out, float* lse,
                                  float* nll, int64_t rows, int64_t vocab, int64_t ld, int64_t ld_tanh, void* stream) {
