@@ -282,3 +282,44 @@ def test_wider_inputs_are_taken_only_if_they_hold_bf16_values():
         fp8.block_scaled_matmul(a.float() + 1e-4, b)
     with pytest.raises(TypeError, match="bf16 cannot hold"):
         fp8._quantize_to_fp8(torch.full((2, 128), 1.0 + 2.0 ** -12, device="cuda"))
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 128, 1), (5, 256, 7), (130, 128, 130), (64, 384, 257), (3, 2176, 1000), (300, 128, 4099)])
+def test_ragged_weight_width(M, K, N):
+    """Weights whose rows start at any alignment (N no multiple of 8): quantised by column straight from where they lie, and as a
+    column slice of a wider matrix; forward against the oracle, gradients of the straight-through mode against torch."""
+    from train_gpt_b200 import fp8
+    rng = np.random.default_rng(M + K + N)
+    a, b = normal_bf16(rng, (M, K), outlier_p=1e-3), normal_bf16(rng, (K, N), std=0.02)
+    ref = fo.block_scaled_matmul(a, b)
+    wide = torch.zeros(K, N + 13, dtype=torch.bfloat16, device="cuda")
+    wide[:, 3:3 + N] = to_torch_bf16(b)
+    for w in (to_torch_bf16(b), wide[:, 3:3 + N]):
+        at = to_torch_bf16(a).requires_grad_(True)
+        wt = w.detach().requires_grad_(True)
+        y = fp8.block_scaled_matmul(at, wt)
+        assert y.shape == (M, N)
+        _close(from_torch_bf16(y.detach()), ref)
+        g = to_torch_bf16(normal_bf16(rng, (M, N)))
+        y.backward(g)
+        assert torch.equal(at.grad, g @ w.t()) and torch.equal(wt.grad, at.detach().t() @ g)
+
+
+@pytest.mark.parametrize("M,K,N", [(100, 128, 128), (1000, 512, 384), (3000, 2048, 2048)])
+@pytest.mark.parametrize("tile,mode", [((128, 128), "fp8"), ((128, 1), "fp8"), ((128, 128), "fp8_blockgrad")])
+def test_linear_quantises_alike_in_one_launch_and_in_several(M, K, N, tile, mode):
+    """The linear's own quantiser launches (several tensors in one, or one each past a size) against the separate entry points,
+    through the GEMMs: bit-identical results."""
+    from train_gpt_b200 import fp8, ops
+    rng = np.random.default_rng(M + K + N)
+    a, b, g = (to_torch_bf16(normal_bf16(rng, s, std=d)) for s, d in (((M, K), 1.0), ((K, N), 0.02), ((M, N), 1.0)))
+    at, bt = a.clone().requires_grad_(True), b.clone().requires_grad_(True)
+    y = fp8.block_scaled_matmul(at, bt, weight_tile=tile, backward=mode)
+    y.backward(g)
+    w = fp8.quantize_weight(b, tile)
+    wd = ops.quantize_rowwise(b) if tile == (128, 1) else w
+    gt = (128, 1) if mode == "fp8" else (128, 128)
+    gc = ops.quantize_colwise(g) if mode == "fp8" else ops.quantize_block128(g)
+    assert torch.equal(y.detach(), ops.gemm_fwd(*ops.quantize_rowwise(a), *w, tile))
+    assert torch.equal(at.grad, ops.gemm_dgrad(*ops.quantize_rowwise(g), *wd, tile))
+    assert torch.equal(bt.grad, ops.gemm_wgrad(*ops.quantize_colwise(a), *gc, grad_tile=gt))

@@ -51,7 +51,7 @@ const auto kF8 = at::kFloat8_e4m3fn;
   X(tg_act_quantize_rowcol) X(tg_quantize_block128) X(tg_rmsnorm_fwd) X(tg_rmsnorm_quant_fwd)                       \
   X(tg_add_rmsnorm_quant_fwd) X(tg_rmsnorm_bwd_scratch_bytes) X(tg_rmsnorm_bwd) X(tg_rmsnorm_bwd_add)               \
   X(tg_softcap_ce_fwd) X(tg_softcap_ce_bwd) X(tg_sumsq_scratch_bytes) X(tg_sumsq_bf16) X(tg_adamw_bf16)             \
-  X(tg_gemm_workspace_bytes) X(tg_gemm_fp8_blockscaled) X(tgh_softcap_ce_fits) X(tgh_softcap_ce)
+  X(tg_gemm_workspace_bytes) X(tg_gemm_fp8_blockscaled) X(tgh_quantize_jobs) X(tgh_softcap_ce_fits) X(tgh_softcap_ce)
 
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;
@@ -503,88 +503,263 @@ Linear validate(const Tensor& a, const Tensor& b, int64_t block_k) {
   return {k, b.size(1)};
 }
 
-struct ForwardOut {
-  Tensor y;                 // (..., N)
-  Tensor w_q, w_s;          // the weight as the forward GEMM read it
-  Tensor x_qc, x_sc;        // the activation's column form, if it was made here
+// Device memory for several temporaries of one call, or for what a node keeps, as ONE allocation: a caching-allocator
+// round trip costs about as much host time as a third of a launch, and a linear has up to ten such buffers.
+class Arena {
+ public:
+  size_t add(int64_t bytes) {
+    const size_t at = size_;
+    size_ += (size_t(bytes) + 255) / 256 * 256;
+    return at;
+  }
+  void make(const Tensor& like) {
+    if (size_ > 0) memory_ = empty({int64_t(size_)}, at::kByte, like);
+    base_ = size_ > 0 ? static_cast<uint8_t*>(memory_.data_ptr()) : nullptr;
+  }
+  void* at(size_t offset) const { return base_ + offset; }
+  const Tensor& memory() const { return memory_; }
+
+ private:
+  size_t size_ = 0;
+  uint8_t* base_ = nullptr;
+  Tensor memory_;
 };
 
-// fp8.py:50-78.  row_q / row_s: the activation's row form made earlier.  want_col: also make its column form, which
-// the weight gradient contracts, from the same read.
-ForwardOut fp8_forward(const Tensor& a, const Tensor& b_, bool w_cols, const Tensor& row_q, const Tensor& row_s, bool want_col) {
+// One quantised matrix: e4m3 bytes and float32 scales
+struct Form {
+  void* q = nullptr;
+  float* s = nullptr;
+  explicit operator bool() const { return q != nullptr; }
+};
+struct FormAt {
+  size_t q = 0, s = 0;
+  Form in(const Arena& m) const { return {m.at(q), static_cast<float*>(m.at(s))}; }
+};
+FormAt add_row(Arena& m, int64_t rows, int64_t cols) { return {m.add(rows * cols), m.add(rows * (cols / kTile) * 4)}; }
+FormAt add_col(Arena& m, int64_t rows, int64_t cols) { return {m.add(rows * cols), m.add(cdiv(rows, kTile) * cols * 4)}; }
+FormAt add_block(Arena& m, int64_t rows, int64_t cols) { return {m.add(rows * cols), m.add(cdiv(rows, kTile) * (cols / kTile) * 4)}; }
+
+// A 2-D bf16 matrix the quantisers can read as it lies: unit stride along a row and, unless it is only wanted by column,
+// rows at 16-byte boundaries.  Anything else is copied.
+Tensor readable(const Tensor& t, bool any_alignment) {
+  if (t.stride(1) == 1 && (t.size(0) <= 1 || t.stride(0) >= t.size(1)) &&
+      (any_alignment || ((t.size(0) <= 1 || t.stride(0) % 8 == 0) && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0)))
+    return t;
+  return t.contiguous();
+}
+int64_t pitch(const Tensor& t) { return t.size(0) > 1 ? t.stride(0) : t.size(1); }
+
+tgh_quantize_job job_of(const Tensor& x) {
+  tgh_quantize_job j = {};
+  j.x = x.data_ptr();
+  j.rows = x.size(0);
+  j.cols = x.size(1);
+  j.ld = pitch(x);
+  return j;
+}
+void want_row(tgh_quantize_job& j, const Form& f) {
+  j.q_row = f.q; j.s_row = f.s; j.q_row_ld = j.cols; j.s_row_ld = j.cols / kTile;
+}
+void want_col(tgh_quantize_job& j, const Form& f, int64_t ld) {
+  j.form = TGH_FORM_COLUMNS; j.q = f.q; j.s = f.s; j.q_ld = j.s_ld = ld;
+}
+void want_block(tgh_quantize_job& j, const Form& f) {
+  j.form = TGH_FORM_BLOCKS; j.q = f.q; j.s = f.s; j.q_ld = j.cols; j.s_ld = j.cols / kTile;
+}
+
+// A GEMM of forms.  (rows of A, columns of B and their contraction; see gemm_fwd / gemm_dgrad / gemm_wgrad for the layouts)
+tg_gemm_args gemm_args(int64_t m, int64_t n, int64_t k, int64_t lda, int a_major, Strides sa, int64_t ldb, int b_major, Strides sb,
+                       bool per_column, int64_t ldd, bool f32, unsigned* status) {
+  tg_gemm_args g = {};
+  g.lda = lda; g.ldb = ldb; g.a_major = a_major; g.b_major = b_major;
+  g.sa_stride_m = sa.row; g.sa_stride_kb = sa.kb; g.sb_stride_n = sb.row; g.sb_stride_kb = sb.kb;
+  g.sb_gran_n = per_column ? 1 : int(kTile);
+  g.ldd = ldd; g.out_dtype = f32 ? TG_OUT_F32 : TG_OUT_BF16;
+  g.M = m; g.N = n; g.K = k;
+  g.status = status;
+  return g;
+}
+void run_gemm(tg_gemm_args& g, const Form& a, const Form& b, void* d, void* workspace, int64_t workspace_bytes) {
+  g.a = a.q; g.sa = a.s; g.b = b.q; g.sb = b.s;
+  g.d = d;
+  g.workspace = workspace_bytes > 0 ? workspace : nullptr;
+  g.workspace_bytes = workspace_bytes;
+  check(api.tg_gemm_fp8_blockscaled(&g, cur_stream()), "tg_gemm_fp8_blockscaled");
+  last_gemm_launches.store(workspace_bytes > 0 ? 2 : 1, std::memory_order_relaxed);
+}
+unsigned* status_of(const Tensor& like) { return static_cast<unsigned*>(ptr(status_word(like.get_device()))); }
+
+int64_t rows_of(const Tensor& a) {
+  int64_t m = 1;
+  for (int64_t i = 0; i + 1 < a.dim(); ++i) m *= a.size(i);
+  return m;
+}
+
+// the 1x128 form of an activation as its caller has it
+Pair row_form(const Tensor& q, const Tensor& s, int64_t k) {
+  if (!q.defined()) return {};
+  if (q.scalar_type() != kF8 || s.scalar_type() != at::kFloat)
+    throw py::type_error(cat("a_quantized must be an e4m3 and a float32 tensor, got ", dtype_name(q.scalar_type()), " and ", dtype_name(s.scalar_type())));
+  return {q.reshape({-1, k}).contiguous(), s.reshape({-1, k / kTile}).contiguous()};
+}
+
+struct ForwardOut {
+  Tensor y;                 // (..., N)
+  Tensor kept;              // memory of the two below
+  Form w;                   // the weight in 128x128 tiles: dgrad reads it too
+  Form x_col;               // the activation's column form, which the weight gradient contracts
+};
+
+// fp8.py:50-78.  row_q / row_s: the activation's row form made earlier.  keep_x / keep_w: what the backward pass will want
+// of the activation (its column form, from the same read) and of the weight outlives the call.
+ForwardOut fp8_forward(const Tensor& a, const Tensor& b_, bool w_cols, const Tensor& row_q, const Tensor& row_s, bool keep_x, bool keep_w) {
   ForwardOut o;
-  const int64_t k = a.size(-1), n = b_.size(1);
-  Tensor a_q = row_q, a_s = row_s;
-  if (!a_q.defined()) {
-    const Tensor a2 = as_bf16(a.reshape({-1, k}), "a");
-    if (want_col) {
-      const RowCol rc = quantize_rowcol(a2);
-      a_q = rc.q_row; a_s = rc.s_row; o.x_qc = rc.q_col; o.x_sc = rc.s_col;
-    } else {
-      std::tie(a_q, a_s) = quantize_rowwise(a2);
-    }
+  const int64_t k = a.size(-1), n = b_.size(1), m = rows_of(a);
+  Tensor x;
+  if (!row_q.defined()) {
+    x = as_bf16(a, "a").reshape({m, k});
+    if (!x.is_cuda()) need(x, at::kBFloat16, "x");
+    x = readable(x, false);
   }
   Tensor b = as_bf16(b_, "b");
-  const int64_t pad = w_cols ? (16 - n % 16) % 16 : 0;
-  // the TMA row pitch of the (K, N) weight must be a multiple of 16 bytes: widen with zero columns (their tiles
-  // quantise to zeros) and drop them from the result
-  if (pad) b = at::constant_pad_nd(b, {0, pad});
-  std::tie(o.w_q, o.w_s) = w_cols ? quantize_colwise(b) : quantize_block128(b);
-  Tensor y = gemm_fwd(a_q, a_s, o.w_q, o.w_s, w_cols, at::kBFloat16, Tensor());
-  if (pad) y = y.narrow(1, 0, n);
-  if (a.dim() == 2) {
-    o.y = y;
-  } else {
-    std::vector<int64_t> shape = with_last(a, n);
-    o.y = y.reshape(shape);
+  if (!b.is_cuda()) need(b, at::kBFloat16, "x");
+  if (!w_cols && n % kTile) throw py::value_error(cat("C=", n, " not divisible by ", kTile));
+  b = readable(b, w_cols);
+  const c10::cuda::CUDAGuard guard(b.device());
+  // the TMA row pitch of the (K, N) weight must be a multiple of 16 bytes: its quantised form is widened with zero
+  // columns and the result's extra columns are dropped
+  const int64_t np = w_cols ? cdiv(n, 16) * 16 : n;
+  o.y = empty(with_last(a, np), at::kBFloat16, b);
+  tg_gemm_args g = gemm_args(m, np, k, k, TG_MAJOR_K, {k / kTile, 1}, np, TG_MAJOR_MN, {1, w_cols ? np : n / kTile}, w_cols, np, false,
+                             status_of(b));
+  const int64_t ws_bytes = api.tg_gemm_workspace_bytes(&g);
+  Arena kept, temp;
+  FormAt x_row_at, x_col_at, w_at;
+  if (x.defined()) {
+    x_row_at = add_row(temp, m, k);
+    if (keep_x) x_col_at = add_col(kept, m, k);
   }
+  w_at = w_cols ? add_col(temp, k, np) : add_block(keep_w ? kept : temp, k, n);
+  const size_t ws_at = temp.add(ws_bytes);
+  kept.make(b);
+  temp.make(b);
+  tgh_quantize_job jobs[2];
+  int n_jobs = 0;
+  Form x_row = {ptr(row_q), fptr(row_s)};
+  if (x.defined()) {
+    tgh_quantize_job& j = jobs[n_jobs++] = job_of(x);
+    want_row(j, x_row = x_row_at.in(temp));
+    if (keep_x) want_col(j, o.x_col = x_col_at.in(kept), k);
+  }
+  tgh_quantize_job& j = jobs[n_jobs++] = job_of(b);
+  Form w = w_at.in(!w_cols && keep_w ? kept : temp);
+  if (w_cols) want_col(j, w, np);
+  else want_block(j, w);
+  check(api.tgh_quantize_jobs(jobs, n_jobs, cur_stream()), "tgh_quantize_jobs");
+  run_gemm(g, x_row, w, ptr(o.y), temp.at(ws_at), ws_bytes);
+  if (np != n) {
+    o.y = o.y.narrow(-1, 0, n);
+    if (o.y.dim() != 2) o.y = o.y.contiguous();
+  }
+  o.kept = kept.memory();
+  if (!w_cols && keep_w) o.w = w;
   return o;
 }
 
 struct BackwardIn {
   bool w_cols;
   Mode mode;
-  Tensor w_q, w_s;                                   // the forward's 128x128 weight tiles, reused by dgrad
-  std::function<Pair()> x_col;                       // the activation's column form
+  Form w;                                            // the forward's 128x128 weight tiles, reused by dgrad
+  Form x_col;                                        // the activation's column form
   std::function<Tensor()> slot_take;                 // where the weight gradient goes instead of a new tensor ...
   std::function<void()> slot_ready;                  // ... and whom to tell that it is there
   bool want_a = true, want_b = true;
 };
 
 // fp8.py:85-98 (mode kSte), or the same two GEMMs in block-scaled e4m3
-Pair fp8_backward(const Tensor& a, const Tensor& b, const Tensor& g, at::IntArrayRef a_shape, at::ScalarType a_dtype,
+Pair fp8_backward(const Tensor& a, const Tensor& b, const Tensor& g_, at::IntArrayRef a_shape, at::ScalarType a_dtype,
                   at::ScalarType b_dtype, int64_t k, int64_t n, const BackwardIn& in) {
-  const Tensor g2 = g.reshape({-1, n}).to(at::kBFloat16);
   Tensor da, db;
   if (in.mode == kSte) {
+    const Tensor g2 = g_.reshape({-1, n}).to(at::kBFloat16);
     if (in.want_a) da = at::mm(g2, b.to(at::kBFloat16).t());                                 // fp8.py:96 (cuBLAS bf16)
     if (in.want_b) db = at::mm(a.reshape({-1, k}).to(at::kBFloat16).t(), g2);                // fp8.py:97
-  } else {
-    TORCH_CHECK_VALUE(n % kTile == 0, "N=", n, " not divisible by block_k=", kTile, " (needed by the FP8 dgrad)");
-    RowCol gq;
-    if (in.mode == kFp8) {
-      gq = quantize_rowcol(g2);                                                              // one read of g for both contractions
-    } else {
-      std::tie(gq.q_row, gq.s_row) = quantize_rowwise(g2);
-      std::tie(gq.q_col, gq.s_col) = quantize_block128(g2);
-    }
-    if (in.want_a) {
-      Tensor w_q = in.w_q, w_s = in.w_s;
-      if (!w_q.defined()) std::tie(w_q, w_s) = in.w_cols ? quantize_rowwise(b.to(at::kBFloat16)) : quantize_block128(b.to(at::kBFloat16));
-      da = gemm_dgrad(gq.q_row, gq.s_row, w_q, w_s, in.w_cols, at::kBFloat16, Tensor());
-    }
+    if (da.defined()) da = (a_shape.size() == 2 ? da : da.reshape(a_shape)).to(a_dtype);
+    if (db.defined()) db = db.to(b_dtype);
+    return {da, db};
+  }
+  TORCH_CHECK_VALUE(n % kTile == 0, "N=", n, " not divisible by block_k=", kTile, " (needed by the FP8 dgrad)");
+  if (!in.want_a && !in.want_b) return {da, db};
+  int64_t m = 1;
+  for (size_t i = 0; i + 1 < a_shape.size(); ++i) m *= a_shape[i];
+  const Tensor g = readable(g_.reshape({m, n}).to(at::kBFloat16), false);
+  const c10::cuda::CUDAGuard guard(g.device());
+  const bool g_cols = in.mode == kFp8;               // the weight gradient's upstream operand: columns, or 128x128 tiles
+  unsigned* status = status_of(g);
+  tg_gemm_args dgrad, wgrad;
+  Tensor db_slot;
+  int64_t ws_bytes[2] = {0, 0};
+  if (in.want_a) {
+    da = empty(a_shape, at::kBFloat16, g);
+    dgrad = gemm_args(m, k, n, n, TG_MAJOR_K, {n / kTile, 1}, n, TG_MAJOR_K, {n / kTile, 1}, in.w_cols, k, false, status);
+    ws_bytes[0] = api.tg_gemm_workspace_bytes(&dgrad);
+  }
+  if (in.want_b) {
+    if (in.slot_take) db_slot = in.slot_take();
+    else db = empty({k, n}, at::kBFloat16, g);
+    const Tensor& out = in.slot_take ? db_slot : db;
+    if (out.sizes() != at::IntArrayRef({k, n}) || out.stride(1) != 1 || !out.is_cuda() ||
+        (out.scalar_type() != at::kBFloat16 && out.scalar_type() != at::kFloat))
+      throw py::value_error(cat("out must be a (", k, ", ", n, ") bf16 or float32 CUDA tensor with unit inner stride"));
+    wgrad = gemm_args(k, n, m, k, TG_MAJOR_MN, {1, k}, n, TG_MAJOR_MN, {1, g_cols ? n : n / kTile}, g_cols, pitch(out),
+                      out.scalar_type() == at::kFloat, status);
+    ws_bytes[1] = api.tg_gemm_workspace_bytes(&wgrad);
+  }
+  // everything that is still to be quantised, in one launch: g once for both contractions, the weight along N, the activation
+  Arena temp;
+  FormAt g_row_at, g_col_at, w_at, x_at;
+  const bool make_w = in.want_a && (in.w_cols || !in.w), make_x = in.want_b && !in.x_col;
+  if (in.want_a) g_row_at = add_row(temp, m, n);
+  if (in.want_b) g_col_at = g_cols ? add_col(temp, m, n) : add_block(temp, m, n);
+  if (make_w) w_at = in.w_cols ? add_row(temp, k, n) : add_block(temp, k, n);
+  if (make_x) x_at = add_col(temp, m, k);
+  const size_t ws_at = temp.add(std::max(ws_bytes[0], ws_bytes[1]));
+  temp.make(g);
+  tgh_quantize_job jobs[3];
+  int n_jobs = 0;
+  Form g_row, g_col, w = in.w, x = in.x_col;
+  {
+    tgh_quantize_job& j = jobs[n_jobs++] = job_of(g);
+    if (in.want_a) want_row(j, g_row = g_row_at.in(temp));
     if (in.want_b) {
-      const Pair x = in.x_col ? in.x_col() : quantize_colwise(a.reshape({-1, k}).to(at::kBFloat16));
-      if (in.slot_take) {
-        gemm_wgrad(x.first, x.second, gq.q_col, gq.s_col, in.mode == kFp8, at::kBFloat16, Tensor(), in.slot_take());
-        in.slot_ready();
-      } else {
-        db = gemm_wgrad(x.first, x.second, gq.q_col, gq.s_col, in.mode == kFp8, at::kBFloat16, Tensor(), Tensor());
-      }
+      g_col = g_col_at.in(temp);
+      if (g_cols) want_col(j, g_col, n);
+      else want_block(j, g_col);
     }
   }
-  if (da.defined()) da = (a_shape.size() == 2 ? da : da.reshape(a_shape)).to(a_dtype);
-  if (db.defined()) db = db.to(b_dtype);
+  Tensor b2, a2;
+  if (make_w) {
+    b2 = readable(b.to(at::kBFloat16), false);
+    tgh_quantize_job& j = jobs[n_jobs++] = job_of(b2);
+    w = w_at.in(temp);
+    if (in.w_cols) want_row(j, w);
+    else want_block(j, w);
+  }
+  if (make_x) {
+    a2 = readable(a.reshape({m, k}).to(at::kBFloat16), false);
+    tgh_quantize_job& j = jobs[n_jobs++] = job_of(a2);
+    want_col(j, x = x_at.in(temp), k);
+  }
+  check(api.tgh_quantize_jobs(jobs, n_jobs, cur_stream()), "tgh_quantize_jobs");
+  if (in.want_a) {
+    run_gemm(dgrad, g_row, w, ptr(da), temp.at(ws_at), ws_bytes[0]);
+    da = da.to(a_dtype);
+  }
+  if (in.want_b) {
+    run_gemm(wgrad, x, g_col, ptr(db.defined() ? db : db_slot), temp.at(ws_at), ws_bytes[1]);
+    if (in.slot_take) in.slot_ready();
+    else db = db.to(b_dtype);
+  }
   return {da, db};
 }
 
@@ -621,7 +796,8 @@ std::shared_ptr<PyHandle> hold(const py::object& o) { return o.is_none() ? nullp
 struct BlockScaledMatmulBackward : public Node {
   SavedVariable a, b;                        // the unquantised residuals (fp8.py:81-82) that the mode needs
   bool has_a = false, has_b = false, released = false;
-  Tensor w_q, w_s, x_qc, x_sc;
+  Tensor kept;                               // memory of `w` and `x_col`
+  Form w, x_col;
   std::shared_ptr<PyHandle> activation, slot;
   std::vector<int64_t> a_shape;
   at::ScalarType a_dtype, b_dtype;
@@ -634,7 +810,7 @@ struct BlockScaledMatmulBackward : public Node {
   void release_variables() override {
     a.reset_data();
     b.reset_data();
-    w_q = w_s = x_qc = x_sc = Tensor();
+    kept = Tensor();
     activation.reset();
     slot.reset();
     released = true;
@@ -649,14 +825,13 @@ struct BlockScaledMatmulBackward : public Node {
     in.mode = mode;
     in.want_a = task_should_compute_output(0);
     in.want_b = task_should_compute_output(1);
-    if (!w_cols && mode != kSte) { in.w_q = w_q; in.w_s = w_s; }
-    if (x_qc.defined()) {
-      in.x_col = [this] { return Pair(x_qc, x_sc); };
-    } else if (activation) {
-      in.x_col = [this] {
-        py::gil_scoped_acquire gil;
-        return activation->get().attr("colwise")().cast<Pair>();
-      };
+    in.w = w;
+    in.x_col = x_col;
+    Pair shared;                             // the activation's own column form, made on first use and kept by it
+    if (activation && !x_col && in.want_b && mode != kSte) {
+      py::gil_scoped_acquire gil;
+      shared = activation->get().attr("colwise")().cast<Pair>();
+      in.x_col = {ptr(shared.first), fptr(shared.second)};
     }
     if (slot) {
       in.slot_take = [this] {
@@ -679,15 +854,12 @@ Tensor block_scaled_matmul(const Tensor& a, const Tensor& b, int64_t block_k, bo
   const Linear d = validate(a, b, block_k);
   const Mode mode = Mode(mode_);
   const bool track = at::GradMode::is_enabled() && (a.requires_grad() || b.requires_grad());
-  Tensor rq = row_q, rs = row_s;
-  if (rq.defined()) {
-    rq = rq.reshape({-1, d.k});
-    rs = rs.reshape({-1, d.k / kTile});
-  }
+  const auto [rq, rs] = row_form(row_q, row_s, d.k);
+  const bool keep = track && mode != kSte, keep_x = keep && b.requires_grad() && activation.is_none() && !rq.defined();
   ForwardOut f;
   {
     at::AutoDispatchBelowADInplaceOrView below;     // none of what happens here is recorded: the node below is the derivative
-    f = fp8_forward(a, b, w_cols, rq, rs, track && b.requires_grad() && mode != kSte && activation.is_none());
+    f = fp8_forward(a, b, w_cols, rq, rs, keep_x, keep);
   }
   if (!track) return f.y;
   std::shared_ptr<BlockScaledMatmulBackward> node(new BlockScaledMatmulBackward(), torch::autograd::deleteNode);
@@ -699,13 +871,13 @@ Tensor block_scaled_matmul(const Tensor& a, const Tensor& b, int64_t block_k, bo
   node->b_dtype = b.scalar_type();
   node->w_cols = w_cols;
   node->mode = mode;
-  node->has_a = mode == kSte || (!f.x_qc.defined() && activation.is_none());
+  node->has_a = mode == kSte || (!f.x_col && activation.is_none());
   node->has_b = mode == kSte || w_cols;
   if (node->has_a) node->a = SavedVariable(a, false);
   if (node->has_b) node->b = SavedVariable(b, false);
-  if (!w_cols && mode != kSte) { node->w_q = f.w_q; node->w_s = f.w_s; }
-  node->x_qc = f.x_qc;
-  node->x_sc = f.x_sc;
+  node->kept = f.kept;
+  node->w = f.w;
+  node->x_col = f.x_col;
   node->activation = hold(activation);
   node->slot = hold(slot);
   torch::autograd::set_history(f.y, node);
@@ -910,22 +1082,20 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("fp8_forward", [](const Tensor& a, const Tensor& b, int64_t block_k, bool w_cols, const std::optional<Tensor>& row_q,
                           const std::optional<Tensor>& row_s) {
     const Linear d = validate(a, b, block_k);
-    Tensor rq = or_none(row_q), rs = or_none(row_s);
-    if (rq.defined()) {
-      rq = rq.reshape({-1, d.k});
-      rs = rs.reshape({-1, d.k / kTile});
-    }
-    const ForwardOut f = fp8_forward(a, b, w_cols, rq, rs, false);
-    return py::make_tuple(f.y, f.w_q, f.w_s);
+    const auto [rq, rs] = row_form(or_none(row_q), or_none(row_s), d.k);
+    return fp8_forward(a, b, w_cols, rq, rs, false, false).y;
   });
   m.def("fp8_backward", [](const Tensor& a, const Tensor& b, const Tensor& g, bool w_cols, int mode, const py::object& activation,
                            const std::optional<Tensor>& w_q, const std::optional<Tensor>& w_s, const py::object& slot) {
     BackwardIn in;
     in.w_cols = w_cols;
     in.mode = Mode(mode);
-    in.w_q = or_none(w_q);
-    in.w_s = or_none(w_s);
-    if (!activation.is_none()) in.x_col = [&] { return activation.attr("colwise")().cast<Pair>(); };
+    in.w = {ptr(or_none(w_q)), fptr(or_none(w_s))};
+    Pair shared;
+    if (!activation.is_none() && in.mode != kSte) {
+      shared = activation.attr("colwise")().cast<Pair>();
+      in.x_col = {ptr(shared.first), fptr(shared.second)};
+    }
     if (!slot.is_none()) {
       in.slot_take = [&] { return slot.attr("take")().cast<Tensor>(); };
       in.slot_ready = [&] { slot.attr("ready")(); };

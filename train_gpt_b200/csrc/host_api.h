@@ -10,6 +10,21 @@
 extern "C" {
 #endif
 
+/* One tensor to quantise: bf16 [rows, cols] of pitch ld in its 1 x 128 form (q_row / s_row, or NULL), and / or a second form
+ * (q / s): a scale per column per 128 rows, or one per 128 x 128 tile.  Pitches of the e4m3 outputs are multiples of 16.
+ * Any number of columns for the column form (also rows that do not start at 16-byte boundaries, where ld is no multiple
+ * of 8); with cols % 8 != 0 its q and s get q_ld columns, the extra ones quantised zeros. */
+enum { TGH_FORM_NONE = 0, TGH_FORM_COLUMNS = 1, TGH_FORM_BLOCKS = 2 };
+typedef struct {
+  const void* x;
+  int64_t rows, cols, ld;
+  void* q_row; float* s_row; int64_t q_row_ld, s_row_ld;
+  int form;
+  void* q; float* s; int64_t q_ld, s_ld;
+} tgh_quantize_job;
+/* Up to six of them in one launch. */
+int tgh_quantize_jobs(const tgh_quantize_job* jobs, int n, void* stream);
+
 /* Whether tgh_softcap_ce takes this problem (a row and its cap fit the one-pass kernel). */
 int tgh_softcap_ce_fits(float cap, int64_t rows, int64_t vocab);
 /* Mean capped cross-entropy AND its gradient from one read of the logits.

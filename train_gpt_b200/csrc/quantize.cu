@@ -3,6 +3,7 @@
 // element, every input byte read once with 128-bit loads and kept in registers between
 // the amax pass and the divide pass.
 #include "common.cuh"
+#include "host_api.h"
 
 namespace tg {
 
@@ -43,9 +44,9 @@ quantize_rowwise_kernel(const uint4* __restrict__ x, uint2* __restrict__ q,
 }
 
 // ---------------------------------------------------------------------------------------
-// 128 x 1 tiles (a scale per column per block of 128 rows).  A thread block owns a
-// 128-row x 128-column panel: a half-warp spans the 128 columns (16 lanes x 8 columns), so
-// each of the 16 half-warps owns every 16th row (8 rows per thread, kept in registers).
+// Panels: what needs a scale per column per 128 rows (128 x 1 tiles), per 128 x 128 tile, or the 1 x 128 form beside
+// either.  A thread block owns a 128-row x 128-column panel: a half-warp spans the 128 columns (16 lanes x 8
+// columns), so each of the 16 half-warps owns every 16th row (8 rows per thread, kept in registers).
 // Column maxima are combined across the warps through shared memory (one thread per column
 // finishes the reduction and the reciprocal), then the same registers are divided and stored.
 // 64 registers: four blocks per SM, so one block's loads overlap the others' arithmetic.
@@ -149,32 +150,61 @@ __device__ __forceinline__ uint4 act_apply(uint4 x, uint4 g) {
   return make_uint4(act_pair<ACT>(x.x, g.x), act_pair<ACT>(x.y, g.y), act_pair<ACT>(x.z, g.z), act_pair<ACT>(x.w, g.w));
 }
 
-// FULL: the panel lies wholly inside the tensor (all 128 rows, all 128 columns), the case of every block of
-// a launch whose sizes are multiples of 128: no bounds predicate is evaluated and row addresses are
+// The second form of a panel beside (or instead of) its 1 x 128 one.
+enum PanelForm { kNoForm = 0, kColForm = 1, kBlockForm = 2 };
+
+struct PanelJob {
+  const __nv_bfloat16* x;      // rows x cols, pitch ld
+  const __nv_bfloat16* gate;   // same layout; read by the *_BWD activations only
+  uint8_t* q_row;              // 1 x 128 form, or NULL
+  float* s_row;
+  uint8_t* q;                  // column or block form
+  float* s;
+  int64_t ld, q_row_ld, s_row_ld, q_ld, s_ld;
+  int rows, cols;
+  int out_cols;                // columns of the column form: >= cols, a multiple of 8; the extra ones are zeros
+  int tiles_x;                 // panels across
+  int first;                   // number of the job's first thread block
+  int form;                    // PanelForm
+};
+
+struct PanelSmem {
+  float max[kColThreads / 32][kColPanelCols];
+  __align__(16) float scale[kColPanelCols];
+  __align__(16) float rcp[kColPanelCols];
+};
+
+// Eight consecutive values of a row of which the first `valid` exist, at any alignment.
+__device__ __forceinline__ uint4 load8_ragged(const __nv_bfloat16* p, int valid) {
+  uint32_t v[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (j < valid) v[j >> 1] |= uint32_t(reinterpret_cast<const unsigned short*>(p)[j]) << (16 * (j & 1));
+  return make_uint4(v[0], v[1], v[2], v[3]);
+}
+
+// FULL: the panel lies wholly inside the tensor (all 128 rows, all 128 columns, rows at 16-byte boundaries), the case of
+// every block of a launch whose sizes are multiples of 128: no bounds predicate is evaluated and row addresses are
 // one 64-bit add apart.  (The kernel is bound by instruction issue; the per-opcode counters showed the
 // address arithmetic and the bounds branches of the general form to be a third of its instructions.)
-template <bool WITH_ROWS, int ACT, bool FULL>
-__device__ __forceinline__ void colwise_panel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q,
-                                              float* __restrict__ scales, uint8_t* __restrict__ q_row,
-                                              float* __restrict__ s_row, int64_t rows, int64_t cols,
-                                              const __nv_bfloat16* __restrict__ gate, int64_t q_row_ld, int64_t s_row_ld,
-                                              int64_t q_col_ld, int64_t s_col_ld, float (*s_max)[kColPanelCols],
-                                              float* s_scale, float* s_rcp) {
+// RAGGED: rows at any alignment, any number of columns (column form only).
+template <bool ROW, int FORM, int ACT, bool FULL, bool RAGGED = false>
+__device__ __forceinline__ void panel(const PanelJob& a, int bx, int by, PanelSmem& sm) {
   const int cx = threadIdx.x & 15, hw = threadIdx.x >> 4;
-  const int64_t col0 = int64_t(blockIdx.x) * kColPanelCols + cx * 8;
-  const int64_t row_blk = blockIdx.y;
-  const int64_t row0 = row_blk * kTile + hw;  // this thread's rows: row0 + 16 r
-  const bool col_ok = FULL || col0 < cols;    // cols % 8 == 0
+  const int col0 = bx * kColPanelCols + cx * 8;
+  const int64_t row0 = int64_t(by) * kTile + hw;     // this thread's rows: row0 + 16 r
+  const int64_t rows = a.rows;
 
   uint4 w[kColRowsPerThread];
   {
-    const __nv_bfloat16* xp = x + row0 * cols + col0;
-    const __nv_bfloat16* gp = gate + row0 * cols + col0;     // only dereferenced by the *_BWD variants
-    const int64_t step = int64_t(kColHalfWarps) * cols;
+    const __nv_bfloat16* xp = a.x + row0 * a.ld + col0;
+    const __nv_bfloat16* gp = a.gate + row0 * a.ld + col0;     // only dereferenced by the *_BWD variants
+    const int64_t step = int64_t(kColHalfWarps) * a.ld;
 #pragma unroll
     for (int r = 0; r < kColRowsPerThread; ++r, xp += step, gp += step) {
-      const bool ok = FULL || (col_ok && row0 + r * kColHalfWarps < rows);
-      w[r] = ok ? ld_nc_v4(xp) : make_uint4(0, 0, 0, 0);
+      const bool ok = FULL || row0 + r * kColHalfWarps < rows;
+      if constexpr (RAGGED) w[r] = load8_ragged(xp, ok ? a.cols - col0 : 0);
+      else w[r] = FULL || (ok && col0 < a.cols) ? ld_nc_v4(xp) : make_uint4(0, 0, 0, 0);
       if constexpr (ACT != TG_ACT_NONE) {
         uint4 g = make_uint4(0, 0, 0, 0);
         if constexpr (ACT == TG_ACT_RELU2_BWD || ACT == TG_ACT_GELU_BWD)
@@ -183,7 +213,7 @@ __device__ __forceinline__ void colwise_panel(const __nv_bfloat16* __restrict__ 
       }
     }
   }
-  if constexpr (WITH_ROWS) {   // cols % 128 == 0 here: every lane holds real columns
+  if constexpr (ROW) {   // cols % 128 == 0 here: every lane holds real columns
     // the 8 row tiles of a half-warp: one exchange leaves lane j with the amax of row j % 8
     uint32_t mr[kColRowsPerThread];
 #pragma unroll
@@ -193,10 +223,10 @@ __device__ __forceinline__ void colwise_panel(const __nv_bfloat16* __restrict__ 
     tile_scales_own<kColRowsPerThread>(exchange_tile_amax<kColRowsPerThread>(mr), sr, rr, s_mine, fin);
     {
       const int64_t row = row0 + int64_t(cx & 7) * kColHalfWarps;   // lane j of the half computed row r = j % 8
-      if (cx < kColRowsPerThread && (FULL || row < rows)) s_row[row * s_row_ld + blockIdx.x] = s_mine;
+      if (cx < kColRowsPerThread && (FULL || row < rows)) a.s_row[row * a.s_row_ld + bx] = s_mine;
     }
-    uint8_t* qp = q_row + row0 * q_row_ld + col0;
-    const int64_t step = int64_t(kColHalfWarps) * q_row_ld;
+    uint8_t* qp = a.q_row + row0 * a.q_row_ld + col0;
+    const int64_t step = int64_t(kColHalfWarps) * a.q_row_ld;
     // one branch around the whole loop, not one per row: a NaN or Inf anywhere in the warp's tiles is the rare case
     if (fin) {
 #pragma unroll
@@ -208,18 +238,37 @@ __device__ __forceinline__ void colwise_panel(const __nv_bfloat16* __restrict__ 
         if (FULL || row0 + r * kColHalfWarps < rows) *reinterpret_cast<uint2*>(qp) = quantize8(w[r], sr[r]);
     }
   }
+  if constexpr (FORM == kNoForm) return;
   uint32_t m2[4];  // packed |.|-maxima of column pairs (0,1) (2,3) (4,5) (6,7) over this thread's rows
   static_assert(kColRowsPerThread == 8, "the tree below takes 8 rows");
   m2[0] = absmax2_tree8(w[0].x, w[1].x, w[2].x, w[3].x, w[4].x, w[5].x, w[6].x, w[7].x);
   m2[1] = absmax2_tree8(w[0].y, w[1].y, w[2].y, w[3].y, w[4].y, w[5].y, w[6].y, w[7].y);
   m2[2] = absmax2_tree8(w[0].z, w[1].z, w[2].z, w[3].z, w[4].z, w[5].z, w[6].z, w[7].z);
   m2[3] = absmax2_tree8(w[0].w, w[1].w, w[2].w, w[3].w, w[4].w, w[5].w, w[6].w, w[7].w);
+  const int wp = threadIdx.x >> 5;
+  uint8_t* qp = a.q + row0 * a.q_ld + col0;
+  const int64_t step = int64_t(kColHalfWarps) * a.q_ld;
+  if constexpr (FORM == kBlockForm) {
+    uint32_t mb = __vmaxu2(__vmaxu2(m2[0], m2[1]), __vmaxu2(m2[2], m2[3]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mb = __vmaxu2(mb, __shfl_xor_sync(0xffffffffu, mb, o));
+    if ((threadIdx.x & 31) == 0) sm.scale[wp] = absmax_to_float(mb);
+    __syncthreads();
+    float m = sm.scale[0];
+#pragma unroll
+    for (int wv = 1; wv < kColThreads / 32; ++wv) m = max_nan(m, sm.scale[wv]);
+    const float sc = scale_from_amax(m);
+    if (threadIdx.x == 0) a.s[int64_t(by) * a.s_ld + bx] = sc;
+#pragma unroll
+    for (int r = 0; r < kColRowsPerThread; ++r, qp += step)
+      if (FULL || row0 + r * kColHalfWarps < rows) *reinterpret_cast<uint2*>(qp) = quantize8(w[r], sc);
+    return;
+  }
   // the two half-warps of a warp hold the same columns: combine them in registers first
 #pragma unroll
   for (int j = 0; j < 4; ++j) m2[j] = __vmaxu2(m2[j], __shfl_xor_sync(0xffffffffu, m2[j], 16));
-  const int wp = threadIdx.x >> 5;
   if ((threadIdx.x & 16) == 0) {
-    float4* dst = reinterpret_cast<float4*>(&s_max[wp][cx * 8]);
+    float4* dst = reinterpret_cast<float4*>(&sm.max[wp][cx * 8]);
     dst[0] = make_float4(__uint_as_float(m2[0] << 16), __uint_as_float(m2[0] & 0xffff0000u),
                          __uint_as_float(m2[1] << 16), __uint_as_float(m2[1] & 0xffff0000u));
     dst[1] = make_float4(__uint_as_float(m2[2] << 16), __uint_as_float(m2[2] & 0xffff0000u),
@@ -229,21 +278,21 @@ __device__ __forceinline__ void colwise_panel(const __nv_bfloat16* __restrict__ 
   // one thread per column finishes the maximum, derives scale and reciprocal once, and
   // publishes both (conflict-free: consecutive threads, consecutive words)
   if (threadIdx.x < kColPanelCols) {
-    float v = s_max[0][threadIdx.x];
+    float v = sm.max[0][threadIdx.x];
 #pragma unroll
-    for (int h = 1; h < kColThreads / 32; ++h) v = max_nan(v, s_max[h][threadIdx.x]);
+    for (int h = 1; h < kColThreads / 32; ++h) v = max_nan(v, sm.max[h][threadIdx.x]);
     const float sc = scale_from_amax(v);
-    s_scale[threadIdx.x] = sc;
-    s_rcp[threadIdx.x] = __frcp_rn(sc);
-    const int64_t col = int64_t(blockIdx.x) * kColPanelCols + threadIdx.x;
-    if (FULL || col < cols) scales[row_blk * s_col_ld + col] = sc;
+    sm.scale[threadIdx.x] = sc;
+    sm.rcp[threadIdx.x] = __frcp_rn(sc);
+    const int col = bx * kColPanelCols + threadIdx.x;
+    if (FULL || col < a.out_cols) a.s[int64_t(by) * a.s_ld + col] = sc;
   }
   __syncthreads();
-  if (!col_ok) return;
+  if (!FULL && col0 >= a.out_cols) return;    // out_cols % 8 == 0
   float s[8], rc[8];
   {
-    const float4 a0 = *reinterpret_cast<const float4*>(&s_scale[cx * 8]), a1 = *reinterpret_cast<const float4*>(&s_scale[cx * 8 + 4]);
-    const float4 b0 = *reinterpret_cast<const float4*>(&s_rcp[cx * 8]), b1 = *reinterpret_cast<const float4*>(&s_rcp[cx * 8 + 4]);
+    const float4 a0 = *reinterpret_cast<const float4*>(&sm.scale[cx * 8]), a1 = *reinterpret_cast<const float4*>(&sm.scale[cx * 8 + 4]);
+    const float4 b0 = *reinterpret_cast<const float4*>(&sm.rcp[cx * 8]), b1 = *reinterpret_cast<const float4*>(&sm.rcp[cx * 8 + 4]);
     s[0] = a0.x; s[1] = a0.y; s[2] = a0.z; s[3] = a0.w; s[4] = a1.x; s[5] = a1.y; s[6] = a1.z; s[7] = a1.w;
     rc[0] = b0.x; rc[1] = b0.y; rc[2] = b0.z; rc[3] = b0.w; rc[4] = b1.x; rc[5] = b1.y; rc[6] = b1.z; rc[7] = b1.w;
   }
@@ -257,8 +306,6 @@ __device__ __forceinline__ void colwise_panel(const __nv_bfloat16* __restrict__ 
     s2[j] = make_float2(s[2 * j], s[2 * j + 1]);
     nr2[j] = make_float2(-rc[2 * j], -rc[2 * j + 1]);
   }
-  uint8_t* qp = q + row0 * q_col_ld + col0;
-  const int64_t step = int64_t(kColHalfWarps) * q_col_ld;
   if (all_finite) {
 #pragma unroll
     for (int r = 0; r < kColRowsPerThread; ++r, qp += step) {
@@ -282,70 +329,119 @@ __device__ __forceinline__ void colwise_panel(const __nv_bfloat16* __restrict__ 
   }
 }
 
-// WITH_ROWS: the same pass also emits the 1 x 128 (row-wise) quantisation of the panel -- a
-// half-warp spans exactly one row tile -- so a tensor that needs both forms (an upstream
-// gradient: row-wise for dgrad, column-wise for wgrad) is read from HBM once, not twice.
-template <bool WITH_ROWS, int ACT = TG_ACT_NONE>
-// Blocks per SM: the plain variants fit 64 registers without a spill and run four (8-14 % faster than three: the
-// top stall is the wait for the panel's loads, and a fourth block is a third more of them in flight); the
-// activation variants take 80 registers and three; the GELU cotangent variant, the one with the most live
-// values, runs 2 % faster with 128 registers and two blocks than with 80 and three, spilling.
-__global__ void __launch_bounds__(kColThreads, ACT == TG_ACT_GELU_BWD ? 2 : (ACT == TG_ACT_NONE ? 4 : 3))
-quantize_colwise_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q,
-                        float* __restrict__ scales, uint8_t* __restrict__ q_row,
-                        float* __restrict__ s_row, int64_t rows, int64_t cols,
-                        const __nv_bfloat16* __restrict__ gate = nullptr, int64_t q_row_ld = 0, int64_t s_row_ld = 0,
-                        int64_t q_col_ld = 0, int64_t s_col_ld = 0) {
-  // row pitches of the outputs (0: dense): a caller may place either form inside a wider matrix, e.g. three
-  // gradients side by side for one GEMM that contracts over all of them or produces all their weight gradients
-  if (WITH_ROWS && q_row_ld == 0) { q_row_ld = cols; s_row_ld = cols / kTile; }
-  if (q_col_ld == 0) { q_col_ld = cols; s_col_ld = cols; }
-  __shared__ float s_max[kColThreads / 32][kColPanelCols];
-  __shared__ __align__(16) float s_scale[kColPanelCols], s_rcp[kColPanelCols];
-  const bool full = (int64_t(blockIdx.y) + 1) * kTile <= rows && (int64_t(blockIdx.x) + 1) * kColPanelCols <= cols;
-  if (full)
-    colwise_panel<WITH_ROWS, ACT, true>(x, q, scales, q_row, s_row, rows, cols, gate, q_row_ld, s_row_ld, q_col_ld, s_col_ld,
-                                        s_max, s_scale, s_rcp);
-  else
-    colwise_panel<WITH_ROWS, ACT, false>(x, q, scales, q_row, s_row, rows, cols, gate, q_row_ld, s_row_ld, q_col_ld,
-                                         s_col_ld, s_max, s_scale, s_rcp);
+__host__ __device__ __forceinline__ bool is_ragged(const PanelJob& a) {
+  return ((a.ld | a.cols) & 7) != 0 || (reinterpret_cast<uintptr_t>(a.x) & 15u) != 0;
 }
 
-// ---------------------------------------------------------------------------------------
-// 128 x 128 tiles, one scale each.  A thread block (256 threads) owns one tile: 16 lanes x
-// 8 columns across, 16 row groups x 8 rows down.
-// ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-quantize_block128_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q,
-                         float* __restrict__ scales, int64_t rows, int64_t cols) {
-  __shared__ float s_max[8];
-  const int cx = threadIdx.x & 15, ry = threadIdx.x >> 4;
-  const int64_t col0 = int64_t(blockIdx.x) * kTile + cx * 8;
-  const int64_t row0 = int64_t(blockIdx.y) * kTile + ry * 8;
-  uint4 w[8];
+template <bool ROW, int FORM, int ACT>
+__device__ __forceinline__ void panel_any(const PanelJob& a, int bx, int by, PanelSmem& sm) {
+  const bool full = (by + 1) * kTile <= a.rows && (bx + 1) * kColPanelCols <= a.cols;
+  if (full) panel<ROW, FORM, ACT, true>(a, bx, by, sm);
+  else panel<ROW, FORM, ACT, false>(a, bx, by, sm);
+}
+
+// One tensor.  Blocks per SM: four at 64 registers, without a spill (8-14 % faster than three: the top stall is the wait for
+// the panel's loads, and a fourth block is a third more of them in flight).
+template <bool ROW, int FORM, bool RAGGED = false>
+__global__ void __launch_bounds__(kColThreads, 4) quantize_panel_kernel(const __grid_constant__ PanelJob a) {
+  __shared__ PanelSmem sm;
+  const int by = int(blockIdx.x) / a.tiles_x, bx = int(blockIdx.x) - by * a.tiles_x;
+  if constexpr (RAGGED) panel<ROW, FORM, TG_ACT_NONE, false, true>(a, bx, by, sm);
+  else panel_any<ROW, FORM, TG_ACT_NONE>(a, bx, by, sm);
+}
+
+// Several tensors in ONE launch: a linear's activation (both its forms from one read) and its weight, or the weights of a
+// layer.  The small ones do not fill the GPU by themselves and every launch costs 2-3 us: at 4096 x 768 -> 3072 the three
+// launches (row form, column form, weight) took 14.3 us, as two jobs of one launch 10.3.  With every form's code in one kernel
+// the compiler spills a few registers (7 % at 32768 x 8192), so past kJointPanels panels -- about 25 us of work, beside
+// which a launch no longer counts -- each tensor takes the kernel of its own.
+constexpr int kMaxJobs = 6;
+constexpr int64_t kJointPanels = 2048;
+struct PanelJobs {
+  PanelJob job[kMaxJobs];
+  int n;
+};
+__global__ void __launch_bounds__(kColThreads, 4) quantize_panels_kernel(const __grid_constant__ PanelJobs jobs) {
+  __shared__ PanelSmem sm;
+  int j = 0;
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int64_t row = row0 + r;
-    w[r] = (row < rows) ? ld_nc_v4(x + row * cols + col0) : make_uint4(0, 0, 0, 0);
+  for (int i = 1; i < kMaxJobs; ++i)
+    if (i < jobs.n && int(blockIdx.x) >= jobs.job[i].first) j = i;
+  const PanelJob& a = jobs.job[j];
+  const int t = int(blockIdx.x) - a.first, by = t / a.tiles_x, bx = t - by * a.tiles_x;
+  if (a.q_row != nullptr) {
+    if (a.form == kColForm) panel_any<true, kColForm, TG_ACT_NONE>(a, bx, by, sm);
+    else if (a.form == kBlockForm) panel_any<true, kBlockForm, TG_ACT_NONE>(a, bx, by, sm);
+    else panel_any<true, kNoForm, TG_ACT_NONE>(a, bx, by, sm);
+  } else {
+    if (a.form == kBlockForm) panel_any<false, kBlockForm, TG_ACT_NONE>(a, bx, by, sm);
+    else if (is_ragged(a)) panel<false, kColForm, TG_ACT_NONE, false, true>(a, bx, by, sm);
+    else panel_any<false, kColForm, TG_ACT_NONE>(a, bx, by, sm);
   }
-  uint32_t mb = 0u;
-#pragma unroll
-  for (int r = 0; r < 8; ++r) mb = absmax8(w[r], mb);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mb = __vmaxu2(mb, __shfl_xor_sync(0xffffffffu, mb, o));
-  float m = absmax_to_float(mb);
-  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
-  __syncthreads();
-  m = s_max[0];
-#pragma unroll
-  for (int wv = 1; wv < 8; ++wv) m = max_nan(m, s_max[wv]);
-  const float s = scale_from_amax(m);
-  if (threadIdx.x == 0) scales[int64_t(blockIdx.y) * (cols / kTile) + blockIdx.x] = s;
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int64_t row = row0 + r;
-    if (row < rows) *reinterpret_cast<uint2*>(q + row * cols + col0) = quantize8(w[r], s);
+}
+
+// Both forms of an activation computed on the fly.  The activation variants take 80 registers and three blocks; the GELU
+// cotangent variant, the one with the most live values, runs 2 % faster with 128 registers and two blocks than with
+// 80 and three, spilling.
+template <int ACT>
+__global__ void __launch_bounds__(kColThreads, ACT == TG_ACT_GELU_BWD ? 2 : 3)
+quantize_act_kernel(const __grid_constant__ PanelJob a) {
+  __shared__ PanelSmem sm;
+  panel_any<true, kColForm, ACT>(a, blockIdx.x, blockIdx.y, sm);
+}
+
+static PanelJob make_job(const void* x, int64_t rows, int64_t cols, int64_t ld) {
+  PanelJob a = {};
+  a.x = static_cast<const __nv_bfloat16*>(x);
+  a.ld = ld;
+  a.rows = int(rows);
+  a.cols = a.out_cols = int(cols);
+  a.tiles_x = int((cols + kColPanelCols - 1) / kColPanelCols);
+  return a;
+}
+static void with_row(PanelJob& a, void* q, int64_t q_ld, float* s, int64_t s_ld) {
+  a.q_row = static_cast<uint8_t*>(q); a.q_row_ld = q_ld; a.s_row = s; a.s_row_ld = s_ld;
+}
+static void with_form(PanelJob& a, int form, void* q, int64_t q_ld, float* s, int64_t s_ld) {
+  a.form = form; a.q = static_cast<uint8_t*>(q); a.q_ld = q_ld; a.s = s; a.s_ld = s_ld;
+}
+
+static int64_t panels_of(const PanelJob& a) { return int64_t(a.tiles_x) * ((a.rows + kTile - 1) / kTile); }
+
+static int launch_panel(const PanelJob& a, cudaStream_t st) {
+  const int64_t blocks = panels_of(a);
+  if (blocks > INT32_MAX) return TG_ERR_TOO_LARGE;
+  const unsigned grid = unsigned(blocks);
+  if (a.q_row != nullptr) {
+    if (a.form == kColForm) quantize_panel_kernel<true, kColForm><<<grid, kColThreads, 0, st>>>(a);
+    else if (a.form == kBlockForm) quantize_panel_kernel<true, kBlockForm><<<grid, kColThreads, 0, st>>>(a);
+    else quantize_panel_kernel<true, kNoForm><<<grid, kColThreads, 0, st>>>(a);
+  } else {
+    if (a.form == kColForm && is_ragged(a)) quantize_panel_kernel<false, kColForm, true><<<grid, kColThreads, 0, st>>>(a);
+    else if (a.form == kColForm) quantize_panel_kernel<false, kColForm><<<grid, kColThreads, 0, st>>>(a);
+    else quantize_panel_kernel<false, kBlockForm><<<grid, kColThreads, 0, st>>>(a);
   }
+  TG_CUDA_CHECK(cudaGetLastError());
+  return TG_OK;
+}
+
+static int launch_panels(PanelJobs& jobs, cudaStream_t st) {
+  int64_t blocks = 0;
+  for (int i = 0; i < jobs.n; ++i) blocks += panels_of(jobs.job[i]);
+  if (jobs.n == 1 || blocks > kJointPanels) {
+    for (int i = 0; i < jobs.n; ++i)
+      if (int rc = launch_panel(jobs.job[i], st)) return rc;
+    return TG_OK;
+  }
+  blocks = 0;
+  for (int i = 0; i < jobs.n; ++i) {
+    jobs.job[i].first = int(blocks);
+    blocks += panels_of(jobs.job[i]);
+  }
+  if (blocks == 0) return TG_OK;
+  quantize_panels_kernel<<<unsigned(blocks), kColThreads, 0, st>>>(jobs);
+  TG_CUDA_CHECK(cudaGetLastError());
+  return TG_OK;
 }
 
 }  // namespace tg
@@ -369,19 +465,18 @@ extern "C" int tg_quantize_rowwise(const void* x, void* q, float* scales, int64_
   return TG_OK;
 }
 
+static bool too_large(int64_t rows, int64_t cols) { return rows > INT32_MAX - 256 || cols > INT32_MAX - 256; }
+
 extern "C" int tg_quantize_colwise(const void* x, void* q, float* scales, int64_t rows,
                                    int64_t cols, void* stream) {
   if (rows < 0 || cols < 0 || cols % 8 != 0) return TG_ERR_SHAPE;
   if (rows == 0 || cols == 0) return TG_OK;
   if (!aligned16(x) || !aligned16(q) || !aligned16(scales)) return TG_ERR_ALIGN;
+  if (too_large(rows, cols)) return TG_ERR_TOO_LARGE;
   if (int rc = check_arch()) return rc;
-  const int64_t gx = (cols + kColPanelCols - 1) / kColPanelCols, gy = (rows + kTile - 1) / kTile;
-  if (gy > 65535) return TG_ERR_TOO_LARGE;
-  quantize_colwise_kernel<false><<<dim3(unsigned(gx), unsigned(gy)), kColThreads, 0,
-                                   static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scales, nullptr, nullptr, rows, cols);
-  TG_CUDA_CHECK(cudaGetLastError());
-  return TG_OK;
+  PanelJob a = make_job(x, rows, cols, cols);
+  with_form(a, kColForm, q, cols, scales, cols);
+  return launch_panel(a, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tg_quantize_rowcol_ld(const void* x, void* q_row, int64_t q_row_ld, float* s_row, int64_t s_row_ld,
@@ -394,15 +489,12 @@ extern "C" int tg_quantize_rowcol_ld(const void* x, void* q_row, int64_t q_row_l
   if (!aligned16(x) || (reinterpret_cast<uintptr_t>(q_row) & 7u) || (reinterpret_cast<uintptr_t>(q_col) & 7u) ||
       (reinterpret_cast<uintptr_t>(s_col) & 3u) || (reinterpret_cast<uintptr_t>(s_row) & 3u))
     return TG_ERR_ALIGN;
+  if (too_large(rows, cols)) return TG_ERR_TOO_LARGE;
   if (int rc = check_arch()) return rc;
-  const int64_t gx = cols / kColPanelCols, gy = (rows + kTile - 1) / kTile;
-  if (gy > 65535) return TG_ERR_TOO_LARGE;
-  quantize_colwise_kernel<true><<<dim3(unsigned(gx), unsigned(gy)), kColThreads, 0,
-                                  static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q_col), s_col, static_cast<uint8_t*>(q_row), s_row, rows,
-      cols, nullptr, q_row_ld, s_row_ld, q_col_ld, s_col_ld);
-  TG_CUDA_CHECK(cudaGetLastError());
-  return TG_OK;
+  PanelJob a = make_job(x, rows, cols, cols);
+  with_row(a, q_row, q_row_ld, s_row, s_row_ld);
+  with_form(a, kColForm, q_col, q_col_ld, s_col, s_col_ld);
+  return launch_panel(a, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tg_quantize_rowcol(const void* x, void* q_row, float* s_row, void* q_col, float* s_col,
@@ -424,18 +516,18 @@ extern "C" int tg_act_quantize_rowcol(const void* x, const void* gate, int act, 
     return TG_ERR_ALIGN;
   if (int rc = check_arch()) return rc;
   const int64_t gx = cols / kColPanelCols, gy = (rows + kTile - 1) / kTile;
-  if (gy > 65535) return TG_ERR_TOO_LARGE;
+  if (gy > 65535 || too_large(rows, cols)) return TG_ERR_TOO_LARGE;
   const dim3 grid{unsigned(gx), unsigned(gy)};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
-  const __nv_bfloat16* gp = static_cast<const __nv_bfloat16*>(gate);
-  uint8_t* qc = static_cast<uint8_t*>(q_col);
-  uint8_t* qr = static_cast<uint8_t*>(q_row);
+  PanelJob a = make_job(x, rows, cols, cols);
+  a.gate = static_cast<const __nv_bfloat16*>(gate);
+  with_row(a, q_row, cols, s_row, cols / kTile);
+  with_form(a, kColForm, q_col, cols, s_col, cols);
   switch (act) {
-    case TG_ACT_RELU2: quantize_colwise_kernel<true, TG_ACT_RELU2><<<grid, kColThreads, 0, st>>>(xp, qc, s_col, qr, s_row, rows, cols, gp); break;
-    case TG_ACT_GELU: quantize_colwise_kernel<true, TG_ACT_GELU><<<grid, kColThreads, 0, st>>>(xp, qc, s_col, qr, s_row, rows, cols, gp); break;
-    case TG_ACT_RELU2_BWD: quantize_colwise_kernel<true, TG_ACT_RELU2_BWD><<<grid, kColThreads, 0, st>>>(xp, qc, s_col, qr, s_row, rows, cols, gp); break;
-    default: quantize_colwise_kernel<true, TG_ACT_GELU_BWD><<<grid, kColThreads, 0, st>>>(xp, qc, s_col, qr, s_row, rows, cols, gp); break;
+    case TG_ACT_RELU2: quantize_act_kernel<TG_ACT_RELU2><<<grid, kColThreads, 0, st>>>(a); break;
+    case TG_ACT_GELU: quantize_act_kernel<TG_ACT_GELU><<<grid, kColThreads, 0, st>>>(a); break;
+    case TG_ACT_RELU2_BWD: quantize_act_kernel<TG_ACT_RELU2_BWD><<<grid, kColThreads, 0, st>>>(a); break;
+    default: quantize_act_kernel<TG_ACT_GELU_BWD><<<grid, kColThreads, 0, st>>>(a); break;
   }
   TG_CUDA_CHECK(cudaGetLastError());
   return TG_OK;
@@ -446,12 +538,44 @@ extern "C" int tg_quantize_block128(const void* x, void* q, float* scales, int64
   if (rows < 0 || cols < 0 || cols % kTile != 0) return TG_ERR_SHAPE;
   if (rows == 0 || cols == 0) return TG_OK;
   if (!aligned16(x) || !aligned16(q) || (reinterpret_cast<uintptr_t>(scales) & 3u)) return TG_ERR_ALIGN;
+  if (too_large(rows, cols)) return TG_ERR_TOO_LARGE;
   if (int rc = check_arch()) return rc;
-  const int64_t gx = cols / kTile, gy = (rows + kTile - 1) / kTile;
-  if (gy > 65535) return TG_ERR_TOO_LARGE;
-  quantize_block128_kernel<<<dim3(unsigned(gx), unsigned(gy)), 256, 0,
-                             static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<uint8_t*>(q), scales, rows, cols);
-  TG_CUDA_CHECK(cudaGetLastError());
-  return TG_OK;
+  PanelJob a = make_job(x, rows, cols, cols);
+  with_form(a, kBlockForm, q, cols, scales, cols / kTile);
+  return launch_panel(a, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int tgh_quantize_jobs(const tgh_quantize_job* in, int n, void* stream) {
+  if (n < 0 || n > kMaxJobs) return TG_ERR_SHAPE;
+  PanelJobs jobs;
+  jobs.n = 0;
+  for (int i = 0; i < n; ++i) {
+    const tgh_quantize_job& b = in[i];
+    const bool col = b.form == TGH_FORM_COLUMNS, block = b.form == TGH_FORM_BLOCKS;
+    if (b.rows < 0 || b.cols < 0 || (b.q_row == nullptr && !col && !block)) return TG_ERR_SHAPE;
+    if ((b.q_row != nullptr || block) && b.cols % kTile != 0) return TG_ERR_SHAPE;
+    if (b.rows == 0 || b.cols == 0) continue;
+    if (b.ld < b.cols || (b.q_row != nullptr && b.q_row_ld % 16 != 0) || (b.q != nullptr && (b.q_ld % 16 != 0 || b.q_ld < b.cols)))
+      return TG_ERR_SHAPE;
+    const bool col_only = col && b.q_row == nullptr;      // reads rows at any alignment
+    if ((!col_only && (b.ld % 8 != 0 || !aligned16(b.x))) || (reinterpret_cast<uintptr_t>(b.x) & 1u) || 
+        (reinterpret_cast<uintptr_t>(b.q_row) & 7u) || (reinterpret_cast<uintptr_t>(b.q) & 7u))
+      return TG_ERR_ALIGN;
+    if (too_large(b.rows, b.cols)) return TG_ERR_TOO_LARGE;
+    PanelJob a = make_job(b.x, b.rows, b.cols, b.ld);
+    if (b.q_row != nullptr) with_row(a, b.q_row, b.q_row_ld, b.s_row, b.s_row_ld);
+    if (col) {
+      with_form(a, kColForm, b.q, b.q_ld, b.s, b.s_ld);
+      if (b.cols % 8 != 0) {                       // ragged columns: zeros up to the pitch of the output
+        a.out_cols = int(b.q_ld);
+        if (b.s_ld < b.q_ld || b.q_ld - b.cols >= 128) return TG_ERR_SHAPE;
+        a.tiles_x = (a.out_cols + kColPanelCols - 1) / kColPanelCols;
+      }
+    }
+    if (block) with_form(a, kBlockForm, b.q, b.q_ld, b.s, b.s_ld);
+    jobs.job[jobs.n++] = a;
+  }
+  if (jobs.n == 0) return TG_OK;
+  if (int rc = check_arch()) return rc;
+  return launch_panels(jobs, static_cast<cudaStream_t>(stream));
 }

@@ -112,8 +112,8 @@ def _fp8_forward(a, b, block_k=DEFAULT_BLOCK_K, weight_tile=(128, 1), a_quantize
     """fp8.py:50-78.  `a_quantized` = (q, scales) of `a` made earlier (e.g. by the fused
     norm+quantise kernel) skips the activation quantiser.  return_weight=True also returns the
     quantised weight pair (128x128 tiles serve the backward's dgrad unchanged)."""
-    y, w_q, w_s = ops._host().fp8_forward(a, b, block_k, _per_column(weight_tile), *_row_form(a_quantized))
-    return (y, (w_q, w_s)) if return_weight else y
+    y = ops._host().fp8_forward(a, b, block_k, _per_column(weight_tile), *_row_form(a_quantized))
+    return (y, quantize_weight(_as_bf16(b, "b"), weight_tile)) if return_weight else y
 
 
 def _fp8_backward(block_k, residuals, g, weight_tile=(128, 1), mode="bf16_ste", a_quantized=None, w_quantized=None,
