@@ -160,3 +160,13 @@ def test_one_pass_loss_of_a_nan_row():
     loss = losses.capped_cross_entropy(x, torch.zeros(3, dtype=torch.int64, device="cuda"), 15.0)
     loss.backward()
     assert bool(torch.isnan(loss)) and bool(torch.isnan(x.grad[1]).all()) and not bool(torch.isnan(x.grad[::2]).any())
+
+
+@pytest.mark.parametrize("rows,vocab", [(5, 8), (9, 256), (7, 264), (33, 2048), (6, 2056), (5, 4096), (5, 8904), (3, 50304)])
+def test_one_pass_gradient_has_the_bits_of_the_two_kernels(rows, vocab):
+    from train_gpt_b200 import losses, ops
+    x, t = _case(rows, vocab, rows + vocab, 5.0)
+    a, tt = to_torch_bf16(x).requires_grad_(True), torch.from_numpy(t).cuda()
+    losses.capped_cross_entropy(a, tt.long(), 15.0).backward()
+    _, lse, th = ops.softcap_ce_fwd(a.detach(), tt, 15.0)
+    assert torch.equal(a.grad, ops.softcap_ce_bwd(th, tt, lse, None, 15.0))

@@ -179,3 +179,20 @@ def test_fp8_loss_curve_matches_bf16_at_the_training_configuration():
     assert float(raw) < 0.01, float(raw)                                     # unsmoothed, step by step, as well
     assert last < 0.01, last
     assert float(gn_rel) < 0.10, float(gn_rel)
+
+
+def test_native_step_reports_a_token_outside_the_vocabulary():
+    """The native step's embedding kernel checks token ids itself: the loss is NaN and the status word says why.  Negative ids
+    count from the end, as an index does."""
+    from train_gpt_b200 import ops
+    from train_gpt_b200.step import SMALL, StepConfig, Trainer, synthetic_batch
+    cfg = StepConfig(**SMALL)
+    ids, tgt = synthetic_batch(cfg, 2, "cuda", seed=0)
+    a, b = (Trainer(cfg, torch.device("cuda", 0), seed=0) for _ in range(2))
+    assert a._program is not None
+    wrapped = torch.where(ids == 3, ids - cfg.vocab_size, ids)
+    assert float(a.step(ids, tgt)[0]) == float(b.step(wrapped, tgt)[0])
+    ids[0, 5] = cfg.vocab_size
+    assert torch.isnan(a.step(ids, tgt)[0])
+    with pytest.raises(RuntimeError, match="outside the vocabulary"):
+        ops.check_status(device="cuda")

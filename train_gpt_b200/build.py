@@ -21,6 +21,8 @@ HOST_PATH = os.path.join(PKG_DIR, "_host.so")
 
 SOURCES = ["runtime.cu", "quantize.cu", "rmsnorm.cu", "gemm_fp8.cu", "selftest.cu", "loss.cu", "optim.cu"]
 
+HOST_SOURCES = ["host.cpp", "step.cpp"]
+
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-std=c++17", "-lineinfo",
@@ -46,33 +48,45 @@ def _stale(target: str, suffixes) -> bool:
 
 
 def _start_host():
-    """Start compiling the host extension (it needs torch's headers and no GPU); None if it is up to date."""
+    """Start compiling the host extension (it needs torch's headers and no GPU); returns what waits for it and links."""
     import sysconfig
     import torch
     from torch.utils import cpp_extension
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     inc = [*cpp_extension.include_paths(), os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include"),
            sysconfig.get_paths()["include"]]
-    # (built under another name and renamed when complete: another process never loads half a file)
-    cmd = ["g++", "-shared", "-fPIC", "-O2", "-std=c++17", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_host",
+    cmd = ["g++", "-fPIC", "-O2", "-std=c++17", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_host",
            "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
-           *[a for i in inc for a in ("-isystem", i)], os.path.join(CSRC, "host.cpp"), "-o", HOST_PATH + ".new",
-           "-L" + lib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda", "-ldl", f"-Wl,-rpath,{lib}"]
-    return subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+           *[a for i in inc for a in ("-isystem", i)]]
+    procs = []
+    for src in HOST_SOURCES:
+        obj = os.path.join(CSRC, src.replace(".cpp", "_host.o"))
+        procs.append((src, obj, subprocess.Popen([*cmd, "-c", os.path.join(CSRC, src), "-o", obj], stdout=subprocess.PIPE,
+                                                 stderr=subprocess.STDOUT, text=True)))
+
+    def finish():
+        outs = [(src, p.communicate()[0], p.returncode) for src, _, p in procs]
+        for src, out, rc in outs:
+            if rc != 0:
+                raise RuntimeError(f"g++ failed on {src}:\n{out}")
+        # (linked under another name and renamed when complete: another process never loads half a file)
+        r = subprocess.run(["g++", "-shared", *[obj for _, obj, _ in procs], "-o", HOST_PATH + ".new",
+                            "-L" + lib, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda", "-ldl",
+                            f"-Wl,-rpath,{lib}"], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"link of _host.so failed:\n{r.stdout}")
+        os.replace(HOST_PATH + ".new", HOST_PATH)
+
+    return finish
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile what is missing or older than its sources; return the library's path."""
-    host = _start_host() if force or _stale(HOST_PATH, (".cpp", ".h")) else None
-    try:
-        if force or _stale(LIB_PATH, (".cu", ".cuh", ".h")):
-            _build_lib(verbose)
-    finally:
-        out, rc = ("", 0) if host is None else (host.communicate()[0], host.returncode)
-    if rc != 0:
-        raise RuntimeError(f"g++ failed on host.cpp:\n{out}")
-    if host is not None:
-        os.replace(HOST_PATH + ".new", HOST_PATH)
+    finish_host = _start_host() if force or _stale(HOST_PATH, (".cpp", ".h")) else None
+    if force or _stale(LIB_PATH, (".cu", ".cuh", ".h")):
+        _build_lib(verbose)
+    if finish_host is not None:
+        finish_host()
     return LIB_PATH
 
 

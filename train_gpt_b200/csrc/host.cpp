@@ -8,56 +8,47 @@
 //
 // The kernels stay behind the C ABI: bind() takes the addresses of the one loaded library (the same image ctypes
 // uses), so a build named by TRAIN_GPT_B200_LIB serves both.
-#include <ATen/cuda/CUDAContext.h>
-#include <c10/cuda/CUDAGuard.h>
+#include "host.h"
+
 #include <dlfcn.h>
 #include <torch/csrc/autograd/engine.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
-#include <torch/extension.h>
 
-#include <array>
-#include <atomic>
 #include <functional>
 #include <memory>
 #include <mutex>
-#include <optional>
-#include <sstream>
-#include <string>
 #include <tuple>
-#include <utility>
-#include <vector>
 
-#include "../../include/train_gpt_b200.h"
-#include "host_api.h"
-
-namespace py = pybind11;
-using at::Tensor;
 using torch::autograd::Node;
 using torch::autograd::SavedVariable;
 using torch::autograd::variable_list;
 
+namespace tgh {
+
+Api api;
+std::atomic<int> last_gemm_launches{0};
+
+// The word a GEMM reports an expired device wait in, one per device, made once (so that a captured CUDA graph
+// keeps pointing at it) and never freed: the CUDA context may be gone by the time static objects are.
+Tensor status_word(int64_t device) {
+  static std::mutex mu;
+  static auto* words = new std::array<Tensor, 64>();
+  if (device < 0) device = c10::cuda::current_device();
+  std::lock_guard<std::mutex> lock(mu);
+  Tensor& w = words->at(size_t(device));
+  if (!w.defined()) w = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, c10::DeviceIndex(device)));
+  return w;
+}
+
+}  // namespace tgh
+
 namespace {
 
-constexpr int64_t kTile = 128;
+using namespace tgh;
+
 constexpr int64_t kAddNormMaxCols = 2048;   // rows the fused add + norm kernels take
-const auto kF8 = at::kFloat8_e4m3fn;
-
-// ---- the C ABI, by address ------------------------------------------------------------------------------------
-
-#define TG_API(X)                                                                                                  \
-  X(tg_last_cuda_error) X(tg_quantize_rowwise) X(tg_quantize_colwise) X(tg_quantize_rowcol) X(tg_quantize_rowcol_ld) \
-  X(tg_act_quantize_rowcol) X(tg_quantize_block128) X(tg_rmsnorm_fwd) X(tg_rmsnorm_quant_fwd)                       \
-  X(tg_add_rmsnorm_quant_fwd) X(tg_rmsnorm_bwd_scratch_bytes) X(tg_rmsnorm_bwd) X(tg_rmsnorm_bwd_add)               \
-  X(tg_softcap_ce_fwd) X(tg_softcap_ce_bwd) X(tg_sumsq_scratch_bytes) X(tg_sumsq_bf16) X(tg_adamw_bf16)             \
-  X(tg_gemm_workspace_bytes) X(tg_gemm_fp8_blockscaled) X(tgh_quantize_jobs) X(tgh_softcap_ce_fits) X(tgh_softcap_ce)
-
-struct Api {
-#define X(name) decltype(&::name) name = nullptr;
-  TG_API(X)
-#undef X
-} api;
 
 void bind(const std::string& path) {
   void* lib = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
@@ -69,65 +60,11 @@ void bind(const std::string& path) {
 #undef X
 }
 
-// a launcher's status as an exception: ValueError for sizes the kernel cannot take, RuntimeError for the rest
-void check(int rc, const char* what) {
-  if (rc == TG_OK) return;
-  const char* name = rc == TG_ERR_SHAPE ? "TG_ERR_SHAPE" : rc == TG_ERR_ALIGN ? "TG_ERR_ALIGN" : rc == TG_ERR_ARCH ? "TG_ERR_ARCH"
-                     : rc == TG_ERR_CUDA ? "TG_ERR_CUDA" : rc == TG_ERR_TOO_LARGE ? "TG_ERR_TOO_LARGE" : "unknown status";
-  const std::string msg = std::string(what) + ": " + name;
-  if (rc == TG_ERR_SHAPE || rc == TG_ERR_TOO_LARGE || rc == TG_ERR_ALIGN) throw py::value_error(msg);
-  throw std::runtime_error(rc == TG_ERR_CUDA ? msg + " " + api.tg_last_cuda_error() : msg);
-}
-
-// ---- small helpers -----------------------------------------------------------------------------------------------
-
-template <typename... A>
-std::string cat(const A&... a) {
-  std::ostringstream o;
-  (o << ... << a);
-  return o.str();
-}
-
-std::string dtype_name(at::ScalarType t) {
-  switch (t) {
-    case at::kBFloat16: return "torch.bfloat16";
-    case at::kFloat: return "torch.float32";
-    case at::kHalf: return "torch.float16";
-    case at::kDouble: return "torch.float64";
-    default: return c10::toString(t);
-  }
-}
-
-Tensor need(const Tensor& t, at::ScalarType dt, const char* name) {
-  if (!t.is_cuda()) throw std::runtime_error(cat(name, " must be a CUDA tensor (there is no CPU path)"));
-  if (t.scalar_type() != dt) throw py::type_error(cat(name, " must be ", dtype_name(dt), ", got ", dtype_name(t.scalar_type())));
-  return t.is_contiguous() ? t : t.contiguous();
-}
-
 void need_2d(const Tensor& t, const char* what) {
   if (t.dim() != 2) throw py::value_error(cat(what, " takes a 2-D tensor"));
 }
 
-int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
-
-Tensor empty(at::IntArrayRef shape, at::ScalarType dt, const Tensor& like) {
-  return at::empty(shape, at::TensorOptions().dtype(dt).device(like.device()));
-}
-
-void* cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
-
-float* fptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
-void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
-
-std::vector<int64_t> with_last(const Tensor& x, int64_t last) {
-  std::vector<int64_t> s(x.sizes().begin(), x.sizes().end());
-  s.back() = last;
-  return s;
-}
-
 // ---- quantisers -----------------------------------------------------------------------------------------------
-
-using Pair = std::pair<Tensor, Tensor>;
 
 void need_tiles(int64_t k) {
   if (k % kTile) throw py::value_error(cat("K=", k, " not divisible by block_k=", kTile));
@@ -394,25 +331,49 @@ void adamw_step(const Tensor& p, const Tensor& g, const Tensor& m, const Tensor&
         "tg_adamw_bf16");
 }
 
-// ---- GEMM ---------------------------------------------------------------------------------------------------------
-
-// The word a GEMM reports an expired device wait in, one per device, made once (so that a captured CUDA graph
-// keeps pointing at it) and never freed: the CUDA context may be gone by the time static objects are.
-Tensor status_word(int64_t device) {
-  static std::mutex mu;
-  static auto* words = new std::array<Tensor, 64>();
-  if (device < 0) device = c10::cuda::current_device();
-  std::lock_guard<std::mutex> lock(mu);
-  Tensor& w = words->at(size_t(device));
-  if (!w.defined()) w = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, c10::DeviceIndex(device)));
-  return w;
+void need_flat_bf16(const Tensor& t, const char* n) {
+  if (!t.is_cuda() || t.scalar_type() != at::kBFloat16 || !t.is_contiguous())
+    throw py::type_error(cat(n, " must be a contiguous bf16 CUDA tensor"));
 }
 
-std::atomic<int> last_gemm_launches{0};    // kernels the most recent GEMM launched (1, or 2 with the reduce of a cut contraction)
+// sqrt of the sum of squares over all of `grads`; scratch from global_norm_scratch
+Tensor global_norm(const std::vector<Tensor>& grads, const Tensor& scratch) {
+  if (grads.empty()) throw py::value_error("no gradients");
+  std::vector<tgh_span> spans(grads.size());
+  for (size_t i = 0; i < grads.size(); ++i) {
+    need_flat_bf16(grads[i], "g");
+    spans[i] = {nullptr, grads[i].data_ptr(), nullptr, nullptr, grads[i].numel()};
+  }
+  const c10::cuda::CUDAGuard guard(grads[0].device());
+  Tensor norm = empty({}, at::kFloat, grads[0]);
+  check(api.tgh_global_norm(spans.data(), int(spans.size()), ptr(scratch), fptr(norm), nullptr, nullptr, nullptr, cur_stream()),
+        "tgh_global_norm");
+  return norm;
+}
+Tensor global_norm_scratch(const Tensor& like, int n) {
+  return at::zeros({api.tgh_global_norm_scratch_bytes(n)}, at::TensorOptions().dtype(at::kByte).device(like.device()));
+}
 
-struct Strides {
-  int64_t row, kb;
-};
+// clip by `norm` and AdamW on all tensors; step: int32 (2,), the step count and a zero
+void clipped_adamw(const std::vector<Tensor>& p, const std::vector<Tensor>& g, const std::vector<Tensor>& m, const std::vector<Tensor>& v,
+                   const Tensor& step, const Tensor& norm, double clip, double lr, double b1, double b2, double eps, double weight_decay) {
+  if (p.empty()) return;
+  if (p.size() != g.size() || p.size() != m.size() || p.size() != v.size()) throw py::value_error("p, g, m, v differ in number");
+  std::vector<tgh_span> spans(p.size());
+  for (size_t i = 0; i < p.size(); ++i) {
+    need_flat_bf16(p[i], "p"); need_flat_bf16(g[i], "g"); need_flat_bf16(m[i], "m"); need_flat_bf16(v[i], "v");
+    if (p[i].numel() != g[i].numel() || p[i].numel() != m[i].numel() || p[i].numel() != v[i].numel())
+      throw py::value_error("p, g, m, v sizes differ");
+    spans[i] = {p[i].data_ptr(), g[i].data_ptr(), m[i].data_ptr(), v[i].data_ptr(), p[i].numel()};
+  }
+  const c10::cuda::CUDAGuard guard(p[0].device());
+  const Tensor n = norm.to(at::kFloat);
+  check(api.tgh_adamw(spans.data(), int(spans.size()), float(lr), float(b1), float(b2), float(eps), float(weight_decay), fptr(n),
+                      float(clip), static_cast<int32_t*>(ptr(step)), cur_stream()),
+        "tgh_adamw");
+}
+
+// ---- GEMM ---------------------------------------------------------------------------------------------------------
 
 Tensor gemm(const Tensor& a, const Tensor& b, const Tensor& sa, const Tensor& sb, int64_t m, int64_t n, int64_t k, int a_major,
             int b_major, Strides sa_st, Strides sb_st, int sb_gran_n, at::ScalarType out_dtype, const Tensor& status_, Tensor out,
@@ -502,92 +463,6 @@ Linear validate(const Tensor& a, const Tensor& b, int64_t block_k) {
     throw py::value_error(cat("block_k=", block_k, " is not supported by the sm_100a kernels (only ", kTile, ")"));
   return {k, b.size(1)};
 }
-
-// Device memory for several temporaries of one call, or for what a node keeps, as ONE allocation: a caching-allocator
-// round trip costs about as much host time as a third of a launch, and a linear has up to ten such buffers.
-class Arena {
- public:
-  size_t add(int64_t bytes) {
-    const size_t at = size_;
-    size_ += (size_t(bytes) + 255) / 256 * 256;
-    return at;
-  }
-  void make(const Tensor& like) {
-    if (size_ > 0) memory_ = empty({int64_t(size_)}, at::kByte, like);
-    base_ = size_ > 0 ? static_cast<uint8_t*>(memory_.data_ptr()) : nullptr;
-  }
-  void* at(size_t offset) const { return base_ + offset; }
-  const Tensor& memory() const { return memory_; }
-
- private:
-  size_t size_ = 0;
-  uint8_t* base_ = nullptr;
-  Tensor memory_;
-};
-
-// One quantised matrix: e4m3 bytes and float32 scales
-struct Form {
-  void* q = nullptr;
-  float* s = nullptr;
-  explicit operator bool() const { return q != nullptr; }
-};
-struct FormAt {
-  size_t q = 0, s = 0;
-  Form in(const Arena& m) const { return {m.at(q), static_cast<float*>(m.at(s))}; }
-};
-FormAt add_row(Arena& m, int64_t rows, int64_t cols) { return {m.add(rows * cols), m.add(rows * (cols / kTile) * 4)}; }
-FormAt add_col(Arena& m, int64_t rows, int64_t cols) { return {m.add(rows * cols), m.add(cdiv(rows, kTile) * cols * 4)}; }
-FormAt add_block(Arena& m, int64_t rows, int64_t cols) { return {m.add(rows * cols), m.add(cdiv(rows, kTile) * (cols / kTile) * 4)}; }
-
-// A 2-D bf16 matrix the quantisers can read as it lies: unit stride along a row and, unless it is only wanted by column,
-// rows at 16-byte boundaries.  Anything else is copied.
-Tensor readable(const Tensor& t, bool any_alignment) {
-  if (t.stride(1) == 1 && (t.size(0) <= 1 || t.stride(0) >= t.size(1)) &&
-      (any_alignment || ((t.size(0) <= 1 || t.stride(0) % 8 == 0) && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0)))
-    return t;
-  return t.contiguous();
-}
-int64_t pitch(const Tensor& t) { return t.size(0) > 1 ? t.stride(0) : t.size(1); }
-
-tgh_quantize_job job_of(const Tensor& x) {
-  tgh_quantize_job j = {};
-  j.x = x.data_ptr();
-  j.rows = x.size(0);
-  j.cols = x.size(1);
-  j.ld = pitch(x);
-  return j;
-}
-void want_row(tgh_quantize_job& j, const Form& f) {
-  j.q_row = f.q; j.s_row = f.s; j.q_row_ld = j.cols; j.s_row_ld = j.cols / kTile;
-}
-void want_col(tgh_quantize_job& j, const Form& f, int64_t ld) {
-  j.form = TGH_FORM_COLUMNS; j.q = f.q; j.s = f.s; j.q_ld = j.s_ld = ld;
-}
-void want_block(tgh_quantize_job& j, const Form& f) {
-  j.form = TGH_FORM_BLOCKS; j.q = f.q; j.s = f.s; j.q_ld = j.cols; j.s_ld = j.cols / kTile;
-}
-
-// A GEMM of forms.  (rows of A, columns of B and their contraction; see gemm_fwd / gemm_dgrad / gemm_wgrad for the layouts)
-tg_gemm_args gemm_args(int64_t m, int64_t n, int64_t k, int64_t lda, int a_major, Strides sa, int64_t ldb, int b_major, Strides sb,
-                       bool per_column, int64_t ldd, bool f32, unsigned* status) {
-  tg_gemm_args g = {};
-  g.lda = lda; g.ldb = ldb; g.a_major = a_major; g.b_major = b_major;
-  g.sa_stride_m = sa.row; g.sa_stride_kb = sa.kb; g.sb_stride_n = sb.row; g.sb_stride_kb = sb.kb;
-  g.sb_gran_n = per_column ? 1 : int(kTile);
-  g.ldd = ldd; g.out_dtype = f32 ? TG_OUT_F32 : TG_OUT_BF16;
-  g.M = m; g.N = n; g.K = k;
-  g.status = status;
-  return g;
-}
-void run_gemm(tg_gemm_args& g, const Form& a, const Form& b, void* d, void* workspace, int64_t workspace_bytes) {
-  g.a = a.q; g.sa = a.s; g.b = b.q; g.sb = b.s;
-  g.d = d;
-  g.workspace = workspace_bytes > 0 ? workspace : nullptr;
-  g.workspace_bytes = workspace_bytes;
-  check(api.tg_gemm_fp8_blockscaled(&g, cur_stream()), "tg_gemm_fp8_blockscaled");
-  last_gemm_launches.store(workspace_bytes > 0 ? 2 : 1, std::memory_order_relaxed);
-}
-unsigned* status_of(const Tensor& like) { return static_cast<unsigned*>(ptr(status_word(like.get_device()))); }
 
 int64_t rows_of(const Tensor& a) {
   int64_t m = 1;
@@ -1059,6 +934,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("softcap_ce_bwd", &softcap_ce_bwd);
   m.def("sumsq", &sumsq);
   m.def("adamw_step", &adamw_step);
+  m.def("global_norm", &global_norm);
+  m.def("global_norm_scratch", &global_norm_scratch);
+  m.def("clipped_adamw", &clipped_adamw);
   m.def("status_word", &status_word);
   m.def("last_gemm_launches", [] { return last_gemm_launches.load(std::memory_order_relaxed); });
   m.def("gemm", [](const Tensor& a, const Tensor& b, const Tensor& sa, const Tensor& sb, int64_t M, int64_t N, int64_t K, int a_major,
@@ -1108,4 +986,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("rms_norm", &rms_norm);
   m.def("capped_cross_entropy", &capped_cross_entropy);
+  register_step(m);
 }

@@ -22,7 +22,7 @@ typedef struct {
   int form;
   void* q; float* s; int64_t q_ld, s_ld;
 } tgh_quantize_job;
-/* Up to six of them in one launch. */
+/* Any number of them: in one launch where they are of block form only (24 a launch) or small and at most six. */
 int tgh_quantize_jobs(const tgh_quantize_job* jobs, int n, void* stream);
 
 /* Whether tgh_softcap_ce takes this problem (a row and its cap fit the one-pass kernel). */
@@ -35,6 +35,24 @@ int tgh_softcap_ce_fits(float cap, int64_t rows, int64_t vocab);
  *   nll       float [rows] or NULL;  loss: float scalar, mean of nll, or NULL */
 int tgh_softcap_ce(const void* logits, const void* targets, int targets_64, float cap, void* dlogits, const float* gscale,
                    int only_if_scaled, float* nll, float* loss, int64_t rows, int64_t vocab, int64_t ld, void* stream);
+
+/* x[b, t, :] = bf16(embed[ids[b, t]] + pos[t]) (train-gpt model.py:83).  Negative ids count from the end; one outside the
+ * vocabulary stores TGH_STATUS_TOKEN in *status and makes its row NaN. */
+enum { TGH_STATUS_TOKEN = 16 };
+int tgh_embed(const int64_t* ids, const void* embed, const void* pos, void* x, int64_t batch, int64_t seq, int64_t d, int64_t vocab,
+              unsigned* status, void* stream);
+
+/* A parameter tensor with its gradient and moments: n contiguous bf16 values each, 16-byte aligned. */
+typedef struct { void* p; const void* g; void* m; void* v; int64_t n; } tgh_span;
+/* norm = sqrt of the sum of squares of every span's g.  scratch: tgh_global_norm_scratch_bytes(n) bytes whose first 16 are
+ * zero before the first use (they are again after each).  loss_out, if not NULL: *loss_in, or NaN where *status is not 0. */
+int64_t tgh_global_norm_scratch_bytes(int n);
+int tgh_global_norm(const tgh_span* spans, int n, void* scratch, float* norm, const float* loss_in, const unsigned* status,
+                    float* loss_out, void* stream);
+/* Clip by *norm (factor clip / norm where norm >= clip) and AdamW step number step[0] + 1 on every span, then ++step[0].
+ * step[1] is 0 before and after. */
+int tgh_adamw(const tgh_span* spans, int n, float lr, float b1, float b2, float eps, float weight_decay, const float* norm,
+              float clip, int32_t* step, void* stream);
 
 #ifdef __cplusplus
 }

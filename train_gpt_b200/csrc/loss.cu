@@ -225,12 +225,16 @@ softcap_ce_bwd_kernel(const __nv_bfloat16* tanh_in, const int32_t* __restrict__ 
 // their capped value is far below half an ulp of anything it meets.  A NaN would look up 1: a row's largest
 // magnitude is tracked and a NaN in it makes the row's sum, and with it the loss and the gradient, NaN.
 //
-// No running maximum: |z| <= c <= 64, so the sum of exp(z) neither overflows nor loses its terms.
+// The sum of exp(z), two ways.  Rows that are whole pieces (the vocabulary a multiple of 8) sum exactly as softcap_ce_fwd_kernel
+// does -- running maximum, 512 threads, the same order -- so that the log-sum and with it every bit of the gradient equal those
+// of the pair of kernels: a last bit there, amplified by the e4m3 roundings of a deep backward pass, is another trajectory.
+// Ragged rows, which that kernel could only sum after a copy, skip the running maximum (|z| <= c <= 64: the sum neither
+// overflows nor loses its terms) and take as many threads as fill their last pass.
 //
 // One thread block per row (one warp for rows up to 2048 columns); a thread meets the same pieces in both passes,
-// so the only synchronisation is the reduction of the sum: one barrier per row.
+// so the only synchronisation is the reduction of the sum.
 // Bound by instruction issue and the ALU pipe (49 warp instructions per 64 logits, two of them ex2 in each pass), no longer by
-// memory.  8192 x 50257: 699 us for the two kernels, 2507 with the copies -> 415 us (DRAM floor 251); 8192 x 50304: 697 -> 414.
+// memory.  8192 x 50257: 699 us for the two kernels, 2507 with the copies -> 415 us (DRAM floor 251); 8192 x 50304: 704 -> 462.
 // ---------------------------------------------------------------------------------------
 constexpr int kCeMaxThreads = 640;
 constexpr int kCeWarpCols = 2048;                 // rows up to this wide take one warp
@@ -263,11 +267,12 @@ __device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
   return v;
 }
 
-template <bool WARP>
-__global__ void __launch_bounds__(WARP ? 256 : kCeMaxThreads, WARP ? 4 : 2) softcap_ce_kernel(const CeArgs p) {
+template <bool WARP, bool WHOLE>
+__global__ void __launch_bounds__(WARP ? 256 : WHOLE ? kLossFwdThreads : kCeMaxThreads, WARP ? 4 : 2) softcap_ce_kernel(const CeArgs p) {
   if (p.only_if_scaled && *p.gscale == 1.0f) return;
   extern __shared__ __align__(16) uint8_t s_ce[];
   __shared__ float s_sum[2][kCeMaxThreads / 32];
+  __shared__ float s_lse;
   const Softcap sc(p.cap);
   // the power-of-two edges of the table as bf16 bits: 2^floor(log2 c) is c with its mantissa cleared
   const uint32_t c_pow = (__float_as_uint(sc.c) >> 16) & 0x7f80u;
@@ -341,30 +346,67 @@ __global__ void __launch_bounds__(WARP ? 256 : kCeMaxThreads, WARP ? 4 : 2) soft
   for (int it = 0; row < p.rows; row += step, ++it) {
     // ---- tanh values and the sum of exp(z)
     float2 acc = make_float2(0.f, 0.f);
+    float m_run = -3.0e38f, s_run = 0.f;          // WHOLE: running maximum and sum (of a lane of one of the row's warps)
+    float m_row = -3.0e38f, s_row = 0.f;          // WARP && WHOLE: what the warps before this pass have found
     uint32_t top = 0u;
-    for (int i = q.first + tid; i < q.last; i += nt) {
+    auto warp_lse = [&] {                         // the sum over a warp's lanes, in lane 0's order
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        lse_merge(m_run, s_run, __shfl_xor_sync(0xffffffffu, m_run, o), __shfl_xor_sync(0xffffffffu, s_run, o));
+    };
+    // (one warp per row takes the part of warp 0, 1, ... of a block in turn: its passes are full up to the last, so that the
+    // shuffles meet every lane)
+    const int end = WARP && WHOLE ? (q.last + 31) & ~31 : q.last;
+    for (int i = q.first + tid; i < end; i += nt) {
       const uint4 w = w0;
       w0 = w1;
       w1 = load(q, i + 2 * nt);
       const uint32_t wi[4] = {w.x, w.y, w.z, w.w};
       uint4 to;
       uint32_t* tp = &to.x;
-      float2 e[4];
+      float2 z[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const uint32_t mag = wi[j] & 0x7fff7fffu;
         top = __vmaxu2(top, mag);
         tp[j] = tanh_pair(wi[j], mag);
-        const float2 zl = __fmul2_rn(capped(tp[j]), l2e);
-        e[j] = make_float2(ex2(zl.x), ex2(zl.y));
+        z[j] = capped(tp[j]);
       }
-      row_t[i] = to;
-      acc = __fadd2_rn(acc, __fadd2_rn(__fadd2_rn(e[0], e[1]), __fadd2_rn(e[2], e[3])));
+      if (!(WARP && WHOLE) || i < q.last) row_t[i] = to;
+      if constexpr (WHOLE) {
+        if (!WARP || i < q.last) {
+          const float mx = fmaxf(fmaxf(fmaxf(z[0].x, z[0].y), fmaxf(z[1].x, z[1].y)), fmaxf(fmaxf(z[2].x, z[2].y), fmaxf(z[3].x, z[3].y)));
+          const float mn = fmaxf(m_run, mx);
+          const float2 nmn = make_float2(-mn, -mn);
+          float2 a2 = make_float2(s_run * __expf(m_run - mn), 0.f);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 dz = __fmul2_rn(__fadd2_rn(z[j], nmn), l2e);
+            a2 = __fadd2_rn(a2, make_float2(ex2(dz.x), ex2(dz.y)));
+          }
+          s_run = a2.x + a2.y;
+          m_run = mn;
+        }
+        if constexpr (WARP) {
+          warp_lse();
+          lse_merge(m_row, s_row, m_run, s_run);
+          m_run = -3.0e38f;
+          s_run = 0.f;
+        }
+      } else {
+        float2 e[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 zl = __fmul2_rn(z[j], l2e);
+          e[j] = make_float2(ex2(zl.x), ex2(zl.y));
+        }
+        acc = __fadd2_rn(acc, __fadd2_rn(__fadd2_rn(e[0], e[1]), __fadd2_rn(e[2], e[3])));
+      }
     }
     const uint16_t* row_e = reinterpret_cast<const uint16_t*>(row_t);
-    const int e_mine = edge_of(q);
+    const int e_mine = WHOLE ? -1 : edge_of(q);
     uint32_t t_edge = 0u;
-    if (e_mine >= 0) {
+    if (!WHOLE && e_mine >= 0) {
       const uint32_t w = reinterpret_cast<const unsigned short*>(q.base)[e_mine];
       t_edge = tanh_pair(w, w & 0x7fffu) & 0xffffu;
       top = __vmaxu2(top, w & 0x7fffu);
@@ -377,18 +419,41 @@ __global__ void __launch_bounds__(WARP ? 256 : kCeMaxThreads, WARP ? 4 : 2) soft
       w0 = load(q, q.first + tid);
       w1 = load(q, q.first + tid + nt);
     }
-    float s = acc.x + acc.y;
-    if ((top & 0xffffu) > 0x7f80u || (top >> 16) > 0x7f80u) s = __int_as_float(0x7fffffff);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (!WARP) {
-      if (lane == 0) s_sum[it & 1][warp] = s;
+    const bool nan = (top & 0xffffu) > 0x7f80u || (top >> 16) > 0x7f80u;
+    float lse;
+    if constexpr (WHOLE && WARP) {
+      lse = __shfl_sync(0xffffffffu, m_row + logf(s_row), 0);
+      if (__any_sync(0xffffffffu, nan)) lse = __int_as_float(0x7fffffff);
+    } else if constexpr (WHOLE) {
+      if (nan) s_run = __int_as_float(0x7fffffff);
+      warp_lse();
+      if (lane == 0) {
+        s_sum[0][warp] = m_run;
+        s_sum[1][warp] = s_run;
+      }
       __syncthreads();
-      s = lane < nt / 32 ? s_sum[it & 1][lane] : 0.f;
+      if (threadIdx.x == 0) {
+        m_run = s_sum[0][0];
+        s_run = s_sum[1][0];
+#pragma unroll
+        for (int wi = 1; wi < kLossFwdThreads / 32; ++wi) lse_merge(m_run, s_run, s_sum[0][wi], s_sum[1][wi]);
+        s_lse = m_run + logf(s_run);
+      }
+      __syncthreads();
+      lse = s_lse;
+    } else {
+      float s = nan ? __int_as_float(0x7fffffff) : acc.x + acc.y;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (!WARP) {
+        if (lane == 0) s_sum[it & 1][warp] = s;
+        __syncthreads();
+        s = lane < nt / 32 ? s_sum[it & 1][lane] : 0.f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      }
+      lse = logf(s);
     }
-    const float lse = logf(s);
     const float2 nl2 = make_float2(-lse, -lse);
     int64_t t = p.targets_64 ? static_cast<const int64_t*>(p.targets)[row] : static_cast<const int32_t*>(p.targets)[row];
     t = t < 0 ? 0 : (t >= p.vocab ? p.vocab - 1 : t);                 // clamped, as jnp.take_along_axis does
@@ -477,15 +542,21 @@ extern "C" int tgh_softcap_ce(const void* logits, const void* targets, int targe
     int dev = 0;
     TG_CUDA_CHECK(cudaGetDevice(&dev));
     if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
-      TG_CUDA_CHECK(cudaFuncSetAttribute(softcap_ce_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeSmemMax));
-      TG_CUDA_CHECK(cudaFuncSetAttribute(softcap_ce_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeSmemMax));
+      for (auto kern : {softcap_ce_kernel<false, false>, softcap_ce_kernel<false, true>, softcap_ce_kernel<true, false>, softcap_ce_kernel<true, true>})
+        TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeSmemMax));
       attr_set[dev & 63].store(true, std::memory_order_release);
     }
     const size_t smem = size_t(ce_smem(vocab));
     const int64_t per_sm_smem = std::max<int64_t>(1, (227 * 1024) / int64_t(smem + 1024));
+    const bool whole = vocab % 8 == 0 && ld % 8 == 0;
     if (vocab <= kCeWarpCols) {
       const int64_t cap_blocks = int64_t(sm_count()) * std::min<int64_t>(per_sm_smem, 4);
-      softcap_ce_kernel<true><<<int(std::min<int64_t>((rows + 7) / 8, cap_blocks)), 256, smem, st>>>(a);
+      const int blocks = int(std::min<int64_t>((rows + 7) / 8, cap_blocks));
+      if (whole) softcap_ce_kernel<true, true><<<blocks, 256, smem, st>>>(a);
+      else softcap_ce_kernel<true, false><<<blocks, 256, smem, st>>>(a);
+    } else if (whole) {
+      const int64_t cap_blocks = int64_t(sm_count()) * std::min<int64_t>(per_sm_smem, 2);
+      softcap_ce_kernel<false, true><<<int(std::min<int64_t>(rows, cap_blocks)), kLossFwdThreads, smem, st>>>(a);
     } else {
       // as many threads as make the last pass over the row nearly full (of at most 640: two blocks an SM at 48 registers)
       const int64_t pieces = (vocab + 7) / 8;
@@ -496,7 +567,7 @@ extern "C" int tgh_softcap_ce(const void* logits, const void* targets, int targe
         if (full > best + 0.02) { best = full; nt = n; }
       }
       const int64_t cap_blocks = int64_t(sm_count()) * std::min<int64_t>(per_sm_smem, 1280 / nt);
-      softcap_ce_kernel<false><<<int(std::min<int64_t>(rows, cap_blocks)), nt, smem, st>>>(a);
+      softcap_ce_kernel<false, false><<<int(std::min<int64_t>(rows, cap_blocks)), nt, smem, st>>>(a);
     }
     TG_CUDA_CHECK(cudaGetLastError());
   }

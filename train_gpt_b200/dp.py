@@ -16,6 +16,7 @@ with one launch.
 """
 from __future__ import annotations
 
+import weakref
 from typing import List, Sequence
 
 import torch
@@ -28,10 +29,21 @@ class GradSlot:
     slice of its bucket, or, for parameters laid out side by side, the one matrix that holds all their
     gradients as column slices -- and `ready()` says that the gradients of `params` are now in place (what
     autograd's post-accumulate hook says for the others).  The op then returns None as that gradient.
-    A slot serves one write per step: a parameter used twice has to go through autograd's accumulation."""
+    A slot serves one write per step: a parameter used twice has to go through autograd's accumulation.
+    (Parameters carry their slot and the buckets hold both, so a slot refers to either weakly: a trainer's
+    memory goes when the trainer does, not when the garbage collector happens to run.)"""
 
     def __init__(self, owner: "GradBuckets", bi: int, params, out: torch.Tensor):
-        self.owner, self.bi, self.params, self.out, self.used = owner, bi, tuple(params), out, False
+        self._owner, self._params = weakref.ref(owner), [weakref.ref(p) for p in params]
+        self.bi, self.out, self.used = bi, out, False
+
+    @property
+    def owner(self):
+        return self._owner()
+
+    @property
+    def params(self):
+        return tuple(r() for r in self._params)
 
     def take(self) -> torch.Tensor:
         if self.used:
@@ -40,8 +52,23 @@ class GradSlot:
         return self.out
 
     def ready(self) -> None:
-        for _ in self.params:
-            self.owner._one_done(self.bi)
+        owner = self.owner
+        for _ in self._params:
+            owner._one_done(self.bi)
+
+
+class SideBySide:
+    """What a parameter laid out side by side with others carries as `side_by_side`: (the whole matrix, the
+    parameters whose column slices it consists of), the latter held weakly as the parameter is one of them."""
+
+    def __init__(self, whole: torch.Tensor, params):
+        self._whole, self._params = whole, [weakref.ref(p) for p in params]
+
+    def __len__(self):
+        return 2
+
+    def __getitem__(self, i):
+        return (self._whole, tuple(r() for r in self._params))[i]
 
 
 class GradBuckets:
@@ -159,14 +186,23 @@ class GradBuckets:
                         left.append((off + n, b))
                 self._zero_ranges[bi] = left
 
+    def bucket_done(self, bi: int) -> None:
+        """All gradients of bucket `bi` are in place (said at once, by a backward pass that does not go through autograd)."""
+        self._pending[bi] = 0
+        self._launch(bi)
+
     def _one_done(self, bi: int) -> None:
         self._pending[bi] -= 1
         if self._pending[bi] == 0:
             self._launch(bi)
 
     def _make_hook(self, bi: int):
+        ref = weakref.ref(self)              # a parameter carries the hook and the buckets hold the parameter
+
         def hook(_param):
-            self._one_done(bi)
+            owner = ref()
+            if owner is not None:
+                owner._one_done(bi)
         return hook
 
     def _launch(self, bi: int):
@@ -211,7 +247,7 @@ class GradBuckets:
     def flatten_parameters(self) -> List[torch.Tensor]:
         """Move every bucket's parameters into one flat tensor per bucket, laid out like its gradients
         (each parameter becomes a view of its slice -- a column slice, not contiguous, for parameters laid
-        out side by side, which also get `side_by_side = (the whole matrix, the parameters in it)`; values
+        out side by side, which also get `side_by_side`, a pair (the whole matrix, the parameters in it); values
         are kept), and return those tensors.  An
         elementwise optimiser whose hyper-parameters are the same for every tensor can then update a
         bucket with one launch over (flat parameters, flat gradients) instead of one per tensor."""
@@ -230,7 +266,7 @@ class GradBuckets:
                 if rows:
                     whole = fp[off:off + rows * cols].view(rows, cols)
                     for q in grp:
-                        q.side_by_side = (whole, grp)
+                        q.side_by_side = SideBySide(whole, grp)
             out.append(fp)
         return out
 

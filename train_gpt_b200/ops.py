@@ -161,6 +161,7 @@ STATUS_ROLES = {
     4: "the MMA issuer waited for its last instructions to retire",
     5: "the promotion warps waited for an accumulator buffer to fill",
 }
+STATUS_TOKEN = 16   # a training step met a token id outside the vocabulary
 
 def default_status(device) -> torch.Tensor:
     """The status word every gemm_* call on `device` uses when the caller passes none: one word per
@@ -173,6 +174,8 @@ def status_error(code: int):
     """The exception for a non-zero GEMM status code, or None for 0."""
     if code == 0:
         return None
+    if int(code) == STATUS_TOKEN:
+        return RuntimeError(f"token id outside the vocabulary (status {int(code)})")
     why = STATUS_ROLES.get(int(code), "unknown role")
     return RuntimeError(f"block-scaled GEMM gave up on a bounded device wait (status {int(code)}: {why}); "
                         "its output is incomplete")

@@ -2,13 +2,12 @@
 clip_norm)` (train.py:114-123) = optax.chain(clip_by_global_norm, adamw), for bf16 parameters
 whose gradients live in flat buckets (`dp.GradBuckets`).
 
-Global norm: one sum-of-squares kernel per bucket, their float32 results added on the device.
-Update: one kernel per parameter tensor -- or, when the parameters of a bucket live in one flat
-tensor laid out like the bucket's gradients (`flat=`; optax's adamw has the same hyper-parameters
-for every leaf, so the update is one elementwise map over the concatenation), one kernel per
-bucket -- that applies the clip factor to the gradient as it reads it, so the clipped gradient is
-never written.  Step count and clip factor stay on the device, which lets the whole step be
-replayed from a CUDA graph.
+Global norm: one kernel over all gradient tensors.  Update: one kernel over all parameter tensors --
+or over the flat tensors that hold a bucket's parameters, laid out like the bucket's gradients
+(`flat=`; optax's adamw has the same hyper-parameters for every leaf, so the update is one
+elementwise map over the concatenation) -- that derives the clip factor from the norm and applies
+it to the gradient as it reads it, so the clipped gradient is never written.  Norm and step count
+stay on the device, which lets the whole step be replayed from a CUDA graph.
 """
 from __future__ import annotations
 
@@ -47,9 +46,9 @@ class ClippedAdamW:
         else:
             self.m = [torch.zeros_like(p) for p in self.params]           # optax: moments in the parameter dtype
             self.v = [torch.zeros_like(p) for p in self.params]
-        self.step_t = torch.zeros((), dtype=torch.int32, device=dev)
-        self._scratch = None
-        self._sq = None
+        self._count = torch.zeros((2,), dtype=torch.int32, device=dev)    # the step count and the update kernel's ticket
+        self.step_t = self._count[0]
+        self._scratch = (0, None)
 
     def state_tensors(self):
         return self.m + self.v + [self.step_t]
@@ -57,23 +56,18 @@ class ClippedAdamW:
     def global_norm(self, flat_grads: Sequence[torch.Tensor]) -> torch.Tensor:
         """optax.global_norm (train.py:132) over the flat gradient buckets."""
         flats = [f for f in flat_grads if f.numel()]
-        if self._sq is None:
-            dev = flats[0].device
-            self._sq = torch.empty((len(flats),), dtype=torch.float32, device=dev)
-            self._scratch = torch.empty((ops._lib.load().tg_sumsq_scratch_bytes(),), dtype=torch.uint8, device=dev)
-        for i, f in enumerate(flats):
-            ops.sumsq(f, out=self._sq[i:i + 1], scratch=self._scratch)
-        return self._sq.sum().sqrt()
+        if self._scratch[0] != len(flats):
+            self._scratch = (len(flats), ops._host().global_norm_scratch(flats[0], len(flats)))
+        return ops._host().global_norm(flats, self._scratch[1])
 
     def step(self, gnorm: torch.Tensor) -> None:
         """Clip by `gnorm` (optax.clip_by_global_norm: factor clip/norm when norm > clip) and update."""
-        scale = torch.where(gnorm < self.clip, torch.ones_like(gnorm), self.clip / gnorm).to(torch.float32)
-        self.step_t += 1
         if self._flat is not None:
-            for fp, fg, fm, fv in self._flat:
-                ops.adamw_step(fp, fg, fm, fv, self.step_t, self.lr, self.b1, self.b2, self.eps, self.wd, gscale=scale)
+            p, g, m, v = zip(*self._flat)
+        else:
+            live = [(q.data, q.grad, m, v) for q, m, v in zip(self.params, self.m, self.v) if q.grad is not None]
+            p, g, m, v = zip(*live) if live else ((), (), (), ())
+        if not p:
+            self.step_t += 1
             return
-        for p, m, v in zip(self.params, self.m, self.v):
-            if p.grad is None:
-                continue
-            ops.adamw_step(p.data, p.grad, m, v, self.step_t, self.lr, self.b1, self.b2, self.eps, self.wd, gscale=scale)
+        ops._host().clipped_adamw(p, g, m, v, self._count, gnorm, self.clip, self.lr, self.b1, self.b2, self.eps, self.wd)

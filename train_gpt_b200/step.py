@@ -389,7 +389,8 @@ class Trainer:
     about 1900 kernel launches through Python, which leaves the GPU idle a quarter of the time
     when they are launched one by one.  Batches are copied into fixed device buffers before each
     replay; the returned loss and gradient norm are the graph's own output tensors (read them
-    before the next step).  Capture needs two eager warm-up steps; parameters and optimizer
+    before the next step).  With the default switches the step itself is a native program (csrc/step.cpp)
+    that launches what the model would through autograd, bit for bit.  Capture needs two eager warm-up steps; parameters and optimizer
     state are restored after them, so a captured run follows the same trajectory as an eager one.
     """
 
@@ -432,7 +433,41 @@ class Trainer:
             self.opt = torch.optim.AdamW(self.model.parameters(), lr=cfg.lr, weight_decay=cfg.weight_decay,
                                          betas=(0.9, 0.999), eps=1e-8, fused=on_gpu, capturable=self._want_graph)
 
+        self._program = self._native_program()
+
+    def _native_program(self):
+        """The step as one native program (csrc/step.cpp) where every switch has its default value; None otherwise."""
+        c, b = self.cfg, self.buckets
+        h = c.n_heads * c.head_dim
+        if not (torch.device(self.device).type == "cuda" and c.mm == "fp8" and c.norm == "fused" and c.mlp == "fused" and c.qkv == "fused"
+                and c.residual == "fused" and c.loss == "fused" and self._fused_opt and c.flat_parameters and c.direct_grads
+                and c.activation in ("gelu", "relu2") and c.d_model <= ops.ADD_NORM_MAX_COLS
+                and not (c.d_model % 128 or h % 128 or c.d_ff % 128)):
+            return None
+        host = ops._host()
+        if not host.softcap_ce_fits(c.logit_cap, 1, c.vocab_size) or not all(p.requires_grad for p in self.model.parameters()):
+            return None
+        m = self.model
+        grads = {id(p): g for bi, params in enumerate(b.params) for p, g in zip(params, b.views(bi, b.flat[bi]))}
+        layers, g_layers = [], []
+        for lp in m.layers:
+            if getattr(lp["wq"], "side_by_side", None) is None or getattr(lp["wq"], "grad_slot", None) is None:
+                return None
+            rest = ("wo", "norm2", "w_up", "w_down")
+            layers.append([lp["norm1"], lp["wq"].side_by_side[0], *(lp[n] for n in rest)])
+            g_layers.append([grads[id(lp["norm1"])], lp["wq"].grad_slot.out, *(grads[id(lp[n])] for n in rest)])
+        from ._lib import TG_ACT
+        many = self.world > 1
+        return host.StepProgram(
+            (c.n_heads, c.head_dim, c.rms_eps, c.logit_cap, TG_ACT[c.activation], TG_ACT[c.activation + "_bwd"]),
+            (self.opt.lr, self.opt.b1, self.opt.b2, self.opt.eps, self.opt.wd, self.opt.clip),
+            m.embed, m.pos, m.final_norm, m.unembed, layers, grads[id(m.embed)], grads[id(m.pos)], grads[id(m.final_norm)],
+            grads[id(m.unembed)], g_layers, [list(f) for f in self.opt._flat], self.opt._count,
+            b.bucket_done if many else None, b.flush if many else None, b.finish if many else None)
+
     def _eager_step(self, ids, targets):
+        if self._program is not None:
+            return self._program.step(ids, targets)
         self.buckets.zero()
         loss = self.model.loss(ids, targets)
         loss.backward()
