@@ -298,6 +298,29 @@ __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
   return r;
 }
 
+// ---- programmatic dependent launch ---------------------------------------------------------
+// Used between the short kernels of an inference call, where a launch's latency is comparable with the work.  (In a training
+// step's graph of longer kernels it measured slower: blocks that sit in their wait hold resources the running kernel's last
+// wave could have used.)  A kernel launched early touches no memory before grid_wait(), so ordering is that of the stream.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A launch that may begin while the kernel before it on the stream is still running.
+template <typename... P, typename... A>
+static cudaError_t launch_early(void (*kern)(P...), int grid, int threads, int smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(grid));
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.dynamicSmemBytes = size_t(smem);
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 #endif  // __CUDACC__
 
 }  // namespace tg

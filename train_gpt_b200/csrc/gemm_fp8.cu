@@ -36,8 +36,8 @@
 // K-major and MN-major storage (only the coordinates swap), and the shared-memory operand
 // descriptors / instruction descriptor carry the major-ness, so dgrad and wgrad read the
 // same buffers the forward wrote, untransposed.  Few output tiles with a long contraction are
-// cut along the contraction (plan_split); few rows against a wide weight run with the operands
-// swapped (plan_skinny).
+// cut along the contraction (plan_split); few rows against a wide weight take the kernel of
+// gemm_skinny.cu.
 //
 // Every wait on an mbarrier is bounded: when the limit runs out the waiting role raises a
 // CTA-wide abort flag, stores a code in *status, and all roles fall through to the common
@@ -46,6 +46,7 @@
 
 #include "common.cuh"
 #include "mbarrier.cuh"
+#include "umma.cuh"
 
 #ifndef TG_X_BAND
 #define TG_X_BAND 16
@@ -59,12 +60,6 @@
 
 namespace tg {
 
-constexpr int BM = 128;          // tile rows (TMEM lanes)
-constexpr int BK = 128;          // contraction block = scale granularity (fp8.py:27)
-constexpr int UMMA_K = 32;       // K of one tcgen05.mma.kind::f8f6f4
-constexpr int kTmemCols = 512;
-constexpr int kTileBytes = 128 * 128;            // one operand TMA box: 128 rows x 128 bytes
-constexpr int kSmemLimit = 227 * 1024;
 constexpr int kBandRows = TG_X_BAND;             // tile rows per band of the tile numbering (see tile_coords)
 
 // Compile-time plan of one kernel variant.
@@ -138,7 +133,6 @@ struct Cfg {
 struct GemmParams {
   const float* sa;
   long long sa_sm, sa_sk;
-  int sa_shift;         // SA is indexed by (row >> sa_shift): 0 = a scale per row, 7 = one per 128 rows
   const float* sb;
   long long sb_sn, sb_sk;
   void* d;              // output, row pitch ldd elements
@@ -157,126 +151,6 @@ struct GemmParams {
   long long slice_elems;
   unsigned* status;
 };
-
-// ---- PTX wrappers ----------------------------------------------------------------------
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
-      : "memory");
-}
-
-// Bulk tensor store of one box from shared memory; completion is tracked by the issuing thread's
-// bulk async-group, so the same lane must commit and later wait.
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(x), "r"(y), "r"(z)
-               : "memory");
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ void tma_store_3d_nocommit(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(x), "r"(y), "r"(z)
-               : "memory");
-}
-// returns once every bulk store this thread committed has finished READING shared memory
-__device__ __forceinline__ void tma_store_wait_read() {
-  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                        uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// 32 lanes x 32 consecutive columns of 32-bit: thread i <- lane (base_lane + i), v[j] <- column j
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-        "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-        "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr)
-      : "memory");
-}
-
-// Wait for this thread's outstanding tcgen05.ld.  The registers are listed as in/out
-// operands so that no use of them can be scheduled above the wait.
-__device__ __forceinline__ void tmem_wait_ld(uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.wait::ld.sync.aligned;"
-      : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
-        "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]),
-        "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]),
-        "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
-      :
-      : "memory");
-}
-
-// 16-column variants (fewer live registers: used by the 64-columns-per-warp tile)
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_wait_ld16(uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.wait::ld.sync.aligned;"
-      : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
-        "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
-      :
-      : "memory");
-}
-
-// 16 lanes x 16 consecutive columns of 32-bit, in the fragment layout of an MMA accumulator: thread
-// t (g = t / 4, j = t % 4) gets, for k = 0, 1:  v[4k], v[4k+1] <- lane base + g,     columns 8k + 2j, 8k + 2j + 1
-//                                               v[4k+2], v[4k+3] <- lane base + g + 8, same columns
-__device__ __forceinline__ void tmem_ld_frag16(uint32_t taddr, uint32_t* v) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-      : "r"(taddr)
-      : "memory");
-}
-
-// Shared-memory operand descriptor, 128-byte swizzle, 8-row groups 1024 bytes apart.
-//   bits  0-13 start address >> 4      bits 16-29 leading byte offset >> 4
-//   bits 32-45 stride byte offset >> 4 bits 46-47 descriptor version (1 on sm_100)
-//   bits 61-63 layout (2 = 128B swizzle)
-// K-major: rows of 128 contraction bytes; 8 rows per swizzle atom; LBO unused.
-// MN-major: rows of 128 m/n bytes, one row per k; SBO = stride between 8-k groups; LBO =
-// stride between 128-wide m/n chunks (one chunk here).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= uint64_t((saddr >> 4) & 0x3FFFu);
-  d |= uint64_t(kTileBytes >> 4) << 16;
-  d |= uint64_t(1024 >> 4) << 32;
-  d |= uint64_t(1) << 46;
-  d |= uint64_t(2) << 61;
-  return d;
-}
-
-__device__ __forceinline__ float ldg_f32(const float* ptr) {
-  float v;
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(ptr));   // L1-allocating: an activation scale's line serves 16-32 blocks
-  return v;
-}
 
 // Staging stores of the epilogue, address = (base + OFF) ^ flip with OFF a compile-time constant.
 // The address is formed inside the asm block so that the compiler cannot hoist one register per
@@ -436,6 +310,8 @@ gemm_fp8_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  grid_trigger();
+  grid_wait();            // (both do nothing where the launch was an ordinary one)
 
   if (warp >= C::promo_warps) {
     if (C::regsteal) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::service_regs));
@@ -604,7 +480,7 @@ gemm_fp8_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a,
       tile_coords(p, tile, tm, tn);
       const int n0 = tn * BN;
       const int m = min(tm * BM + r, p.M - 1);       // rows past M: a valid scale, results never stored
-      sa_off = uint32_t(m >> p.sa_shift) * uint32_t(p.sa_sm) + kb_off * uint32_t(p.sa_sk);
+      sa_off = uint32_t(m) * uint32_t(p.sa_sm) + kb_off * uint32_t(p.sa_sk);
       if (SB_GRAN == 1) {
         const int col = min(n0 + c0 + kPerLane * lane, p.N - kPerLane);   // N % 8 == 0: a pair is in or out together
         sb_off = uint32_t(col) * uint32_t(p.sb_sn) + kb_off * uint32_t(p.sb_sk);
@@ -849,42 +725,6 @@ gemm_fp8_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
 // ---- host ------------------------------------------------------------------------------
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static int get_encode_fn(EncodeTiledFn* out) {
-  static EncodeTiledFn cached = nullptr;
-  if (cached == nullptr) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    TG_CUDA_CHECK(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres));
-    if (qres != cudaDriverEntryPointSuccess || fn == nullptr)
-      return record_cuda_error(cudaErrorSymbolNotFound, "cuTensorMapEncodeTiled entry point");
-    cached = reinterpret_cast<EncodeTiledFn>(fn);
-  }
-  *out = cached;
-  return TG_OK;
-}
-
-// 2-D tensor [outer][inner] of `esize`-byte elements, row pitch `pitch_bytes`; box of
-// `box_inner_bytes` (32, 64 or 128, = the swizzle span) x `box_rows`.
-static int make_tmap(CUtensorMap* map, CUtensorMapDataType dt, int esize, const void* base, int64_t inner,
-                     int64_t outer, int64_t pitch_bytes, int box_inner_bytes, int box_rows) {
-  EncodeTiledFn enc;
-  if (int rc = get_encode_fn(&enc)) return rc;
-  cuuint64_t dims[2] = {cuuint64_t(inner), cuuint64_t(outer)};
-  cuuint64_t strides[1] = {cuuint64_t(pitch_bytes)};
-  cuuint32_t box[2] = {cuuint32_t(box_inner_bytes / esize), cuuint32_t(box_rows)};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   box_inner_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
-                   : box_inner_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return record_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled");
-  return TG_OK;
-}
-
 template <int BN_, int SB_GRAN, bool OUT_F32>
 static int launch_gemm(const tg_gemm_args* a, GemmParams p, cudaStream_t st) {
   using C = Cfg<BN_, SB_GRAN, OUT_F32>;
@@ -941,6 +781,11 @@ static int launch_gemm(const tg_gemm_args* a, GemmParams p, cudaStream_t st) {
     TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem_bytes));
     attr_set[dev] = true;
   }
+  // few tokens: an inference call, whose kernels are short enough for an early launch to show
+  if (p.a_mn == 0 && a->M <= 256) {
+    TG_CUDA_CHECK(launch_early(kern, grid, C::threads, C::smem_bytes, st, ta, tb, td, p));
+    return TG_OK;
+  }
   kern<<<grid, C::threads, C::smem_bytes, st>>>(ta, tb, td, p);
   TG_CUDA_CHECK(cudaGetLastError());
   return TG_OK;
@@ -975,39 +820,6 @@ splitk_reduce_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, 
   }
 }
 
-// The same reduction for a problem that ran with its operands swapped (see plan_skinny): the slices
-// hold D^T, [S][N][pitch] float32 with the M tokens along the fast axis; the output is D [M][ldd].
-// One block transposes a 32 x 32 patch through shared memory so that reads and writes both coalesce.
-template <bool OUT_F32>
-__global__ void __launch_bounds__(256)
-splitk_reduce_transpose_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, int N, long long ldd, int S,
-                               long long slice_elems, int pitch) {
-  __shared__ float tile[32][33];
-  const int n0 = blockIdx.x * 32, m0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;      // 32 x 8
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int n = n0 + ty + 8 * i, m = m0 + tx;
-    float acc = 0.f;
-    if (n < N && m < M) {
-      const float* q = ws + (long long)n * pitch + m;
-      acc = q[0];
-      for (int sl = 1; sl < S; ++sl) acc += q[sl * slice_elems];
-    }
-    tile[ty + 8 * i][tx] = acc;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty + 8 * i, n = n0 + tx;
-    if (n < N && m < M) {
-      const float v = tile[tx][ty + 8 * i];
-      if (OUT_F32) static_cast<float*>(d)[(long long)m * ldd + n] = v;
-      else static_cast<__nv_bfloat16*>(d)[(long long)m * ldd + n] = __float2bfloat16_rn(v);
-    }
-  }
-}
-
 struct SplitPlan {
   int S;             // 1 = no split
   int64_t bytes;     // workspace the split needs
@@ -1035,40 +847,6 @@ static SplitPlan plan_split(const tg_gemm_args* a, int bn) {
     if (S == 1 || cost < best * 0.98) { best = cost; pl.S = S; }
   }
   if (pl.S > 1) pl.bytes = int64_t(pl.S) * a->M * a->N * int64_t(sizeof(float));
-  return pl;
-}
-
-// ---- few tokens, wide weight ---------------------------------------------------------------
-// With M <= 128 rows a 128-row MMA tile is mostly dead rows and there are only N / 256 output tiles
-// for 148 SMs, while the whole job is one pass over the weight (K x N bytes): it is bound by HBM, not by
-// the tensor core.  Such a problem runs TRANSPOSED: the weight's N becomes the MMA's 128-row dimension
-// (no dead rows, N / 128 tiles), the M tokens its 128 columns, the contraction is cut so that every SM
-// streams its own piece of the weight, and the float32 partial sums of D^T are added and transposed
-// back by splitk_reduce_transpose_kernel.  The per-token scales become per-column scales, the weight's
-// scales per-row (one per 128 rows for 128 x 128 weight tiles).  Measured at K = N = 8192 (CUDA-graph
-// replays): M = 16 20.6 us against 29.6 us the ordinary way (3.3 against 2.3 TB/s of weight stream),
-// M = 64 22.8 / 30.3, M = 128 27.2; from M = 192 on the ordinary tiling is faster (37 against ~33 us).
-struct SkinnyPlan {
-  bool on;
-  int bn;            // tile width over the tokens
-  int S;             // contraction ranges
-  int pitch;         // row pitch of a D^T slice, in floats
-  int64_t bytes;     // workspace
-};
-
-static SkinnyPlan plan_skinny(const tg_gemm_args* a) {
-  SkinnyPlan pl = {false, 0, 1, 0, 0};
-  if (a->M > 128 || a->M % 8 != 0 || a->N < 1024 || a->K % BK != 0 || a->K < 1024) return pl;
-  if (a->a_major != TG_MAJOR_K) return pl;          // the activation must be [M][K]: it becomes the K-major B operand
-  const int sms = gemm_sms();
-  if (sms <= 0) return pl;
-  pl.on = true;
-  pl.bn = 128;
-  const int64_t tiles = ((a->N + BM - 1) / BM) * ((a->M + pl.bn - 1) / pl.bn);
-  const int64_t nkb = a->K / BK;
-  while (pl.S < 8 && tiles * pl.S < sms && nkb % (2 * pl.S) == 0 && nkb / (2 * pl.S) >= 4) pl.S *= 2;
-  pl.pitch = int((a->M + 3) / 4 * 4);
-  pl.bytes = int64_t(pl.S) * a->N * pl.pitch * int64_t(sizeof(float));
   return pl;
 }
 
@@ -1104,40 +882,8 @@ static int validate_gemm(const tg_gemm_args* a) {
 
 extern "C" int64_t tg_gemm_workspace_bytes(const tg_gemm_args* a) {
   if (validate_gemm(a) != TG_OK || a->M == 0 || a->N == 0 || a->K == 0) return 0;
-  const SkinnyPlan sk = plan_skinny(a);
-  if (sk.on) return sk.bytes;
+  if (skinny_takes(a)) return skinny_workspace_bytes(a);
   return plan_split(a, tile_width(a)).bytes;
-}
-
-// The transposed run of a few-token problem (plan_skinny): D^T = B A^T into the workspace, then reduce + transpose.
-static int run_skinny(const tg_gemm_args* a, const SkinnyPlan& sk, cudaStream_t st) {
-  tg_gemm_args t = *a;
-  t.a = a->b; t.lda = a->ldb; t.a_major = a->b_major;
-  t.b = a->a; t.ldb = a->lda; t.b_major = a->a_major;
-  t.M = a->N; t.N = a->M;
-  GemmParams p;
-  p.sa = a->sb; p.sa_sm = a->sb_stride_n; p.sa_sk = a->sb_stride_kb; p.sa_shift = a->sb_gran_n == 128 ? 7 : 0;
-  p.sb = a->sa; p.sb_sn = a->sa_stride_m; p.sb_sk = a->sa_stride_kb;
-  p.d = a->workspace; p.ldd = sk.pitch;
-  p.M = int(t.M); p.N = int(t.N); p.nkb = int(a->K / BK) / sk.S;
-  p.nkb_rem = 0;
-  p.a_mn = t.a_major == TG_MAJOR_MN; p.b_mn = false;
-  p.tiles_m = p.tiles_n = 0;
-  p.band = 1;
-  p.ksplit = sk.S;
-  p.slice_elems = t.M * sk.pitch;
-  p.status = a->status;
-  const int rc = launch_gemm<128, 1, true>(&t, p, st);
-  if (rc != TG_OK) return rc;
-  const dim3 grid(unsigned((a->N + 31) / 32), unsigned((a->M + 31) / 32));
-  if (a->out_dtype == TG_OUT_F32)
-    splitk_reduce_transpose_kernel<true><<<grid, 256, 0, st>>>(static_cast<const float*>(a->workspace), a->d, int(a->M), int(a->N),
-                                                                  a->ldd, sk.S, p.slice_elems, sk.pitch);
-  else
-    splitk_reduce_transpose_kernel<false><<<grid, 256, 0, st>>>(static_cast<const float*>(a->workspace), a->d, int(a->M), int(a->N),
-                                                                   a->ldd, sk.S, p.slice_elems, sk.pitch);
-  TG_CUDA_CHECK(cudaGetLastError());
-  return TG_OK;
 }
 
 extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
@@ -1161,13 +907,10 @@ extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
         n_sb * a->sb_stride_n + nkb_all * a->sb_stride_kb > INT32_MAX)
       return TG_ERR_TOO_LARGE;
   }
-  {
-    const SkinnyPlan sk = plan_skinny(a);
-    if (sk.on && a->workspace != nullptr && a->workspace_bytes >= sk.bytes && aligned16(a->workspace))
-      return run_skinny(a, sk, st);
-  }
+  if (skinny_takes(a) && a->workspace != nullptr && a->workspace_bytes >= skinny_workspace_bytes(a) && aligned16(a->workspace))
+    return skinny_run(a, st);
   GemmParams p;
-  p.sa = a->sa; p.sa_sm = a->sa_stride_m; p.sa_sk = a->sa_stride_kb; p.sa_shift = 0;
+  p.sa = a->sa; p.sa_sm = a->sa_stride_m; p.sa_sk = a->sa_stride_kb;
   p.sb = a->sb; p.sb_sn = a->sb_stride_n; p.sb_sk = a->sb_stride_kb;
   p.d = a->d; p.ldd = a->ldd;
   p.M = int(a->M); p.N = int(a->N); p.nkb = int((a->K + BK - 1) / BK);

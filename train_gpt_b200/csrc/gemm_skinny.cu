@@ -1,0 +1,395 @@
+// Block-scaled e4m3 GEMM for few tokens (M <= 128) against a wide weight: D[m][n] = sum_kb SX(m,kb) SW(n,kb) X[m] . W[n].
+//
+// One pass over the weight is the work: at 16 x 8192 x 8192 it is 67 MB (10.2 us at the measured copy rate) against 0.7 us of
+// tensor-core time.  What the tiled kernel (gemm_fp8.cu) does badly there, and what is done instead:
+//   * the weight's N dimension takes the MMA's 128 rows and the tokens its columns (16, 32, 64 or 128 of them): no dead
+//     rows, and a stage of the pipeline is 16 KB of weight plus as little as 2 KB of tokens, so that 12 of them are in
+//     flight per SM;
+//   * the (tile, contraction block) units are numbered tile by tile and every block of the grid takes as many consecutive ones; it
+//     leaves each tile's part of float32 sums in a slot of the workspace.  Preferably a whole number of blocks shares a tile:
+//     all tiles are then at the same contraction rows at the same time, and what the SMs read together is whole rows of
+//     the weight, not 128-byte pieces of rows 8 KB apart (8192 x 8192: 5.0 against 4.5 TB/s);
+//   * scales arrive several blocks early (see the promotion warps);
+//   * a thread holds one weight row's sums over the tokens, so a slot is written 128 consecutive bytes per warp and token, and
+//     the reduce kernel, which adds a tile's slots in order, reads and writes along N: nothing is transposed;
+//   * programmatic dependent launch: barriers, tensor memory and an L2 prefetch of this block's first weight boxes (the L2 is
+//     coherent: a prefetch of bytes the kernel before is still writing is harmless) happen while the kernel before runs, and
+//     the reduce kernel is resident when the last sums arrive.
+// Bound by the weight's bytes plus about 5.5 us of two launches' ramps.  Microseconds per GEMM in a chain of them, before (split
+// contraction, transposing reduce) -> now: 16 x 8192 x 8192 24.8 -> 16.4, 16 x 2048 x 6144 13.5 -> 6.8, 1 x 2048 x 6144
+// 9.9 -> 6.6, 64 x 2048 x 8192 14.2 -> 10.4, 16 x 1024 x 1024 8.8 -> 5.8.
+#include "umma.cuh"
+
+namespace tg {
+
+// From 129 tokens on the tokens fill 128 MMA rows themselves, a token scale is a thread's own number instead of a column's,
+// and the tiled kernel is the faster one (200 x 2048 x 8192: 13.5 us against 17 for this kernel with 256 columns).
+constexpr int kSkinnyMaxTokens = 128;
+
+template <int BN_>
+struct SkinnyCfg {
+  static constexpr int BN = BN_;                                    // tokens
+  // at most 32 columns of sums per warp (with 64 a warp's own chain of loads was longer than a unit: M = 64 21 us)
+  static constexpr int promo_warps = BN == 16 ? 4 : BN == 128 ? 16 : 8;
+  static constexpr int cols = BN / (promo_warps / 4);
+  static constexpr int producer_warp = promo_warps, issuer_warp = promo_warps + 1;
+  // two issuers take alternate units: a thread gets a tcgen05 instruction out every ~80 cycles whatever its size, and a unit's
+  // five would hold an SM to 16 KB per 330 ns
+  static constexpr int issuers = 2;
+  static constexpr int threads = 32 * (promo_warps + 1 + issuers);
+  static constexpr int bufs = 4;                                    // accumulator buffers in tensor memory
+  static constexpr int tmem_cols = BN * bufs < 32 ? 32 : BN * bufs;
+  static constexpr int stage_bytes = kTileBytes + BN * 128;
+  // scales, per promotion warp: the block's column factors, double-buffered, and a ring of `ahead` blocks' column and row scales
+  static constexpr int ahead = 8;
+  static constexpr int ring_slot = cols + 32;
+  static constexpr int warp_scales = 2 * cols + ahead * ring_slot;
+  static constexpr int scale_bytes = promo_warps * warp_scales * 4;
+  static constexpr int stages_fit = (kSmemLimit - 1024 - scale_bytes) / stage_bytes;
+  static constexpr int stages = stages_fit > 12 ? 12 : stages_fit;
+  static constexpr int smem_bytes = stages * stage_bytes + scale_bytes;
+  static constexpr int n_bars = 2 * stages + 2 * bufs + 1;
+  static_assert(n_bars <= 40, "control block too small");
+};
+
+struct SkinnyParams {
+  const float* sx;               // token scales, [m * sx_m + kb * sx_k]
+  const float* sw;               // weight scales, [n * sw_n + kb * sw_k], n in rows or in blocks of 128 (W_ROWS or not)
+  unsigned sx_m, sx_k, sw_n, sw_k;
+  float* ws;                     // slots of [M][128] sums
+  int M, N, nkb;
+  int units, w_mn;               // units = tiles * nkb; w_mn: the weight is stored [K][N]
+  unsigned* status;
+};
+
+// Block c of g takes units [c * units / g, (c + 1) * units / g); unit u belongs to block ((u + 1) g - 1) / units.  The part that
+// block c does of tile t has slot c + t: each step along the units enters a new block, a new tile, or both.
+__host__ __device__ __forceinline__ int skinny_first(int c, int g, int units) { return int((long long)c * units / g); }
+__host__ __device__ __forceinline__ int skinny_block_of(int u, int g, int units) { return int(((long long)(u + 1) * g - 1) / units); }
+
+__device__ __forceinline__ void l2_prefetch_2d(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y) : "memory");
+}
+
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// W_ROWS: a weight scale per row (128 x 1 tiles), else one per 128 rows
+template <int BN_, bool W_ROWS>
+__global__ void __launch_bounds__((SkinnyCfg<BN_>::threads), 1)
+gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const SkinnyParams p) {
+  using C = SkinnyCfg<BN_>;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ __align__(16) uint64_t ctl_bars[40];
+  __shared__ uint32_t ctl_tmem_ptr;
+  __shared__ int ctl_abort;
+  const uint32_t sbase = smem_u32(smem), bar0 = smem_u32(ctl_bars);
+  const uint32_t full0 = bar0, empty0 = bar0 + 8u * C::stages, tfull0 = bar0 + 16u * C::stages, tempty0 = tfull0 + 8u * C::bufs;
+  const uint32_t drain_bar = tempty0 + 8u * C::bufs;
+  volatile int* abort_flag = &ctl_abort;
+  if ((sbase & 1023u) != 0) {
+    if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0u, 6u);
+    return;
+  }
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int u0 = skinny_first(int(blockIdx.x), int(gridDim.x), p.units), u1 = skinny_first(int(blockIdx.x) + 1, int(gridDim.x), p.units);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::stages; ++s) {
+      mbar_init(full0 + 8u * s, 1);
+      mbar_init(empty0 + 8u * s, 1);
+    }
+    for (int b = 0; b < C::bufs; ++b) {
+      mbar_init(tfull0 + 8u * b, 1);
+      mbar_init(tempty0 + 8u * b, C::promo_warps);
+    }
+    mbar_init(drain_bar, C::issuers);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == C::producer_warp && elect_one()) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_x)) : "memory");
+    int kb = u0 % p.nkb, n0 = u0 / p.nkb * BM;
+    for (int u = u0; u < u1 && u < u0 + C::stages; ++u) {
+      l2_prefetch_2d(&tmap_w, p.w_mn ? n0 : kb * BK, p.w_mn ? kb * BK : n0);
+      if (++kb == p.nkb) { kb = 0; n0 += BM; }
+    }
+  }
+  if (warp == C::issuer_warp) {
+    tmem_alloc(smem_u32(&ctl_tmem_ptr), C::tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *static_cast<volatile uint32_t*>(&ctl_tmem_ptr);
+  grid_wait();            // what the kernels before wrote is visible from here on, and what they read may be overwritten
+  grid_trigger();
+
+  if (warp == C::producer_warp) {
+    uint32_t s = 0, ph = 1;
+    bool ok = true;
+    int kb = u0 % p.nkb, n0 = u0 / p.nkb * BM;
+    for (int u = u0; u < u1; ++u) {
+      ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8u * s, ph, abort_flag, p.status, 1u));
+      if (!ok) break;
+      if (elect_one()) {
+        const uint32_t dst = sbase + s * C::stage_bytes, fb = full0 + 8u * s;
+        const int k0 = kb * BK;
+        mbar_expect_tx(fb, C::stage_bytes);
+        tma_load_2d(dst, &tmap_w, fb, p.w_mn ? n0 : k0, p.w_mn ? k0 : n0);
+        tma_load_2d(dst + kTileBytes, &tmap_x, fb, k0, 0);
+      }
+      __syncwarp();
+      if (++s == C::stages) { s = 0; ph ^= 1u; }
+      if (++kb == p.nkb) { kb = 0; n0 += BM; }
+    }
+  } else if (warp >= C::issuer_warp) {
+    // columns of the MMA: the tokens there are, in sixteens
+    const uint32_t n_mma = uint32_t((p.M + 15) / 16 * 16);
+    const uint32_t idesc = (1u << 4) | (uint32_t(p.w_mn) << 15) | ((n_mma >> 3) << 17) | (uint32_t(BM >> 4) << 24);
+    const uint32_t a_step = p.w_mn ? (UMMA_K * 128) >> 4 : UMMA_K >> 4, b_step = UMMA_K >> 4;
+    const uint64_t desc_a0 = make_smem_desc(sbase), desc_b0 = make_smem_desc(sbase + kTileBytes);
+    const uint32_t desc_hi = uint32_t(desc_a0 >> 32), a_lo0 = uint32_t(desc_a0), b_lo0 = uint32_t(desc_b0);
+    const bool stage_lane = lane >= 16;
+    uint32_t s = uint32_t(warp - C::issuer_warp), sph = 0, buf = s, bph = 1;
+    bool ok = true;
+    for (int u = u0 + int(s); u < u1; u += C::issuers) {
+      const uint32_t bar = stage_lane ? full0 + 8u * s : tempty0 + 8u * buf;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar, stage_lane ? sph : bph, abort_flag, p.status, stage_lane ? 3u : 2u));
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t d_tmem = tmem_base + buf * uint32_t(BN_), soff = s * uint32_t(C::stage_bytes >> 4);
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k)
+          umma_f8(d_tmem, (uint64_t(desc_hi) << 32) | (a_lo0 + soff + k * a_step), (uint64_t(desc_hi) << 32) | (b_lo0 + soff + k * b_step),
+                  idesc, k > 0 ? 1u : 0u);
+        umma_commit(tfull0 + 8u * buf);      // (a promotion warp that sees this frees the stage)
+      }
+      __syncwarp();
+      if ((s += C::issuers) >= uint32_t(C::stages)) { s -= C::stages; sph ^= 1u; }
+      if ((buf += C::issuers) >= uint32_t(C::bufs)) { buf -= C::bufs; bph ^= 1u; }
+    }
+    if (elect_one()) {
+      umma_commit(drain_bar);
+      mbar_wait(drain_bar, 0u, abort_flag, p.status, 4u);
+    }
+    __syncwarp();
+  } else {
+    const int quarter = warp & 3, c0 = (warp >> 2) * C::cols, r = quarter * 32 + lane;
+    float* s_sc = reinterpret_cast<float*>(smem + C::stages * C::stage_bytes) + warp * C::warp_scales;
+    float* ring = s_sc + 2 * C::cols;
+    const uint32_t ring0 = smem_u32(ring);
+    const uint32_t tcol0 = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(c0);
+    // Scales come `ahead` blocks early into the warp's own ring (cp.async: no registers, no barrier).  A block's weight scales
+    // are in memory nobody has touched yet, so fetching them one block ahead made every block wait out a DRAM access:
+    // 8192 x 8192 took 18 us with a scale per 128 rows and 25 with one per row, whatever the token count.
+    constexpr int kPer = (C::cols + 31) / 32;          // column scales a lane fetches per block: columns c0 + lane (+ 32)
+    unsigned sx_off[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) sx_off[i] = unsigned(min(c0 + lane + 32 * i, p.M - 1)) * p.sx_m;      // past M: a valid scale, unused sums
+    int f_u = u0, f_kb = u0 % p.nkb, f_tile = u0 / p.nkb, f_slot = 0;      // the next block to fetch scales for
+    auto fetch = [&] {
+      if (f_u < u1) {
+        const uint32_t dst = ring0 + uint32_t(f_slot) * (C::ring_slot * 4);
+#pragma unroll
+        for (int i = 0; i < kPer; ++i)
+          if (C::cols % 32 == 0 || lane < C::cols)
+            cp_async4(dst + 4u * uint32_t(lane + 32 * i), p.sx + sx_off[i] + unsigned(f_kb) * p.sx_k);
+        if (W_ROWS) cp_async4(dst + 4u * uint32_t(C::cols + lane), p.sw + unsigned(min(f_tile * BM + r, p.N - 1)) * p.sw_n + unsigned(f_kb) * p.sw_k);
+        else if (lane == 0) cp_async4(dst + 4u * uint32_t(C::cols), p.sw + unsigned(f_tile) * p.sw_n + unsigned(f_kb) * p.sw_k);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");         // an empty group keeps the wait count uniform
+      ++f_u;
+      if (++f_kb == p.nkb) { f_kb = 0; ++f_tile; }
+      if (++f_slot == C::ahead) f_slot = 0;
+    };
+    for (int i = 0; i < C::ahead; ++i) fetch();
+    int kb = u0 % p.nkb, tile = u0 / p.nkb, slot = 0;
+    float2 acc[C::cols / 2];
+#pragma unroll
+    for (int j = 0; j < C::cols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
+    uint32_t buf = 0, bph = 0, stage_s = 0;
+    bool ok = true;
+    for (int u = u0; u < u1; ++u) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(C::ahead - 1) : "memory");
+      __syncwarp();
+      float* stage = s_sc + (u & 1) * C::cols;
+      const float* in = ring + slot * C::ring_slot;
+      const float sw = in[C::cols + (W_ROWS ? lane : 0)];
+      // column scale of the block, times the weight's where that is one number
+#pragma unroll
+      for (int i = 0; i < kPer; ++i)
+        if (C::cols % 32 == 0 || lane < C::cols) stage[lane + 32 * i] = W_ROWS ? in[lane + 32 * i] : in[lane + 32 * i] * sw;
+      __syncwarp();
+      fetch();                                                       // into the slot just read
+      if (++slot == C::ahead) slot = 0;
+      const bool ends = kb + 1 == p.nkb || u + 1 == u1;              // the last block of this tile here
+      const int tile_now = tile;
+      if (++kb == p.nkb) { kb = 0; ++tile; }
+      ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8u * buf, bph, abort_flag, p.status, 5u));
+      if (!ok) break;
+      tc_fence_after();
+      if (warp == 0) mbar_arrive_if(empty0 + 8u * stage_s, lane == 0);   // the unit's MMAs have read their operands
+      if (++stage_s == uint32_t(C::stages)) stage_s = 0;
+      const uint32_t taddr = tcol0 + buf * uint32_t(BN_);
+      const float2 sw2 = make_float2(sw, sw);
+#pragma unroll
+      for (int q = 0; q < C::cols / 16; ++q) {
+        uint32_t v[16];
+        tmem_ld16(taddr + 16 * q, v);
+        tmem_wait_ld16(v);
+        if (q == C::cols / 16 - 1) {                                 // every sum of the buffer is in registers: hand it back
+          tc_fence_before();
+          __syncwarp();
+          mbar_arrive_if(tempty0 + 8u * buf, lane == 0);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float4 sc = *reinterpret_cast<const float4*>(stage + 16 * q + 4 * j);
+          const float2 p0 = make_float2(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]));
+          const float2 p1 = make_float2(__uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+          float2 &a0 = acc[8 * q + 2 * j], &a1 = acc[8 * q + 2 * j + 1];
+          if (W_ROWS) {
+            a0 = __ffma2_rn(__fmul2_rn(p0, make_float2(sc.x, sc.y)), sw2, a0);
+            a1 = __ffma2_rn(__fmul2_rn(p1, make_float2(sc.z, sc.w)), sw2, a1);
+          } else {
+            a0 = __ffma2_rn(p0, make_float2(sc.x, sc.y), a0);
+            a1 = __ffma2_rn(p1, make_float2(sc.z, sc.w), a1);
+          }
+        }
+      }
+      if (++buf == C::bufs) { buf = 0; bph ^= 1u; }
+      if (ends) {
+        float* out = p.ws + size_t(int(blockIdx.x) + tile_now) * size_t(p.M) * BM + r;
+        const bool row_ok = tile_now * BM + r < p.N;
+#pragma unroll
+        for (int j = 0; j < C::cols; ++j)
+          if (row_ok && c0 + j < p.M) out[size_t(c0 + j) * BM] = (j & 1) ? acc[j / 2].y : acc[j / 2].x;
+#pragma unroll
+        for (int j = 0; j < C::cols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == C::issuer_warp) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem_base, C::tmem_cols);
+  }
+}
+
+// D[m][n] = the sum of a tile's slots, in block order.  A thread makes four consecutive n of one token.
+template <bool OUT_F32>
+__global__ void __launch_bounds__(256)
+skinny_reduce_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, int N, long long ldd, int nkb, int units, int g) {
+  const int i = int(blockIdx.x) * 256 + int(threadIdx.x), quads = (N + 3) / 4, m = i / quads, n = (i - m * quads) * 4;
+  grid_trigger();
+  grid_wait();
+  if (m >= M) return;
+  const int tile = n / BM;
+  const int c0 = skinny_block_of(tile * nkb, g, units), c1 = skinny_block_of(tile * nkb + nkb - 1, g, units);
+  const float* src = ws + (size_t(c0 + tile) * M + m) * BM + (n - tile * BM);
+  float4 a = __ldcg(reinterpret_cast<const float4*>(src));
+  for (int c = c0 + 1; c <= c1; ++c) {
+    src += size_t(M) * BM;
+    const float4 b = __ldcg(reinterpret_cast<const float4*>(src));
+    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+  }
+  if (OUT_F32) *reinterpret_cast<float4*>(static_cast<float*>(d) + m * ldd + n) = a;
+  else *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(d) + m * ldd + n) = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w));
+}
+
+// ---- host --------------------------------------------------------------------------------
+
+// The activation must be [M][K] (it becomes the K-major B operand).  Below 512 of contraction or 256 of width the weight is
+// nothing to stream and the tiled kernel's single launch is the shorter way.
+bool skinny_takes(const tg_gemm_args* a) {
+  return a->M > 0 && a->M <= kSkinnyMaxTokens && a->a_major == TG_MAJOR_K && a->K % BK == 0 && a->K >= 512 && a->N >= 256 && a->N <= (1 << 22) && a->K <= (1 << 22);
+}
+
+struct SkinnyPlan {
+  int tiles, nkb, units, grid;
+};
+static SkinnyPlan plan(const tg_gemm_args* a) {
+  SkinnyPlan p;
+  p.tiles = int((a->N + BM - 1) / BM);
+  p.nkb = int(a->K / BK);
+  p.units = p.tiles * p.nkb;
+  const int sms = gemm_sms();
+  p.grid = p.units < sms ? p.units : sms;
+  // Ranges that end where tiles end (tiles * s blocks, s to a tile) read whole rows together and leave fewer slots; all SMs
+  // (ranges that end anywhere) is the better balance.  In microseconds: 0.33 per unit on one SM (16 KB at 50 GB/s), all units
+  // at the measured 5.0 / 4.5 TB/s, a slot written and read at ~6 TB/s.
+  const double slot = double(a->M) * BM * 8 / 6.0e6;
+  auto cost = [&](int g, int slots, double rate) {
+    const double sm = 0.33 * ((p.units + g - 1) / g), hbm = double(p.units) * kTileBytes / rate;
+    return (sm > hbm ? sm : hbm) + slot * slots;
+  };
+  const int most = p.grid;
+  double best = cost(most, most + p.tiles, 4.5e6);
+  for (int s = 1; p.tiles * s <= most; ++s) {
+    const double c = cost(p.tiles * s, p.tiles * s, 5.0e6);
+    if (c < best) { best = c; p.grid = p.tiles * s; }
+  }
+  return p;
+}
+
+int64_t skinny_workspace_bytes(const tg_gemm_args* a) {
+  const SkinnyPlan p = plan(a);
+  return int64_t(p.grid + p.tiles) * a->M * BM * int64_t(sizeof(float));
+}
+
+template <int BN_, bool W_ROWS>
+static int launch(const tg_gemm_args* a, const SkinnyPlan& pl, SkinnyParams p, cudaStream_t st) {
+  using C = SkinnyCfg<BN_>;
+  auto kern = gemm_skinny_kernel<BN_, W_ROWS>;
+  CUtensorMap tw, tx;
+  const int64_t w_inner = p.w_mn ? a->N : a->K, w_outer = p.w_mn ? a->K : a->N;
+  if (int rc = make_tmap(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->b, w_inner, w_outer, a->ldb, 128, 128)) return rc;
+  if (int rc = make_tmap(&tx, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->a, a->K, a->M, a->lda, 128, BN_)) return rc;
+  static std::atomic<bool> attr_set[64];
+  int dev = 0;
+  TG_CUDA_CHECK(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return TG_ERR_SHAPE;
+  if (!attr_set[dev].load(std::memory_order_acquire)) {
+    TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem_bytes));
+    attr_set[dev].store(true, std::memory_order_release);
+  }
+  TG_CUDA_CHECK(launch_early(kern, pl.grid, C::threads, C::smem_bytes, st, tw, tx, p));
+  return TG_OK;
+}
+
+int skinny_run(const tg_gemm_args* a, cudaStream_t st) {
+  const SkinnyPlan pl = plan(a);
+  SkinnyParams p;
+  p.sx = a->sa; p.sx_m = unsigned(a->sa_stride_m); p.sx_k = unsigned(a->sa_stride_kb);
+  p.sw = a->sb; p.sw_n = unsigned(a->sb_stride_n); p.sw_k = unsigned(a->sb_stride_kb);
+  p.ws = static_cast<float*>(a->workspace);
+  p.M = int(a->M); p.N = int(a->N); p.nkb = pl.nkb;
+  p.units = pl.units;
+  p.w_mn = a->b_major == TG_MAJOR_MN;
+  p.status = a->status;
+  const bool rows = a->sb_gran_n == 1;
+  int rc;
+  if (a->M <= 16) rc = rows ? launch<16, true>(a, pl, p, st) : launch<16, false>(a, pl, p, st);
+  else if (a->M <= 32) rc = rows ? launch<32, true>(a, pl, p, st) : launch<32, false>(a, pl, p, st);
+  else if (a->M <= 64) rc = rows ? launch<64, true>(a, pl, p, st) : launch<64, false>(a, pl, p, st);
+  else rc = rows ? launch<128, true>(a, pl, p, st) : launch<128, false>(a, pl, p, st);
+  if (rc != TG_OK) return rc;
+  const int64_t threads = a->M * ((a->N + 3) / 4);
+  const int blocks = int((threads + 255) / 256);
+  if (a->out_dtype == TG_OUT_F32)
+    TG_CUDA_CHECK(launch_early(skinny_reduce_kernel<true>, blocks, 256, 0, st, static_cast<const float*>(p.ws), a->d, p.M, p.N,
+                               static_cast<long long>(a->ldd), p.nkb, p.units, pl.grid));
+  else
+    TG_CUDA_CHECK(launch_early(skinny_reduce_kernel<false>, blocks, 256, 0, st, static_cast<const float*>(p.ws), a->d, p.M, p.N,
+                               static_cast<long long>(a->ldd), p.nkb, p.units, pl.grid));
+  return TG_OK;
+}
+
+}  // namespace tg

@@ -556,6 +556,9 @@ Pair fp8_backward(const Tensor& a, const Tensor& b, const Tensor& g_, at::IntArr
                   at::ScalarType b_dtype, int64_t k, int64_t n, const BackwardIn& in) {
   Tensor da, db;
   if (in.mode == kSte) {
+    // (the engine's thread may not have touched the device yet, and cuBLAS wants a context when it makes its handle)
+    const c10::cuda::CUDAGuard guard(g_.device());
+    cudaFree(nullptr);
     const Tensor g2 = g_.reshape({-1, n}).to(at::kBFloat16);
     if (in.want_a) da = at::mm(g2, b.to(at::kBFloat16).t());                                 // fp8.py:96 (cuBLAS bf16)
     if (in.want_b) db = at::mm(a.reshape({-1, k}).to(at::kBFloat16).t(), g2);                // fp8.py:97

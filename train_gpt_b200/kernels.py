@@ -26,6 +26,8 @@ class NormedQuantized:
     usable as `a_quantized=` of `fp8.block_scaled_matmul` by every GEMM that consumes the
     same normed activation, plus the bf16 tensor itself when it was asked for."""
 
+    __slots__ = ("q", "scales", "y")
+
     def __init__(self, q, scales, y):
         self.q, self.scales, self.y = q, scales, y
 
@@ -36,5 +38,5 @@ class NormedQuantized:
 def rms_norm_quant(x, scale, eps: float, pure: bool = False, want_y: bool = False) -> NormedQuantized:
     """model.py:76-77 `_norm(...)` followed by the quantiser of fp8.py:66, one kernel.
     Forward only (no autograd); training code pairs it with `rms_norm`'s backward."""
-    q, s, y, _ = ops.rmsnorm_quant_fwd(x, scale, float(eps), pure=pure, want_y=want_y)
+    q, s, y, _ = ops._host().rmsnorm_quant_fwd(x, scale, eps, pure, want_y, False)
     return NormedQuantized(q, s, y)
