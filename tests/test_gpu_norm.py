@@ -177,3 +177,26 @@ def test_backward_matches_reference_vectors_and_autograd(golden):
     dg_ref = np.asarray(golden["norm_dgamma"]).view(BF16).astype(np.float32)
     assert np.abs(dg - dg_ref).max() <= 2.0 ** -6 * np.abs(dg_ref).max()
     assert x.grad.dtype == torch.bfloat16 and gamma.grad.shape == (256,)
+
+
+@pytest.mark.parametrize("rows,cols", [(8200, 128), (4100, 384), (1030, 1024), (700, 2048), (500, 2176), (460, 2560), (401, 3000), (371, 4096),
+                                       (301, 4352), (150, 5640), (180, 6144), (160, 6656), (155, 7040), (140, 8192)])
+@pytest.mark.parametrize("pure", [False, True])
+def test_every_split_of_a_row_over_warps(rows, cols, pure):
+    """Enough rows for the kernels that give one to eight warps to a row (fewer take a block per row): every number of chunks per
+    warp, whole and ragged, forward, quantised and backward, against the oracle."""
+    from train_gpt_b200 import ops
+    eps = 1e-6
+    x, gamma = _inputs((rows, cols), rows, eps)
+    xt, gt = to_torch_bf16(x), to_torch_bf16(gamma)
+    y, rn = ops.rmsnorm_fwd(xt, gt, eps, pure=pure, want_rnorm=True)
+    rn = rn.cpu().numpy()[..., None]
+    assert _ulp_diff_f32(rn, no.rnorm_of(x, eps)).max() <= 2
+    ref = (no.rms_norm_pure if pure else no.rms_norm)(x, gamma, eps, rnorm=rn)
+    assert np.array_equal(from_torch_bf16(y).view(np.uint16), ref.view(np.uint16))
+    if cols % 128 == 0:
+        q, s, y2, _ = ops.rmsnorm_quant_fwd(xt, gt, eps, pure=pure, want_y=True)
+        q_ref, s_ref = ops.quantize_rowwise(y)
+        assert torch.equal(y2, y) and torch.equal(q.view(torch.uint8), q_ref.view(torch.uint8)) and torch.equal(s, s_ref)
+    if not pure:
+        test_backward((rows, cols))

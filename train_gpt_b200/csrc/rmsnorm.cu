@@ -5,9 +5,9 @@
 // kernels.py:104-118 for the backward, fp8.py:39-47 + :66 for the quantiser that consumes
 // the norm's bf16 output.
 //
-// Layout: a row is split over WPR warps; each warp owns NCHUNK chunks of 256 columns and
-// each lane 8 consecutive columns (one 128-bit load) per chunk, so a half-warp owns
-// exactly one 128-column quantisation tile.  The whole row stays in registers between the
+// Layout: a row is split over WPR warps (norm_geom, bwd_geom); each warp owns
+// NCHUNK chunks of 256 columns and each lane 8 consecutive columns (one 128-bit load) per chunk, so a half-warp owns
+// exactly one 128-column quantisation tile.  The row stays on the SM (registers or shared memory) between the
 // sum-of-squares pass and the normalise/quantise pass: x is read from HBM once.
 #include <cstdlib>
 
@@ -37,34 +37,31 @@ __device__ __forceinline__ float tree_sum(float (&v)[N]) {
   return v[0];
 }
 
+// Sum over the lanes of a warp and, where a row has several, over its WPR warps in order.  `red` holds one float per warp of
+// the block and alternates between two buffers from row to row: a warp writes one only after its group's barrier of the row
+// before, which every warp of the group reaches after reading the other.
 template <int WPR>
-__device__ __forceinline__ float row_sum(float v, float* s_red, int warp, int lane) {
+__device__ __forceinline__ float row_sum(float v, float* red, int warp, int lane) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   if constexpr (WPR > 1) {
-    // s_red: [kNormWarps] floats; the caller separates uses with __syncthreads()
-    if (lane == 0) s_red[warp] = v;
-    __syncthreads();
+    if (lane == 0) red[warp] = v;
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / WPR), "n"(WPR * 32) : "memory");   // this row's warps only
     const int g0 = (warp / WPR) * WPR;
-    v = s_red[g0];
+    v = red[g0];
 #pragma unroll
-    for (int i = 1; i < WPR; ++i) v += s_red[g0 + i];
+    for (int i = 1; i < WPR; ++i) v += red[g0 + i];
   }
   return v;
 }
 
-// Two blocks per SM when the fused kernel holds a 2048-wide row per warp (three would spill),
-// three otherwise.
-template <int NCHUNK, int WPR, bool QUANT, bool PURE>
-__global__ void __launch_bounds__(kNormWarps * 32, (QUANT && NCHUNK >= 8) ? 2 : 3)
+// Plain norm of rows that one warp holds in registers.
+template <int NCHUNK, bool PURE>
+__global__ void __launch_bounds__(kNormWarps * 32, 3)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
-                   float eps, uint8_t* __restrict__ q, float* __restrict__ scales,
-                   __nv_bfloat16* __restrict__ y, float* __restrict__ rnorm_out, int64_t rows,
-                   int cols) {
-  __shared__ float s_red[2][kNormWarps];
-  constexpr int RPB = kNormWarps / WPR;  // rows per block per iteration
+                   float eps, __nv_bfloat16* __restrict__ y, float* __restrict__ rnorm_out, int64_t rows, int cols) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int col_base = (warp % WPR) * NCHUNK * 256 + lane * 8;
+  const int col_base = lane * 8;
 
   // gamma lives in shared memory, already widened to float (one conversion per block
   // instead of one per row), not in registers, so that more blocks fit on an SM
@@ -76,38 +73,27 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   }
   __syncthreads();
 
-  int it = 0;
-  for (int64_t row_base = int64_t(blockIdx.x) * RPB; row_base < rows;
-       row_base += int64_t(gridDim.x) * RPB, ++it) {
-    const int64_t row = row_base + warp / WPR;
-    const bool row_ok = row < rows;
+  for (int64_t row = int64_t(blockIdx.x) * kNormWarps + warp; row < rows; row += int64_t(gridDim.x) * kNormWarps) {
     uint4 w[NCHUNK];
 #pragma unroll
     for (int c = 0; c < NCHUNK; ++c) {
       const int col = col_base + c * 256;
-      w[c] = (row_ok && col < cols) ? ld_nc_v4(x + row * cols + col) : make_uint4(0, 0, 0, 0);
+      w[c] = col < cols ? ld_nc_v4(x + row * cols + col) : make_uint4(0, 0, 0, 0);
     }
     float part[NCHUNK];
 #pragma unroll
     for (int c = 0; c < NCHUNK; ++c) part[c] = sumsq8(w[c]);
-    const float ss = row_sum<WPR>(tree_sum(part), s_red[it & 1], warp, lane);
-    const float var = __fdiv_rn(ss, float(cols));
-    const float rn = __frsqrt_rn(var + eps);
-    if (row_ok && rnorm_out != nullptr && lane == 0 && (warp % WPR) == 0) rnorm_out[row] = rn;
+    const float ss = row_sum<1>(tree_sum(part), nullptr, warp, lane);
+    const float rn = __frsqrt_rn(__fdiv_rn(ss, float(cols)) + eps);
+    if (rnorm_out != nullptr && lane == 0) rnorm_out[row] = rn;
     const float rn_b = __bfloat162float(__float2bfloat16_rn(rn));  // kernels.py:32 `.astype(x.dtype)`
-
-    // pass 2a: normalise, round to bf16 (the value the reference's norm returns), per-tile amax
     const float2 rn2 = PURE ? make_float2(rn_b, rn_b) : make_float2(rn, rn);
-    uint32_t amax_bits[NCHUNK];
 #pragma unroll
     for (int c = 0; c < NCHUNK; ++c) {
       const int col = col_base + c * 256;
+      if (col >= cols) continue;
       const uint32_t xi[4] = {w[c].x, w[c].y, w[c].z, w[c].w};
-      float4 g0 = make_float4(0.f, 0.f, 0.f, 0.f), g1 = g0;
-      if (col < cols) {
-        g0 = s_gamma[col >> 2];
-        g1 = s_gamma[(col >> 2) + 1];
-      }
+      const float4 g0 = s_gamma[col >> 2], g1 = s_gamma[(col >> 2) + 1];
       const float2 gf[4] = {make_float2(g0.x, g0.y), make_float2(g0.z, g0.w), make_float2(g1.x, g1.y), make_float2(g1.z, g1.w)};
       uint4 yo;
       uint32_t* yp = &yo.x;
@@ -118,41 +104,22 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
         t = __fmul2_rn(t, gf[j]);
         yp[j] = pack_bf16x2(t.x, t.y);
       }
-      if (y != nullptr && row_ok && col < cols) *reinterpret_cast<uint4*>(y + row * cols + col) = yo;
-      w[c] = yo;  // the row registers now hold the normalised bf16 values
-      if constexpr (QUANT) amax_bits[c] = absmax8(yo);
-    }
-    if constexpr (QUANT) {
-      // pass 2b: one exchange brings lane j of each half the amax of chunk j % NCHUNK; that lane
-      // computes the tile's scale and reciprocal, and shuffles hand them to the lanes that need them
-      float s[NCHUNK], r[NCHUNK], s_mine;
-      bool fin;
-      tile_scales_own<NCHUNK>(exchange_tile_amax<NCHUNK>(amax_bits), s, r, s_mine, fin);
-      {
-        const int j = lane & 15;                       // lane j of a half computed chunk j % NCHUNK
-        const int col = col_base - (lane & 15) * 8 + j * 256;   // = first column of that chunk's tile for this half
-        if (j < NCHUNK && row_ok && col < cols) scales[row * (cols / kTile) + col / kTile] = s_mine;
-      }
-      // pass 2c: divide and store
-#pragma unroll
-      for (int c = 0; c < NCHUNK; ++c) {
-        const int col = col_base + c * 256;
-        if (row_ok && col < cols)
-          *reinterpret_cast<uint2*>(q + row * cols + col) = fin ? quantize8_sr(w[c], s[c], r[c]) : quantize8(w[c], s[c]);
-      }
+      *reinterpret_cast<uint4*>(y + row * cols + col) = yo;
     }
   }
 }
 
 // ---------------------------------------------------------------------------------------
-// Fused norm + quantise for rows that one warp can hold (cols <= 2048), staged through shared
-// memory.  The register-resident kernel above needs ~120 registers at 2048 columns, so only
+// Norm (+ quantise) staged through shared memory: fused forms, and every form of rows wider than 2048 columns.  A
+// register-resident kernel needs ~120 registers at 2048 columns per warp, so only
 // 16 warps fit on an SM and every warp idles while its next row's loads are in flight.  Here
-// each warp owns two row-sized slots of shared memory: cp.async fetches row i+1 into one
-// slot while the warp makes its three passes (sum of squares; normalise + amax, writing the
-// bf16 result back in place; divide + store) over row i in the other.  A lane only ever
-// touches the 16-byte pieces it fetched itself, so cp.async.wait_group is the only
-// synchronisation; nothing spins.  Same arithmetic, same results as rmsnorm_fwd_kernel.
+// each warp owns two slots of shared memory for its part of a row: cp.async fetches row i+1 into one
+// slot while the warp makes its passes (sum of squares; normalise + amax; divide + store) over row i in the other.  A lane
+// only ever touches the 16-byte pieces it fetched itself, so cp.async.wait_group is the only
+// synchronisation within a warp; the warps of a wide row meet once, at the sum.
+// Wide rows, register-resident -> staged, microseconds (DRAM floor): 3001 x 4096 plain 12.2 -> 9.0 (7.5), quantised 14.6 -> 10.9
+// (5.7); 4096 x 8192 29.7 -> 22.3 (20.5), 32.3 -> 24.6 (15.5); 16384 x 8192 quantised 110.7 -> 84.7 (62).  Eight warps per row of
+// four chunks, or gamma in registers and a third slot, were no better (3001 x 4096 10.5, 4096 x 8192 25.4 and 29.7).
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -166,25 +133,27 @@ __device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-constexpr int kStagedBlocksPerSm = 3;
-constexpr int kGroup = 8;   // chunks normalised, scaled and quantised together (their bf16 values stay in registers)
+constexpr int staged_blocks(int wpr) { return wpr == 1 ? 3 : 2; }      // per SM: 72 KB each up to 2048 columns, 80-96 beyond
+constexpr int pow2_at_least(int n) { return n <= 1 ? 1 : 2 * pow2_at_least((n + 1) / 2); }
 
 // ADD: the row that is normalised is bf16(x + res) -- the residual add of model.py:68 / :72 folded into
 // the norm that follows it -- and is also written to `sum_out` (the new residual stream); `res` rows
 // are staged beside the x rows and the sum replaces the x row in shared memory before the first pass.
-// q may be NULL (ADD only: the final norm has no quantised consumer), then only y is produced.
-template <int NCHUNK, bool PURE, bool FULL, bool ADD = false>
-__global__ void __launch_bounds__(kNormWarps * 32, kStagedBlocksPerSm)
+// q may be NULL: then only y is produced (the plain norm, or with ADD the final norm, which has no quantised consumer).
+template <int NCHUNK, bool PURE, bool FULL, bool ADD = false, int WPR = 1>
+__global__ void __launch_bounds__(kNormWarps * 32, staged_blocks(WPR))
 rmsnorm_quant_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
                             float eps, uint8_t* __restrict__ q, float* __restrict__ scales,
                             __nv_bfloat16* __restrict__ y, float* __restrict__ rnorm_out, int64_t rows,
                             int cols, const __nv_bfloat16* __restrict__ res = nullptr,
                             __nv_bfloat16* __restrict__ sum_out = nullptr) {
+  constexpr int RPB = kNormWarps / WPR;  // rows in work per block
+  __shared__ float s_red[2][kNormWarps];
   constexpr int kRowBytes = NCHUNK * 512;
   constexpr int kSlotBytes = ADD ? 2 * kRowBytes : kRowBytes;     // x row (then: the sum), res row
   extern __shared__ float4 s_gamma[];   // [cols] floats, then [warps][2][slot] bf16
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int col_base = lane * 8;
+  const int col_base = (warp % WPR) * (NCHUNK * 256) + lane * 8;
   const uint32_t slot0 = uint32_t(__cvta_generic_to_shared(s_gamma)) + uint32_t(cols) * 4u +
                          uint32_t(warp) * 2u * kSlotBytes + uint32_t(lane) * 16u;
 
@@ -198,8 +167,8 @@ rmsnorm_quant_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bflo
   }
   __syncthreads();
 
-  const int64_t stride = int64_t(gridDim.x) * kNormWarps;
-  int64_t row = int64_t(blockIdx.x) * kNormWarps + warp;
+  const int64_t stride = int64_t(gridDim.x) * RPB;
+  int64_t row = int64_t(blockIdx.x) * RPB + warp / WPR;
   auto prefetch = [&](int64_t r, int slot) {
     if (r < rows) {
 #pragma unroll
@@ -244,66 +213,61 @@ rmsnorm_quant_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bflo
     float part[NCHUNK];
 #pragma unroll
     for (int c = 0; c < NCHUNK; ++c) part[c] = (FULL || col_base + c * 256 < cols) ? sumsq8(lds128(base + c * 512)) : 0.f;
-    float ss = tree_sum(part);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float ss = row_sum<WPR>(tree_sum(part), s_red[it & 1], warp, lane);
     const float var = __fdiv_rn(ss, float(cols));
     const float rn = __frsqrt_rn(var + eps);
-    if (rnorm_out != nullptr && lane == 0) rnorm_out[row] = rn;
+    if (rnorm_out != nullptr && lane == 0 && warp % WPR == 0) rnorm_out[row] = rn;
     const float rn_b = __bfloat162float(__float2bfloat16_rn(rn));  // kernels.py:32 `.astype(x.dtype)`
 
-    // pass 2, in groups of G chunks whose normalised values stay in registers: normalise, round
-    // to bf16 (the value the reference's norm returns), per-tile amax; one exchange brings lane j
-    // of each half the amax of the group's chunk j % G, that lane computes the tile's scale and
+    // pass 2: normalise, round to bf16 (the value the reference's norm returns), per-tile amax; one exchange brings lane j
+    // of each half the amax of chunk j % G, that lane computes the tile's scale and
     // reciprocal, shuffles hand them to the lanes that need them; divide and store.
     const float2 rn2 = PURE ? make_float2(rn_b, rn_b) : make_float2(rn, rn);
-    constexpr int G = NCHUNK < kGroup ? NCHUNK : kGroup;
+    constexpr int G = pow2_at_least(NCHUNK);     // (the exchange wants a power of two; chunks past NCHUNK are constant zeros)
+    uint4 yo[NCHUNK];
+    uint32_t amax_bits[G];
 #pragma unroll
-    for (int g = 0; g < NCHUNK / G; ++g) {
-      uint4 yo[G];
-      uint32_t amax_bits[G];
+    for (int u = NCHUNK; u < G; ++u) amax_bits[u] = 0u;
 #pragma unroll
-      for (int u = 0; u < G; ++u) {
-        const int c = g * G + u;
-        const int col = col_base + c * 256;
-        amax_bits[u] = 0u;
-        yo[u] = make_uint4(0u, 0u, 0u, 0u);
-        if (FULL || col < cols) {
-          const uint4 xv = lds128(base + c * 512);
-          const uint32_t xi[4] = {xv.x, xv.y, xv.z, xv.w};
-          const float4 g0 = s_gamma[col >> 3], g1 = s_gamma[pieces + (col >> 3)];
-          const float2 gf[4] = {make_float2(g0.x, g0.y), make_float2(g0.z, g0.w), make_float2(g1.x, g1.y), make_float2(g1.z, g1.w)};
-          uint32_t* yp = &yo[u].x;
+    for (int c = 0; c < NCHUNK; ++c) {
+      const int col = col_base + c * 256;
+      amax_bits[c] = 0u;
+      yo[c] = make_uint4(0u, 0u, 0u, 0u);
+      if (FULL || col < cols) {
+        const uint4 xv = lds128(base + c * 512);
+        const uint32_t xi[4] = {xv.x, xv.y, xv.z, xv.w};
+        const float4 g0 = s_gamma[col >> 3], g1 = s_gamma[pieces + (col >> 3)];
+        const float2 gf[4] = {make_float2(g0.x, g0.y), make_float2(g0.z, g0.w), make_float2(g1.x, g1.y), make_float2(g1.z, g1.w)};
+        uint32_t* yp = &yo[c].x;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float2 t = __fmul2_rn(bf16x2_unpack(xi[j]), rn2);
-            if (PURE) t = bf16x2_unpack(pack_bf16x2(t.x, t.y));   // kernels.py:32 rounds before the gamma multiply
-            t = __fmul2_rn(t, gf[j]);
-            yp[j] = pack_bf16x2(t.x, t.y);
-          }
-          if (y != nullptr) *reinterpret_cast<uint4*>(y + row * cols + col) = yo[u];
-          amax_bits[u] = absmax8_h(yo[u]);
+        for (int j = 0; j < 4; ++j) {
+          float2 t = __fmul2_rn(bf16x2_unpack(xi[j]), rn2);
+          if (PURE) t = bf16x2_unpack(pack_bf16x2(t.x, t.y));   // kernels.py:32 rounds before the gamma multiply
+          t = __fmul2_rn(t, gf[j]);
+          yp[j] = pack_bf16x2(t.x, t.y);
         }
+        if (y != nullptr) *reinterpret_cast<uint4*>(y + row * cols + col) = yo[c];
+        amax_bits[c] = absmax8_h(yo[c]);
       }
-      float s[G], r[G], s_mine;
-      bool fin;
-      tile_scales_own<G>(exchange_tile_amax<G>(amax_bits), s, r, s_mine, fin);
-      {
-        const int j = lane & 15;
-        const int col = (g * G + j) * 256 + (lane & 16) * 8;     // first column of the tile this lane computed
-        if (j < G && (FULL || col < cols) && (!ADD || q != nullptr)) scales[row * (cols / kTile) + col / kTile] = s_mine;
-      }
-      if (ADD && q == nullptr) continue;
-      uint8_t* qp = q + row * cols + col_base + g * G * 256;
-      if (fin) {   // one branch per group: a NaN or Inf in any of the warp's tiles is the rare case
+    }
+    if (q == nullptr) continue;
+    float s[G], r[G], s_mine;
+    bool fin;
+    tile_scales_own<G>(exchange_tile_amax<G>(amax_bits), s, r, s_mine, fin);
+    {
+      const int j = lane & 15;
+      const int col = col_base - lane * 8 + j * 256 + (lane & 16) * 8;     // first column of the tile this lane computed
+      if (j < NCHUNK && (FULL || col < cols)) scales[row * (cols / kTile) + col / kTile] = s_mine;
+    }
+    uint8_t* qp = q + row * cols + col_base;
+    if (fin) {   // one branch: a NaN or Inf in any of the warp's tiles is the rare case
 #pragma unroll
-        for (int u = 0; u < G; ++u)
-          if (FULL || col_base + (g * G + u) * 256 < cols) *reinterpret_cast<uint2*>(qp + u * 256) = quantize8_sr(yo[u], s[u], r[u]);
-      } else {
+      for (int c = 0; c < NCHUNK; ++c)
+        if (FULL || col_base + c * 256 < cols) *reinterpret_cast<uint2*>(qp + c * 256) = quantize8_sr(yo[c], s[c], r[c]);
+    } else {
 #pragma unroll
-        for (int u = 0; u < G; ++u)
-          if (FULL || col_base + (g * G + u) * 256 < cols) *reinterpret_cast<uint2*>(qp + u * 256) = quantize8(yo[u], s[u]);
-      }
+      for (int c = 0; c < NCHUNK; ++c)
+        if (FULL || col_base + c * 256 < cols) *reinterpret_cast<uint2*>(qp + c * 256) = quantize8(yo[c], s[c]);
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -315,136 +279,30 @@ rmsnorm_quant_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bflo
 // dgamma = sum_rows g*normed, accumulated per lane in registers over all rows the block
 // visits, combined across the block's warps in shared memory, written as one float32 row
 // of `partial` per block and reduced over blocks (in block order) by a second kernel.
-// ---------------------------------------------------------------------------------------
-template <int NCHUNK, int WPR>
-__global__ void __launch_bounds__(kNormWarps * 32)
-rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
-                   const __nv_bfloat16* __restrict__ g, float eps, __nv_bfloat16* __restrict__ dx,
-                   float* __restrict__ partial, int64_t rows, int cols) {
-  extern __shared__ float s_dyn[];  // [cols] column sums of this block
-  __shared__ float s_red[4][kNormWarps];
-  constexpr int RPB = kNormWarps / WPR;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int col_base = (warp % WPR) * NCHUNK * 256 + lane * 8;
-  const float inv_d = __fdiv_rn(1.0f, float(cols));
-
-  float acc[NCHUNK][8];
-#pragma unroll
-  for (int c = 0; c < NCHUNK; ++c)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[c][j] = 0.f;
-
-  int it = 0;
-  for (int64_t row_base = int64_t(blockIdx.x) * RPB; row_base < rows;
-       row_base += int64_t(gridDim.x) * RPB, ++it) {
-    const int64_t row = row_base + warp / WPR;
-    const bool row_ok = row < rows;
-    uint4 w[NCHUNK], gv[NCHUNK];
-#pragma unroll
-    for (int c = 0; c < NCHUNK; ++c) {
-      const int col = col_base + c * 256;
-      const bool ok = row_ok && col < cols;
-      w[c] = ok ? ld_nc_v4(x + row * cols + col) : make_uint4(0, 0, 0, 0);
-      gv[c] = ok ? ld_nc_v4(g + row * cols + col) : make_uint4(0, 0, 0, 0);
-    }
-    float part[NCHUNK];
-#pragma unroll
-    for (int c = 0; c < NCHUNK; ++c) part[c] = sumsq8(w[c]);
-    const float ss = row_sum<WPR>(tree_sum(part), s_red[(it & 1) * 2], warp, lane);
-    const float rn = __frsqrt_rn(__fdiv_rn(ss, float(cols)) + eps);
-
-    // gs*normed summed over the row; dgamma accumulation in the same sweep
-    float dpart[NCHUNK];
-#pragma unroll
-    for (int c = 0; c < NCHUNK; ++c) {
-      float dsum = 0.f;
-      const int col = col_base + c * 256;
-      const uint4 gm = (col < cols) ? *reinterpret_cast<const uint4*>(gamma + col) : make_uint4(0, 0, 0, 0);
-      const uint32_t xi[4] = {w[c].x, w[c].y, w[c].z, w[c].w};
-      const uint32_t gi[4] = {gv[c].x, gv[c].y, gv[c].z, gv[c].w};
-      const uint32_t mi[4] = {gm.x, gm.y, gm.z, gm.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float n0 = __fmul_rn(bf16lo(xi[j]), rn), n1 = __fmul_rn(bf16hi(xi[j]), rn);
-        const float g0 = bf16lo(gi[j]), g1 = bf16hi(gi[j]);
-        acc[c][2 * j] = fmaf(g0, n0, acc[c][2 * j]);
-        acc[c][2 * j + 1] = fmaf(g1, n1, acc[c][2 * j + 1]);
-        dsum = fmaf(__fmul_rn(g0, bf16lo(mi[j])), n0, dsum);
-        dsum = fmaf(__fmul_rn(g1, bf16hi(mi[j])), n1, dsum);
-      }
-      dpart[c] = dsum;
-    }
-    const float dsum = row_sum<WPR>(tree_sum(dpart), s_red[(it & 1) * 2 + 1], warp, lane);
-    const float dot = __fmul_rn(dsum, inv_d);
-
-#pragma unroll
-    for (int c = 0; c < NCHUNK; ++c) {
-      const int col = col_base + c * 256;
-      if (!(row_ok && col < cols)) continue;
-      const uint4 gm = *reinterpret_cast<const uint4*>(gamma + col);
-      const uint32_t xi[4] = {w[c].x, w[c].y, w[c].z, w[c].w};
-      const uint32_t gi[4] = {gv[c].x, gv[c].y, gv[c].z, gv[c].w};
-      const uint32_t mi[4] = {gm.x, gm.y, gm.z, gm.w};
-      uint4 o;
-      uint32_t* op = &o.x;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float n0 = __fmul_rn(bf16lo(xi[j]), rn), n1 = __fmul_rn(bf16hi(xi[j]), rn);
-        const float gs0 = __fmul_rn(bf16lo(gi[j]), bf16lo(mi[j]));
-        const float gs1 = __fmul_rn(bf16hi(gi[j]), bf16hi(mi[j]));
-        // rnorm * (gs - normed*dot), the subtraction fused as kernels.py:114 allows XLA to
-        const float d0 = __fmul_rn(rn, fmaf(-n0, dot, gs0));
-        const float d1 = __fmul_rn(rn, fmaf(-n1, dot, gs1));
-        op[j] = pack_bf16x2(d0, d1);
-      }
-      *reinterpret_cast<uint4*>(dx + row * cols + col) = o;
-    }
-  }
-
-  // combine the block's warps in a fixed order, then publish the block's row of partials
-  for (int i = threadIdx.x; i < cols; i += blockDim.x) s_dyn[i] = 0.f;
-  __syncthreads();
-  for (int turn = 0; turn < RPB; ++turn) {
-    if (warp / WPR == turn) {
-#pragma unroll
-      for (int c = 0; c < NCHUNK; ++c) {
-        const int col = col_base + c * 256;
-        if (col < cols) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) s_dyn[col + j] += acc[c][j];
-        }
-      }
-    }
-    __syncthreads();
-  }
-  for (int i = threadIdx.x; i < cols; i += blockDim.x) partial[int64_t(blockIdx.x) * cols + i] = s_dyn[i];
-}
-
-// ---------------------------------------------------------------------------------------
-// Backward for rows that one warp can hold (cols <= 2048), staged through shared memory.
-// The register-resident kernel above keeps x, g and 8 column sums per 16-byte piece live at
-// once (246 registers at 2048 columns: one block of eight warps per SM, each idle while its
-// next row is in flight; it reached 55 % of the copy bandwidth).  Here each warp owns SLOTS
-// pairs of row-sized shared-memory slots and cp.async keeps SLOTS - 1 rows of x and g in flight
-// while one is processed:
-// x goes to registers once, g is read from shared memory in the column-sum pass and again in
+//
+// Staged through shared memory: register-resident it kept x, g and 8 column sums per 16-byte piece live at
+// once (246 registers at 2048 columns per warp: one block of eight warps per SM, each idle while its
+// next row is in flight; 55 % of the copy bandwidth).  Here each warp owns SLOTS
+// pairs of slots for its part of a row and cp.async keeps SLOTS - 1 rows of x and g in flight
+// while one is processed: x goes to registers once, g is read from shared memory in the column-sum pass and again in
 // the dx pass, gamma sits in shared memory widened to float.  Every lane reads only the
-// 16-byte pieces it fetched itself, so cp.async.wait_group is the only synchronisation.
-// The arithmetic per row is the same sequence as in rmsnorm_bwd_kernel: dx comes out
-// bit-identical; dgamma sums the same products in another (still fixed) order.
+// 16-byte pieces it fetched itself, so cp.async.wait_group is the only synchronisation within a warp; the warps of a wide row
+// meet at its two sums.  Wide rows, register-resident -> staged, microseconds (DRAM floor): 3001 x 4096 33.1 -> 19.6 (11.2),
+// 16384 x 8192 232.6 -> 135.9 (122.8), 4096 x 2304 35.0 -> 17.0 (8.6), 8192 x 6144 111.8 -> 56.8 (46).
 // ---------------------------------------------------------------------------------------
 // ADD: dx = bf16(addend + the norm's input gradient) -- the gradient fan-in at a residual junction (the
 // skip path's gradient plus the branch's) folded into the kernel, one rounding instead of two.
-template <int NCHUNK, int WARPS, int SLOTS, bool FULL, bool ADD = false>
+template <int NCHUNK, int WARPS, int SLOTS, bool FULL, bool ADD = false, int WPR = 1>
 __global__ void __launch_bounds__(WARPS * 32, 1)
 rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
                           const __nv_bfloat16* __restrict__ g, float eps, __nv_bfloat16* __restrict__ dx,
                           float* __restrict__ partial, int64_t rows, int cols,
                           const __nv_bfloat16* __restrict__ addend = nullptr) {
-  constexpr int kRowBytes = NCHUNK * 512;
+  constexpr int kRowBytes = NCHUNK * 512, RPB = WARPS / WPR;      // a warp's part of a row; rows in work per block
+  __shared__ float s_red[2][2][WARPS];
   extern __shared__ float4 s_gamma[];   // [cols] floats in two planes, then [warps][SLOTS][x row | g row] bf16
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int col_base = lane * 8;
+  const int col_base = (warp % WPR) * (NCHUNK * 256) + lane * 8;
   const uint32_t stage0 = uint32_t(__cvta_generic_to_shared(s_gamma)) + uint32_t(cols) * 4u;
   const uint32_t slot0 = stage0 + uint32_t(warp) * uint32_t(SLOTS * 2 * kRowBytes) + uint32_t(lane) * 16u;
   const float inv_d = __fdiv_rn(1.0f, float(cols));
@@ -463,8 +321,8 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[c][j] = 0.f;
 
-  const int64_t stride = int64_t(gridDim.x) * WARPS;
-  int64_t row = int64_t(blockIdx.x) * WARPS + warp;
+  const int64_t stride = int64_t(gridDim.x) * RPB;
+  int64_t row = int64_t(blockIdx.x) * RPB + warp / WPR;
   auto prefetch = [&](int64_t r, int slot) {
     if (r < rows) {
       const uint32_t dst = slot0 + uint32_t(slot) * 2u * kRowBytes;
@@ -483,7 +341,7 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
 #pragma unroll
   for (int d = 0; d < SLOTS - 1; ++d) prefetch(row + d * stride, d);
   int slot = 0, slot_in = SLOTS - 1;
-  for (; row < rows; row += stride) {
+  for (int it = 0; row < rows; row += stride, ++it) {
     const uint32_t xs = slot0 + uint32_t(slot) * 2u * kRowBytes, gs = xs + kRowBytes;
     prefetch(row + (SLOTS - 1) * stride, slot_in);    // into the slot the previous iteration finished with
     asm volatile("cp.async.wait_group %0;" ::"n"(SLOTS - 1) : "memory");
@@ -497,9 +355,7 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
       w[c] = (FULL || col_base + c * 256 < cols) ? lds128(xs + c * 512) : make_uint4(0, 0, 0, 0);
       part[c] = sumsq8(w[c]);
     }
-    float ss = tree_sum(part);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float ss = row_sum<WPR>(tree_sum(part), s_red[it & 1][0], warp, lane);
     const float rn = __frsqrt_rn(__fdiv_rn(ss, float(cols)) + eps);
 
     // (ADD) the addend's pieces are fetched here, ahead of the pass that uses them, when the row is
@@ -536,9 +392,7 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
       }
       dpart[c] = dsum;
     }
-    float dsum = tree_sum(dpart);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
+    const float dsum = row_sum<WPR>(tree_sum(dpart), s_red[it & 1][1], warp, lane);
     const float dot = __fmul_rn(dsum, inv_d);
 
     // (no instruction: stops the compiler from keeping the 8 * NCHUNK normalised values of the pass
@@ -578,14 +432,15 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 
-  // combine the block's warps in warp order over the (now idle) staging area, then publish the
+  grid_trigger();          // the reduction's blocks may take the places of this kernel's as they leave
+  // combine the block's rows in order over the (now idle) staging area, then publish the
   // block's row of partial column sums
   __syncthreads();
   float* s_sum = reinterpret_cast<float*>(s_gamma) + cols;
   for (int i = threadIdx.x; i < cols; i += blockDim.x) s_sum[i] = 0.f;
   __syncthreads();
-  for (int turn = 0; turn < WARPS; ++turn) {
-    if (warp == turn) {
+  for (int turn = 0; turn < RPB; ++turn) {
+    if (warp / WPR == turn) {
 #pragma unroll
       for (int c = 0; c < NCHUNK; ++c) {
         const int col = col_base + c * 256;
@@ -603,36 +458,33 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
   for (int i = threadIdx.x; i < cols; i += blockDim.x) partial[int64_t(blockIdx.x) * cols + i] = s_sum[i];
 }
 
-// Column sums of the per-block partials.  A thread block owns 32 columns; its eight warps take the
-// partial rows b = warp, warp + 8, ... (four independent sums each, so a warp has four loads in
-// flight), and the eight results are added in warp order: the order of additions is fixed by
-// (n_blocks, cols) alone.  With one thread per column walking all rows the kernel was a chain of
-// ~n_blocks / 4 dependent L2 round trips on eight thread blocks: 13 us at 1024 columns.
-__global__ void __launch_bounds__(256)
+// Column sums of the per-block partials.  A thread block owns 32 columns; its 32 warps take the
+// partial rows b = warp, warp + 32, ..., and the 32 results are added by a fixed tree: the order of additions is fixed by
+// (n_blocks, cols) alone.  A warp has all of its (at most five) loads in flight at once: with eight warps the kernel was a
+// chain of five L2 round trips, 5.2 us at 2048 columns.
+__global__ void __launch_bounds__(1024)
 rmsnorm_dgamma_reduce_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dgamma,
                              int n_blocks, int cols) {
-  __shared__ float s_part[8][32];
+  __shared__ float s_part[32][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + lane;
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+  grid_wait();
+  float t = 0.f;
   if (col < cols) {
-    int b = warp;
-    for (; b + 24 < n_blocks; b += 32) {
-      s0 += partial[int64_t(b) * cols + col];
-      s1 += partial[int64_t(b + 8) * cols + col];
-      s2 += partial[int64_t(b + 16) * cols + col];
-      s3 += partial[int64_t(b + 24) * cols + col];
-    }
-    for (; b < n_blocks; b += 8) s0 += partial[int64_t(b) * cols + col];
-  }
-  s_part[warp][lane] = (s0 + s1) + (s2 + s3);
-  __syncthreads();
-  if (warp == 0 && col < cols) {
-    float t = s_part[0][lane];
+    for (int b = warp; b < n_blocks; b += 160) {
+      float v[5];
 #pragma unroll
-    for (int w = 1; w < 8; ++w) t += s_part[w][lane];
-    dgamma[col] = __float2bfloat16_rn(t);
+      for (int i = 0; i < 5; ++i) v[i] = b + 32 * i < n_blocks ? __ldcg(partial + int64_t(b + 32 * i) * cols + col) : 0.f;
+      t += ((v[0] + v[1]) + (v[2] + v[3])) + v[4];
+    }
   }
+  s_part[warp][lane] = t;
+  __syncthreads();
+  // warp w sums column w of the block over the 32 partial sums
+  t = s_part[lane][warp];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0 && blockIdx.x * 32 + warp < cols) dgamma[blockIdx.x * 32 + warp] = __float2bfloat16_rn(t);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -704,17 +556,23 @@ struct NormGeom {
   int nchunk, wpr;
 };
 
-// Smallest (NCHUNK, WPR) with WPR * NCHUNK * 256 >= cols; NCHUNK <= 8 keeps the row in
-// registers, WPR <= 4 keeps at least two rows per block.
+// Forward.  Rows of up to 2048 columns: one warp, 1, 2, 4 or 8 chunks.  Wider ones: two or four warps with 5 to 8 chunks each, as
+// many as the row needs (rounded up to eight, 2304 columns would be 2048 in one warp and 256 in the other).
 static bool norm_geom(int64_t cols, NormGeom* g) {
   if (cols <= 0 || cols > 8192) return false;
   const int chunks = int((cols + 255) / 256);
-  int wpr = 1;
-  while (chunks > wpr * 8) wpr *= 2;
-  int nchunk = 1;
-  while (nchunk * wpr < chunks) nchunk *= 2;
-  g->nchunk = nchunk;
-  g->wpr = wpr;
+  g->wpr = chunks <= 8 ? 1 : chunks <= 16 ? 2 : 4;
+  g->nchunk = g->wpr == 1 ? pow2_at_least(chunks) : (chunks + g->wpr - 1) / g->wpr;
+  return true;
+}
+// Backward.  Sixteen warps of 3 or 4 chunks where a row fits them evenly: more warps hide the row's two sums better than eight of
+// twice the width (32768 x 1296: 51.8 us against 58.4).  Rows of 7 and 8 chunks stay with one warp (74 us at 32768 x 2048
+// either way); above 6144 columns eight warps per row of four chunks spill (16384 x 8192 173 us), so four of 7 or 8.
+static bool bwd_geom(int64_t cols, NormGeom* g) {
+  if (cols <= 0 || cols > 8192) return false;
+  const int chunks = int((cols + 255) / 256);
+  g->wpr = chunks <= 4 ? 1 : chunks <= 6 ? 2 : chunks <= 8 ? 1 : chunks <= 16 ? 4 : chunks <= 24 ? 8 : 4;
+  g->nchunk = g->wpr == 1 ? pow2_at_least(chunks) : (chunks + g->wpr - 1) / g->wpr;
   return true;
 }
 
@@ -723,6 +581,58 @@ static int norm_blocks(int64_t rows, int wpr, int per_sm) {
   int64_t need = (rows + rpb - 1) / rpb;
   const int64_t cap = int64_t(sm_count()) * per_sm;
   return int(need < cap ? need : cap);
+}
+
+// Dynamic shared memory of `bytes` for `kern`, once per device.
+template <typename K>
+static int allow_smem(K kern, int bytes, std::atomic<bool> (&done)[64]) {
+  int dev = 0;
+  TG_CUDA_CHECK(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return TG_ERR_SHAPE;
+  if (!done[dev].load(std::memory_order_acquire)) {
+    TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    done[dev].store(true, std::memory_order_release);
+  }
+  return TG_OK;
+}
+
+struct NormFwd {
+  const __nv_bfloat16 *x, *gamma, *res;
+  float eps;
+  uint8_t* q;
+  float* scales;
+  __nv_bfloat16* y;
+  float* rnorm;
+  int64_t rows;
+  int cols;
+  __nv_bfloat16* sum_out;
+};
+
+template <int NC, bool PURE, bool FULL, bool ADD, int WPR>
+static int launch_staged(const NormFwd& a, cudaStream_t st) {
+  static std::atomic<bool> done[64];
+  auto kern = rmsnorm_quant_staged_kernel<NC, PURE, FULL, ADD, WPR>;
+  constexpr int slots = kNormWarps * 2 * NC * 512 * (ADD ? 2 : 1);
+  if (int rc = allow_smem(kern, WPR * NC * 1024 + slots, done)) return rc;
+  kern<<<norm_blocks(a.rows, WPR, staged_blocks(WPR)), kNormWarps * 32, size_t(a.cols) * 4 + slots, st>>>(
+      a.x, a.gamma, a.eps, a.q, a.scales, a.y, a.rnorm, a.rows, a.cols, a.res, a.sum_out);
+  TG_CUDA_CHECK(cudaGetLastError());
+  return TG_OK;
+}
+template <bool ADD>
+static int launch_staged(const NormGeom& g, bool pure, const NormFwd& a, cudaStream_t st) {
+  const bool full = a.cols == g.wpr * g.nchunk * 256;   // no ragged chunk: the column guards compile away
+#define TG_STAGED_CASE(NC, W)                                                                                  \
+  if (g.nchunk == NC && g.wpr == W)                                                                            \
+    return pure ? (full ? launch_staged<NC, true, true, ADD, W>(a, st) : launch_staged<NC, true, false, ADD, W>(a, st)) \
+                : (full ? launch_staged<NC, false, true, ADD, W>(a, st) : launch_staged<NC, false, false, ADD, W>(a, st));
+  TG_STAGED_CASE(1, 1) TG_STAGED_CASE(2, 1) TG_STAGED_CASE(4, 1) TG_STAGED_CASE(8, 1)
+  if constexpr (!ADD) {
+    TG_STAGED_CASE(5, 2) TG_STAGED_CASE(6, 2) TG_STAGED_CASE(7, 2) TG_STAGED_CASE(8, 2)
+    TG_STAGED_CASE(5, 4) TG_STAGED_CASE(6, 4) TG_STAGED_CASE(7, 4) TG_STAGED_CASE(8, 4)
+  }
+#undef TG_STAGED_CASE
+  return TG_ERR_SHAPE;
 }
 
 template <bool QUANT>
@@ -737,62 +647,63 @@ static int launch_fwd(const void* x, const void* gamma, float eps, void* q, floa
                                static_cast<__nv_bfloat16*>(y), rnorm, int(cols), g.nchunk, g.wpr));
     return TG_OK;
   }
-  if (QUANT && g.wpr == 1) {
-    const size_t smem = size_t(cols) * 4 + size_t(kNormWarps) * 2 * g.nchunk * 512;
-    const int blocks = norm_blocks(rows, 1, kStagedBlocksPerSm);
-    int dev = 0;
-    TG_CUDA_CHECK(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return TG_ERR_SHAPE;
-#define TG_STAGED_CASE(NC)                                                                       \
-  if (g.nchunk == NC) {                                                                          \
-    const bool full = cols == NC * 256;   /* no ragged chunk: the column guards compile away */ \
-    auto kern = mode == TG_NORM_PURE                                                             \
-                    ? (full ? rmsnorm_quant_staged_kernel<NC, true, true> : rmsnorm_quant_staged_kernel<NC, true, false>)   \
-                    : (full ? rmsnorm_quant_staged_kernel<NC, false, true> : rmsnorm_quant_staged_kernel<NC, false, false>); \
-    static bool attr_set[4][64] = {};                                                            \
-    if (!attr_set[(mode == TG_NORM_PURE) * 2 + full][dev]) {                                     \
-      TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
-                                         int(2048 * 4 + kNormWarps * 2 * NC * 512)));            \
-      attr_set[(mode == TG_NORM_PURE) * 2 + full][dev] = true;                                   \
-    }                                                                                            \
-    kern<<<blocks, kNormWarps * 32, smem, st>>>(                                                 \
-        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), eps,     \
-        static_cast<uint8_t*>(q), scales, static_cast<__nv_bfloat16*>(y), rnorm, rows,           \
-        int(cols), nullptr, nullptr);                                                            \
+  const NormFwd a = {static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), nullptr, eps, static_cast<uint8_t*>(q),
+                     scales, static_cast<__nv_bfloat16*>(y), rnorm, rows, int(cols), nullptr};
+  if (QUANT || g.wpr > 1) return launch_staged<false>(g, mode == TG_NORM_PURE, a, st);
+  const int blocks = norm_blocks(rows, 1, 16);
+#define TG_FWD_CASE(NC)                                                                                       \
+  if (g.nchunk == NC) {                                                                                       \
+    auto kern = mode == TG_NORM_PURE ? rmsnorm_fwd_kernel<NC, true> : rmsnorm_fwd_kernel<NC, false>;          \
+    kern<<<blocks, kNormWarps * 32, size_t(cols) * 4, st>>>(a.x, a.gamma, eps, a.y, rnorm, rows, int(cols)); \
   } else
-    TG_STAGED_CASE(1) TG_STAGED_CASE(2) TG_STAGED_CASE(4) TG_STAGED_CASE(8) { return TG_ERR_SHAPE; }
-#undef TG_STAGED_CASE
-    TG_CUDA_CHECK(cudaGetLastError());
-    return TG_OK;
-  }
-  const int blocks = norm_blocks(rows, g.wpr, 16);
-#define TG_FWD_CASE(NC, W)                                                                      \
-  if (g.nchunk == NC && g.wpr == W) {                                                           \
-    auto kern = mode == TG_NORM_PURE ? rmsnorm_fwd_kernel<NC, W, QUANT, true>                   \
-                                     : rmsnorm_fwd_kernel<NC, W, QUANT, false>;                 \
-    kern<<<blocks, kNormWarps * 32, size_t(cols) * 4, st>>>(                                    \
-        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), eps,    \
-        static_cast<uint8_t*>(q), scales, static_cast<__nv_bfloat16*>(y), rnorm, rows,          \
-        int(cols));                                                                             \
-  } else
-  TG_FWD_CASE(1, 1) TG_FWD_CASE(2, 1) TG_FWD_CASE(4, 1) TG_FWD_CASE(8, 1) TG_FWD_CASE(8, 2)
-  TG_FWD_CASE(8, 4) { return TG_ERR_SHAPE; }
+  TG_FWD_CASE(1) TG_FWD_CASE(2) TG_FWD_CASE(4) TG_FWD_CASE(8) { return TG_ERR_SHAPE; }
 #undef TG_FWD_CASE
   TG_CUDA_CHECK(cudaGetLastError());
   return TG_OK;
 }
 
-constexpr int kBwdBlocksPerSm = 2;
-
-// Rows one warp can hold run staged, one block per SM with 192 KB of row slots: 8 warps x 3 slots
-// at 2048 columns, 12 x 4 at 1024, 16 x 4 below; wider rows stay register-resident.
-static int bwd_staged_warps(const NormGeom& g) { return g.wpr != 1 ? 0 : g.nchunk >= 8 ? 8 : g.nchunk == 4 ? 12 : 16; }
+// One block per SM with up to 192 KB of slots.
+constexpr int bwd_warps(int nchunk, int wpr) { return nchunk > 4 ? 8 : nchunk == 4 && wpr == 1 ? 12 : 16; }
+constexpr int bwd_slots(int nchunk, int wpr) { return nchunk > 4 || (nchunk == 4 && wpr > 1) ? 3 : 4; }
 
 static int bwd_blocks(int64_t rows, const NormGeom& g) {
-  const int w = bwd_staged_warps(g);
-  if (w == 0) return norm_blocks(rows, g.wpr, kBwdBlocksPerSm);
-  const int64_t need = (rows + w - 1) / w, cap = sm_count();
+  const int rpb = bwd_warps(g.nchunk, g.wpr) / g.wpr;
+  const int64_t need = (rows + rpb - 1) / rpb, cap = sm_count();
   return int(need < cap ? need : cap);
+}
+
+struct NormBwd {
+  const __nv_bfloat16 *x, *gamma, *g, *addend;
+  float eps;
+  __nv_bfloat16* dx;
+  float* partial;
+  int64_t rows;
+  int cols, blocks;
+};
+template <int NC, bool FULL, bool ADD, int WPR>
+static int launch_bwd(const NormBwd& a, cudaStream_t st) {
+  static std::atomic<bool> done[64];
+  constexpr int warps = bwd_warps(NC, WPR), slots = bwd_slots(NC, WPR), stage = warps * slots * 2 * NC * 512;
+  static_assert(WPR * NC * 1024 + stage + 256 <= 227 * 1024, "row slots exceed shared memory");
+  auto kern = rmsnorm_bwd_staged_kernel<NC, warps, slots, FULL, ADD, WPR>;
+  if (int rc = allow_smem(kern, WPR * NC * 1024 + stage, done)) return rc;
+  kern<<<a.blocks, warps * 32, size_t(a.cols) * 4 + size_t(stage), st>>>(a.x, a.gamma, a.g, a.eps, a.dx, a.partial, a.rows, a.cols, a.addend);
+  TG_CUDA_CHECK(cudaGetLastError());
+  return TG_OK;
+}
+static int launch_bwd(const NormGeom& g, const NormBwd& a, cudaStream_t st) {
+  const bool full = a.cols == g.wpr * g.nchunk * 256, add = a.addend != nullptr;
+#define TG_BWD_CASE(NC, W)                                                                          \
+  if (g.nchunk == NC && g.wpr == W) {                                                               \
+    if constexpr (W <= 2) {                                                                         \
+      if (add) return full ? launch_bwd<NC, true, true, W>(a, st) : launch_bwd<NC, false, true, W>(a, st); \
+    }                                                                                               \
+    return full ? launch_bwd<NC, true, false, W>(a, st) : launch_bwd<NC, false, false, W>(a, st);   \
+  }
+  TG_BWD_CASE(1, 1) TG_BWD_CASE(2, 1) TG_BWD_CASE(4, 1) TG_BWD_CASE(8, 1) TG_BWD_CASE(3, 2)
+  TG_BWD_CASE(3, 4) TG_BWD_CASE(4, 4) TG_BWD_CASE(3, 8) TG_BWD_CASE(7, 4) TG_BWD_CASE(8, 4)
+#undef TG_BWD_CASE
+  return TG_ERR_SHAPE;
 }
 
 }  // namespace tg
@@ -832,38 +743,15 @@ extern "C" int tg_add_rmsnorm_quant_fwd(const void* x, const void* res, const vo
   NormGeom g;
   if (!norm_geom(cols, &g)) return cols > 8192 ? TG_ERR_TOO_LARGE : TG_ERR_SHAPE;
   if (g.wpr != 1) return TG_ERR_TOO_LARGE;      // rows one warp holds (cols <= 2048): the staged kernel
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const size_t smem = size_t(cols) * 4 + size_t(kNormWarps) * 2 * 2 * g.nchunk * 512;
-  const int blocks = norm_blocks(rows, 1, kStagedBlocksPerSm);
-  int dev = 0;
-  TG_CUDA_CHECK(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return TG_ERR_SHAPE;
-#define TG_ADD_CASE(NC)                                                                          \
-  if (g.nchunk == NC) {                                                                          \
-    const bool full = cols == NC * 256;                                                          \
-    auto kern = mode == TG_NORM_PURE                                                             \
-                    ? (full ? rmsnorm_quant_staged_kernel<NC, true, true, true> : rmsnorm_quant_staged_kernel<NC, true, false, true>)   \
-                    : (full ? rmsnorm_quant_staged_kernel<NC, false, true, true> : rmsnorm_quant_staged_kernel<NC, false, false, true>); \
-    static bool attr_set[4][64] = {};                                                            \
-    if (!attr_set[(mode == TG_NORM_PURE) * 2 + full][dev]) {                                     \
-      TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
-                                         int(2048 * 4 + kNormWarps * 2 * 2 * NC * 512)));        \
-      attr_set[(mode == TG_NORM_PURE) * 2 + full][dev] = true;                                   \
-    }                                                                                            \
-    kern<<<blocks, kNormWarps * 32, smem, st>>>(                                                 \
-        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), eps,     \
-        static_cast<uint8_t*>(q), scales, static_cast<__nv_bfloat16*>(y), rnorm, rows,           \
-        int(cols), static_cast<const __nv_bfloat16*>(res), static_cast<__nv_bfloat16*>(sum_out)); \
-  } else
-  TG_ADD_CASE(1) TG_ADD_CASE(2) TG_ADD_CASE(4) TG_ADD_CASE(8) { return TG_ERR_SHAPE; }
-#undef TG_ADD_CASE
-  TG_CUDA_CHECK(cudaGetLastError());
-  return TG_OK;
+  const NormFwd a = {static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(res), eps,
+                     static_cast<uint8_t*>(q), scales, static_cast<__nv_bfloat16*>(y), rnorm, rows, int(cols),
+                     static_cast<__nv_bfloat16*>(sum_out)};
+  return launch_staged<true>(g, mode == TG_NORM_PURE, a, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int64_t tg_rmsnorm_bwd_scratch_bytes(int64_t rows, int64_t cols) {
   NormGeom g;
-  if (rows <= 0 || !norm_geom(cols, &g)) return 0;
+  if (rows <= 0 || !bwd_geom(cols, &g)) return 0;
   return int64_t(bwd_blocks(rows, g)) * cols * int64_t(sizeof(float));
 }
 
@@ -871,8 +759,8 @@ static int rmsnorm_bwd_impl(const void* x, const void* gamma, const void* g, con
                             void* dgamma, void* scratch, int64_t rows, int64_t cols, void* stream) {
   if (rows < 0 || cols <= 0 || cols % 8 != 0) return TG_ERR_SHAPE;
   NormGeom geo;
-  if (!norm_geom(cols, &geo)) return cols > 8192 ? TG_ERR_TOO_LARGE : TG_ERR_SHAPE;
-  if (addend != nullptr && bwd_staged_warps(geo) == 0) return TG_ERR_TOO_LARGE;   // the fused add exists for rows one warp holds
+  if (!bwd_geom(cols, &geo)) return cols > 8192 ? TG_ERR_TOO_LARGE : TG_ERR_SHAPE;
+  if (addend != nullptr && cols > 2048) return TG_ERR_TOO_LARGE;   // the fused add exists for rows one warp holds
   if (!aligned16(x) || !aligned16(gamma) || !aligned16(g) || !aligned16(dx) || !aligned16(scratch) || !aligned16(addend))
     return TG_ERR_ALIGN;
   if (int rc = check_arch()) return rc;
@@ -882,54 +770,12 @@ static int rmsnorm_bwd_impl(const void* x, const void* gamma, const void* g, con
     return TG_OK;
   }
   const int blocks = bwd_blocks(rows, geo);
-  if (bwd_staged_warps(geo) != 0) {
-    int dev = 0;
-    TG_CUDA_CHECK(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return TG_ERR_SHAPE;
-    const bool full = cols == int64_t(geo.nchunk) * 256;   // no ragged chunk: the column guards compile away
-#define TG_BWD_STAGED_CASE(NC, WARPS, SLOTS)                                                      \
-  if (geo.nchunk == NC) {                                                                         \
-    const bool add = addend != nullptr;                                                           \
-    auto kern = add ? (full ? rmsnorm_bwd_staged_kernel<NC, WARPS, SLOTS, true, true>             \
-                            : rmsnorm_bwd_staged_kernel<NC, WARPS, SLOTS, false, true>)           \
-                    : (full ? rmsnorm_bwd_staged_kernel<NC, WARPS, SLOTS, true, false>            \
-                            : rmsnorm_bwd_staged_kernel<NC, WARPS, SLOTS, false, false>);         \
-    constexpr int kStage = WARPS * SLOTS * 2 * NC * 512;                                          \
-    static_assert(NC * 256 * 4 + kStage <= 227 * 1024, "row slots exceed shared memory");         \
-    static bool attr_set[4][64] = {};                                                             \
-    if (!attr_set[add * 2 + full][dev]) {                                                         \
-      TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
-                                         NC * 256 * 4 + kStage));                                 \
-      attr_set[add * 2 + full][dev] = true;                                                       \
-    }                                                                                             \
-    kern<<<blocks, WARPS * 32, size_t(cols) * 4 + size_t(kStage), st>>>(                          \
-        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma),           \
-        static_cast<const __nv_bfloat16*>(g), eps, static_cast<__nv_bfloat16*>(dx),               \
-        static_cast<float*>(scratch), rows, int(cols), static_cast<const __nv_bfloat16*>(addend)); \
-  } else
-    TG_BWD_STAGED_CASE(1, 16, 4) TG_BWD_STAGED_CASE(2, 16, 4) TG_BWD_STAGED_CASE(4, 12, 4) TG_BWD_STAGED_CASE(8, 8, 3) { return TG_ERR_SHAPE; }
-#undef TG_BWD_STAGED_CASE
-    TG_CUDA_CHECK(cudaGetLastError());
-    rmsnorm_dgamma_reduce_kernel<<<int((cols + 31) / 32), 256, 0, st>>>(
-        static_cast<const float*>(scratch), static_cast<__nv_bfloat16*>(dgamma), blocks, int(cols));
-    TG_CUDA_CHECK(cudaGetLastError());
-    return TG_OK;
-  }
-  const size_t smem = size_t(cols) * sizeof(float);
-#define TG_BWD_CASE(NC, W)                                                                      \
-  if (geo.nchunk == NC && geo.wpr == W) {                                                       \
-    rmsnorm_bwd_kernel<NC, W><<<blocks, kNormWarps * 32, smem, st>>>(                           \
-        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma),         \
-        static_cast<const __nv_bfloat16*>(g), eps, static_cast<__nv_bfloat16*>(dx),             \
-        static_cast<float*>(scratch), rows, int(cols));                                         \
-  } else
-  TG_BWD_CASE(1, 1) TG_BWD_CASE(2, 1) TG_BWD_CASE(4, 1) TG_BWD_CASE(8, 1) TG_BWD_CASE(8, 2)
-  TG_BWD_CASE(8, 4) { return TG_ERR_SHAPE; }
-#undef TG_BWD_CASE
-  TG_CUDA_CHECK(cudaGetLastError());
-  rmsnorm_dgamma_reduce_kernel<<<int((cols + 31) / 32), 256, 0, st>>>(
-      static_cast<const float*>(scratch), static_cast<__nv_bfloat16*>(dgamma), blocks, int(cols));
-  TG_CUDA_CHECK(cudaGetLastError());
+  const NormBwd a = {static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma), static_cast<const __nv_bfloat16*>(g),
+                     static_cast<const __nv_bfloat16*>(addend), eps, static_cast<__nv_bfloat16*>(dx), static_cast<float*>(scratch), rows,
+                     int(cols), blocks};
+  if (int rc = launch_bwd(geo, a, st)) return rc;
+  TG_CUDA_CHECK(launch_early(rmsnorm_dgamma_reduce_kernel, int((cols + 31) / 32), 1024, 0, st, static_cast<const float*>(scratch),
+                             static_cast<__nv_bfloat16*>(dgamma), blocks, int(cols)));
   return TG_OK;
 }
 
