@@ -315,11 +315,11 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
   }
   __syncthreads();
 
-  float acc[NCHUNK][8];
+  float2 acc[NCHUNK][4];
 #pragma unroll
   for (int c = 0; c < NCHUNK; ++c)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[c][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[c][j] = make_float2(0.f, 0.f);
 
   const int64_t stride = int64_t(gridDim.x) * RPB;
   int64_t row = int64_t(blockIdx.x) * RPB + warp / WPR;
@@ -357,6 +357,7 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
     }
     const float ss = row_sum<WPR>(tree_sum(part), s_red[it & 1][0], warp, lane);
     const float rn = __frsqrt_rn(__fdiv_rn(ss, float(cols)) + eps);
+    const float2 rn2 = make_float2(rn, rn);
 
     // (ADD) the addend's pieces are fetched here, ahead of the pass that uses them, when the row is
     // narrow enough for the registers; wider rows fetch them where they are used
@@ -377,23 +378,23 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
       if (FULL || col < cols) {
         const uint4 gv = lds128(gs + c * 512);
         const float4 m0 = s_gamma[col >> 3], m1 = s_gamma[pieces + (col >> 3)];
-        const float mf[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+        const float2 mf[4] = {make_float2(m0.x, m0.y), make_float2(m0.z, m0.w), make_float2(m1.x, m1.y), make_float2(m1.z, m1.w)};
         const uint32_t xi[4] = {w[c].x, w[c].y, w[c].z, w[c].w};
         const uint32_t gi[4] = {gv.x, gv.y, gv.z, gv.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float n0 = __fmul_rn(bf16lo(xi[j]), rn), n1 = __fmul_rn(bf16hi(xi[j]), rn);
-          const float g0 = bf16lo(gi[j]), g1 = bf16hi(gi[j]);
-          acc[c][2 * j] = fmaf(g0, n0, acc[c][2 * j]);
-          acc[c][2 * j + 1] = fmaf(g1, n1, acc[c][2 * j + 1]);
-          dsum = fmaf(__fmul_rn(g0, mf[2 * j]), n0, dsum);
-          dsum = fmaf(__fmul_rn(g1, mf[2 * j + 1]), n1, dsum);
+          const float2 n2 = __fmul2_rn(bf16x2_unpack(xi[j]), rn2), g2 = bf16x2_unpack(gi[j]);
+          acc[c][j] = __ffma2_rn(g2, n2, acc[c][j]);
+          const float2 gm = __fmul2_rn(g2, mf[j]);
+          dsum = fmaf(gm.x, n2.x, dsum);
+          dsum = fmaf(gm.y, n2.y, dsum);
         }
       }
       dpart[c] = dsum;
     }
     const float dsum = row_sum<WPR>(tree_sum(dpart), s_red[it & 1][1], warp, lane);
     const float dot = __fmul_rn(dsum, inv_d);
+    const float2 ndot2 = make_float2(-dot, -dot);
 
     // (no instruction: stops the compiler from keeping the 8 * NCHUNK normalised values of the pass
     // above alive for the pass below, which costs more registers than recomputing them)
@@ -405,7 +406,7 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
       if (!(FULL || col < cols)) continue;
       const uint4 gv = lds128(gs + c * 512);
       const float4 m0 = s_gamma[col >> 3], m1 = s_gamma[pieces + (col >> 3)];
-      const float mf[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+      const float2 mf[4] = {make_float2(m0.x, m0.y), make_float2(m0.z, m0.w), make_float2(m1.x, m1.y), make_float2(m1.z, m1.w)};
       const uint32_t xi[4] = {w[c].x, w[c].y, w[c].z, w[c].w};
       const uint32_t gi[4] = {gv.x, gv.y, gv.z, gv.w};
       uint4 av = make_uint4(0, 0, 0, 0);
@@ -415,17 +416,11 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
       uint32_t* op = &o.x;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float n0 = __fmul_rn(bf16lo(xi[j]), rn), n1 = __fmul_rn(bf16hi(xi[j]), rn);
-        const float gs0 = __fmul_rn(bf16lo(gi[j]), mf[2 * j]);
-        const float gs1 = __fmul_rn(bf16hi(gi[j]), mf[2 * j + 1]);
+        const float2 n2 = __fmul2_rn(bf16x2_unpack(xi[j]), rn2), gm = __fmul2_rn(bf16x2_unpack(gi[j]), mf[j]);
         // rnorm * (gs - normed*dot), the subtraction fused as kernels.py:114 allows XLA to
-        float d0 = __fmul_rn(rn, fmaf(-n0, dot, gs0));
-        float d1 = __fmul_rn(rn, fmaf(-n1, dot, gs1));
-        if constexpr (ADD) {
-          d0 = __fadd_rn(d0, bf16lo(ai[j]));
-          d1 = __fadd_rn(d1, bf16hi(ai[j]));
-        }
-        op[j] = pack_bf16x2(d0, d1);
+        float2 d = __fmul2_rn(rn2, __ffma2_rn(n2, ndot2, gm));
+        if constexpr (ADD) d = __fadd2_rn(d, bf16x2_unpack(ai[j]));
+        op[j] = pack_bf16x2(d.x, d.y);
       }
       *reinterpret_cast<uint4*>(dx + row * cols + col) = o;
     }
@@ -447,8 +442,8 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
         if (FULL || col < cols) {
           float4* dst = reinterpret_cast<float4*>(s_sum + col);
           float4 a = dst[0], b = dst[1];
-          a.x += acc[c][0]; a.y += acc[c][1]; a.z += acc[c][2]; a.w += acc[c][3];
-          b.x += acc[c][4]; b.y += acc[c][5]; b.z += acc[c][6]; b.w += acc[c][7];
+          a.x += acc[c][0].x; a.y += acc[c][0].y; a.z += acc[c][1].x; a.w += acc[c][1].y;
+          b.x += acc[c][2].x; b.y += acc[c][2].y; b.z += acc[c][3].x; b.w += acc[c][3].y;
           dst[0] = a; dst[1] = b;
         }
       }
