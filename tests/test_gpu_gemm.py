@@ -323,3 +323,27 @@ def test_linear_quantises_alike_in_one_launch_and_in_several(M, K, N, tile, mode
     assert torch.equal(y.detach(), ops.gemm_fwd(*ops.quantize_rowwise(a), *w, tile))
     assert torch.equal(at.grad, ops.gemm_dgrad(*ops.quantize_rowwise(g), *wd, tile))
     assert torch.equal(bt.grad, ops.gemm_wgrad(*ops.quantize_colwise(a), *gc, grad_tile=gt))
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 512, 4096), (3, 640, 4232), (16, 1024, 6144), (17, 768, 9600), (64, 2048, 8192), (100, 896, 5000),
+                                   (128, 640, 4224)])
+@pytest.mark.parametrize("tile", [(128, 1), (128, 128)])
+def test_few_tokens_against_a_wide_weight_in_clusters(M, K, N, tile):
+    """32 and more 128-row tiles of the weight: the blocks that share a tile add their sums up through their cluster's shared
+    memory, in one launch.  Against the oracle, at ragged token counts and weight widths, bf16 and float32 outputs."""
+    from train_gpt_b200 import fp8, ops
+    if tile == (128, 128) and N % 128:
+        pytest.skip("128x128 weight tiles need N % 128 == 0")
+    rng = np.random.default_rng(M + K + N)
+    a, b = normal_bf16(rng, (M, K), outlier_p=1e-3), normal_bf16(rng, (K, N), std=0.02)
+    a_q, a_s = ops.quantize_rowwise(to_torch_bf16(a))
+    if N % 16:
+        y = fp8.block_scaled_matmul(to_torch_bf16(a), to_torch_bf16(b))          # pads the weight's width itself
+    else:
+        w_q, w_s = fp8.quantize_weight(to_torch_bf16(b), tile)
+        y = ops.gemm_fwd(a_q, a_s, w_q, w_s, tile)
+        assert ops.last_gemm_kernel_launches == 1
+        y32 = ops.gemm_fwd(a_q, a_s, w_q, w_s, tile, out_dtype=torch.float32)
+        assert torch.equal(y32.to(torch.bfloat16), y)
+    _close(from_torch_bf16(y), fo.block_scaled_matmul(a, b, weight_tile=tile))
+    ops.check_status(device="cuda")

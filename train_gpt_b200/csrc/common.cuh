@@ -307,18 +307,25 @@ __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.la
 
 // A launch that may begin while the kernel before it on the stream is still running.
 template <typename... P, typename... A>
-static cudaError_t launch_early(void (*kern)(P...), int grid, int threads, int smem, cudaStream_t st, A... args) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+static cudaError_t launch_early_clusters(void (*kern)(P...), int cluster, int grid, int threads, int smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = unsigned(cluster);
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(grid));
   cfg.blockDim = dim3(unsigned(threads));
   cfg.dynamicSmemBytes = size_t(smem);
   cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+template <typename... P, typename... A>
+static cudaError_t launch_early(void (*kern)(P...), int grid, int threads, int smem, cudaStream_t st, A... args) {
+  return launch_early_clusters(kern, 1, grid, threads, smem, st, args...);
 }
 
 #endif  // __CUDACC__

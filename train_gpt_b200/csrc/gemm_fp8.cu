@@ -907,8 +907,10 @@ extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
         n_sb * a->sb_stride_n + nkb_all * a->sb_stride_kb > INT32_MAX)
       return TG_ERR_TOO_LARGE;
   }
-  if (skinny_takes(a) && a->workspace != nullptr && a->workspace_bytes >= skinny_workspace_bytes(a) && aligned16(a->workspace))
-    return skinny_run(a, st);
+  if (skinny_takes(a)) {
+    const int64_t need = skinny_workspace_bytes(a);
+    if (need == 0 || (a->workspace != nullptr && a->workspace_bytes >= need && aligned16(a->workspace))) return skinny_run(a, st);
+  }
   GemmParams p;
   p.sa = a->sa; p.sa_sm = a->sa_stride_m; p.sa_sk = a->sa_stride_kb;
   p.sb = a->sb; p.sb_sn = a->sb_stride_n; p.sb_sk = a->sb_stride_kb;

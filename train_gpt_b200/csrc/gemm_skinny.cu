@@ -12,6 +12,8 @@
 //   * scales arrive several blocks early (see the promotion warps);
 //   * a thread holds one weight row's sums over the tokens, so a slot is written 128 consecutive bytes per warp and token, and
 //     the reduce kernel, which adds a tile's slots in order, reads and writes along N: nothing is transposed;
+//   * where a tile is shared by at most four blocks (32 tiles and more), these form a thread-block cluster, the slots are
+//     their shared memories and the blocks add them up themselves: one launch, no workspace, the same order of additions;
 //   * programmatic dependent launch: barriers, tensor memory and an L2 prefetch of this block's first weight boxes (the L2 is
 //     coherent: a prefetch of bytes the kernel before is still writing is harmless) happen while the kernel before runs, and
 //     the reduce kernel is resident when the last sums arrive.
@@ -59,6 +61,10 @@ struct SkinnyParams {
   float* ws;                     // slots of [M][128] sums
   int M, N, nkb;
   int units, w_mn;               // units = tiles * nkb; w_mn: the weight is stored [K][N]
+  int share;                     // > 0: the `share` blocks of a tile are a cluster and finish the tile themselves
+  void* d;                       // (share > 0) the result
+  long long ldd;
+  int d_f32;
   unsigned* status;
 };
 
@@ -73,6 +79,18 @@ __device__ __forceinline__ void l2_prefetch_2d(const CUtensorMap* map, int x, in
 
 __device__ __forceinline__ void cp_async4(uint32_t dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// Barrier over all threads of the cluster (a cluster of one where the launch has none); it ends because every path above does.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// four floats at shared-memory address `addr` of the cluster's block `rank`
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr, int rank) {
+  float4 v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
+  return v;
 }
 
 // W_ROWS: a weight scale per row (128 x 1 tiles), else one per 128 rows
@@ -262,7 +280,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       }
       if (++buf == C::bufs) { buf = 0; bph ^= 1u; }
       if (ends) {
-        float* out = p.ws + size_t(int(blockIdx.x) + tile_now) * size_t(p.M) * BM + r;
+        // (share > 0: this is the block's last unit, every stage has been read; the pipeline's shared memory becomes the slot)
+        float* out = (p.share > 0 ? reinterpret_cast<float*>(smem) : p.ws + size_t(int(blockIdx.x) + tile_now) * size_t(p.M) * BM) + r;
         const bool row_ok = tile_now * BM + r < p.N;
 #pragma unroll
         for (int j = 0; j < C::cols; ++j)
@@ -272,6 +291,25 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+  }
+
+  if (p.share > 0) {
+    __syncwarp();
+    cluster_sync();                      // every block's slot is written
+    const int tile = int(blockIdx.x) / p.share, rank = int(blockIdx.x) - tile * p.share;
+    const uint32_t base = smem_u32(smem);
+    for (int i = rank * C::threads + int(threadIdx.x); i < p.M * (BM / 4); i += p.share * C::threads) {
+      const int m = i / (BM / 4), n = tile * BM + (i % (BM / 4)) * 4;
+      if (n >= p.N) continue;
+      float4 a = ld_cluster_f32x4(base + uint32_t(i) * 16u, 0);
+      for (int k = 1; k < p.share; ++k) {
+        const float4 b = ld_cluster_f32x4(base + uint32_t(i) * 16u, k);
+        a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+      }
+      if (p.d_f32) *reinterpret_cast<float4*>(static_cast<float*>(p.d) + m * p.ldd + n) = a;
+      else *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(p.d) + m * p.ldd + n) = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w));
+    }
+    cluster_sync();                      // nobody reads this block's shared memory any more
   }
 
   tc_fence_before();
@@ -313,8 +351,38 @@ bool skinny_takes(const tg_gemm_args* a) {
 }
 
 struct SkinnyPlan {
-  int tiles, nkb, units, grid;
+  int tiles, nkb, units, grid, share;
 };
+
+// Clusters of `size` blocks of this kernel that fit on the device together (an SM holds one block; GPCs are not multiples of
+// every size).
+static int clusters_that_fit(int size) {
+  static std::atomic<int> known[64][5];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = known[dev][size].load(std::memory_order_relaxed);
+  if (n == 0) {
+    using C = SkinnyCfg<16>;
+    auto kern = gemm_skinny_kernel<16, false>;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = unsigned(size);
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(size) * 64u);
+    cfg.blockDim = dim3(C::threads);
+    cfg.dynamicSmemBytes = C::smem_bytes;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem_bytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = -1;
+    }
+    known[dev][size].store(n, std::memory_order_relaxed);
+  }
+  return n < 0 ? 0 : n;
+}
 static SkinnyPlan plan(const tg_gemm_args* a) {
   SkinnyPlan p;
   p.tiles = int((a->N + BM - 1) / BM);
@@ -336,11 +404,21 @@ static SkinnyPlan plan(const tg_gemm_args* a) {
     const double c = cost(p.tiles * s, p.tiles * s, 5.0e6);
     if (c < best) { best = c; p.grid = p.tiles * s; }
   }
+  // A cluster per tile saves the second launch (about 2.5 us) and its slots' way through memory.
+  p.share = 0;
+  if (p.tiles >= 32) {
+    best += 2.5;
+    for (int s = 1; s <= 4 && s <= p.nkb && p.tiles * s <= most; ++s) {
+      const double c = cost(p.tiles * s, 0, 5.0e6);
+      if (c < best && (s == 1 || clusters_that_fit(s) >= p.tiles)) { best = c; p.grid = p.tiles * s; p.share = s; }
+    }
+  }
   return p;
 }
 
 int64_t skinny_workspace_bytes(const tg_gemm_args* a) {
   const SkinnyPlan p = plan(a);
+  if (p.share > 0) return 0;
   return int64_t(p.grid + p.tiles) * a->M * BM * int64_t(sizeof(float));
 }
 
@@ -360,7 +438,7 @@ static int launch(const tg_gemm_args* a, const SkinnyPlan& pl, SkinnyParams p, c
     TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem_bytes));
     attr_set[dev].store(true, std::memory_order_release);
   }
-  TG_CUDA_CHECK(launch_early(kern, pl.grid, C::threads, C::smem_bytes, st, tw, tx, p));
+  TG_CUDA_CHECK(launch_early_clusters(kern, pl.share > 1 ? pl.share : 1, pl.grid, C::threads, C::smem_bytes, st, tw, tx, p));
   return TG_OK;
 }
 
@@ -373,6 +451,8 @@ int skinny_run(const tg_gemm_args* a, cudaStream_t st) {
   p.M = int(a->M); p.N = int(a->N); p.nkb = pl.nkb;
   p.units = pl.units;
   p.w_mn = a->b_major == TG_MAJOR_MN;
+  p.share = pl.share;
+  p.d = a->d; p.ldd = static_cast<long long>(a->ldd); p.d_f32 = a->out_dtype == TG_OUT_F32;
   p.status = a->status;
   const bool rows = a->sb_gran_n == 1;
   int rc;
@@ -380,7 +460,7 @@ int skinny_run(const tg_gemm_args* a, cudaStream_t st) {
   else if (a->M <= 32) rc = rows ? launch<32, true>(a, pl, p, st) : launch<32, false>(a, pl, p, st);
   else if (a->M <= 64) rc = rows ? launch<64, true>(a, pl, p, st) : launch<64, false>(a, pl, p, st);
   else rc = rows ? launch<128, true>(a, pl, p, st) : launch<128, false>(a, pl, p, st);
-  if (rc != TG_OK) return rc;
+  if (rc != TG_OK || pl.share > 0) return rc;
   const int64_t threads = a->M * ((a->N + 3) / 4);
   const int blocks = int((threads + 255) / 256);
   if (a->out_dtype == TG_OUT_F32)
