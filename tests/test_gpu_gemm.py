@@ -347,3 +347,38 @@ def test_few_tokens_against_a_wide_weight_in_clusters(M, K, N, tile):
         assert torch.equal(y32.to(torch.bfloat16), y)
     _close(from_torch_bf16(y), fo.block_scaled_matmul(a, b, weight_tile=tile))
     ops.check_status(device="cuda")
+
+
+@pytest.mark.parametrize("K,N,T,gran", [(256, 512, 5000, 1), (256, 512, 5000, 128), (384, 128, 3001, 1), (1024, 1024, 2100, 1)])
+def test_wgrad_of_a_ragged_token_count_split_and_not(K, N, T, gran):
+    """A contraction that ends inside a block is cut like any other: the same sums as uncut, up to float32 summation order."""
+    from train_gpt_b200 import _lib, ops
+    rng = np.random.default_rng(K + N + T)
+    xq, xs = ops.quantize_colwise(to_torch_bf16(normal_bf16(rng, (T, K))))
+    quantise = ops.quantize_colwise if gran == 1 else ops.quantize_block128
+    gq, gs = quantise(to_torch_bf16(normal_bf16(rng, (T, N))))
+    plain = ops.gemm_blockscaled(xq, gq, xs, gs, M=K, N=N, K=T, a_major=_lib.TG_MAJOR_MN, b_major=_lib.TG_MAJOR_MN, sa_strides=(1, K),
+                                 sb_strides=(1, gs.shape[1]), sb_gran_n=gran, out_dtype=torch.float32, split=False)
+    cut = ops.gemm_wgrad(xq, xs, gq, gs, out_dtype=torch.float32, grad_tile=(128, 1) if gran == 1 else (128, 128))
+    assert torch.allclose(plain, cut, rtol=1e-5, atol=1e-5 * float(plain.abs().max()))
+    deq = lambda q, s, rep: q.float() * (s if rep == 1 else s.repeat_interleave(128, 1)).repeat_interleave(128, 0)[:T]
+    ref = deq(xq, xs, 1).double().T @ deq(gq, gs, gran).double()
+    assert float((plain.double() - ref).norm() / ref.norm()) < 1e-5
+    ops.check_status(device="cuda")
+
+
+@pytest.mark.parametrize("M,K,N", [(129, 256, 256), (200, 1024, 8192), (300, 512, 528), (1024, 1024, 1024), (2048, 384, 1536)])
+def test_narrow_and_wide_tiles_give_the_same_bits(M, K, N):
+    """Problems of one or two waves take 128-column tiles; the same rows inside a problem of many waves take wide ones.  A result
+    does not depend on it."""
+    from train_gpt_b200 import fp8, ops
+    rng = np.random.default_rng(M + K + N)
+    x, w = to_torch_bf16(normal_bf16(rng, (M, K))), to_torch_bf16(normal_bf16(rng, (K, N), std=0.02))
+    big = x.repeat(-(-40960 // M), 1)
+    for tile in ((128, 1), (128, 128)):
+        if N % 128 and tile == (128, 128):
+            continue
+        wq = fp8.quantize_weight(w, tile)
+        y = ops.gemm_fwd(*ops.quantize_rowwise(x), *wq, tile)
+        if ops.last_gemm_kernel_launches == 1:
+            assert torch.equal(y, ops.gemm_fwd(*ops.quantize_rowwise(big), *wq, tile)[:M])

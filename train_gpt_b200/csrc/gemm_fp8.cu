@@ -36,7 +36,7 @@
 // K-major and MN-major storage (only the coordinates swap), and the shared-memory operand
 // descriptors / instruction descriptor carry the major-ness, so dgrad and wgrad read the
 // same buffers the forward wrote, untransposed.  Few output tiles with a long contraction are
-// cut along the contraction (plan_split); few rows against a wide weight take the kernel of
+// cut along the contraction (plan_gemm); few rows against a wide weight take the kernel of
 // gemm_skinny.cu.
 //
 // Every wait on an mbarrier is bounded: when the limit runs out the waiting role raises a
@@ -820,31 +820,68 @@ splitk_reduce_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, 
   }
 }
 
-struct SplitPlan {
-  int S;             // 1 = no split
-  int64_t bytes;     // workspace the split needs
+// Tile width and number of contraction ranges of a problem, by modelled time.
+//
+// Wide tiles (256 columns with one scale per 128 columns, 192 with a scale per column) do a full GPU's work with a quarter less
+// traffic and promotion overhead per output than 128; 128-column tiles cut a problem of one or two waves finer: 1024^3 is 32
+// tiles of 256 on 148 SMs, or 64 of 128 (8.3 -> 6.5 us); 200 x 2048 x 8192 64 or 128 (12.7 -> 8.2).  A contraction cut into S
+// ranges (the first nkb % S one block longer) fills the SMs of a problem with few tiles and pays for a second kernel that adds S
+// float32 slices.
+//
+// The constants are microseconds measured on single GEMMs of 4 to 64 blocks: a launch with its ramps, a contraction block of a
+// tile (wide tiles in fewer than three waves contend less; the forward with column scales waits longer for them than the weight
+// gradient, whose scales were just written), a tile's set-up and stores, the reduction's launch and its bytes.
+// The model is within 10-15 % of the measurements it was made from; a narrower tile or a cut has to win by 3 %.
+//
+// The tile width does not show in the result; the number of ranges does, in the last bit of float32 sums, and a training run
+// amplifies that over its steps.  So where the tokens are whole blocks of 128, as a training step's are, the number of
+// ranges is a rule of its own (training_ranges) that the tile width has no part in.
+struct GemmPlan {
+  int bn, S;
+  int64_t bytes;     // workspace the cut needs
 };
-
-// S in {1, 2, 4, 8} (dividing the block count, every range at least 8 blocks) with the lowest
-// modelled time, in units of one contraction block on one SM: waves x (blocks per item + ~3 for an
-// item's ramp and stores), plus for S > 1 the reduce pass over S float32 slices at ~4 MB per unit.
-// A 2048 x 6144 weight gradient is 512 tiles = 3.5 waves of 256 blocks; cut in two it is 6.9 waves
-// of 128 (measured 6 % faster with the reduce); 2048 x 8192 (4.6 waves) is left whole.
-static SplitPlan plan_split(const tg_gemm_args* a, int bn) {
-  SplitPlan pl = {1, 0};
-  if (a->K % BK != 0) return pl;
-  const int64_t nkb = a->K / BK;
-  const int64_t tiles = ((a->M + BM - 1) / BM) * ((a->N + bn - 1) / bn);
+// S of 1 to 8 ranges of at least 8 blocks by waves of wide tiles x (blocks per item + 3 for an item's ramp and stores), plus for
+// S > 1 the reduction over S float32 slices at 4 MB per block time.
+static int training_ranges(const tg_gemm_args* a, int wide) {
+  const int64_t nkb = a->K / BK, tiles = ((a->M + BM - 1) / BM) * ((a->N + wide - 1) / wide);
   const int sms = gemm_sms();
-  if (sms <= 0) return pl;
-  // S ranges of nkb / S blocks, the first nkb % S of them one longer; the longest sets the pace of a wave
+  int ranges = 1;
   double best = 0.0;
   for (int S = 1; S <= 8; ++S) {
     if (S > 1 && nkb / S < 8) break;
-    const int64_t waves = (tiles * S + sms - 1) / sms;
-    double cost = double(waves) * (double((nkb + S - 1) / S) + 3.0);
+    double cost = double((tiles * S + sms - 1) / sms) * (double((nkb + S - 1) / S) + 3.0);
     if (S > 1) cost += double(4 * S + 2) * double(a->M) * double(a->N) / 4.0e6;
-    if (S == 1 || cost < best * 0.98) { best = cost; pl.S = S; }
+    if (S == 1 || cost < best * 0.98) { best = cost; ranges = S; }
+  }
+  return ranges;
+}
+
+static GemmPlan plan_gemm(const tg_gemm_args* a) {
+  const bool columns = a->sb_gran_n == 1;
+  const int wide = a->N <= 128 ? 128 : columns ? 192 : 256;
+  GemmPlan pl = {wide, 1, 0};
+  const int64_t nkb = (a->K + BK - 1) / BK;
+  const int sms = gemm_sms();
+  const bool whole = a->K % BK == 0 && (a->a_major == TG_MAJOR_MN || a->M % 128 == 0);      // (weight gradient: the tokens are K)
+  const int fixed = whole ? training_ranges(a, wide) : 0;
+  double best = 0.0;
+  for (const int bn : {wide, 128}) {
+    const int64_t tiles = ((a->M + BM - 1) / BM) * ((a->N + bn - 1) / bn);
+    for (int S = 1; S <= 8; ++S) {
+      if (S > 1 && nkb / S < 8) break;
+      if (fixed != 0 && S != fixed) continue;
+      const int64_t waves = (tiles * S + sms - 1) / sms;
+      const double block = bn == 256 ? (waves < 3 ? 0.44 : 0.50) : bn == 192 ? 0.47 : !columns ? 0.355 : a->a_major == TG_MAJOR_K ? 0.42 : 0.38;
+      const double tile = bn == 128 ? (columns ? 0.5 : 0.1) : 1.0;
+      double us = 3.0 + double(waves) * (block * double((nkb + S - 1) / S) + tile);
+      if (S > 1) us += 3.5 + double(4 * S + 2) * double(a->M) * double(a->N) / 8.0e6;
+      if (best == 0.0 || us < best * 0.97) {
+        best = us;
+        pl.bn = bn;
+        pl.S = S;
+      }
+    }
+    if (wide == 128) break;
   }
   if (pl.S > 1) pl.bytes = int64_t(pl.S) * a->M * a->N * int64_t(sizeof(float));
   return pl;
@@ -853,16 +890,6 @@ static SplitPlan plan_split(const tg_gemm_args* a, int bn) {
 }  // namespace tg
 
 using namespace tg;
-
-// Tile width of a problem.  One scale per 128 columns: 128 x 256 tiles, 16 promotion warps
-// (measured 1.70 / 1.92 PFLOP/s forward / dgrad against 1.53 / 1.59 for 128 x 192).  A scale per
-// column (the weight gradient): 128 x 192 tiles with 12 promotion warps, whose 128 registers per
-// thread hold the 64 accumulator columns plus the scale staging that 96 do not (1.04 PFLOP/s
-// against 0.85 for 128 x 128).
-static int tile_width(const tg_gemm_args* a) {
-  if (a->N <= 128) return 128;
-  return a->sb_gran_n == 1 ? 192 : 256;
-}
 
 static int validate_gemm(const tg_gemm_args* a) {
   if (a == nullptr) return TG_ERR_SHAPE;
@@ -883,7 +910,7 @@ static int validate_gemm(const tg_gemm_args* a) {
 extern "C" int64_t tg_gemm_workspace_bytes(const tg_gemm_args* a) {
   if (validate_gemm(a) != TG_OK || a->M == 0 || a->N == 0 || a->K == 0) return 0;
   if (skinny_takes(a)) return skinny_workspace_bytes(a);
-  return plan_split(a, tile_width(a)).bytes;
+  return plan_gemm(a).bytes;
 }
 
 extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
@@ -924,8 +951,8 @@ extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
   p.slice_elems = 0;
   p.status = a->status;
   const bool g1 = a->sb_gran_n == 1;
-  const int bn = tile_width(a);
-  const SplitPlan pl = plan_split(a, bn);
+  const GemmPlan pl = plan_gemm(a);
+  const int bn = pl.bn;
   if (pl.S > 1 && a->workspace != nullptr && a->workspace_bytes >= pl.bytes && aligned16(a->workspace)) {
     p.ksplit = pl.S;
     p.nkb_rem = p.nkb % pl.S;
