@@ -5,6 +5,8 @@ Stated bar: loss curves over 200 steps within 1 %.  Compared here on the 20-step
 average (single-batch losses of a 0.5 M-parameter model jitter by more than 1 % between ANY two
 runs, bf16 against bf16 included) over all 200 steps, plus the mean of the last 50 steps.
 """
+import ctypes
+
 import pytest
 import torch
 
@@ -196,3 +198,23 @@ def test_native_step_reports_a_token_outside_the_vocabulary():
     assert torch.isnan(a.step(ids, tgt)[0])
     with pytest.raises(RuntimeError, match="outside the vocabulary"):
         ops.check_status(device="cuda")
+
+
+@pytest.mark.parametrize("tokens,d,vocab,kind", [(1, 128, 3, "one"), (33, 128, 5, "few"), (97, 264, 7, "one"), (512, 1024, 50304, "many"),
+                                                 (1024, 2048, 40, "few"), (300, 768, 31, "negative")])
+def test_embedding_gradient_adds_as_an_accumulating_index_put(tokens, d, vocab, kind):
+    """Ids that occur once, often and always, columns that end inside a warp's 256 and ids that count from the end: the sums, rounded
+    to bf16 after every addition in token order, have index_put's bits."""
+    from train_gpt_b200 import _lib
+    gen = torch.Generator("cuda").manual_seed(tokens)
+    low, high = {"one": (vocab - 1, vocab), "negative": (-vocab, 0)}.get(kind, (0, vocab))
+    ids = torch.randint(low, high, (tokens,), device="cuda", generator=gen)
+    dx = torch.randn(tokens, d, device="cuda", generator=gen).to(torch.bfloat16)
+    want = torch.zeros(vocab, d, dtype=torch.bfloat16, device="cuda").index_put_((ids,), dx, accumulate=True)
+    got = torch.full((vocab, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    table = torch.empty(vocab * 8, dtype=torch.uint8, device="cuda")
+    lib = _lib.load()
+    rc = lib.tgh_embed_bwd(*(ctypes.c_void_p(t.data_ptr()) for t in (ids, dx, got, table)), *(ctypes.c_int64(n) for n in (tokens, d, vocab)),
+                           ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    assert torch.equal(got, want)

@@ -35,7 +35,7 @@ constexpr auto kF8 = at::kFloat8_e4m3fn;
   X(tg_add_rmsnorm_quant_fwd) X(tg_rmsnorm_bwd_scratch_bytes) X(tg_rmsnorm_bwd) X(tg_rmsnorm_bwd_add)               \
   X(tg_softcap_ce_fwd) X(tg_softcap_ce_bwd) X(tg_sumsq_scratch_bytes) X(tg_sumsq_bf16) X(tg_adamw_bf16)             \
   X(tg_gemm_workspace_bytes) X(tg_gemm_fp8_blockscaled) X(tgh_quantize_jobs) X(tgh_softcap_ce_fits) X(tgh_softcap_ce) \
-  X(tgh_global_norm_scratch_bytes) X(tgh_global_norm) X(tgh_adamw) X(tgh_embed)
+  X(tgh_global_norm_scratch_bytes) X(tgh_global_norm) X(tgh_adamw) X(tgh_embed) X(tgh_embed_bwd)
 
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;

@@ -42,6 +42,10 @@ enum { TGH_STATUS_TOKEN = 16 };
 int tgh_embed(const int64_t* ids, const void* embed, const void* pos, void* x, int64_t batch, int64_t seq, int64_t d, int64_t vocab,
               unsigned* status, void* stream);
 
+/* The gradient of embed: the rows of dx [tokens, d] added up by token id in token order, rounded to bf16 after every addition (as
+ * an accumulating index_put does); zeros for ids that do not occur.  table: vocab * 8 bytes of scratch. */
+int tgh_embed_bwd(const int64_t* ids, const void* dx, void* g_embed, void* table, int64_t tokens, int64_t d, int64_t vocab, void* stream);
+
 /* A parameter tensor with its gradient and moments: n contiguous bf16 values each, 16-byte aligned. */
 typedef struct { void* p; const void* g; void* m; void* v; int64_t n; } tgh_span;
 /* norm = sqrt of the sum of squares of every span's g.  scratch: tgh_global_norm_scratch_bytes(n) bytes whose first 16 are

@@ -15,7 +15,6 @@
 #include "host.h"
 
 #include <ATen/ops/_fused_sdp_choice.h>
-#include <ATen/ops/_index_put_impl.h>
 #include <ATen/ops/_scaled_dot_product_cudnn_attention.h>
 #include <ATen/ops/_scaled_dot_product_cudnn_attention_backward.h>
 #include <ATen/ops/_scaled_dot_product_flash_attention.h>
@@ -37,11 +36,14 @@ struct Attention {
   Tensor q, k, v, out, lse, cum_q, cum_k, seed, offset;
   c10::SymInt max_q, max_k;
 
-  // q, k, v: (B, H, T, D)
-  void forward(const Tensor& q_, const Tensor& k_, const Tensor& v_) {
+  static int64_t choose(const Tensor& q, const Tensor& k, const Tensor& v) {
+    return at::_fused_sdp_choice(q.detach().set_requires_grad(true), k, v, {}, 0.0, true);
+  }
+  // q, k, v: (B, H, T, D); choice: what choose() says of them
+  void forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, int64_t choice) {
     q = q_; k = k_; v = v_;
     Tensor debug;
-    backend = at::_fused_sdp_choice(q.detach().set_requires_grad(true), k, v, {}, 0.0, true);
+    backend = choice;
     if (backend == kCudnn) {
       std::tie(out, lse, cum_q, cum_k, max_q, max_k, seed, offset, debug) =
           at::_scaled_dot_product_cudnn_attention(q, k, v, {}, true, 0.0, true, false, std::nullopt);
@@ -129,6 +131,14 @@ class StepProgram {
     quantize_weights();
 
     const int64_t n_layers = int64_t(layers_.size());
+    // one attention backend for the step, as all its layers have one shape; the library ones need none of autograd's dispatch
+    attention_ = -1;
+    std::optional<at::AutoDispatchBelowADInplaceOrView> below;
+    if (n_layers > 0) {
+      const Tensor qkv = act(3 * hd_);
+      attention_ = Attention::choose(heads(qkv, 0), heads(qkv, 1), heads(qkv, 2));
+      if (attention_ == kCudnn || (attention_ == kFlash && c_.head_dim % 8 == 0)) below.emplace();
+    }
     std::vector<Kept> kept(n_layers);
     Tensor x = act(d_), branch;
     check(api.tgh_embed(ids.data_ptr<int64_t>(), ptr(embed_), ptr(pos_), ptr(x), b_, t_, d_, vocab_, status_, cur_stream()), "tgh_embed");
@@ -168,12 +178,7 @@ class StepProgram {
     Tensor g_seq = g_pos_.narrow(0, 0, t_);
     at::sum_out(g_seq, d.view({b_, t_, d_}), at::IntArrayRef({0}));
     if (t_ < g_pos_.size(0)) g_pos_.narrow(0, t_, g_pos_.size(0) - t_).zero_();
-    g_embed_.zero_();
-    {
-      c10::List<std::optional<Tensor>> index;
-      index.push_back(ids.view({-1}));
-      at::_index_put_impl_(g_embed_, index, d, true, true);
-    }
+    check(api.tgh_embed_bwd(ids.data_ptr<int64_t>(), ptr(d), ptr(g_embed_), token_table_, m_, d_, vocab_, cur_stream()), "tgh_embed_bwd");
     bucket_done(int(n_layers + 1));
     if (!on_end_.is_none()) on_end_();
     scratch_ = weights_memory_ = Tensor();
@@ -231,7 +236,7 @@ class StepProgram {
       for (tg_gemm_args g : {fwd(k, n), dgrad(k, n), wgrad(k, n)}) ws = std::max(ws, api.tg_gemm_workspace_bytes(&g));
     Arena a;
     const FormAt row = add_row(a, m_, wide), col = add_col(a, m_, wide), third = add_col(a, m_, d_);
-    const size_t norm = a.add(std::max<int64_t>(api.tg_rmsnorm_bwd_scratch_bytes(m_, d_), 16)), gemm = a.add(ws);
+    const size_t norm = a.add(std::max<int64_t>(api.tg_rmsnorm_bwd_scratch_bytes(m_, d_), 16)), gemm = a.add(ws), table = a.add(vocab_ * 8);
     a.make(embed_);
     scratch_ = a.memory();
     row_ = row.in(a);
@@ -239,6 +244,7 @@ class StepProgram {
     third_ = third.in(a);
     norm_partial_ = a.at(norm);
     workspace_ = a.at(gemm);
+    token_table_ = a.at(table);
   }
 
   void quantize_weights() {
@@ -286,10 +292,14 @@ class StepProgram {
   }
   void quantize(const tgh_quantize_job* jobs, int n) { check(api.tgh_quantize_jobs(jobs, n, cur_stream()), "tgh_quantize_jobs"); }
   Tensor heads(const Tensor& qkv, int64_t which) const {        // (B, H, T, D), a view
-    return qkv.narrow(1, which * hd_, hd_).view({b_, t_, c_.heads, c_.head_dim}).transpose(1, 2);
+    return qkv.as_strided({b_, c_.heads, t_, c_.head_dim}, {t_ * 3 * hd_, c_.head_dim, 3 * hd_, 1}, which * hd_);
   }
   // a (B, H, T, D) tensor as (tokens, H D), without a copy where it lies that way
-  Tensor tokens(const Tensor& o) const { return o.transpose(1, 2).reshape({m_, hd_}); }
+  Tensor tokens(const Tensor& o) const {
+    if (o.stride(3) == 1 && o.stride(1) == c_.head_dim && o.stride(2) == hd_ && o.stride(0) == t_ * hd_)
+      return o.as_strided({m_, hd_}, {hd_, 1});
+    return o.transpose(1, 2).reshape({m_, hd_});
+  }
 
   void forward_layer(int64_t l, Kept& k, Tensor& x, Tensor& branch) {
     const LayerTensors& p = layers_[l];
@@ -297,7 +307,7 @@ class StepProgram {
     k.x1 = norm_fwd(x, branch, p.norm1, k.h1);                                  // model.py:72 of the layer before, :76
     Tensor qkv = act(3 * hd_);
     run(fwd(d_, 3 * hd_), row_, w.qkv, ptr(qkv));                               // model.py:63-65
-    k.attention.forward(heads(qkv, 0), heads(qkv, 1), heads(qkv, 2));
+    k.attention.forward(heads(qkv, 0), heads(qkv, 1), heads(qkv, 2), attention_);
     const Tensor o = readable(tokens(k.attention.out), false);
     Arena keep;
     const FormAt o_col = add_col(keep, m_, hd_), a_col = add_col(keep, m_, ff_);
@@ -401,7 +411,8 @@ class StepProgram {
   Tensor scratch_, weights_memory_;
   std::vector<Weights> weights_;
   Form row_, col_, third_;
-  void *norm_partial_ = nullptr, *workspace_ = nullptr;
+  void *norm_partial_ = nullptr, *workspace_ = nullptr, *token_table_ = nullptr;
+  int64_t attention_ = -1;
 };
 
 }  // namespace
