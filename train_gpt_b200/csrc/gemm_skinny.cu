@@ -3,23 +3,24 @@
 // One pass over the weight is the work: at 16 x 8192 x 8192 it is 67 MB (10.2 us at the measured copy rate) against 0.7 us of
 // tensor-core time.  What the tiled kernel (gemm_fp8.cu) does badly there, and what is done instead:
 //   * the weight's N dimension takes the MMA's 128 rows and the tokens its columns (16, 32, 64 or 128 of them): no dead
-//     rows, and a stage of the pipeline is 16 KB of weight plus as little as 2 KB of tokens, so that 12 of them are in
-//     flight per SM;
+//     rows, and a stage of the pipeline is 16 KB of weight plus as little as 2 KB of tokens.  Seven of them in flight per SM: with
+//     twelve, or with an L2 prefetch of the first ones while the kernel before runs, the SMs read from more places of the
+//     weight at once and 16 x 8192 x 8192 takes 14.7 instead of 14.0 us;
 //   * the (tile, contraction block) units are numbered tile by tile and every block of the grid takes as many consecutive ones; it
 //     leaves each tile's part of float32 sums in a slot of the workspace.  Preferably a whole number of blocks shares a tile:
 //     all tiles are then at the same contraction rows at the same time, and what the SMs read together is whole rows of
 //     the weight, not 128-byte pieces of rows 8 KB apart (8192 x 8192: 5.0 against 4.5 TB/s);
-//   * scales arrive several blocks early (see the promotion warps);
+//   * scales arrive with the stage they belong to (see the producer warp);
 //   * a thread holds one weight row's sums over the tokens, so a slot is written 128 consecutive bytes per warp and token, and
 //     the reduce kernel, which adds a tile's slots in order, reads and writes along N: nothing is transposed;
 //   * where a tile is shared by at most four blocks (32 tiles and more), these form a thread-block cluster, the slots are
 //     their shared memories and the blocks add them up themselves: one launch, no workspace, the same order of additions;
-//   * programmatic dependent launch: barriers, tensor memory and an L2 prefetch of this block's first weight boxes (the L2 is
-//     coherent: a prefetch of bytes the kernel before is still writing is harmless) happen while the kernel before runs, and
-//     the reduce kernel is resident when the last sums arrive.
-// Bound by the weight's bytes plus about 5.5 us of two launches' ramps.  Microseconds per GEMM in a chain of them, before (split
-// contraction, transposing reduce) -> now: 16 x 8192 x 8192 24.8 -> 16.4, 16 x 2048 x 6144 13.5 -> 6.8, 1 x 2048 x 6144
-// 9.9 -> 6.6, 64 x 2048 x 8192 14.2 -> 10.4, 16 x 1024 x 1024 8.8 -> 5.8.
+//   * programmatic dependent launch: barriers and tensor memory are set up while the kernel before runs, and the reduce kernel is
+//     resident when the last sums arrive.
+// Bound by the weight's bytes plus about 4 us of ramps; 128 tokens by the L2's, 32 KB per block of contraction.  Microseconds per
+// GEMM in a chain of them: split contraction and transposing reduce -> scales fetched by the promotion warps -> now:
+// 16 x 8192 x 8192 24.8 -> 15.1 -> 14.0, 64 x 8192 x 8192 18.8 -> 16.9, 128 x 8192 x 8192 26.8 -> 21.5,
+// 16 x 2048 x 6144 13.5 -> 6.8 -> 5.9.
 #include "umma.cuh"
 
 namespace tg {
@@ -42,13 +43,11 @@ struct SkinnyCfg {
   static constexpr int bufs = 4;                                    // accumulator buffers in tensor memory
   static constexpr int tmem_cols = BN * bufs < 32 ? 32 : BN * bufs;
   static constexpr int stage_bytes = kTileBytes + BN * 128;
-  // scales, per promotion warp: the block's column factors, double-buffered, and a ring of `ahead` blocks' column and row scales
-  static constexpr int ahead = 8;
-  static constexpr int ring_slot = cols + 32;
-  static constexpr int warp_scales = 2 * cols + ahead * ring_slot;
-  static constexpr int scale_bytes = promo_warps * warp_scales * 4;
-  static constexpr int stages_fit = (kSmemLimit - 1024 - scale_bytes) / stage_bytes;
-  static constexpr int stages = stages_fit > 12 ? 12 : stages_fit;
+  // a stage's scales: a factor per token, then one per weight row (or one for all of them)
+  static constexpr int stage_scales = BN + 128;
+  static constexpr int stages_fit = (kSmemLimit - 1024) / (stage_bytes + 4 * stage_scales);
+  static constexpr int stages = stages_fit > 7 ? 7 : stages_fit;
+  static constexpr int scale_bytes = stages * 4 * stage_scales;
   static constexpr int smem_bytes = stages * stage_bytes + scale_bytes;
   static constexpr int n_bars = 2 * stages + 2 * bufs + 1;
   static_assert(n_bars <= 40, "control block too small");
@@ -73,12 +72,12 @@ struct SkinnyParams {
 __host__ __device__ __forceinline__ int skinny_first(int c, int g, int units) { return int((long long)c * units / g); }
 __host__ __device__ __forceinline__ int skinny_block_of(int u, int g, int units) { return int(((long long)(u + 1) * g - 1) / units); }
 
-__device__ __forceinline__ void l2_prefetch_2d(const CUtensorMap* map, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y) : "memory");
-}
-
 __device__ __forceinline__ void cp_async4(uint32_t dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+// arrive on `bar` (one of the arrivals it counts) when this thread's cp.async so far are done
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 // Barrier over all threads of the cluster (a cluster of one where the launch has none); it ends because every path above does.
@@ -114,8 +113,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   const int u0 = skinny_first(int(blockIdx.x), int(gridDim.x), p.units), u1 = skinny_first(int(blockIdx.x) + 1, int(gridDim.x), p.units);
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::stages; ++s) {
-      mbar_init(full0 + 8u * s, 1);
-      mbar_init(empty0 + 8u * s, 1);
+      mbar_init(full0 + 8u * s, 1 + 32);           // the boxes, and each producer lane's scales
+      mbar_init(empty0 + 8u * s, C::promo_warps);
     }
     for (int b = 0; b < C::bufs; ++b) {
       mbar_init(tfull0 + 8u * b, 1);
@@ -126,12 +125,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == C::producer_warp && elect_one()) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_w)) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_x)) : "memory");
-    int kb = u0 % p.nkb, n0 = u0 / p.nkb * BM;
-    for (int u = u0; u < u1 && u < u0 + C::stages; ++u) {
-      l2_prefetch_2d(&tmap_w, p.w_mn ? n0 : kb * BK, p.w_mn ? kb * BK : n0);
-      if (++kb == p.nkb) { kb = 0; n0 += BM; }
-    }
   }
   if (warp == C::issuer_warp) {
     tmem_alloc(smem_u32(&ctl_tmem_ptr), C::tmem_cols);
@@ -145,23 +140,44 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   grid_trigger();
 
   if (warp == C::producer_warp) {
+    // Scales come with the stage they belong to: cp.async by all lanes, which arrive on its barrier as the boxes do.  (The
+    // promotion warps fetched their own, eight units ahead: with the staging in shared memory that was most of a
+    // unit's 330 ns at 16 tokens and 630 at 128, weight from the L2.)
+    constexpr int kPer = (BN_ + 31) / 32;
     uint32_t s = 0, ph = 1;
     bool ok = true;
-    int kb = u0 % p.nkb, n0 = u0 / p.nkb * BM;
+    int kb = u0 % p.nkb, tile = u0 / p.nkb;
+    unsigned sx_off[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) sx_off[i] = unsigned(min(lane + 32 * i, p.M - 1)) * p.sx_m;      // past M: a valid scale, unused sums
     for (int u = u0; u < u1; ++u) {
       ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8u * s, ph, abort_flag, p.status, 1u));
       if (!ok) break;
+      const uint32_t fb = full0 + 8u * s;
       if (elect_one()) {
-        const uint32_t dst = sbase + s * C::stage_bytes, fb = full0 + 8u * s;
-        const int k0 = kb * BK;
+        const uint32_t dst = sbase + s * C::stage_bytes;
+        const int k0 = kb * BK, n0 = tile * BM;
         mbar_expect_tx(fb, C::stage_bytes);
         tma_load_2d(dst, &tmap_w, fb, p.w_mn ? n0 : k0, p.w_mn ? k0 : n0);
         tma_load_2d(dst + kTileBytes, &tmap_x, fb, k0, 0);
       }
       __syncwarp();
+      const uint32_t sc = sbase + uint32_t(C::stages * C::stage_bytes) + s * uint32_t(4 * C::stage_scales) + 4u * uint32_t(lane);
+#pragma unroll
+      for (int i = 0; i < kPer; ++i)
+        if (BN_ % 32 == 0 || lane < BN_) cp_async4(sc + 128u * i, p.sx + sx_off[i] + unsigned(kb) * p.sx_k);
+      if (W_ROWS) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          cp_async4(sc + 4u * BN_ + 128u * i, p.sw + unsigned(min(tile * BM + lane + 32 * i, p.N - 1)) * p.sw_n + unsigned(kb) * p.sw_k);
+      } else if (lane == 0) {
+        cp_async4(sc + 4u * BN_, p.sw + unsigned(tile) * p.sw_n + unsigned(kb) * p.sw_k);
+      }
+      cp_async_arrive(fb);
       if (++s == C::stages) { s = 0; ph ^= 1u; }
-      if (++kb == p.nkb) { kb = 0; n0 += BM; }
+      if (++kb == p.nkb) { kb = 0; ++tile; }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp >= C::issuer_warp) {
     // columns of the MMA: the tokens there are, in sixteens
     const uint32_t n_mma = uint32_t((p.M + 15) / 16 * 16);
@@ -183,7 +199,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         for (int k = 0; k < BK / UMMA_K; ++k)
           umma_f8(d_tmem, (uint64_t(desc_hi) << 32) | (a_lo0 + soff + k * a_step), (uint64_t(desc_hi) << 32) | (b_lo0 + soff + k * b_step),
                   idesc, k > 0 ? 1u : 0u);
-        umma_commit(tfull0 + 8u * buf);      // (a promotion warp that sees this frees the stage)
+        umma_commit(tfull0 + 8u * buf);      // (the promotion warps, which see this, free the stage)
       }
       __syncwarp();
       if ((s += C::issuers) >= uint32_t(C::stages)) { s -= C::stages; sph ^= 1u; }
@@ -196,88 +212,63 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     __syncwarp();
   } else {
     const int quarter = warp & 3, c0 = (warp >> 2) * C::cols, r = quarter * 32 + lane;
-    float* s_sc = reinterpret_cast<float*>(smem + C::stages * C::stage_bytes) + warp * C::warp_scales;
-    float* ring = s_sc + 2 * C::cols;
-    const uint32_t ring0 = smem_u32(ring);
+    const float* scales0 = reinterpret_cast<const float*>(smem + C::stages * C::stage_bytes);
     const uint32_t tcol0 = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(c0);
-    // Scales come `ahead` blocks early into the warp's own ring (cp.async: no registers, no barrier).  A block's weight scales
-    // are in memory nobody has touched yet, so fetching them one block ahead made every block wait out a DRAM access:
-    // 8192 x 8192 took 18 us with a scale per 128 rows and 25 with one per row, whatever the token count.
-    constexpr int kPer = (C::cols + 31) / 32;          // column scales a lane fetches per block: columns c0 + lane (+ 32)
-    unsigned sx_off[kPer];
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) sx_off[i] = unsigned(min(c0 + lane + 32 * i, p.M - 1)) * p.sx_m;      // past M: a valid scale, unused sums
-    int f_u = u0, f_kb = u0 % p.nkb, f_tile = u0 / p.nkb, f_slot = 0;      // the next block to fetch scales for
-    auto fetch = [&] {
-      if (f_u < u1) {
-        const uint32_t dst = ring0 + uint32_t(f_slot) * (C::ring_slot * 4);
-#pragma unroll
-        for (int i = 0; i < kPer; ++i)
-          if (C::cols % 32 == 0 || lane < C::cols)
-            cp_async4(dst + 4u * uint32_t(lane + 32 * i), p.sx + sx_off[i] + unsigned(f_kb) * p.sx_k);
-        if (W_ROWS) cp_async4(dst + 4u * uint32_t(C::cols + lane), p.sw + unsigned(min(f_tile * BM + r, p.N - 1)) * p.sw_n + unsigned(f_kb) * p.sw_k);
-        else if (lane == 0) cp_async4(dst + 4u * uint32_t(C::cols), p.sw + unsigned(f_tile) * p.sw_n + unsigned(f_kb) * p.sw_k);
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");         // an empty group keeps the wait count uniform
-      ++f_u;
-      if (++f_kb == p.nkb) { f_kb = 0; ++f_tile; }
-      if (++f_slot == C::ahead) f_slot = 0;
-    };
-    for (int i = 0; i < C::ahead; ++i) fetch();
-    int kb = u0 % p.nkb, tile = u0 / p.nkb, slot = 0;
+    int kb = u0 % p.nkb, tile = u0 / p.nkb;
     float2 acc[C::cols / 2];
 #pragma unroll
     for (int j = 0; j < C::cols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
-    uint32_t buf = 0, bph = 0, stage_s = 0;
+    uint32_t buf = 0, bph = 0, stage_s = 0, sph = 0;
     bool ok = true;
     for (int u = u0; u < u1; ++u) {
-      asm volatile("cp.async.wait_group %0;" ::"n"(C::ahead - 1) : "memory");
-      __syncwarp();
-      float* stage = s_sc + (u & 1) * C::cols;
-      const float* in = ring + slot * C::ring_slot;
-      const float sw = in[C::cols + (W_ROWS ? lane : 0)];
-      // column scale of the block, times the weight's where that is one number
-#pragma unroll
-      for (int i = 0; i < kPer; ++i)
-        if (C::cols % 32 == 0 || lane < C::cols) stage[lane + 32 * i] = W_ROWS ? in[lane + 32 * i] : in[lane + 32 * i] * sw;
-      __syncwarp();
-      fetch();                                                       // into the slot just read
-      if (++slot == C::ahead) slot = 0;
       const bool ends = kb + 1 == p.nkb || u + 1 == u1;              // the last block of this tile here
       const int tile_now = tile;
       if (++kb == p.nkb) { kb = 0; ++tile; }
+      // the stage's scales (its barrier was complete before the MMAs were issued: the first probe succeeds)
+      ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8u * stage_s, sph, abort_flag, p.status, 5u));
+      if (!ok) break;
+      const float* in = scales0 + stage_s * C::stage_scales;
+      const float sw = in[BN_ + (W_ROWS ? r : 0)];
+      const float2 sw2 = make_float2(sw, sw);
+      // token factors of sixteen columns, times the weight's where that is one number
+      float2 f[8];
+      auto factors = [&](int q) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float4 sc = *reinterpret_cast<const float4*>(in + c0 + 16 * q + 4 * j);
+          f[2 * j] = make_float2(sc.x, sc.y);
+          f[2 * j + 1] = make_float2(sc.z, sc.w);
+        }
+        if (!W_ROWS) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] = __fmul2_rn(f[j], sw2);
+        }
+      };
+      factors(0);
       ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8u * buf, bph, abort_flag, p.status, 5u));
       if (!ok) break;
       tc_fence_after();
-      if (warp == 0) mbar_arrive_if(empty0 + 8u * stage_s, lane == 0);   // the unit's MMAs have read their operands
-      if (++stage_s == uint32_t(C::stages)) stage_s = 0;
       const uint32_t taddr = tcol0 + buf * uint32_t(BN_);
-      const float2 sw2 = make_float2(sw, sw);
 #pragma unroll
       for (int q = 0; q < C::cols / 16; ++q) {
         uint32_t v[16];
         tmem_ld16(taddr + 16 * q, v);
         tmem_wait_ld16(v);
-        if (q == C::cols / 16 - 1) {                                 // every sum of the buffer is in registers: hand it back
+        if (q > 0) factors(q);
+        if (q == C::cols / 16 - 1) {                                 // every sum of the buffer and every scale is in registers: hand both back
           tc_fence_before();
           __syncwarp();
           mbar_arrive_if(tempty0 + 8u * buf, lane == 0);
+          mbar_arrive_if(empty0 + 8u * stage_s, lane == 0);
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 sc = *reinterpret_cast<const float4*>(stage + 16 * q + 4 * j);
-          const float2 p0 = make_float2(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]));
-          const float2 p1 = make_float2(__uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
-          float2 &a0 = acc[8 * q + 2 * j], &a1 = acc[8 * q + 2 * j + 1];
-          if (W_ROWS) {
-            a0 = __ffma2_rn(__fmul2_rn(p0, make_float2(sc.x, sc.y)), sw2, a0);
-            a1 = __ffma2_rn(__fmul2_rn(p1, make_float2(sc.z, sc.w)), sw2, a1);
-          } else {
-            a0 = __ffma2_rn(p0, make_float2(sc.x, sc.y), a0);
-            a1 = __ffma2_rn(p1, make_float2(sc.z, sc.w), a1);
-          }
+        for (int j = 0; j < 8; ++j) {
+          const float2 pj = make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+          float2& a = acc[8 * q + j];
+          a = W_ROWS ? __ffma2_rn(__fmul2_rn(pj, f[j]), sw2, a) : __ffma2_rn(pj, f[j], a);
         }
       }
+      if (++stage_s == uint32_t(C::stages)) { stage_s = 0; sph ^= 1u; }
       if (++buf == C::bufs) { buf = 0; bph ^= 1u; }
       if (ends) {
         // (share > 0: this is the block's last unit, every stage has been read; the pipeline's shared memory becomes the slot)
@@ -290,7 +281,6 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         for (int j = 0; j < C::cols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
       }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
   }
 
   if (p.share > 0) {
@@ -391,11 +381,11 @@ static SkinnyPlan plan(const tg_gemm_args* a) {
   const int sms = gemm_sms();
   p.grid = p.units < sms ? p.units : sms;
   // Ranges that end where tiles end (tiles * s blocks, s to a tile) read whole rows together and leave fewer slots; all SMs
-  // (ranges that end anywhere) is the better balance.  In microseconds: 0.33 per unit on one SM (16 KB at 50 GB/s), all units
-  // at the measured 5.0 / 4.5 TB/s, a slot written and read at ~6 TB/s.
-  const double slot = double(a->M) * BM * 8 / 6.0e6;
+  // (ranges that end anywhere) is the better balance.  In microseconds: 0.33 per unit on one SM (16 KB at 50 GB/s; 0.41 with
+  // 128 tokens beside it), all units at the measured 5.0 / 4.5 TB/s, a slot written and read at ~6 TB/s.
+  const double slot = double(a->M) * BM * 8 / 6.0e6, unit = a->M <= 64 ? 0.33 : 0.41;
   auto cost = [&](int g, int slots, double rate) {
-    const double sm = 0.33 * ((p.units + g - 1) / g), hbm = double(p.units) * kTileBytes / rate;
+    const double sm = unit * ((p.units + g - 1) / g), hbm = double(p.units) * kTileBytes / rate;
     return (sm > hbm ? sm : hbm) + slot * slots;
   };
   const int most = p.grid;
