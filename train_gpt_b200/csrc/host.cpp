@@ -180,7 +180,7 @@ Pair rmsnorm_fwd(const Tensor& x_, const Tensor& gamma_, double eps, bool pure, 
   const int64_t d = x.size(-1);
   need_gamma(gamma, d);
   const c10::cuda::CUDAGuard guard(x.device());
-  Tensor y = at::empty_like(x), rn;
+  Tensor y = empty_as(x), rn;
   if (want_rnorm) rn = empty(x.sizes().slice(0, x.dim() - 1), at::kFloat, x);
   check(api.tg_rmsnorm_fwd(ptr(x), ptr(gamma), float(eps), ptr(y), fptr(rn), x.numel() / d, d, pure ? TG_NORM_PURE : TG_NORM_FUSED,
                            cur_stream()),
@@ -201,7 +201,7 @@ NormQuant rmsnorm_quant_fwd(const Tensor& x_, const Tensor& gamma_, double eps, 
   NormQuant o;
   o.q = empty(x.sizes(), kF8, x);
   o.s = empty(with_last(x, d / kTile), at::kFloat, x);
-  if (want_y) o.y = at::empty_like(x);
+  if (want_y) o.y = empty_as(x);
   if (want_rnorm) o.rn = empty(x.sizes().slice(0, x.dim() - 1), at::kFloat, x);
   check(api.tg_rmsnorm_quant_fwd(ptr(x), ptr(gamma), float(eps), ptr(o.q), fptr(o.s), ptr(o.y), fptr(o.rn), x.numel() / d, d,
                                  pure ? TG_NORM_PURE : TG_NORM_FUSED, cur_stream()),
@@ -224,12 +224,12 @@ AddNorm add_rmsnorm_quant_fwd(const Tensor& x_, const Tensor& res_, const Tensor
   if (!want_q && !want_y) throw py::value_error("nothing to compute: neither the quantised nor the bf16 output is wanted");
   const c10::cuda::CUDAGuard guard(x.device());
   AddNorm o;
-  o.sum = at::empty_like(x);
+  o.sum = empty_as(x);
   if (want_q) {
     o.q = empty(x.sizes(), kF8, x);
     o.s = empty(with_last(x, d / kTile), at::kFloat, x);
   }
-  if (want_y) o.y = at::empty_like(x);
+  if (want_y) o.y = empty_as(x);
   check(api.tg_add_rmsnorm_quant_fwd(ptr(x), ptr(res), ptr(gamma), float(eps), ptr(o.sum), ptr(o.q), fptr(o.s), ptr(o.y), nullptr,
                                      x.numel() / d, d, pure ? TG_NORM_PURE : TG_NORM_FUSED, cur_stream()),
         "tg_add_rmsnorm_quant_fwd");
@@ -247,7 +247,7 @@ Pair rmsnorm_bwd(const Tensor& x_, const Tensor& gamma_, const Tensor& g_, doubl
     if (d > kAddNormMaxCols) throw py::value_error(cat("the fused add takes rows of at most ", kAddNormMaxCols));
   }
   const c10::cuda::CUDAGuard guard(x.device());
-  Tensor dx = at::empty_like(x), dgamma = empty({d}, at::kBFloat16, x);
+  Tensor dx = empty_as(x), dgamma = empty({d}, at::kBFloat16, x);
   const int64_t bytes = std::max<int64_t>(api.tg_rmsnorm_bwd_scratch_bytes(rows, d), 16);
   Tensor scratch = empty({bytes}, at::kByte, x);
   if (addend.defined())
@@ -367,7 +367,7 @@ void clipped_adamw(const std::vector<Tensor>& p, const std::vector<Tensor>& g, c
     spans[i] = {p[i].data_ptr(), g[i].data_ptr(), m[i].data_ptr(), v[i].data_ptr(), p[i].numel()};
   }
   const c10::cuda::CUDAGuard guard(p[0].device());
-  const Tensor n = norm.to(at::kFloat);
+  const Tensor n = to(norm, at::kFloat);
   check(api.tgh_adamw(spans.data(), int(spans.size()), float(lr), float(b1), float(b2), float(eps), float(weight_decay), fptr(n),
                       float(clip), static_cast<int32_t*>(ptr(step)), cur_stream()),
         "tgh_adamw");
@@ -492,7 +492,7 @@ ForwardOut fp8_forward(const Tensor& a, const Tensor& b_, bool w_cols, const Ten
   const int64_t k = a.size(-1), n = b_.size(1), m = rows_of(a);
   Tensor x;
   if (!row_q.defined()) {
-    x = as_bf16(a, "a").reshape({m, k});
+    x = as_rows(as_bf16(a, "a"), m, k);
     if (!x.is_cuda()) need(x, at::kBFloat16, "x");
     x = readable(x, false);
   }
@@ -559,18 +559,18 @@ Pair fp8_backward(const Tensor& a, const Tensor& b, const Tensor& g_, at::IntArr
     // (the engine's thread may not have touched the device yet, and cuBLAS wants a context when it makes its handle)
     const c10::cuda::CUDAGuard guard(g_.device());
     cudaFree(nullptr);
-    const Tensor g2 = g_.reshape({-1, n}).to(at::kBFloat16);
-    if (in.want_a) da = at::mm(g2, b.to(at::kBFloat16).t());                                 // fp8.py:96 (cuBLAS bf16)
-    if (in.want_b) db = at::mm(a.reshape({-1, k}).to(at::kBFloat16).t(), g2);                // fp8.py:97
-    if (da.defined()) da = (a_shape.size() == 2 ? da : da.reshape(a_shape)).to(a_dtype);
-    if (db.defined()) db = db.to(b_dtype);
+    const Tensor g2 = to(g_.dim() == 2 ? g_ : g_.reshape({-1, n}), at::kBFloat16);
+    if (in.want_a) da = at::mm(g2, to(b, at::kBFloat16).t());                                 // fp8.py:96 (cuBLAS bf16)
+    if (in.want_b) db = at::mm(to(a.dim() == 2 ? a : a.reshape({-1, k}), at::kBFloat16).t(), g2);                // fp8.py:97
+    if (da.defined()) da = to(a_shape.size() == 2 ? da : da.reshape(a_shape), a_dtype);
+    if (db.defined()) db = to(db, b_dtype);
     return {da, db};
   }
   TORCH_CHECK_VALUE(n % kTile == 0, "N=", n, " not divisible by block_k=", kTile, " (needed by the FP8 dgrad)");
   if (!in.want_a && !in.want_b) return {da, db};
   int64_t m = 1;
   for (size_t i = 0; i + 1 < a_shape.size(); ++i) m *= a_shape[i];
-  const Tensor g = readable(g_.reshape({m, n}).to(at::kBFloat16), false);
+  const Tensor g = readable(to(as_rows(g_, m, n), at::kBFloat16), false);
   const c10::cuda::CUDAGuard guard(g.device());
   const bool g_cols = in.mode == kFp8;               // the weight gradient's upstream operand: columns, or 128x128 tiles
   unsigned* status = status_of(g);
@@ -617,26 +617,26 @@ Pair fp8_backward(const Tensor& a, const Tensor& b, const Tensor& g_, at::IntArr
   }
   Tensor b2, a2;
   if (make_w) {
-    b2 = readable(b.to(at::kBFloat16), false);
+    b2 = readable(to(b, at::kBFloat16), false);
     tgh_quantize_job& j = jobs[n_jobs++] = job_of(b2);
     w = w_at.in(temp);
     if (in.w_cols) want_row(j, w);
     else want_block(j, w);
   }
   if (make_x) {
-    a2 = readable(a.reshape({m, k}).to(at::kBFloat16), false);
+    a2 = readable(to(as_rows(a, m, k), at::kBFloat16), false);
     tgh_quantize_job& j = jobs[n_jobs++] = job_of(a2);
     want_col(j, x = x_at.in(temp), k);
   }
   check(api.tgh_quantize_jobs(jobs, n_jobs, cur_stream()), "tgh_quantize_jobs");
   if (in.want_a) {
     run_gemm(dgrad, g_row, w, ptr(da), temp.at(ws_at), ws_bytes[0]);
-    da = da.to(a_dtype);
+    da = to(da, a_dtype);
   }
   if (in.want_b) {
     run_gemm(wgrad, x, g_col, ptr(db.defined() ? db : db_slot), temp.at(ws_at), ws_bytes[1]);
     if (in.slot_take) in.slot_ready();
-    else db = db.to(b_dtype);
+    else db = to(db, b_dtype);
   }
   return {da, db};
 }
@@ -698,6 +698,8 @@ struct BlockScaledMatmulBackward : public Node {
     variable_list out(2);
     if (!grads[0].defined()) return out;
     if (released) backward_twice();
+    std::optional<at::AutoDispatchBelowADInplaceOrView> below;      // (under create_graph the straight-through GEMMs are recorded)
+    if (!at::GradMode::is_enabled()) below.emplace();
     BackwardIn in;
     in.w_cols = w_cols;
     in.mode = mode;
@@ -775,7 +777,7 @@ struct RmsNormBackward : public Node {
   variable_list apply(variable_list&& grads) override {
     variable_list out(2);
     if (!grads[0].defined()) return out;
-    std::tie(out[0], out[1]) = rmsnorm_bwd(x.unpack(), gamma.unpack(), grads[0].to(at::kBFloat16), eps, std::nullopt);   // kernels.py:104-118
+    std::tie(out[0], out[1]) = rmsnorm_bwd(x.unpack(), gamma.unpack(), to(grads[0], at::kBFloat16), eps, std::nullopt);   // kernels.py:104-118
     return out;
   }
 };
@@ -822,7 +824,7 @@ struct CappedCEBackward : public Node {
     const int64_t vocab = x.size(-1), rows = x.numel() / vocab;
     const Tensor g = grads[0].to(at::kFloat).contiguous();
     const bool again = given;
-    if (again) d = at::empty_like(d);
+    if (again) d = empty_as(d);
     const c10::cuda::CUDAGuard guard(x.device());
     check(api.tgh_softcap_ce(ptr(x), ptr(targets), targets.scalar_type() == at::kLong, float(cap), ptr(d), fptr(g), !again, nullptr,
                              nullptr, rows, vocab, vocab, cur_stream()),
@@ -864,7 +866,7 @@ Tensor capped_cross_entropy(const Tensor& logits_, const Tensor& target_ids, dou
     {
       at::AutoDispatchBelowADInplaceOrView below;
       if (reinterpret_cast<uintptr_t>(ptr(logits)) & 15u) logits = logits.clone();
-      if (track) d = at::empty_like(logits);
+      if (track) d = empty_as(logits);
       Tensor nll = empty({rows}, at::kFloat, logits);
       loss = empty({}, at::kFloat, logits);
       check(api.tgh_softcap_ce(ptr(logits), ptr(t), t.scalar_type() == at::kLong, float(cap), ptr(d), nullptr, 0, fptr(nll), fptr(loss),

@@ -4,6 +4,7 @@
 #define TRAIN_GPT_B200_HOST_H_
 
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -81,9 +82,16 @@ inline Tensor need(const Tensor& t, at::ScalarType dt, const char* name) {
 
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
+// New CUDA memory straight from the allocator: at::empty is the same behind a dispatcher call.  With it, and with the conversions that
+// change nothing also going through the dispatcher, the two calls of a decode step took the host 10.7 us instead of 9.7.
 inline Tensor empty(at::IntArrayRef shape, at::ScalarType dt, const Tensor& like) {
-  return at::empty(shape, at::TensorOptions().dtype(dt).device(like.device()));
+  return at::detail::empty_cuda(shape, dt, like.device(), std::nullopt);
 }
+inline Tensor empty_as(const Tensor& contiguous) { return empty(contiguous.sizes(), contiguous.scalar_type(), contiguous); }
+
+// t in another type or shape; no dispatcher call where it has them
+inline Tensor to(const Tensor& t, at::ScalarType dt) { return t.scalar_type() == dt ? t : t.to(dt); }
+inline Tensor as_rows(const Tensor& t, int64_t rows, int64_t cols) { return t.dim() == 2 ? t : t.reshape({rows, cols}); }
 
 inline void* cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
