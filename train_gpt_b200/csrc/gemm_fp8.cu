@@ -781,8 +781,8 @@ static int launch_gemm(const tg_gemm_args* a, GemmParams p, cudaStream_t st) {
     TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem_bytes));
     attr_set[dev] = true;
   }
-  // few tokens: an inference call, whose kernels are short enough for an early launch to show
-  if (p.a_mn == 0 && a->M <= 256) {
+  // few tokens, or one short item per SM: kernels short enough for an early launch to show
+  if ((p.a_mn == 0 && a->M <= 256) || (n_items <= sms && p.nkb <= 16)) {
     TG_CUDA_CHECK(launch_early(kern, grid, C::threads, C::smem_bytes, st, ta, tb, td, p));
     return TG_OK;
   }

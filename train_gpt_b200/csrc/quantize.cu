@@ -345,6 +345,8 @@ __device__ __forceinline__ void panel_any(const PanelJob& a, int bx, int by, Pan
 template <bool ROW, int FORM, bool RAGGED = false>
 __global__ void __launch_bounds__(kColThreads, 4) quantize_panel_kernel(const __grid_constant__ PanelJob a) {
   __shared__ PanelSmem sm;
+  grid_trigger();
+  grid_wait();
   const int by = int(blockIdx.x) / a.tiles_x, bx = int(blockIdx.x) - by * a.tiles_x;
   if constexpr (RAGGED) panel<ROW, FORM, TG_ACT_NONE, false, true>(a, bx, by, sm);
   else panel_any<ROW, FORM, TG_ACT_NONE>(a, bx, by, sm);
@@ -372,6 +374,8 @@ __device__ __forceinline__ int job_of_block(const PanelJobList<MAX>& jobs) {
 }
 __global__ void __launch_bounds__(kColThreads, 4) quantize_panels_kernel(const __grid_constant__ PanelJobs jobs) {
   __shared__ PanelSmem sm;
+  grid_trigger();
+  grid_wait();
   const int j = job_of_block(jobs);
   const PanelJob& a = jobs.job[j];
   const int t = int(blockIdx.x) - a.first, by = t / a.tiles_x, bx = t - by * a.tiles_x;
@@ -392,6 +396,8 @@ constexpr int kMaxBlockJobs = 24;
 using BlockJobs = PanelJobList<kMaxBlockJobs>;
 __global__ void __launch_bounds__(kColThreads, 4) quantize_weights_kernel(const __grid_constant__ BlockJobs jobs) {
   __shared__ PanelSmem sm;
+  grid_trigger();
+  grid_wait();
   const PanelJob& a = jobs.job[job_of_block(jobs)];
   const int t = int(blockIdx.x) - a.first, by = t / a.tiles_x, bx = t - by * a.tiles_x;
   panel_any<false, kBlockForm, TG_ACT_NONE>(a, bx, by, sm);
@@ -404,6 +410,8 @@ template <int ACT>
 __global__ void __launch_bounds__(kColThreads, ACT == TG_ACT_GELU_BWD ? 2 : 3)
 quantize_act_kernel(const __grid_constant__ PanelJob a) {
   __shared__ PanelSmem sm;
+  grid_trigger();
+  grid_wait();
   panel_any<true, kColForm, ACT>(a, blockIdx.x, blockIdx.y, sm);
 }
 
@@ -425,20 +433,19 @@ static void with_form(PanelJob& a, int form, void* q, int64_t q_ld, float* s, in
 
 static int64_t panels_of(const PanelJob& a) { return int64_t(a.tiles_x) * ((a.rows + kTile - 1) / kTile); }
 
+// up to two panels per SM: a few microseconds
+static bool is_short(int64_t panels) { return panels <= 2 * sm_count(); }
+
 static int launch_panel(const PanelJob& a, cudaStream_t st) {
   const int64_t blocks = panels_of(a);
   if (blocks > INT32_MAX) return TG_ERR_TOO_LARGE;
-  const unsigned grid = unsigned(blocks);
-  if (a.q_row != nullptr) {
-    if (a.form == kColForm) quantize_panel_kernel<true, kColForm><<<grid, kColThreads, 0, st>>>(a);
-    else if (a.form == kBlockForm) quantize_panel_kernel<true, kBlockForm><<<grid, kColThreads, 0, st>>>(a);
-    else quantize_panel_kernel<true, kNoForm><<<grid, kColThreads, 0, st>>>(a);
-  } else {
-    if (a.form == kColForm && is_ragged(a)) quantize_panel_kernel<false, kColForm, true><<<grid, kColThreads, 0, st>>>(a);
-    else if (a.form == kColForm) quantize_panel_kernel<false, kColForm><<<grid, kColThreads, 0, st>>>(a);
-    else quantize_panel_kernel<false, kBlockForm><<<grid, kColThreads, 0, st>>>(a);
-  }
-  TG_CUDA_CHECK(cudaGetLastError());
+  auto kern = a.q_row != nullptr ? (a.form == kColForm     ? quantize_panel_kernel<true, kColForm>
+                                    : a.form == kBlockForm ? quantize_panel_kernel<true, kBlockForm>
+                                                           : quantize_panel_kernel<true, kNoForm>)
+              : a.form != kColForm ? quantize_panel_kernel<false, kBlockForm>
+              : is_ragged(a)       ? quantize_panel_kernel<false, kColForm, true>
+                                   : quantize_panel_kernel<false, kColForm>;
+  TG_CUDA_CHECK(launch_if_short(is_short(blocks), kern, dim3(unsigned(blocks)), kColThreads, 0, st, a));
   return TG_OK;
 }
 
@@ -533,13 +540,11 @@ extern "C" int tg_act_quantize_rowcol(const void* x, const void* gate, int act, 
   a.gate = static_cast<const __nv_bfloat16*>(gate);
   with_row(a, q_row, cols, s_row, cols / kTile);
   with_form(a, kColForm, q_col, cols, s_col, cols);
-  switch (act) {
-    case TG_ACT_RELU2: quantize_act_kernel<TG_ACT_RELU2><<<grid, kColThreads, 0, st>>>(a); break;
-    case TG_ACT_GELU: quantize_act_kernel<TG_ACT_GELU><<<grid, kColThreads, 0, st>>>(a); break;
-    case TG_ACT_RELU2_BWD: quantize_act_kernel<TG_ACT_RELU2_BWD><<<grid, kColThreads, 0, st>>>(a); break;
-    default: quantize_act_kernel<TG_ACT_GELU_BWD><<<grid, kColThreads, 0, st>>>(a); break;
-  }
-  TG_CUDA_CHECK(cudaGetLastError());
+  auto kern = act == TG_ACT_RELU2       ? quantize_act_kernel<TG_ACT_RELU2>
+              : act == TG_ACT_GELU       ? quantize_act_kernel<TG_ACT_GELU>
+              : act == TG_ACT_RELU2_BWD  ? quantize_act_kernel<TG_ACT_RELU2_BWD>
+                                         : quantize_act_kernel<TG_ACT_GELU_BWD>;
+  TG_CUDA_CHECK(launch_if_short(is_short(gx * gy), kern, grid, kColThreads, 0, st, a));
   return TG_OK;
 }
 
@@ -602,8 +607,7 @@ extern "C" int tgh_quantize_jobs(const tgh_quantize_job* in, int n, void* stream
     const int64_t blocks = number_blocks(jobs);
     if (blocks < 0) return TG_ERR_TOO_LARGE;
     if (blocks == 0) return TG_OK;
-    kernel<<<unsigned(blocks), kColThreads, 0, st>>>(jobs);
-    TG_CUDA_CHECK(cudaGetLastError());
+    TG_CUDA_CHECK(launch_if_short(is_short(blocks), kernel, dim3(unsigned(blocks)), kColThreads, 0, st, jobs));
     return TG_OK;
   };
   if (weights) {
