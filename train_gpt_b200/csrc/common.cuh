@@ -299,11 +299,18 @@ __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
 }
 
 // ---- programmatic dependent launch ---------------------------------------------------------
-// Used between the short kernels of an inference call, where a launch's latency is comparable with the work.  (In a training
-// step's graph of longer kernels it measured slower: blocks that sit in their wait hold resources the running kernel's last
-// wave could have used.)  A kernel launched early touches no memory before grid_wait(), so ordering is that of the stream.
+// Used between short kernels, where a launch's latency is comparable with the work.  (Between long GEMMs and quantisers it measured
+// slower: blocks that sit in their wait hold resources the running kernel's last wave could have used.)  A kernel launched early
+// touches no memory before grid_wait(), and every block of it waits, so ordering is that of the stream.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A pointer whose loads are to stay below grid_wait(): those of a const __restrict__ parameter may move otherwise.
+template <typename T>
+__device__ __forceinline__ T* loads_below(T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
 
 // A launch that may begin while the kernel before it on the stream is still running.
 template <typename... P, typename... A>
@@ -328,7 +335,7 @@ static cudaError_t launch_early(void (*kern)(P...), int grid, int threads, int s
   return launch_early_clusters(kern, 1, grid, threads, smem, st, args...);
 }
 // The same where the work is short beside a launch, an ordinary launch elsewhere.  (A step of the small model is a chain of 76 kernels
-// of 4 us: 424 us with an ordinary launch each, 352 with the quantisers', the norms' and the GEMMs' early.)
+// of 4 us: 424 us with an ordinary launch each, 328 with the short ones early.  Where the line lies is measured, kernel by kernel.)
 template <typename... P, typename... A>
 static cudaError_t launch_if_short(bool is_short, void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchAttribute attr;

@@ -781,8 +781,9 @@ static int launch_gemm(const tg_gemm_args* a, GemmParams p, cudaStream_t st) {
     TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem_bytes));
     attr_set[dev] = true;
   }
-  // few tokens, or one short item per SM: kernels short enough for an early launch to show
-  if ((p.a_mn == 0 && a->M <= 256) || (n_items <= sms && p.nkb <= 16)) {
+  // Few tokens, or few short items per SM: kernels short enough for an early launch to show (4096 x 768 x 3072 with its backward
+  // pass: 78.1 -> 74.9 us).  At every size a layer of 32768 x 2048 is 9 % slower.
+  if ((p.a_mn == 0 && a->M <= 256) || (n_items <= 4 * sms && p.nkb <= 32)) {
     TG_CUDA_CHECK(launch_early(kern, grid, C::threads, C::smem_bytes, st, ta, tb, td, p));
     return TG_OK;
   }
@@ -803,6 +804,9 @@ __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, int N, long long ldd, int S,
                      long long slice_elems) {
   const long long quads = (long long)M * (N / 4);
+  grid_trigger();
+  grid_wait();
+  ws = loads_below(ws);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < quads; i += (long long)gridDim.x * blockDim.x) {
     const long long m = i / (N / 4);
     const int n = int(i % (N / 4)) * 4;
@@ -967,13 +971,9 @@ extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
     if (rc != TG_OK) return rc;
     const long long quads = a->M * (a->N / 4);
     const int blocks = int(quads / 256 + 1 < 4096 ? quads / 256 + 1 : 4096);
-    if (f32)
-      splitk_reduce_kernel<true><<<blocks, 256, 0, st>>>(static_cast<const float*>(a->workspace), a->d, int(a->M),
-                                                         int(a->N), a->ldd, pl.S, p.slice_elems);
-    else
-      splitk_reduce_kernel<false><<<blocks, 256, 0, st>>>(static_cast<const float*>(a->workspace), a->d, int(a->M),
-                                                          int(a->N), a->ldd, pl.S, p.slice_elems);
-    TG_CUDA_CHECK(cudaGetLastError());
+    TG_CUDA_CHECK(launch_if_short(blocks <= 8 * gemm_sms(), f32 ? splitk_reduce_kernel<true> : splitk_reduce_kernel<false>, dim3(unsigned(blocks)), 256, 0,
+                                  st, static_cast<const float*>(a->workspace), a->d, int(a->M), int(a->N), static_cast<long long>(a->ldd), pl.S,
+                                  static_cast<long long>(p.slice_elems)));
     return TG_OK;
   }
   if (bn == 256) return f32 ? launch_gemm<256, 128, true>(a, p, st) : launch_gemm<256, 128, false>(a, p, st);

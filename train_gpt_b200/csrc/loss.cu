@@ -269,7 +269,11 @@ __device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
 
 template <bool WARP, bool WHOLE>
 __global__ void __launch_bounds__(WARP ? 256 : WHOLE ? kLossFwdThreads : kCeMaxThreads, WARP ? 4 : 2) softcap_ce_kernel(const CeArgs p) {
-  if (p.only_if_scaled && *p.gscale == 1.0f) return;
+  grid_trigger();
+  if (p.only_if_scaled) {
+    grid_wait();
+    if (*p.gscale == 1.0f) return;
+  }
   extern __shared__ __align__(16) uint8_t s_ce[];
   __shared__ float s_sum[2][kCeMaxThreads / 32];
   __shared__ float s_lse;
@@ -281,6 +285,7 @@ __global__ void __launch_bounds__(WARP ? 256 : WHOLE ? kLossFwdThreads : kCeMaxT
   for (uint32_t i = threadIdx.x; i <= hi - lo; i += blockDim.x)
     table[i] = uint16_t(__float_as_uint(tanh_bf16(sc.quotient(__uint_as_float((lo + i) << 16)))) >> 16);
   __syncthreads();
+  grid_wait();            // (the table comes from the cap alone)
 
   const uint32_t lo2 = lo * 0x10001u, hi2 = hi * 0x10001u;
   // (address of entry 0) - 2 lo, once per half: the sum with a pair of doubled indexes is two 16-bit addresses
@@ -494,6 +499,9 @@ __global__ void __launch_bounds__(WARP ? 256 : WHOLE ? kLossFwdThreads : kCeMaxT
 // mean of n floats, in a fixed order
 __global__ void __launch_bounds__(1024) mean_kernel(const float* __restrict__ v, int n, float* __restrict__ out) {
   __shared__ float s_part[32];
+  grid_trigger();
+  grid_wait();
+  v = loads_below(v);
   float a = 0.f, b = 0.f;
   for (int i = threadIdx.x; i < n; i += 2048) {
     a += v[i];
@@ -548,15 +556,16 @@ extern "C" int tgh_softcap_ce(const void* logits, const void* targets, int targe
     }
     const size_t smem = size_t(ce_smem(vocab));
     const int64_t per_sm_smem = std::max<int64_t>(1, (227 * 1024) / int64_t(smem + 1024));
-    const bool whole = vocab % 8 == 0 && ld % 8 == 0;
+    const bool whole = vocab % 8 == 0 && ld % 8 == 0, is_short = rows * vocab <= 1 << 20;
     if (vocab <= kCeWarpCols) {
       const int64_t cap_blocks = int64_t(sm_count()) * std::min<int64_t>(per_sm_smem, 4);
       const int blocks = int(std::min<int64_t>((rows + 7) / 8, cap_blocks));
-      if (whole) softcap_ce_kernel<true, true><<<blocks, 256, smem, st>>>(a);
-      else softcap_ce_kernel<true, false><<<blocks, 256, smem, st>>>(a);
+      TG_CUDA_CHECK(launch_if_short(is_short, whole ? softcap_ce_kernel<true, true> : softcap_ce_kernel<true, false>, dim3(unsigned(blocks)), 256,
+                                    smem, st, a));
     } else if (whole) {
       const int64_t cap_blocks = int64_t(sm_count()) * std::min<int64_t>(per_sm_smem, 2);
-      softcap_ce_kernel<false, true><<<int(std::min<int64_t>(rows, cap_blocks)), kLossFwdThreads, smem, st>>>(a);
+      TG_CUDA_CHECK(launch_if_short(is_short, softcap_ce_kernel<false, true>, dim3(unsigned(std::min<int64_t>(rows, cap_blocks))), kLossFwdThreads,
+                                    smem, st, a));
     } else {
       // as many threads as make the last pass over the row nearly full (of at most 640: two blocks an SM at 48 registers)
       const int64_t pieces = (vocab + 7) / 8;
@@ -567,13 +576,11 @@ extern "C" int tgh_softcap_ce(const void* logits, const void* targets, int targe
         if (full > best + 0.02) { best = full; nt = n; }
       }
       const int64_t cap_blocks = int64_t(sm_count()) * std::min<int64_t>(per_sm_smem, 1280 / nt);
-      softcap_ce_kernel<false, false><<<int(std::min<int64_t>(rows, cap_blocks)), nt, smem, st>>>(a);
+      TG_CUDA_CHECK(launch_if_short(is_short, softcap_ce_kernel<false, false>, dim3(unsigned(std::min<int64_t>(rows, cap_blocks))), nt, smem, st, a));
     }
-    TG_CUDA_CHECK(cudaGetLastError());
   }
   if (loss != nullptr) {
-    mean_kernel<<<1, 1024, 0, st>>>(nll, int(rows), loss);
-    TG_CUDA_CHECK(cudaGetLastError());
+    TG_CUDA_CHECK(launch_early(mean_kernel, 1, 1024, 0, st, static_cast<const float*>(nll), int(rows), loss));
   }
   return TG_OK;
 }

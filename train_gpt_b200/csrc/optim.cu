@@ -176,6 +176,10 @@ global_norm_kernel(const __grid_constant__ Spans t, double* __restrict__ partial
                    float* __restrict__ loss_out) {
   __shared__ double s_w[kOptThreads / 32];
   __shared__ bool s_last;
+  grid_trigger();
+  grid_wait();
+  loss_in = loads_below(loss_in);
+  status = loads_below(status);
   double acc = 0.0;
   auto sumsq = [](const uint4& w) {
     const float2 a = bf16x2_unpack(w.x), b = bf16x2_unpack(w.y), c = bf16x2_unpack(w.z), d = bf16x2_unpack(w.w);
@@ -235,6 +239,9 @@ global_norm_kernel(const __grid_constant__ Spans t, double* __restrict__ partial
 __global__ void __launch_bounds__(kOptThreads)
 adamw_spans_kernel(const __grid_constant__ Spans t, AdamwArgs a, const float* __restrict__ norm, float clip, int* step, int count) {
   __shared__ bool s_last;
+  grid_trigger();
+  grid_wait();
+  norm = loads_below(norm);
   const float n = *norm;
   const AdamwElement one(a, float(step[0] + 1), n < clip ? 1.0f : __fdiv_rn(clip, n));
   for_chunks(
@@ -266,6 +273,11 @@ __global__ void __launch_bounds__(kOptThreads)
 embed_kernel(const int64_t* __restrict__ ids, const __nv_bfloat16* __restrict__ embed, const __nv_bfloat16* __restrict__ pos,
              __nv_bfloat16* __restrict__ x, long long tokens, int seq, int d, int64_t vocab, unsigned* status) {
   const int per_row = d / 8;
+  grid_trigger();
+  grid_wait();
+  ids = loads_below(ids);
+  embed = loads_below(embed);
+  pos = loads_below(pos);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tokens * per_row; i += (long long)gridDim.x * blockDim.x) {
     const long long tok = i / per_row;
     const int c = int(i - tok * per_row) * 8;
@@ -295,6 +307,9 @@ embed_kernel(const int64_t* __restrict__ ids, const __nv_bfloat16* __restrict__ 
 __global__ void __launch_bounds__(kOptThreads)
 token_count_kernel(const int64_t* __restrict__ ids, int tokens, int64_t vocab, uint2* __restrict__ table) {
   const int t = int(blockIdx.x) * kOptThreads + int(threadIdx.x);
+  grid_trigger();
+  grid_wait();
+  ids = loads_below(ids);
   if (t >= tokens) return;
   int64_t id = ids[t];
   if (id < 0) id += vocab;
@@ -320,6 +335,10 @@ embed_bwd_kernel(const int64_t* __restrict__ ids, const __nv_bfloat16* __restric
   const int chunks = (d + 255) / 256, lane = threadIdx.x & 31;
   const long long unit = (long long)blockIdx.x * (kOptThreads / 32) + (threadIdx.x >> 5);
   const int first = int(unit / chunks), col = int(unit - (long long)first * chunks) * 256 + lane * 8;
+  grid_trigger();
+  grid_wait();
+  ids = loads_below(ids);
+  table = loads_below(table);
   if (first >= tokens) return;
   const bool ok = col < d;
   int64_t id = ids[first];
@@ -354,6 +373,9 @@ embed_bwd_kernel(const int64_t* __restrict__ ids, const __nv_bfloat16* __restric
   }
   if (ok) *reinterpret_cast<uint4*>(g_embed + id * d + col) = acc;
 }
+
+// at most a chunk per SM: a few microseconds
+static bool is_short(int64_t chunks) { return chunks <= sm_count(); }
 
 static int64_t number_chunks(Spans& t, const tgh_span* in, int n) {
   int64_t c = 0;
@@ -431,9 +453,8 @@ extern "C" int tgh_global_norm(const tgh_span* spans, int n, void* scratch, floa
     const int64_t cap = int64_t(sm_count()) * 4 < kNormBlocks ? int64_t(sm_count()) * 4 : kNormBlocks;
     const int blocks = int(chunks < 1 ? 1 : chunks < cap ? chunks : cap);
     const bool last = i + kMaxSpans >= n;
-    global_norm_kernel<<<blocks, kOptThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        t, partial, part, part + blocks, ticket, norm, loss_in, status, last ? loss_out : nullptr);
-    TG_CUDA_CHECK(cudaGetLastError());
+    TG_CUDA_CHECK(launch_if_short(is_short(chunks), global_norm_kernel, dim3(unsigned(blocks)), kOptThreads, 0, static_cast<cudaStream_t>(stream), t,
+                                  partial, part, part + blocks, ticket, norm, loss_in, status, last ? loss_out : static_cast<float*>(nullptr)));
     part += blocks;
   }
   return TG_OK;
@@ -454,8 +475,8 @@ extern "C" int tgh_adamw(const tgh_span* spans, int n, float lr, float b1, float
     if (chunks < 0) return TG_ERR_TOO_LARGE;
     const int64_t cap = int64_t(sm_count()) * 8;
     const int blocks = int(chunks < 1 ? 1 : chunks < cap ? chunks : cap);
-    adamw_spans_kernel<<<blocks, kOptThreads, 0, static_cast<cudaStream_t>(stream)>>>(t, a, norm, clip, step, i + kMaxSpans >= n);
-    TG_CUDA_CHECK(cudaGetLastError());
+    TG_CUDA_CHECK(launch_if_short(is_short(chunks), adamw_spans_kernel, dim3(unsigned(blocks)), kOptThreads, 0, static_cast<cudaStream_t>(stream), t, a,
+                                  norm, clip, step, int(i + kMaxSpans >= n)));
   }
   return TG_OK;
 }
@@ -467,10 +488,10 @@ extern "C" int tgh_embed(const int64_t* ids, const void* embed, const void* pos,
   if (!aligned16(embed) || !aligned16(pos) || !aligned16(x)) return TG_ERR_ALIGN;
   if (int rc = check_arch()) return rc;
   const int64_t blocks = (batch * seq * (d / 8) + kOptThreads - 1) / kOptThreads, cap = int64_t(sm_count()) * 16;
-  embed_kernel<<<unsigned(blocks < cap ? blocks : cap), kOptThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      ids, static_cast<const __nv_bfloat16*>(embed), static_cast<const __nv_bfloat16*>(pos), static_cast<__nv_bfloat16*>(x),
-      batch * seq, int(seq), int(d), vocab, status);
-  TG_CUDA_CHECK(cudaGetLastError());
+  TG_CUDA_CHECK(launch_if_short(batch * seq * d <= 1 << 20, embed_kernel, dim3(unsigned(blocks < cap ? blocks : cap)), kOptThreads, 0,
+                                static_cast<cudaStream_t>(stream), ids, static_cast<const __nv_bfloat16*>(embed),
+                                static_cast<const __nv_bfloat16*>(pos), static_cast<__nv_bfloat16*>(x), static_cast<long long>(batch * seq),
+                                int(seq), int(d), vocab, status));
   return TG_OK;
 }
 
@@ -487,9 +508,7 @@ extern "C" int tgh_embed_bwd(const int64_t* ids, const void* dx, void* g_embed, 
   TG_CUDA_CHECK(cudaGetLastError());
   const int64_t per_block = kOptThreads / 32, blocks = (tokens * ((d + 255) / 256) + per_block - 1) / per_block;
   if (blocks > INT32_MAX) return TG_ERR_TOO_LARGE;
-  embed_bwd_kernel<<<unsigned(blocks), kOptThreads, 0, st>>>(
-      ids, static_cast<const __nv_bfloat16*>(dx), static_cast<__nv_bfloat16*>(g_embed), static_cast<const uint2*>(table), int(tokens), int(d),
-      vocab);
-  TG_CUDA_CHECK(cudaGetLastError());
+  TG_CUDA_CHECK(launch_early(embed_bwd_kernel, int(blocks), kOptThreads, 0, st, ids, static_cast<const __nv_bfloat16*>(dx),
+                             static_cast<__nv_bfloat16*>(g_embed), static_cast<const uint2*>(table), int(tokens), int(d), vocab));
   return TG_OK;
 }

@@ -433,8 +433,8 @@ static void with_form(PanelJob& a, int form, void* q, int64_t q_ld, float* s, in
 
 static int64_t panels_of(const PanelJob& a) { return int64_t(a.tiles_x) * ((a.rows + kTile - 1) / kTile); }
 
-// up to two panels per SM: a few microseconds
-static bool is_short(int64_t panels) { return panels <= 2 * sm_count(); }
+// up to eight panels per SM.  (Early at every size, the 24-layer step and a wide layer are 1 to 2 % slower.)
+static bool is_short(int64_t panels) { return panels <= 8 * sm_count(); }
 
 static int launch_panel(const PanelJob& a, cudaStream_t st) {
   const int64_t blocks = panels_of(a);

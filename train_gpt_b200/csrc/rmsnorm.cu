@@ -162,7 +162,7 @@ rmsnorm_quant_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bflo
   const int pieces = cols / 8;
   grid_trigger();
   grid_wait();
-  asm volatile("" : "+l"(gamma)::"memory");       // (its loads stay below the wait)
+  gamma = loads_below(gamma);
   for (int i = threadIdx.x; i < pieces; i += blockDim.x) {
     const uint4 gq = reinterpret_cast<const uint4*>(gamma)[i];
     s_gamma[i] = make_float4(bf16lo(gq.x), bf16hi(gq.x), bf16lo(gq.y), bf16hi(gq.y));
@@ -312,7 +312,7 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
 
   const int pieces = cols / 8;
   grid_wait();
-  asm volatile("" : "+l"(gamma)::"memory");       // (its loads stay below the wait)
+  gamma = loads_below(gamma);
   for (int i = threadIdx.x; i < pieces; i += blockDim.x) {
     const uint4 gq = reinterpret_cast<const uint4*>(gamma)[i];
     s_gamma[i] = make_float4(bf16lo(gq.x), bf16hi(gq.x), bf16lo(gq.y), bf16hi(gq.y));
@@ -596,9 +596,6 @@ static int allow_smem(K kern, int bytes, std::atomic<bool> (&done)[64]) {
   return TG_OK;
 }
 
-// a million elements, 2 us of traffic: the launch counts
-static bool is_short(int64_t rows, int64_t cols) { return rows * cols <= 1 << 20; }
-
 struct NormFwd {
   const __nv_bfloat16 *x, *gamma, *res;
   float eps;
@@ -617,9 +614,9 @@ static int launch_staged(const NormFwd& a, cudaStream_t st) {
   auto kern = rmsnorm_quant_staged_kernel<NC, PURE, FULL, ADD, WPR>;
   constexpr int slots = kNormWarps * 2 * NC * 512 * (ADD ? 2 : 1);
   if (int rc = allow_smem(kern, WPR * NC * 1024 + slots, done)) return rc;
-  TG_CUDA_CHECK(launch_if_short(is_short(a.rows, a.cols), kern, dim3(unsigned(norm_blocks(a.rows, WPR, staged_blocks(WPR)))), kNormWarps * 32,
-                                size_t(a.cols) * 4 + slots, st, a.x, a.gamma, a.eps, a.q, a.scales, a.y, a.rnorm, a.rows, a.cols, a.res,
-                                a.sum_out));
+  // early at every size: one wave of blocks, whose set-up then hides (32768 x 2048, forward and backward: 116.8 -> 113.8 us)
+  TG_CUDA_CHECK(launch_early(kern, norm_blocks(a.rows, WPR, staged_blocks(WPR)), kNormWarps * 32, a.cols * 4 + slots, st, a.x, a.gamma, a.eps, a.q, a.scales,
+                             a.y, a.rnorm, a.rows, a.cols, a.res, a.sum_out));
   return TG_OK;
 }
 template <bool ADD>
@@ -690,8 +687,8 @@ static int launch_bwd(const NormBwd& a, cudaStream_t st) {
   static_assert(WPR * NC * 1024 + stage + 256 <= 227 * 1024, "row slots exceed shared memory");
   auto kern = rmsnorm_bwd_staged_kernel<NC, warps, slots, FULL, ADD, WPR>;
   if (int rc = allow_smem(kern, WPR * NC * 1024 + stage, done)) return rc;
-  TG_CUDA_CHECK(launch_if_short(is_short(a.rows, a.cols), kern, dim3(unsigned(a.blocks)), warps * 32, size_t(a.cols) * 4 + size_t(stage), st,
-                                a.x, a.gamma, a.g, a.eps, a.dx, a.partial, a.rows, a.cols, a.addend));
+  TG_CUDA_CHECK(launch_early(kern, a.blocks, warps * 32, a.cols * 4 + stage, st, a.x, a.gamma, a.g, a.eps, a.dx, a.partial, a.rows, a.cols,
+                             a.addend));
   return TG_OK;
 }
 static int launch_bwd(const NormGeom& g, const NormBwd& a, cudaStream_t st) {
