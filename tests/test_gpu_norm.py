@@ -163,6 +163,30 @@ def test_backward_with_the_skip_gradient_added(shape):
     assert (np.abs(got - two) <= np.abs(two) * 2.0 ** -7 + np.abs(b) * 2.0 ** -8 + 1e-30).all()
 
 
+@pytest.mark.parametrize("cols", [128, 384, 512, 1024, 2048])
+def test_the_skip_gradient_is_added_to_the_rounded_product(cols):
+    """dx = bf16(f32(f32(rnorm * (gs - normed * dot)) + addend)): two float32 roundings, not one.  Constant rows c with
+    eps = 0 have rnorm = RN(1/c) and normed = 1 exactly, an upstream gradient of pairs (v, -v) has dot = 0 exactly, so dx is known to the
+    bit whatever the order of the sums; where the addend cancels the product's leading bits, the two forms differ."""
+    from train_gpt_b200 import ops
+    c = np.arange(128, 256, dtype=np.float32) / 64.0
+    rn = (1.0 / c.astype(np.float64)).astype(np.float32)
+    ok = c * rn == 1.0
+    c, rn = c[ok], rn[ok]
+    rows = len(c)
+    rng = np.random.default_rng(cols)
+    v = rng.integers(1, 256, (rows, cols // 2)).astype(np.float32) / 128.0
+    g = np.stack((v, -v), axis=2).reshape(rows, cols)
+    exact = rn[:, None].astype(np.float64) * g                       # 32 bits: exact in float64
+    a = (-exact).astype(np.float32).astype(BF16)
+    want = (exact.astype(np.float32) + a.astype(np.float32)).astype(BF16)
+    fused = (exact + a.astype(np.float64)).astype(np.float32).astype(BF16)
+    assert (want != fused).sum() >= 8
+    dx, _ = ops.rmsnorm_bwd(to_torch_bf16(np.broadcast_to(c[:, None], g.shape)), to_torch_bf16(np.ones(cols)), to_torch_bf16(g), 0.0,
+                            addend=to_torch_bf16(a))
+    assert np.array_equal(from_torch_bf16(dx).astype(np.float32), want.astype(np.float32))
+
+
 def test_backward_matches_reference_vectors_and_autograd(golden):
     from train_gpt_b200 import kernels
     x = to_torch_bf16(np.asarray(golden["norm_x"]).view(BF16)).requires_grad_(True)

@@ -424,7 +424,12 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
         const float2 n2 = __fmul2_rn(bf16x2_unpack(xi[j]), rn2), gm = __fmul2_rn(bf16x2_unpack(gi[j]), mf[j]);
         // rnorm * (gs - normed*dot), the subtraction fused as kernels.py:114 allows XLA to
         float2 d = __fmul2_rn(rn2, __ffma2_rn(n2, ndot2, gm));
-        if constexpr (ADD) d = __fadd2_rn(d, bf16x2_unpack(ai[j]));
+        // (scalar: a packed add of a packed product is contracted into one fma, which rounds the sum once instead of
+        // twice -- another last bit, that the e4m3 roundings further down a backward pass amplify)
+        if constexpr (ADD) {
+          const float2 a2 = bf16x2_unpack(ai[j]);
+          d = make_float2(__fadd_rn(d.x, a2.x), __fadd_rn(d.y, a2.y));
+        }
         op[j] = pack_bf16x2(d.x, d.y);
       }
       *reinterpret_cast<uint4*>(dx + row * cols + col) = o;
