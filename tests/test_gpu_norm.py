@@ -187,6 +187,49 @@ def test_the_skip_gradient_is_added_to_the_rounded_product(cols):
     assert np.array_equal(from_torch_bf16(dx).astype(np.float32), want.astype(np.float32))
 
 
+def _weight_gradient(partial):
+    """The norm-weight gradient of (blocks, cols) float32 partial sums, added in the order that the kernel states."""
+    n = len(partial)
+    total = None
+    for w in range(8):
+        s = np.zeros((4, partial.shape[1]), np.float32)
+        b = w
+        while b + 24 < n:
+            for i in range(4):
+                s[i] += partial[b + 8 * i]
+            b += 32
+        for b in range(b, n, 8):
+            s[0] += partial[b]
+        u = (s[0] + s[1]) + (s[2] + s[3])
+        total = u if total is None else total + u
+    return total.astype(BF16)
+
+
+@pytest.mark.parametrize("blocks", [1, 7, 8, 24, 25, 31, 33, 57, 96, 121, 147, 148])
+@pytest.mark.parametrize("cols", [128, 1000])
+def test_order_of_the_weight_gradients_sums(blocks, cols):
+    """dgamma is the sum of the thread blocks' partial sums in an order that depends on their number alone, to the bit: another
+    order is another last bit, which a training run amplifies."""
+    from train_gpt_b200 import _lib
+    lib = _lib.load()
+    per_block = 16 if cols <= 512 else 12
+    rows = per_block * (blocks - 1) + 3
+    x, gamma = _inputs((rows, cols), blocks, 1e-6)
+    gy = normal_bf16(np.random.default_rng(blocks), (rows, cols), std=30.0)
+    x[-1] = 1.0                              # the last row takes the columns' sums back, so that their last bits show in bf16
+    wide = x.astype(np.float64)
+    normed = wide / np.sqrt((wide * wide).mean(1, keepdims=True) + 1e-6)
+    gy[-1] = -(gy[:-1].astype(np.float64) * normed[:-1]).sum(0)
+    t = [to_torch_bf16(v) for v in (x, gamma, gy)]
+    need = lib.tg_rmsnorm_bwd_scratch_bytes(rows, cols)
+    assert need == blocks * cols * 4
+    partial = torch.zeros((blocks, cols), device="cuda")
+    dx, dgamma = torch.empty_like(t[0]), torch.empty_like(t[1])
+    _lib.check(lib.tg_rmsnorm_bwd(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), 1e-6, dx.data_ptr(), dgamma.data_ptr(),
+                                  partial.data_ptr(), rows, cols, torch.cuda.current_stream().cuda_stream), "tg_rmsnorm_bwd")
+    assert np.array_equal(from_torch_bf16(dgamma).view(np.uint16), _weight_gradient(partial.cpu().numpy()).view(np.uint16))
+
+
 def test_backward_matches_reference_vectors_and_autograd(golden):
     from train_gpt_b200 import kernels
     x = to_torch_bf16(np.asarray(golden["norm_x"]).view(BF16)).requires_grad_(True)

@@ -463,33 +463,51 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
   for (int i = threadIdx.x; i < cols; i += blockDim.x) partial[int64_t(blockIdx.x) * cols + i] = s_sum[i];
 }
 
-// Column sums of the per-block partials.  A thread block owns 32 columns; its 32 warps take the
-// partial rows b = warp, warp + 32, ..., and the 32 results are added by a fixed tree: the order of additions is fixed by
-// (n_blocks, cols) alone.  A warp has all of its (at most five) loads in flight at once: with eight warps the kernel was a
-// chain of five L2 round trips, 5.2 us at 2048 columns.
+// Column sums of the per-block partials.  A thread block owns 32 columns.  The order of additions is fixed by (n_blocks, cols)
+// alone: row class w = b mod 8 has four sums, the i-th over b = w + 8 i, w + 8 i + 32, ..., the rows left over when a class's
+// groups of four are complete go to its first; the four are added in pairs, the eight classes in order.  Warp w + 8 i keeps the i-th
+// sum of class w and has all of its (at most eight) loads in flight at once: with eight warps of four sums each the kernel was
+// a chain of five L2 round trips, 5.2 us at 2048 columns.
 __global__ void __launch_bounds__(1024)
 rmsnorm_dgamma_reduce_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dgamma,
                              int n_blocks, int cols) {
-  __shared__ float s_part[32][33];
+  __shared__ float s_part[32][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + lane;
   grid_wait();
+  partial = loads_below(partial);
   float t = 0.f;
   if (col < cols) {
-    for (int b = warp; b < n_blocks; b += 160) {
+    const int w = warp & 7;
+    const int groups = n_blocks >= w + 25 ? (n_blocks - w - 25) / 32 + 1 : 0;      // complete groups of four rows of class w
+    const float* p = partial + int64_t(warp) * cols + col;
+    for (int k = 0; k < groups; k += 5) {
       float v[5];
 #pragma unroll
-      for (int i = 0; i < 5; ++i) v[i] = b + 32 * i < n_blocks ? __ldcg(partial + int64_t(b + 32 * i) * cols + col) : 0.f;
-      t += ((v[0] + v[1]) + (v[2] + v[3])) + v[4];
+      for (int i = 0; i < 5; ++i) v[i] = k + i < groups ? __ldcg(p + int64_t(k + i) * 32 * cols) : 0.f;
+#pragma unroll
+      for (int i = 0; i < 5; ++i) t += v[i];                                        // (x + 0 is x)
+    }
+    if (warp < 8) {
+      float v[3];
+      const int b = w + 32 * groups;                                                // at most three rows are left
+#pragma unroll
+      for (int i = 0; i < 3; ++i) v[i] = b + 8 * i < n_blocks ? __ldcg(partial + int64_t(b + 8 * i) * cols + col) : 0.f;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) t += v[i];
     }
   }
   s_part[warp][lane] = t;
   __syncthreads();
-  // warp w sums column w of the block over the 32 partial sums
-  t = s_part[lane][warp];
+  if (warp == 0 && col < cols) {
+    t = 0.f;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if (lane == 0 && blockIdx.x * 32 + warp < cols) dgamma[blockIdx.x * 32 + warp] = __float2bfloat16_rn(t);
+    for (int w = 0; w < 8; ++w) {
+      const float u = (s_part[w][lane] + s_part[w + 8][lane]) + (s_part[w + 16][lane] + s_part[w + 24][lane]);
+      t = w == 0 ? u : t + u;
+    }
+    dgamma[col] = __float2bfloat16_rn(t);
+  }
 }
 
 // ---------------------------------------------------------------------------------------
