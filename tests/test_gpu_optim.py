@@ -79,3 +79,51 @@ def test_clipped_adamw_follows_oracle_over_steps():
         gap = _ulp_gap(from_torch_bf16(p.data), ref)
         assert (gap == 0).mean() > 0.98                         # five steps of compounding last-bit differences
         assert np.abs(got - ref.astype(np.float32)).max() <= 2.0 ** -6 * np.abs(ref.astype(np.float32)).max()
+
+
+def _halving_tree(v):
+    h = 1 << (len(v).bit_length() - 1)
+    while h:
+        top = v[h:2 * h].copy()
+        v = v[:h]
+        v[:len(top)] += top
+        h //= 2
+    return v[0]
+
+
+@pytest.mark.parametrize("tensors", [1, 2, 4, 26, 64, 65, 127, 130, 600])
+def test_global_norm_has_the_bits_of_one_sum_per_tensor(tensors):
+    """One launch over all tensors against tg_sumsq_bf16 on each and the sum of the results (torch's, whose order for up to 127
+    values is the halving tree): the same order of additions, hence the same bits, with ragged tails, tensors of one block and, in the last
+    round, of more blocks than there are partial sums; several times, as the tickets have to be zero again after a call."""
+    from train_gpt_b200 import ops, optim
+    gen = torch.Generator("cuda").manual_seed(tensors)
+    opt = optim.ClippedAdamW([torch.nn.Parameter(torch.zeros(8, dtype=torch.bfloat16, device="cuda"))], lr=1e-3)
+    for turn in range(8):
+        sizes = [1 + (i * 7919 + turn) % 5000 for i in range(tensors)]
+        sizes[-1] = 2048 * 37 + turn
+        if turn == 7:
+            sizes[0] = 2048 * 1024 * 3 + 13
+        grads = [torch.randn(n, device="cuda", generator=gen).to(torch.bfloat16) for n in sizes]
+        sums = torch.stack([ops.sumsq(g).reshape(()) for g in grads])
+        want = np.sqrt(_halving_tree(sums.cpu().numpy()))
+        if tensors < 128:
+            assert float(sums.sum().sqrt()) == float(want)
+        assert float(opt.global_norm(grads)) == float(want)
+
+
+@pytest.mark.parametrize("clip", [1.0, 0.7, 1e9])
+def test_clip_factor_has_the_bits_of_the_tensor_expression(clip):
+    """tgh_adamw derives the factor from the norm as `clip / norm` on a tensor does: reciprocal, then product."""
+    from train_gpt_b200 import ops
+    gen = torch.Generator("cuda").manual_seed(3)
+    n = 100_003
+    p, g, m = (torch.randn(n, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(3))
+    v = torch.rand(n, device="cuda", generator=gen).to(torch.bfloat16)
+    for norm in torch.rand(12, device="cuda", generator=gen) * 30 + 1:
+        a, b = [t.clone() for t in (p, m, v)], [t.clone() for t in (p, m, v)]
+        scale = torch.where(norm < clip, torch.ones_like(norm), clip / norm).to(torch.float32)
+        ops.adamw_step(a[0], g, a[1], a[2], torch.tensor(4, dtype=torch.int32, device="cuda"), 1e-2, 0.9, 0.999, 1e-8, 0.1, gscale=scale)
+        count = torch.tensor([3, 0], dtype=torch.int32, device="cuda")
+        ops._host().clipped_adamw([b[0]], [g], [b[1]], [b[2]], count, norm, clip, 1e-2, 0.9, 0.999, 1e-8, 0.1)
+        assert count.tolist() == [4, 0] and all(torch.equal(s, t) for s, t in zip(a, b))

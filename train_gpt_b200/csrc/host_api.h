@@ -48,8 +48,9 @@ int tgh_embed_bwd(const int64_t* ids, const void* dx, void* g_embed, void* table
 
 /* A parameter tensor with its gradient and moments: n contiguous bf16 values each, 16-byte aligned. */
 typedef struct { void* p; const void* g; void* m; void* v; int64_t n; } tgh_span;
-/* norm = sqrt of the sum of squares of every span's g.  scratch: tgh_global_norm_scratch_bytes(n) bytes whose first 16 are
- * zero before the first use (they are again after each).  loss_out, if not NULL: *loss_in, or NaN where *status is not 0. */
+/* norm = sqrt of the sum of squares of every span's g: the spans' sums as tg_sumsq_bf16 gives them, added as a halving tree.
+ * scratch: tgh_global_norm_scratch_bytes(n) bytes for this n, all zero before the first use; calls that share one are ordered by
+ * one stream.  loss_out, if not NULL: *loss_in, or NaN where *status is not 0. */
 int64_t tgh_global_norm_scratch_bytes(int n);
 int tgh_global_norm(const tgh_span* spans, int n, void* scratch, float* norm, const float* loss_in, const unsigned* status,
                     float* loss_out, void* stream);

@@ -13,16 +13,19 @@ constexpr int kSumsqBlocks = 1024;   // partial sums of tg_sumsq_bf16 (caller sc
 
 __device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
+__device__ __forceinline__ float sumsq8(const uint4& w) {
+  const float2 a = bf16x2_unpack(w.x), b = bf16x2_unpack(w.y), c = bf16x2_unpack(w.z), d = bf16x2_unpack(w.w);
+  const float2 t = __fadd2_rn(__ffma2_rn(c, c, __fmul2_rn(a, a)), __ffma2_rn(d, d, __fmul2_rn(b, b)));
+  return t.x + t.y;
+}
+
 __global__ void __launch_bounds__(kOptThreads)
 sumsq_partial_kernel(const __nv_bfloat16* __restrict__ x, long long n, float* __restrict__ partial) {
   __shared__ float s_w[kOptThreads / 32];
   float acc = 0.f;
   const long long vecs = n / 8;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < vecs; i += (long long)gridDim.x * blockDim.x) {
-    const uint4 w = ld_nc_v4(x + 8 * i);
-    const float2 a = bf16x2_unpack(w.x), b = bf16x2_unpack(w.y), c = bf16x2_unpack(w.z), d = bf16x2_unpack(w.w);
-    const float2 t = __fadd2_rn(__ffma2_rn(c, c, __fmul2_rn(a, a)), __ffma2_rn(d, d, __fmul2_rn(b, b)));
-    acc += t.x + t.y;
+    acc += sumsq8(ld_nc_v4(x + 8 * i));
   }
   if (blockIdx.x == 0)   // ragged tail (n % 8 elements)
     for (long long i = vecs * 8 + threadIdx.x; i < n; i += blockDim.x) {
@@ -134,18 +137,17 @@ adamw_kernel(AdamwSpan s, AdamwArgs a, const int* __restrict__ step, const float
 // and five elementwise torch kernels for the clip factor and the step count: 215 us of launches beside the 1.3 ms of memory
 // traffic at 406 M parameters, and nothing but launches for a small model.
 //
-// Work is handed out in chunks of kChunk elements numbered through all tensors; a block's chunk numbers only grow, so it
-// walks the table of tensors once.  Both kernels wait for memory: with four 16-byte loads in flight per thread instead of one the
-// norm of 406 M elements takes 120 us (it was 215; 6.75 TB/s), with two pieces (eight loads) in flight the update 966 us (1031; 5.9 TB/s).
+// The update's work is handed out in chunks of kChunk elements numbered through all tensors; a block's chunk numbers only grow, so it
+// walks the table of tensors once.  It waits for memory: with two pieces (eight 16-byte loads) in flight per thread instead of one
+// the update of 406 M elements takes 966 us (1031; 5.9 TB/s).
 // ---------------------------------------------------------------------------------------
 constexpr int kMaxSpans = 64;
 constexpr int kPieces = 4;                   // of 8 elements per thread and chunk
 constexpr int kChunk = kOptThreads * 8 * kPieces;
-constexpr int kNormBlocks = 592;             // 4 per SM; partial sums of one launch
 
 struct Spans {
   AdamwSpan s[kMaxSpans];
-  int first[kMaxSpans + 1];                  // number of the tensor's first chunk
+  int first[kMaxSpans + 1];                  // number of the tensor's first chunk (norm: of its first thread block)
   int n;
 };
 // Over this block's chunks: whole(span, first piece of this thread) for a chunk that lies inside its tensor -- the thread's
@@ -168,74 +170,141 @@ __device__ __forceinline__ void for_chunks(const Spans& t, W&& whole, P&& part) 
   }
 }
 
-// Sum of squares in double from the eighth element on, so that the norm does not depend on how the gradients are laid out
-// over tensors.  The block that finishes last adds the blocks' partial sums in order and resets the ticket.
+// The norm's sums have the order of tg_sumsq_bf16 on each tensor -- as many thread blocks, each thread's pieces, lanes, warps and
+// blocks added alike -- and of a halving tree over the tensors' sums (see below), so the bits are those of one
+// launch per tensor and a torch sum of up to 127 of them.  They matter: the clip factor multiplies every gradient, and the e4m3 roundings of the
+// steps that follow amplify its last bit.
+//
+// The block of a tensor that finishes last adds its blocks' sums, the last of these the tensors'; both reset their tickets.  Where
+// the grid is small (`few`), the last block of all does both, which saves a round through a ticket: the small model's
+// 0.5 M elements 4.8 us, 6.3 without.  406 M elements: 122 us (6.7 TB/s).
+// Scratch: the ticket of the tensors in 16 bytes, then per tensor a ticket, a sum and kSumsqBlocks partial sums.
+struct NormScratch {
+  unsigned* done;
+  unsigned* ticket;          // [n]
+  float* sum;                // [n]
+  float* partial;            // [n][kSumsqBlocks]
+};
+__host__ __device__ __forceinline__ NormScratch norm_scratch(void* p, int n) {
+  NormScratch s;
+  s.done = static_cast<unsigned*>(p);
+  s.ticket = s.done + 4;
+  s.sum = reinterpret_cast<float*>(s.ticket + n);
+  s.partial = s.sum + n;
+  return s;
+}
+static int64_t sumsq_blocks(int64_t n) {
+  const int64_t want = (n / 8 + kOptThreads - 1) / kOptThreads;
+  return want < 1 ? 1 : want > kSumsqBlocks ? kSumsqBlocks : want;
+}
+
 __global__ void __launch_bounds__(kOptThreads)
-global_norm_kernel(const __grid_constant__ Spans t, double* __restrict__ partial, int first_part, int parts, unsigned* ticket,
-                   float* __restrict__ norm, const float* __restrict__ loss_in, const unsigned* __restrict__ status,
-                   float* __restrict__ loss_out) {
-  __shared__ double s_w[kOptThreads / 32];
-  __shared__ bool s_last;
+global_norm_kernel(const __grid_constant__ Spans t, void* scratch, int from, int n, int few, float* __restrict__ norm, const float* __restrict__ loss_in,
+                   const unsigned* __restrict__ status, float* __restrict__ loss_out) {
+  __shared__ float s_w[kOptThreads / 32];
+  __shared__ int s_last, s_very_last;
+  constexpr int kTree = 2 * kOptThreads;
+  __shared__ float s_tree[kTree];
   grid_trigger();
   grid_wait();
   loss_in = loads_below(loss_in);
   status = loads_below(status);
-  double acc = 0.0;
-  auto sumsq = [](const uint4& w) {
-    const float2 a = bf16x2_unpack(w.x), b = bf16x2_unpack(w.y), c = bf16x2_unpack(w.z), d = bf16x2_unpack(w.w);
-    const float2 q = __fadd2_rn(__ffma2_rn(c, c, __fmul2_rn(a, a)), __ffma2_rn(d, d, __fmul2_rn(b, b)));
-    return double(q.x + q.y);
-  };
-  for_chunks(
-      t,
-      [&](const AdamwSpan& s, long long i) {
-        uint4 w[kPieces];
+  const NormScratch sc = norm_scratch(scratch, n);
+  int k = 0;                                             // this block's tensor: the last whose first block is not above it
 #pragma unroll
-        for (int u = 0; u < kPieces; ++u) w[u] = ld_nc_v4(s.g + 8 * (i + u * kOptThreads));
+  for (int step = kMaxSpans / 2; step > 0; step >>= 1)
+    if (k + step < t.n && t.first[k + step] <= int(blockIdx.x)) k += step;
+  const int block = int(blockIdx.x) - t.first[k], blocks = t.first[k + 1] - t.first[k], lane = threadIdx.x & 31;
+  const AdamwSpan& s = t.s[k];
+  k += from;
+  const long long vecs = s.n / 8, stride = (long long)blocks * kOptThreads;
+  float acc = 0.f;
+  for (long long i = (long long)block * kOptThreads + threadIdx.x; i < vecs; i += kPieces * stride) {
+    uint4 w[kPieces];
 #pragma unroll
-        for (int u = 0; u < kPieces; ++u) acc += sumsq(w[u]);
-      },
-      [&](const AdamwSpan& s, long long i) {
-        if (8 * i + 8 <= s.n) {
-          acc += sumsq(ld_nc_v4(s.g + 8 * i));
-        } else {
-          for (long long e = 8 * i; e < s.n; ++e) {
-            const float f = __bfloat162float(s.g[e]);
-            acc += double(f * f);
-          }
-        }
-      });
-  auto block_sum = [&](double v) {
+    for (int u = 0; u < kPieces; ++u) w[u] = i + u * stride < vecs ? ld_nc_v4(s.g + 8 * (i + u * stride)) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = v;
-    __syncthreads();
-    v = s_w[0];
+    for (int u = 0; u < kPieces; ++u) acc += sumsq8(w[u]);          // (what does not exist adds +0: no change)
+  }
+  if (block == 0)
+    for (long long i = vecs * 8 + threadIdx.x; i < s.n; i += kOptThreads) {
+      const float f = __bfloat162float(s.g[i]);
+      acc = fmaf(f, f, acc);
+    }
 #pragma unroll
-    for (int i = 1; i < kOptThreads / 32; ++i) v += s_w[i];
-    return v;
-  };
-  acc = block_sum(acc);
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) s_w[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  float* partial = sc.partial + (long long)k * kSumsqBlocks;
   if (threadIdx.x == 0) {
-    partial[first_part + blockIdx.x] = acc;
+    acc = s_w[0];
+#pragma unroll
+    for (int i = 1; i < kOptThreads / 32; ++i) acc += s_w[i];
+    partial[block] = acc;
     __threadfence();
-    s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    s_last = few ? atomicAdd(sc.done, 1u) == gridDim.x - 1u : atomicAdd(sc.ticket + k, 1u) == unsigned(blocks) - 1u;
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  acc = 0.0;
-  for (int i = threadIdx.x; i < parts; i += kOptThreads) acc += __ldcg(partial + i);
-  acc = block_sum(acc);
+  // a tensor's sum over its blocks, by one warp
+  auto tensor_sum = [&](const float* part, int count) {
+    float v = 0.f;
+    for (int i = lane; i < count; i += 32 * 8) {
+      float w[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) w[u] = i + 32 * u < count ? __ldcg(part + i + 32 * u) : 0.f;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v += w[u];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+  const bool here = n <= kTree;
+  if (few) {
+    for (int j = threadIdx.x >> 5; j < n; j += kOptThreads / 32) {
+      const float v = tensor_sum(sc.partial + (long long)j * kSumsqBlocks, t.first[j + 1] - t.first[j]);
+      if (lane == 0) s_tree[j] = v;
+    }
+  } else {
+    if (threadIdx.x < 32) {
+      const float v = tensor_sum(partial, blocks);
+      if (lane == 0) {
+        __stcg(sc.sum + k, v);
+        sc.ticket[k] = 0u;
+        __threadfence();
+        s_very_last = atomicAdd(sc.done, 1u) == unsigned(n) - 1u;
+      }
+    }
+    __syncthreads();
+    if (!s_very_last) return;
+    __threadfence();
+    if (here)
+      for (int i = threadIdx.x; i < n; i += kOptThreads) s_tree[i] = __ldcg(sc.sum + i);
+  }
+  __syncthreads();
+  // the tensors' sums as torch.sum adds a short vector: with p the largest power of two in n, v[i] + v[i + p], then halves of p
+  int p = 1;
+  while (2 * p <= n) p *= 2;
+  auto at = [&](int i) { return here ? s_tree[i] : __ldcg(sc.sum + i); };
+  for (int h = p; h > 0; h >>= 1) {
+    for (int i = threadIdx.x; i < h && i + h < n; i += kOptThreads) {
+      const float v = at(i) + at(i + h);
+      if (here) s_tree[i] = v;
+      else __stcg(sc.sum + i, v);
+    }
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
-    *ticket = 0u;
-    *norm = float(sqrt(acc));
+    *sc.done = 0u;
+    *norm = __fsqrt_rn(at(0));
     if (loss_out != nullptr) *loss_out = *status != 0u ? __int_as_float(0x7fffffff) : *loss_in;
   }
 }
 
-// clip (optax.clip_by_global_norm: clip / norm where the norm is not below clip) and update; the last launch's last
-// block counts the step
+// clip (optax.clip_by_global_norm: the reciprocal of the norm times clip where the norm is not below clip) and update; the last
+// launch's last block counts the step
 __global__ void __launch_bounds__(kOptThreads)
 adamw_spans_kernel(const __grid_constant__ Spans t, AdamwArgs a, const float* __restrict__ norm, float clip, int* step, int count) {
   __shared__ bool s_last;
@@ -243,7 +312,7 @@ adamw_spans_kernel(const __grid_constant__ Spans t, AdamwArgs a, const float* __
   grid_wait();
   norm = loads_below(norm);
   const float n = *norm;
-  const AdamwElement one(a, float(step[0] + 1), n < clip ? 1.0f : __fdiv_rn(clip, n));
+  const AdamwElement one(a, float(step[0] + 1), n < clip ? 1.0f : __fmul_rn(__frcp_rn(n), clip));
   for_chunks(
       t,
       [&](const AdamwSpan& s, long long i) {
@@ -377,14 +446,15 @@ embed_bwd_kernel(const int64_t* __restrict__ ids, const __nv_bfloat16* __restric
 // at most a chunk per SM: a few microseconds
 static bool is_short(int64_t chunks) { return chunks <= sm_count(); }
 
-static int64_t number_chunks(Spans& t, const tgh_span* in, int n) {
+// numbers the tensors' chunks (blocks: the thread blocks that the norm takes) through; returns how many there are, or -1
+static int64_t number_chunks(Spans& t, const tgh_span* in, int n, bool blocks) {
   int64_t c = 0;
   t.n = n;
   for (int i = 0; i < n; ++i) {
     t.s[i] = {static_cast<__nv_bfloat16*>(in[i].p), static_cast<const __nv_bfloat16*>(in[i].g), static_cast<__nv_bfloat16*>(in[i].m),
               static_cast<__nv_bfloat16*>(in[i].v), static_cast<long long>(in[i].n)};
     t.first[i] = int(c);
-    c += (in[i].n + kChunk - 1) / kChunk;
+    c += blocks ? sumsq_blocks(in[i].n) : (in[i].n + kChunk - 1) / kChunk;
     if (c > INT32_MAX) return -1;
   }
   t.first[n] = int(c);
@@ -402,8 +472,7 @@ extern "C" int tg_sumsq_bf16(const void* x, int64_t n, float* out, void* scratch
   if (!aligned16(x) || !aligned16(scratch)) return TG_ERR_ALIGN;
   if (int rc = check_arch()) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int64_t want = (n / 8 + kOptThreads - 1) / kOptThreads;
-  const int blocks = int(want < 1 ? 1 : (want > kSumsqBlocks ? kSumsqBlocks : want));
+  const int blocks = int(sumsq_blocks(n));
   sumsq_partial_kernel<<<blocks, kOptThreads, 0, st>>>(static_cast<const __nv_bfloat16*>(x), n, static_cast<float*>(scratch));
   TG_CUDA_CHECK(cudaGetLastError());
   sumsq_final_kernel<<<1, 32, 0, st>>>(static_cast<const float*>(scratch), blocks, out);
@@ -429,9 +498,7 @@ extern "C" int tg_adamw_bf16(void* p, const void* g, void* m, void* v, int64_t n
   return TG_OK;
 }
 
-extern "C" int64_t tgh_global_norm_scratch_bytes(int n) {
-  return 16 + int64_t(sizeof(double)) * kNormBlocks * ((n + kMaxSpans - 1) / kMaxSpans);
-}
+extern "C" int64_t tgh_global_norm_scratch_bytes(int n) { return 16 + int64_t(n) * (8 + int64_t(sizeof(float)) * kSumsqBlocks); }
 
 extern "C" int tgh_global_norm(const tgh_span* spans, int n, void* scratch, float* norm, const float* loss_in, const unsigned* status,
                                float* loss_out, void* stream) {
@@ -443,19 +510,13 @@ extern "C" int tgh_global_norm(const tgh_span* spans, int n, void* scratch, floa
   }
   if (!aligned16(scratch)) return TG_ERR_ALIGN;
   if (int rc = check_arch()) return rc;
-  unsigned* ticket = static_cast<unsigned*>(scratch);
-  double* partial = reinterpret_cast<double*>(static_cast<char*>(scratch) + 16);
-  int part = 0;
   for (int i = 0; i < n; i += kMaxSpans) {
     Spans t;
-    const int64_t chunks = number_chunks(t, spans + i, n - i < kMaxSpans ? n - i : kMaxSpans);
-    if (chunks < 0) return TG_ERR_TOO_LARGE;
-    const int64_t cap = int64_t(sm_count()) * 4 < kNormBlocks ? int64_t(sm_count()) * 4 : kNormBlocks;
-    const int blocks = int(chunks < 1 ? 1 : chunks < cap ? chunks : cap);
-    const bool last = i + kMaxSpans >= n;
-    TG_CUDA_CHECK(launch_if_short(is_short(chunks), global_norm_kernel, dim3(unsigned(blocks)), kOptThreads, 0, static_cast<cudaStream_t>(stream), t,
-                                  partial, part, part + blocks, ticket, norm, loss_in, status, last ? loss_out : static_cast<float*>(nullptr)));
-    part += blocks;
+    const int64_t blocks = number_chunks(t, spans + i, n - i < kMaxSpans ? n - i : kMaxSpans, true);
+    if (blocks < 0) return TG_ERR_TOO_LARGE;
+    const bool few = blocks <= int64_t(kPieces) * sm_count();         // at most a chunk's worth per SM
+    TG_CUDA_CHECK(launch_if_short(few, global_norm_kernel, dim3(unsigned(blocks)), kOptThreads, 0, static_cast<cudaStream_t>(stream), t, scratch,
+                                  i, n, int(few && n <= kMaxSpans), norm, loss_in, status, loss_out));
   }
   return TG_OK;
 }
@@ -471,7 +532,7 @@ extern "C" int tgh_adamw(const tgh_span* spans, int n, float lr, float b1, float
   const AdamwArgs a = {lr, b1, b2, eps, weight_decay};
   for (int i = 0; i < n; i += kMaxSpans) {
     Spans t;
-    const int64_t chunks = number_chunks(t, spans + i, n - i < kMaxSpans ? n - i : kMaxSpans);
+    const int64_t chunks = number_chunks(t, spans + i, n - i < kMaxSpans ? n - i : kMaxSpans, false);
     if (chunks < 0) return TG_ERR_TOO_LARGE;
     const int64_t cap = int64_t(sm_count()) * 8;
     const int blocks = int(chunks < 1 ? 1 : chunks < cap ? chunks : cap);
