@@ -170,3 +170,15 @@ def test_one_pass_gradient_has_the_bits_of_the_two_kernels(rows, vocab):
     losses.capped_cross_entropy(a, tt.long(), 15.0).backward()
     _, lse, th = ops.softcap_ce_fwd(a.detach(), tt, 15.0)
     assert torch.equal(a.grad, ops.softcap_ce_bwd(th, tt, lse, None, 15.0))
+
+
+@pytest.mark.parametrize("rows,vocab", [(128, 256), (1000, 512), (1024, 256), (3001, 264), (8192, 2056)])
+def test_loss_has_the_bits_of_the_mean_over_tokens(rows, vocab):
+    """The loss is the mean that torch takes of the rows' values (which have the bits of the separate forward kernel's)."""
+    from train_gpt_b200 import losses, ops
+    for seed in range(4):
+        x, t = _case(rows, vocab, seed)
+        x, t = to_torch_bf16(x), torch.from_numpy(t).cuda()
+        want = ops.softcap_ce_fwd(x, t, 15.0)[0].mean()
+        assert float(losses.capped_cross_entropy(x, t, 15.0)) == float(want)
+        assert float(losses.capped_cross_entropy(x.clone().requires_grad_(), t, 15.0)) == float(want)

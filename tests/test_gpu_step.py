@@ -6,6 +6,7 @@ average (single-batch losses of a 0.5 M-parameter model jitter by more than 1 % 
 runs, bf16 against bf16 included) over all 200 steps, plus the mean of the last 50 steps.
 """
 import ctypes
+import zlib
 
 import pytest
 import torch
@@ -134,6 +135,33 @@ def test_flat_optimizer_state_and_direct_weight_gradients_change_no_bit():
                         assert p_.data_ptr() - base == g_.data_ptr() - b.buckets.flat[bi].data_ptr()
                         assert p_.stride() == g_.stride()
                 assert lp["wq"].is_contiguous() != direct
+
+
+# Three steps of the small model, eight sequences, as the step launched operation by operation through autograd gave them: loss and
+# norm of every step, a checksum of the parameters after the last.
+SMALL_STEPS = {
+    "relu2": ([("0x1.6511200000000p+2", "0x1.7efbd20000000p-1"), ("0x1.6477900000000p+2", "0x1.8307360000000p-1"),
+               ("0x1.64e7b20000000p+2", "0x1.75c11a0000000p-1")], 0xc1905a0a),
+    "gelu": ([("0x1.651d400000000p+2", "0x1.c101400000000p-1"), ("0x1.646b1a0000000p+2", "0x1.c6983a0000000p-1"),
+              ("0x1.64c3c00000000p+2", "0x1.b7a6200000000p-1")], 0x639c5cb5)}
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("act", ["relu2", "gelu"])
+def test_small_model_repeats_recorded_steps(act, graph):
+    """Every kernel of this step is deterministic (the attention too, at this length), so a trajectory that was recorded once comes
+    back to the last bit: a changed order of additions or rounding in any kernel shows here.  (Attention and the bf16 GEMMs are the
+    libraries': another version of those may move it too.)"""
+    from train_gpt_b200.step import SMALL, StepConfig, Trainer, synthetic_batch
+    cfg = StepConfig(activation=act, **SMALL)
+    tr = Trainer(cfg, torch.device("cuda", 0), seed=5, graph=graph)
+    steps, crc = [], 0
+    for i in range(3):
+        loss, norm = tr.step(*synthetic_batch(cfg, 8, "cuda", seed=5 + i))
+        steps.append((float(loss).hex(), float(norm).hex()))
+    for p in tr.model.parameters():
+        crc = zlib.crc32(p.detach().contiguous().view(torch.int16).cpu().numpy().tobytes(), crc)
+    assert (steps, crc) == SMALL_STEPS[act]
 
 
 def test_fp8_loss_curve_matches_bf16_at_the_training_configuration():

@@ -827,7 +827,7 @@ struct CappedCEBackward : public Node {
     if (again) d = empty_as(d);
     const c10::cuda::CUDAGuard guard(x.device());
     check(api.tgh_softcap_ce(ptr(x), ptr(targets), targets.scalar_type() == at::kLong, float(cap), ptr(d), fptr(g), !again, nullptr,
-                             nullptr, rows, vocab, vocab, cur_stream()),
+                             rows, vocab, vocab, cur_stream()),
           "tgh_softcap_ce");
     given = true;
     out[0] = d;
@@ -868,10 +868,10 @@ Tensor capped_cross_entropy(const Tensor& logits_, const Tensor& target_ids, dou
       if (reinterpret_cast<uintptr_t>(ptr(logits)) & 15u) logits = logits.clone();
       if (track) d = empty_as(logits);
       Tensor nll = empty({rows}, at::kFloat, logits);
-      loss = empty({}, at::kFloat, logits);
-      check(api.tgh_softcap_ce(ptr(logits), ptr(t), t.scalar_type() == at::kLong, float(cap), ptr(d), nullptr, 0, fptr(nll), fptr(loss),
-                               rows, vocab, vocab, cur_stream()),
+      check(api.tgh_softcap_ce(ptr(logits), ptr(t), t.scalar_type() == at::kLong, float(cap), ptr(d), nullptr, 0, fptr(nll), rows, vocab,
+                               vocab, cur_stream()),
             "tgh_softcap_ce");
+      loss = nll.mean();                                                             // losses.py:12
     }
     if (!track) return loss;
     std::shared_ptr<CappedCEBackward> node(new CappedCEBackward(), torch::autograd::deleteNode);

@@ -27,14 +27,14 @@ int tgh_quantize_jobs(const tgh_quantize_job* jobs, int n, void* stream);
 
 /* Whether tgh_softcap_ce takes this problem (a row and its cap fit the one-pass kernel). */
 int tgh_softcap_ce_fits(float cap, int64_t rows, int64_t vocab);
-/* Mean capped cross-entropy AND its gradient from one read of the logits.
+/* Capped cross-entropy of each row AND the gradient of their mean from one read of the logits.
  *   logits    bf16 [rows, ld], row r starting at logits + r * ld (any alignment; the base 16-byte aligned)
  *   targets   int64 [rows], or int32 if !targets_64
  *   dlogits   bf16 [rows, ld] (base 16-byte aligned) or NULL: gscale / rows * d(sum nll)/dlogits
  *   gscale    device float or NULL for 1;  only_if_scaled: the launch does nothing where *gscale is 1
- *   nll       float [rows] or NULL;  loss: float scalar, mean of nll, or NULL */
+ *   nll       float [rows] or NULL */
 int tgh_softcap_ce(const void* logits, const void* targets, int targets_64, float cap, void* dlogits, const float* gscale,
-                   int only_if_scaled, float* nll, float* loss, int64_t rows, int64_t vocab, int64_t ld, void* stream);
+                   int only_if_scaled, float* nll, int64_t rows, int64_t vocab, int64_t ld, void* stream);
 
 /* x[b, t, :] = bf16(embed[ids[b, t]] + pos[t]) (train-gpt model.py:83).  Negative ids count from the end; one outside the
  * vocabulary stores TGH_STATUS_TOKEN in *status and makes its row NaN. */

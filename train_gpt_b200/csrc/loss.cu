@@ -496,30 +496,6 @@ __global__ void __launch_bounds__(WARP ? 256 : WHOLE ? kLossFwdThreads : kCeMaxT
   }
 }
 
-// mean of n floats, in a fixed order
-__global__ void __launch_bounds__(1024) mean_kernel(const float* __restrict__ v, int n, float* __restrict__ out) {
-  __shared__ float s_part[32];
-  grid_trigger();
-  grid_wait();
-  v = loads_below(v);
-  float a = 0.f, b = 0.f;
-  for (int i = threadIdx.x; i < n; i += 2048) {
-    a += v[i];
-    if (i + 1024 < n) b += v[i + 1024];
-  }
-  a += b;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = a;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    a = s_part[threadIdx.x];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (threadIdx.x == 0) *out = a / float(n);
-  }
-}
-
 constexpr int kCeSmemMax = 226 * 1024;
 static int64_t ce_smem(int64_t vocab) {
   const int64_t row = (vocab + 14) / 8 * 16;
@@ -536,8 +512,8 @@ extern "C" int tgh_softcap_ce_fits(float cap, int64_t rows, int64_t vocab) {
 }
 
 extern "C" int tgh_softcap_ce(const void* logits, const void* targets, int targets_64, float cap, void* dlogits, const float* gscale,
-                              int only_if_scaled, float* nll, float* loss, int64_t rows, int64_t vocab, int64_t ld, void* stream) {
-  if (rows < 0 || vocab <= 0 || ld < vocab || (loss != nullptr && nll == nullptr) || (only_if_scaled && gscale == nullptr))
+                              int only_if_scaled, float* nll, int64_t rows, int64_t vocab, int64_t ld, void* stream) {
+  if (rows < 0 || vocab <= 0 || ld < vocab || (only_if_scaled && gscale == nullptr))
     return TG_ERR_SHAPE;
   if (!tgh_softcap_ce_fits(cap, rows, vocab)) return TG_ERR_TOO_LARGE;
   if (!aligned16(logits) || !aligned16(dlogits)) return TG_ERR_ALIGN;
@@ -578,9 +554,6 @@ extern "C" int tgh_softcap_ce(const void* logits, const void* targets, int targe
       const int64_t cap_blocks = int64_t(sm_count()) * std::min<int64_t>(per_sm_smem, 1280 / nt);
       TG_CUDA_CHECK(launch_if_short(is_short, softcap_ce_kernel<false, false>, dim3(unsigned(std::min<int64_t>(rows, cap_blocks))), nt, smem, st, a));
     }
-  }
-  if (loss != nullptr) {
-    TG_CUDA_CHECK(launch_early(mean_kernel, 1, 1024, 0, st, static_cast<const float*>(nll), int(rows), loss));
   }
   return TG_OK;
 }

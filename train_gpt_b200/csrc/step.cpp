@@ -156,10 +156,11 @@ class StepProgram {
     }
     x = branch = Tensor();
     Tensor logits = at::mm(hf, unembed_);                      // stays bf16 (bench_fp8_norm.py:86)
-    Tensor dlogits = empty_as(logits), loss = empty({}, at::kFloat, embed_), nll = empty({m_}, at::kFloat, embed_);
+    Tensor dlogits = empty_as(logits), nll = empty({m_}, at::kFloat, embed_);
     check(api.tgh_softcap_ce(ptr(logits), ptr(targets), targets.scalar_type() == at::kLong, float(c_.cap), ptr(dlogits), nullptr, 0,
-                             fptr(nll), fptr(loss), m_, vocab_, vocab_, cur_stream()),
+                             fptr(nll), m_, vocab_, vocab_, cur_stream()),
           "tgh_softcap_ce");
+    const Tensor loss = nll.mean();
     logits = Tensor();
     // ---- backward
     at::mm_out(g_unembed_, hf.t(), dlogits);
