@@ -211,6 +211,36 @@ def test_fp8_loss_curve_matches_bf16_at_the_training_configuration():
     assert float(gn_rel) < 0.10, float(gn_rel)
 
 
+def test_hyper_parameters_and_requires_grad_are_read_at_every_step():
+    """What a program changes between eager steps -- a schedule's learning rate, the clip norm, a frozen parameter -- takes effect at the next
+    one, in the native step as in the one through autograd."""
+    from train_gpt_b200.step import SMALL, StepConfig, Trainer, synthetic_batch
+    cfg = StepConfig(**SMALL)
+    a, b = (Trainer(cfg, torch.device("cuda", 0), seed=1) for _ in range(2))
+    assert a._program is not None
+    b._program = None
+    changes = [{}, {"lr": 2e-3}, {"clip": 0.05}, {"wd": 0.5, "b1": 0.5}, {"b2": 0.9, "eps": 1e-3}, {"lr": 0.0}, "freeze", "thaw"]
+    for i, change in enumerate(changes):
+        before = a.model.embed.detach().clone()
+        for tr in (a, b):
+            if isinstance(change, str):
+                for lp in tr.model.layers:
+                    lp["norm1"].requires_grad_(change == "thaw")
+                tr.opt.lr = 1e-3
+            else:
+                for k, v in change.items():
+                    assert hasattr(tr.opt, k)
+                    setattr(tr.opt, k, v)
+        ids, tgt = synthetic_batch(cfg, 2, "cuda", seed=i)
+        (la, na), (lb, nb) = a.step(ids, tgt), b.step(ids if i else ids.cpu(), tgt)
+        assert float(la) == float(lb) and float(na) == float(nb), change
+        assert torch.equal(before, a.model.embed) == (change == {"lr": 0.0})
+        for s, t in zip(a.model.parameters() + a.opt.state_tensors(), b.model.parameters() + b.opt.state_tensors()):
+            assert torch.equal(s, t), change
+    ids, tgt = synthetic_batch(cfg, 2, "cuda", seed=0)
+    assert float(a.step(ids.cpu(), tgt)[0]) == float(b.step(ids, tgt)[0])          # ids in host memory
+
+
 def test_native_step_reports_a_token_outside_the_vocabulary():
     """The native step's embedding kernel checks token ids itself: the loss is NaN and the status word says why.  Negative ids
     count from the end, as an index does."""

@@ -94,10 +94,10 @@ class StepProgram {
   // Parameters and, in the same structure, the slices of the flat gradient tensors; `flat`: per bucket the flat parameters,
   // gradients and moments; count: int32 (2,), see tgh_adamw.  on_bucket(i) / on_attention() / on_end(), or None: a bucket's
   // gradients are complete / an attention backward is about to be launched / the backward pass is over.
-  StepProgram(Config c, Hyper h, Tensor embed, Tensor pos, Tensor final_norm, Tensor unembed, std::vector<std::vector<Tensor>> layers,
+  StepProgram(Config c, Tensor embed, Tensor pos, Tensor final_norm, Tensor unembed, std::vector<std::vector<Tensor>> layers,
               Tensor g_embed, Tensor g_pos, Tensor g_final_norm, Tensor g_unembed, std::vector<std::vector<Tensor>> g_layers,
               std::vector<std::vector<Tensor>> flat, Tensor count, py::object on_bucket, py::object on_attention, py::object on_end)
-      : c_(c), h_(h), embed_(embed), pos_(pos), final_norm_(final_norm), unembed_(unembed), g_embed_(g_embed), g_pos_(g_pos),
+      : c_(c), embed_(embed), pos_(pos), final_norm_(final_norm), unembed_(unembed), g_embed_(g_embed), g_pos_(g_pos),
         g_final_norm_(g_final_norm), g_unembed_(g_unembed), count_(count), on_bucket_(on_bucket), on_attention_(on_attention),
         on_end_(on_end) {
     auto layer = [](const std::vector<Tensor>& t) { return LayerTensors{t.at(0), t.at(1), t.at(2), t.at(3), t.at(4), t.at(5)}; };
@@ -114,13 +114,14 @@ class StepProgram {
     norm_scratch_ = at::zeros({api.tgh_global_norm_scratch_bytes(int(flat_.size()))}, embed.options().dtype(at::kByte));
   }
 
-  // (loss, global gradient norm); the loss is NaN if a GEMM gave up on a device wait
-  Pair step(const Tensor& ids_, const Tensor& targets_) {
+  // (loss, global gradient norm); the loss is NaN if a GEMM gave up on a device wait.  The hyper-parameters come with every step: a
+  // schedule changes them between steps.
+  Pair step(const Tensor& ids_, const Tensor& targets_, const Hyper& h) {
     const at::NoGradGuard no_grad;
     const c10::cuda::CUDAGuard guard(embed_.device());
-    Tensor ids = ids_.to(at::kLong).contiguous(), targets = targets_.contiguous();
-    if (ids.dim() != 2 || targets.sizes() != ids.sizes() || !ids.is_cuda() || !targets.is_cuda())
-      throw py::value_error("ids and targets are (batch, tokens) CUDA tensors of one shape");
+    Tensor ids = ids_.to(embed_.device(), at::kLong).contiguous(), targets = targets_.contiguous();
+    if (ids.dim() != 2 || targets.sizes() != ids.sizes() || !targets.is_cuda())
+      throw py::value_error("ids and targets are (batch, tokens) tensors of one shape, targets on the GPU");
     if (targets.scalar_type() != at::kLong) targets = targets.to(at::kInt);
     b_ = ids.size(0);
     t_ = ids.size(1);
@@ -190,8 +191,8 @@ class StepProgram {
     check(api.tgh_global_norm(spans.data(), int(spans.size()), ptr(norm_scratch_), fptr(norm), fptr(loss), status_, fptr(loss_out),
                               cur_stream()),
           "tgh_global_norm");
-    check(api.tgh_adamw(spans.data(), int(spans.size()), float(h_.lr), float(h_.b1), float(h_.b2), float(h_.eps), float(h_.weight_decay),
-                        fptr(norm), float(h_.clip), static_cast<int32_t*>(ptr(count_)), cur_stream()),
+    check(api.tgh_adamw(spans.data(), int(spans.size()), float(h.lr), float(h.b1), float(h.b2), float(h.eps), float(h.weight_decay),
+                        fptr(norm), float(h.clip), static_cast<int32_t*>(ptr(count_)), cur_stream()),
           "tgh_adamw");
     return {loss_out, norm};
   }
@@ -400,7 +401,6 @@ class StepProgram {
   }
 
   Config c_;
-  Hyper h_;
   Tensor embed_, pos_, final_norm_, unembed_, g_embed_, g_pos_, g_final_norm_, g_unembed_, count_, norm_scratch_;
   std::vector<LayerTensors> layers_, grads_;
   std::vector<std::vector<Tensor>> flat_;
@@ -420,16 +420,15 @@ class StepProgram {
 
 void tgh::register_step(py::module_& m) {
   py::class_<StepProgram>(m, "StepProgram")
-      .def(py::init([](std::tuple<int64_t, int64_t, double, double, int, int> c, std::tuple<double, double, double, double, double, double> h,
-                       Tensor embed, Tensor pos, Tensor final_norm, Tensor unembed, std::vector<std::vector<Tensor>> layers, Tensor g_embed,
+      .def(py::init([](std::tuple<int64_t, int64_t, double, double, int, int> c, Tensor embed, Tensor pos, Tensor final_norm, Tensor unembed, std::vector<std::vector<Tensor>> layers, Tensor g_embed,
                        Tensor g_pos, Tensor g_final_norm, Tensor g_unembed, std::vector<std::vector<Tensor>> g_layers,
                        std::vector<std::vector<Tensor>> flat, Tensor count, py::object on_bucket, py::object on_attention, py::object on_end) {
         const auto [heads, head_dim, eps, cap, act, act_bwd] = c;
-        const auto [lr, b1, b2, adam_eps, wd, clip] = h;
-        return std::make_unique<StepProgram>(Config{heads, head_dim, eps, cap, act, act_bwd}, Hyper{lr, b1, b2, adam_eps, wd, clip}, embed,
-                                             pos, final_norm, unembed, layers, g_embed, g_pos, g_final_norm, g_unembed, g_layers, flat, count,
+        return std::make_unique<StepProgram>(Config{heads, head_dim, eps, cap, act, act_bwd}, embed, pos,
+                                             final_norm, unembed, layers, g_embed, g_pos, g_final_norm, g_unembed, g_layers, flat, count,
                                              on_bucket, on_attention, on_end);
       }))
-      .def("step", &StepProgram::step);
+      .def("step", [](StepProgram& p, const Tensor& ids, const Tensor& targets, double lr, double b1, double b2, double eps, double weight_decay,
+                      double clip) { return p.step(ids, targets, Hyper{lr, b1, b2, eps, weight_decay, clip}); });
   m.def("softcap_ce_fits", [](double cap, int64_t rows, int64_t vocab) { return bool(api.tgh_softcap_ce_fits(float(cap), rows, vocab)); });
 }

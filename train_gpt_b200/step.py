@@ -433,6 +433,7 @@ class Trainer:
             self.opt = torch.optim.AdamW(self.model.parameters(), lr=cfg.lr, weight_decay=cfg.weight_decay,
                                          betas=(0.9, 0.999), eps=1e-8, fused=on_gpu, capturable=self._want_graph)
 
+        self._params = self.model.parameters()
         self._program = self._native_program()
 
     def _native_program(self):
@@ -445,7 +446,7 @@ class Trainer:
                 and not (c.d_model % 128 or h % 128 or c.d_ff % 128)):
             return None
         host = ops._host()
-        if not host.softcap_ce_fits(c.logit_cap, 1, c.vocab_size) or not all(p.requires_grad for p in self.model.parameters()):
+        if not host.softcap_ce_fits(c.logit_cap, 1, c.vocab_size) or not all(p.requires_grad for p in self._params):
             return None
         m = self.model
         grads = {id(p): g for bi, params in enumerate(b.params) for p, g in zip(params, b.views(bi, b.flat[bi]))}
@@ -460,14 +461,15 @@ class Trainer:
         many = self.world > 1
         return host.StepProgram(
             (c.n_heads, c.head_dim, c.rms_eps, c.logit_cap, TG_ACT[c.activation], TG_ACT[c.activation + "_bwd"]),
-            (self.opt.lr, self.opt.b1, self.opt.b2, self.opt.eps, self.opt.wd, self.opt.clip),
             m.embed, m.pos, m.final_norm, m.unembed, layers, grads[id(m.embed)], grads[id(m.pos)], grads[id(m.final_norm)],
             grads[id(m.unembed)], g_layers, [list(f) for f in self.opt._flat], self.opt._count,
             b.bucket_done if many else None, b.flush if many else None, b.finish if many else None)
 
     def _eager_step(self, ids, targets):
-        if self._program is not None:
-            return self._program.step(ids, targets)
+        # the native program computes every gradient, so it runs only while every parameter wants one
+        if self._program is not None and all(p.requires_grad for p in self._params):
+            o = self.opt                          # read at every step: a schedule changes them
+            return self._program.step(ids, targets, o.lr, o.b1, o.b2, o.eps, o.wd, o.clip)
         self.buckets.zero()
         loss = self.model.loss(ids, targets)
         loss.backward()
