@@ -318,6 +318,7 @@ skinny_reduce_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, 
   const int i = int(blockIdx.x) * 256 + int(threadIdx.x), quads = (N + 3) / 4, m = i / quads, n = (i - m * quads) * 4;
   grid_trigger();
   grid_wait();
+  ws = loads_below(ws);
   if (m >= M) return;
   const int tile = n / BM;
   const int c0 = skinny_block_of(tile * nkb, g, units), c1 = skinny_block_of(tile * nkb + nkb - 1, g, units);

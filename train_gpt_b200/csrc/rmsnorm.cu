@@ -528,6 +528,7 @@ rmsnorm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   const int64_t row = blockIdx.x;
   grid_trigger();
   grid_wait();
+  gamma = loads_below(gamma);              // (in a training step the optimiser's kernel, not far ahead, writes it)
   const bool ok = col < cols;
   const uint4 w = ok ? ld_nc_v4(x + row * cols + col) : make_uint4(0, 0, 0, 0);
   const uint4 gq = ok ? *reinterpret_cast<const uint4*>(gamma + col) : make_uint4(0, 0, 0, 0);
