@@ -64,3 +64,12 @@ def test_plain_loads_stay_below_the_wait(f, name, params, body):
         assert not any(re.search(u, before) for u in uses), (f, name, p)
         if plain:
             assert re.search(rf"\b{p} = loads_below\({p}\);", after), (f, name, p)
+
+
+def test_no_load_takes_the_non_coherent_path():
+    """`ld.global.nc` is for memory that nothing writes while the kernel runs.  A kernel launched early runs from before its input is
+    written, and scratch that several kernels of a step reuse may still be held by that path with what it was."""
+    for f in sorted(os.listdir(CSRC)):
+        if f.endswith((".cu", ".cuh")):
+            text = _strip(open(os.path.join(CSRC, f)).read())
+            assert "ld.global.nc" not in text and "__ldg(" not in text, f

@@ -463,13 +463,13 @@ gemm_fp8_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a,
     auto load_sb_lane = [&](int g) {
       float v = 0.f;
       const int kb = 32 * g + lane;
-      if (kb < open_nkb) v = ldg_f32(p.sb + sb_off + uint32_t(kb) * uint32_t(p.sb_sk));
+      if (kb < open_nkb) v = ld_f32(p.sb + sb_off + uint32_t(kb) * uint32_t(p.sb_sk));
       return v;
     };
     auto load_sb_cols = [&]() {     // per-column scales of the block sb_off points at
       float2 v;
-      v.x = ldg_f32(p.sb + sb_off);
-      v.y = kPerLane == 2 ? ldg_f32(p.sb + sb_off + uint32_t(p.sb_sn)) : 0.f;
+      v.x = ld_f32(p.sb + sb_off);
+      v.y = kPerLane == 2 ? ld_f32(p.sb + sb_off + uint32_t(p.sb_sn)) : 0.f;
       return v;
     };
     auto open_tile = [&](int item) {
@@ -491,7 +491,7 @@ gemm_fp8_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a,
         sb_off = uint32_t(nblk) * uint32_t(p.sb_sn) + kb_off * uint32_t(p.sb_sk);
         sb_grp = load_sb_lane(0);
       }
-      sa_q0 = ldg_f32(p.sa + sa_off);
+      sa_q0 = ld_f32(p.sa + sa_off);
       sa_off += uint32_t(p.sa_sk);
     };
     const uint32_t is_lane0 = lane == 0;
@@ -516,7 +516,7 @@ gemm_fp8_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const float sa_v = sa_q0;
         float2 sb_v = sb_q0;
         const bool more = kb + 1 < nkb;
-        if (more) sa_q0 = ldg_f32(p.sa + sa_off);
+        if (more) sa_q0 = ld_f32(p.sa + sa_off);
         sa_off += uint32_t(p.sa_sk);
         if (SB_GRAN == 1) {
           if (more) sb_q0 = load_sb_cols();

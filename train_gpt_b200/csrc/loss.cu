@@ -96,10 +96,10 @@ softcap_ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const int32_t* _
     float m = -3.0e38f, s = 0.f;
     // the next piece is loaded before this one is worked on: the kernel's top stall was the wait for its
     // one 16-byte load per thread
-    uint4 w_next = threadIdx.x * 8 < vocab ? ld_nc_v4(p + threadIdx.x * 8) : make_uint4(0u, 0u, 0u, 0u);
+    uint4 w_next = threadIdx.x * 8 < vocab ? ld_stream_v4(p + threadIdx.x * 8) : make_uint4(0u, 0u, 0u, 0u);
     for (int i = threadIdx.x * 8; i < vocab; i += kLossFwdThreads * 8) {
       const uint4 w = w_next;
-      if (i + kLossFwdThreads * 8 < vocab) w_next = ld_nc_v4(p + i + kLossFwdThreads * 8);
+      if (i + kLossFwdThreads * 8 < vocab) w_next = ld_stream_v4(p + i + kLossFwdThreads * 8);
       const uint32_t xi[4] = {w.x, w.y, w.z, w.w};
       float2 z[4];
       uint4 to;
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(WARP ? 256 : WHOLE ? kLossFwdThreads : kCeMaxT
     q.last = (q.off + p.vocab) >> 3;
     return q;
   };
-  auto load = [&](const Row& q, int i) -> uint4 { return i < q.last ? ld_nc_v4(q.base + i * 8) : make_uint4(0u, 0u, 0u, 0u); };
+  auto load = [&](const Row& q, int i) -> uint4 { return i < q.last ? ld_stream_v4(q.base + i * 8) : make_uint4(0u, 0u, 0u, 0u); };
   // the tanh values of a pair of logits
   auto tanh_pair = [&](uint32_t w, uint32_t mag) {
     const uint32_t m = __vmaxu2(mag, kCeFloor2);

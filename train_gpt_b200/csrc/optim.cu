@@ -25,7 +25,7 @@ sumsq_partial_kernel(const __nv_bfloat16* __restrict__ x, long long n, float* __
   float acc = 0.f;
   const long long vecs = n / 8;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < vecs; i += (long long)gridDim.x * blockDim.x) {
-    acc += sumsq8(ld_nc_v4(x + 8 * i));
+    acc += sumsq8(ld_stream_v4(x + 8 * i));
   }
   if (blockIdx.x == 0)   // ragged tail (n % 8 elements)
     for (long long i = vecs * 8 + threadIdx.x; i < n; i += blockDim.x) {
@@ -86,7 +86,7 @@ struct AdamwPiece {
   uint4 p, g, m, v;
   __device__ __forceinline__ void load(const AdamwSpan& s, long long i) {
     p = *reinterpret_cast<const uint4*>(s.p + 8 * i);
-    g = ld_nc_v4(s.g + 8 * i);
+    g = ld_stream_v4(s.g + 8 * i);
     m = *reinterpret_cast<const uint4*>(s.m + 8 * i);
     v = *reinterpret_cast<const uint4*>(s.v + 8 * i);
   }
@@ -222,7 +222,7 @@ global_norm_kernel(const __grid_constant__ Spans t, void* scratch, int from, int
   for (long long i = (long long)block * kOptThreads + threadIdx.x; i < vecs; i += kPieces * stride) {
     uint4 w[kPieces];
 #pragma unroll
-    for (int u = 0; u < kPieces; ++u) w[u] = i + u * stride < vecs ? ld_nc_v4(s.g + 8 * (i + u * stride)) : make_uint4(0u, 0u, 0u, 0u);
+    for (int u = 0; u < kPieces; ++u) w[u] = i + u * stride < vecs ? ld_stream_v4(s.g + 8 * (i + u * stride)) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
     for (int u = 0; u < kPieces; ++u) acc += sumsq8(w[u]);          // (what does not exist adds +0: no change)
   }
@@ -417,7 +417,7 @@ embed_bwd_kernel(const int64_t* __restrict__ ids, const __nv_bfloat16* __restric
   if (int(entry.x) != tokens - first) return;               // not the id's first token
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   uint4 acc = zero;
-  add8(acc, ok ? ld_nc_v4(dx + (long long)first * d + col) : zero);
+  add8(acc, ok ? ld_stream_v4(dx + (long long)first * d + col) : zero);
   int left = int(entry.y) - 1;
   for (int t0 = first + 1; left > 0 && t0 < tokens; t0 += 32) {
     const int t = t0 + lane;
@@ -431,7 +431,7 @@ embed_bwd_kernel(const int64_t* __restrict__ ids, const __nv_bfloat16* __restric
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int at = __ffs(hits) - 1;
-        w[i] = at >= 0 && ok ? ld_nc_v4(dx + (long long)(t0 + at) * d + col) : zero;
+        w[i] = at >= 0 && ok ? ld_stream_v4(dx + (long long)(t0 + at) * d + col) : zero;
         n += at >= 0;
         hits &= hits - 1u;
       }

@@ -26,7 +26,7 @@ quantize_rowwise_kernel(const uint4* __restrict__ x, uint2* __restrict__ q,
 #pragma unroll
     for (int u = 0; u < kRowUnroll; ++u) {
       const int64_t t = t0 + u;
-      w[u] = (t < n_tiles) ? ld_nc_v4(x + t * 16 + lane16) : make_uint4(0, 0, 0, 0);
+      w[u] = (t < n_tiles) ? ld_stream_v4(x + t * 16 + lane16) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int u = 0; u < kRowUnroll; ++u) {
@@ -204,11 +204,11 @@ __device__ __forceinline__ void panel(const PanelJob& a, int bx, int by, PanelSm
     for (int r = 0; r < kColRowsPerThread; ++r, xp += step, gp += step) {
       const bool ok = FULL || row0 + r * kColHalfWarps < rows;
       if constexpr (RAGGED) w[r] = load8_ragged(xp, ok ? a.cols - col0 : 0);
-      else w[r] = FULL || (ok && col0 < a.cols) ? ld_nc_v4(xp) : make_uint4(0, 0, 0, 0);
+      else w[r] = FULL || (ok && col0 < a.cols) ? ld_stream_v4(xp) : make_uint4(0, 0, 0, 0);
       if constexpr (ACT != TG_ACT_NONE) {
         uint4 g = make_uint4(0, 0, 0, 0);
         if constexpr (ACT == TG_ACT_RELU2_BWD || ACT == TG_ACT_GELU_BWD)
-          if (ok) g = ld_nc_v4(gp);
+          if (ok) g = ld_stream_v4(gp);
         w[r] = act_apply<ACT>(w[r], g);   // rows past the end stay zero: every variant maps (0, 0) to 0
       }
     }

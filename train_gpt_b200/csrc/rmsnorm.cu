@@ -78,7 +78,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 #pragma unroll
     for (int c = 0; c < NCHUNK; ++c) {
       const int col = col_base + c * 256;
-      w[c] = col < cols ? ld_nc_v4(x + row * cols + col) : make_uint4(0, 0, 0, 0);
+      w[c] = col < cols ? ld_stream_v4(x + row * cols + col) : make_uint4(0, 0, 0, 0);
     }
     float part[NCHUNK];
 #pragma unroll
@@ -371,7 +371,7 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
     if constexpr (kAddEarly) {
 #pragma unroll
       for (int c = 0; c < NCHUNK; ++c)
-        ad[c] = (FULL || col_base + c * 256 < cols) ? ld_nc_v4(addend + row * cols + col_base + c * 256) : make_uint4(0, 0, 0, 0);
+        ad[c] = (FULL || col_base + c * 256 < cols) ? ld_stream_v4(addend + row * cols + col_base + c * 256) : make_uint4(0, 0, 0, 0);
     }
 
     // column sums of g * normed, and gs * normed summed over the row
@@ -415,7 +415,7 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
       const uint32_t xi[4] = {w[c].x, w[c].y, w[c].z, w[c].w};
       const uint32_t gi[4] = {gv.x, gv.y, gv.z, gv.w};
       uint4 av = make_uint4(0, 0, 0, 0);
-      if constexpr (ADD) av = kAddEarly ? ad[kAddEarly ? c : 0] : ld_nc_v4(addend + row * cols + col);
+      if constexpr (ADD) av = kAddEarly ? ad[kAddEarly ? c : 0] : ld_stream_v4(addend + row * cols + col);
       const uint32_t ai[4] = {av.x, av.y, av.z, av.w};
       uint4 o;
       uint32_t* op = &o.x;
@@ -530,7 +530,7 @@ rmsnorm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   grid_wait();
   gamma = loads_below(gamma);              // (in a training step the optimiser's kernel, not far ahead, writes it)
   const bool ok = col < cols;
-  const uint4 w = ok ? ld_nc_v4(x + row * cols + col) : make_uint4(0, 0, 0, 0);
+  const uint4 w = ok ? ld_stream_v4(x + row * cols + col) : make_uint4(0, 0, 0, 0);
   const uint4 gq = ok ? *reinterpret_cast<const uint4*>(gamma + col) : make_uint4(0, 0, 0, 0);
   s_part[warp][lane] = sumsq8(w);
   __syncthreads();

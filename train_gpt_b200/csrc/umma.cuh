@@ -132,9 +132,10 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
   return d;
 }
 
-__device__ __forceinline__ float ldg_f32(const float* ptr) {
+__device__ __forceinline__ float ld_f32(const float* ptr) {
   float v;
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(ptr));   // L1-allocating: an activation scale's line serves 16-32 blocks
+  // L1-allocating: an activation scale's line serves 16-32 blocks.  Coherent, as ld_stream_v4 is and for its reason.
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(ptr));
   return v;
 }
 
