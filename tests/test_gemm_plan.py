@@ -1,0 +1,71 @@
+"""The rule that picks the GEMM's tile width and contraction ranges, on the CPU, against times measured on a B200 with either width
+forced (microseconds of single launches in a graph): the width taken is at most 4 % slower than the other."""
+import ctypes
+
+import pytest
+
+# (what, tokens, K, N, scale per column, us with wide tiles, us with 128-column tiles)
+MEASURED = [
+    ("wgrad", 16, 8192, 8192, 0, 28.8, 31.7),
+    ("wgrad", 64, 8192, 8192, 0, 29.0, 31.9),
+    ("wgrad", 256, 8192, 8192, 0, 37.4, 42.0),
+    ("wgrad", 512, 8192, 8192, 0, 57.8, 62.9),
+    ("wgrad", 16, 2048, 8192, 0, 10.9, 12.3),
+    ("wgrad", 128, 4096, 4096, 0, 10.7, 10.8),
+    ("wgrad", 64, 1024, 4096, 0, 5.8, 4.8),
+    ("wgrad", 256, 2048, 2048, 0, 6.4, 5.3),
+    ("wgrad", 384, 3072, 3072, 0, 10.5, 9.5),
+    ("fwd", 8192, 256, 8192, 0, 31.8, 38.5),
+    ("fwd", 32768, 256, 1024, 0, 18.2, 21.4),
+    ("fwd", 4096, 256, 4096, 0, 11.5, 12.5),
+    ("fwd", 32768, 128, 8192, 0, 107.1, 112.9),
+    ("fwd", 32768, 512, 4096, 0, 84.9, 106.4),
+    ("fwd", 4096, 128, 1024, 0, 4.9, 4.5),
+    ("fwd", 4096, 512, 1024, 0, 6.3, 6.2),
+    ("fwd", 200, 1024, 8192, 0, 7.5, 5.9),
+    ("fwd", 4096, 2048, 4096, 0, 33.4, 41.2),
+    ("fwd", 32768, 128, 8192, 1, 103.7, 116.9),
+    ("fwd", 8192, 256, 8192, 1, 37.6, 42.3),
+    ("fwd", 8192, 512, 8192, 1, 57.9, 62.9),
+    ("fwd", 4096, 512, 1024, 1, 8.7, 6.9),
+    ("fwd", 200, 2048, 8192, 1, 11.9, 9.8),
+    ("dgrad", 8192, 8192, 256, 0, 31.8, 38.6),
+    ("dgrad", 32768, 8192, 128, 1, 103.0, 117.0),
+    ("dgrad", 4096, 1024, 512, 1, 8.7, 6.9),
+]
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from train_gpt_b200 import build, _lib
+    build.build()
+    return _lib.load()
+
+
+def _plan(lib, what, tokens, k, n, columns):
+    from train_gpt_b200 import _lib
+    major, mn = _lib.TG_MAJOR_K, _lib.TG_MAJOR_MN
+    if what == "wgrad":
+        args = _lib.GemmArgs(M=k, N=n, K=tokens, lda=(k + 15) // 16 * 16, ldb=n, a_major=mn, b_major=mn, sb_gran_n=1, ldd=n)
+    elif what == "fwd":
+        args = _lib.GemmArgs(M=tokens, N=n, K=k, lda=k, ldb=n, a_major=major, b_major=mn, sb_gran_n=1 if columns else 128, ldd=n)
+    else:
+        args = _lib.GemmArgs(M=tokens, N=k, K=n, lda=n, ldb=n, a_major=major, b_major=major, sb_gran_n=1 if columns else 128, ldd=k)
+    width, ranges = ctypes.c_int(), ctypes.c_int()
+    assert lib.tgh_gemm_plan(ctypes.byref(args), ctypes.byref(width), ctypes.byref(ranges)) == _lib.TG_OK
+    return width.value, ranges.value
+
+
+@pytest.mark.parametrize("what,tokens,k,n,columns,wide_us,narrow_us", MEASURED)
+def test_takes_the_faster_width(lib, what, tokens, k, n, columns, wide_us, narrow_us):
+    width, ranges = _plan(lib, what, tokens, k, n, columns)
+    assert width in (128, 192, 256) and ranges == 1
+    assert (narrow_us if width == 128 else wide_us) <= 1.04 * min(wide_us, narrow_us), width
+
+
+@pytest.mark.parametrize("what,tokens,k,n,ranges", [("wgrad", 8192, 1024, 1024, 3), ("wgrad", 8192, 1024, 4096, 2), ("wgrad", 8192, 4096, 1024, 2),
+                                                    ("wgrad", 8192, 1024, 3072, 1), ("wgrad", 32768, 1024, 1024, 3),
+                                                    ("fwd", 8192, 1024, 4096, 1), ("dgrad", 1024, 128, 512, 1)])
+def test_a_training_steps_contraction_ranges(lib, what, tokens, k, n, ranges):
+    """The number of ranges shows in the last bit of a weight gradient, so it does not change for whole blocks of tokens."""
+    assert _plan(lib, what, tokens, k, n, 0)[1] == ranges

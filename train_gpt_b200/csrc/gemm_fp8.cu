@@ -44,7 +44,10 @@
 // teardown (TMEM is always freed).
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "common.cuh"
+#include "host_api.h"
 #include "mbarrier.cuh"
 #include "umma.cuh"
 
@@ -837,6 +840,12 @@ splitk_reduce_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, 
 // gradient, whose scales were just written), a tile's set-up and stores, the reduction's launch and its bytes.
 // The model is within 10-15 % of the measurements it was made from; a narrower tile or a cut has to win by 3 %.
 //
+// Contractions of fewer than eight blocks over five waves and more are bound by their stores: a tile then takes at least what its
+// part of the result takes (`stores`, measured on 200 to 32768 rows, 512 to 8192 columns).  Wide against 128-column tiles,
+// microseconds: weight gradient 8192 x 8192 of 64 tokens 29.0 / 31.9, of 256 37.4 / 42.1 and 8192 x 256 -> 8192 31.8 / 38.5 (both took the
+// narrow ones without this term); 4096 x 128 -> 1024, two waves, 4.9 / 4.5.  Over 288 problems of fewer than eight blocks the width
+// taken is 0.2 % slower than the better one on average (2.7 % without the term).
+//
 // The tile width does not show in the result; the number of ranges does, in the last bit of float32 sums, and a training run
 // amplifies that over its steps.  So where the tokens are whole blocks of 128, as a training step's are, the number of
 // ranges is a rule of its own (training_ranges) that the tile width has no part in.
@@ -877,7 +886,9 @@ static GemmPlan plan_gemm(const tg_gemm_args* a) {
       const int64_t waves = (tiles * S + sms - 1) / sms;
       const double block = bn == 256 ? (waves < 3 ? 0.44 : 0.50) : bn == 192 ? 0.47 : !columns ? 0.355 : a->a_major == TG_MAJOR_K ? 0.42 : 0.38;
       const double tile = bn == 128 ? (columns ? 0.5 : 0.1) : 1.0;
-      double us = 3.0 + double(waves) * (block * double((nkb + S - 1) / S) + tile);
+      const double blocks = double((nkb + S - 1) / S);
+      const double stores = nkb >= 8 || waves < 5 ? 0.0 : bn == 256 ? 2.0 : bn == 192 ? 1.4 : columns ? 0.65 + 0.38 * blocks : 0.75 + 0.29 * blocks;
+      double us = 3.0 + double(waves) * std::max(block * blocks + tile, stores);
       if (S > 1) us += 3.5 + double(4 * S + 2) * double(a->M) * double(a->N) / 8.0e6;
       if (best == 0.0 || us < best * 0.97) {
         best = us;
@@ -915,6 +926,15 @@ extern "C" int64_t tg_gemm_workspace_bytes(const tg_gemm_args* a) {
   if (validate_gemm(a) != TG_OK || a->M == 0 || a->N == 0 || a->K == 0) return 0;
   if (skinny_takes(a)) return skinny_workspace_bytes(a);
   return plan_gemm(a).bytes;
+}
+
+extern "C" int tgh_gemm_plan(const tg_gemm_args* a, int* tile_columns, int* ranges) {
+  if (int rc = validate_gemm(a)) return rc;
+  if (a->M == 0 || a->N == 0 || a->K == 0 || skinny_takes(a)) return TG_ERR_TOO_LARGE;
+  const GemmPlan pl = plan_gemm(a);
+  *tile_columns = pl.bn;
+  *ranges = pl.S;
+  return TG_OK;
 }
 
 extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {

@@ -6,6 +6,8 @@
 
 #include <stdint.h>
 
+#include "../../include/train_gpt_b200.h"
+
 #ifdef __cplusplus
 extern "C" {
 #endif
@@ -24,6 +26,10 @@ typedef struct {
 } tgh_quantize_job;
 /* Any number of them: in one launch where they are of block form only (24 a launch) or small and at most six. */
 int tgh_quantize_jobs(const tgh_quantize_job* jobs, int n, void* stream);
+
+/* Columns of the output tiles, and ranges that the contraction is cut into, for a problem that the tiled GEMM takes (TG_ERR_TOO_LARGE:
+ * the few-token kernel does).  Needs no GPU. */
+int tgh_gemm_plan(const tg_gemm_args* args, int* tile_columns, int* ranges);
 
 /* Whether tgh_softcap_ce takes this problem (a row and its cap fit the one-pass kernel). */
 int tgh_softcap_ce_fits(float cap, int64_t rows, int64_t vocab);
