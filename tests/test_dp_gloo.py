@@ -200,3 +200,36 @@ def test_deferred_exchange_waits_for_flush():
         for h in gb._hooks:
             h.remove()
         a.grad = b.grad = None
+
+
+def test_a_slot_counts_once_beside_the_hook():
+    """An op that writes a gradient into its slot returns None to autograd, whose post-accumulate hook fires all the same: only `ready()`
+    counts, so a bucket is exchanged once, when the last of its gradients is in place, not at half of them and again at the end."""
+    from train_gpt_b200.dp import GradBuckets
+
+    class Scale(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x, w):
+            ctx.save_for_backward(x)
+            ctx.w = w
+            return x * w.sum()
+
+        @staticmethod
+        def backward(ctx, g):
+            (x,) = ctx.saved_tensors
+            ctx.w.grad_slot.take().fill_(float((g * x).sum()))
+            ctx.w.grad_slot.ready()
+            return g * ctx.w.detach().sum(), None
+
+    first, a, b, last = torch.nn.Parameter(torch.ones(4)), *(torch.nn.Parameter(torch.ones(2, 2)) for _ in range(2)), torch.nn.Parameter(torch.ones(4))
+    gb = GradBuckets([[first, a, b, last]], world_size=2, average=False)
+    gb.enable_direct([a, b])
+    sent = []
+    gb._exchange = lambda bi: sent.append(gb.flat[bi].clone())
+    for _ in range(2):
+        gb.flat[0].fill_(float("nan"))
+        gb.zero()
+        y = Scale.apply(Scale.apply(first * 1.0, a), b) * last
+        y.sum().backward()
+        gb.finish()
+    assert len(sent) == 2 and all(torch.isfinite(s).all() for s in sent) and torch.equal(sent[0], sent[1])

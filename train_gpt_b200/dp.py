@@ -199,9 +199,10 @@ class GradBuckets:
     def _make_hook(self, bi: int):
         ref = weakref.ref(self)              # a parameter carries the hook and the buckets hold the parameter
 
-        def hook(_param):
+        def hook(param):
+            # (fires for a parameter whose op returned None too: with a slot it is `ready()` that counts)
             owner = ref()
-            if owner is not None:
+            if owner is not None and getattr(param, "grad_slot", None) is None:
                 owner._one_done(bi)
         return hook
 
