@@ -241,6 +241,63 @@ def test_hyper_parameters_and_requires_grad_are_read_at_every_step():
     assert float(a.step(ids.cpu(), tgt)[0]) == float(b.step(ids, tgt)[0])          # ids in host memory
 
 
+@pytest.mark.parametrize("defer", [True, False])
+@pytest.mark.parametrize("layers", [1, 3])
+def test_native_step_exchanges_every_bucket_once_it_is_complete(layers, defer):
+    """The native step's multi-rank path on one GPU: an exchange that stands in for a second rank with the same gradients (the sum is
+    twice the bucket; `finish` then takes half).  Buckets are exchanged in the order and at the points of the backward pass in which the step
+    through autograd exchanges them, with the same contents, each once; and the step is that of a single rank, bit for bit, which it is not
+    where a bucket is exchanged before its last gradient is written, or not before the norm reads it."""
+    from train_gpt_b200.step import SMALL, StepConfig, Trainer, synthetic_batch
+    cfg = StepConfig(**{**SMALL, "n_layers": layers}, defer_exchange=defer)
+
+    def run(world, native):
+        tr = Trainer(cfg, torch.device("cuda", 0), world_size=world, seed=2)
+        log, sent, b = [], [], tr.buckets
+        if not native:
+            tr._program = None
+        elif world > 1:
+            assert tr._program is not None
+
+        def exchange(bi):
+            log.append(bi)
+            sent.append(b.flat[bi].clone())
+            b.flat[bi].mul_(2.0)
+
+        b._exchange = exchange
+        flush = b.flush
+
+        def flush_and_note():
+            log.append("flush")
+            flush()
+
+        b.flush = flush_and_note
+        if native and world > 1:
+            tr._program = tr._native_program()             # takes the callbacks as they are now
+        results = []
+        for i in range(3):
+            log.append("step")
+            results += [float(v) for v in tr.step(*synthetic_batch(cfg, 2, "cuda", seed=i))]
+        return tr, log, sent, results
+
+    one, _, _, want = run(1, True)
+    native, log, sent, got = run(2, True)
+    auto, log_auto, sent_auto, got_auto = run(2, False)
+    assert got == want
+    assert got_auto == want, (log_auto, log)
+    per_step = [e for e in log[:log.index("step", 1)] if isinstance(e, int)]
+    assert per_step == list(range(layers + 2))                # head, layers from the last to the first, embeddings
+    if defer:
+        assert [e for e in log if e != "step"][:3] == ["flush", 0, "flush"]      # the head's goes out before the last layer's attention
+    assert [e for e in log if e != "flush"] == [e for e in log_auto if e != "flush"]
+    if defer:
+        assert log == log_auto
+    assert len(sent) == len(sent_auto) and all(torch.equal(s, t) for s, t in zip(sent, sent_auto))
+    for tr in (native, auto):
+        for s, t in zip(one.model.parameters() + one.opt.state_tensors(), tr.model.parameters() + tr.opt.state_tensors()):
+            assert torch.equal(s, t)
+
+
 def test_native_step_reports_a_token_outside_the_vocabulary():
     """The native step's embedding kernel checks token ids itself: the loss is NaN and the status word says why.  Negative ids
     count from the end, as an index does."""
