@@ -382,3 +382,24 @@ def test_narrow_and_wide_tiles_give_the_same_bits(M, K, N):
         y = ops.gemm_fwd(*ops.quantize_rowwise(x), *wq, tile)
         if ops.last_gemm_kernel_launches == 1:
             assert torch.equal(y, ops.gemm_fwd(*ops.quantize_rowwise(big), *wq, tile)[:M])
+
+
+@pytest.mark.parametrize("shape,n,tile", [((5, 256), 256, (128, 128)), ((130, 384), 512, (128, 128)), ((40, 256), 192, (128, 1)),
+                                          ((2, 7, 256), 100, (128, 1)), ((300, 128), 136, (128, 1)), ((3, 640), 8, (128, 1))])
+def test_forward_returns_the_weight_pair_it_used(shape, n, tile):
+    """`_fp8_forward(return_weight=True)`: the result of the plain call and the quantised pair of the (zero-padded) weight, from one
+    quantisation; contracting with that pair gives the result again."""
+    from train_gpt_b200 import fp8, ops
+    gen = torch.Generator("cuda").manual_seed(n)
+    a = torch.randn(*shape, device="cuda", generator=gen).to(torch.bfloat16)
+    b = (torch.randn(shape[-1], n, device="cuda", generator=gen) * 0.02).to(torch.bfloat16)
+    want = fp8._fp8_forward(a, b, weight_tile=tile)
+    y, (w_q, w_s) = fp8._fp8_forward(a, b, weight_tile=tile, return_weight=True)
+    assert y.shape == want.shape and torch.equal(y, want)
+    padded = torch.nn.functional.pad(b, (0, -n % 16)) if tile == (128, 1) else b
+    q, s = fp8.quantize_weight(padded, tile)
+    assert torch.equal(w_q.view(torch.uint8), q.view(torch.uint8)) and torch.equal(w_s, s)
+    again = ops.gemm_fwd(*ops.quantize_rowwise(a.reshape(-1, shape[-1])), w_q, w_s, tile)
+    assert torch.equal(again[:, :n].reshape(y.shape), y)
+    with pytest.raises(ValueError):
+        fp8._fp8_forward(a, b[:-1], weight_tile=tile, return_weight=True)

@@ -486,8 +486,9 @@ struct ForwardOut {
 };
 
 // fp8.py:50-78.  row_q / row_s: the activation's row form made earlier.  keep_x / keep_w: what the backward pass will want
-// of the activation (its column form, from the same read) and of the weight outlives the call.
-ForwardOut fp8_forward(const Tensor& a, const Tensor& b_, bool w_cols, const Tensor& row_q, const Tensor& row_s, bool keep_x, bool keep_w) {
+// of the activation (its column form, from the same read) and of the weight outlives the call.  weight: receives the quantised weight.
+ForwardOut fp8_forward(const Tensor& a, const Tensor& b_, bool w_cols, const Tensor& row_q, const Tensor& row_s, bool keep_x, bool keep_w,
+                       Pair* weight = nullptr) {
   ForwardOut o;
   const int64_t k = a.size(-1), n = b_.size(1), m = rows_of(a);
   Tensor x;
@@ -514,7 +515,7 @@ ForwardOut fp8_forward(const Tensor& a, const Tensor& b_, bool w_cols, const Ten
     x_row_at = add_row(temp, m, k);
     if (keep_x) x_col_at = add_col(kept, m, k);
   }
-  w_at = w_cols ? add_col(temp, k, np) : add_block(keep_w ? kept : temp, k, n);
+  if (weight == nullptr) w_at = w_cols ? add_col(temp, k, np) : add_block(keep_w ? kept : temp, k, n);
   const size_t ws_at = temp.add(ws_bytes);
   kept.make(b);
   temp.make(b);
@@ -527,7 +528,13 @@ ForwardOut fp8_forward(const Tensor& a, const Tensor& b_, bool w_cols, const Ten
     if (keep_x) want_col(j, o.x_col = x_col_at.in(kept), k);
   }
   tgh_quantize_job& j = jobs[n_jobs++] = job_of(b);
-  Form w = w_at.in(!w_cols && keep_w ? kept : temp);
+  Form w;
+  if (weight != nullptr) {
+    *weight = {empty({k, np}, kF8, b), empty({k / kTile, w_cols ? np : n / kTile}, at::kFloat, b)};
+    w = {ptr(weight->first), fptr(weight->second)};
+  } else {
+    w = w_at.in(!w_cols && keep_w ? kept : temp);
+  }
   if (w_cols) want_col(j, w, np);
   else want_block(j, w);
   check(api.tgh_quantize_jobs(jobs, n_jobs, cur_stream()), "tgh_quantize_jobs");
@@ -963,10 +970,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return gemm_wgrad(xq, xs, gq, gs, g_cols, f32 ? at::kFloat : at::kBFloat16, or_none(status), or_none(out));
   });
   m.def("fp8_forward", [](const Tensor& a, const Tensor& b, int64_t block_k, bool w_cols, const std::optional<Tensor>& row_q,
-                          const std::optional<Tensor>& row_s) {
+                          const std::optional<Tensor>& row_s, bool return_weight) -> py::object {
     const Linear d = validate(a, b, block_k);
     const auto [rq, rs] = row_form(or_none(row_q), or_none(row_s), d.k);
-    return fp8_forward(a, b, w_cols, rq, rs, false, false).y;
+    Pair weight;
+    const Tensor y = fp8_forward(a, b, w_cols, rq, rs, false, false, return_weight ? &weight : nullptr).y;
+    return return_weight ? py::object(py::make_tuple(y, weight)) : py::cast(y);
   });
   m.def("fp8_backward", [](const Tensor& a, const Tensor& b, const Tensor& g, bool w_cols, int mode, const py::object& activation,
                            const std::optional<Tensor>& w_q, const std::optional<Tensor>& w_s, const py::object& slot) {

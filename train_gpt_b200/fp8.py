@@ -111,9 +111,16 @@ def _row_form(a_quantized):
 def _fp8_forward(a, b, block_k=DEFAULT_BLOCK_K, weight_tile=(128, 1), a_quantized=None, return_weight=False):
     """fp8.py:50-78.  `a_quantized` = (q, scales) of `a` made earlier (e.g. by the fused
     norm+quantise kernel) skips the activation quantiser.  return_weight=True also returns the
-    quantised weight pair (128x128 tiles serve the backward's dgrad unchanged)."""
-    y = ops._host().fp8_forward(a, b, block_k, _per_column(weight_tile), *_row_form(a_quantized))
-    return (y, quantize_weight(_as_bf16(b, "b"), weight_tile)) if return_weight else y
+    quantised weight pair that the GEMM read (128x128 tiles serve the backward's dgrad unchanged; with 128x1
+    tiles it has the columns up to the next multiple of 16)."""
+    columns, row = _per_column(weight_tile), _row_form(a_quantized)
+    n = b.shape[-1]
+    if not return_weight or not columns or n % 16 == 0:
+        return ops._host().fp8_forward(a, b, block_k, columns, *row, return_weight)
+    b = torch.nn.functional.pad(_as_bf16(b, "b"), (0, -n % 16))          # the columns that the pair has and the result has not
+    y, weight = ops._host().fp8_forward(a, b, block_k, columns, *row, True)
+    y = y[..., :n]
+    return (y if y.dim() == 2 else y.contiguous()), weight
 
 
 def _fp8_backward(block_k, residuals, g, weight_tile=(128, 1), mode="bf16_ste", a_quantized=None, w_quantized=None,
