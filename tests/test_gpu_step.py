@@ -333,3 +333,30 @@ def test_embedding_gradient_adds_as_an_accumulating_index_put(tokens, d, vocab, 
                            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
     assert rc == 0
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("tokens,d,vocab", [(4, 8, 1), (5, 8, 1), (31, 56, 1), (28, 56, 1), (29, 56, 1), (32, 64, 1), (33, 64, 1), (300, 264, 9), (2000, 520, 61),
+                                            (4099, 1024, 50304), (3001, 2048, 1500), (20000, 128, 600)])
+def test_embedding_gradient_of_listed_and_of_frequent_ids(tokens, d, vocab):
+    """Ids with as many tokens as a row's list holds (32, or half the row's width), one fewer and one more, and mixtures.  (Rows of 8 values
+    torch adds another way: there the sum is written out.)"""
+    from train_gpt_b200 import _lib
+    lib = _lib.load()
+    gen = torch.Generator("cuda").manual_seed(tokens + d)
+    for turn in range(2):
+        ids = torch.randint(0, vocab, (tokens,), device="cuda", generator=gen)
+        if turn == 1 and vocab > 1:
+            ids[torch.rand(tokens, device="cuda", generator=gen) < 0.2] = vocab - 1
+            ids[-1] -= vocab
+        dx = torch.randn(tokens, d, device="cuda", generator=gen).to(torch.bfloat16)
+        want = torch.zeros(vocab, d, dtype=torch.bfloat16, device="cuda")
+        if d > 8:
+            want.index_put_((ids,), dx, accumulate=True)
+        else:
+            for i, t in zip(ids.tolist(), dx):
+                want[i] += t
+        got = torch.full((vocab, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        table = torch.empty(vocab * 8, dtype=torch.uint8, device="cuda")
+        assert lib.tgh_embed_bwd(*(ctypes.c_void_p(t.data_ptr()) for t in (ids, dx, got, table)), *(ctypes.c_int64(n) for n in (tokens, d, vocab)),
+                                 ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        assert torch.equal(got, want)
