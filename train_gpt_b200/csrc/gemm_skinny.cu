@@ -26,7 +26,11 @@
 namespace tg {
 
 // From 129 tokens on the tokens fill 128 MMA rows themselves, a token scale is a thread's own number instead of a column's,
-// and the tiled kernel is the faster one (200 x 2048 x 8192: 13.5 us against 17 for this kernel with 256 columns).
+// and the tiled kernel is the faster one: 200 tokens, tiled / this kernel with 256 columns, a scale per 128 weight columns (per
+// column): 2048 x 8192 8.6 / 14.1 us (10.1 / 13.7), 4096 x 4096 12.0 / 16.2 (14.1 / 15.7), 8192 x 8192 25.0 / 40.4 (37.4 / 37.3).
+// Below, both sides with the weight from memory, this kernel / tiled: 64 tokens 8192 x 8192 16.3 / 18.0 (16.7 / 20.9), 4096 x 4096
+// 9.2 / 9.4 (9.4 / 11.0); 100 tokens 20.2 / 18.7 (20.5 / 22.0), 10.7 / 9.8 (10.9 / 11.5), 2048 x 8192 9.7 / 8.3 (9.8 / 11.7).  So with a
+// scale per 128 columns the line would be better drawn at 64.
 constexpr int kSkinnyMaxTokens = 128;
 
 template <int BN_>
