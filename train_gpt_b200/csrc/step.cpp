@@ -3,7 +3,8 @@
 // native program instead of some 150 autograd nodes and tensor operations in Python.
 //
 // It launches the same kernels on the same operands in the same order as the model does through autograd, so its results
-// are bit-identical (tests/test_gpu_step.py compares the two); what it saves is what autograd cannot see:
+// are bit-identical to that path's (tests/test_gpu_step.py compares the two, and a trajectory recorded with the step launched
+// operation by operation).  What it saves is what autograd cannot see:
 //   * host time: a launch costs 2-4 us here, 15-25 us through Python -- train-gpt's small model spent 3.4 ms per step on
 //     0.45 ms of kernels;
 //   * launches: every weight of the model is quantised in one, a backward step's quantisers (upstream gradients and the
