@@ -293,7 +293,8 @@ __device__ __forceinline__ float amax8(const uint4& w, float m = 0.f) {
 // Sixteen bytes that pass through once.  A coherent load, although the data is constant while the kernel works: a kernel launched early
 // (below) may begin before its input is written, and what the non-coherent path holds of the address -- from an earlier kernel that
 // read the same scratch, say -- need not be what was written since.  The two are equally fast (32768 x 2048 norm forward
-// and backward 113.7 us non-coherent, 113.9 so; decoder layer of 32768 tokens 6880 and 6863 us).
+// and backward 113.7 us non-coherent, 113.9 so; decoder layer of 32768 tokens 6880 and 6863 us) as long as a loop's loads do not
+// follow its stores: those keep their order (see the addend of the norm backward).
 __device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
   uint4 r;
   asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"

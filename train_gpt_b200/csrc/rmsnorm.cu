@@ -328,6 +328,9 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
 
   const int64_t stride = int64_t(gridDim.x) * RPB;
   int64_t row = int64_t(blockIdx.x) * RPB + warp / WPR;
+  // the addend's row, for which shared memory has no room, comes as far as the L2 (GB/s at 32768 rows without -> with it: 2048
+  // columns 5860 -> 6000, 1280 5390 -> 5520, 512 4570 -> 4650; 1024 5480 -> 5400)
+  constexpr bool kFetchAddend = ADD && NCHUNK != 4;
   auto prefetch = [&](int64_t r, int slot) {
     if (r < rows) {
       const uint32_t dst = slot0 + uint32_t(slot) * 2u * kRowBytes;
@@ -338,6 +341,10 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
           cp_async16(dst + c * 512, x + r * cols + col);
           cp_async16(dst + kRowBytes + c * 512, g + r * cols + col);
         }
+      }
+      if (kFetchAddend) {
+        const int col = col_base + lane * 56;                            // a line of 128 bytes per lane
+        if (lane < NCHUNK * 4 && col < cols) asm volatile("prefetch.global.L2 [%0];" ::"l"(addend + r * cols + col) : "memory");
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");   // an empty group keeps the wait count uniform
@@ -364,14 +371,17 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
     const float rn = __frsqrt_rn(__fdiv_rn(ss, float(cols)) + eps);
     const float2 rn2 = make_float2(rn, rn);
 
-    // (ADD) the addend's pieces are fetched here, ahead of the pass that uses them, when the row is
-    // narrow enough for the registers; wider rows fetch them where they are used
-    constexpr bool kAddEarly = ADD && NCHUNK <= 4;
-    uint4 ad[kAddEarly ? NCHUNK : 1];
-    if constexpr (kAddEarly) {
+    // (ADD) the addend's first pieces are fetched here, ahead of the pass that uses them, as many as there are registers for;
+    // the rest that many pieces ahead of their use, and always before a store: dx may alias the addend, so a load that
+    // follows a store in the program waits its turn (32768 x 2048: 90 us, and 165 with each piece fetched where it is used)
+    constexpr int kAhead = !ADD ? 1 : NCHUNK < 4 ? NCHUNK : 4;
+    uint4 ad[kAhead];
+    auto fetch_addend = [&](int c) {
+      return FULL || col_base + c * 256 < cols ? ld_stream_v4(addend + row * cols + col_base + c * 256) : make_uint4(0, 0, 0, 0);
+    };
+    if constexpr (ADD) {
 #pragma unroll
-      for (int c = 0; c < NCHUNK; ++c)
-        ad[c] = (FULL || col_base + c * 256 < cols) ? ld_stream_v4(addend + row * cols + col_base + c * 256) : make_uint4(0, 0, 0, 0);
+      for (int c = 0; c < kAhead; ++c) ad[c] = fetch_addend(c);
     }
 
     // column sums of g * normed, and gs * normed summed over the row
@@ -415,7 +425,10 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
       const uint32_t xi[4] = {w[c].x, w[c].y, w[c].z, w[c].w};
       const uint32_t gi[4] = {gv.x, gv.y, gv.z, gv.w};
       uint4 av = make_uint4(0, 0, 0, 0);
-      if constexpr (ADD) av = kAddEarly ? ad[kAddEarly ? c : 0] : ld_stream_v4(addend + row * cols + col);
+      if constexpr (ADD) {
+        av = ad[c % kAhead];
+        if (c + kAhead < NCHUNK) ad[c % kAhead] = fetch_addend(c + kAhead);
+      }
       const uint32_t ai[4] = {av.x, av.y, av.z, av.w};
       uint4 o;
       uint32_t* op = &o.x;
@@ -466,7 +479,7 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
 // Column sums of the per-block partials.  A thread block owns 32 columns.  The order of additions is fixed by (n_blocks, cols)
 // alone: row class w = b mod 8 has four sums, the i-th over b = w + 8 i, w + 8 i + 32, ..., the rows left over when a class's
 // groups of four are complete go to its first; the four are added in pairs, the eight classes in order.  Warp w + 8 i keeps the i-th
-// sum of class w and has all of its (at most eight) loads in flight at once: with eight warps of four sums each the kernel was
+// sum of class w and has all of its (at most seven) loads in flight at once: with eight warps of four sums each the kernel was
 // a chain of five L2 round trips, 5.2 us at 2048 columns.
 __global__ void __launch_bounds__(1024)
 rmsnorm_dgamma_reduce_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dgamma,
@@ -481,21 +494,17 @@ rmsnorm_dgamma_reduce_kernel(const float* __restrict__ partial, __nv_bfloat16* _
     const int w = warp & 7;
     const int groups = n_blocks >= w + 25 ? (n_blocks - w - 25) / 32 + 1 : 0;      // complete groups of four rows of class w
     const float* p = partial + int64_t(warp) * cols + col;
-    for (int k = 0; k < groups; k += 5) {
-      float v[5];
+    const int b = w + 32 * groups;                                                  // at most three rows are left
+    float v[4], u[3];
 #pragma unroll
-      for (int i = 0; i < 5; ++i) v[i] = k + i < groups ? __ldcg(p + int64_t(k + i) * 32 * cols) : 0.f;
+    for (int i = 0; i < 4; ++i) v[i] = i < groups ? __ldcg(p + int64_t(i) * 32 * cols) : 0.f;
 #pragma unroll
-      for (int i = 0; i < 5; ++i) t += v[i];                                        // (x + 0 is x)
-    }
-    if (warp < 8) {
-      float v[3];
-      const int b = w + 32 * groups;                                                // at most three rows are left
+    for (int i = 0; i < 3; ++i) u[i] = warp < 8 && b + 8 * i < n_blocks ? __ldcg(partial + int64_t(b + 8 * i) * cols + col) : 0.f;
 #pragma unroll
-      for (int i = 0; i < 3; ++i) v[i] = b + 8 * i < n_blocks ? __ldcg(partial + int64_t(b + 8 * i) * cols + col) : 0.f;
+    for (int i = 0; i < 4; ++i) t += v[i];                                          // (x + 0 is x)
+    for (int k = 4; k < groups; ++k) t += __ldcg(p + int64_t(k) * 32 * cols);       // (a GPU of more than 160 SMs)
 #pragma unroll
-      for (int i = 0; i < 3; ++i) t += v[i];
-    }
+    for (int i = 0; i < 3; ++i) t += u[i];
   }
   s_part[warp][lane] = t;
   __syncthreads();

@@ -24,7 +24,7 @@ import time
 
 import torch
 
-from . import fp8, ops
+from . import fp8, losses, ops
 
 L2_BYTES = 126e6
 
@@ -134,12 +134,17 @@ def bench_quant(rows, cols, warmup, iters, acts=True):
 
 
 def bench_loss(rows, vocab, warmup, iters):
-    """Capped-logit cross-entropy: forward reads the logits and writes the tanh values (4 B per
-    element), backward rewrites them as the gradient in place (4 B per element)."""
+    """Capped-logit cross-entropy.  One pass: the logits are read and their gradient written (4 B per element).  As two
+    kernels: the forward writes the tanh values (4 B), the backward rewrites them as the gradient in place (4 B)."""
     E = rows * vocab
     g = torch.Generator(device="cuda").manual_seed(0)
     xs = [(torch.randn(rows, vocab, device="cuda", generator=g) * 4).to(torch.bfloat16) for _ in range(2)]
     tg = torch.randint(0, vocab, (rows,), device="cuda", generator=g).to(torch.int32)
+    ls = [x.detach().requires_grad_() for x in xs]
+    m, b = _time(lambda i: losses.capped_cross_entropy(ls[i], tg, 15.0), 2, warmup, iters)
+    _report("capped_cross_entropy (loss and gradient)", m, b, bytes_=4.0 * E + 8 * rows, shape=[rows, vocab])
+    if vocab % 8:
+        return
     m, b = _time(lambda i: ops.softcap_ce_fwd(xs[i], tg, 15.0), 2, warmup, iters)
     _report("softcap_ce_fwd", m, b, bytes_=4.0 * E + 12 * rows, shape=[rows, vocab])
     _, lse, th = ops.softcap_ce_fwd(xs[0], tg, 15.0)
