@@ -239,6 +239,14 @@ def test_hyper_parameters_and_requires_grad_are_read_at_every_step():
             assert torch.equal(s, t), change
     ids, tgt = synthetic_batch(cfg, 2, "cuda", seed=0)
     assert float(a.step(ids.cpu(), tgt)[0]) == float(b.step(ids, tgt)[0])          # ids in host memory
+    # a gradient hook on a parameter sees, and may change, its gradient
+    seen = []
+    hooks = [tr.model.embed.register_hook(lambda g: seen.append(1) or 2 * g) for tr in (a, b)]
+    ids, tgt = synthetic_batch(cfg, 2, "cuda", seed=9)
+    assert float(a.step(ids, tgt)[1]) == float(b.step(ids, tgt)[1]) and len(seen) == 2
+    for h in hooks:
+        h.remove()
+    assert float(a.step(ids, tgt)[1]) == float(b.step(ids, tgt)[1]) and len(seen) == 2
 
 
 @pytest.mark.parametrize("defer", [True, False])

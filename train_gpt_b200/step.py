@@ -391,7 +391,8 @@ class Trainer:
     With the default switches the step itself is a native program (csrc/step.cpp) that launches what the
     model would through autograd, bit for bit: launched one by one a step of the small model takes 334 us,
     replayed 290, where launches through Python took 3500.  An eager step reads `opt.lr` and the other
-    hyper-parameters every time; while a parameter does not require a gradient it goes through autograd.
+    hyper-parameters every time; while a parameter does not require a gradient, or has a gradient hook, it goes
+    through autograd.
     Capture needs two eager warm-up steps; parameters and optimizer
     state are restored after them, so a captured run follows the same trajectory as an eager one.
     """
@@ -468,8 +469,9 @@ class Trainer:
             b.bucket_done if many else None, b.flush if many else None, b.finish if many else None)
 
     def _eager_step(self, ids, targets):
-        # the native program computes every gradient, so it runs only while every parameter wants one
-        if self._program is not None and all(p.requires_grad for p in self._params):
+        # the native program computes every gradient and hands none to autograd, so it runs only while every parameter wants one
+        # and none has a hook that expects to see it
+        if self._program is not None and all(p.requires_grad and not p._backward_hooks for p in self._params):
             o = self.opt                          # read at every step: a schedule changes them
             return self._program.step(ids, targets, o.lr, o.b1, o.b2, o.eps, o.wd, o.clip)
         self.buckets.zero()
