@@ -172,7 +172,8 @@ def test_one_pass_gradient_has_the_bits_of_the_two_kernels(rows, vocab):
     assert torch.equal(a.grad, ops.softcap_ce_bwd(th, tt, lse, None, 15.0))
 
 
-@pytest.mark.parametrize("rows,vocab", [(128, 256), (1000, 512), (1024, 256), (3001, 264), (8192, 2056)])
+@pytest.mark.parametrize("rows,vocab", [(1, 256), (2, 8), (3, 40), (31, 8), (100, 64), (127, 16), (128, 256), (130, 8), (255, 8), (511, 24), (1000, 512),
+                                        (1024, 256), (2047, 8), (3001, 264), (8192, 2056), (32769, 16), (65536, 8), (70001, 8)])
 def test_loss_has_the_bits_of_the_mean_over_tokens(rows, vocab):
     """The loss is the mean that torch takes of the rows' values (which have the bits of the separate forward kernel's)."""
     from train_gpt_b200 import losses, ops

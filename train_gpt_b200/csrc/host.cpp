@@ -878,7 +878,7 @@ Tensor capped_cross_entropy(const Tensor& logits_, const Tensor& target_ids, dou
       check(api.tgh_softcap_ce(ptr(logits), ptr(t), t.scalar_type() == at::kLong, float(cap), ptr(d), nullptr, 0, fptr(nll), rows, vocab,
                                vocab, cur_stream()),
             "tgh_softcap_ce");
-      loss = nll.mean();                                                             // losses.py:12
+      loss = mean_of(nll);
     }
     if (!track) return loss;
     std::shared_ptr<CappedCEBackward> node(new CappedCEBackward(), torch::autograd::deleteNode);

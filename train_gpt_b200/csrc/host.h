@@ -35,7 +35,7 @@ constexpr auto kF8 = at::kFloat8_e4m3fn;
   X(tg_act_quantize_rowcol) X(tg_quantize_block128) X(tg_rmsnorm_fwd) X(tg_rmsnorm_quant_fwd)                       \
   X(tg_add_rmsnorm_quant_fwd) X(tg_rmsnorm_bwd_scratch_bytes) X(tg_rmsnorm_bwd) X(tg_rmsnorm_bwd_add)               \
   X(tg_softcap_ce_fwd) X(tg_softcap_ce_bwd) X(tg_sumsq_scratch_bytes) X(tg_sumsq_bf16) X(tg_adamw_bf16)             \
-  X(tg_gemm_workspace_bytes) X(tg_gemm_fp8_blockscaled) X(tgh_quantize_jobs) X(tgh_softcap_ce_fits) X(tgh_softcap_ce) \
+  X(tg_gemm_workspace_bytes) X(tg_gemm_fp8_blockscaled) X(tgh_quantize_jobs) X(tgh_softcap_ce_fits) X(tgh_softcap_ce) X(tgh_mean) \
   X(tgh_global_norm_scratch_bytes) X(tgh_global_norm) X(tgh_adamw) X(tgh_embed) X(tgh_embed_bwd)
 
 struct Api {
@@ -102,6 +102,14 @@ inline std::vector<int64_t> with_last(const Tensor& x, int64_t last) {
   std::vector<int64_t> s(x.sizes().begin(), x.sizes().end());
   s.back() = last;
   return s;
+}
+
+// losses.py:12: the mean of the tokens' values
+inline Tensor mean_of(const Tensor& nll) {
+  if (nll.numel() > 65536) return nll.mean();
+  const Tensor m = empty({}, at::kFloat, nll);
+  check(api.tgh_mean(fptr(nll), nll.numel(), fptr(m), cur_stream()), "tgh_mean");
+  return m;
 }
 
 // The word a GEMM reports an expired device wait in, one per device (-1: the current one), made once.

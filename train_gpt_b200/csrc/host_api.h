@@ -42,6 +42,9 @@ int tgh_softcap_ce_fits(float cap, int64_t rows, int64_t vocab);
 int tgh_softcap_ce(const void* logits, const void* targets, int targets_64, float cap, void* dlogits, const float* gscale,
                    int only_if_scaled, float* nll, int64_t rows, int64_t vocab, int64_t ld, void* stream);
 
+/* The mean of n floats (16-byte aligned) with the bits of torch's; n up to 65536, TG_ERR_TOO_LARGE beyond. */
+int tgh_mean(const float* v, int64_t n, float* out, void* stream);
+
 /* x[b, t, :] = bf16(embed[ids[b, t]] + pos[t]) (train-gpt model.py:83).  Negative ids count from the end; one outside the
  * vocabulary stores TGH_STATUS_TOKEN in *status and makes its row NaN. */
 enum { TGH_STATUS_TOKEN = 16 };
