@@ -93,13 +93,13 @@ struct Hyper {
 class StepProgram {
  public:
   // Parameters and, in the same structure, the slices of the flat gradient tensors; `flat`: per bucket the flat parameters,
-  // gradients and moments; count: int32 (2,), see tgh_adamw.  on_bucket(i) / on_attention() / on_end(), or None: a bucket's
+  // gradients and moments; params: all parameters, as autograd knows them; count: int32 (2,), see tgh_adamw.  on_bucket(i) / on_attention() / on_end(), or None: a bucket's
   // gradients are complete / an attention backward is about to be launched / the backward pass is over.
   StepProgram(Config c, Tensor embed, Tensor pos, Tensor final_norm, Tensor unembed, std::vector<std::vector<Tensor>> layers,
               Tensor g_embed, Tensor g_pos, Tensor g_final_norm, Tensor g_unembed, std::vector<std::vector<Tensor>> g_layers,
-              std::vector<std::vector<Tensor>> flat, Tensor count, py::object on_bucket, py::object on_attention, py::object on_end)
+              std::vector<std::vector<Tensor>> flat, std::vector<Tensor> params, Tensor count, py::object on_bucket, py::object on_attention, py::object on_end)
       : c_(c), embed_(embed), pos_(pos), final_norm_(final_norm), unembed_(unembed), g_embed_(g_embed), g_pos_(g_pos),
-        g_final_norm_(g_final_norm), g_unembed_(g_unembed), count_(count), on_bucket_(on_bucket), on_attention_(on_attention),
+        g_final_norm_(g_final_norm), g_unembed_(g_unembed), count_(count), params_(std::move(params)), on_bucket_(on_bucket), on_attention_(on_attention),
         on_end_(on_end) {
     auto layer = [](const std::vector<Tensor>& t) { return LayerTensors{t.at(0), t.at(1), t.at(2), t.at(3), t.at(4), t.at(5)}; };
     for (const auto& t : layers) layers_.push_back(layer(t));
@@ -113,6 +113,14 @@ class StepProgram {
     hd_ = c.heads * c.head_dim;
     ff_ = layers_.empty() ? 0 : layers_[0].w_up.size(1);
     norm_scratch_ = at::zeros({api.tgh_global_norm_scratch_bytes(int(flat_.size()))}, embed.options().dtype(at::kByte));
+  }
+
+  // Whether this step may run here: every gradient is computed and none handed to autograd, so only while every parameter wants one and
+  // none has a hook that expects to see it.
+  bool applies() const {
+    for (const Tensor& p : params_)
+      if (!p.requires_grad() || !torch::autograd::impl::hooks(p).empty()) return false;
+    return true;
   }
 
   // (loss, global gradient norm); the loss is NaN if a GEMM gave up on a device wait.  The hyper-parameters come with every step: a
@@ -162,7 +170,7 @@ class StepProgram {
     check(api.tgh_softcap_ce(ptr(logits), ptr(targets), targets.scalar_type() == at::kLong, float(c_.cap), ptr(dlogits), nullptr, 0,
                              fptr(nll), m_, vocab_, vocab_, cur_stream()),
           "tgh_softcap_ce");
-    const Tensor loss = nll.mean();
+    const Tensor loss = mean_of(nll);
     logits = Tensor();
     // ---- backward
     at::mm_out(g_unembed_, hf.t(), dlogits);
@@ -403,6 +411,7 @@ class StepProgram {
 
   Config c_;
   Tensor embed_, pos_, final_norm_, unembed_, g_embed_, g_pos_, g_final_norm_, g_unembed_, count_, norm_scratch_;
+  std::vector<Tensor> params_;
   std::vector<LayerTensors> layers_, grads_;
   std::vector<std::vector<Tensor>> flat_;
   py::object on_bucket_, on_attention_, on_end_;
@@ -423,13 +432,14 @@ void tgh::register_step(py::module_& m) {
   py::class_<StepProgram>(m, "StepProgram")
       .def(py::init([](std::tuple<int64_t, int64_t, double, double, int, int> c, Tensor embed, Tensor pos, Tensor final_norm, Tensor unembed, std::vector<std::vector<Tensor>> layers, Tensor g_embed,
                        Tensor g_pos, Tensor g_final_norm, Tensor g_unembed, std::vector<std::vector<Tensor>> g_layers,
-                       std::vector<std::vector<Tensor>> flat, Tensor count, py::object on_bucket, py::object on_attention, py::object on_end) {
+                       std::vector<std::vector<Tensor>> flat, std::vector<Tensor> params, Tensor count, py::object on_bucket, py::object on_attention,
+                       py::object on_end) {
         const auto [heads, head_dim, eps, cap, act, act_bwd] = c;
         return std::make_unique<StepProgram>(Config{heads, head_dim, eps, cap, act, act_bwd}, embed, pos,
-                                             final_norm, unembed, layers, g_embed, g_pos, g_final_norm, g_unembed, g_layers, flat, count,
+                                             final_norm, unembed, layers, g_embed, g_pos, g_final_norm, g_unembed, g_layers, flat, params, count,
                                              on_bucket, on_attention, on_end);
       }))
       .def("step", [](StepProgram& p, const Tensor& ids, const Tensor& targets, double lr, double b1, double b2, double eps, double weight_decay,
-                      double clip) { return p.step(ids, targets, Hyper{lr, b1, b2, eps, weight_decay, clip}); });
+                      double clip) { return p.applies() ? std::optional(p.step(ids, targets, Hyper{lr, b1, b2, eps, weight_decay, clip})) : std::nullopt; });
   m.def("softcap_ce_fits", [](double cap, int64_t rows, int64_t vocab) { return bool(api.tgh_softcap_ce_fits(float(cap), rows, vocab)); });
 }

@@ -389,8 +389,8 @@ class Trainer:
     fixed device buffers before each replay; the returned loss and gradient norm are the graph's own
     output tensors (read them before the next step), and the hyper-parameters are those of the capture.
     With the default switches the step itself is a native program (csrc/step.cpp) that launches what the
-    model would through autograd, bit for bit: launched one by one a step of the small model takes 334 us,
-    replayed 290, where launches through Python took 3500.  An eager step reads `opt.lr` and the other
+    model would through autograd, bit for bit: launched one by one a step of the small model takes 347 us,
+    replayed 285, where launches through Python took 3500.  An eager step reads `opt.lr` and the other
     hyper-parameters every time; while a parameter does not require a gradient, or has a gradient hook, it goes
     through autograd.
     Capture needs two eager warm-up steps; parameters and optimizer
@@ -465,15 +465,15 @@ class Trainer:
         return host.StepProgram(
             (c.n_heads, c.head_dim, c.rms_eps, c.logit_cap, TG_ACT[c.activation], TG_ACT[c.activation + "_bwd"]),
             m.embed, m.pos, m.final_norm, m.unembed, layers, grads[id(m.embed)], grads[id(m.pos)], grads[id(m.final_norm)],
-            grads[id(m.unembed)], g_layers, [list(f) for f in self.opt._flat], self.opt._count,
+            grads[id(m.unembed)], g_layers, [list(f) for f in self.opt._flat], self._params, self.opt._count,
             b.bucket_done if many else None, b.flush if many else None, b.finish if many else None)
 
     def _eager_step(self, ids, targets):
-        # the native program computes every gradient and hands none to autograd, so it runs only while every parameter wants one
-        # and none has a hook that expects to see it
-        if self._program is not None and all(p.requires_grad and not p._backward_hooks for p in self._params):
+        if self._program is not None:
             o = self.opt                          # read at every step: a schedule changes them
-            return self._program.step(ids, targets, o.lr, o.b1, o.b2, o.eps, o.wd, o.clip)
+            out = self._program.step(ids, targets, o.lr, o.b1, o.b2, o.eps, o.wd, o.clip)
+            if out is not None:                   # (None: a parameter is frozen or has a gradient hook)
+                return out
         self.buckets.zero()
         loss = self.model.loss(ids, targets)
         loss.backward()
