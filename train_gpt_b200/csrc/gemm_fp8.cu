@@ -47,6 +47,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "gemm_tiles.cuh"
 #include "host_api.h"
 #include "mbarrier.cuh"
 #include "umma.cuh"
@@ -133,126 +134,7 @@ struct Cfg {
   static_assert(smem_bytes + static_reserve <= kSmemLimit, "shared-memory plan exceeds the 227 KB a CTA may use");
 };
 
-struct GemmParams {
-  const float* sa;
-  long long sa_sm, sa_sk;
-  const float* sb;
-  long long sb_sn, sb_sk;
-  void* d;              // output, row pitch ldd elements
-  long long ldd;
-  int M, N, nkb;        // nkb = contraction blocks per work item (all of them unless the contraction is split)
-  int nkb_rem;          // ... plus one for the first nkb_rem ranges of a split contraction (ranges need not be equal)
-  int a_mn, b_mn;       // 1 = MN-major storage
-  int tiles_m, tiles_n;
-  int band;             // tile rows per band of the tile numbering
-  // ceil(2^40 / d) for the three divisors of the item -> tile arithmetic (tiles per contraction range,
-  // tiles per band, rows of the last band), 0 = divide the slow way (the exactness bound x * d < 2^40
-  // does not hold); rows of a full band = `band`, its reciprocal in mg_band
-  unsigned long long mg_tiles, mg_per_band, mg_band, mg_last;
-  int ksplit;           // the contraction is cut into this many ranges; range s of a tile is its own
-                        // work item and writes its float32 partial sums to d + s * slice_elems
-  long long slice_elems;
-  unsigned* status;
-};
-
-// Staging stores of the epilogue, address = (base + OFF) ^ flip with OFF a compile-time constant.
-// The address is formed inside the asm block so that the compiler cannot hoist one register per
-// store out of the unrolled loops: the accumulators leave no room for that (it spilled loop
-// invariants of the mainloop instead).  `base` has bits 4-6 clear or small enough that adding OFF
-// never carries past bit 6, so the xor is the 128-byte swizzle of the 16-byte chunk index.
-template <int OFF>
-__device__ __forceinline__ void sts_swz_b32(uint32_t base, uint32_t flip, uint32_t x) {
-  asm volatile("{\n\t.reg .b32 t;\n\tadd.u32 t, %0, %1;\n\txor.b32 t, t, %2;\n\tst.shared.b32 [t], %3;\n\t}"
-               ::"r"(base), "n"(OFF), "r"(flip), "r"(x) : "memory");
-}
-// (float operands are passed as floats: routing accumulator halves through integer registers kept
-// ptxas from leaving them in their packed pairs and cost ~25 spilled registers)
-template <int OFF>
-__device__ __forceinline__ void sts_swz_f32x2(uint32_t base, uint32_t flip, float2 v) {
-  asm volatile("{\n\t.reg .b32 t;\n\tadd.u32 t, %0, %1;\n\txor.b32 t, t, %2;\n\tst.shared.v2.f32 [t], {%3, %4};\n\t}"
-               ::"r"(base), "n"(OFF), "r"(flip), "f"(v.x), "f"(v.y) : "memory");
-}
-template <int OFF>
-__device__ __forceinline__ void sts_swz_f32x4(uint32_t base, uint32_t flip, float2 v, float2 w) {
-  asm volatile("{\n\t.reg .b32 t;\n\tadd.u32 t, %0, %1;\n\txor.b32 t, t, %2;\n\tst.shared.v4.f32 [t], {%3, %4, %5, %6};\n\t}"
-               ::"r"(base), "n"(OFF), "r"(flip), "f"(v.x), "f"(v.y), "f"(w.x), "f"(w.y) : "memory");
-}
-template <int OFF>
-__device__ __forceinline__ void sts_swz_v4(uint32_t base, uint32_t flip, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-  asm volatile("{\n\t.reg .b32 t;\n\tadd.u32 t, %0, %1;\n\txor.b32 t, t, %2;\n\tst.shared.v4.b32 [t], {%3, %4, %5, %6};\n\t}"
-               ::"r"(base), "n"(OFF), "r"(flip), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
-}
-
 // ---- kernel ----------------------------------------------------------------------------
-
-// which accumulator buffer a block uses: a constant, or the value of the carried counter
-template <int B> struct StaticBuf { __device__ static constexpr uint32_t get(uint32_t) { return uint32_t(B); } };
-struct DynBuf { __device__ static uint32_t get(uint32_t b) { return b; } };
-
-// f(integral_constant<int, 0>) ... f(integral_constant<int, N-1>): a loop whose index is a constant
-// expression inside the body (template arguments, "n" asm operands)
-template <int I> struct IntC { static constexpr int value = I; };
-template <int N, int I = 0, typename F>
-__device__ __forceinline__ void static_loop(F&& f) {
-  if constexpr (I < N) {
-    f(IntC<I>{});
-    static_loop<N, I + 1>(f);
-  }
-}
-
-// acc[j] += scale * v[2j..2j+1] for NC TMEM columns; SB_GRAN == 1 multiplies by the per-column
-// scales staged in shared memory first.
-template <int SB_GRAN, int NC>
-__device__ __forceinline__ void promote(float2* acc, const uint32_t (&v)[NC], const float* stage, float sa_v, float s_scalar) {
-  if (SB_GRAN == 1) {
-    const float2 sa2 = make_float2(sa_v, sa_v);
-#pragma unroll
-    for (int j = 0; j < NC / 4; ++j) {
-      const float4 sb4 = *reinterpret_cast<const float4*>(stage + 4 * j);
-      const float2 p0 = make_float2(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]));
-      const float2 p1 = make_float2(__uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
-      acc[2 * j] = __ffma2_rn(__fmul2_rn(p0, make_float2(sb4.x, sb4.y)), sa2, acc[2 * j]);
-      acc[2 * j + 1] = __ffma2_rn(__fmul2_rn(p1, make_float2(sb4.z, sb4.w)), sa2, acc[2 * j + 1]);
-    }
-  } else {
-    const float2 s2 = make_float2(s_scalar, s_scalar);
-#pragma unroll
-    for (int j = 0; j < NC / 2; ++j) {
-      const float2 pv = make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
-      acc[j] = __ffma2_rn(pv, s2, acc[j]);
-    }
-  }
-}
-
-// Work item -> tile coordinates.  Tiles are numbered in bands of `band` tile rows; inside a band
-// the numbering runs down the rows first, then across the columns, so that the CTAs of a wave
-// (consecutive numbers) cover a near-square patch of the output: the A and B panels they fetch
-// together are as few as possible, which is what keeps the operands' L2 lines alive between the
-// CTAs that share them.  (Row-major numbering made a 148-CTA wave touch every B panel of a
-// 24-tile-wide problem plus 7 A panels; in bands of 16 it touches 16 + 10.)
-// x / d through a multiplication by mg = ceil(2^40 / d): exact while x * d < 2^40 (the host checks
-// and passes 0 otherwise).  A 32-bit division by a run-time value costs ~20 dependent instructions,
-// and every role does three of them at each tile boundary.
-__device__ __forceinline__ int fast_div(int x, int d, unsigned long long mg) {
-  return mg != 0 ? int((static_cast<unsigned long long>(static_cast<unsigned>(x)) * mg) >> 40) : x / d;
-}
-__device__ __forceinline__ void tile_coords(const GemmParams& p, int tile, int& tm, int& tn) {
-  const int per_band = p.band * p.tiles_n;
-  const int b = fast_div(tile, per_band, p.mg_per_band), w = tile - b * per_band;
-  const int left = p.tiles_m - b * p.band;
-  const bool full = left >= p.band;
-  const int rows = full ? p.band : left;
-  tn = fast_div(w, rows, full ? p.mg_band : p.mg_last);
-  tm = b * p.band + (w - tn * rows);
-}
-// work item -> (contraction range, tile)
-__device__ __forceinline__ void item_split(const GemmParams& p, int item, int n_tiles, int& ks, int& tile) {
-  ks = fast_div(item, n_tiles, p.mg_tiles);
-  tile = item - ks * n_tiles;
-}
-// contraction range -> its first block and its number of blocks
-__device__ __forceinline__ int range_blocks(const GemmParams& p, int ks) { return p.nkb + (ks < p.nkb_rem ? 1 : 0); }
-__device__ __forceinline__ int range_first(const GemmParams& p, int ks) { return ks * p.nkb + min(ks, p.nkb_rem); }
 
 template <int BN_, int SB_GRAN, bool OUT_F32>
 __global__ void __launch_bounds__((Cfg<BN_, SB_GRAN, OUT_F32>::threads), 1)
@@ -732,49 +614,19 @@ template <int BN_, int SB_GRAN, bool OUT_F32>
 static int launch_gemm(const tg_gemm_args* a, GemmParams p, cudaStream_t st) {
   using C = Cfg<BN_, SB_GRAN, OUT_F32>;
   auto kern = gemm_fp8_blockscaled_kernel<BN_, SB_GRAN, OUT_F32>;
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb, td;
   const int64_t a_inner = p.a_mn ? a->M : a->K, a_outer = p.a_mn ? a->K : a->M;
   const int64_t b_inner = p.b_mn ? a->N : a->K, b_outer = p.b_mn ? a->K : a->N;
   if (int rc = make_tmap(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->a, a_inner, a_outer, a->lda, 128, 128)) return rc;
   if (int rc = make_tmap(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->b, b_inner, b_outer, a->ldb, 128, 128)) return rc;
-  // output map: [contraction slice][row][column]; a launch that is not cut has one slice
-  CUtensorMap td;
-  {
-    EncodeTiledFn enc;
-    if (int rc = get_encode_fn(&enc)) return rc;
-    const int esz = C::esize;
-    cuuint64_t dims[3] = {cuuint64_t(a->N), cuuint64_t(a->M), cuuint64_t(p.ksplit)};
-    cuuint64_t strides[2] = {cuuint64_t(p.ldd) * esz, cuuint64_t(p.ksplit > 1 ? p.slice_elems : a->M * p.ldd) * esz};
-    cuuint32_t box[3] = {cuuint32_t(C::phase_cols), 32u, 1u};
-    cuuint32_t estr[3] = {1, 1, 1};
-    constexpr int span = C::phase_row_bytes;
-    CUresult r = enc(&td, OUT_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, p.d, dims, strides,
-                     box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     span == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : span == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
-                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return record_cuda_error(cudaErrorInvalidValue, "cuTensorMapEncodeTiled (output)");
-  }
+  if (int rc = make_output_map(&td, OUT_F32, a, p, C::phase_cols, C::phase_row_bytes)) return rc;
   p.tiles_m = int((a->M + BM - 1) / BM);
   p.tiles_n = int((a->N + BN_ - 1) / BN_);
   p.band = p.tiles_m < kBandRows ? p.tiles_m : kBandRows;
-  const int64_t n_items = int64_t(p.tiles_m) * p.tiles_n * p.ksplit;
-  {
-    // reciprocals for the kernel's item -> tile arithmetic: q = (x * ceil(2^40 / d)) >> 40 is x / d
-    // for every x <= x_max when x_max * d < 2^40
-    auto magic = [](int64_t x_max, int64_t d) -> unsigned long long {
-      if (d <= 0 || x_max >= (int64_t(1) << 31) || x_max * d >= (int64_t(1) << 40)) return 0ull;
-      return ((1ull << 40) + uint64_t(d) - 1) / uint64_t(d);
-    };
-    const int64_t n_tiles = int64_t(p.tiles_m) * p.tiles_n, per_band = int64_t(p.band) * p.tiles_n;
-    const int64_t last_rows = p.tiles_m % p.band;
-    p.mg_tiles = magic(n_items, n_tiles);
-    p.mg_per_band = magic(n_tiles, per_band);
-    p.mg_band = magic(per_band, p.band);
-    p.mg_last = last_rows > 0 ? magic(per_band, last_rows) : 0ull;
-  }
-  if (n_items > INT32_MAX || n_items * (p.nkb + 1) > INT32_MAX) return TG_ERR_TOO_LARGE;
+  if (int rc = set_reciprocals(p)) return rc;
+  const int n_items = p.tiles_m * p.tiles_n * p.ksplit;
   const int sms = gemm_sms();
-  const int grid = int(n_items < sms ? n_items : sms);
+  const int grid = n_items < sms ? n_items : sms;
   // the attribute is per device: set it once for each device this instantiation runs on
   static bool attr_set[64] = {};
   int dev = 0;
@@ -846,12 +698,20 @@ splitk_reduce_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, 
 // narrow ones without this term); 4096 x 128 -> 1024, two waves, 4.9 / 4.5.  Over 288 problems of fewer than eight blocks the width
 // taken is 0.2 % slower than the better one on average (2.7 % without the term).
 //
+// A pair of SMs with a 256 x 256 tile (gemm_pair.cu) moves a third less from the L2 per block and promotes with fewer instructions, but it
+// starts later and a wave of it is coarser.  Measured on 720 uncut problems of 130 to 32768 rows, in turn with the widths above: three
+// waves of pairs and more 1.04-1.12 times as fast with a scale per 128 columns, 1.05-1.4 with a scale per column (8192 x 2048 -> 8192 147
+// against 158 us and 176 against 230; weight gradient 2048 x 8192 of 8192 tokens 203 / 234), half a wave or less 0.66-0.76.  Where
+// column scales lie apart (the data gradient's, quantised along the other axis) the narrower kernels take half as long again per
+// block, once enough of them run at a time.  The rule takes the slower of the two by more than 2 % in none of the 720.
+//
 // The tile width does not show in the result; the number of ranges does, in the last bit of float32 sums, and a training run
 // amplifies that over its steps.  So where the tokens are whole blocks of 128, as a training step's are, the number of
 // ranges is a rule of its own (training_ranges) that the tile width has no part in.
 struct GemmPlan {
   int bn, S;
   int64_t bytes;     // workspace the cut needs
+  bool pair;         // 256 x 256 tiles on pairs of SMs (gemm_pair.cu)
 };
 // S of 1 to 8 ranges of at least 8 blocks by waves of wide tiles x (blocks per item + 3 for an item's ramp and stores), plus for
 // S > 1 the reduction over S float32 slices at 4 MB per block time.
@@ -872,12 +732,12 @@ static int training_ranges(const tg_gemm_args* a, int wide) {
 static GemmPlan plan_gemm(const tg_gemm_args* a) {
   const bool columns = a->sb_gran_n == 1;
   const int wide = a->N <= 128 ? 128 : columns ? 192 : 256;
-  GemmPlan pl = {wide, 1, 0};
+  GemmPlan pl = {wide, 1, 0, false};
   const int64_t nkb = (a->K + BK - 1) / BK;
   const int sms = gemm_sms();
   const bool whole = a->K % BK == 0 && (a->a_major == TG_MAJOR_MN || a->M % 128 == 0);      // (weight gradient: the tokens are K)
   const int fixed = whole ? training_ranges(a, wide) : 0;
-  double best = 0.0;
+  double best = 0.0, best_blocks = 0.0;
   for (const int bn : {wide, 128}) {
     const int64_t tiles = ((a->M + BM - 1) / BM) * ((a->N + bn - 1) / bn);
     for (int S = 1; S <= 8; ++S) {
@@ -892,6 +752,7 @@ static GemmPlan plan_gemm(const tg_gemm_args* a) {
       if (S > 1) us += 3.5 + double(4 * S + 2) * double(a->M) * double(a->N) / 8.0e6;
       if (best == 0.0 || us < best * 0.97) {
         best = us;
+        best_blocks = double(waves) * block * blocks;
         pl.bn = bn;
         pl.S = S;
       }
@@ -899,6 +760,15 @@ static GemmPlan plan_gemm(const tg_gemm_args* a) {
     if (wide == 128) break;
   }
   if (pl.S > 1) pl.bytes = int64_t(pl.S) * a->M * a->N * int64_t(sizeof(float));
+  if (a->M > 128 && a->N > 128) {
+    const int64_t pairs = std::max(1, sms / 2), items = ((a->M + 255) / 256) * ((a->N + 255) / 256) * pl.S, waves = (items + pairs - 1) / pairs;
+    const double blocks = double((nkb + pl.S - 1) / pl.S);
+    double us = 4.3 + double(waves) * ((columns ? 0.54 : 0.42) * blocks + 0.86);
+    if (pl.S > 1) us += 3.5 + double(4 * pl.S + 2) * double(a->M) * double(a->N) / 8.0e6;
+    if (columns && a->sb_stride_n != 1 && 2 * items > pairs) best += 0.5 * best_blocks;
+    pl.pair = us < best && (nkb >= 8 || waves >= 3);
+    if (pl.pair) pl.bn = 256;
+  }
   return pl;
 }
 
@@ -934,6 +804,12 @@ extern "C" int tgh_gemm_plan(const tg_gemm_args* a, int* tile_columns, int* rang
   const GemmPlan pl = plan_gemm(a);
   *tile_columns = pl.bn;
   *ranges = pl.S;
+  return TG_OK;
+}
+
+extern "C" int tgh_gemm_takes_pairs(const tg_gemm_args* a, int* pairs) {
+  if (int rc = validate_gemm(a)) return rc;
+  *pairs = a->M > 0 && a->N > 0 && a->K > 0 && !skinny_takes(a) && plan_gemm(a).pair;
   return TG_OK;
 }
 
@@ -985,7 +861,8 @@ extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
     p.d = a->workspace;
     p.ldd = a->N;
     int rc;
-    if (bn == 256) rc = launch_gemm<256, 128, true>(a, p, st);
+    if (pl.pair) rc = pair_run(a, p, true, st);
+    else if (bn == 256) rc = launch_gemm<256, 128, true>(a, p, st);
     else if (bn == 192) rc = launch_gemm<192, 1, true>(a, p, st);
     else rc = g1 ? launch_gemm<128, 1, true>(a, p, st) : launch_gemm<128, 128, true>(a, p, st);
     if (rc != TG_OK) return rc;
@@ -996,6 +873,7 @@ extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
                                   static_cast<long long>(p.slice_elems)));
     return TG_OK;
   }
+  if (pl.pair) return pair_run(a, p, f32, st);
   if (bn == 256) return f32 ? launch_gemm<256, 128, true>(a, p, st) : launch_gemm<256, 128, false>(a, p, st);
   if (bn == 192) return f32 ? launch_gemm<192, 1, true>(a, p, st) : launch_gemm<192, 1, false>(a, p, st);
   if (g1) return f32 ? launch_gemm<128, 1, true>(a, p, st) : launch_gemm<128, 1, false>(a, p, st);

@@ -1,0 +1,586 @@
+// Block-scaled e4m3 GEMM on pairs of SMs (tcgen05 cta_group::2): a cluster of two CTAs computes a 256 x 256 tile of
+//     D[m,n] = sum_kb SA(m,kb) SB(n,kb) sum_{k in kb} A[m,k] B[n,k].
+// CTA r of a pair owns rows 128 r.. of the tile (its tensor memory holds their accumulators) and loads its 128 rows of A and half of
+// the 256 rows of B; the tensor cores read the other half of B from the partner's shared memory.  Promotion is as in gemm_fp8.cu:
+// float32 scales, so every 128-deep contraction block is a chain of its own into a fresh accumulator buffer, which promotion warps
+// read, scale and add in registers; the same operations in the same order, hence the same bits.
+//
+// Warp roles of a CTA (384 threads):
+//   0-7   promotion + epilogue: warp w reads TMEM lanes 32 (w % 4).. (a hardware rule), accumulator columns 128 (w / 4)..
+//   8     TMA producer: one box of A, one of B per stage
+//   9     MMA issuer, in the pair's first CTA only
+//   10    scales: the block's row and column scales go into a ring in shared memory, as many blocks ahead as there are stages
+//   11    the tile's bulk stores
+//
+// What bounds it: for large problems the board's power cap (1000 W; 32768 x 2048 -> 6144 in a loop of half a second runs at 1.36-1.40
+// GHz), else the promotion warps, which never find an accumulator missing: on each scheduler 2 x 64 packed FMAs of two cycles (twice that
+// with a scale per column) and the register writes of the TMEM loads, which hold the FMA pipe up: 375 cycles of a block's 512 on
+// the tensor core alone (666 with column scales), measured without MMAs, TMA or barriers; about 700 (1000) with everything.  So
+// the design keeps promotion short rather than wide:
+//   - A pair moves 32 KB per SM and block from the L2 instead of 48, and one thread issues for two SMs.
+//   - Eight warps of 128 columns instead of sixteen of 64 (registers handed over, 224 each): half the barrier operations, scale loads and
+//     set-up per block.  1400 warp instructions per block of a tile instead of 1821.  (Sixteen: 434 us for the problem above, eight 415.)
+//   - No scale is fetched by a promotion warp and none is waited for separately: the accumulator's barrier counts the MMAs' commit and
+//     the scale warp's announcement.  (A barrier of its own for the scales: 630 instead of 560 us for the weight gradient.)
+//   - A wait's outcome is looked at once a tile, not voted on in every block.
+//   - The buffer goes back by an arrival with CTA scope on the first CTA's barrier.  With cluster scope the release is a fence that waits
+//     for the SM's copies in flight: 700 us instead of 360.
+// Forward 32768 x 2048 -> 6144 in a loop: 435 us on single CTAs, 415 here (1.90 / 1.99 PFLOP/s); with a scale per column 555 / 500;
+// its weight gradient 584 / 550 (six waves where 5.2 would do); in short bursts 383 / 355, 530 / 435, 530 / 500.
+// Tried and left out: the next block's barrier probed during a block (a try_wait that comes too early suspends the warp; with test_wait
+// 2 % slower), a ready counter in shared memory polled instead of the barrier (5 % slower), 32-column pieces in two register buffers
+// (spills), column-scale pieces in two register buffers (3 % slower: the FMA pipe, not the load's latency, is the limit).
+//
+// Every wait on an mbarrier is bounded, as in gemm_fp8.cu (codes of its roles; 9 = scales).
+#include <cuda.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "gemm_tiles.cuh"
+#include "host_api.h"
+#include "mbarrier.cuh"
+#include "umma.cuh"
+
+namespace tg {
+
+// ---- cluster forms of the PTX wrappers ---------------------------------------------------
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// the same shared-memory offset in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster_if(uint32_t bar, uint32_t pred) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}"
+               ::"r"(bar), "r"(pred) : "memory");
+}
+// a load into this CTA's shared memory whose bytes are counted by a barrier of either CTA of the pair
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrives on the barrier at this offset in both CTAs once the MMAs issued before are done
+__device__ __forceinline__ void umma_commit_both(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"(uint16_t(3)) : "memory");
+}
+__device__ __forceinline__ void umma_commit_here(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// four bytes from memory to shared memory (any 4-byte alignment), through L1: a row scale's sector serves eight blocks
+__device__ __forceinline__ void cp_async_4(uint32_t dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+// ---- kernel --------------------------------------------------------------------------------
+
+constexpr int kPairBandRows = 8;      // tile rows per band of the numbering: 74 pairs cover a patch of about 8 x 9 tiles
+
+template <int SB_GRAN, bool OUT_F32>
+struct PairCfg {
+  static constexpr int BN = 256;
+  static constexpr int promo_warps = 8;
+  static constexpr int producer_warp = promo_warps, issuer_warp = promo_warps + 1, scale_warp = promo_warps + 2, store_warp = promo_warps + 3;
+  static constexpr int threads = 32 * (promo_warps + 4);
+  // 168 registers a thread at launch; the service warpgroup hands over what the two promotion warpgroups grow by
+  static constexpr int launch_regs = 168, promo_regs = 224, service_regs = 56;
+  static_assert(service_regs + promo_warps / 4 * promo_regs <= (promo_warps / 4 + 1) * launch_regs, "register hand-over asks for more than is released");
+  static constexpr int cols = 1024 / promo_warps, pieces = cols / 16;
+                             // accumulator columns of a warp
+  static constexpr int stage_bytes = 2 * kTileBytes;           // A and half of B
+  static constexpr int box_bytes = 32 * 128;                   // an output box: 32 rows of 128 bytes
+  static constexpr int warp_boxes = 16 / promo_warps;                         // staged at a time
+  static constexpr int esize = OUT_F32 ? 4 : 2;
+  static constexpr int box_cols = 128 / esize;
+  static constexpr int phases = cols / (warp_boxes * box_cols);
+  static constexpr int out_bytes = promo_warps * warp_boxes * box_bytes;
+  // a ring slot: 128 row scales, then the column scales (256, or one per 128 columns)
+  static constexpr int slot_floats = 128 + (SB_GRAN == 1 ? 256 : 4);
+  static constexpr int static_reserve = 1024;
+  static constexpr int stages_fit = (kSmemLimit - static_reserve - out_bytes - 2 * 4 * slot_floats) / (stage_bytes + 4 * slot_floats);
+  static constexpr int stages = stages_fit > 6 ? 6 : stages_fit;
+  // The scales of block i go into slot i % ring once the stage of block i is free, that is, once the MMAs of block i - stages are
+  // done.  Those were issued after every promotion warp had given back the accumulator of block i - stages - 2, which it does
+  // after its last look at that block's scales.
+  static constexpr int ring = stages + 2;
+  static constexpr int off_out = stages * stage_bytes;
+  static constexpr int off_ring = off_out + out_bytes;
+  static constexpr int smem_bytes = off_ring + ring * slot_floats * 4;
+  static constexpr int n_bars = 2 * stages + 2 * 2 + 3;
+  static_assert(n_bars <= 24, "control block too small");
+  static_assert(stages >= 3 && smem_bytes + static_reserve <= kSmemLimit, "shared-memory plan");
+};
+
+template <int SB_GRAN, bool OUT_F32>
+__global__ void __launch_bounds__((PairCfg<SB_GRAN, OUT_F32>::threads), 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                 const __grid_constant__ CUtensorMap tmap_d, const GemmParams p) {
+  using C = PairCfg<SB_GRAN, OUT_F32>;
+  constexpr int BN = C::BN, kStages = C::stages, kRing = C::ring;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ __align__(16) uint64_t ctl_bars[24];
+  __shared__ uint32_t ctl_tmem_ptr;
+  __shared__ int ctl_abort;
+  const uint32_t sbase = smem_u32(smem);
+  const uint32_t full0 = smem_u32(ctl_bars), empty0 = full0 + 8u * kStages;
+  const uint32_t tfull0 = empty0 + 8u * kStages, tempty0 = tfull0 + 16u;
+  const uint32_t drain_bar = tempty0 + 16u, staged_bar = drain_bar + 8u, unstaged_bar = drain_bar + 16u;
+  volatile uint32_t* tmem_ptr_smem = &ctl_tmem_ptr;
+  volatile int* abort_flag = &ctl_abort;
+
+  if ((sbase & 1023u) != 0) {   // the swizzled operand layout needs this alignment (both CTAs have the same layout)
+    if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0u, 6u);
+    return;
+  }
+
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  const int n_tiles = p.tiles_m * p.tiles_n;
+  const int n_items = n_tiles * p.ksplit;
+  const int first_item = int(blockIdx.x >> 1), item_step = int(gridDim.x >> 1);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(full0 + 8u * s, 1);            // (the first CTA's counts the bytes of both)
+      mbar_init(empty0 + 8u * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(tfull0 + 8u * b, 2);           // the block's MMAs and its scales
+      mbar_init(tempty0 + 8u * b, 2 * C::promo_warps);
+    }
+    mbar_init(drain_bar, 1);
+    mbar_init(staged_bar, C::promo_warps);
+    mbar_init(unstaged_bar, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_a)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_b)) : "memory");
+  }
+  if (warp == C::issuer_warp) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl_tmem_ptr)), "r"(uint32_t(kTmemCols)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  cluster_sync();              // both CTAs' barriers exist before either signals across
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_ptr_smem;
+  grid_trigger();
+  grid_wait();
+
+  if (warp >= C::promo_warps) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::service_regs));
+    if (warp == C::producer_warp) {
+      // ------------------------------ TMA producer -------------------------------------
+      uint32_t s = 0, ph = 1;
+      bool ok = true;
+      const uint32_t full_leader = map_rank(full0, 0u);
+      for (int item = first_item; ok && item < n_items; item += item_step) {
+        int ks, tile, tm, tn;
+        item_split(p, item, n_tiles, ks, tile);
+        tile_coords(p, tile, tm, tn);
+        const int m0 = tm * 2 * BM + int(rank) * BM, n0 = tn * BN + int(rank) * 128;     // (past M or N: zeros)
+        int k0 = range_first(p, ks) * BK;
+        const int nkb = range_blocks(p, ks);
+        for (int kb = 0; kb < nkb; ++kb, k0 += BK) {
+          ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8u * s, ph, abort_flag, p.status, 1u));
+          if (!ok) break;
+          if (elect_one()) {
+            const uint32_t dst = sbase + s * C::stage_bytes, fb = full_leader + 8u * s;
+            // The first CTA announces the bytes of both.  The second's may land before that: its barrier phase is the same one,
+            // since the stage was free in both CTAs only after the phase before had completed.
+            if (rank == 0) mbar_expect_tx(full0 + 8u * s, 2 * C::stage_bytes);
+            tma_load_2d_pair(dst, &tmap_a, fb, p.a_mn ? m0 : k0, p.a_mn ? k0 : m0);
+            tma_load_2d_pair(dst + kTileBytes, &tmap_b, fb, p.b_mn ? n0 : k0, p.b_mn ? k0 : n0);
+          }
+          __syncwarp();
+          if (++s == kStages) { s = 0; ph ^= 1u; }
+        }
+      }
+    } else if (warp == C::issuer_warp) {
+      // ------------------------------ MMA issuer (first CTA) ----------------------------
+      if (rank == 0) {
+        // D f32 (bit 4), A/B e4m3 (0), major bits 15/16, N>>3 at 17, M>>4 at 24
+        const uint32_t idesc = (1u << 4) | (uint32_t(p.a_mn) << 15) | (uint32_t(p.b_mn) << 16) | (uint32_t(BN >> 3) << 17) |
+                               (uint32_t(2 * BM >> 4) << 24);
+        const uint32_t a_step = p.a_mn ? (UMMA_K * 128) >> 4 : UMMA_K >> 4;
+        const uint32_t b_step = p.b_mn ? (UMMA_K * 128) >> 4 : UMMA_K >> 4;
+        const uint64_t desc_a0 = make_smem_desc(sbase), desc_b0 = make_smem_desc(sbase + kTileBytes);
+        const uint32_t desc_hi = uint32_t(desc_a0 >> 32);
+        const uint32_t a_lo0 = uint32_t(desc_a0), b_lo0 = uint32_t(desc_b0);
+        uint32_t total = 0;
+        for (int item = first_item; item < n_items; item += item_step) {
+          int ks, tile;
+          item_split(p, item, n_tiles, ks, tile);
+          total += uint32_t(range_blocks(p, ks));
+        }
+        bool ok = true;
+        const bool stage_lane = lane >= 16;      // one wait instruction per block: half the lanes poll either barrier
+        uint32_t s = 0, sph = 0, buf = 0, bph = 1, soff = 0;
+        for (uint32_t it = 0; ok && it < total; ++it) {
+          const uint32_t bar = stage_lane ? full0 + 8u * s : tempty0 + 8u * buf;
+          const uint32_t par = stage_lane ? sph : bph;
+          ok = __all_sync(0xffffffffu, mbar_wait(bar, par, abort_flag, p.status, stage_lane ? 3u : 2u));
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+            const uint32_t d_tmem = tmem_base + buf * uint32_t(BN);
+#pragma unroll
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma_f8_pair(d_tmem, (uint64_t(desc_hi) << 32) | (a_lo0 + soff + k * a_step),
+                           (uint64_t(desc_hi) << 32) | (b_lo0 + soff + k * b_step), idesc, k > 0 ? 1u : 0u);
+            umma_commit_both(tfull0 + 8u * buf);
+            umma_commit_both(empty0 + 8u * s);
+          }
+          __syncwarp();
+          soff += uint32_t(C::stage_bytes >> 4);
+          if (++s == kStages) { s = 0; sph ^= 1u; soff = 0; }
+          buf ^= 1u;
+          bph ^= buf ^ 1u;
+        }
+        // nothing issued here may still be running when tensor memory is freed
+        if (elect_one()) {
+          umma_commit_here(drain_bar);
+          mbar_wait(drain_bar, 0u, abort_flag, p.status, 4u);
+        }
+        __syncwarp();
+      }
+    } else if (warp == C::scale_warp) {
+      // ------------------------------ scales --------------------------------------------
+      // Copies run two blocks ahead of the announcement: block j's scales are announced on its accumulator's barrier, beside its MMAs,
+      // once that barrier is through with block j - 2.  The MMAs of block i wait for the announcement of block i - 2, which comes after
+      // the copy of block i: so while that copy waits for its stage, the stage's barrier cannot go on to the phase after.  (The first
+      // blocks' MMAs wait for no announcement: their copies must not look at the barrier, and need not.)
+      uint32_t s = 0, ph = 1, slot = 0, buf = 0, bph = 1, copied = 0;
+      bool ok = true;
+      const uint32_t is_lane0 = lane == 0;
+      auto announce = [&]() {
+        ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8u * buf, bph, abort_flag, p.status, 9u));
+        mbar_arrive_if(tfull0 + 8u * buf, is_lane0);
+        buf ^= 1u;
+        bph ^= buf ^ 1u;
+      };
+      for (int item = first_item; ok && item < n_items; item += item_step) {
+        int ks, tile, tm, tn;
+        item_split(p, item, n_tiles, ks, tile);
+        tile_coords(p, tile, tm, tn);
+        const int m0 = tm * 2 * BM + int(rank) * BM, n0 = tn * BN;
+        const uint32_t kb0 = uint32_t(range_first(p, ks));
+        // element offsets (the host checks that they fit 32 bits); rows and columns past the end read a valid scale
+        uint32_t sa_off[4], sb_off[SB_GRAN == 1 ? 8 : 1];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sa_off[i] = uint32_t(min(m0 + lane + 32 * i, p.M - 1)) * uint32_t(p.sa_sm) + kb0 * uint32_t(p.sa_sk);
+        if (SB_GRAN == 1) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) sb_off[i] = uint32_t(min(n0 + lane + 32 * i, p.N - 1)) * uint32_t(p.sb_sn) + kb0 * uint32_t(p.sb_sk);
+        } else {
+          sb_off[0] = uint32_t(min(n0 / 128 + (lane & 1), (p.N - 1) / 128)) * uint32_t(p.sb_sn) + kb0 * uint32_t(p.sb_sk);
+        }
+        const int nkb = range_blocks(p, ks);
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (copied >= uint32_t(kStages)) {
+            ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8u * s, ph, abort_flag, p.status, 9u));
+            if (!ok) break;
+          }
+          const uint32_t dst = sbase + C::off_ring + slot * uint32_t(C::slot_floats * 4) + 4u * lane;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            cp_async_4(dst + 128u * i, p.sa + sa_off[i]);
+            sa_off[i] += uint32_t(p.sa_sk);
+          }
+          if (SB_GRAN == 1) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              cp_async_4(dst + 512u + 128u * i, p.sb + sb_off[i]);
+              sb_off[i] += uint32_t(p.sb_sk);
+            }
+          } else {
+            if (lane < 2) cp_async_4(dst + 512u, p.sb + sb_off[0]);
+            sb_off[0] += uint32_t(p.sb_sk);
+          }
+          asm volatile("cp.async.commit_group;" ::: "memory");
+          if (++s == kStages) { s = 0; ph ^= 1u; }
+          if (++slot == kRing) slot = 0;
+          if (++copied > 2) {
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
+            announce();
+            if (!ok) break;
+          }
+        }
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      if (ok && copied > 1) announce();
+      if (ok && copied > 0) announce();
+    } else {
+      // ------------------------------ tile stores ----------------------------------------
+      uint32_t sph = 0;
+      bool ok = true;
+      for (int item = first_item; ok && item < n_items; item += item_step) {
+        int ks, tile, tm, tn;
+        item_split(p, item, n_tiles, ks, tile);
+        tile_coords(p, tile, tm, tn);
+#pragma unroll 1
+        for (int phase = 0; phase < C::phases; ++phase) {
+          ok = __all_sync(0xffffffffu, mbar_wait(staged_bar, sph, abort_flag, p.status, 7u));
+          if (!ok) break;
+          sph ^= 1u;
+          if (elect_one()) {
+#pragma unroll 1
+            for (int w = 0; w < C::promo_warps; ++w) {
+#pragma unroll
+              for (int h = 0; h < C::warp_boxes; ++h)
+                tma_store_3d_nocommit(&tmap_d, sbase + C::off_out + uint32_t(w * C::warp_boxes + h) * C::box_bytes,
+                                      tn * BN + (w >> 2) * C::cols + (phase * C::warp_boxes + h) * C::box_cols,
+                                      tm * 2 * BM + int(rank) * BM + (w & 3) * 32, ks);
+            }
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            tma_store_wait_read();
+            mbar_arrive(unstaged_bar);
+          }
+          __syncwarp();
+        }
+      }
+    }
+  } else {
+    // ------------------------------ promotion + epilogue --------------------------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::promo_regs));
+    const int quarter = warp & 3, cg = warp >> 2;
+    const int r = quarter * 32 + lane;
+    constexpr bool kFrag = SB_GRAN == 1;
+    const int fg = lane >> 2, fj = lane & 3;     // fragment coordinates: rows fg + 8 i, column pairs 8 k + 2 fj
+    const float* ring = reinterpret_cast<const float*>(smem + C::off_ring);
+    const uint32_t tcol0 = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(cg * C::cols);
+    const int sb_index = cg * C::cols / 128;
+    const uint32_t wb = sbase + C::off_out + uint32_t(warp) * (C::warp_boxes * C::box_bytes);
+    const uint32_t tempty_leader = map_rank(tempty0, 0u);
+    const uint32_t is_lane0 = lane == 0;
+    uint32_t buf = 0, bph = 0, uph = 1, slot = 0;
+    // A wait that gives up has raised the abort flag, and every wait after it returns at once: the warps look at `ok` once a tile.
+    bool ok = true;
+    auto release = [&](uint32_t b) {
+      tc_fence_before();
+      __syncwarp();
+      mbar_arrive_cluster_if(tempty_leader + 8u * b, is_lane0);
+    };
+    for (int item = first_item; item < n_items; item += item_step) {
+      float2 acc[C::cols / 2];
+#pragma unroll
+      for (int j = 0; j < C::cols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
+      int nkb;
+      {
+        int ks, tile;
+        item_split(p, item, n_tiles, ks, tile);
+        nkb = range_blocks(p, ks);
+      }
+      auto enter_block = [&]() {
+        ok &= mbar_wait(tfull0 + 8u * buf, bph, abort_flag, p.status, 5u);
+        __syncwarp();
+        tc_fence_after();
+        const float* sc = ring + slot * C::slot_floats;
+        if (++slot == kRing) slot = 0;
+        return sc;
+      };
+      auto leave_block = [&]() {
+        release(buf);
+        buf ^= 1u;
+        bph ^= buf ^ 1u;
+      };
+      if constexpr (kFrag) {
+#pragma unroll 1
+        for (int kb = 0; kb < nkb; ++kb) {
+          const float* sc = enter_block();
+          const uint32_t taddr = tcol0 + buf * uint32_t(BN);
+          float sa_r[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) sa_r[i] = sc[quarter * 32 + fg + 8 * i];
+          const float* scol = sc + 128 + cg * C::cols + 2 * fj;
+          // acc[(4 q + i) * 2 + k] holds rows fg + 8 i, columns 16 q + 8 k + 2 fj (+1)
+#pragma unroll
+          for (int q = 0; q < C::pieces; ++q) {
+            uint32_t v[16];
+            float2 sb2[2];
+            sb2[0] = *reinterpret_cast<const float2*>(scol + 16 * q);
+            sb2[1] = *reinterpret_cast<const float2*>(scol + 16 * q + 8);
+            tmem_ld_frag16(taddr + 16 * q, v);
+            tmem_ld_frag16(taddr + (16u << 16) + 16 * q, v + 8);
+            tmem_wait_ld16(v);
+            if (q == C::pieces - 1) leave_block();         // (after the last look at the scales, see PairCfg::ring)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int o = 8 * (i >> 1) + 4 * k + 2 * (i & 1);
+                const float2 pv = make_float2(__uint_as_float(v[o]), __uint_as_float(v[o + 1]));
+                float2& a = acc[(4 * q + i) * 2 + k];
+                a = __ffma2_rn(__fmul2_rn(pv, sb2[k]), make_float2(sa_r[i], sa_r[i]), a);
+              }
+            }
+          }
+        }
+      } else {
+        // two register buffers: the next piece is on its way while one is promoted, across blocks too
+        uint32_t v[2][16];
+        const float* sc = enter_block();
+        float s = sc[r] * sc[128 + sb_index];
+        uint32_t taddr = tcol0 + buf * uint32_t(BN);
+        tmem_ld16(taddr, v[0]);
+#pragma unroll 1
+        for (int kb = 0; kb < nkb; ++kb) {
+          const bool more = kb + 1 < nkb;
+#pragma unroll
+          for (int q = 0; q < C::pieces - 1; ++q) {
+            tmem_wait_ld16(v[q & 1]);
+            tmem_ld16(taddr + 16 * (q + 1), v[(q + 1) & 1]);
+            promote<128, 16>(acc + 8 * q, v[q & 1], nullptr, 0.f, s);
+          }
+          tmem_wait_ld16(v[1]);
+          leave_block();
+          float s_next = 0.f;
+          if (more) {
+            sc = enter_block();
+            taddr = tcol0 + buf * uint32_t(BN);
+            tmem_ld16(taddr, v[0]);
+            s_next = sc[r] * sc[128 + sb_index];
+          }
+          promote<128, 16>(acc + 8 * (C::pieces - 1), v[1], nullptr, 0.f, s);
+          s = s_next;
+        }
+      }
+      if (!__all_sync(0xffffffffu, ok)) break;
+
+      // ---- epilogue: registers -> this warp's swizzled staging rows; the store warp does the rest ----
+#pragma unroll
+      for (int phase = 0; phase < C::phases; ++phase) {
+        // (the first pass finds the rows free)
+        ok = __all_sync(0xffffffffu, mbar_wait(unstaged_bar, uph, abort_flag, p.status, 8u));
+        if (!ok) break;
+        uph ^= 1u;
+        if constexpr (kFrag && OUT_F32) {
+          // 16-byte chunk 4 (q % 2) + 2 k + (fj >> 1) of box q / 2, half fj & 1
+          const uint32_t base = wb + uint32_t(fg) * 128u + (uint32_t(fj >> 1) << 4) + 8u * uint32_t(fj & 1), flip = uint32_t(fg) << 4;
+          static_loop<2 * C::warp_boxes>([&](auto qq) {
+            static_loop<4>([&](auto i) {
+              static_loop<2>([&](auto k) {
+                const float2 a = acc[(4 * (2 * C::warp_boxes * phase + qq.value) + i.value) * 2 + k.value];
+                sts_swz_f32x2<(qq.value >> 1) * C::box_bytes + i.value * 1024 + (4 * (qq.value & 1) + 2 * k.value) * 16>(base, flip, a);
+              });
+            });
+          });
+        } else if constexpr (kFrag) {
+          // 16-byte chunk 2 (q % 4) + k of box q / 4, 4 fj bytes in
+          const uint32_t base = wb + uint32_t(fg) * 128u + 4u * uint32_t(fj), flip = uint32_t(fg) << 4;
+          static_loop<C::pieces>([&](auto q) {
+            static_loop<4>([&](auto i) {
+              static_loop<2>([&](auto k) {
+                const float2 a = acc[(4 * q.value + i.value) * 2 + k.value];
+                sts_swz_b32<(q.value >> 2) * C::box_bytes + i.value * 1024 + (2 * (q.value & 3) + k.value) * 16>(base, flip, pack_bf16x2(a.x, a.y));
+              });
+            });
+          });
+        } else if constexpr (OUT_F32) {
+          const uint32_t base = wb + uint32_t(lane) * 128u, flip = uint32_t(lane & 7) << 4;
+          static_loop<8 * C::warp_boxes>([&](auto c) {
+            const int j = 16 * C::warp_boxes * phase + 2 * c.value;
+            sts_swz_f32x4<(c.value >> 3) * C::box_bytes + (c.value & 7) * 16>(base, flip, acc[j], acc[j + 1]);
+          });
+        } else {
+          const uint32_t base = wb + uint32_t(lane) * 128u, flip = uint32_t(lane & 7) << 4;
+          static_loop<8 * C::warp_boxes>([&](auto c) {
+            const int j = 4 * c.value;
+            sts_swz_v4<(c.value >> 3) * C::box_bytes + (c.value & 7) * 16>(
+                base, flip, pack_bf16x2(acc[j].x, acc[j].y), pack_bf16x2(acc[j + 1].x, acc[j + 1].y),
+                pack_bf16x2(acc[j + 2].x, acc[j + 2].y), pack_bf16x2(acc[j + 3].x, acc[j + 3].y));
+          });
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the copy engine
+        __syncwarp();
+        mbar_arrive_if(staged_bar, is_lane0);
+      }
+      if (!ok) break;
+    }
+  }
+
+  // ------------------------------ teardown ----------------------------------------------
+  tc_fence_before();
+  cluster_sync();              // the partner no longer reads this CTA's shared memory or signals its barriers
+  if (warp == C::issuer_warp) {
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(uint32_t(kTmemCols)) : "memory");
+  }
+}
+
+// ---- host ------------------------------------------------------------------------------
+
+template <int SB_GRAN, bool OUT_F32>
+static int launch_pair(const tg_gemm_args* a, GemmParams p, cudaStream_t st) {
+  using C = PairCfg<SB_GRAN, OUT_F32>;
+  auto kern = gemm_pair_kernel<SB_GRAN, OUT_F32>;
+  CUtensorMap ta, tb, td;
+  const int64_t a_inner = p.a_mn ? a->M : a->K, a_outer = p.a_mn ? a->K : a->M;
+  const int64_t b_inner = p.b_mn ? a->N : a->K, b_outer = p.b_mn ? a->K : a->N;
+  if (int rc = make_tmap(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->a, a_inner, a_outer, a->lda, 128, 128)) return rc;
+  if (int rc = make_tmap(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->b, b_inner, b_outer, a->ldb, 128, 128)) return rc;
+  if (int rc = make_output_map(&td, OUT_F32, a, p, C::box_cols, 128)) return rc;
+  p.tiles_m = int((a->M + 2 * BM - 1) / (2 * BM));
+  p.tiles_n = int((a->N + C::BN - 1) / C::BN);
+  p.band = std::min(p.tiles_m, kPairBandRows);
+  if (int rc = set_reciprocals(p)) return rc;
+  const int n_items = p.tiles_m * p.tiles_n * p.ksplit;
+  int dev = 0;
+  TG_CUDA_CHECK(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return TG_ERR_SHAPE;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = 2;
+  attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(C::threads);
+  cfg.dynamicSmemBytes = C::smem_bytes;
+  cfg.attrs = attrs;
+  cfg.numAttrs = 1;
+  // once per device: the kernel's shared memory, and how many pairs run at a time (a pair takes two SMs of one cluster group)
+  static std::atomic<int> pairs_of[64];
+  int fit = pairs_of[dev].load(std::memory_order_acquire);
+  if (fit == 0) {
+    TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem_bytes));
+    cfg.gridDim = dim3(unsigned(sm_count() & ~1));
+    TG_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&fit, kern, &cfg));
+    if (fit < 1) return record_cuda_error(cudaErrorLaunchOutOfResources, "no CTA pair fits on this device");
+    pairs_of[dev].store(fit, std::memory_order_release);
+  }
+  const int pairs = std::max(1, std::min(fit, gemm_sms() / 2));
+  cfg.gridDim = dim3(unsigned(2 * std::min(n_items, pairs)));
+  cfg.stream = st;
+  if (n_items <= 4 * pairs && p.nkb <= 32) cfg.numAttrs = 2;      // a short kernel starts early, as in gemm_fp8.cu
+  TG_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, ta, tb, td, p));
+  return TG_OK;
+}
+
+int pair_run(const tg_gemm_args* a, const GemmParams& p, bool out_f32, cudaStream_t st) {
+  if (a->sb_gran_n == 1) return out_f32 ? launch_pair<1, true>(a, p, st) : launch_pair<1, false>(a, p, st);
+  return out_f32 ? launch_pair<128, true>(a, p, st) : launch_pair<128, false>(a, p, st);
+}
+
+}  // namespace tg

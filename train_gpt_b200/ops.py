@@ -160,6 +160,9 @@ STATUS_ROLES = {
     3: "the MMA issuer waited for operands to land",
     4: "the MMA issuer waited for its last instructions to retire",
     5: "the promotion warps waited for an accumulator buffer to fill",
+    7: "the store warp waited for a staged tile",
+    8: "the promotion warps waited for their staging rows",
+    9: "the scale warp waited for a free slot or its block's turn",
 }
 STATUS_TOKEN = 16   # a training step met a token id outside the vocabulary
 
