@@ -1,20 +1,22 @@
-"""The GEMM on pairs of SMs against the single-CTA kernels: a row (or column) of the result depends on its own operands only and is
-summed in the same order by either, so a problem computed in slices too small for pairs has the same bits."""
+"""The kernel with the scale ring.  On pairs of SMs it is compared with the other tiled kernel: a row (or column) of the result depends on
+its own operands only and is summed in the same order by either, so a problem computed in slices too small for pairs has the same
+bits.  On single SMs it is compared with the product in float64."""
 import ctypes
 
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+SINGLE, PAIRS = 1, 2
 
 
 def _plan(M, N, K, major, gran):
     from train_gpt_b200 import _lib
     mn = _lib.TG_MAJOR_MN
-    args = _lib.GemmArgs(M=M, N=N, K=K, lda=(M if major == mn else K) + 15 & ~15, ldb=N + 15 & ~15, a_major=major, b_major=mn, sb_gran_n=gran, ldd=N)
-    pair = ctypes.c_int()
-    assert _lib.load().tgh_gemm_takes_pairs(ctypes.byref(args), ctypes.byref(pair)) == _lib.TG_OK
-    return bool(pair.value)
+    args = _lib.GemmArgs(M=M, N=N, K=K, lda=(M if major == mn else K) + 15 & ~15, ldb=N + 15 & ~15, a_major=major, b_major=mn, sb_gran_n=gran, sb_stride_n=1, ldd=N)
+    kernel = ctypes.c_int(-1)
+    rc = _lib.load().tgh_gemm_kernel(ctypes.byref(args), ctypes.byref(kernel))
+    return kernel.value if rc == _lib.TG_OK else -1            # (-1: the few-token kernel's)
 
 
 def _f8(gen, *shape):
@@ -39,12 +41,12 @@ def test_forward_has_the_bits_of_its_slices(M, K, N, tile, out):
     sw = _scales(gen, K // 128, N if tile == (128, 1) else N // 128)
     gran = 1 if tile == (128, 1) else 128
     kw = dict(N=N, K=K, a_major=_lib.TG_MAJOR_K, b_major=_lib.TG_MAJOR_MN, sa_strides=(sa.stride(0), 1), sb_strides=(1, sw.stride(0)), sb_gran_n=gran, out_dtype=out, split=False)
-    assert _plan(M, N, K, _lib.TG_MAJOR_K, gran)
+    assert _plan(M, N, K, _lib.TG_MAJOR_K, gran) == PAIRS
     status = ops.new_status("cuda")
     y = ops.gemm_blockscaled(a, w, sa, sw, M=M, status=status, **kw)
     for r in range(0, M, 512):
         m = min(512, M - r)
-        assert not _plan(m, N, K, _lib.TG_MAJOR_K, gran)
+        assert _plan(m, N, K, _lib.TG_MAJOR_K, gran) != PAIRS
         if m <= 128:
             continue               # (the few-token kernel adds in another order)
         assert torch.equal(y[r:r + m], ops.gemm_blockscaled(a[r:r + m], w, sa[r:r + m], sw, M=m, status=status, **kw)), r
@@ -64,15 +66,53 @@ def test_weight_gradient_has_the_bits_of_its_slices(T, K, N):
     tb = (T + 127) // 128
     sx, sg = _scales(gen, tb, K), _scales(gen, tb, N)
     kw = dict(N=N, K=T, a_major=_lib.TG_MAJOR_MN, b_major=_lib.TG_MAJOR_MN, sa_strides=(1, sx.stride(0)), sb_strides=(1, N), sb_gran_n=1, split=False)
-    assert _plan(K, N, T, _lib.TG_MAJOR_MN, 1)
+    assert _plan(K, N, T, _lib.TG_MAJOR_MN, 1) == PAIRS
     status = ops.new_status("cuda")
     dw = ops.gemm_blockscaled(x, g, sx, sg, M=K, status=status, **kw)
     for r in range(0, K, 384):
         m = min(384, K - r)
-        assert not _plan(m, N, T, _lib.TG_MAJOR_MN, 1)
+        assert _plan(m, N, T, _lib.TG_MAJOR_MN, 1) != PAIRS
         xs = x[:, r:r + m].contiguous()
         part = ops.gemm_blockscaled(xs, g, sx[:, r:r + m].contiguous(), sg, M=m, status=status, **dict(kw, sa_strides=(1, m)))
         assert torch.equal(dw[r:r + m], part), r
+    assert int(status.item()) == 0
+
+
+def _close(y, ref):
+    """One rounding to the output type, and float32 sums of at most 128 blocks of 128 products."""
+    ulp = 2.0 ** -8 if y.dtype == torch.bfloat16 else 0.0
+    assert bool(((y.double() - ref).abs() <= ulp * ref.abs() + 1e-5 * ref.square().mean().sqrt()).all())
+
+
+# 128-column tiles (two of them wider than N), 192-column tiles (a ragged last one); twelve blocks, more than the ring, one past it
+@pytest.mark.parametrize("M,K,N,out", [(200, 1536, 1000, torch.bfloat16), (129, 1664, 8192, torch.float32), (1000, 2048, 136, torch.bfloat16),
+                                        (1100, 1792, 2952, torch.bfloat16), (640, 4096, 4096, torch.bfloat16)])
+def test_column_scales_on_single_sms_forward(M, K, N, out):
+    from train_gpt_b200 import _lib, ops
+    gen = torch.Generator("cuda").manual_seed(K)
+    a, sa = _f8(gen, M, K), _scales(gen, M, K // 128)
+    w, sw = _f8(gen, K, N + 15 & ~15)[:, :N], _scales(gen, K // 128, N)
+    if M % 128:
+        assert _plan(M, N, K, _lib.TG_MAJOR_K, 1) == SINGLE
+    status = ops.new_status("cuda")
+    y = ops.gemm_blockscaled(a, w, sa, sw, M=M, N=N, K=K, a_major=_lib.TG_MAJOR_K, b_major=_lib.TG_MAJOR_MN, sa_strides=(K // 128, 1),
+                             sb_strides=(1, N), sb_gran_n=1, out_dtype=out, status=status)
+    _close(y, (a.double() * sa.double().repeat_interleave(128, 1)) @ (w.double() * sw.double().repeat_interleave(128, 0)))
+    assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("T,K,N", [(1537, 256, 384), (4096, 768, 3072), (2000, 1024, 1160), (1700, 128, 200)])
+def test_column_scales_on_single_sms_weight_gradient(T, K, N):
+    from train_gpt_b200 import _lib, ops
+    gen = torch.Generator("cuda").manual_seed(T)
+    x, g = _f8(gen, T, K), _f8(gen, T, N + 15 & ~15)[:, :N]
+    tb = (T + 127) // 128
+    sx, sg = _scales(gen, tb, K), _scales(gen, tb, N)
+    assert _plan(K, N, T, _lib.TG_MAJOR_MN, 1) == SINGLE
+    status = ops.new_status("cuda")
+    dw = ops.gemm_blockscaled(x, g, sx, sg, M=K, N=N, K=T, a_major=_lib.TG_MAJOR_MN, b_major=_lib.TG_MAJOR_MN, sa_strides=(1, K), sb_strides=(1, N),
+                              sb_gran_n=1, status=status)
+    _close(dw, (x.double() * sx.double().repeat_interleave(128, 0)[:T]).t() @ (g.double() * sg.double().repeat_interleave(128, 0)[:T]))
     assert int(status.item()) == 0
 
 

@@ -19,7 +19,7 @@ INCLUDE = os.path.join(os.path.dirname(PKG_DIR), "include")
 LIB_PATH = os.path.join(PKG_DIR, "libtrain_gpt_b200.so")
 HOST_PATH = os.path.join(PKG_DIR, "_host.so")
 
-SOURCES = ["runtime.cu", "quantize.cu", "rmsnorm.cu", "gemm_fp8.cu", "gemm_pair.cu", "gemm_skinny.cu", "selftest.cu", "loss.cu", "optim.cu"]
+SOURCES = ["runtime.cu", "quantize.cu", "rmsnorm.cu", "gemm_fp8.cu", "gemm_ring.cu", "gemm_skinny.cu", "selftest.cu", "loss.cu", "optim.cu"]
 
 HOST_SOURCES = ["host.cpp", "step.cpp"]
 

@@ -698,7 +698,7 @@ splitk_reduce_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, 
 // narrow ones without this term); 4096 x 128 -> 1024, two waves, 4.9 / 4.5.  Over 288 problems of fewer than eight blocks the width
 // taken is 0.2 % slower than the better one on average (2.7 % without the term).
 //
-// A pair of SMs with a 256 x 256 tile (gemm_pair.cu) moves a third less from the L2 per block and promotes with fewer instructions, but it
+// A pair of SMs with a 256 x 256 tile (gemm_ring.cu) moves a third less from the L2 per block and promotes with fewer instructions, but it
 // starts later and a wave of it is coarser.  Measured on 720 uncut problems of 130 to 32768 rows, in turn with the widths above: three
 // waves of pairs and more 1.04-1.12 times as fast with a scale per 128 columns, 1.05-1.4 with a scale per column (8192 x 2048 -> 8192 147
 // against 158 us and 176 against 230; weight gradient 2048 x 8192 of 8192 tokens 203 / 234), half a wave or less 0.66-0.76.  Where
@@ -711,7 +711,8 @@ splitk_reduce_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, 
 struct GemmPlan {
   int bn, S;
   int64_t bytes;     // workspace the cut needs
-  bool pair;         // 256 x 256 tiles on pairs of SMs (gemm_pair.cu)
+  bool pair;         // 256 x 256 tiles on pairs of SMs (gemm_ring.cu)
+  bool ring;         // bn-wide tiles by gemm_ring.cu
 };
 // S of 1 to 8 ranges of at least 8 blocks by waves of wide tiles x (blocks per item + 3 for an item's ramp and stores), plus for
 // S > 1 the reduction over S float32 slices at 4 MB per block time.
@@ -732,7 +733,7 @@ static int training_ranges(const tg_gemm_args* a, int wide) {
 static GemmPlan plan_gemm(const tg_gemm_args* a) {
   const bool columns = a->sb_gran_n == 1;
   const int wide = a->N <= 128 ? 128 : columns ? 192 : 256;
-  GemmPlan pl = {wide, 1, 0, false};
+  GemmPlan pl = {wide, 1, 0, false, false};
   const int64_t nkb = (a->K + BK - 1) / BK;
   const int sms = gemm_sms();
   const bool whole = a->K % BK == 0 && (a->a_major == TG_MAJOR_MN || a->M % 128 == 0);      // (weight gradient: the tokens are K)
@@ -769,6 +770,9 @@ static GemmPlan plan_gemm(const tg_gemm_args* a) {
     pl.pair = us < best && (nkb >= 8 || waves >= 3);
     if (pl.pair) pl.bn = 256;
   }
+  // Column scales through gemm_ring.cu's ring, where the contraction is long enough for its later start (the measurement is there).
+  // Cut problems of 192-column tiles stay: their float32 tiles leave in three steps there (0.95-1.08 times as fast).
+  pl.ring = !pl.pair && columns && (nkb + pl.S - 1) / pl.S >= 12 && (pl.bn == 128 || (pl.bn == 192 && (pl.S == 1 && a->out_dtype == TG_OUT_BF16)));
   return pl;
 }
 
@@ -807,9 +811,11 @@ extern "C" int tgh_gemm_plan(const tg_gemm_args* a, int* tile_columns, int* rang
   return TG_OK;
 }
 
-extern "C" int tgh_gemm_takes_pairs(const tg_gemm_args* a, int* pairs) {
+extern "C" int tgh_gemm_kernel(const tg_gemm_args* a, int* kernel) {
   if (int rc = validate_gemm(a)) return rc;
-  *pairs = a->M > 0 && a->N > 0 && a->K > 0 && !skinny_takes(a) && plan_gemm(a).pair;
+  if (a->M == 0 || a->N == 0 || a->K == 0 || skinny_takes(a)) return TG_ERR_TOO_LARGE;
+  const GemmPlan pl = plan_gemm(a);
+  *kernel = pl.pair ? 2 : pl.ring ? 1 : 0;
   return TG_OK;
 }
 
@@ -861,7 +867,7 @@ extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
     p.d = a->workspace;
     p.ldd = a->N;
     int rc;
-    if (pl.pair) rc = pair_run(a, p, true, st);
+    if (pl.pair || pl.ring) rc = ring_run(a, p, pl.pair, bn, true, st);
     else if (bn == 256) rc = launch_gemm<256, 128, true>(a, p, st);
     else if (bn == 192) rc = launch_gemm<192, 1, true>(a, p, st);
     else rc = g1 ? launch_gemm<128, 1, true>(a, p, st) : launch_gemm<128, 128, true>(a, p, st);
@@ -873,7 +879,7 @@ extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
                                   static_cast<long long>(p.slice_elems)));
     return TG_OK;
   }
-  if (pl.pair) return pair_run(a, p, f32, st);
+  if (pl.pair || pl.ring) return ring_run(a, p, pl.pair, bn, f32, st);
   if (bn == 256) return f32 ? launch_gemm<256, 128, true>(a, p, st) : launch_gemm<256, 128, false>(a, p, st);
   if (bn == 192) return f32 ? launch_gemm<192, 1, true>(a, p, st) : launch_gemm<192, 1, false>(a, p, st);
   if (g1) return f32 ? launch_gemm<128, 1, true>(a, p, st) : launch_gemm<128, 1, false>(a, p, st);

@@ -1,22 +1,25 @@
-// Block-scaled e4m3 GEMM on pairs of SMs (tcgen05 cta_group::2): a cluster of two CTAs computes a 256 x 256 tile of
-//     D[m,n] = sum_kb SA(m,kb) SB(n,kb) sum_{k in kb} A[m,k] B[n,k].
-// CTA r of a pair owns rows 128 r.. of the tile (its tensor memory holds their accumulators) and loads its 128 rows of A and half of
-// the 256 rows of B; the tensor cores read the other half of B from the partner's shared memory.  Promotion is as in gemm_fp8.cu:
-// float32 scales, so every 128-deep contraction block is a chain of its own into a fresh accumulator buffer, which promotion warps
-// read, scale and add in registers; the same operations in the same order, hence the same bits.
+// Block-scaled e4m3 GEMM for large problems and long contractions,
+//     D[m,n] = sum_kb SA(m,kb) SB(n,kb) sum_{k in kb} A[m,k] B[n,k],
+// with the scales brought into a ring in shared memory and eight wide promotion warps.  Two forms:
+//   CG = 2  pairs of SMs (tcgen05 cta_group::2): a cluster of two CTAs computes a 256 x 256 tile.  CTA r of a pair owns rows 128 r.. of
+//           the tile (its tensor memory holds their accumulators) and loads its 128 rows of A and half of the 256 rows of B; the
+//           tensor cores read the other half of B from the partner's shared memory.
+//   CG = 1  one SM, 128 x 192 or 128 x 128 tiles, with a scale per column.
+// Promotion is as in gemm_fp8.cu: float32 scales, so every 128-deep contraction block is a chain of its own into a fresh accumulator
+// buffer, which promotion warps read, scale and add in registers; the same operations in the same order, hence the same bits.
 //
 // Warp roles of a CTA (384 threads):
-//   0-7   promotion + epilogue: warp w reads TMEM lanes 32 (w % 4).. (a hardware rule), accumulator columns 128 (w / 4)..
-//   8     TMA producer: one box of A, one of B per stage
-//   9     MMA issuer, in the pair's first CTA only
-//   10    scales: the block's row and column scales go into a ring in shared memory, as many blocks ahead as there are stages
+//   0-7   promotion + epilogue: warp w reads TMEM lanes 32 (w % 4).. (a hardware rule), columns BN / 2 (w / 4).. of the accumulator
+//   8     TMA producer
+//   9     MMA issuer (of a pair: in the first CTA only)
+//   10    scales: the block's row and column scales go into the ring, as many blocks ahead as there are stages
 //   11    the tile's bulk stores
 //
-// What bounds it: for large problems the board's power cap (1000 W; 32768 x 2048 -> 6144 in a loop of half a second runs at 1.36-1.40
-// GHz), else the promotion warps, which never find an accumulator missing: on each scheduler 2 x 64 packed FMAs of two cycles (twice that
-// with a scale per column) and the register writes of the TMEM loads, which hold the FMA pipe up: 375 cycles of a block's 512 on
-// the tensor core alone (666 with column scales), measured without MMAs, TMA or barriers; about 700 (1000) with everything.  So
-// the design keeps promotion short rather than wide:
+// What bounds the pairs: for large problems the board's power cap (1000 W; 32768 x 2048 -> 6144 in a loop of half a second runs at
+// 1.36-1.40 GHz), else the promotion warps, which never find an accumulator missing: on each scheduler 2 x 64 packed FMAs of two
+// cycles (twice that with a scale per column) and the register writes of the TMEM loads, which hold the FMA pipe up: 375 cycles of a
+// block's 512 on the tensor core alone (666 with column scales), measured without MMAs, TMA or barriers; about 700 (1000) with
+// everything.  So the design keeps promotion short rather than wide:
 //   - A pair moves 32 KB per SM and block from the L2 instead of 48, and one thread issues for two SMs.
 //   - Eight warps of 128 columns instead of sixteen of 64 (registers handed over, 224 each): half the barrier operations, scale loads and
 //     set-up per block.  1400 warp instructions per block of a tile instead of 1821.  (Sixteen: 434 us for the problem above, eight 415.)
@@ -25,8 +28,14 @@
 //   - A wait's outcome is looked at once a tile, not voted on in every block.
 //   - The buffer goes back by an arrival with CTA scope on the first CTA's barrier.  With cluster scope the release is a fence that waits
 //     for the SM's copies in flight: 700 us instead of 360.
-// Forward 32768 x 2048 -> 6144 in a loop: 435 us on single CTAs, 415 here (1.90 / 1.99 PFLOP/s); with a scale per column 555 / 500;
+// Forward 32768 x 2048 -> 6144 in a loop: 435 us with gemm_fp8.cu, 415 here (1.90 / 1.99 PFLOP/s); with a scale per column 555 / 500;
 // its weight gradient 584 / 550 (six waves where 5.2 would do); in short bursts 383 / 355, 530 / 435, 530 / 500.
+//
+// One SM with column scales: gemm_fp8.cu's promotion warps fetch and stage the scales of every block themselves, here they find them.
+// From twelve blocks on 1.05-1.4 times as fast in one wave (200 x 2048 -> 8192 9.6 / 8.8 us, 500 x 4096 -> 4096 19.4 / 14.7, weight gradient
+// 768 x 3072 of 4096 tokens 15.6 / 14.6), below it loses 0.2 us: scales come later to the first block, and eight warps take longer
+// over the last tile than sixteen.  The same with a scale per 128 columns (not built: 2 % slower below twelve blocks, +-2 % above).
+//
 // Tried and left out: the next block's barrier probed during a block (a try_wait that comes too early suspends the warp; with test_wait
 // 2 % slower), a ready counter in shared memory polled instead of the barrier (5 % slower), 32-column pieces in two register buffers
 // (spills), column-scale pieces in two register buffers (3 % slower: the FMA pipe, not the load's latency, is the limit).
@@ -88,63 +97,87 @@ __device__ __forceinline__ void umma_commit_both(uint32_t bar) {
 __device__ __forceinline__ void umma_commit_here(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+template <int CG>
+__device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  if constexpr (CG == 2) tma_load_2d_pair(dst, map, bar, x, y);
+  else tma_load_2d(dst, map, bar, x, y);
+}
+template <int CG>
+__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (CG == 2) umma_f8_pair(d_tmem, a_desc, b_desc, idesc, accumulate);
+  else umma_f8(d_tmem, a_desc, b_desc, idesc, accumulate);
+}
+template <int CG>
+__device__ __forceinline__ void commit(uint32_t bar) {
+  if constexpr (CG == 2) umma_commit_both(bar);
+  else umma_commit(bar);
+}
 // four bytes from memory to shared memory (any 4-byte alignment), through L1: a row scale's sector serves eight blocks
 __device__ __forceinline__ void cp_async_4(uint32_t dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 // ---- kernel --------------------------------------------------------------------------------
 
-constexpr int kPairBandRows = 8;      // tile rows per band of the numbering: 74 pairs cover a patch of about 8 x 9 tiles
+constexpr int kBandRows = 16;      // 128-row tiles per band of the numbering (see tile_coords)
 
-template <int SB_GRAN, bool OUT_F32>
-struct PairCfg {
-  static constexpr int BN = 256;
+// Compile-time plan of one variant: CG CTAs (a cluster of two, or one) on a tile of 128 CG rows x BN columns.
+template <int CG, int BN_, int SB_GRAN, bool OUT_F32>
+struct RingCfg {
+  static constexpr int BN = BN_;
   static constexpr int promo_warps = 8;
-  static constexpr int producer_warp = promo_warps, issuer_warp = promo_warps + 1, scale_warp = promo_warps + 2, store_warp = promo_warps + 3;
-  static constexpr int threads = 32 * (promo_warps + 4);
+  static constexpr int producer_warp = 8, issuer_warp = 9, scale_warp = 10, store_warp = 11;
+  static constexpr int threads = 384;
   // 168 registers a thread at launch; the service warpgroup hands over what the two promotion warpgroups grow by
   static constexpr int launch_regs = 168, promo_regs = 224, service_regs = 56;
-  static_assert(service_regs + promo_warps / 4 * promo_regs <= (promo_warps / 4 + 1) * launch_regs, "register hand-over asks for more than is released");
-  static constexpr int cols = 1024 / promo_warps, pieces = cols / 16;
-                             // accumulator columns of a warp
-  static constexpr int stage_bytes = 2 * kTileBytes;           // A and half of B
-  static constexpr int box_bytes = 32 * 128;                   // an output box: 32 rows of 128 bytes
-  static constexpr int warp_boxes = 16 / promo_warps;                         // staged at a time
+  static_assert(service_regs + 2 * promo_regs <= 3 * launch_regs, "register hand-over asks for more than is released");
+  static constexpr int cols = BN / 2, pieces = cols / 16;      // accumulator columns of a warp, in pieces of 16
+  // Column scales: the fragment layout of an MMA accumulator (a thread holds 4 rows x cols / 4 columns instead of one row), in which a
+  // column scale is shared by 8 lanes instead of all 32.
+  static constexpr bool frag = SB_GRAN == 1;
+  static_assert(frag || pieces % 2 == 0, "two register buffers take turns");
+  static constexpr int tmem_bufs = BN > 128 ? 2 : 4, tmem_stride = kTmemCols / tmem_bufs;
+  static constexpr int b_boxes = CG == 2 ? 1 : (BN + 127) / 128;   // (a CTA of a pair loads half of B)
+  static_assert(CG == 1 || BN == 256, "a pair's tile");
+  static constexpr int stage_bytes = (1 + b_boxes) * kTileBytes;
+  // output boxes: 32 rows of box_cols columns; warp_boxes of them are staged at a time
   static constexpr int esize = OUT_F32 ? 4 : 2;
-  static constexpr int box_cols = 128 / esize;
+  static constexpr int box_cols = cols % (128 / esize) == 0 ? 128 / esize : 32;
+  static constexpr int box_row = box_cols * esize, box_bytes = 32 * box_row, box_pieces = box_cols / 16;
+  static constexpr int warp_boxes = cols / box_cols * box_bytes <= 8192 ? cols / box_cols : BN == 256 ? 2 : 1;
   static constexpr int phases = cols / (warp_boxes * box_cols);
+  static_assert(phases * warp_boxes * box_cols == cols && (box_row == 128 || (box_row == 64 && frag)), "output boxes");
   static constexpr int out_bytes = promo_warps * warp_boxes * box_bytes;
-  // a ring slot: 128 row scales, then the column scales (256, or one per 128 columns)
-  static constexpr int slot_floats = 128 + (SB_GRAN == 1 ? 256 : 4);
+  // a ring slot: 128 row scales, then the column scales (BN, or one per 128 columns)
+  static constexpr int slot_floats = 128 + (SB_GRAN == 1 ? BN : 4);
   static constexpr int static_reserve = 1024;
-  static constexpr int stages_fit = (kSmemLimit - static_reserve - out_bytes - 2 * 4 * slot_floats) / (stage_bytes + 4 * slot_floats);
+  static constexpr int stages_fit = (kSmemLimit - static_reserve - out_bytes - tmem_bufs * 4 * slot_floats) / (stage_bytes + 4 * slot_floats);
   static constexpr int stages = stages_fit > 6 ? 6 : stages_fit;
   // The scales of block i go into slot i % ring once the stage of block i is free, that is, once the MMAs of block i - stages are
-  // done.  Those were issued after every promotion warp had given back the accumulator of block i - stages - 2, which it does
+  // done.  Those were issued after every promotion warp had given back the accumulator of block i - stages - tmem_bufs, which it does
   // after its last look at that block's scales.
-  static constexpr int ring = stages + 2;
+  static constexpr int ring = stages + tmem_bufs;
   static constexpr int off_out = stages * stage_bytes;
   static constexpr int off_ring = off_out + out_bytes;
   static constexpr int smem_bytes = off_ring + ring * slot_floats * 4;
-  static constexpr int n_bars = 2 * stages + 2 * 2 + 3;
+  static constexpr int n_bars = 2 * stages + 2 * tmem_bufs + 3;
   static_assert(n_bars <= 24, "control block too small");
-  static_assert(stages >= 3 && smem_bytes + static_reserve <= kSmemLimit, "shared-memory plan");
+  static_assert(stages >= 3 && stages >= tmem_bufs && smem_bytes + static_reserve <= kSmemLimit, "shared-memory plan");
 };
 
-template <int SB_GRAN, bool OUT_F32>
-__global__ void __launch_bounds__((PairCfg<SB_GRAN, OUT_F32>::threads), 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+template <int CG, int BN_, int SB_GRAN, bool OUT_F32>
+__global__ void __launch_bounds__((RingCfg<CG, BN_, SB_GRAN, OUT_F32>::threads), 1)
+gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const __grid_constant__ CUtensorMap tmap_d, const GemmParams p) {
-  using C = PairCfg<SB_GRAN, OUT_F32>;
-  constexpr int BN = C::BN, kStages = C::stages, kRing = C::ring;
+  using C = RingCfg<CG, BN_, SB_GRAN, OUT_F32>;
+  constexpr int BN = C::BN, kStages = C::stages, kRing = C::ring, kBufs = C::tmem_bufs;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(16) uint64_t ctl_bars[24];
   __shared__ uint32_t ctl_tmem_ptr;
   __shared__ int ctl_abort;
   const uint32_t sbase = smem_u32(smem);
   const uint32_t full0 = smem_u32(ctl_bars), empty0 = full0 + 8u * kStages;
-  const uint32_t tfull0 = empty0 + 8u * kStages, tempty0 = tfull0 + 16u;
-  const uint32_t drain_bar = tempty0 + 16u, staged_bar = drain_bar + 8u, unstaged_bar = drain_bar + 16u;
+  const uint32_t tfull0 = empty0 + 8u * kStages, tempty0 = tfull0 + 8u * kBufs;
+  const uint32_t drain_bar = tempty0 + 8u * kBufs, staged_bar = drain_bar + 8u, unstaged_bar = drain_bar + 16u;
   volatile uint32_t* tmem_ptr_smem = &ctl_tmem_ptr;
   volatile int* abort_flag = &ctl_abort;
 
@@ -154,19 +187,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   }
 
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_rank();
+  const uint32_t rank = CG == 2 ? cluster_rank() : 0u;
   const int n_tiles = p.tiles_m * p.tiles_n;
   const int n_items = n_tiles * p.ksplit;
-  const int first_item = int(blockIdx.x >> 1), item_step = int(gridDim.x >> 1);
+  const int first_item = int(blockIdx.x) / CG, item_step = int(gridDim.x) / CG;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(full0 + 8u * s, 1);            // (the first CTA's counts the bytes of both)
       mbar_init(empty0 + 8u * s, 1);
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kBufs; ++b) {
       mbar_init(tfull0 + 8u * b, 2);           // the block's MMAs and its scales
-      mbar_init(tempty0 + 8u * b, 2 * C::promo_warps);
+      mbar_init(tempty0 + 8u * b, CG * C::promo_warps);
     }
     mbar_init(drain_bar, 1);
     mbar_init(staged_bar, C::promo_warps);
@@ -177,11 +210,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_b)) : "memory");
   }
   if (warp == C::issuer_warp) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl_tmem_ptr)), "r"(uint32_t(kTmemCols)) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    if constexpr (CG == 2) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl_tmem_ptr)), "r"(uint32_t(kTmemCols)) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      tmem_alloc(smem_u32(&ctl_tmem_ptr), kTmemCols);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
-  cluster_sync();              // both CTAs' barriers exist before either signals across
+  if constexpr (CG == 2) cluster_sync();              // both CTAs' barriers exist before either signals across
+  else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
   grid_trigger();
@@ -193,12 +232,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       // ------------------------------ TMA producer -------------------------------------
       uint32_t s = 0, ph = 1;
       bool ok = true;
-      const uint32_t full_leader = map_rank(full0, 0u);
+      const uint32_t full_leader = CG == 2 ? map_rank(full0, 0u) : full0;
       for (int item = first_item; ok && item < n_items; item += item_step) {
         int ks, tile, tm, tn;
         item_split(p, item, n_tiles, ks, tile);
         tile_coords(p, tile, tm, tn);
-        const int m0 = tm * 2 * BM + int(rank) * BM, n0 = tn * BN + int(rank) * 128;     // (past M or N: zeros)
+        const int m0 = (tm * CG + int(rank)) * BM, n0 = tn * BN + int(rank) * 128;     // (past M or N: zeros)
         int k0 = range_first(p, ks) * BK;
         const int nkb = range_blocks(p, ks);
         for (int kb = 0; kb < nkb; ++kb, k0 += BK) {
@@ -208,9 +247,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             const uint32_t dst = sbase + s * C::stage_bytes, fb = full_leader + 8u * s;
             // The first CTA announces the bytes of both.  The second's may land before that: its barrier phase is the same one,
             // since the stage was free in both CTAs only after the phase before had completed.
-            if (rank == 0) mbar_expect_tx(full0 + 8u * s, 2 * C::stage_bytes);
-            tma_load_2d_pair(dst, &tmap_a, fb, p.a_mn ? m0 : k0, p.a_mn ? k0 : m0);
-            tma_load_2d_pair(dst + kTileBytes, &tmap_b, fb, p.b_mn ? n0 : k0, p.b_mn ? k0 : n0);
+            if (rank == 0) mbar_expect_tx(full0 + 8u * s, CG * C::stage_bytes);
+            tma_load<CG>(dst, &tmap_a, fb, p.a_mn ? m0 : k0, p.a_mn ? k0 : m0);
+#pragma unroll
+            for (int b = 0; b < C::b_boxes; ++b) {
+              const int nb = n0 + b * 128;
+              tma_load<CG>(dst + (1 + b) * kTileBytes, &tmap_b, fb, p.b_mn ? nb : k0, p.b_mn ? k0 : nb);
+            }
           }
           __syncwarp();
           if (++s == kStages) { s = 0; ph ^= 1u; }
@@ -221,7 +264,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       if (rank == 0) {
         // D f32 (bit 4), A/B e4m3 (0), major bits 15/16, N>>3 at 17, M>>4 at 24
         const uint32_t idesc = (1u << 4) | (uint32_t(p.a_mn) << 15) | (uint32_t(p.b_mn) << 16) | (uint32_t(BN >> 3) << 17) |
-                               (uint32_t(2 * BM >> 4) << 24);
+                               (uint32_t(CG * BM >> 4) << 24);
         const uint32_t a_step = p.a_mn ? (UMMA_K * 128) >> 4 : UMMA_K >> 4;
         const uint32_t b_step = p.b_mn ? (UMMA_K * 128) >> 4 : UMMA_K >> 4;
         const uint64_t desc_a0 = make_smem_desc(sbase), desc_b0 = make_smem_desc(sbase + kTileBytes);
@@ -243,55 +286,56 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
-            const uint32_t d_tmem = tmem_base + buf * uint32_t(BN);
+            const uint32_t d_tmem = tmem_base + buf * uint32_t(C::tmem_stride);
 #pragma unroll
             for (int k = 0; k < BK / UMMA_K; ++k)
-              umma_f8_pair(d_tmem, (uint64_t(desc_hi) << 32) | (a_lo0 + soff + k * a_step),
+              umma<CG>(d_tmem, (uint64_t(desc_hi) << 32) | (a_lo0 + soff + k * a_step),
                            (uint64_t(desc_hi) << 32) | (b_lo0 + soff + k * b_step), idesc, k > 0 ? 1u : 0u);
-            umma_commit_both(tfull0 + 8u * buf);
-            umma_commit_both(empty0 + 8u * s);
+            if constexpr (CG == 1) commit<CG>(empty0 + 8u * s);
+            commit<CG>(tfull0 + 8u * buf);
+            if constexpr (CG == 2) commit<CG>(empty0 + 8u * s);
           }
           __syncwarp();
           soff += uint32_t(C::stage_bytes >> 4);
           if (++s == kStages) { s = 0; sph ^= 1u; soff = 0; }
-          buf ^= 1u;
-          bph ^= buf ^ 1u;
+          if (++buf == kBufs) { buf = 0; bph ^= 1u; }
         }
         // nothing issued here may still be running when tensor memory is freed
         if (elect_one()) {
-          umma_commit_here(drain_bar);
+          if constexpr (CG == 2) umma_commit_here(drain_bar);
+          else umma_commit(drain_bar);
           mbar_wait(drain_bar, 0u, abort_flag, p.status, 4u);
         }
         __syncwarp();
       }
     } else if (warp == C::scale_warp) {
       // ------------------------------ scales --------------------------------------------
-      // Copies run two blocks ahead of the announcement: block j's scales are announced on its accumulator's barrier, beside its MMAs,
-      // once that barrier is through with block j - 2.  The MMAs of block i wait for the announcement of block i - 2, which comes after
-      // the copy of block i: so while that copy waits for its stage, the stage's barrier cannot go on to the phase after.  (The first
-      // blocks' MMAs wait for no announcement: their copies must not look at the barrier, and need not.)
+      // Copies run as many blocks ahead of the announcement as there are accumulators: block j's scales are announced on its
+      // accumulator's barrier, beside its MMAs, once that barrier is through with the block before.  The MMAs of block i wait for the
+      // announcement of block i - tmem_bufs, which comes after the copy of block i: so while that copy waits for its stage, the stage's
+      // barrier cannot go on to the phase after.  (The first blocks' MMAs wait for no announcement: their copies must not look at the
+      // barrier, and need not.)
       uint32_t s = 0, ph = 1, slot = 0, buf = 0, bph = 1, copied = 0;
       bool ok = true;
       const uint32_t is_lane0 = lane == 0;
       auto announce = [&]() {
         ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8u * buf, bph, abort_flag, p.status, 9u));
         mbar_arrive_if(tfull0 + 8u * buf, is_lane0);
-        buf ^= 1u;
-        bph ^= buf ^ 1u;
+        if (++buf == kBufs) { buf = 0; bph ^= 1u; }
       };
       for (int item = first_item; ok && item < n_items; item += item_step) {
         int ks, tile, tm, tn;
         item_split(p, item, n_tiles, ks, tile);
         tile_coords(p, tile, tm, tn);
-        const int m0 = tm * 2 * BM + int(rank) * BM, n0 = tn * BN;
+        const int m0 = (tm * CG + int(rank)) * BM, n0 = tn * BN;
         const uint32_t kb0 = uint32_t(range_first(p, ks));
         // element offsets (the host checks that they fit 32 bits); rows and columns past the end read a valid scale
-        uint32_t sa_off[4], sb_off[SB_GRAN == 1 ? 8 : 1];
+        uint32_t sa_off[4], sb_off[SB_GRAN == 1 ? BN / 32 : 1];
 #pragma unroll
         for (int i = 0; i < 4; ++i) sa_off[i] = uint32_t(min(m0 + lane + 32 * i, p.M - 1)) * uint32_t(p.sa_sm) + kb0 * uint32_t(p.sa_sk);
         if (SB_GRAN == 1) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) sb_off[i] = uint32_t(min(n0 + lane + 32 * i, p.N - 1)) * uint32_t(p.sb_sn) + kb0 * uint32_t(p.sb_sk);
+          for (int i = 0; i < BN / 32; ++i) sb_off[i] = uint32_t(min(n0 + lane + 32 * i, p.N - 1)) * uint32_t(p.sb_sn) + kb0 * uint32_t(p.sb_sk);
         } else {
           sb_off[0] = uint32_t(min(n0 / 128 + (lane & 1), (p.N - 1) / 128)) * uint32_t(p.sb_sn) + kb0 * uint32_t(p.sb_sk);
         }
@@ -309,32 +353,32 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
           if (SB_GRAN == 1) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < BN / 32; ++i) {
               cp_async_4(dst + 512u + 128u * i, p.sb + sb_off[i]);
               sb_off[i] += uint32_t(p.sb_sk);
             }
           } else {
-            if (lane < 2) cp_async_4(dst + 512u, p.sb + sb_off[0]);
+            if (lane < BN / 128) cp_async_4(dst + 512u, p.sb + sb_off[0]);
             sb_off[0] += uint32_t(p.sb_sk);
           }
           asm volatile("cp.async.commit_group;" ::: "memory");
           if (++s == kStages) { s = 0; ph ^= 1u; }
           if (++slot == kRing) slot = 0;
-          if (++copied > 2) {
-            asm volatile("cp.async.wait_group 2;" ::: "memory");
+          if (++copied > kBufs) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kBufs) : "memory");
             announce();
             if (!ok) break;
           }
         }
       }
       asm volatile("cp.async.wait_all;" ::: "memory");
-      if (ok && copied > 1) announce();
-      if (ok && copied > 0) announce();
+#pragma unroll 1
+      for (uint32_t left = min(copied, uint32_t(kBufs)); ok && left > 0; --left) announce();
     } else {
       // ------------------------------ tile stores ----------------------------------------
       uint32_t sph = 0;
       bool ok = true;
-      for (int item = first_item; ok && item < n_items; item += item_step) {
+      for (int item = first_item; ok && item + item_step < n_items; item += item_step) {      // (all but the last)
         int ks, tile, tm, tn;
         item_split(p, item, n_tiles, ks, tile);
         tile_coords(p, tile, tm, tn);
@@ -350,7 +394,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
               for (int h = 0; h < C::warp_boxes; ++h)
                 tma_store_3d_nocommit(&tmap_d, sbase + C::off_out + uint32_t(w * C::warp_boxes + h) * C::box_bytes,
                                       tn * BN + (w >> 2) * C::cols + (phase * C::warp_boxes + h) * C::box_cols,
-                                      tm * 2 * BM + int(rank) * BM + (w & 3) * 32, ks);
+                                      (tm * CG + int(rank)) * BM + (w & 3) * 32, ks);
             }
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             tma_store_wait_read();
@@ -365,13 +409,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::promo_regs));
     const int quarter = warp & 3, cg = warp >> 2;
     const int r = quarter * 32 + lane;
-    constexpr bool kFrag = SB_GRAN == 1;
+    constexpr bool kFrag = C::frag;
     const int fg = lane >> 2, fj = lane & 3;     // fragment coordinates: rows fg + 8 i, column pairs 8 k + 2 fj
     const float* ring = reinterpret_cast<const float*>(smem + C::off_ring);
     const uint32_t tcol0 = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(cg * C::cols);
     const int sb_index = cg * C::cols / 128;
     const uint32_t wb = sbase + C::off_out + uint32_t(warp) * (C::warp_boxes * C::box_bytes);
-    const uint32_t tempty_leader = map_rank(tempty0, 0u);
+    const uint32_t tempty_leader = CG == 2 ? map_rank(tempty0, 0u) : tempty0;
     const uint32_t is_lane0 = lane == 0;
     uint32_t buf = 0, bph = 0, uph = 1, slot = 0;
     // A wait that gives up has raised the abort flag, and every wait after it returns at once: the warps look at `ok` once a tile.
@@ -379,7 +423,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     auto release = [&](uint32_t b) {
       tc_fence_before();
       __syncwarp();
-      mbar_arrive_cluster_if(tempty_leader + 8u * b, is_lane0);
+      if constexpr (CG == 2) mbar_arrive_cluster_if(tempty_leader + 8u * b, is_lane0);
+      else mbar_arrive_if(tempty_leader + 8u * b, is_lane0);
     };
     for (int item = first_item; item < n_items; item += item_step) {
       float2 acc[C::cols / 2];
@@ -401,14 +446,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       };
       auto leave_block = [&]() {
         release(buf);
-        buf ^= 1u;
-        bph ^= buf ^ 1u;
+        if (++buf == kBufs) { buf = 0; bph ^= 1u; }
       };
       if constexpr (kFrag) {
 #pragma unroll 1
         for (int kb = 0; kb < nkb; ++kb) {
           const float* sc = enter_block();
-          const uint32_t taddr = tcol0 + buf * uint32_t(BN);
+          const uint32_t taddr = tcol0 + buf * uint32_t(C::tmem_stride);
           float sa_r[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) sa_r[i] = sc[quarter * 32 + fg + 8 * i];
@@ -423,7 +467,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             tmem_ld_frag16(taddr + 16 * q, v);
             tmem_ld_frag16(taddr + (16u << 16) + 16 * q, v + 8);
             tmem_wait_ld16(v);
-            if (q == C::pieces - 1) leave_block();         // (after the last look at the scales, see PairCfg::ring)
+            if (q == C::pieces - 1) leave_block();         // (after the last look at the scales, see RingCfg::ring)
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
 #pragma unroll
@@ -441,7 +485,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         uint32_t v[2][16];
         const float* sc = enter_block();
         float s = sc[r] * sc[128 + sb_index];
-        uint32_t taddr = tcol0 + buf * uint32_t(BN);
+        uint32_t taddr = tcol0 + buf * uint32_t(C::tmem_stride);
         tmem_ld16(taddr, v[0]);
 #pragma unroll 1
         for (int kb = 0; kb < nkb; ++kb) {
@@ -457,7 +501,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           float s_next = 0.f;
           if (more) {
             sc = enter_block();
-            taddr = tcol0 + buf * uint32_t(BN);
+            taddr = tcol0 + buf * uint32_t(C::tmem_stride);
             tmem_ld16(taddr, v[0]);
             s_next = sc[r] * sc[128 + sb_index];
           }
@@ -467,32 +511,32 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       }
       if (!__all_sync(0xffffffffu, ok)) break;
 
-      // ---- epilogue: registers -> this warp's swizzled staging rows; the store warp does the rest ----
+      // ---- epilogue: registers -> this warp's swizzled staging rows -> bulk stores ----
+      const bool last = item + item_step >= n_items;
 #pragma unroll
       for (int phase = 0; phase < C::phases; ++phase) {
-        // (the first pass finds the rows free)
-        ok = __all_sync(0xffffffffu, mbar_wait(unstaged_bar, uph, abort_flag, p.status, 8u));
-        if (!ok) break;
-        uph ^= 1u;
-        if constexpr (kFrag && OUT_F32) {
-          // 16-byte chunk 4 (q % 2) + 2 k + (fj >> 1) of box q / 2, half fj & 1
-          const uint32_t base = wb + uint32_t(fg) * 128u + (uint32_t(fj >> 1) << 4) + 8u * uint32_t(fj & 1), flip = uint32_t(fg) << 4;
-          static_loop<2 * C::warp_boxes>([&](auto qq) {
+        // The store warp hands a tile's boxes to the copy engine one after the other (40 cycles each), beside the next tile's first
+        // blocks.  After the last tile nothing hides that: every warp issues its own.
+        if (!last || phase == 0) {         // (the first pass finds the rows free)
+          ok = __all_sync(0xffffffffu, mbar_wait(unstaged_bar, uph, abort_flag, p.status, 8u));
+          if (!ok) break;
+          uph ^= 1u;
+        } else {
+          if (is_lane0) tma_store_wait_read();
+          __syncwarp();
+        }
+        if constexpr (kFrag) {
+          // rows fg + 8 i; bf16: 16-byte chunk 2 q + k of the box's row, 4 fj bytes in; float32: chunk 4 q + 2 k + (fj >> 1), half fj & 1.
+          // Swizzle: chunk xor the row's low three bits, with 64-byte rows xor the two above the lowest.
+          const uint32_t base = wb + uint32_t(fg) * C::box_row + (OUT_F32 ? (uint32_t(fj >> 1) << 4) + 8u * uint32_t(fj & 1) : 4u * uint32_t(fj));
+          const uint32_t flip = (C::box_row == 128 ? uint32_t(fg) : uint32_t(fg >> 1)) << 4;
+          static_loop<C::warp_boxes * C::box_pieces>([&](auto qq) {
             static_loop<4>([&](auto i) {
               static_loop<2>([&](auto k) {
-                const float2 a = acc[(4 * (2 * C::warp_boxes * phase + qq.value) + i.value) * 2 + k.value];
-                sts_swz_f32x2<(qq.value >> 1) * C::box_bytes + i.value * 1024 + (4 * (qq.value & 1) + 2 * k.value) * 16>(base, flip, a);
-              });
-            });
-          });
-        } else if constexpr (kFrag) {
-          // 16-byte chunk 2 (q % 4) + k of box q / 4, 4 fj bytes in
-          const uint32_t base = wb + uint32_t(fg) * 128u + 4u * uint32_t(fj), flip = uint32_t(fg) << 4;
-          static_loop<C::pieces>([&](auto q) {
-            static_loop<4>([&](auto i) {
-              static_loop<2>([&](auto k) {
-                const float2 a = acc[(4 * q.value + i.value) * 2 + k.value];
-                sts_swz_b32<(q.value >> 2) * C::box_bytes + i.value * 1024 + (2 * (q.value & 3) + k.value) * 16>(base, flip, pack_bf16x2(a.x, a.y));
+                constexpr int q = qq.value % C::box_pieces, off = (qq.value / C::box_pieces) * C::box_bytes + i.value * 8 * C::box_row;
+                const float2 a = acc[(4 * (phase * C::warp_boxes * C::box_pieces + qq.value) + i.value) * 2 + k.value];
+                if constexpr (OUT_F32) sts_swz_f32x2<off + (4 * q + 2 * k.value) * 16>(base, flip, a);
+                else sts_swz_b32<off + (2 * q + k.value) * 16>(base, flip, pack_bf16x2(a.x, a.y));
               });
             });
           });
@@ -513,37 +557,56 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the copy engine
         __syncwarp();
-        mbar_arrive_if(staged_bar, is_lane0);
+        if (!last) {
+          mbar_arrive_if(staged_bar, is_lane0);
+        } else if (is_lane0) {
+          int ks, tile, tm, tn;
+          item_split(p, item, n_tiles, ks, tile);
+          tile_coords(p, tile, tm, tn);
+#pragma unroll
+          for (int h = 0; h < C::warp_boxes; ++h)
+            tma_store_3d_nocommit(&tmap_d, wb + uint32_t(h) * C::box_bytes, tn * BN + cg * C::cols + (phase * C::warp_boxes + h) * C::box_cols,
+                                  (tm * CG + int(rank)) * BM + quarter * 32, ks);
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+        __syncwarp();
       }
       if (!ok) break;
     }
   }
 
   // ------------------------------ teardown ----------------------------------------------
+  // the last bulk stores must have read their staging rows before the CTA's shared memory goes away
+  if (warp < C::promo_warps && lane == 0) tma_store_wait_read();
+  __syncwarp();
   tc_fence_before();
-  cluster_sync();              // the partner no longer reads this CTA's shared memory or signals its barriers
+  if constexpr (CG == 2) cluster_sync();              // the partner no longer reads this CTA's shared memory or signals its barriers
+  else __syncthreads();
   if (warp == C::issuer_warp) {
     __syncwarp();
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(uint32_t(kTmemCols)) : "memory");
+    if constexpr (CG == 2)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(uint32_t(kTmemCols)) : "memory");
+    else
+      tmem_dealloc(tmem_base, kTmemCols);
   }
 }
 
 // ---- host ------------------------------------------------------------------------------
 
-template <int SB_GRAN, bool OUT_F32>
-static int launch_pair(const tg_gemm_args* a, GemmParams p, cudaStream_t st) {
-  using C = PairCfg<SB_GRAN, OUT_F32>;
-  auto kern = gemm_pair_kernel<SB_GRAN, OUT_F32>;
+template <int CG, int BN, int SB_GRAN, bool OUT_F32>
+static int launch_ring(const tg_gemm_args* a, GemmParams p, cudaStream_t st) {
+  using C = RingCfg<CG, BN, SB_GRAN, OUT_F32>;
+  auto kern = gemm_ring_kernel<CG, BN, SB_GRAN, OUT_F32>;
   CUtensorMap ta, tb, td;
   const int64_t a_inner = p.a_mn ? a->M : a->K, a_outer = p.a_mn ? a->K : a->M;
   const int64_t b_inner = p.b_mn ? a->N : a->K, b_outer = p.b_mn ? a->K : a->N;
   if (int rc = make_tmap(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->a, a_inner, a_outer, a->lda, 128, 128)) return rc;
   if (int rc = make_tmap(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->b, b_inner, b_outer, a->ldb, 128, 128)) return rc;
-  if (int rc = make_output_map(&td, OUT_F32, a, p, C::box_cols, 128)) return rc;
-  p.tiles_m = int((a->M + 2 * BM - 1) / (2 * BM));
-  p.tiles_n = int((a->N + C::BN - 1) / C::BN);
-  p.band = std::min(p.tiles_m, kPairBandRows);
+  if (int rc = make_output_map(&td, OUT_F32, a, p, C::box_cols, C::box_row)) return rc;
+  p.tiles_m = int((a->M + CG * BM - 1) / (CG * BM));
+  p.tiles_n = int((a->N + BN - 1) / BN);
+  p.band = std::min(p.tiles_m, kBandRows / CG);
   if (int rc = set_reciprocals(p)) return rc;
   const int n_items = p.tiles_m * p.tiles_n * p.ksplit;
   int dev = 0;
@@ -551,7 +614,7 @@ static int launch_pair(const tg_gemm_args* a, GemmParams p, cudaStream_t st) {
   if (dev < 0 || dev >= 64) return TG_ERR_SHAPE;
   cudaLaunchAttribute attrs[2];
   attrs[0].id = cudaLaunchAttributeClusterDimension;
-  attrs[0].val.clusterDim.x = 2;
+  attrs[0].val.clusterDim.x = CG;
   attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
   attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attrs[1].val.programmaticStreamSerializationAllowed = 1;
@@ -561,26 +624,31 @@ static int launch_pair(const tg_gemm_args* a, GemmParams p, cudaStream_t st) {
   cfg.attrs = attrs;
   cfg.numAttrs = 1;
   // once per device: the kernel's shared memory, and how many pairs run at a time (a pair takes two SMs of one cluster group)
-  static std::atomic<int> pairs_of[64];
-  int fit = pairs_of[dev].load(std::memory_order_acquire);
+  static std::atomic<int> units_of[64];
+  int fit = units_of[dev].load(std::memory_order_acquire);
   if (fit == 0) {
     TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem_bytes));
-    cfg.gridDim = dim3(unsigned(sm_count() & ~1));
-    TG_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&fit, kern, &cfg));
+    fit = sm_count();
+    if (CG == 2) {
+      cfg.gridDim = dim3(unsigned(sm_count() & ~1));
+      TG_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&fit, kern, &cfg));
+    }
     if (fit < 1) return record_cuda_error(cudaErrorLaunchOutOfResources, "no CTA pair fits on this device");
-    pairs_of[dev].store(fit, std::memory_order_release);
+    units_of[dev].store(fit, std::memory_order_release);
   }
-  const int pairs = std::max(1, std::min(fit, gemm_sms() / 2));
-  cfg.gridDim = dim3(unsigned(2 * std::min(n_items, pairs)));
+  const int units = std::max(1, std::min(fit, gemm_sms() / CG));
+  cfg.gridDim = dim3(unsigned(CG * std::min(n_items, units)));
   cfg.stream = st;
-  if (n_items <= 4 * pairs && p.nkb <= 32) cfg.numAttrs = 2;      // a short kernel starts early, as in gemm_fp8.cu
+  if ((p.a_mn == 0 && a->M <= 256) || (n_items <= 4 * units && p.nkb <= 32)) cfg.numAttrs = 2;
   TG_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, ta, tb, td, p));
   return TG_OK;
 }
 
-int pair_run(const tg_gemm_args* a, const GemmParams& p, bool out_f32, cudaStream_t st) {
-  if (a->sb_gran_n == 1) return out_f32 ? launch_pair<1, true>(a, p, st) : launch_pair<1, false>(a, p, st);
-  return out_f32 ? launch_pair<128, true>(a, p, st) : launch_pair<128, false>(a, p, st);
+int ring_run(const tg_gemm_args* a, const GemmParams& p, bool pair, int bn, bool f32, cudaStream_t st) {
+  if (pair && a->sb_gran_n == 1) return f32 ? launch_ring<2, 256, 1, true>(a, p, st) : launch_ring<2, 256, 1, false>(a, p, st);
+  if (pair) return f32 ? launch_ring<2, 256, 128, true>(a, p, st) : launch_ring<2, 256, 128, false>(a, p, st);
+  if (bn == 192) return launch_ring<1, 192, 1, false>(a, p, st);
+  return f32 ? launch_ring<1, 128, 1, true>(a, p, st) : launch_ring<1, 128, 1, false>(a, p, st);
 }
 
 }  // namespace tg

@@ -1,4 +1,4 @@
-// What the two tiled block-scaled GEMM kernels (gemm_fp8.cu, gemm_pair.cu) share: their parameters, the numbering of the work items,
+// What the two tiled block-scaled GEMM kernels (gemm_fp8.cu, gemm_ring.cu) share: their parameters, the numbering of the work items,
 // the promotion of a piece of an accumulator, the epilogue's staging stores.
 #pragma once
 
@@ -160,7 +160,7 @@ inline int set_reciprocals(GemmParams& p) {
   return n_items > INT32_MAX || n_items * (p.nkb + 1) > INT32_MAX ? TG_ERR_TOO_LARGE : TG_OK;
 }
 
-// The kernel on pairs of SMs (gemm_pair.cu).
-int pair_run(const tg_gemm_args* a, const GemmParams& p, bool out_f32, cudaStream_t st);
+// The kernel of gemm_ring.cu: on pairs of SMs, or 128 x bn tiles with a scale per column.
+int ring_run(const tg_gemm_args* a, const GemmParams& p, bool pair, int bn, bool f32, cudaStream_t st);
 
 }  // namespace tg

@@ -30,8 +30,8 @@ int tgh_quantize_jobs(const tgh_quantize_job* jobs, int n, void* stream);
 /* Columns of the output tiles, and ranges that the contraction is cut into, for a problem that the tiled GEMM takes (TG_ERR_TOO_LARGE:
  * the few-token kernel does).  Needs no GPU. */
 int tgh_gemm_plan(const tg_gemm_args* args, int* tile_columns, int* ranges);
-/* Whether a problem goes to the kernel on pairs of SMs.  Needs no GPU. */
-int tgh_gemm_takes_pairs(const tg_gemm_args* args, int* pairs);
+/* Which tiled kernel a problem goes to: 0 gemm_fp8.cu, 1 gemm_ring.cu on single SMs, 2 the same on pairs of SMs.  Needs no GPU. */
+int tgh_gemm_kernel(const tg_gemm_args* args, int* kernel);
 
 /* Whether tgh_softcap_ce takes this problem (a row and its cap fit the one-pass kernel). */
 int tgh_softcap_ce_fits(float cap, int64_t rows, int64_t vocab);
