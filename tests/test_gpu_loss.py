@@ -183,3 +183,57 @@ def test_loss_has_the_bits_of_the_mean_over_tokens(rows, vocab):
         want = ops.softcap_ce_fwd(x, t, 15.0)[0].mean()
         assert float(losses.capped_cross_entropy(x, t, 15.0)) == float(want)
         assert float(losses.capped_cross_entropy(x.clone().requires_grad_(), t, 15.0)) == float(want)
+
+
+# at the edges of the kernel that keeps a row's exponentials in tensor memory: just wide and large enough, one piece more than tensor memory
+# holds, the widest (and one column too wide), rows that start at every alignment; more rows than the GPU takes at a time
+@pytest.mark.parametrize("rows,vocab,cap", [(2200, 8193, 15.0), (560, 32769, 15.0), (549, 32775, 64.0), (340, 53247, 30.0), (339, 53249, 15.0),
+                                            (1500, 12301, 0.5)])
+def test_large_ragged_rows(rows, vocab, cap):
+    from train_gpt_b200 import losses
+    gen = torch.Generator("cuda").manual_seed(rows + vocab)
+    x = (torch.randn(rows, vocab, device="cuda", generator=gen) * 0.4 * cap).to(torch.bfloat16)
+    t = torch.randint(0, vocab, (rows,), device="cuda", generator=gen)
+    t[:8] = torch.tensor([0, 1, 6, 7, vocab - 1, vocab - 2, vocab - 8, 4096])          # in a ragged piece before, after, and in whole ones
+    x[3, 5], x[4, 7000], x[5, 9] = float("inf"), float("-inf"), 3e38
+    x.requires_grad_(True)
+    loss = losses.capped_cross_entropy(x, t, cap)
+    with torch.no_grad():
+        assert abs(float(losses.capped_cross_entropy(x, t, cap)) - float(loss.detach())) <= 1e-6 * abs(float(loss.detach()))
+    loss.backward(retain_graph=True)
+    c = torch.tensor(cap, dtype=torch.bfloat16).double()
+    bf = lambda v: v.to(torch.bfloat16).double()
+    got, total = x.grad, 0.0
+    x.grad = None
+    (loss * 1e-3).backward()
+    for r in range(0, rows, 100):
+        th = bf(torch.tanh(bf(x.detach()[r:r + 100].double() / c)))
+        z, tt = bf(c * th), t[r:r + 100, None]
+        lse = torch.logsumexp(z, -1, keepdim=True)
+        total += float((lse - z.gather(1, tt)).sum())
+        ref = torch.exp(z - lse).scatter_add_(1, tt, torch.full_like(lse, -1.0)) * (1 - th * th) / rows
+        for g, scale in ((got, 1.0), (x.grad, 1e-3)):
+            # one bf16 rounding of a float32 value; a tanh at a rounding boundary may fall to its neighbour
+            off = (g[r:r + 100].double() - scale * ref).abs() > 2.0 ** -8 * (scale * ref).abs() + 1e-35
+            assert float(off.double().mean()) < 1e-4
+            assert bool(((g[r:r + 100].double() - scale * ref).abs() <= 2e-2 * (scale * ref).abs() + 1e-2 * scale * ref.square().mean().sqrt()).all())
+    assert abs(float(loss.detach()) - total / rows) <= 1e-5 * abs(total / rows)
+
+
+def test_large_ragged_rows_nan_and_small_scale():
+    """A NaN spoils its own row alone; a scale whose product with 1 / sum is no normal number does not lose the gradient."""
+    from train_gpt_b200 import losses
+    x = torch.randn(2000, 9001, device="cuda").mul(60).to(torch.bfloat16)
+    x[7, 1234] = float("nan")
+    x.requires_grad_(True)
+    t = torch.zeros(2000, dtype=torch.int64, device="cuda")
+    loss = losses.capped_cross_entropy(x, t, 64.0)
+    loss.backward()
+    assert bool(torch.isnan(loss)) and bool(torch.isnan(x.grad[7]).all()) and int(torch.isnan(x.grad).any(1).sum()) == 1
+    x = x.detach()[8:].contiguous().requires_grad_(True)
+    loss = losses.capped_cross_entropy(x, t[8:], 64.0)
+    loss.backward(retain_graph=True)
+    base, x.grad = x.grad, None
+    (loss * 2.0 ** -40).backward()
+    big = base.abs() > 1e-12
+    assert bool((x.grad[big] == base[big] * 2.0 ** -40).all())

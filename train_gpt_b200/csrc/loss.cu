@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "host_api.h"
+#include "mbarrier.cuh"
 
 namespace tg {
 
@@ -238,6 +239,7 @@ softcap_ce_bwd_kernel(const __nv_bfloat16* tanh_in, const int32_t* __restrict__ 
 // ---------------------------------------------------------------------------------------
 constexpr int kCeMaxThreads = 640;
 constexpr int kCeWarpCols = 2048;                 // rows up to this wide take one warp
+constexpr int kCeSmemLimit = 226 * 1024;
 constexpr int kCeTableMax = 11 * 128 + 2;
 constexpr int kCeTableBytes = (kCeTableMax * 2 + 15) / 16 * 16;
 constexpr uint32_t kCeFloor2 = 0x08000800u;
@@ -496,6 +498,261 @@ __global__ void __launch_bounds__(WARP ? 256 : WHOLE ? kLossFwdThreads : kCeMaxT
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// The same for ragged rows of a large problem, with the exponentials taken once.  softcap_ce_kernel keeps the tanh values of a row and takes
+// exp(z) again for the gradient; here the first pass leaves g = exp(z) (1 - t^2) behind in float32, and the second is a scaling,
+//     gradient = g / sum * gscale / rows      (the target's element is computed by itself, with its -1),
+// a load, two packed multiplications and a conversion per pair.  A row of 50257 such values is 201 KB: eight pieces of each thread go to
+// tensor memory, which nothing else here uses (a group of 512 threads has 128 KB of it), the others to shared memory, so that TWO rows
+// are in flight on an SM, one in its first pass while the other is in its second.  One thread block per SM, so there is
+// room for tanh of every bf16 magnitude (64 KB) as well: a look-up is then an address and a load, with no range tests and no
+// bookkeeping for NaN.
+//
+// 37 warp instructions per 64 logits instead of 49.  What bounds it: three fifths of the peak of instruction issue and of the shared-memory
+// pipe each (a look-up of 32 random entries takes 3.5 cycles) and three quarters of the copy rate.  The loads come through the L2: one
+// thread fetches its row's pieces four passes ahead with a bulk prefetch (without: 383 us at 8192 x 50257, with whole rows ahead 398, so 336).
+//
+// The exponent's argument is z log2 e instead of (z - lse) log2 e: smaller, so its rounding costs the gradient less (the sum's order
+// and the last bits of the gradient are other ones than softcap_ce_kernel's).
+//
+// 8192 x 50257 406 -> 336 us (4.9 TB/s), 8192 x 25001 226 -> 179, 2048 x 50257 105 -> 93, 4096 x 9001 60 -> 51.  The rule: two rows per SM at a time
+// need rows to fill 296 of them, and the table's 64 KB are worth it from 18 M logits on (1024 x 9001 18.8 / 18.9 us, 512 x 25001 18.7 / 19.3,
+// 512 x 50257 32.2 / 31.0, 2048 x 9001 30.6 / 28.2); rows of up to 8192 columns leave too many of 512 threads without a piece in their last
+// pass (8192 x 4101 73.0 / 74.3, x 6001 77.1 / 79.1, x 5001 91.1 / 76.1).
+// ---------------------------------------------------------------------------------------
+constexpr int kCgMinCols = 8192;
+constexpr int64_t kCgMinLogits = 18'000'000;
+constexpr int kCgThreads = 512, kCgGroups = 2;
+constexpr int kCgAhead = 4;                                  // pieces of a thread that are on their way to the L2
+constexpr int kCgTmemSlots = 8;                              // pieces of a thread in tensor memory
+constexpr int kCgSlotBytes = kCgThreads * 32;                // a piece of every thread: eight floats each
+constexpr int kCgSmemSlots = (kCeSmemLimit - kTanhBytes) / (kCgGroups * kCgSlotBytes);
+constexpr int kCgMaxCols = (kCgTmemSlots + kCgSmemSlots) * kCgThreads * 8;
+
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float2 (&v)[4]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "f"(v[0].x), "f"(v[0].y), "f"(v[1].x), "f"(v[1].y), "f"(v[2].x), "f"(v[2].y), "f"(v[3].x), "f"(v[3].y) : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float2 (&v)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[2].x), "=f"(v[2].y), "=f"(v[3].x), "=f"(v[3].y)
+               : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld8(float2 (&v)[4]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+f"(v[0].x), "+f"(v[0].y), "+f"(v[1].x), "+f"(v[1].y), "+f"(v[2].x), "+f"(v[2].y), "+f"(v[3].x), "+f"(v[3].y)::"memory");
+}
+
+__global__ void __launch_bounds__(kCgThreads * kCgGroups, 1) softcap_ce_groups_kernel(const CeArgs p, int smem_slots) {
+  grid_trigger();
+  if (p.only_if_scaled) {
+    grid_wait();
+    if (*p.gscale == 1.0f) return;
+  }
+  extern __shared__ __align__(16) uint8_t s_cg[];
+  __shared__ float s_sum[kCgGroups][2][kCgThreads / 32];
+  __shared__ uint32_t s_tmem;
+  const Softcap sc(p.cap);
+  const uint32_t lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0);
+  const int group = warp / (kCgThreads / 32), gw = warp % (kCgThreads / 32), tid = int(threadIdx.x) % kCgThreads;
+  if (warp == 0) {
+    tmem_alloc(smem_u32(&s_tmem), 512);
+    tmem_relinquish();
+  }
+  {
+    // bf16(tanh(bf16(x / c))) by the magnitude of x.  From 4 c on it is 1, for infinity too; a NaN stays one.
+    const uint32_t one_from = ((__float_as_uint(sc.c) >> 16) & 0x7f80u) + (3u << 7);
+    uint16_t* table = reinterpret_cast<uint16_t*>(s_cg);
+    for (uint32_t i = threadIdx.x; i < uint32_t(kTanhEntries); i += blockDim.x)
+      table[i] = i > 0x7f80u ? uint16_t(0x7fffu) : i >= one_from ? uint16_t(0x3f80u)
+                 : uint16_t(__float_as_uint(tanh_bf16(sc.quotient(__uint_as_float(i << 16)))) >> 16);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  grid_wait();            // (the table comes from the cap alone)
+
+  // a warp reads and writes the lanes 32 (warp % 4).. of tensor memory; the four warps of a group that share them have 64 columns each
+  const uint32_t taddr0 = *reinterpret_cast<volatile uint32_t*>(&s_tmem) + (uint32_t(warp & 3) << 21) + uint32_t(group * 256 + (gw >> 2) * 64);
+  float4* spill = reinterpret_cast<float4*>(s_cg + kTanhBytes) + group * smem_slots * (kCgSlotBytes / 16) + tid;
+  const uint32_t tab = smem_u32(s_cg);
+  const float gs = (p.gscale != nullptr ? *p.gscale : 1.0f) * (1.0f / float(p.rows));
+  const float2 l2e = make_float2(kLog2e, kLog2e), one = make_float2(1.f, 1.f), minus1 = make_float2(-1.f, -1.f), gs2 = make_float2(gs, gs);
+  const __nv_bfloat162 c2 = __float2bfloat162_rn(sc.c);
+  const int step = int(gridDim.x) * kCgGroups;
+  int row = int(blockIdx.x) * kCgGroups + group;
+
+  struct Row {
+    const __nv_bfloat16* base;     // the row's first 16-byte boundary at or below its start
+    int off;                       // elements of that piece which belong to the row before
+    int first, last;               // the whole pieces [first, last): at most one ragged piece before and one after
+  };
+  auto row_of = [&](int r) {
+    Row q;
+    const __nv_bfloat16* s = p.logits + int64_t(r) * p.ld;
+    q.off = int((reinterpret_cast<uintptr_t>(s) & 15u) >> 1);
+    q.base = s - q.off;
+    q.first = q.off != 0;
+    q.last = (q.off + p.vocab) >> 3;
+    return q;
+  };
+  auto target_of = [&](int r) {
+    const int64_t t = p.targets_64 ? static_cast<const int64_t*>(p.targets)[r] : static_cast<const int32_t*>(p.targets)[r];
+    return int(t < 0 ? 0 : (t >= p.vocab ? p.vocab - 1 : t));         // clamped, as jnp.take_along_axis does
+  };
+  // (past the end: the last piece again, whose values are then not used)
+  auto load = [&](const Row& q, int i) -> uint4 { return ld_stream_v4(q.base + min(i, q.last - 1) * 8); };
+  // n pieces of a row, from its whole piece `at` on, into the L2
+  auto prefetch = [&](const Row& q, int at, int n) {
+    n = min(n, q.last - q.first - at);
+    if (n > 0) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(q.base + (q.first + at) * 8), "r"(n * 16) : "memory");
+  };
+  auto tanh_pair = [&](uint32_t w) {
+    const uint32_t lo = lds_u16(tab + ((w << 1) & 0xfffeu)), hi = lds_u16(tab + ((w >> 15) & 0xfffeu));
+    return __byte_perm(lo, hi, 0x5410) | (w & 0x80008000u);
+  };
+  // bf16(c t) of a pair: the product of two bf16 values rounded once, as the float product rounded to bf16 is
+  auto capped = [&](uint32_t t2) {
+    const __nv_bfloat162 z = __hmul2(c2, *reinterpret_cast<const __nv_bfloat162*>(&t2));
+    return bf16x2_unpack(*reinterpret_cast<const uint32_t*>(&z));
+  };
+  // the ragged pieces, an element per lane of the group's last warp: lanes 0..7 the piece before the whole ones, 8..15 the one after
+  auto edge_of = [&](const Row& q) {
+    const int end = q.off + p.vocab;
+    if (gw != kCgThreads / 32 - 1) return -1;
+    if (lane < 8) return q.off != 0 && int(lane) >= q.off && int(lane) < end ? int(lane) : -1;
+    const int e = q.last * 8 + int(lane) - 8;
+    return lane < 16 && q.last >= q.first && e < end ? e : -1;
+  };
+  auto grad1 = [&](float t, float z, float lse, bool hit) {
+    const float pr = ex2(__fmul_rn(z - lse, kLog2e)) - (hit ? 1.0f : 0.0f);
+    return __float2bfloat16_rn(__fmul_rn(__fmul_rn(pr, gs), __fmaf_rn(__fmul_rn(t, t), -1.0f, 1.0f)));
+  };
+
+  if (row < p.rows) {
+    Row q = row_of(row);
+    int target = target_of(row);
+    uint4 w0 = load(q, q.first + tid), w1 = load(q, q.first + tid + kCgThreads);
+    for (int it = 0; row < p.rows; row += step, ++it) {
+      const int at = target + q.off;                                  // the target's place in the row's pieces
+      const uint32_t x_at = reinterpret_cast<const unsigned short*>(q.base)[at];
+      if (row + step < p.rows) target = target_of(row + step);
+      // ---- the sum of exp(z), and g of every element.  (Whole warps: a store to tensor memory is the warp's.)
+      float2 acc = make_float2(0.f, 0.f);
+      const int mine = q.first + tid, n_k = (q.last - q.first - gw * 32 + kCgThreads - 1) / kCgThreads;
+      auto first_pass = [&](const uint4& w, int k, float2 (&g)[4]) {
+        const uint32_t wi[4] = {w.x, w.y, w.z, w.w};
+        float2 e[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t t2 = tanh_pair(wi[j]);
+          const float2 tf = bf16x2_unpack(t2), zl = __fmul2_rn(capped(t2), l2e);
+          e[j] = make_float2(ex2(zl.x), ex2(zl.y));
+          g[j] = __fmul2_rn(e[j], __ffma2_rn(__fmul2_rn(tf, tf), minus1, one));   // t^2 is exact
+        }
+        const float2 sum = __fadd2_rn(__fadd2_rn(e[0], e[1]), __fadd2_rn(e[2], e[3]));
+        if (mine + k * kCgThreads < q.last) acc = __fadd2_rn(acc, sum);
+      };
+      auto keep = [&](int k, const float2 (&g)[4]) {
+        if (k < kCgTmemSlots) {
+          tmem_st8(taddr0 + 8 * k, g);
+          return;
+        }
+        float4* d = spill + (k - kCgTmemSlots) * (2 * kCgThreads);
+        d[0] = make_float4(g[0].x, g[0].y, g[1].x, g[1].y);
+        d[kCgThreads] = make_float4(g[2].x, g[2].y, g[3].x, g[3].y);
+      };
+#pragma unroll 1
+      for (int k = 0; k < n_k; k += 2) {
+        float2 g[4];
+        if (tid == 0) prefetch(q, (k + kCgAhead) * kCgThreads, 2 * kCgThreads);
+        first_pass(w0, k, g);
+        w0 = load(q, mine + (k + 2) * kCgThreads);
+        if (p.d != nullptr) keep(k, g);
+        if (k + 1 < n_k) {
+          first_pass(w1, k + 1, g);
+          w1 = load(q, mine + (k + 3) * kCgThreads);
+          if (p.d != nullptr) keep(k + 1, g);
+        }
+      }
+      const int e_mine = edge_of(q);
+      uint32_t t_edge = 0u;
+      if (e_mine >= 0) {
+        t_edge = tanh_pair(reinterpret_cast<const unsigned short*>(q.base)[e_mine]) & 0xffffu;
+        acc.x += ex2(__fmul_rn(capped(t_edge).x, kLog2e));
+      }
+      // the next row's first pieces are on their way while this one is finished
+      const Row now = q;
+      if (row + step < p.rows) {
+        q = row_of(row + step);
+        if (tid == 0) prefetch(q, 2 * kCgThreads, (kCgAhead - 2) * kCgThreads);
+        w0 = load(q, q.first + tid);
+        w1 = load(q, q.first + tid + kCgThreads);
+      }
+      float s = acc.x + acc.y;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) s_sum[group][it & 1][gw] = s;
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kCgThreads) : "memory");
+      s = lane < kCgThreads / 32 ? s_sum[group][it & 1][lane] : 0.f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      const float lse = logf(s), inv = __frcp_rn(s);
+      const int piece = at >> 3;
+      const bool own = piece >= now.first && piece < now.last && (piece - now.first) % kCgThreads == tid;
+      const uint32_t t_at = tanh_pair(x_at) & 0xffffu;
+      // ---- the gradient.  (g / sum first: the factors may be small, their product with g need not be.)
+      if (p.d != nullptr) {
+        __nv_bfloat16* dp = p.d + (now.base - p.logits);
+        // g / sum * gs in one product where the factor is a normal number (its product with g then is what it should be), else in two
+        const float factor = __fmul_rn(inv, gs);
+        const bool one_product = !(fabsf(factor) < 1.2e-38f);
+        const float2 f2 = one_product ? make_float2(factor, factor) : make_float2(inv, inv);
+        auto second_pass = [&](float2 (&g)[4], int i) {
+          uint4 o;
+          uint32_t* op = &o.x;
+          if (!one_product) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) g[j] = __fmul2_rn(g[j], gs2);
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 r = __fmul2_rn(g[j], f2);
+            op[j] = pack_bf16x2(r.x, r.y);
+          }
+          if (i < now.last) *reinterpret_cast<uint4*>(dp + i * 8) = o;
+        };
+#pragma unroll 2
+        for (int k = 0; k < min(n_k, kCgTmemSlots); ++k) {
+          float2 g[4];
+          tmem_ld8(taddr0 + 8 * k, g);
+          tmem_wait_ld8(g);
+          second_pass(g, mine + k * kCgThreads);
+        }
+#pragma unroll 2
+        for (int k = kCgTmemSlots; k < n_k; ++k) {
+          const float4* d = spill + (k - kCgTmemSlots) * (2 * kCgThreads);
+          const float4 a = d[0], b = d[kCgThreads];
+          float2 g[4] = {make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w)};
+          second_pass(g, mine + k * kCgThreads);
+        }
+        if (e_mine >= 0) dp[e_mine] = grad1(bf16lo(t_edge), capped(t_edge).x, lse, e_mine == at);
+        if (own) dp[at] = grad1(bf16lo(t_at), capped(t_at).x, lse, true);      // the target's own element again, now with its -1
+      }
+      // ---- the target's log-probability
+      if (p.nll != nullptr && (own || e_mine == at)) p.nll[row] = lse - capped(t_at).x;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(*reinterpret_cast<volatile uint32_t*>(&s_tmem), 512);
+  }
+}
+
 // Mean of n floats, to the bit what torch's mean of a contiguous vector gives (measured up to 65536 values): T threads, T the largest
 // power of two in n / 4 but at most 512; thread j adds the 16-byte pieces j, j + T, ... value by value, the first thread's values also those
 // after the last whole piece, one per thread; the four sums in order, then halves of T.  Below 128 values T is the largest power of
@@ -536,7 +793,7 @@ __global__ void __launch_bounds__(kMeanThreads) mean_kernel(const float* __restr
   }
 }
 
-constexpr int kCeSmemMax = 226 * 1024;
+constexpr int kCeSmemMax = kCeSmemLimit;
 static int64_t ce_smem(int64_t vocab) {
   const int64_t row = (vocab + 14) / 8 * 16;
   return kCeTableBytes + (vocab <= kCeWarpCols ? 8 * row : row);
@@ -580,6 +837,7 @@ extern "C" int tgh_softcap_ce(const void* logits, const void* targets, int targe
     if (!attr_set[dev & 63].load(std::memory_order_acquire)) {
       for (auto kern : {softcap_ce_kernel<false, false>, softcap_ce_kernel<false, true>, softcap_ce_kernel<true, false>, softcap_ce_kernel<true, true>})
         TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeSmemMax));
+      TG_CUDA_CHECK(cudaFuncSetAttribute(softcap_ce_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeSmemMax));
       attr_set[dev & 63].store(true, std::memory_order_release);
     }
     const size_t smem = size_t(ce_smem(vocab));
@@ -594,6 +852,11 @@ extern "C" int tgh_softcap_ce(const void* logits, const void* targets, int targe
       const int64_t cap_blocks = int64_t(sm_count()) * std::min<int64_t>(per_sm_smem, 2);
       TG_CUDA_CHECK(launch_if_short(is_short, softcap_ce_kernel<false, true>, dim3(unsigned(std::min<int64_t>(rows, cap_blocks))), kLossFwdThreads,
                                     smem, st, a));
+    } else if (vocab > kCgMinCols && vocab <= kCgMaxCols && rows * vocab >= kCgMinLogits) {
+      const int slots = int(std::max<int64_t>(0, (vocab / 8 + kCgThreads - 1) / kCgThreads - kCgTmemSlots));
+      const int blocks = int(std::min<int64_t>((rows + kCgGroups - 1) / kCgGroups, sm_count()));
+      TG_CUDA_CHECK(launch_if_short(is_short, softcap_ce_groups_kernel, dim3(unsigned(blocks)), kCgThreads * kCgGroups,
+                                    size_t(kTanhBytes + kCgGroups * slots * kCgSlotBytes), st, a, slots));
     } else {
       // as many threads as make the last pass over the row nearly full (of at most 640: two blocks an SM at 48 registers)
       const int64_t pieces = (vocab + 7) / 8;

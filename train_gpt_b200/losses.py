@@ -24,7 +24,7 @@ def capped_cross_entropy(logits: torch.Tensor, target_ids: torch.Tensor, cap: fl
     With gradients on and logits that require one, the FORWARD writes the gradient too (for an upstream
     gradient of 1; another one is seen in the backward pass and the gradient made again from the logits): one
     read of the logits serves both.  The logits and a tensor of their size stay allocated until the backward pass
-    or the result's end, and a loss that is never differentiated pays for the write: 8192 x 50257 430 us with it,
-    277 under `torch.no_grad()`.  (A vocabulary or cap that a row in shared memory cannot hold
+    or the result's end, and a loss that is never differentiated pays for the write: 8192 x 50257 359 us with it,
+    230 under `torch.no_grad()`.  (A vocabulary or cap that a row in shared memory cannot hold
     takes two passes, which keep one tensor of that size.)"""
     return ops._host().capped_cross_entropy(logits, target_ids, cap)
