@@ -1,0 +1,28 @@
+"""A linear's data and weight gradient in one launch: the bits of the two launches."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# one tile each; ragged tokens; sizes that fit one wave together and sizes that do not (two launches); the modes' three kinds of scales
+@pytest.mark.parametrize("tokens,k,n", [(130, 128, 128), (1000, 384, 256), (1024, 512, 128), (700, 640, 768), (1024, 1152, 640), (1024, 128, 17920),
+                                        (1025, 1280, 640), (300, 128, 4096)])
+@pytest.mark.parametrize("tile,mode", [((128, 128), "fp8"), ((128, 1), "fp8"), ((128, 128), "fp8_blockgrad")])
+def test_backward_has_the_bits_of_two_launches(tokens, k, n, tile, mode):
+    from train_gpt_b200 import fp8, ops
+    gen = torch.Generator("cuda").manual_seed(tokens + k + n)
+    x = torch.randn(tokens, k, device="cuda", generator=gen).to(torch.bfloat16).requires_grad_()
+    w = (torch.randn(k, n, device="cuda", generator=gen) * 0.05).to(torch.bfloat16).requires_grad_()
+    g = torch.randn(tokens, n, device="cuda", generator=gen).to(torch.bfloat16)
+    fp8.block_scaled_matmul(x, w, weight_tile=tile, backward=mode).backward(g)
+    status = ops.new_status("cuda")
+    x_q, x_s = ops.quantize_colwise(x.detach())
+    g_q, g_s = ops.quantize_rowwise(g)
+    w_q, w_s = ops.quantize_block128(w.detach()) if tile == (128, 128) else ops.quantize_rowwise(w.detach())
+    grad_tile = (128, 128) if mode == "fp8_blockgrad" else (128, 1)
+    c_q, c_s = ops.quantize_block128(g) if mode == "fp8_blockgrad" else ops.quantize_colwise(g)
+    assert torch.equal(x.grad, ops.gemm_dgrad(g_q, g_s, w_q, w_s, tile, status=status))
+    assert torch.equal(w.grad, ops.gemm_wgrad(x_q, x_s, c_q, c_s, grad_tile=grad_tile, status=status))
+    assert int(status.item()) == 0
+    ops.check_status()

@@ -636,12 +636,13 @@ Pair fp8_backward(const Tensor& a, const Tensor& b, const Tensor& g_, at::IntArr
     want_col(j, x = x_at.in(temp), k);
   }
   check(api.tgh_quantize_jobs(jobs, n_jobs, cur_stream()), "tgh_quantize_jobs");
-  if (in.want_a) {
-    run_gemm(dgrad, g_row, w, ptr(da), temp.at(ws_at), ws_bytes[0]);
-    da = to(da, a_dtype);
-  }
+  if (in.want_a) set_operands(dgrad, g_row, w, ptr(da), temp.at(ws_at), ws_bytes[0]);
+  if (in.want_b) set_operands(wgrad, x, g_col, ptr(db.defined() ? db : db_slot), temp.at(ws_at), ws_bytes[1]);
+  if (in.want_a && in.want_b) check(api.tgh_gemm_two(&dgrad, &wgrad, cur_stream()), "tgh_gemm_two");
+  else check(api.tg_gemm_fp8_blockscaled(in.want_a ? &dgrad : &wgrad, cur_stream()), "tg_gemm_fp8_blockscaled");
+  last_gemm_launches.store(ws_bytes[in.want_b ? 1 : 0] > 0 ? 2 : 1, std::memory_order_relaxed);
+  if (in.want_a) da = to(da, a_dtype);
   if (in.want_b) {
-    run_gemm(wgrad, x, g_col, ptr(db.defined() ? db : db_slot), temp.at(ws_at), ws_bytes[1]);
     if (in.slot_take) in.slot_ready();
     else db = to(db, b_dtype);
   }

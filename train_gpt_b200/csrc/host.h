@@ -35,7 +35,7 @@ constexpr auto kF8 = at::kFloat8_e4m3fn;
   X(tg_act_quantize_rowcol) X(tg_quantize_block128) X(tg_rmsnorm_fwd) X(tg_rmsnorm_quant_fwd)                       \
   X(tg_add_rmsnorm_quant_fwd) X(tg_rmsnorm_bwd_scratch_bytes) X(tg_rmsnorm_bwd) X(tg_rmsnorm_bwd_add)               \
   X(tg_softcap_ce_fwd) X(tg_softcap_ce_bwd) X(tg_sumsq_scratch_bytes) X(tg_sumsq_bf16) X(tg_adamw_bf16)             \
-  X(tg_gemm_workspace_bytes) X(tg_gemm_fp8_blockscaled) X(tgh_quantize_jobs) X(tgh_softcap_ce_fits) X(tgh_softcap_ce) X(tgh_mean) \
+  X(tg_gemm_workspace_bytes) X(tg_gemm_fp8_blockscaled) X(tgh_gemm_two) X(tgh_quantize_jobs) X(tgh_softcap_ce_fits) X(tgh_softcap_ce) X(tgh_mean) \
   X(tgh_global_norm_scratch_bytes) X(tgh_global_norm) X(tgh_adamw) X(tgh_embed) X(tgh_embed_bwd)
 
 struct Api {
@@ -198,11 +198,14 @@ inline tg_gemm_args gemm_args(int64_t m, int64_t n, int64_t k, int64_t lda, int 
   g.status = status;
   return g;
 }
-inline void run_gemm(tg_gemm_args& g, const Form& a, const Form& b, void* d, void* workspace, int64_t workspace_bytes) {
+inline void set_operands(tg_gemm_args& g, const Form& a, const Form& b, void* d, void* workspace, int64_t workspace_bytes) {
   g.a = a.q; g.sa = a.s; g.b = b.q; g.sb = b.s;
   g.d = d;
   g.workspace = workspace_bytes > 0 ? workspace : nullptr;
   g.workspace_bytes = workspace_bytes;
+}
+inline void run_gemm(tg_gemm_args& g, const Form& a, const Form& b, void* d, void* workspace, int64_t workspace_bytes) {
+  set_operands(g, a, b, d, workspace, workspace_bytes);
   check(api.tg_gemm_fp8_blockscaled(&g, cur_stream()), "tg_gemm_fp8_blockscaled");
   last_gemm_launches.store(workspace_bytes > 0 ? 2 : 1, std::memory_order_relaxed);
 }

@@ -237,6 +237,14 @@ class StepProgram {
     run_gemm(g, a, b, d, workspace_, api.tg_gemm_workspace_bytes(&g));
   }
 
+  // the data gradient of a (k, n) linear into dx and its weight gradient into dw, from the gradient's two forms in row_ and col_
+  void run_backward(int64_t k, int64_t n, const Form& w, void* dx, const Form& x_col, void* dw) {
+    tg_gemm_args a = dgrad(k, n), b = wgrad(k, n);
+    set_operands(a, row_, w, dx, workspace_, api.tg_gemm_workspace_bytes(&a));
+    set_operands(b, x_col, col_, dw, workspace_, api.tg_gemm_workspace_bytes(&b));
+    check(api.tgh_gemm_two(&a, &b, cur_stream()), "tgh_gemm_two");
+  }
+
   // Scratch for the widest of every use: a row form, a column form beside it, a third one, the norm backward's partial
   // sums, the GEMMs' workspace.
   void plan() {
@@ -353,12 +361,10 @@ class StepProgram {
       want_col(j[1], third_, d_);
       quantize(j, 2);
       Tensor da = act(ff_);
-      run(dgrad(ff_, d_), row_, w.down, ptr(da));
-      run(wgrad(ff_, d_), k.a_col, col_, ptr(g.w_down));
+      run_backward(ff_, d_, w.down, ptr(da), k.a_col, ptr(g.w_down));
       check(api.tg_act_quantize_rowcol(ptr(k.u), ptr(da), c_.act_bwd, row_.q, row_.s, col_.q, col_.s, m_, ff_, cur_stream()),
             "tg_act_quantize_rowcol");
-      run(dgrad(d_, ff_), row_, w.up, ptr(dh));
-      run(wgrad(d_, ff_), third_, col_, ptr(g.w_up));
+      run_backward(d_, ff_, w.up, ptr(dh), third_, ptr(g.w_up));
     }
     k.u = k.h2 = Tensor();
     Tensor d2 = act(d_);
@@ -370,8 +376,7 @@ class StepProgram {
       want_row(j, row_);
       want_col(j, col_, d_);
       quantize(&j, 1);
-      run(dgrad(hd_, d_), row_, w.o, ptr(dov));
-      run(wgrad(hd_, d_), k.o_col, col_, ptr(g.wo));
+      run_backward(hd_, d_, w.o, ptr(dov), k.o_col, ptr(g.wo));
     }
     if (!on_attention_.is_none()) on_attention_();
     std::array<Tensor, 3> dq = k.attention.backward(dov.transpose(1, 2));
@@ -393,8 +398,7 @@ class StepProgram {
       j[3] = job_of(k.h1);
       want_col(j[3], third_, d_);
       quantize(j, 4);
-      run(dgrad(d_, 3 * hd_), row_, w.qkv, ptr(dh));
-      run(wgrad(d_, 3 * hd_), third_, col_, ptr(g.wqkv));
+      run_backward(d_, 3 * hd_, w.qkv, ptr(dh), third_, ptr(g.wqkv));
     }
     k.h1 = Tensor();
     if (l > 0) {
