@@ -33,10 +33,10 @@ constexpr auto kF8 = at::kFloat8_e4m3fn;
 #define TG_API(X)                                                                                                  \
   X(tg_last_cuda_error) X(tg_quantize_rowwise) X(tg_quantize_colwise) X(tg_quantize_rowcol) X(tg_quantize_rowcol_ld) \
   X(tg_act_quantize_rowcol) X(tg_quantize_block128) X(tg_rmsnorm_fwd) X(tg_rmsnorm_quant_fwd)                       \
-  X(tg_add_rmsnorm_quant_fwd) X(tg_rmsnorm_bwd_scratch_bytes) X(tg_rmsnorm_bwd) X(tg_rmsnorm_bwd_add)               \
+  X(tg_add_rmsnorm_quant_fwd) X(tg_rmsnorm_bwd_scratch_bytes) X(tg_rmsnorm_bwd) X(tg_rmsnorm_bwd_add) X(tgh_rmsnorm_bwd_parts) X(tgh_dgamma_reduce) \
   X(tg_softcap_ce_fwd) X(tg_softcap_ce_bwd) X(tg_sumsq_scratch_bytes) X(tg_sumsq_bf16) X(tg_adamw_bf16)             \
   X(tg_gemm_workspace_bytes) X(tg_gemm_fp8_blockscaled) X(tgh_gemm_two) X(tgh_quantize_jobs) X(tgh_softcap_ce_fits) X(tgh_softcap_ce) X(tgh_mean) \
-  X(tgh_global_norm_scratch_bytes) X(tgh_global_norm) X(tgh_adamw) X(tgh_embed) X(tgh_embed_bwd)
+  X(tgh_global_norm_scratch_bytes) X(tgh_global_norm) X(tgh_adamw) X(tgh_embed) X(tgh_embed_bwd_cleared)
 
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;

@@ -36,6 +36,13 @@ int tgh_gemm_kernel(const tg_gemm_args* args, int* kernel);
  * together uses none): in one launch where they are small, else one after the other. */
 int tgh_gemm_two(const tg_gemm_args* a, const tg_gemm_args* b, void* stream);
 
+/* tg_rmsnorm_bwd (addend NULL) or tg_rmsnorm_bwd_add up to the partial sums of the weight's gradient, tg_rmsnorm_bwd_scratch_bytes(rows, cols)
+ * of them, and the weight gradients of any number of norms of one size from those. */
+typedef struct { const void* partial; void* dgamma; } tgh_dgamma_job;
+int tgh_rmsnorm_bwd_parts(const void* x, const void* gamma, const void* g, const void* addend, float eps, void* dx, void* partial, int64_t rows,
+                          int64_t cols, void* stream);
+int tgh_dgamma_reduce(const tgh_dgamma_job* jobs, int n, int64_t rows, int64_t cols, void* stream);
+
 /* Whether tgh_softcap_ce takes this problem (a row and its cap fit the one-pass kernel). */
 int tgh_softcap_ce_fits(float cap, int64_t rows, int64_t vocab);
 /* Capped cross-entropy of each row AND the gradient of their mean from one read of the logits.
@@ -51,14 +58,16 @@ int tgh_softcap_ce(const void* logits, const void* targets, int targets_64, floa
 int tgh_mean(const float* v, int64_t n, float* out, void* stream);
 
 /* x[b, t, :] = bf16(embed[ids[b, t]] + pos[t]) (train-gpt model.py:83).  Negative ids count from the end; one outside the
- * vocabulary stores TGH_STATUS_TOKEN in *status and makes its row NaN. */
+ * vocabulary stores TGH_STATUS_TOKEN in *status and makes its row NaN.  Also clears tgh_embed_bwd's table and the
+ * gradient [vocab, d]. */
 enum { TGH_STATUS_TOKEN = 16 };
 int tgh_embed(const int64_t* ids, const void* embed, const void* pos, void* x, int64_t batch, int64_t seq, int64_t d, int64_t vocab,
-              unsigned* status, void* stream);
+              unsigned* status, void* table, void* g_embed, void* stream);
 
 /* The gradient of embed: the rows of dx [tokens, d] added up by token id in token order, rounded to bf16 after every addition (as
- * an accumulating index_put does); zeros for ids that do not occur.  table: vocab * 8 bytes of scratch. */
+ * an accumulating index_put does); zeros for ids that do not occur.  table: vocab * 8 bytes of scratch.  (_cleared: both are all zero already.) */
 int tgh_embed_bwd(const int64_t* ids, const void* dx, void* g_embed, void* table, int64_t tokens, int64_t d, int64_t vocab, void* stream);
+int tgh_embed_bwd_cleared(const int64_t* ids, const void* dx, void* g_embed, void* table, int64_t tokens, int64_t d, int64_t vocab, void* stream);
 
 /* A parameter tensor with its gradient and moments: n contiguous bf16 values each, 16-byte aligned. */
 typedef struct { void* p; const void* g; void* m; void* v; int64_t n; } tgh_span;

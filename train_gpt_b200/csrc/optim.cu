@@ -337,13 +337,17 @@ adamw_spans_kernel(const __grid_constant__ Spans t, AdamwArgs a, const float* __
   }
 }
 
-// Token and position embeddings of a step: one 16-byte piece per thread.
+// Token and position embeddings of a step: one 16-byte piece per thread.  The embedding gradient's memory is cleared here, where that is no
+// launch of its own (as two fills they were 6 us of a small step's host time).
 __global__ void __launch_bounds__(kOptThreads)
 embed_kernel(const int64_t* __restrict__ ids, const __nv_bfloat16* __restrict__ embed, const __nv_bfloat16* __restrict__ pos,
-             __nv_bfloat16* __restrict__ x, long long tokens, int seq, int d, int64_t vocab, unsigned* status) {
+             __nv_bfloat16* __restrict__ x, long long tokens, int seq, int d, int64_t vocab, unsigned* status, uint2* table, uint4* g_embed) {
   const int per_row = d / 8;
   grid_trigger();
   grid_wait();
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  for (long long i = first; i < vocab; i += step) table[i] = make_uint2(0u, 0u);
+  for (long long i = first; i < vocab * per_row; i += step) g_embed[i] = make_uint4(0u, 0u, 0u, 0u);
   ids = loads_below(ids);
   embed = loads_below(embed);
   pos = loads_below(pos);
@@ -587,34 +591,44 @@ extern "C" int tgh_adamw(const tgh_span* spans, int n, float lr, float b1, float
 }
 
 extern "C" int tgh_embed(const int64_t* ids, const void* embed, const void* pos, void* x, int64_t batch, int64_t seq, int64_t d,
-                         int64_t vocab, unsigned* status, void* stream) {
+                         int64_t vocab, unsigned* status, void* table, void* g_embed, void* stream) {
   if (batch < 0 || seq < 0 || d <= 0 || d % 8 != 0 || d > INT32_MAX || seq > INT32_MAX || status == nullptr) return TG_ERR_SHAPE;
   if (batch == 0 || seq == 0) return TG_OK;
-  if (!aligned16(embed) || !aligned16(pos) || !aligned16(x)) return TG_ERR_ALIGN;
+  if (!aligned16(embed) || !aligned16(pos) || !aligned16(x) || !aligned16(table) || !aligned16(g_embed)) return TG_ERR_ALIGN;
   if (int rc = check_arch()) return rc;
-  const int64_t blocks = (batch * seq * (d / 8) + kOptThreads - 1) / kOptThreads, cap = int64_t(sm_count()) * 16;
-  TG_CUDA_CHECK(launch_if_short(batch * seq * d <= 1 << 20, embed_kernel, dim3(unsigned(blocks < cap ? blocks : cap)), kOptThreads, 0,
+  const int64_t pieces = std::max(batch * seq, vocab) * (d / 8);
+  const int64_t blocks = (pieces + kOptThreads - 1) / kOptThreads, cap = int64_t(sm_count()) * 16;
+  TG_CUDA_CHECK(launch_if_short(pieces <= 1 << 17, embed_kernel, dim3(unsigned(blocks < cap ? blocks : cap)), kOptThreads, 0,
                                 static_cast<cudaStream_t>(stream), ids, static_cast<const __nv_bfloat16*>(embed),
                                 static_cast<const __nv_bfloat16*>(pos), static_cast<__nv_bfloat16*>(x), static_cast<long long>(batch * seq),
-                                int(seq), int(d), vocab, status));
+                                int(seq), int(d), vocab, status, static_cast<uint2*>(table), static_cast<uint4*>(g_embed)));
   return TG_OK;
 }
 
-extern "C" int tgh_embed_bwd(const int64_t* ids, const void* dx, void* g_embed, void* table, int64_t tokens, int64_t d, int64_t vocab,
-                             void* stream) {
+static int embed_bwd(const int64_t* ids, const void* dx, void* g_embed, void* table, int64_t tokens, int64_t d, int64_t vocab, bool clear, void* stream) {
   if (tokens <= 0 || d <= 0 || d % 8 != 0 || vocab <= 0) return TG_ERR_SHAPE;
   if (d > INT32_MAX || tokens > INT32_MAX) return TG_ERR_TOO_LARGE;
   if (!aligned16(dx) || !aligned16(g_embed) || !aligned16(table)) return TG_ERR_ALIGN;
   if (int rc = check_arch()) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  TG_CUDA_CHECK(cudaMemsetAsync(table, 0, size_t(vocab) * sizeof(uint2), st));
-  TG_CUDA_CHECK(cudaMemsetAsync(g_embed, 0, size_t(vocab) * size_t(d) * 2, st));
-  token_count_kernel<<<int((tokens + kOptThreads - 1) / kOptThreads), kOptThreads, 0, st>>>(ids, int(tokens), int(d), vocab, static_cast<uint2*>(table),
-                                                                                                 static_cast<__nv_bfloat16*>(g_embed));
-  TG_CUDA_CHECK(cudaGetLastError());
+  if (clear) {
+    TG_CUDA_CHECK(cudaMemsetAsync(table, 0, size_t(vocab) * sizeof(uint2), st));
+    TG_CUDA_CHECK(cudaMemsetAsync(g_embed, 0, size_t(vocab) * size_t(d) * 2, st));
+  }
+  TG_CUDA_CHECK(launch_early(token_count_kernel, int((tokens + kOptThreads - 1) / kOptThreads), kOptThreads, 0, st, ids, int(tokens), int(d), vocab,
+                             static_cast<uint2*>(table), static_cast<__nv_bfloat16*>(g_embed)));
   const int64_t per_block = kOptThreads / 32, blocks = (tokens * ((d + 255) / 256) + per_block - 1) / per_block;
   if (blocks > INT32_MAX) return TG_ERR_TOO_LARGE;
   TG_CUDA_CHECK(launch_early(embed_bwd_kernel, int(blocks), kOptThreads, 0, st, ids, static_cast<const __nv_bfloat16*>(dx),
                              static_cast<__nv_bfloat16*>(g_embed), static_cast<const uint2*>(table), int(tokens), int(d), vocab));
   return TG_OK;
+}
+
+extern "C" int tgh_embed_bwd(const int64_t* ids, const void* dx, void* g_embed, void* table, int64_t tokens, int64_t d, int64_t vocab,
+                             void* stream) {
+  return embed_bwd(ids, dx, g_embed, table, tokens, d, vocab, true, stream);
+}
+extern "C" int tgh_embed_bwd_cleared(const int64_t* ids, const void* dx, void* g_embed, void* table, int64_t tokens, int64_t d, int64_t vocab,
+                                     void* stream) {
+  return embed_bwd(ids, dx, g_embed, table, tokens, d, vocab, false, stream);
 }

@@ -13,7 +13,10 @@
 
 #include <atomic>
 
+#include <algorithm>
+
 #include "common.cuh"
+#include "host_api.h"
 
 namespace tg {
 
@@ -481,14 +484,19 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
 // groups of four are complete go to its first; the four are added in pairs, the eight classes in order.  Warp w + 8 i keeps the i-th
 // sum of class w and has all of its (at most seven) loads in flight at once: with eight warps of four sums each the kernel was
 // a chain of five L2 round trips, 5.2 us at 2048 columns.
-__global__ void __launch_bounds__(1024)
-rmsnorm_dgamma_reduce_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dgamma,
-                             int n_blocks, int cols) {
+// The norms of a step can be finished together (row y of the grid is job y): alone each is a launch of 2 us, 49 of them in a step
+// of 24 layers.
+constexpr int kDgammaJobs = 64;
+struct DgammaJobs {
+  tgh_dgamma_job job[kDgammaJobs];
+};
+__global__ void __launch_bounds__(1024) rmsnorm_dgamma_reduce_kernel(const __grid_constant__ DgammaJobs jobs, int n_blocks, int cols) {
   __shared__ float s_part[32][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + lane;
+  const float* partial = static_cast<const float*>(jobs.job[blockIdx.y].partial);
+  __nv_bfloat16* dgamma = static_cast<__nv_bfloat16*>(jobs.job[blockIdx.y].dgamma);
   grid_wait();
-  partial = loads_below(partial);
   float t = 0.f;
   if (col < cols) {
     const int w = warp & 7;
@@ -788,6 +796,16 @@ extern "C" int64_t tg_rmsnorm_bwd_scratch_bytes(int64_t rows, int64_t cols) {
   return int64_t(bwd_blocks(rows, g)) * cols * int64_t(sizeof(float));
 }
 
+static int reduce_dgamma(const tgh_dgamma_job* jobs, int n, int blocks, int cols, cudaStream_t st) {
+  for (int i = 0; i < n; i += kDgammaJobs) {
+    DgammaJobs a;
+    const int m = std::min(n - i, kDgammaJobs);
+    std::copy(jobs + i, jobs + i + m, a.job);
+    TG_CUDA_CHECK(launch_if_short(true, rmsnorm_dgamma_reduce_kernel, dim3(unsigned((cols + 31) / 32), unsigned(m)), 1024, 0, st, a, blocks, cols));
+  }
+  return TG_OK;
+}
+
 static int rmsnorm_bwd_impl(const void* x, const void* gamma, const void* g, const void* addend, float eps, void* dx,
                             void* dgamma, void* scratch, int64_t rows, int64_t cols, void* stream) {
   if (rows < 0 || cols <= 0 || cols % 8 != 0) return TG_ERR_SHAPE;
@@ -799,7 +817,7 @@ static int rmsnorm_bwd_impl(const void* x, const void* gamma, const void* g, con
   if (int rc = check_arch()) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (rows == 0) {
-    TG_CUDA_CHECK(cudaMemsetAsync(dgamma, 0, size_t(cols) * 2, st));
+    if (dgamma != nullptr) TG_CUDA_CHECK(cudaMemsetAsync(dgamma, 0, size_t(cols) * 2, st));
     return TG_OK;
   }
   const int blocks = bwd_blocks(rows, geo);
@@ -807,9 +825,9 @@ static int rmsnorm_bwd_impl(const void* x, const void* gamma, const void* g, con
                      static_cast<const __nv_bfloat16*>(addend), eps, static_cast<__nv_bfloat16*>(dx), static_cast<float*>(scratch), rows,
                      int(cols), blocks};
   if (int rc = launch_bwd(geo, a, st)) return rc;
-  TG_CUDA_CHECK(launch_early(rmsnorm_dgamma_reduce_kernel, int((cols + 31) / 32), 1024, 0, st, static_cast<const float*>(scratch),
-                             static_cast<__nv_bfloat16*>(dgamma), blocks, int(cols)));
-  return TG_OK;
+  if (dgamma == nullptr) return TG_OK;
+  const tgh_dgamma_job job = {scratch, dgamma};
+  return reduce_dgamma(&job, 1, blocks, int(cols), st);
 }
 
 extern "C" int tg_rmsnorm_bwd(const void* x, const void* gamma, const void* g, float eps, void* dx,
@@ -821,6 +839,18 @@ extern "C" int tg_rmsnorm_bwd_add(const void* x, const void* gamma, const void* 
                                   void* dx, void* dgamma, void* scratch, int64_t rows, int64_t cols, void* stream) {
   if (addend == nullptr) return TG_ERR_SHAPE;
   return rmsnorm_bwd_impl(x, gamma, g, addend, eps, dx, dgamma, scratch, rows, cols, stream);
+}
+
+extern "C" int tgh_rmsnorm_bwd_parts(const void* x, const void* gamma, const void* g, const void* addend, float eps, void* dx, void* partial,
+                                     int64_t rows, int64_t cols, void* stream) {
+  return rmsnorm_bwd_impl(x, gamma, g, addend, eps, dx, nullptr, partial, rows, cols, stream);
+}
+
+extern "C" int tgh_dgamma_reduce(const tgh_dgamma_job* jobs, int n, int64_t rows, int64_t cols, void* stream) {
+  NormGeom g;
+  if (rows <= 0 || cols <= 0 || !bwd_geom(cols, &g)) return TG_ERR_SHAPE;
+  if (int rc = check_arch()) return rc;
+  return reduce_dgamma(jobs, n, bwd_blocks(rows, g), int(cols), static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------------------

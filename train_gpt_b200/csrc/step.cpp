@@ -137,6 +137,7 @@ class StepProgram {
     m_ = b_ * t_;
     if (t_ > pos_.size(0)) throw py::value_error(cat("sequence of ", t_, " tokens, positions for ", pos_.size(0)));
     status_ = static_cast<unsigned*>(ptr(status_word(embed_.get_device())));
+    norms_.clear();
     plan();
     quantize_weights();
 
@@ -151,7 +152,8 @@ class StepProgram {
     }
     std::vector<Kept> kept(n_layers);
     Tensor x = act(d_), branch;
-    check(api.tgh_embed(ids.data_ptr<int64_t>(), ptr(embed_), ptr(pos_), ptr(x), b_, t_, d_, vocab_, status_, cur_stream()), "tgh_embed");
+    check(api.tgh_embed(ids.data_ptr<int64_t>(), ptr(embed_), ptr(pos_), ptr(x), b_, t_, d_, vocab_, status_, token_table_, ptr(g_embed_), cur_stream()),
+          "tgh_embed");
     for (int64_t l = 0; l < n_layers; ++l) forward_layer(l, kept[l], x, branch);
     // the head: x + branch, norm, logits, loss and the logits' gradient
     Tensor xs = x, hf = act(d_);
@@ -189,8 +191,9 @@ class StepProgram {
     Tensor g_seq = g_pos_.narrow(0, 0, t_);
     at::sum_out(g_seq, d.view({b_, t_, d_}), at::IntArrayRef({0}));
     if (t_ < g_pos_.size(0)) g_pos_.narrow(0, t_, g_pos_.size(0) - t_).zero_();
-    check(api.tgh_embed_bwd(ids.data_ptr<int64_t>(), ptr(d), ptr(g_embed_), token_table_, m_, d_, vocab_, cur_stream()), "tgh_embed_bwd");
+    check(api.tgh_embed_bwd_cleared(ids.data_ptr<int64_t>(), ptr(d), ptr(g_embed_), token_table_, m_, d_, vocab_, cur_stream()), "tgh_embed_bwd");
     bucket_done(int(n_layers + 1));
+    finish_norms();
     if (!on_end_.is_none()) on_end_();
     scratch_ = weights_memory_ = Tensor();
     // ---- optimiser
@@ -255,7 +258,9 @@ class StepProgram {
       for (tg_gemm_args g : {fwd(k, n), dgrad(k, n), wgrad(k, n)}) ws = std::max(ws, api.tg_gemm_workspace_bytes(&g));
     Arena a;
     const FormAt row = add_row(a, m_, wide), col = add_col(a, m_, wide), third = add_col(a, m_, d_);
-    const size_t norm = a.add(std::max<int64_t>(api.tg_rmsnorm_bwd_scratch_bytes(m_, d_), 16)), gemm = a.add(ws), table = a.add(vocab_ * 8);
+    norm_bytes_ = (std::max<int64_t>(api.tg_rmsnorm_bwd_scratch_bytes(m_, d_), 16) + 255) / 256 * 256;
+    norms_at_once_ = std::min<int64_t>(kNormsAtOnce, 2 * int64_t(layers_.size()) + 1);
+    const size_t norm = a.add(norm_bytes_ * norms_at_once_), gemm = a.add(ws), table = a.add(vocab_ * 8);
     a.make(embed_);
     scratch_ = a.memory();
     row_ = row.in(a);
@@ -301,13 +306,18 @@ class StepProgram {
     return x = sum;
   }
   void norm_bwd(const Tensor& x, const Tensor& gamma, const Tensor& g, const Tensor& addend, const Tensor& dx, const Tensor& dgamma) {
-    if (addend.defined())
-      check(api.tg_rmsnorm_bwd_add(ptr(x), ptr(gamma), ptr(g), ptr(addend), float(c_.eps), ptr(dx), ptr(dgamma), norm_partial_, m_, d_,
-                                   cur_stream()),
-            "tg_rmsnorm_bwd_add");
-    else
-      check(api.tg_rmsnorm_bwd(ptr(x), ptr(gamma), ptr(g), float(c_.eps), ptr(dx), ptr(dgamma), norm_partial_, m_, d_, cur_stream()),
-            "tg_rmsnorm_bwd");
+    if (int64_t(norms_.size()) == norms_at_once_) finish_norms();
+    void* partial = static_cast<char*>(norm_partial_) + norms_.size() * norm_bytes_;
+    check(api.tgh_rmsnorm_bwd_parts(ptr(x), ptr(gamma), ptr(g), addend.defined() ? ptr(addend) : nullptr, float(c_.eps), ptr(dx), partial, m_, d_,
+                                    cur_stream()),
+          "tgh_rmsnorm_bwd_parts");
+    norms_.push_back({partial, ptr(dgamma)});
+  }
+  // the weight gradients of the norms whose backward kernels ran since the last call, in one launch
+  void finish_norms() {
+    if (norms_.empty()) return;
+    check(api.tgh_dgamma_reduce(norms_.data(), int(norms_.size()), m_, d_, cur_stream()), "tgh_dgamma_reduce");
+    norms_.clear();
   }
   void quantize(const tgh_quantize_job* jobs, int n) { check(api.tgh_quantize_jobs(jobs, n, cur_stream()), "tgh_quantize_jobs"); }
   Tensor heads(const Tensor& qkv, int64_t which) const {        // (B, H, T, D), a view
@@ -410,7 +420,9 @@ class StepProgram {
   }
 
   void bucket_done(int i) {
-    if (!on_bucket_.is_none()) on_bucket_(i);
+    if (on_bucket_.is_none()) return;
+    finish_norms();                            // (a bucket that is exchanged holds a norm's weight gradient)
+    on_bucket_(i);
   }
 
   Config c_;
@@ -428,6 +440,9 @@ class StepProgram {
   Form row_, col_, third_;
   void *norm_partial_ = nullptr, *workspace_ = nullptr, *token_table_ = nullptr;
   int64_t attention_ = -1;
+  static constexpr int64_t kNormsAtOnce = 16;  // partial sums of so many norms are kept (1.8 MB each at 8192 x 1024)
+  int64_t norm_bytes_ = 0, norms_at_once_ = 0;
+  std::vector<tgh_dgamma_job> norms_;
 };
 
 }  // namespace
