@@ -267,3 +267,19 @@ def test_every_split_of_a_row_over_warps(rows, cols, pure):
         assert torch.equal(y2, y) and torch.equal(q.view(torch.uint8), q_ref.view(torch.uint8)) and torch.equal(s, s_ref)
     if not pure:
         test_backward((rows, cols))
+
+
+# the largest tensors that take a block per row, and one row more, which takes warps: rows of one, two and four groups of pieces, a group
+# that is not full, the widest
+@pytest.mark.parametrize("rows,cols", [(1024, 1024), (2048, 1536), (1536, 2048), (910, 2304), (682, 3072), (409, 5120), (256, 8192), (291, 7168)])
+def test_block_per_row_has_the_bits_of_warps_per_row(rows, cols):
+    from train_gpt_b200 import ops
+    gen = torch.Generator("cuda").manual_seed(cols)
+    x = torch.randn(rows + 400, cols, device="cuda", generator=gen).to(torch.bfloat16)
+    w = (1 + 0.1 * torch.randn(cols, device="cuda", generator=gen)).to(torch.bfloat16)
+    for pure in (False, True):
+        few = ops.rmsnorm_quant_fwd(x[:rows], w, 1e-6, pure, want_y=True, want_rnorm=True)
+        many = ops.rmsnorm_quant_fwd(x, w, 1e-6, pure, want_y=True, want_rnorm=True)
+        for a, b in zip(few, many):
+            assert torch.equal(a.view(torch.uint8), b[:rows].view(torch.uint8))
+        assert torch.equal(ops.rmsnorm_fwd(x[:rows], w, 1e-6, pure), many[2][:rows])

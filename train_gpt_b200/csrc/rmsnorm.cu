@@ -529,8 +529,8 @@ __global__ void __launch_bounds__(1024) rmsnorm_dgamma_reduce_kernel(const __gri
 
 // ---------------------------------------------------------------------------------------
 // Forward for few rows (a decode batch): one thread block per row, one 16-byte piece per thread.  The kernels above give a row
-// to one to four warps, which is right when there are rows to fill the GPU with; for a handful the time is one warp's chain of
-// loads and passes over 8 KB and more of row, plus widening gamma into shared memory.  16 x 8192: 5.0 -> 3.4 us, 1 x 2048: 3.1 -> 2.1.
+// to one to four warps, which is right when there are rows to fill the GPU with; for a few the time is one warp's chain of
+// loads and passes over 8 KB and more of row, plus widening gamma into shared memory.  16 x 8192: 5.0 -> 2.5 us, 1 x 2048: 3.1 -> 1.5.
 // The sum of squares is added in the order of those kernels (a lane's pieces of every 256 columns as a tree, eight of them to
 // a warp, then the lanes, then the warps), so which of them runs does not show in the result.
 // Launched early (see common.cuh): in a decode loop the kernel before it is the last GEMM's reduction.
@@ -551,16 +551,30 @@ rmsnorm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   const uint4 gq = ok ? *reinterpret_cast<const uint4*>(gamma + col) : make_uint4(0, 0, 0, 0);
   s_part[warp][lane] = sumsq8(w);
   __syncthreads();
-  float ss = 0.f;
   const int warps = int(blockDim.x >> 5);
-  for (int g = 0; g < groups; ++g) {
+  auto group_sum = [&](int g) {
     float v[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) v[c] = c < chunks && g * chunks + c < warps ? s_part[g * chunks + c][lane] : 0.f;
-    float t = tree_sum(v);
+    float s = tree_sum(v);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    ss = g == 0 ? t : ss + t;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+  };
+  // One group: every warp adds it up for itself.  Two to four: a warp each, and one more barrier (all warps through all groups were
+  // 1024 shared-memory reads of an 8192-wide row: 16 x 8192 3.4 us, now 2.6).
+  float ss;
+  if (groups == 1) {
+    ss = group_sum(0);
+  } else {
+    __shared__ float s_group[4];
+    if (warp < groups) {
+      const float s = group_sum(warp);
+      if (lane == 0) s_group[warp] = s;
+    }
+    __syncthreads();
+    ss = s_group[0];
+    for (int g = 1; g < groups; ++g) ss += s_group[g];
   }
   const float rn = __frsqrt_rn(__fdiv_rn(ss, float(cols)) + eps);
   if (rnorm_out != nullptr && threadIdx.x == 0) rnorm_out[row] = rn;
@@ -588,10 +602,11 @@ rmsnorm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     }
   }
 }
-// Where the two meet (graph replays, microseconds, this kernel / the ones above): 2048 x 512 2.6 / 2.7, 512 x 2048 with the
-// quantiser 3.2 / 3.6 and 1024 x 2048 3.8 / 3.7, 256 x 4096 3.5 / 4.3, 64 x 8192 4.2 / 4.3, 128 x 8192 5.4 / 4.3 (a block of 1024
-// threads leaves room for one more).
-static bool few_rows(int64_t rows, int64_t cols) { return rows * cols <= (cols > 4096 ? 1 << 19 : 1 << 20); }
+// Where the two meet (graph replays, microseconds with the quantiser, this kernel / the ones above): 1023 x 1024 3.0 / 3.8, 2047 x 1024 3.8 / 3.9
+// but without the quantiser 3.3 / 2.9; 1023 x 2048 3.8 / 5.2, 1447 x 2048 4.6 / 5.8, 2047 x 2048 5.9 / 6.0; 681 x 3072 3.6 / 4.3, 964 x 3072
+// 4.7 / 4.4; 511 x 4096 3.7 / 4.7, 723 x 4096 4.6 / 4.8 and 3.5 / 4.4; 255 x 8192 3.9 / 5.1, 361 x 8192 5.5 / 5.3; narrower rows fill warps of their own
+// (2895 x 512 4.0 / 3.0).
+static bool few_rows(int64_t rows, int64_t cols) { return rows * cols <= (cols < 1536 ? 1 << 20 : cols <= 2048 ? 3 << 20 : 1 << 21); }
 
 struct NormGeom {
   int nchunk, wpr;
