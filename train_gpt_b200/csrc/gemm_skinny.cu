@@ -28,9 +28,14 @@ namespace tg {
 // From 129 tokens on the tokens fill 128 MMA rows themselves, a token scale is a thread's own number instead of a column's,
 // and the tiled kernel is the faster one: 200 tokens, tiled / this kernel with 256 columns, a scale per 128 weight columns (per
 // column): 2048 x 8192 8.6 / 14.1 us (10.1 / 13.7), 4096 x 4096 12.0 / 16.2 (14.1 / 15.7), 8192 x 8192 25.0 / 40.4 (37.4 / 37.3).
-// Below, both sides with the weight from memory, this kernel / tiled: 64 tokens 8192 x 8192 16.3 / 18.0 (16.7 / 20.9), 4096 x 4096
-// 9.2 / 9.4 (9.4 / 11.0); 100 tokens 20.2 / 18.7 (20.5 / 22.0), 10.7 / 9.8 (10.9 / 11.5), 2048 x 8192 9.7 / 8.3 (9.8 / 11.7).  So with a
-// scale per 128 columns the line would be better drawn at 64.
+// Below, both sides with the weight from memory, this kernel / tiled (a scale per 128 weight columns; per column in brackets):
+//   100 tokens  512 x 512 5.4 / 4.0 (5.4 / 4.1), 1024 x 4096 7.5 / 5.8 (7.5 / 6.2), 2048 x 8192 9.7 / 8.3 (9.8 / 8.9), 4096 x 4096 10.8 / 10.1
+//               (10.9 / 11.0), 8192 x 8192 20.1 / 18.6 (20.3 / 21.6), 2048 x 2048 7.5 / 7.9 (7.6 / 8.4), 4096 x 1024 8.3 / 8.1 (8.3 / 9.1)
+//   48 tokens   512 x 512 4.8 / 3.9 (4.9 / 4.0), 640 x 7680 6.1 / 5.3 (6.1 / 5.6), 1024 x 1024 5.7 / 5.1 (5.8 / 5.4), 1024 x 4096 6.3 / 5.7
+//               (6.3 / 6.1), 2048 x 6144 7.9 / 8.0 (8.0 / 8.5), 4096 x 4096 8.9 / 9.1 (9.1 / 9.9), 8192 x 8192 15.9 / 17.6 (16.2 / 19.6)
+//   16 tokens   512 x 512 4.0 / 3.8 (4.1 / 3.9), 3072 x 512 7.9 / 6.7 (7.8 / 6.9), 1024 x 1024 4.7 / 5.0, 1024 x 4096 5.1 / 5.7, 8192 x 8192 13.4 / 16.9
+// So with more than 64 tokens and a scale per 128 columns the line is at the narrow weights, else at short contractions: the few-token
+// kernel's sums meet in a cluster or a second kernel, the tiled one's chain is then short.
 constexpr int kSkinnyMaxTokens = 128;
 
 template <int BN_>
@@ -342,7 +347,14 @@ skinny_reduce_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, 
 // The activation must be [M][K] (it becomes the K-major B operand).  Below 512 of contraction or 256 of width the weight is
 // nothing to stream and the tiled kernel's single launch is the shorter way.
 bool skinny_takes(const tg_gemm_args* a) {
-  return a->M > 0 && a->M <= kSkinnyMaxTokens && a->a_major == TG_MAJOR_K && a->K % BK == 0 && a->K >= 512 && a->N >= 256 && a->N <= (1 << 22) && a->K <= (1 << 22);
+  if (a->M <= 0 || a->M > kSkinnyMaxTokens || a->a_major != TG_MAJOR_K || a->K % BK != 0 || a->K < 512 || a->N < 256 || a->N > (1 << 22) ||
+      a->K > (1 << 22))
+    return false;
+  const bool columns = a->sb_gran_n == 1;
+  if (a->N <= 512 && (a->K <= 1024 || a->M <= 32)) return false;
+  if (a->M <= 32) return true;
+  if (a->M <= 64) return a->K > (columns || a->N < 4096 ? 768 : 1024);
+  return a->K > 1024 && (columns || (a->N <= 2048 && a->K <= 4096));
 }
 
 struct SkinnyPlan {
