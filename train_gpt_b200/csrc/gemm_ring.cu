@@ -28,8 +28,9 @@
 //   - A wait's outcome is looked at once a tile, not voted on in every block.
 //   - The buffer goes back by an arrival with CTA scope on the first CTA's barrier.  With cluster scope the release is a fence that waits
 //     for the SM's copies in flight: 700 us instead of 360.
-// Forward 32768 x 2048 -> 6144 in a loop: 435 us with gemm_fp8.cu, 415 here (1.90 / 1.99 PFLOP/s); with a scale per column 555 / 500;
-// its weight gradient 584 / 550 (six waves where 5.2 would do); in short bursts 383 / 355, 530 / 435, 530 / 500.
+//   - In the last block of a bf16 tile each piece is converted and staged as soon as it is complete (forward 421 -> 413 us).
+// Forward 32768 x 2048 -> 6144 in a loop: 435 us with gemm_fp8.cu, 413 here (1.90 / 2.00 PFLOP/s); with a scale per column 555 / 512;
+// its weight gradient 584 / 548 (six waves where 5.2 would do); in short bursts 383 / 346, 530 / 435, 530 / 480.
 //
 // One SM with column scales: gemm_fp8.cu's promotion warps fetch and stage the scales of every block themselves, here they find them.
 // From twelve blocks on 1.05-1.4 times as fast in one wave (200 x 2048 -> 8192 9.6 / 8.8 us, 500 x 4096 -> 4096 19.4 / 14.7, weight gradient
@@ -436,6 +437,45 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         item_split(p, item, n_tiles, ks, tile);
         nkb = range_blocks(p, ks);
       }
+      // Rows in bf16: the last block stages each piece as soon as it is complete, beside the promotion of the next (forward and data
+      // gradient 2 % faster at 8 and 16 blocks a tile; in fragments, whose stores are four bytes each, 0.5 % slower)
+      constexpr bool kStageInBlock = C::phases == 1 && !OUT_F32 && !kFrag;
+      const int plain = kStageInBlock ? nkb - 1 : nkb;
+      const bool last = item + item_step >= n_items;
+      auto rows_free = [&]() {      // the staging rows have been read (the first pass finds them free)
+        ok &= mbar_wait(unstaged_bar, uph, abort_flag, p.status, 8u);
+        __syncwarp();
+        uph ^= 1u;
+      };
+      // Piece q (of the phase, which begins with piece q0 of the accumulator).  Fragments: rows fg + 8 i; bf16: 16-byte chunk 2 q + k of the
+      // box's row, 4 fj bytes in; float32: chunk 4 q + 2 k + (fj >> 1), half fj & 1.  Rows: chunks 2 q, 2 q + 1 (float32: 4 q ...).
+      // Swizzle: chunk xor the row's low three bits, with 64-byte rows xor the two above the lowest.
+      const uint32_t st_base = wb + (kFrag ? uint32_t(fg) * C::box_row + (OUT_F32 ? (uint32_t(fj >> 1) << 4) + 8u * uint32_t(fj & 1) : 4u * uint32_t(fj))
+                                           : uint32_t(lane) * 128u);
+      const uint32_t st_flip = (!kFrag ? uint32_t(lane & 7) : C::box_row == 128 ? uint32_t(fg) : uint32_t(fg >> 1)) << 4;
+      auto stage = [&](auto qc, auto q0c) {
+        constexpr int qq = decltype(qc)::value, q0 = decltype(q0c)::value, q = qq % C::box_pieces, box = (qq / C::box_pieces) * C::box_bytes;
+        if constexpr (kFrag) {
+          static_loop<4>([&](auto i) {
+            static_loop<2>([&](auto k) {
+              const float2 a = acc[(4 * (q0 + qq) + i.value) * 2 + k.value];
+              if constexpr (OUT_F32) sts_swz_f32x2<box + i.value * 8 * C::box_row + (4 * q + 2 * k.value) * 16>(st_base, st_flip, a);
+              else sts_swz_b32<box + i.value * 8 * C::box_row + (2 * q + k.value) * 16>(st_base, st_flip, pack_bf16x2(a.x, a.y));
+            });
+          });
+        } else if constexpr (OUT_F32) {
+          static_loop<4>([&](auto c) {
+            const int j = 8 * (q0 + qq) + 2 * c.value;
+            sts_swz_f32x4<box + (4 * q + c.value) * 16>(st_base, st_flip, acc[j], acc[j + 1]);
+          });
+        } else {
+          static_loop<2>([&](auto c) {
+            const int j = 8 * (q0 + qq) + 4 * c.value;
+            sts_swz_v4<box + (2 * q + c.value) * 16>(st_base, st_flip, pack_bf16x2(acc[j].x, acc[j].y), pack_bf16x2(acc[j + 1].x, acc[j + 1].y),
+                                                     pack_bf16x2(acc[j + 2].x, acc[j + 2].y), pack_bf16x2(acc[j + 3].x, acc[j + 3].y));
+          });
+        }
+      };
       auto enter_block = [&]() {
         ok &= mbar_wait(tfull0 + 8u * buf, bph, abort_flag, p.status, 5u);
         __syncwarp();
@@ -449,17 +489,16 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         if (++buf == kBufs) { buf = 0; bph ^= 1u; }
       };
       if constexpr (kFrag) {
-#pragma unroll 1
-        for (int kb = 0; kb < nkb; ++kb) {
+        // acc[(4 q + i) * 2 + k] holds rows fg + 8 i, columns 16 q + 8 k + 2 fj (+1)
+        auto block = [&](auto staging) {
           const float* sc = enter_block();
           const uint32_t taddr = tcol0 + buf * uint32_t(C::tmem_stride);
           float sa_r[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) sa_r[i] = sc[quarter * 32 + fg + 8 * i];
           const float* scol = sc + 128 + cg * C::cols + 2 * fj;
-          // acc[(4 q + i) * 2 + k] holds rows fg + 8 i, columns 16 q + 8 k + 2 fj (+1)
-#pragma unroll
-          for (int q = 0; q < C::pieces; ++q) {
+          static_loop<C::pieces>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
             uint32_t v[16];
             float2 sb2[2];
             sb2[0] = *reinterpret_cast<const float2*>(scol + 16 * q);
@@ -478,7 +517,14 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 a = __ffma2_rn(__fmul2_rn(pv, sb2[k]), make_float2(sa_r[i], sa_r[i]), a);
               }
             }
-          }
+            if constexpr (decltype(staging)::value != 0) stage(qc, IntC<0>{});
+          });
+        };
+#pragma unroll 1
+        for (int kb = 0; kb < plain; ++kb) block(IntC<0>{});
+        if constexpr (kStageInBlock) {
+          rows_free();
+          block(IntC<1>{});
         }
       } else {
         // two register buffers: the next piece is on its way while one is promoted, across blocks too
@@ -488,7 +534,7 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         uint32_t taddr = tcol0 + buf * uint32_t(C::tmem_stride);
         tmem_ld16(taddr, v[0]);
 #pragma unroll 1
-        for (int kb = 0; kb < nkb; ++kb) {
+        for (int kb = 0; kb < plain; ++kb) {
           const bool more = kb + 1 < nkb;
 #pragma unroll
           for (int q = 0; q < C::pieces - 1; ++q) {
@@ -508,52 +554,33 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           promote<128, 16>(acc + 8 * (C::pieces - 1), v[1], nullptr, 0.f, s);
           s = s_next;
         }
+        if constexpr (kStageInBlock) {
+          rows_free();
+          static_loop<C::pieces>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            tmem_wait_ld16(v[q & 1]);
+            if constexpr (q + 1 < C::pieces) tmem_ld16(taddr + 16 * (q + 1), v[(q + 1) & 1]);
+            else leave_block();
+            promote<128, 16>(acc + 8 * q, v[q & 1], nullptr, 0.f, s);
+            stage(qc, IntC<0>{});
+          });
+        }
       }
       if (!__all_sync(0xffffffffu, ok)) break;
 
       // ---- epilogue: registers -> this warp's swizzled staging rows -> bulk stores ----
-      const bool last = item + item_step >= n_items;
-#pragma unroll
-      for (int phase = 0; phase < C::phases; ++phase) {
-        // The store warp hands a tile's boxes to the copy engine one after the other (40 cycles each), beside the next tile's first
-        // blocks.  After the last tile nothing hides that: every warp issues its own.
-        if (!last || phase == 0) {         // (the first pass finds the rows free)
-          ok = __all_sync(0xffffffffu, mbar_wait(unstaged_bar, uph, abort_flag, p.status, 8u));
-          if (!ok) break;
-          uph ^= 1u;
-        } else {
-          if (is_lane0) tma_store_wait_read();
-          __syncwarp();
-        }
-        if constexpr (kFrag) {
-          // rows fg + 8 i; bf16: 16-byte chunk 2 q + k of the box's row, 4 fj bytes in; float32: chunk 4 q + 2 k + (fj >> 1), half fj & 1.
-          // Swizzle: chunk xor the row's low three bits, with 64-byte rows xor the two above the lowest.
-          const uint32_t base = wb + uint32_t(fg) * C::box_row + (OUT_F32 ? (uint32_t(fj >> 1) << 4) + 8u * uint32_t(fj & 1) : 4u * uint32_t(fj));
-          const uint32_t flip = (C::box_row == 128 ? uint32_t(fg) : uint32_t(fg >> 1)) << 4;
-          static_loop<C::warp_boxes * C::box_pieces>([&](auto qq) {
-            static_loop<4>([&](auto i) {
-              static_loop<2>([&](auto k) {
-                constexpr int q = qq.value % C::box_pieces, off = (qq.value / C::box_pieces) * C::box_bytes + i.value * 8 * C::box_row;
-                const float2 a = acc[(4 * (phase * C::warp_boxes * C::box_pieces + qq.value) + i.value) * 2 + k.value];
-                if constexpr (OUT_F32) sts_swz_f32x2<off + (4 * q + 2 * k.value) * 16>(base, flip, a);
-                else sts_swz_b32<off + (2 * q + k.value) * 16>(base, flip, pack_bf16x2(a.x, a.y));
-              });
-            });
-          });
-        } else if constexpr (OUT_F32) {
-          const uint32_t base = wb + uint32_t(lane) * 128u, flip = uint32_t(lane & 7) << 4;
-          static_loop<8 * C::warp_boxes>([&](auto c) {
-            const int j = 16 * C::warp_boxes * phase + 2 * c.value;
-            sts_swz_f32x4<(c.value >> 3) * C::box_bytes + (c.value & 7) * 16>(base, flip, acc[j], acc[j + 1]);
-          });
-        } else {
-          const uint32_t base = wb + uint32_t(lane) * 128u, flip = uint32_t(lane & 7) << 4;
-          static_loop<8 * C::warp_boxes>([&](auto c) {
-            const int j = 4 * c.value;
-            sts_swz_v4<(c.value >> 3) * C::box_bytes + (c.value & 7) * 16>(
-                base, flip, pack_bf16x2(acc[j].x, acc[j].y), pack_bf16x2(acc[j + 1].x, acc[j + 1].y),
-                pack_bf16x2(acc[j + 2].x, acc[j + 2].y), pack_bf16x2(acc[j + 3].x, acc[j + 3].y));
-          });
+      // The store warp hands a tile's boxes to the copy engine one after the other (40 cycles each), beside the next tile's first
+      // blocks.  After the last tile nothing hides that: every warp issues its own.
+      static_loop<C::phases>([&](auto pc) {
+        constexpr int phase = decltype(pc)::value;
+        if constexpr (!kStageInBlock) {
+          if (!last || phase == 0) {
+            rows_free();
+          } else {
+            if (is_lane0) tma_store_wait_read();
+            __syncwarp();
+          }
+          static_loop<C::warp_boxes * C::box_pieces>([&](auto qc) { stage(qc, IntC<phase * C::warp_boxes * C::box_pieces>{}); });
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the copy engine
         __syncwarp();
@@ -570,8 +597,8 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
         __syncwarp();
-      }
-      if (!ok) break;
+      });
+      if (!__all_sync(0xffffffffu, ok)) break;
     }
   }
 
