@@ -10,6 +10,18 @@ pytestmark = pytest.mark.gpu
                                         (1025, 1280, 640), (300, 128, 4096)])
 @pytest.mark.parametrize("tile,mode", [((128, 128), "fp8"), ((128, 1), "fp8"), ((128, 128), "fp8_blockgrad")])
 def test_backward_has_the_bits_of_two_launches(tokens, k, n, tile, mode):
+    _compare(tokens, k, n, tile, mode)
+
+
+# Both on pairs of SMs: a weight gradient cut in two, in three, uncut; several rounds of it, one, less than one; idle pairs that take all of
+# the data gradient's tiles, a round of them, or none; ragged tokens and columns (an odd number of 128-column blocks)
+@pytest.mark.parametrize("tokens,k,n", [(8192, 2048, 2048), (5000, 2048, 4224), (24576, 1024, 1024), (5000, 1024, 4096), (6145, 2048, 2176),
+                                        (24576, 1024, 3072), (2048, 2048, 2048), (700, 4096, 4096), (12000, 768, 3072), (4100, 640, 3200)])
+def test_backward_on_pairs_has_the_bits_of_two_launches(tokens, k, n):
+    _compare(tokens, k, n, (128, 128), "fp8")
+
+
+def _compare(tokens, k, n, tile, mode):
     from train_gpt_b200 import fp8, ops
     gen = torch.Generator("cuda").manual_seed(tokens + k + n)
     x = torch.randn(tokens, k, device="cuda", generator=gen).to(torch.bfloat16).requires_grad_()

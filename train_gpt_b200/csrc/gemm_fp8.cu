@@ -748,6 +748,7 @@ struct GemmPlan {
   int64_t bytes;     // workspace the cut needs
   bool pair;         // 256 x 256 tiles on pairs of SMs (gemm_ring.cu)
   bool ring;         // bn-wide tiles by gemm_ring.cu
+  double us;         // modelled time
 };
 // S of 1 to 8 ranges of at least 8 blocks by waves of wide tiles x (blocks per item + 3 for an item's ramp and stores), plus for
 // S > 1 the reduction over S float32 slices at 4 MB per block time.
@@ -768,7 +769,7 @@ static int training_ranges(const tg_gemm_args* a, int wide) {
 static GemmPlan plan_gemm(const tg_gemm_args* a) {
   const bool columns = a->sb_gran_n == 1;
   const int wide = a->N <= 128 ? 128 : columns ? 192 : 256;
-  GemmPlan pl = {wide, 1, 0, false, false};
+  GemmPlan pl = {wide, 1, 0, false, false, 0.0};
   const int64_t nkb = (a->K + BK - 1) / BK;
   const int sms = gemm_sms();
   const bool whole = a->K % BK == 0 && (a->a_major == TG_MAJOR_MN || a->M % 128 == 0);      // (weight gradient: the tokens are K)
@@ -799,12 +800,14 @@ static GemmPlan plan_gemm(const tg_gemm_args* a) {
   if (a->M > 128 && a->N > 128) {
     const int64_t pairs = std::max(1, sms / 2), items = ((a->M + 255) / 256) * ((a->N + 255) / 256) * pl.S, waves = (items + pairs - 1) / pairs;
     const double blocks = double((nkb + pl.S - 1) / pl.S);
-    double us = 4.3 + double(waves) * ((columns ? 0.54 : 0.42) * blocks + 0.86);
+    double us = 4.3 + double(waves) * pair_item_us(columns, blocks);
     if (pl.S > 1) us += 3.5 + double(4 * pl.S + 2) * double(a->M) * double(a->N) / 8.0e6;
     if (columns && a->sb_stride_n != 1 && 2 * items > pairs) best += 0.5 * best_blocks;
     pl.pair = us < best && (nkb >= 8 || waves >= 3);
     if (pl.pair) pl.bn = 256;
+    best = std::min(best, us);
   }
+  pl.us = best;
   // Column scales through gemm_ring.cu's ring, where the contraction is long enough for its later start (the measurement is there).
   // Cut problems of 192-column tiles stay: their float32 tiles leave in three steps there (0.95-1.08 times as fast).
   pl.ring = !pl.pair && columns && (nkb + pl.S - 1) / pl.S >= 12 && (pl.bn == 128 || (pl.bn == 192 && (pl.S == 1 && a->out_dtype == TG_OUT_BF16)));
@@ -880,6 +883,26 @@ static GemmParams params_of(const tg_gemm_args* a) {
   return p;
 }
 
+static bool cut_fits(const tg_gemm_args* a, const GemmPlan& pl) {
+  return pl.S > 1 && a->workspace != nullptr && a->workspace_bytes >= pl.bytes && aligned16(a->workspace);
+}
+static void cut_params(const tg_gemm_args* a, int S, GemmParams& p) {
+  p.ksplit = S;
+  p.nkb_rem = p.nkb % S;
+  p.nkb /= S;
+  p.slice_elems = a->M * a->N;
+  p.d = a->workspace;
+  p.ldd = a->N;
+}
+static int reduce_ranges(const tg_gemm_args* a, int S, cudaStream_t st) {
+  const long long quads = a->M * (a->N / 4);
+  const int blocks = int(quads / 256 + 1 < 4096 ? quads / 256 + 1 : 4096);
+  TG_CUDA_CHECK(launch_if_short(blocks <= 8 * gemm_sms(), a->out_dtype == TG_OUT_F32 ? splitk_reduce_kernel<true> : splitk_reduce_kernel<false>,
+                                dim3(unsigned(blocks)), 256, 0, st, static_cast<const float*>(a->workspace), a->d, int(a->M), int(a->N),
+                                static_cast<long long>(a->ldd), S, static_cast<long long>(a->M * a->N)));
+  return TG_OK;
+}
+
 extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
   if (int rc = validate_gemm(a)) return rc;
   if (a->M == 0 || a->N == 0) return TG_OK;
@@ -901,25 +924,15 @@ extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
   const bool g1 = a->sb_gran_n == 1;
   const GemmPlan pl = plan_gemm(a);
   const int bn = pl.bn;
-  if (pl.S > 1 && a->workspace != nullptr && a->workspace_bytes >= pl.bytes && aligned16(a->workspace)) {
-    p.ksplit = pl.S;
-    p.nkb_rem = p.nkb % pl.S;
-    p.nkb /= pl.S;
-    p.slice_elems = a->M * a->N;
-    p.d = a->workspace;
-    p.ldd = a->N;
+  if (cut_fits(a, pl)) {
+    cut_params(a, pl.S, p);
     int rc;
     if (pl.pair || pl.ring) rc = ring_run(a, p, pl.pair, bn, true, st);
     else if (bn == 256) rc = launch_gemm<256, 128, true>(a, p, st);
     else if (bn == 192) rc = launch_gemm<192, 1, true>(a, p, st);
     else rc = g1 ? launch_gemm<128, 1, true>(a, p, st) : launch_gemm<128, 128, true>(a, p, st);
     if (rc != TG_OK) return rc;
-    const long long quads = a->M * (a->N / 4);
-    const int blocks = int(quads / 256 + 1 < 4096 ? quads / 256 + 1 : 4096);
-    TG_CUDA_CHECK(launch_if_short(blocks <= 8 * gemm_sms(), f32 ? splitk_reduce_kernel<true> : splitk_reduce_kernel<false>, dim3(unsigned(blocks)), 256, 0,
-                                  st, static_cast<const float*>(a->workspace), a->d, int(a->M), int(a->N), static_cast<long long>(a->ldd), pl.S,
-                                  static_cast<long long>(p.slice_elems)));
-    return TG_OK;
+    return reduce_ranges(a, pl.S, st);
   }
   if (pl.pair || pl.ring) return ring_run(a, p, pl.pair, bn, f32, st);
   if (bn == 256) return f32 ? launch_gemm<256, 128, true>(a, p, st) : launch_gemm<256, 128, false>(a, p, st);
@@ -935,6 +948,23 @@ static int two_tiles(const tg_gemm_args* a) {
   const GemmPlan pl = plan_gemm(a);
   const int64_t tiles = ((a->M + 127) / 128) * ((a->N + 127) / 128);
   return pl.pair || pl.ring || pl.bn != 128 || pl.S != 1 || tiles > INT32_MAX / 2 ? 0 : int(tiles);
+}
+
+// Whether a problem passes all checks and could run in 256 x 256 tiles.
+static bool tiled(const tg_gemm_args* a) {
+  if (validate_gemm(a) != TG_OK || a->M <= 128 || a->N <= 128 || a->K == 0 || skinny_takes(a)) return false;
+  return aligned16(a->a) && aligned16(a->b) && aligned16(a->d) && check_scales(a) == TG_OK;
+}
+
+// Modelled time of a (column scales) in S ranges and then b (block scales), both on pairs in one launch.
+static double pairs_together_us(const tg_gemm_args* a, int S, const tg_gemm_args* b) {
+  auto tiles = [](const tg_gemm_args* x) { return ((x->M + 255) / 256) * ((x->N + 255) / 256); };
+  auto blocks = [](const tg_gemm_args* x, int n) { return double(((x->K + BK - 1) / BK + n - 1) / n); };
+  int rounds = 0;
+  double us = 4.3 + two_problems_us(tiles(a) * S, pair_item_us(true, blocks(a, S)), tiles(b), pair_item_us(false, blocks(b, 1)),
+                                    std::max(1, gemm_sms() / 2), rounds);
+  if (S > 1) us += 3.5 + double(4 * S + 2) * double(a->M) * double(a->N) / 8.0e6;
+  return us;
 }
 
 template <int GRAN1, int GRAN2>
@@ -966,6 +996,22 @@ extern "C" int tgh_gemm_two(const tg_gemm_args* a, const tg_gemm_args* b, void* 
     if (a->sb_gran_n == 128 && b->sb_gran_n == 1) return launch_two<128, 1>(a, b, n1, n2, st);
     if (a->sb_gran_n == 1 && b->sb_gran_n == 1) return launch_two<1, 1>(a, b, n1, n2, st);
     if (a->sb_gran_n == 128 && b->sb_gran_n == 128) return launch_two<128, 128>(a, b, n1, n2, st);
+  }
+  // Both on pairs of SMs, where one launch fills the last rounds (gemm_ring_two_kernel).  The modelled saving is 4 to 8 % too high (four
+  // linears of 32768 tokens: 6-8 % modelled, -0.1 to 3 % measured in short runs, -1 to 2 % at the power cap); from a twelfth on every
+  // measured pair of problems gained (2-17 %, 700 x 4096 -> 4096 54.1 / 47.2 us with the quantisers).  A data gradient with a scale per
+  // column stays apart: 12000 x 768 -> 3072 115 / 123 us, 4096 x 768 -> 3072 49.5 / 60, though 24576 x 1024 -> 1024 110 / 92.
+  if (a->sb_gran_n == 128 && b->sb_gran_n == 1 && a->out_dtype == TG_OUT_BF16 && tiled(a) && tiled(b)) {
+    const GemmPlan one = plan_gemm(b), two = plan_gemm(a);
+    const bool cut = cut_fits(b, one);
+    if (two.S == 1 && (cut || b->out_dtype == TG_OUT_BF16) && pairs_together_us(b, cut ? one.S : 1, a) < (11.0 / 12.0) * (one.us + two.us)) {
+      if (int rc = check_arch()) return rc;
+      cudaStream_t st = static_cast<cudaStream_t>(stream);
+      GemmParams p = params_of(b);
+      if (cut) cut_params(b, one.S, p);
+      if (int rc = ring_pair_two(b, p, cut, a, params_of(a), st)) return rc;
+      return cut ? reduce_ranges(b, one.S, st) : TG_OK;
+    }
   }
   if (int rc = tg_gemm_fp8_blockscaled(a, stream)) return rc;
   return tg_gemm_fp8_blockscaled(b, stream);

@@ -124,7 +124,8 @@ constexpr int kBandRows = 16;      // 128-row tiles per band of the numbering (s
 // Compile-time plan of one variant: CG CTAs (a cluster of two, or one) on a tile of 128 CG rows x BN columns.
 template <int CG, int BN_, int SB_GRAN, bool OUT_F32>
 struct RingCfg {
-  static constexpr int BN = BN_;
+  static constexpr int BN = BN_, sb_gran = SB_GRAN;
+  static constexpr bool out_f32 = OUT_F32;
   static constexpr int promo_warps = 8;
   static constexpr int producer_warp = 8, issuer_warp = 9, scale_warp = 10, store_warp = 11;
   static constexpr int threads = 384;
@@ -165,12 +166,36 @@ struct RingCfg {
   static_assert(stages >= 3 && stages >= tmem_bufs && smem_bytes + static_reserve <= kSmemLimit, "shared-memory plan");
 };
 
-template <int CG, int BN_, int SB_GRAN, bool OUT_F32>
-__global__ void __launch_bounds__((RingCfg<CG, BN_, SB_GRAN, OUT_F32>::threads), 1)
-gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const __grid_constant__ CUtensorMap tmap_d, const GemmParams p) {
-  using C = RingCfg<CG, BN_, SB_GRAN, OUT_F32>;
+struct RingProblem {
+  CUtensorMap a, b, d;
+  GemmParams p;
+};
+
+// The items of a problem that one unit (a CTA or a pair) works on, in order: `early` of them from `early_first` on in steps of
+// `early_step`, then from `first` on in steps of `step`, while they are below n.
+struct Walk {
+  int early, early_first, early_step, first, step, n;
+};
+__device__ __forceinline__ int walk_item(const Walk& w, int k) {
+  const int i = k < w.early ? w.early_first + k * w.early_step : w.first + (k - w.early) * w.step;
+  return i < w.n ? i : -1;
+}
+// Two problems on the same units: the first one's items go round, and the units that its last round leaves idle take `rounds` rounds of the
+// second one's meanwhile, before all take it up.
+__device__ __forceinline__ Walk walk_alone(int unit, int units, int n) { return Walk{0, 0, 0, unit, units, n}; }
+__device__ __forceinline__ Walk walk_second(int unit, int units, int n1, int n2, int rounds) {
+  const int busy = n1 % units, idle = units - busy;
+  if (busy == 0) return walk_alone(unit, units, n2);
+  const int place = unit >= busy ? unit - busy : unit + idle;         // the idle ones come first
+  return Walk{unit >= busy ? rounds : 0, place, idle, rounds * idle + place, units, n2};
+}
+
+// C and D: the plans of the two problems (TWO) or C twice.
+template <int CG, typename C, typename D, bool TWO, typename START>
+__device__ __forceinline__ void ring_body(const RingProblem& one, const RingProblem& two, int rounds, START&& start) {
   constexpr int BN = C::BN, kStages = C::stages, kRing = C::ring, kBufs = C::tmem_bufs;
+  static_assert(C::BN == D::BN && C::stages == D::stages && C::out_bytes == D::out_bytes && C::stage_bytes == D::stage_bytes, "one layout for both");
+  constexpr int kSlot = C::slot_floats > D::slot_floats ? C::slot_floats : D::slot_floats;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(16) uint64_t ctl_bars[24];
   __shared__ uint32_t ctl_tmem_ptr;
@@ -182,16 +207,20 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   volatile uint32_t* tmem_ptr_smem = &ctl_tmem_ptr;
   volatile int* abort_flag = &ctl_abort;
 
+  unsigned* const status = one.p.status;
   if ((sbase & 1023u) != 0) {   // the swizzled operand layout needs this alignment (both CTAs have the same layout)
-    if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0u, 6u);
+    if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0u, 6u);
     return;
   }
 
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t rank = CG == 2 ? cluster_rank() : 0u;
-  const int n_tiles = p.tiles_m * p.tiles_n;
-  const int n_items = n_tiles * p.ksplit;
-  const int first_item = int(blockIdx.x) / CG, item_step = int(gridDim.x) / CG;
+  const int unit = int(blockIdx.x) / CG, units = int(gridDim.x) / CG;
+  auto items_of = [](const GemmParams& p) { return p.tiles_m * p.tiles_n * p.ksplit; };
+  const Walk walk1 = walk_alone(unit, units, items_of(one.p));
+  const Walk walk2 = TWO ? walk_second(unit, units, items_of(one.p), items_of(two.p), rounds) : walk1;
+  // is there an item after the k-th of this problem?
+  auto followed = [&](const Walk& w, int k, bool first) { return walk_item(w, k + 1) >= 0 || (TWO && first && walk_item(walk2, 0) >= 0); };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -207,8 +236,8 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     mbar_init(unstaged_bar, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_a)) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap_b)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&one.a)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&one.b)) : "memory");
   }
   if (warp == C::issuer_warp) {
     if constexpr (CG == 2) {
@@ -224,8 +253,7 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
-  grid_trigger();
-  grid_wait();
+  start();
 
   if (warp >= C::promo_warps) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::service_regs));
@@ -234,78 +262,88 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       uint32_t s = 0, ph = 1;
       bool ok = true;
       const uint32_t full_leader = CG == 2 ? map_rank(full0, 0u) : full0;
-      for (int item = first_item; ok && item < n_items; item += item_step) {
+      auto produce = [&](const RingProblem& q, const Walk& w) {
+       const GemmParams& p = q.p;
+       for (int k = 0, item; ok && (item = walk_item(w, k)) >= 0; ++k) {
         int ks, tile, tm, tn;
-        item_split(p, item, n_tiles, ks, tile);
+        item_split(p, item, p.tiles_m * p.tiles_n, ks, tile);
         tile_coords(p, tile, tm, tn);
         const int m0 = (tm * CG + int(rank)) * BM, n0 = tn * BN + int(rank) * 128;     // (past M or N: zeros)
         int k0 = range_first(p, ks) * BK;
         const int nkb = range_blocks(p, ks);
         for (int kb = 0; kb < nkb; ++kb, k0 += BK) {
-          ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8u * s, ph, abort_flag, p.status, 1u));
+          ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8u * s, ph, abort_flag, status, 1u));
           if (!ok) break;
           if (elect_one()) {
             const uint32_t dst = sbase + s * C::stage_bytes, fb = full_leader + 8u * s;
             // The first CTA announces the bytes of both.  The second's may land before that: its barrier phase is the same one,
             // since the stage was free in both CTAs only after the phase before had completed.
             if (rank == 0) mbar_expect_tx(full0 + 8u * s, CG * C::stage_bytes);
-            tma_load<CG>(dst, &tmap_a, fb, p.a_mn ? m0 : k0, p.a_mn ? k0 : m0);
+            tma_load<CG>(dst, &q.a, fb, p.a_mn ? m0 : k0, p.a_mn ? k0 : m0);
 #pragma unroll
             for (int b = 0; b < C::b_boxes; ++b) {
               const int nb = n0 + b * 128;
-              tma_load<CG>(dst + (1 + b) * kTileBytes, &tmap_b, fb, p.b_mn ? nb : k0, p.b_mn ? k0 : nb);
+              tma_load<CG>(dst + (1 + b) * kTileBytes, &q.b, fb, p.b_mn ? nb : k0, p.b_mn ? k0 : nb);
             }
           }
           __syncwarp();
           if (++s == kStages) { s = 0; ph ^= 1u; }
         }
-      }
+       }
+      };
+      produce(one, walk1);
+      if constexpr (TWO) produce(two, walk2);
     } else if (warp == C::issuer_warp) {
       // ------------------------------ MMA issuer (first CTA) ----------------------------
       if (rank == 0) {
-        // D f32 (bit 4), A/B e4m3 (0), major bits 15/16, N>>3 at 17, M>>4 at 24
-        const uint32_t idesc = (1u << 4) | (uint32_t(p.a_mn) << 15) | (uint32_t(p.b_mn) << 16) | (uint32_t(BN >> 3) << 17) |
-                               (uint32_t(CG * BM >> 4) << 24);
-        const uint32_t a_step = p.a_mn ? (UMMA_K * 128) >> 4 : UMMA_K >> 4;
-        const uint32_t b_step = p.b_mn ? (UMMA_K * 128) >> 4 : UMMA_K >> 4;
         const uint64_t desc_a0 = make_smem_desc(sbase), desc_b0 = make_smem_desc(sbase + kTileBytes);
         const uint32_t desc_hi = uint32_t(desc_a0 >> 32);
         const uint32_t a_lo0 = uint32_t(desc_a0), b_lo0 = uint32_t(desc_b0);
-        uint32_t total = 0;
-        for (int item = first_item; item < n_items; item += item_step) {
-          int ks, tile;
-          item_split(p, item, n_tiles, ks, tile);
-          total += uint32_t(range_blocks(p, ks));
-        }
         bool ok = true;
         const bool stage_lane = lane >= 16;      // one wait instruction per block: half the lanes poll either barrier
         uint32_t s = 0, sph = 0, buf = 0, bph = 1, soff = 0;
-        for (uint32_t it = 0; ok && it < total; ++it) {
-          const uint32_t bar = stage_lane ? full0 + 8u * s : tempty0 + 8u * buf;
-          const uint32_t par = stage_lane ? sph : bph;
-          ok = __all_sync(0xffffffffu, mbar_wait(bar, par, abort_flag, p.status, stage_lane ? 3u : 2u));
-          if (!ok) break;
-          tc_fence_after();
-          if (elect_one()) {
-            const uint32_t d_tmem = tmem_base + buf * uint32_t(C::tmem_stride);
-#pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k)
-              umma<CG>(d_tmem, (uint64_t(desc_hi) << 32) | (a_lo0 + soff + k * a_step),
-                           (uint64_t(desc_hi) << 32) | (b_lo0 + soff + k * b_step), idesc, k > 0 ? 1u : 0u);
-            if constexpr (CG == 1) commit<CG>(empty0 + 8u * s);
-            commit<CG>(tfull0 + 8u * buf);
-            if constexpr (CG == 2) commit<CG>(empty0 + 8u * s);
+        auto issue = [&](const RingProblem& q, const Walk& w) {
+          const GemmParams& p = q.p;
+          // D f32 (bit 4), A/B e4m3 (0), major bits 15/16, N>>3 at 17, M>>4 at 24
+          const uint32_t idesc = (1u << 4) | (uint32_t(p.a_mn) << 15) | (uint32_t(p.b_mn) << 16) | (uint32_t(BN >> 3) << 17) |
+                                 (uint32_t(CG * BM >> 4) << 24);
+          const uint32_t a_step = p.a_mn ? (UMMA_K * 128) >> 4 : UMMA_K >> 4;
+          const uint32_t b_step = p.b_mn ? (UMMA_K * 128) >> 4 : UMMA_K >> 4;
+          uint32_t total = 0;
+          for (int k = 0, item; (item = walk_item(w, k)) >= 0; ++k) {
+            int ks, tile;
+            item_split(p, item, p.tiles_m * p.tiles_n, ks, tile);
+            total += uint32_t(range_blocks(p, ks));
           }
-          __syncwarp();
-          soff += uint32_t(C::stage_bytes >> 4);
-          if (++s == kStages) { s = 0; sph ^= 1u; soff = 0; }
-          if (++buf == kBufs) { buf = 0; bph ^= 1u; }
-        }
+          for (uint32_t it = 0; ok && it < total; ++it) {
+            const uint32_t bar = stage_lane ? full0 + 8u * s : tempty0 + 8u * buf;
+            const uint32_t par = stage_lane ? sph : bph;
+            ok = __all_sync(0xffffffffu, mbar_wait(bar, par, abort_flag, status, stage_lane ? 3u : 2u));
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
+              const uint32_t d_tmem = tmem_base + buf * uint32_t(C::tmem_stride);
+#pragma unroll
+              for (int k = 0; k < BK / UMMA_K; ++k)
+                umma<CG>(d_tmem, (uint64_t(desc_hi) << 32) | (a_lo0 + soff + k * a_step),
+                         (uint64_t(desc_hi) << 32) | (b_lo0 + soff + k * b_step), idesc, k > 0 ? 1u : 0u);
+              if constexpr (CG == 1) commit<CG>(empty0 + 8u * s);
+              commit<CG>(tfull0 + 8u * buf);
+              if constexpr (CG == 2) commit<CG>(empty0 + 8u * s);
+            }
+            __syncwarp();
+            soff += uint32_t(C::stage_bytes >> 4);
+            if (++s == kStages) { s = 0; sph ^= 1u; soff = 0; }
+            if (++buf == kBufs) { buf = 0; bph ^= 1u; }
+          }
+        };
+        issue(one, walk1);
+        if constexpr (TWO) issue(two, walk2);
         // nothing issued here may still be running when tensor memory is freed
         if (elect_one()) {
           if constexpr (CG == 2) umma_commit_here(drain_bar);
           else umma_commit(drain_bar);
-          mbar_wait(drain_bar, 0u, abort_flag, p.status, 4u);
+          mbar_wait(drain_bar, 0u, abort_flag, status, 4u);
         }
         __syncwarp();
       }
@@ -320,13 +358,16 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       bool ok = true;
       const uint32_t is_lane0 = lane == 0;
       auto announce = [&]() {
-        ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8u * buf, bph, abort_flag, p.status, 9u));
+        ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8u * buf, bph, abort_flag, status, 9u));
         mbar_arrive_if(tfull0 + 8u * buf, is_lane0);
         if (++buf == kBufs) { buf = 0; bph ^= 1u; }
       };
-      for (int item = first_item; ok && item < n_items; item += item_step) {
+      auto copy = [&](const RingProblem& q, const Walk& w, auto cfg) {
+       constexpr int SB_GRAN = decltype(cfg)::sb_gran;
+       const GemmParams& p = q.p;
+       for (int k = 0, item; ok && (item = walk_item(w, k)) >= 0; ++k) {
         int ks, tile, tm, tn;
-        item_split(p, item, n_tiles, ks, tile);
+        item_split(p, item, p.tiles_m * p.tiles_n, ks, tile);
         tile_coords(p, tile, tm, tn);
         const int m0 = (tm * CG + int(rank)) * BM, n0 = tn * BN;
         const uint32_t kb0 = uint32_t(range_first(p, ks));
@@ -343,10 +384,10 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const int nkb = range_blocks(p, ks);
         for (int kb = 0; kb < nkb; ++kb) {
           if (copied >= uint32_t(kStages)) {
-            ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8u * s, ph, abort_flag, p.status, 9u));
+            ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8u * s, ph, abort_flag, status, 9u));
             if (!ok) break;
           }
-          const uint32_t dst = sbase + C::off_ring + slot * uint32_t(C::slot_floats * 4) + 4u * lane;
+          const uint32_t dst = sbase + C::off_ring + slot * uint32_t(kSlot * 4) + 4u * lane;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             cp_async_4(dst + 128u * i, p.sa + sa_off[i]);
@@ -372,6 +413,9 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
         }
       }
+      };
+      copy(one, walk1, C());
+      if constexpr (TWO) copy(two, walk2, D());
       asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll 1
       for (uint32_t left = min(copied, uint32_t(kBufs)); ok && left > 0; --left) announce();
@@ -379,42 +423,48 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       // ------------------------------ tile stores ----------------------------------------
       uint32_t sph = 0;
       bool ok = true;
-      for (int item = first_item; ok && item + item_step < n_items; item += item_step) {      // (all but the last)
-        int ks, tile, tm, tn;
-        item_split(p, item, n_tiles, ks, tile);
-        tile_coords(p, tile, tm, tn);
+      auto store = [&](const RingProblem& q, const Walk& w, bool first, auto cfg) {
+        using Q = decltype(cfg);
+        const GemmParams& p = q.p;
+        for (int k = 0, item; ok && (item = walk_item(w, k)) >= 0 && followed(w, k, first); ++k) {       // (all but the last)
+          int ks, tile, tm, tn;
+          item_split(p, item, p.tiles_m * p.tiles_n, ks, tile);
+          tile_coords(p, tile, tm, tn);
 #pragma unroll 1
-        for (int phase = 0; phase < C::phases; ++phase) {
-          ok = __all_sync(0xffffffffu, mbar_wait(staged_bar, sph, abort_flag, p.status, 7u));
-          if (!ok) break;
-          sph ^= 1u;
-          if (elect_one()) {
+          for (int phase = 0; phase < Q::phases; ++phase) {
+            ok = __all_sync(0xffffffffu, mbar_wait(staged_bar, sph, abort_flag, status, 7u));
+            if (!ok) break;
+            sph ^= 1u;
+            if (elect_one()) {
 #pragma unroll 1
-            for (int w = 0; w < C::promo_warps; ++w) {
+              for (int pw = 0; pw < Q::promo_warps; ++pw) {
 #pragma unroll
-              for (int h = 0; h < C::warp_boxes; ++h)
-                tma_store_3d_nocommit(&tmap_d, sbase + C::off_out + uint32_t(w * C::warp_boxes + h) * C::box_bytes,
-                                      tn * BN + (w >> 2) * C::cols + (phase * C::warp_boxes + h) * C::box_cols,
-                                      (tm * CG + int(rank)) * BM + (w & 3) * 32, ks);
+                for (int h = 0; h < Q::warp_boxes; ++h)
+                  tma_store_3d_nocommit(&q.d, sbase + C::off_out + uint32_t(pw * Q::warp_boxes + h) * Q::box_bytes,
+                                        tn * BN + (pw >> 2) * Q::cols + (phase * Q::warp_boxes + h) * Q::box_cols,
+                                        (tm * CG + int(rank)) * BM + (pw & 3) * 32, ks);
+              }
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+              tma_store_wait_read();
+              mbar_arrive(unstaged_bar);
             }
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            tma_store_wait_read();
-            mbar_arrive(unstaged_bar);
+            __syncwarp();
           }
-          __syncwarp();
         }
-      }
+      };
+      store(one, walk1, true, C());
+      if constexpr (TWO) store(two, walk2, false, D());
     }
   } else {
     // ------------------------------ promotion + epilogue --------------------------------
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::promo_regs));
     const int quarter = warp & 3, cg = warp >> 2;
     const int r = quarter * 32 + lane;
-    constexpr bool kFrag = C::frag;
     const int fg = lane >> 2, fj = lane & 3;     // fragment coordinates: rows fg + 8 i, column pairs 8 k + 2 fj
     const float* ring = reinterpret_cast<const float*>(smem + C::off_ring);
     const uint32_t tcol0 = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(cg * C::cols);
     const int sb_index = cg * C::cols / 128;
+    static_assert(C::warp_boxes * C::box_bytes == D::warp_boxes * D::box_bytes, "one layout for both");
     const uint32_t wb = sbase + C::off_out + uint32_t(warp) * (C::warp_boxes * C::box_bytes);
     const uint32_t tempty_leader = CG == 2 ? map_rank(tempty0, 0u) : tempty0;
     const uint32_t is_lane0 = lane == 0;
@@ -427,7 +477,12 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       if constexpr (CG == 2) mbar_arrive_cluster_if(tempty_leader + 8u * b, is_lane0);
       else mbar_arrive_if(tempty_leader + 8u * b, is_lane0);
     };
-    for (int item = first_item; item < n_items; item += item_step) {
+    auto promote_items = [&](const RingProblem& prob, const Walk& w, bool first, auto cfg) {
+     using Q = decltype(cfg);
+     constexpr bool kFrag = Q::frag, OUT_F32 = Q::out_f32;
+     const GemmParams& p = prob.p;
+     const int n_tiles = p.tiles_m * p.tiles_n;
+     for (int walked = 0, item; (item = walk_item(w, walked)) >= 0; ++walked) {
       float2 acc[C::cols / 2];
 #pragma unroll
       for (int j = 0; j < C::cols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
@@ -439,28 +494,28 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       }
       // Rows in bf16: the last block stages each piece as soon as it is complete, beside the promotion of the next (forward and data
       // gradient 2 % faster at 8 and 16 blocks a tile; in fragments, whose stores are four bytes each, 0.5 % slower)
-      constexpr bool kStageInBlock = C::phases == 1 && !OUT_F32 && !kFrag;
+      constexpr bool kStageInBlock = Q::phases == 1 && !OUT_F32 && !kFrag;
       const int plain = kStageInBlock ? nkb - 1 : nkb;
-      const bool last = item + item_step >= n_items;
+      const bool last = !followed(w, walked, first);
       auto rows_free = [&]() {      // the staging rows have been read (the first pass finds them free)
-        ok &= mbar_wait(unstaged_bar, uph, abort_flag, p.status, 8u);
+        ok &= mbar_wait(unstaged_bar, uph, abort_flag, status, 8u);
         __syncwarp();
         uph ^= 1u;
       };
       // Piece q (of the phase, which begins with piece q0 of the accumulator).  Fragments: rows fg + 8 i; bf16: 16-byte chunk 2 q + k of the
       // box's row, 4 fj bytes in; float32: chunk 4 q + 2 k + (fj >> 1), half fj & 1.  Rows: chunks 2 q, 2 q + 1 (float32: 4 q ...).
       // Swizzle: chunk xor the row's low three bits, with 64-byte rows xor the two above the lowest.
-      const uint32_t st_base = wb + (kFrag ? uint32_t(fg) * C::box_row + (OUT_F32 ? (uint32_t(fj >> 1) << 4) + 8u * uint32_t(fj & 1) : 4u * uint32_t(fj))
+      const uint32_t st_base = wb + (kFrag ? uint32_t(fg) * Q::box_row + (OUT_F32 ? (uint32_t(fj >> 1) << 4) + 8u * uint32_t(fj & 1) : 4u * uint32_t(fj))
                                            : uint32_t(lane) * 128u);
-      const uint32_t st_flip = (!kFrag ? uint32_t(lane & 7) : C::box_row == 128 ? uint32_t(fg) : uint32_t(fg >> 1)) << 4;
+      const uint32_t st_flip = (!kFrag ? uint32_t(lane & 7) : Q::box_row == 128 ? uint32_t(fg) : uint32_t(fg >> 1)) << 4;
       auto stage = [&](auto qc, auto q0c) {
-        constexpr int qq = decltype(qc)::value, q0 = decltype(q0c)::value, q = qq % C::box_pieces, box = (qq / C::box_pieces) * C::box_bytes;
+        constexpr int qq = decltype(qc)::value, q0 = decltype(q0c)::value, q = qq % Q::box_pieces, box = (qq / Q::box_pieces) * Q::box_bytes;
         if constexpr (kFrag) {
           static_loop<4>([&](auto i) {
             static_loop<2>([&](auto k) {
               const float2 a = acc[(4 * (q0 + qq) + i.value) * 2 + k.value];
-              if constexpr (OUT_F32) sts_swz_f32x2<box + i.value * 8 * C::box_row + (4 * q + 2 * k.value) * 16>(st_base, st_flip, a);
-              else sts_swz_b32<box + i.value * 8 * C::box_row + (2 * q + k.value) * 16>(st_base, st_flip, pack_bf16x2(a.x, a.y));
+              if constexpr (OUT_F32) sts_swz_f32x2<box + i.value * 8 * Q::box_row + (4 * q + 2 * k.value) * 16>(st_base, st_flip, a);
+              else sts_swz_b32<box + i.value * 8 * Q::box_row + (2 * q + k.value) * 16>(st_base, st_flip, pack_bf16x2(a.x, a.y));
             });
           });
         } else if constexpr (OUT_F32) {
@@ -477,10 +532,10 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
       };
       auto enter_block = [&]() {
-        ok &= mbar_wait(tfull0 + 8u * buf, bph, abort_flag, p.status, 5u);
+        ok &= mbar_wait(tfull0 + 8u * buf, bph, abort_flag, status, 5u);
         __syncwarp();
         tc_fence_after();
-        const float* sc = ring + slot * C::slot_floats;
+        const float* sc = ring + slot * kSlot;
         if (++slot == kRing) slot = 0;
         return sc;
       };
@@ -571,7 +626,7 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       // ---- epilogue: registers -> this warp's swizzled staging rows -> bulk stores ----
       // The store warp hands a tile's boxes to the copy engine one after the other (40 cycles each), beside the next tile's first
       // blocks.  After the last tile nothing hides that: every warp issues its own.
-      static_loop<C::phases>([&](auto pc) {
+      static_loop<Q::phases>([&](auto pc) {
         constexpr int phase = decltype(pc)::value;
         if constexpr (!kStageInBlock) {
           if (!last || phase == 0) {
@@ -580,7 +635,7 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             if (is_lane0) tma_store_wait_read();
             __syncwarp();
           }
-          static_loop<C::warp_boxes * C::box_pieces>([&](auto qc) { stage(qc, IntC<phase * C::warp_boxes * C::box_pieces>{}); });
+          static_loop<Q::warp_boxes * Q::box_pieces>([&](auto qc) { stage(qc, IntC<phase * Q::warp_boxes * Q::box_pieces>{}); });
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the copy engine
         __syncwarp();
@@ -591,14 +646,19 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           item_split(p, item, n_tiles, ks, tile);
           tile_coords(p, tile, tm, tn);
 #pragma unroll
-          for (int h = 0; h < C::warp_boxes; ++h)
-            tma_store_3d_nocommit(&tmap_d, wb + uint32_t(h) * C::box_bytes, tn * BN + cg * C::cols + (phase * C::warp_boxes + h) * C::box_cols,
+          for (int h = 0; h < Q::warp_boxes; ++h)
+            tma_store_3d_nocommit(&prob.d, wb + uint32_t(h) * Q::box_bytes, tn * BN + cg * C::cols + (phase * Q::warp_boxes + h) * Q::box_cols,
                                   (tm * CG + int(rank)) * BM + quarter * 32, ks);
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
         __syncwarp();
       });
       if (!__all_sync(0xffffffffu, ok)) break;
+     }
+    };
+    promote_items(one, walk1, true, C());
+    if constexpr (TWO) {
+      if (__all_sync(0xffffffffu, ok)) promote_items(two, walk2, false, D());
     }
   }
 
@@ -619,55 +679,94 @@ gemm_ring_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   }
 }
 
+template <int CG, int BN, int SB_GRAN, bool OUT_F32>
+__global__ void __launch_bounds__((RingCfg<CG, BN, SB_GRAN, OUT_F32>::threads), 1) gemm_ring_kernel(const __grid_constant__ RingProblem one) {
+  using C = RingCfg<CG, BN, SB_GRAN, OUT_F32>;
+  ring_body<CG, C, C, false>(one, one, 0, [] {
+    grid_trigger();
+    grid_wait();
+  });
+}
+
+// A linear's weight gradient and then its data gradient on the same pairs, barriers and buffers running on from one to the other.  What
+// bounds the two apart is their last rounds: 5000 x 1024 -> 4096 has 64 tiles of 40 blocks and 80 of 32 for 74 pairs.  The long items go
+// first, and pairs that their last round leaves idle begin with the short ones.  With the quantisers, in a loop: 82 -> 67.5 us; 24576 x
+// 1024 -> 1024 101 -> 85 us, -> 3072 226 -> 208, 8192 x 2048 -> 2048 101 -> 97.
+template <bool OUT_F32>
+__global__ void __launch_bounds__((RingCfg<2, 256, 1, OUT_F32>::threads), 1)
+gemm_ring_two_kernel(const __grid_constant__ RingProblem one, const __grid_constant__ RingProblem two, int rounds) {
+  ring_body<2, RingCfg<2, 256, 1, OUT_F32>, RingCfg<2, 256, 128, false>, true>(one, two, rounds, [] {
+    grid_trigger();
+    grid_wait();
+  });
+}
+
 // ---- host ------------------------------------------------------------------------------
 
-template <int CG, int BN, int SB_GRAN, bool OUT_F32>
-static int launch_ring(const tg_gemm_args* a, GemmParams p, cudaStream_t st) {
-  using C = RingCfg<CG, BN, SB_GRAN, OUT_F32>;
-  auto kern = gemm_ring_kernel<CG, BN, SB_GRAN, OUT_F32>;
-  CUtensorMap ta, tb, td;
+template <int CG, typename C>
+static int prepare_ring(const tg_gemm_args* a, const GemmParams& p0, RingProblem& q) {
+  GemmParams& p = q.p;
+  p = p0;
   const int64_t a_inner = p.a_mn ? a->M : a->K, a_outer = p.a_mn ? a->K : a->M;
   const int64_t b_inner = p.b_mn ? a->N : a->K, b_outer = p.b_mn ? a->K : a->N;
-  if (int rc = make_tmap(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->a, a_inner, a_outer, a->lda, 128, 128)) return rc;
-  if (int rc = make_tmap(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->b, b_inner, b_outer, a->ldb, 128, 128)) return rc;
-  if (int rc = make_output_map(&td, OUT_F32, a, p, C::box_cols, C::box_row)) return rc;
+  if (int rc = make_tmap(&q.a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->a, a_inner, a_outer, a->lda, 128, 128)) return rc;
+  if (int rc = make_tmap(&q.b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->b, b_inner, b_outer, a->ldb, 128, 128)) return rc;
+  if (int rc = make_output_map(&q.d, C::out_f32, a, p, C::box_cols, C::box_row)) return rc;
   p.tiles_m = int((a->M + CG * BM - 1) / (CG * BM));
-  p.tiles_n = int((a->N + BN - 1) / BN);
+  p.tiles_n = int((a->N + C::BN - 1) / C::BN);
   p.band = std::min(p.tiles_m, kBandRows / CG);
-  if (int rc = set_reciprocals(p)) return rc;
-  const int n_items = p.tiles_m * p.tiles_n * p.ksplit;
-  int dev = 0;
-  TG_CUDA_CHECK(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return TG_ERR_SHAPE;
+  return set_reciprocals(p);
+}
+
+// The launch of one of the kernels above; `units_of`, per device: how many units run at a time (a pair takes two SMs of one cluster group).
+struct RingLaunch {
   cudaLaunchAttribute attrs[2];
-  attrs[0].id = cudaLaunchAttributeClusterDimension;
-  attrs[0].val.clusterDim.x = CG;
-  attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
-  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attrs[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(C::threads);
-  cfg.dynamicSmemBytes = C::smem_bytes;
-  cfg.attrs = attrs;
-  cfg.numAttrs = 1;
-  // once per device: the kernel's shared memory, and how many pairs run at a time (a pair takes two SMs of one cluster group)
-  static std::atomic<int> units_of[64];
-  int fit = units_of[dev].load(std::memory_order_acquire);
-  if (fit == 0) {
-    TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem_bytes));
-    fit = sm_count();
-    if (CG == 2) {
-      cfg.gridDim = dim3(unsigned(sm_count() & ~1));
-      TG_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&fit, kern, &cfg));
+  template <typename K>
+  int prepare(K kern, int cg, int threads, int smem, std::atomic<int>* units_of, int& units, cudaStream_t st) {
+    int dev = 0;
+    TG_CUDA_CHECK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return TG_ERR_SHAPE;
+    attrs[0].id = cudaLaunchAttributeClusterDimension;
+    attrs[0].val.clusterDim.x = cg;
+    attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
+    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = attrs;
+    cfg.numAttrs = 1;
+    cfg.stream = st;
+    int fit = units_of[dev].load(std::memory_order_acquire);      // with the kernel's shared memory: set once per device
+    if (fit == 0) {
+      TG_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      fit = sm_count();
+      if (cg == 2) {
+        cfg.gridDim = dim3(unsigned(sm_count() & ~1));
+        TG_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&fit, kern, &cfg));
+      }
+      if (fit < 1) return record_cuda_error(cudaErrorLaunchOutOfResources, "no CTA pair fits on this device");
+      units_of[dev].store(fit, std::memory_order_release);
     }
-    if (fit < 1) return record_cuda_error(cudaErrorLaunchOutOfResources, "no CTA pair fits on this device");
-    units_of[dev].store(fit, std::memory_order_release);
+    units = std::max(1, std::min(fit, gemm_sms() / cg));
+    return TG_OK;
   }
-  const int units = std::max(1, std::min(fit, gemm_sms() / CG));
-  cfg.gridDim = dim3(unsigned(CG * std::min(n_items, units)));
-  cfg.stream = st;
-  if ((p.a_mn == 0 && a->M <= 256) || (n_items <= 4 * units && p.nkb <= 32)) cfg.numAttrs = 2;
-  TG_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, ta, tb, td, p));
+};
+
+template <int CG, int BN, int SB_GRAN, bool OUT_F32>
+static int launch_ring(const tg_gemm_args* a, const GemmParams& p, cudaStream_t st) {
+  using C = RingCfg<CG, BN, SB_GRAN, OUT_F32>;
+  static std::atomic<int> units_of[64];
+  auto kern = gemm_ring_kernel<CG, BN, SB_GRAN, OUT_F32>;
+  RingProblem q;
+  RingLaunch l;
+  int units = 0;
+  if (int rc = prepare_ring<CG, C>(a, p, q)) return rc;
+  if (int rc = l.prepare(kern, CG, C::threads, C::smem_bytes, units_of, units, st)) return rc;
+  const int n_items = q.p.tiles_m * q.p.tiles_n * q.p.ksplit;
+  l.cfg.gridDim = dim3(unsigned(CG * std::min(n_items, units)));
+  if ((p.a_mn == 0 && a->M <= 256) || (n_items <= 4 * units && p.nkb <= 32)) l.cfg.numAttrs = 2;
+  TG_CUDA_CHECK(cudaLaunchKernelEx(&l.cfg, kern, q));
   return TG_OK;
 }
 
@@ -676,6 +775,31 @@ int ring_run(const tg_gemm_args* a, const GemmParams& p, bool pair, int bn, bool
   if (pair) return f32 ? launch_ring<2, 256, 128, true>(a, p, st) : launch_ring<2, 256, 128, false>(a, p, st);
   if (bn == 192) return launch_ring<1, 192, 1, false>(a, p, st);
   return f32 ? launch_ring<1, 128, 1, true>(a, p, st) : launch_ring<1, 128, 1, false>(a, p, st);
+}
+
+template <bool OUT_F32>
+static int launch_ring_two(const tg_gemm_args* a, const GemmParams& pa, const tg_gemm_args* b, const GemmParams& pb, cudaStream_t st) {
+  using C = RingCfg<2, 256, 1, OUT_F32>;
+  using D = RingCfg<2, 256, 128, false>;
+  static std::atomic<int> units_of[64];
+  auto kern = gemm_ring_two_kernel<OUT_F32>;
+  RingProblem one, two;
+  RingLaunch l;
+  int units = 0;
+  if (int rc = prepare_ring<2, C>(a, pa, one)) return rc;
+  if (int rc = prepare_ring<2, D>(b, pb, two)) return rc;
+  if (int rc = l.prepare(kern, 2, C::threads, std::max(C::smem_bytes, D::smem_bytes), units_of, units, st)) return rc;
+  const int n1 = one.p.tiles_m * one.p.tiles_n * one.p.ksplit, n2 = two.p.tiles_m * two.p.tiles_n;
+  units = std::min(units, n1 + n2);
+  l.cfg.gridDim = dim3(unsigned(2 * units));
+  int rounds = 0;
+  two_problems_us(n1, pair_item_us(true, pa.nkb + (pa.nkb_rem > 0)), n2, pair_item_us(false, pb.nkb), units, rounds);
+  TG_CUDA_CHECK(cudaLaunchKernelEx(&l.cfg, kern, one, two, rounds));
+  return TG_OK;
+}
+
+int ring_pair_two(const tg_gemm_args* a, const GemmParams& pa, bool f32, const tg_gemm_args* b, const GemmParams& pb, cudaStream_t st) {
+  return f32 ? launch_ring_two<true>(a, pa, b, pb, st) : launch_ring_two<false>(a, pa, b, pb, st);
 }
 
 }  // namespace tg

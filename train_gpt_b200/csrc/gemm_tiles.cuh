@@ -162,5 +162,28 @@ inline int set_reciprocals(GemmParams& p) {
 
 // The kernel of gemm_ring.cu: on pairs of SMs, or 128 x bn tiles with a scale per column.
 int ring_run(const tg_gemm_args* a, const GemmParams& p, bool pair, int bn, bool f32, cudaStream_t st);
+// Problem a (column scales; f32: cut into ranges, p.d the slices), then problem b (block scales, bf16, uncut), both on pairs in one launch.
+int ring_pair_two(const tg_gemm_args* a, const GemmParams& pa, bool f32, const tg_gemm_args* b, const GemmParams& pb, cudaStream_t st);
+
+// Microseconds of one 256 x 256 item of so many blocks on a pair, as the plans count them.
+inline double pair_item_us(bool columns, double blocks) { return (columns ? 0.54 : 0.42) * blocks + 0.86; }
+
+// Two problems of n1 items of t1 and n2 of t2 microseconds on `units` units: the units that the first one's last round leaves idle begin
+// with the second, for `rounds` rounds, and then all take what is left of it.  Returns the time of the best such order.
+inline double two_problems_us(int64_t n1, double t1, int64_t n2, double t2, int64_t units, int& rounds) {
+  const int64_t busy = n1 % units, idle = units - busy;
+  rounds = 0;
+  if (busy == 0) return double(n1 / units) * t1 + double((n2 + units - 1) / units) * t2;
+  double best = 0.0;
+  for (int e = 0; e <= int(t1 / t2) + 1; ++e) {
+    const int64_t rest = std::max<int64_t>(0, n2 - e * idle), each = rest / units, more = rest % units;
+    const double us = std::max(t1 + t2 * double(each + (more > idle)), t2 * double(e + each + (more > 0)));
+    if (e == 0 || us < best) {
+      best = us;
+      rounds = e;
+    }
+  }
+  return double(n1 / units) * t1 + best;
+}
 
 }  // namespace tg
