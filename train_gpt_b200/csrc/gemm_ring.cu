@@ -171,23 +171,19 @@ struct RingProblem {
   GemmParams p;
 };
 
-// The items of a problem that one unit (a CTA or a pair) works on, in order: `early` of them from `early_first` on in steps of
-// `early_step`, then from `first` on in steps of `step`, while they are below n.
+// The items of a problem that one unit (a CTA or a pair) works on: from `first` on in steps of `early_step` below early_end and of `step`
+// from there on, while they are below n.
 struct Walk {
-  int early, early_first, early_step, first, step, n;
+  int first, early_step, early_end, step, n;
+  __device__ __forceinline__ int next(int item) const { return item + (item < early_end ? early_step : step); }
 };
-__device__ __forceinline__ int walk_item(const Walk& w, int k) {
-  const int i = k < w.early ? w.early_first + k * w.early_step : w.first + (k - w.early) * w.step;
-  return i < w.n ? i : -1;
-}
+__device__ __forceinline__ Walk walk_alone(int unit, int units, int n) { return Walk{unit, 0, 0, units, n}; }
 // Two problems on the same units: the first one's items go round, and the units that its last round leaves idle take `rounds` rounds of the
-// second one's meanwhile, before all take it up.
-__device__ __forceinline__ Walk walk_alone(int unit, int units, int n) { return Walk{0, 0, 0, unit, units, n}; }
+// second one's meanwhile, before all take it up, the idle ones first.
 __device__ __forceinline__ Walk walk_second(int unit, int units, int n1, int n2, int rounds) {
-  const int busy = n1 % units, idle = units - busy;
+  const int busy = n1 % units, idle = units - busy, early_end = rounds * idle;
   if (busy == 0) return walk_alone(unit, units, n2);
-  const int place = unit >= busy ? unit - busy : unit + idle;         // the idle ones come first
-  return Walk{unit >= busy ? rounds : 0, place, idle, rounds * idle + place, units, n2};
+  return Walk{unit >= busy ? unit - busy : early_end + idle + unit, idle, early_end, units, n2};
 }
 
 // C and D: the plans of the two problems (TWO) or C twice.
@@ -219,8 +215,8 @@ __device__ __forceinline__ void ring_body(const RingProblem& one, const RingProb
   auto items_of = [](const GemmParams& p) { return p.tiles_m * p.tiles_n * p.ksplit; };
   const Walk walk1 = walk_alone(unit, units, items_of(one.p));
   const Walk walk2 = TWO ? walk_second(unit, units, items_of(one.p), items_of(two.p), rounds) : walk1;
-  // is there an item after the k-th of this problem?
-  auto followed = [&](const Walk& w, int k, bool first) { return walk_item(w, k + 1) >= 0 || (TWO && first && walk_item(walk2, 0) >= 0); };
+  // is there an item after this one?
+  auto followed = [&](const Walk& w, int item, bool first) { return w.next(item) < w.n || (TWO && first && walk2.first < walk2.n); };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -264,7 +260,7 @@ __device__ __forceinline__ void ring_body(const RingProblem& one, const RingProb
       const uint32_t full_leader = CG == 2 ? map_rank(full0, 0u) : full0;
       auto produce = [&](const RingProblem& q, const Walk& w) {
        const GemmParams& p = q.p;
-       for (int k = 0, item; ok && (item = walk_item(w, k)) >= 0; ++k) {
+       for (int item = w.first; ok && item < w.n; item = w.next(item)) {
         int ks, tile, tm, tn;
         item_split(p, item, p.tiles_m * p.tiles_n, ks, tile);
         tile_coords(p, tile, tm, tn);
@@ -310,7 +306,7 @@ __device__ __forceinline__ void ring_body(const RingProblem& one, const RingProb
           const uint32_t a_step = p.a_mn ? (UMMA_K * 128) >> 4 : UMMA_K >> 4;
           const uint32_t b_step = p.b_mn ? (UMMA_K * 128) >> 4 : UMMA_K >> 4;
           uint32_t total = 0;
-          for (int k = 0, item; (item = walk_item(w, k)) >= 0; ++k) {
+          for (int item = w.first; item < w.n; item = w.next(item)) {
             int ks, tile;
             item_split(p, item, p.tiles_m * p.tiles_n, ks, tile);
             total += uint32_t(range_blocks(p, ks));
@@ -365,7 +361,7 @@ __device__ __forceinline__ void ring_body(const RingProblem& one, const RingProb
       auto copy = [&](const RingProblem& q, const Walk& w, auto cfg) {
        constexpr int SB_GRAN = decltype(cfg)::sb_gran;
        const GemmParams& p = q.p;
-       for (int k = 0, item; ok && (item = walk_item(w, k)) >= 0; ++k) {
+       for (int item = w.first; ok && item < w.n; item = w.next(item)) {
         int ks, tile, tm, tn;
         item_split(p, item, p.tiles_m * p.tiles_n, ks, tile);
         tile_coords(p, tile, tm, tn);
@@ -426,7 +422,7 @@ __device__ __forceinline__ void ring_body(const RingProblem& one, const RingProb
       auto store = [&](const RingProblem& q, const Walk& w, bool first, auto cfg) {
         using Q = decltype(cfg);
         const GemmParams& p = q.p;
-        for (int k = 0, item; ok && (item = walk_item(w, k)) >= 0 && followed(w, k, first); ++k) {       // (all but the last)
+        for (int item = w.first; ok && item < w.n && followed(w, item, first); item = w.next(item)) {       // (all but the last)
           int ks, tile, tm, tn;
           item_split(p, item, p.tiles_m * p.tiles_n, ks, tile);
           tile_coords(p, tile, tm, tn);
@@ -482,7 +478,7 @@ __device__ __forceinline__ void ring_body(const RingProblem& one, const RingProb
      constexpr bool kFrag = Q::frag, OUT_F32 = Q::out_f32;
      const GemmParams& p = prob.p;
      const int n_tiles = p.tiles_m * p.tiles_n;
-     for (int walked = 0, item; (item = walk_item(w, walked)) >= 0; ++walked) {
+     for (int item = w.first; item < w.n; item = w.next(item)) {
       float2 acc[C::cols / 2];
 #pragma unroll
       for (int j = 0; j < C::cols / 2; ++j) acc[j] = make_float2(0.f, 0.f);
@@ -496,7 +492,7 @@ __device__ __forceinline__ void ring_body(const RingProblem& one, const RingProb
       // gradient 2 % faster at 8 and 16 blocks a tile; in fragments, whose stores are four bytes each, 0.5 % slower)
       constexpr bool kStageInBlock = Q::phases == 1 && !OUT_F32 && !kFrag;
       const int plain = kStageInBlock ? nkb - 1 : nkb;
-      const bool last = !followed(w, walked, first);
+      const bool last = !followed(w, item, first);
       auto rows_free = [&]() {      // the staging rows have been read (the first pass finds them free)
         ok &= mbar_wait(unstaged_bar, uph, abort_flag, status, 8u);
         __syncwarp();
