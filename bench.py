@@ -316,7 +316,7 @@ def main():
         elif tag not in missing:
             missing.append(tag)
     roofline = {
-        "bound": "tensor", "kernel": "gemm_fp8_blockscaled_kernel", "achieved": achieved, "peak": fp8_peak,
+        "bound": "tensor", "kernel": "gemm_ring_kernel", "achieved": achieved, "peak": fp8_peak,
         "unit": "TFLOP/s", "frac": achieved / fp8_peak,
         "traffic": None if (missing or not gemm_events) else traffic / len(gemm_events),
         "traffic_note": ("no ncu capture on record for " + str(missing)) if missing else
