@@ -260,6 +260,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmap_a, const CUten
         const uint32_t par = stage_lane ? sph : bph;
         ok = __all_sync(0xffffffffu, mbar_wait(bar, par, abort_flag, p.status, stage_lane ? 3u : 2u));
         if (!ok) break;
+        __syncwarp();                  // (the vote is no memory barrier, and the elected lane has seen one of the two only)
         tc_fence_after();
         if (elect_one()) {
           const uint32_t d_tmem = tmem_base + buf * uint32_t(C::tmem_stride);

@@ -316,6 +316,7 @@ __device__ __forceinline__ void ring_body(const RingProblem& one, const RingProb
             const uint32_t par = stage_lane ? sph : bph;
             ok = __all_sync(0xffffffffu, mbar_wait(bar, par, abort_flag, status, stage_lane ? 3u : 2u));
             if (!ok) break;
+            __syncwarp();                  // (the vote is no memory barrier, and the elected lane has seen one of the two only)
             tc_fence_after();
             if (elect_one()) {
               const uint32_t d_tmem = tmem_base + buf * uint32_t(C::tmem_stride);
@@ -355,6 +356,7 @@ __device__ __forceinline__ void ring_body(const RingProblem& one, const RingProb
       const uint32_t is_lane0 = lane == 0;
       auto announce = [&]() {
         ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8u * buf, bph, abort_flag, status, 9u));
+        __syncwarp();                // every lane's copies, before lane 0 announces them (a vote is no memory barrier)
         mbar_arrive_if(tfull0 + 8u * buf, is_lane0);
         if (++buf == kBufs) { buf = 0; bph ^= 1u; }
       };

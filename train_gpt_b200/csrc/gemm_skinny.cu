@@ -201,6 +201,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       const uint32_t bar = stage_lane ? full0 + 8u * s : tempty0 + 8u * buf;
       ok = __all_sync(0xffffffffu, mbar_wait(bar, stage_lane ? sph : bph, abort_flag, p.status, stage_lane ? 3u : 2u));
       if (!ok) break;
+      __syncwarp();                  // (the vote is no memory barrier, and the elected lane has seen one of the two only)
       tc_fence_after();
       if (elect_one()) {
         const uint32_t d_tmem = tmem_base + buf * uint32_t(BN_), soff = s * uint32_t(C::stage_bytes >> 4);
