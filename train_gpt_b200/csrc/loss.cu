@@ -544,7 +544,6 @@ __device__ __forceinline__ void tmem_wait_ld8(float2 (&v)[4]) {
 }
 
 __global__ void __launch_bounds__(kCgThreads * kCgGroups, 1) softcap_ce_groups_kernel(const CeArgs p, int smem_slots) {
-  grid_trigger();
   if (p.only_if_scaled) {
     grid_wait();
     if (*p.gscale == 1.0f) return;
@@ -571,6 +570,7 @@ __global__ void __launch_bounds__(kCgThreads * kCgGroups, 1) softcap_ce_groups_k
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_trigger();         // (not before the tensor memory is there: a kernel that started early could take it and wait for this one)
   grid_wait();            // (the table comes from the cap alone)
 
   // a warp reads and writes the lanes 32 (warp % 4).. of tensor memory; the four warps of a group that share them have 64 columns each
