@@ -181,6 +181,7 @@ int64_t tg_rmsnorm_bwd_scratch_bytes(int64_t rows, int64_t cols);
  * rnorm from x, returns dx = bf16(rnorm * (g*gamma - normed * mean(g*gamma*normed)))
  * and dgamma = bf16(sum_rows g * normed).
  *   x, g, dx [rows, cols] bf16; gamma, dgamma [cols] bf16; cols % 8 == 0, cols <= 8192
+ *   dgamma NULL: TG_ERR_SHAPE (in the two calls below as well)
  *   scratch: tg_rmsnorm_bwd_scratch_bytes(rows, cols) bytes, 16-byte aligned, contents
  *   undefined on entry and exit.  Deterministic (no atomics).                         */
 int tg_rmsnorm_bwd(const void* x, const void* gamma, const void* g, float eps, void* dx,

@@ -101,3 +101,13 @@ def test_nonzero_gemm_status_raises():
     loss = torch.tensor(2.5)
     assert float(ops.poison_if_failed(loss, ok)) == 2.5
     assert torch.isnan(ops.poison_if_failed(loss, torch.tensor([3], dtype=torch.int32)))
+
+
+@pytest.mark.parametrize("rows", [0, 8])
+def test_norm_backward_without_a_place_for_the_weight_gradient_is_refused(lib, rows):
+    """(aligned numbers stand for addresses: the refusal comes before anything is launched)"""
+    from train_gpt_b200._lib import TG_ERR_SHAPE
+    x, gamma, g, dx, scratch = (ctypes.c_void_p(4096 * i) for i in range(1, 6))
+    assert lib.tg_rmsnorm_bwd(x, gamma, g, 1e-6, dx, None, scratch, rows, 128, None) == TG_ERR_SHAPE
+    assert lib.tg_rmsnorm_bwd_add(x, gamma, g, x, 1e-6, dx, None, scratch, rows, 128, None) == TG_ERR_SHAPE
+    assert lib.tg_rmsnorm_bwd_static(x, gamma, g, 1e-6, dx, None, rows, 128, None) == TG_ERR_SHAPE

@@ -821,6 +821,7 @@ static int reduce_dgamma(const tgh_dgamma_job* jobs, int n, int blocks, int cols
   return TG_OK;
 }
 
+// (dgamma NULL: up to the partial sums; the public calls below refuse it)
 static int rmsnorm_bwd_impl(const void* x, const void* gamma, const void* g, const void* addend, float eps, void* dx,
                             void* dgamma, void* scratch, int64_t rows, int64_t cols, void* stream) {
   if (rows < 0 || cols <= 0 || cols % 8 != 0) return TG_ERR_SHAPE;
@@ -847,12 +848,13 @@ static int rmsnorm_bwd_impl(const void* x, const void* gamma, const void* g, con
 
 extern "C" int tg_rmsnorm_bwd(const void* x, const void* gamma, const void* g, float eps, void* dx,
                               void* dgamma, void* scratch, int64_t rows, int64_t cols, void* stream) {
+  if (dgamma == nullptr) return TG_ERR_SHAPE;
   return rmsnorm_bwd_impl(x, gamma, g, nullptr, eps, dx, dgamma, scratch, rows, cols, stream);
 }
 
 extern "C" int tg_rmsnorm_bwd_add(const void* x, const void* gamma, const void* g, const void* addend, float eps,
                                   void* dx, void* dgamma, void* scratch, int64_t rows, int64_t cols, void* stream) {
-  if (addend == nullptr) return TG_ERR_SHAPE;
+  if (addend == nullptr || dgamma == nullptr) return TG_ERR_SHAPE;
   return rmsnorm_bwd_impl(x, gamma, g, addend, eps, dx, dgamma, scratch, rows, cols, stream);
 }
 
@@ -891,7 +893,7 @@ extern "C" int tg_rmsnorm_bwd_static(const void* x, const void* gamma, const voi
   // In host code `g_bwd_scratch` is only a handle for the runtime, not an address a kernel
   // can use; the device address is looked up once per device, with that device current.
   static std::atomic<void*> dev_ptr[64] = {};   // written once per device; host threads may race to be first
-  if (rows < 0 || cols <= 0 || cols % 8 != 0) return TG_ERR_SHAPE;
+  if (rows < 0 || cols <= 0 || cols % 8 != 0 || dgamma == nullptr) return TG_ERR_SHAPE;
   const int64_t need = tg_rmsnorm_bwd_scratch_bytes(rows, cols);
   if (need > tg::kStaticBwdScratchBytes) {
     // message for tg_last_cuda_error(): the size limit is the caller's to handle
