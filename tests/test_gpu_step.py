@@ -306,6 +306,28 @@ def test_native_step_exchanges_every_bucket_once_it_is_complete(layers, defer):
             assert torch.equal(s, t)
 
 
+def test_native_step_reserves_the_norm_sums_it_uses():
+    """The partial sums of up to sixteen norms wait for one launch; where buckets are exchanged, each finishes the two that it holds, and
+    no more are reserved."""
+    from train_gpt_b200 import _lib
+    from train_gpt_b200.step import SMALL, StepConfig, Trainer, synthetic_batch
+    cfg = StepConfig(**{**SMALL, "n_layers": 9})
+    ids, tgt = synthetic_batch(cfg, 2, "cuda", seed=0)
+    peaks = []
+    for world in (1, 2):
+        tr = Trainer(cfg, torch.device("cuda", 0), world_size=world, seed=2)
+        tr.buckets._exchange = lambda bi: None
+        tr._program = tr._native_program()
+        tr.step(ids, tgt)
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        tr.step(ids, tgt)
+        peaks.append(torch.cuda.max_memory_allocated() - before)
+        del tr
+    sums = _lib.load().tg_rmsnorm_bwd_scratch_bytes(ids.numel(), cfg.d_model)
+    assert sums >= 1 << 12 and peaks[1] <= peaks[0] - 13 * sums, (peaks, sums)
+
+
 def test_native_step_reports_a_token_outside_the_vocabulary():
     """The native step's embedding kernel checks token ids itself: the loss is NaN and the status word says why.  Negative ids
     count from the end, as an index does."""

@@ -259,7 +259,8 @@ class StepProgram {
     Arena a;
     const FormAt row = add_row(a, m_, wide), col = add_col(a, m_, wide), third = add_col(a, m_, d_);
     norm_bytes_ = (std::max<int64_t>(api.tg_rmsnorm_bwd_scratch_bytes(m_, d_), 16) + 255) / 256 * 256;
-    norms_at_once_ = std::min<int64_t>(kNormsAtOnce, 2 * int64_t(layers_.size()) + 1);
+    // (where buckets are exchanged each finishes its own: the head's norm, or a layer's two)
+    norms_at_once_ = std::min<int64_t>(on_bucket_.is_none() ? kNormsAtOnce : 2, 2 * int64_t(layers_.size()) + 1);
     const size_t norm = a.add(norm_bytes_ * norms_at_once_), gemm = a.add(ws), table = a.add(vocab_ * 8);
     a.make(embed_);
     scratch_ = a.memory();
