@@ -69,3 +69,23 @@ def test_takes_the_faster_width(lib, what, tokens, k, n, columns, wide_us, narro
 def test_a_training_steps_contraction_ranges(lib, what, tokens, k, n, ranges):
     """The number of ranges shows in the last bit of a weight gradient, so it does not change for whole blocks of tokens."""
     assert _plan(lib, what, tokens, k, n, 0)[1] == ranges
+
+
+def test_pairs_leave_reserved_sms_room_wherever_their_blocks_lie(lib):
+    """A block of another kernel on one SM of a pair keeps the pair waiting until that kernel ends: with n SMs reserved a launch takes n pairs
+    fewer, and a problem that this leaves too few goes to single SMs."""
+    from train_gpt_b200 import _lib
+    args = _lib.GemmArgs(M=32768, N=6144, K=2048, lda=2048, ldb=6144, a_major=_lib.TG_MAJOR_K, b_major=_lib.TG_MAJOR_MN, sb_gran_n=128, ldd=6144)
+    kernel = ctypes.c_int()
+    before = lib.tg_set_gemm_reserved_sms(0)
+    try:
+        for reserved, on_pairs in ((0, True), (8, True), (64, False)):
+            lib.tg_set_gemm_reserved_sms(reserved)
+            assert lib.tgh_gemm_kernel(ctypes.byref(args), ctypes.byref(kernel)) == _lib.TG_OK
+            assert (kernel.value == 2) == on_pairs, reserved
+        lib.tg_set_gemm_reserved_sms(0)
+        all_pairs = lib.tgh_gemm_pairs()
+        lib.tg_set_gemm_reserved_sms(8)
+        assert lib.tgh_gemm_pairs() == all_pairs - 8
+    finally:
+        lib.tg_set_gemm_reserved_sms(before)

@@ -21,6 +21,9 @@ int check_arch();
 int sm_count();
 // SMs a persistent GEMM grid may occupy: sm_count() minus what tg_set_gemm_reserved_sms left for others.
 int gemm_sms();
+// Pairs of SMs (of one TPC) that it may occupy so that all run at a time: the blocks of the kernel that the SMs are reserved for may lie
+// anywhere, so that each can cost a pair.
+int gemm_pairs();
 
 #define TG_CUDA_CHECK(expr)                                        \
   do {                                                             \

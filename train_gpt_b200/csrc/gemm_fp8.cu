@@ -798,8 +798,9 @@ static GemmPlan plan_gemm(const tg_gemm_args* a) {
     if (wide == 128) break;
   }
   if (pl.S > 1) pl.bytes = int64_t(pl.S) * a->M * a->N * int64_t(sizeof(float));
-  if (a->M > 128 && a->N > 128) {
-    const int64_t pairs = std::max(1, sms / 2), items = ((a->M + 255) / 256) * ((a->N + 255) / 256) * pl.S, waves = (items + pairs - 1) / pairs;
+  const int64_t pairs = gemm_pairs();
+  if (pairs > 0 && a->M > 128 && a->N > 128) {
+    const int64_t items = ((a->M + 255) / 256) * ((a->N + 255) / 256) * pl.S, waves = (items + pairs - 1) / pairs;
     const double blocks = double((nkb + pl.S - 1) / pl.S);
     double us = 4.3 + double(waves) * pair_item_us(columns, blocks);
     if (pl.S > 1) us += 3.5 + double(4 * pl.S + 2) * double(a->M) * double(a->N) / 8.0e6;
@@ -953,7 +954,7 @@ static int two_tiles(const tg_gemm_args* a) {
 
 // Whether a problem passes all checks and could run in 256 x 256 tiles.
 static bool tiled(const tg_gemm_args* a) {
-  if (validate_gemm(a) != TG_OK || a->M <= 128 || a->N <= 128 || a->K == 0 || skinny_takes(a)) return false;
+  if (validate_gemm(a) != TG_OK || a->M <= 128 || a->N <= 128 || a->K == 0 || skinny_takes(a) || gemm_pairs() == 0) return false;
   return aligned16(a->a) && aligned16(a->b) && aligned16(a->d) && check_scales(a) == TG_OK;
 }
 
@@ -963,7 +964,7 @@ static double pairs_together_us(const tg_gemm_args* a, int S, const tg_gemm_args
   auto blocks = [](const tg_gemm_args* x, int n) { return double(((x->K + BK - 1) / BK + n - 1) / n); };
   int rounds = 0;
   double us = 4.3 + two_problems_us(tiles(a) * S, pair_item_us(true, blocks(a, S)), tiles(b), pair_item_us(false, blocks(b, 1)),
-                                    std::max(1, gemm_sms() / 2), rounds);
+                                    std::max(1, gemm_pairs()), rounds);
   if (S > 1) us += 3.5 + double(4 * S + 2) * double(a->M) * double(a->N) / 8.0e6;
   return us;
 }

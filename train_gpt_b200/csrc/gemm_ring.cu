@@ -746,7 +746,7 @@ struct RingLaunch {
       if (fit < 1) return record_cuda_error(cudaErrorLaunchOutOfResources, "no CTA pair fits on this device");
       units_of[dev].store(fit, std::memory_order_release);
     }
-    units = std::max(1, std::min(fit, gemm_sms() / cg));
+    units = std::max(1, std::min(fit, cg == 2 ? gemm_pairs() : gemm_sms()));
     return TG_OK;
   }
 };

@@ -32,6 +32,8 @@ int tgh_quantize_jobs(const tgh_quantize_job* jobs, int n, void* stream);
 int tgh_gemm_plan(const tg_gemm_args* args, int* tile_columns, int* ranges);
 /* Which tiled kernel a problem goes to: 0 gemm_fp8.cu, 1 gemm_ring.cu on single SMs, 2 the same on pairs of SMs.  Needs no GPU. */
 int tgh_gemm_kernel(const tg_gemm_args* args, int* kernel);
+/* Pairs of SMs that a launch on pairs uses at most. */
+int tgh_gemm_pairs(void);
 /* Two products that do not depend on one another (and do not share a workspace unless at most one of them uses it: a pair that runs
  * together uses none): in one launch where they are small, else one after the other. */
 int tgh_gemm_two(const tg_gemm_args* a, const tg_gemm_args* b, void* stream);

@@ -56,7 +56,14 @@ int gemm_sms() {
   return n < 1 ? 1 : n;
 }
 
+int gemm_pairs() {
+  const int n = sm_count() / 2 - g_reserved_sms.load(std::memory_order_relaxed);
+  return n < 0 ? 0 : n;
+}
+
 }  // namespace tg
+
+extern "C" int tgh_gemm_pairs(void) { return tg::gemm_pairs(); }
 
 extern "C" int tg_version(void) { return 101; }
 
