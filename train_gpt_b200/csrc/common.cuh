@@ -22,7 +22,8 @@ int sm_count();
 // SMs a persistent GEMM grid may occupy: sm_count() minus what tg_set_gemm_reserved_sms left for others.
 int gemm_sms();
 // Pairs of SMs (of one TPC) that it may occupy so that all run at a time: the blocks of the kernel that the SMs are reserved for may lie
-// anywhere, so that each can cost a pair.
+// anywhere, so that each can cost a pair.  32768 x 2048 -> 6144 with 8 SMs reserved and held by blocks that lay apart: 629 us with all 70 pairs
+// that are left, 371 with 66 (single SMs 387); where the blocks happened to fill whole TPCs 358 and 371.  16 held: 664 / 399 (408).
 int gemm_pairs();
 
 #define TG_CUDA_CHECK(expr)                                        \
