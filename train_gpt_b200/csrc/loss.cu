@@ -703,10 +703,11 @@ __global__ void __launch_bounds__(kCgThreads * kCgGroups, 1) softcap_ce_groups_k
       const int piece = at >> 3;
       const bool own = piece >= now.first && piece < now.last && (piece - now.first) % kCgThreads == tid;
       const uint32_t t_at = tanh_pair(x_at) & 0xffffu;
-      // ---- the gradient.  (g / sum first: the factors may be small, their product with g need not be.)
+      // ---- the gradient: g, 1 / sum and gscale / rows multiplied
       if (p.d != nullptr) {
         __nv_bfloat16* dp = p.d + (now.base - p.logits);
-        // g / sum * gs in one product where the factor is a normal number (its product with g then is what it should be), else in two
+        // by the product of the last two where that is a normal number, else by gscale / rows and then by 1 / sum: the factors may be small,
+        // their product with g need not be
         const float factor = __fmul_rn(inv, gs);
         const bool one_product = !(fabsf(factor) < 1.2e-38f);
         const float2 f2 = one_product ? make_float2(factor, factor) : make_float2(inv, inv);
