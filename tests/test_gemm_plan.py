@@ -89,3 +89,28 @@ def test_pairs_leave_reserved_sms_room_wherever_their_blocks_lie(lib):
         assert lib.tgh_gemm_pairs() == all_pairs - 8
     finally:
         lib.tg_set_gemm_reserved_sms(before)
+
+
+def _joint(lib, tokens, k, n, tile, mode):
+    """How a linear's backward pass runs its two products: tgh_gemm_two_plan's answer and rounds."""
+    from train_gpt_b200 import _lib
+    major, mn, columns, g_columns = _lib.TG_MAJOR_K, _lib.TG_MAJOR_MN, tile == (128, 1), mode == "fp8"
+    dgrad = _lib.GemmArgs(M=tokens, N=k, K=n, lda=n, ldb=n, a_major=major, b_major=major, sa_stride_m=n // 128, sa_stride_kb=1,
+                          sb_stride_n=n // 128, sb_stride_kb=1, sb_gran_n=1 if columns else 128, ldd=k)
+    wgrad = _lib.GemmArgs(M=k, N=n, K=tokens, lda=k, ldb=n, a_major=mn, b_major=mn, sa_stride_m=1, sa_stride_kb=k, sb_stride_n=1,
+                          sb_stride_kb=n if g_columns else n // 128, sb_gran_n=1 if g_columns else 128, ldd=n)
+    for args in (dgrad, wgrad):
+        args.workspace_bytes = lib.tg_gemm_workspace_bytes(ctypes.byref(args))
+        args.workspace = 4096 if args.workspace_bytes else None            # (never read here)
+    rounds = ctypes.c_int()
+    return lib.tgh_gemm_two_plan(ctypes.byref(dgrad), ctypes.byref(wgrad), ctypes.byref(rounds)), rounds.value
+
+
+def test_two_products_run_as_their_gpu_tests_say(lib):
+    """The sizes that test_gpu_gemm_two compares with two launches do take one, and the launch that they stand for."""
+    from test_gpu_gemm_two import APART, MODES, ON_PAIRS, ONE_WAVE, PAIRS_APART
+    for tile, mode in MODES:
+        assert {_joint(lib, *s, tile, mode) for s in ONE_WAVE} == {(1, 0)}
+        assert {_joint(lib, *s, tile, mode) for s in APART} == {(0, 0)}
+    assert [_joint(lib, *s[:3], (128, 128), "fp8") for s in ON_PAIRS] == [(2, s[3]) for s in ON_PAIRS]
+    assert {_joint(lib, *s, (128, 128), "fp8") for s in PAIRS_APART} == {(0, 0)}

@@ -5,18 +5,27 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# one tile each; ragged tokens; sizes that fit one wave together and sizes that do not (two launches); the modes' three kinds of scales
-@pytest.mark.parametrize("tokens,k,n", [(130, 128, 128), (1000, 384, 256), (1024, 512, 128), (700, 640, 768), (1024, 1152, 640), (1024, 128, 17920),
-                                        (1025, 1280, 640), (300, 128, 4096)])
-@pytest.mark.parametrize("tile,mode", [((128, 128), "fp8"), ((128, 1), "fp8"), ((128, 128), "fp8_blockgrad")])
+# one tile each; ragged tokens; sizes that fit one wave together and, at the end, sizes that do not (two launches); the modes' three kinds of scales
+ONE_WAVE = [(130, 128, 128), (1000, 384, 256), (1024, 512, 128), (700, 640, 768), (1024, 1152, 640), (1025, 1280, 640)]
+APART = [(1024, 128, 17920), (300, 128, 4096)]
+MODES = [((128, 128), "fp8"), ((128, 1), "fp8"), ((128, 128), "fp8_blockgrad")]
+
+
+@pytest.mark.parametrize("tokens,k,n", ONE_WAVE + APART)
+@pytest.mark.parametrize("tile,mode", MODES)
 def test_backward_has_the_bits_of_two_launches(tokens, k, n, tile, mode):
     _compare(tokens, k, n, tile, mode)
 
 
 # Both on pairs of SMs: a weight gradient cut in two, in three, uncut; several rounds of it, one, less than one; idle pairs that take all of
-# the data gradient's tiles, a round of them, or none; ragged tokens and columns (an odd number of 128-column blocks)
-@pytest.mark.parametrize("tokens,k,n", [(8192, 2048, 2048), (5000, 2048, 4224), (24576, 1024, 1024), (5000, 1024, 4096), (6145, 2048, 2176),
-                                        (24576, 1024, 3072), (2048, 2048, 2048), (700, 4096, 4096), (12000, 768, 3072), (4100, 640, 3200)])
+# the data gradient's tiles, a round of them, or none; ragged tokens and columns (an odd number of 128-column blocks).  With the rounds
+# of data-gradient tiles that idle pairs take first.  The others stay apart.
+ON_PAIRS = [(8192, 2048, 2048, 1), (5000, 2048, 4224, 0), (24576, 1024, 1024, 6), (5000, 1024, 4096, 0), (24576, 1024, 3072, 9), (2048, 2048, 2048, 0),
+            (700, 4096, 4096, 0), (12000, 768, 3072, 3), (4100, 640, 3200, 1)]
+PAIRS_APART = [(6145, 2048, 2176), (32768, 2048, 6144)]
+
+
+@pytest.mark.parametrize("tokens,k,n", [s[:3] for s in ON_PAIRS] + PAIRS_APART[:1])
 def test_backward_on_pairs_has_the_bits_of_two_launches(tokens, k, n):
     _compare(tokens, k, n, (128, 128), "fp8")
 

@@ -905,26 +905,10 @@ static int reduce_ranges(const tg_gemm_args* a, int S, cudaStream_t st) {
   return TG_OK;
 }
 
-extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
-  if (int rc = validate_gemm(a)) return rc;
-  if (a->M == 0 || a->N == 0) return TG_OK;
-  if (!aligned16(a->a) || !aligned16(a->b) || !aligned16(a->d)) return TG_ERR_ALIGN;
-  if (int rc = check_arch()) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const bool f32 = a->out_dtype == TG_OUT_F32;
-  if (a->K == 0) {
-    const size_t esz = f32 ? 4 : 2;
-    TG_CUDA_CHECK(cudaMemset2DAsync(a->d, size_t(a->ldd) * esz, 0, size_t(a->N) * esz, size_t(a->M), st));
-    return TG_OK;
-  }
-  if (int rc = check_scales(a)) return rc;
-  if (skinny_takes(a)) {
-    const int64_t need = skinny_workspace_bytes(a);
-    if (need == 0 || (a->workspace != nullptr && a->workspace_bytes >= need && aligned16(a->workspace))) return skinny_run(a, st);
-  }
+// A problem that passed all checks and is not the few-token kernel's, as planned.
+static int run_tiled(const tg_gemm_args* a, const GemmPlan& pl, cudaStream_t st) {
   GemmParams p = params_of(a);
-  const bool g1 = a->sb_gran_n == 1;
-  const GemmPlan pl = plan_gemm(a);
+  const bool g1 = a->sb_gran_n == 1, f32 = a->out_dtype == TG_OUT_F32;
   const int bn = pl.bn;
   if (cut_fits(a, pl)) {
     cut_params(a, pl.S, p);
@@ -943,30 +927,83 @@ extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
   return f32 ? launch_gemm<128, 128, true>(a, p, st) : launch_gemm<128, 128, false>(a, p, st);
 }
 
-// Whether a problem is uncut, of 128-column tiles in bf16 by this file's kernel, and in how many of them.
-static int two_tiles(const tg_gemm_args* a) {
-  if (validate_gemm(a) != TG_OK || a->M == 0 || a->N == 0 || a->K == 0 || a->out_dtype != TG_OUT_BF16 || skinny_takes(a)) return 0;
-  if (!aligned16(a->a) || !aligned16(a->b) || !aligned16(a->d) || check_scales(a) != TG_OK) return 0;
-  const GemmPlan pl = plan_gemm(a);
-  const int64_t tiles = ((a->M + 127) / 128) * ((a->N + 127) / 128);
-  return pl.pair || pl.ring || pl.bn != 128 || pl.S != 1 || tiles > INT32_MAX / 2 ? 0 : int(tiles);
+extern "C" int tg_gemm_fp8_blockscaled(const tg_gemm_args* a, void* stream) {
+  if (int rc = validate_gemm(a)) return rc;
+  if (a->M == 0 || a->N == 0) return TG_OK;
+  if (!aligned16(a->a) || !aligned16(a->b) || !aligned16(a->d)) return TG_ERR_ALIGN;
+  if (int rc = check_arch()) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (a->K == 0) {
+    const size_t esz = a->out_dtype == TG_OUT_F32 ? 4 : 2;
+    TG_CUDA_CHECK(cudaMemset2DAsync(a->d, size_t(a->ldd) * esz, 0, size_t(a->N) * esz, size_t(a->M), st));
+    return TG_OK;
+  }
+  if (int rc = check_scales(a)) return rc;
+  if (skinny_takes(a)) {
+    const int64_t need = skinny_workspace_bytes(a);
+    if (need == 0 || (a->workspace != nullptr && a->workspace_bytes >= need && aligned16(a->workspace))) return skinny_run(a, st);
+  }
+  return run_tiled(a, plan_gemm(a), st);
 }
 
-// Whether a problem passes all checks and could run in 256 x 256 tiles.
-static bool tiled(const tg_gemm_args* a) {
-  if (validate_gemm(a) != TG_OK || a->M <= 128 || a->N <= 128 || a->K == 0 || skinny_takes(a) || gemm_pairs() == 0) return false;
+// Whether a problem passes all checks of the public call and is a tiled kernel's.
+static bool ready(const tg_gemm_args* a) {
+  if (validate_gemm(a) != TG_OK || a->M == 0 || a->N == 0 || a->K == 0 || skinny_takes(a)) return false;
   return aligned16(a->a) && aligned16(a->b) && aligned16(a->d) && check_scales(a) == TG_OK;
 }
 
 // Modelled time of a (column scales) in S ranges and then b (block scales), both on pairs in one launch.
-static double pairs_together_us(const tg_gemm_args* a, int S, const tg_gemm_args* b) {
+static double pairs_together_us(const tg_gemm_args* a, int S, const tg_gemm_args* b, int& rounds) {
   auto tiles = [](const tg_gemm_args* x) { return ((x->M + 255) / 256) * ((x->N + 255) / 256); };
   auto blocks = [](const tg_gemm_args* x, int n) { return double(((x->K + BK - 1) / BK + n - 1) / n); };
-  int rounds = 0;
   double us = 4.3 + two_problems_us(tiles(a) * S, pair_item_us(true, blocks(a, S)), tiles(b), pair_item_us(false, blocks(b, 1)),
                                     std::max(1, gemm_pairs()), rounds);
   if (S > 1) us += 3.5 + double(4 * S + 2) * double(a->M) * double(a->N) / 8.0e6;
   return us;
+}
+
+// How two products run: each by itself (`planned`: as a and b say), in one wave of n1 + n2 tiles, or both on pairs.
+struct TwoPlan {
+  int joint;         // TGH_TWO_*
+  bool planned;
+  GemmPlan a, b;
+  int n1, n2;        // one wave: the tiles of a and of b
+  bool cut;          // on pairs: b in ranges
+  int rounds;        // on pairs: of a's items on the pairs that b's last round leaves idle
+};
+
+static TwoPlan plan_two(const tg_gemm_args* a, const tg_gemm_args* b) {
+  TwoPlan t = {};
+  t.joint = TGH_TWO_APART;
+  t.planned = ready(a) && ready(b);
+  if (!t.planned) return t;
+  t.a = plan_gemm(a);
+  t.b = plan_gemm(b);
+  // Together they are one wave, uncut, of 128-column tiles in bf16 by this file's kernel.  (One wave is also what an early launch asks for:
+  // gemm_fp8_blockscaled_kernel's rule.)
+  auto wave_tiles = [](const tg_gemm_args* x, const GemmPlan& pl) -> int64_t {
+    if (x->out_dtype != TG_OUT_BF16 || pl.pair || pl.ring || pl.bn != 128 || pl.S != 1 || (x->K + BK - 1) / BK > 32) return 0;
+    return ((x->M + 127) / 128) * ((x->N + 127) / 128);
+  };
+  const int64_t n1 = wave_tiles(a, t.a), n2 = wave_tiles(b, t.b);
+  if (n1 > 0 && n2 > 0 && n1 + n2 <= gemm_sms() && (a->sb_gran_n == 128 || b->sb_gran_n == 1)) {
+    t.joint = TGH_TWO_WAVE;
+    t.n1 = int(n1);
+    t.n2 = int(n2);
+    return t;
+  }
+  // Both on pairs of SMs, where one launch fills the last rounds (gemm_ring_two_kernel).  The modelled saving is 4 to 8 % too high (four
+  // linears of 32768 tokens: 6-8 % modelled, -0.1 to 3 % measured in short runs, -1 to 2 % at the power cap); from a twelfth on every
+  // measured pair of problems gained (2-17 %, 700 x 4096 -> 4096 54.1 / 47.2 us with the quantisers).  A data gradient with a scale per
+  // column stays apart: 12000 x 768 -> 3072 115 / 123 us, 4096 x 768 -> 3072 49.5 / 60, though 24576 x 1024 -> 1024 110 / 92.
+  // (a is uncut: the callers hand both the same workspace, which only b may use in a joint launch.)
+  auto wide = [](const tg_gemm_args* x) { return x->M > 128 && x->N > 128; };
+  if (a->sb_gran_n == 128 && b->sb_gran_n == 1 && a->out_dtype == TG_OUT_BF16 && wide(a) && wide(b) && gemm_pairs() > 0 && t.a.S == 1) {
+    t.cut = cut_fits(b, t.b);
+    if ((t.cut || b->out_dtype == TG_OUT_BF16) && pairs_together_us(b, t.cut ? t.b.S : 1, a, t.rounds) < (11.0 / 12.0) * (t.b.us + t.a.us))
+      t.joint = TGH_TWO_PAIRS;
+  }
+  return t;
 }
 
 template <int GRAN1, int GRAN2>
@@ -989,32 +1026,30 @@ static int launch_two(const tg_gemm_args* a, const tg_gemm_args* b, int n1, int 
   return TG_OK;
 }
 
+extern "C" int tgh_gemm_two_plan(const tg_gemm_args* a, const tg_gemm_args* b, int* rounds) {
+  const TwoPlan t = plan_two(a, b);
+  *rounds = t.joint == TGH_TWO_PAIRS ? t.rounds : 0;
+  return t.joint;
+}
+
 extern "C" int tgh_gemm_two(const tg_gemm_args* a, const tg_gemm_args* b, void* stream) {
-  // Together they are one wave.  (One wave is also what an early launch asks for: gemm_fp8_blockscaled_kernel's rule.)
-  const int n1 = two_tiles(a), n2 = two_tiles(b);
-  if (n1 > 0 && n2 > 0 && n1 + n2 <= gemm_sms() && (a->K + BK - 1) / BK <= 32 && (b->K + BK - 1) / BK <= 32) {
-    if (int rc = check_arch()) return rc;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (a->sb_gran_n == 128 && b->sb_gran_n == 1) return launch_two<128, 1>(a, b, n1, n2, st);
-    if (a->sb_gran_n == 1 && b->sb_gran_n == 1) return launch_two<1, 1>(a, b, n1, n2, st);
-    if (a->sb_gran_n == 128 && b->sb_gran_n == 128) return launch_two<128, 128>(a, b, n1, n2, st);
+  const TwoPlan t = plan_two(a, b);
+  if (!t.planned) {
+    if (int rc = tg_gemm_fp8_blockscaled(a, stream)) return rc;
+    return tg_gemm_fp8_blockscaled(b, stream);
   }
-  // Both on pairs of SMs, where one launch fills the last rounds (gemm_ring_two_kernel).  The modelled saving is 4 to 8 % too high (four
-  // linears of 32768 tokens: 6-8 % modelled, -0.1 to 3 % measured in short runs, -1 to 2 % at the power cap); from a twelfth on every
-  // measured pair of problems gained (2-17 %, 700 x 4096 -> 4096 54.1 / 47.2 us with the quantisers).  A data gradient with a scale per
-  // column stays apart: 12000 x 768 -> 3072 115 / 123 us, 4096 x 768 -> 3072 49.5 / 60, though 24576 x 1024 -> 1024 110 / 92.
-  if (a->sb_gran_n == 128 && b->sb_gran_n == 1 && a->out_dtype == TG_OUT_BF16 && tiled(a) && tiled(b)) {
-    const GemmPlan one = plan_gemm(b), two = plan_gemm(a);
-    const bool cut = cut_fits(b, one);
-    if (two.S == 1 && (cut || b->out_dtype == TG_OUT_BF16) && pairs_together_us(b, cut ? one.S : 1, a) < (11.0 / 12.0) * (one.us + two.us)) {
-      if (int rc = check_arch()) return rc;
-      cudaStream_t st = static_cast<cudaStream_t>(stream);
-      GemmParams p = params_of(b);
-      if (cut) cut_params(b, one.S, p);
-      if (int rc = ring_pair_two(b, p, cut, a, params_of(a), st)) return rc;
-      return cut ? reduce_ranges(b, one.S, st) : TG_OK;
-    }
+  if (int rc = check_arch()) return rc;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (t.joint == TGH_TWO_WAVE) {
+    if (a->sb_gran_n == 1) return launch_two<1, 1>(a, b, t.n1, t.n2, st);
+    return b->sb_gran_n == 1 ? launch_two<128, 1>(a, b, t.n1, t.n2, st) : launch_two<128, 128>(a, b, t.n1, t.n2, st);
   }
-  if (int rc = tg_gemm_fp8_blockscaled(a, stream)) return rc;
-  return tg_gemm_fp8_blockscaled(b, stream);
+  if (t.joint == TGH_TWO_PAIRS) {
+    GemmParams p = params_of(b);
+    if (t.cut) cut_params(b, t.b.S, p);
+    if (int rc = ring_pair_two(b, p, t.cut, a, params_of(a), st)) return rc;
+    return t.cut ? reduce_ranges(b, t.b.S, st) : TG_OK;
+  }
+  if (int rc = run_tiled(a, t.a, st)) return rc;
+  return run_tiled(b, t.b, st);
 }

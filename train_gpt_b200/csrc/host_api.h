@@ -34,9 +34,13 @@ int tgh_gemm_plan(const tg_gemm_args* args, int* tile_columns, int* ranges);
 int tgh_gemm_kernel(const tg_gemm_args* args, int* kernel);
 /* Pairs of SMs that a launch on pairs uses at most. */
 int tgh_gemm_pairs(void);
-/* Two products that do not depend on one another (and do not share a workspace unless at most one of them uses it: a pair that runs
- * together uses none): in one launch where they are small, else one after the other. */
+/* Two products that do not depend on one another: in one launch where that is faster, else a and then b.  They may share a workspace: what runs
+ * apart runs in stream order, and of a joint launch only b is ever cut. */
 int tgh_gemm_two(const tg_gemm_args* a, const tg_gemm_args* b, void* stream);
+/* How it runs them: apart, in one wave of 128-column tiles, or b and then a on pairs of SMs, with `rounds` rounds of a's items on the pairs
+ * that b's last round leaves idle.  Needs no GPU. */
+enum { TGH_TWO_APART = 0, TGH_TWO_WAVE = 1, TGH_TWO_PAIRS = 2 };
+int tgh_gemm_two_plan(const tg_gemm_args* a, const tg_gemm_args* b, int* rounds);
 
 /* tg_rmsnorm_bwd (addend NULL) or tg_rmsnorm_bwd_add up to the partial sums of the weight's gradient, tg_rmsnorm_bwd_scratch_bytes(rows, cols)
  * of them, and the weight gradients of any number of norms of one size from those. */
