@@ -6,15 +6,15 @@ import pytest
 
 # (what, tokens, K, N, scale per column, us with wide tiles, us with 128-column tiles)
 MEASURED = [
-    ("wgrad", 16, 8192, 8192, 0, 28.8, 31.7),
-    ("wgrad", 64, 8192, 8192, 0, 29.0, 31.9),
-    ("wgrad", 256, 8192, 8192, 0, 37.4, 42.0),
-    ("wgrad", 512, 8192, 8192, 0, 57.8, 62.9),
-    ("wgrad", 16, 2048, 8192, 0, 10.9, 12.3),
-    ("wgrad", 128, 4096, 4096, 0, 10.7, 10.8),
-    ("wgrad", 64, 1024, 4096, 0, 5.8, 4.8),
-    ("wgrad", 256, 2048, 2048, 0, 6.4, 5.3),
-    ("wgrad", 384, 3072, 3072, 0, 10.5, 9.5),
+    ("wgrad", 16, 8192, 8192, 1, 28.8, 31.7),
+    ("wgrad", 64, 8192, 8192, 1, 29.0, 31.9),
+    ("wgrad", 256, 8192, 8192, 1, 37.4, 42.0),
+    ("wgrad", 512, 8192, 8192, 1, 57.8, 62.9),
+    ("wgrad", 16, 2048, 8192, 1, 10.9, 12.3),
+    ("wgrad", 128, 4096, 4096, 1, 10.7, 10.8),
+    ("wgrad", 64, 1024, 4096, 1, 5.8, 4.8),
+    ("wgrad", 256, 2048, 2048, 1, 6.4, 5.3),
+    ("wgrad", 384, 3072, 3072, 1, 10.5, 9.5),
     ("fwd", 8192, 256, 8192, 0, 31.8, 38.5),
     ("fwd", 32768, 256, 1024, 0, 18.2, 21.4),
     ("fwd", 4096, 256, 4096, 0, 11.5, 12.5),
@@ -35,6 +35,30 @@ MEASURED = [
 ]
 
 
+# Single SMs or pairs, with either forced: (what, tokens, K, N, scale per column, us on single SMs, us on pairs).  The data gradients with a scale
+# per column have those apart in memory.  Contractions of one to 58 blocks, cut in up to eight ranges or not, half a wave of pairs and more.
+PAIRS_MEASURED = [
+    ("dgrad", 445, 4736, 3456, 1, 13.0, 21.0), ("dgrad", 269, 6144, 5888, 1, 23.1, 35.3), ("dgrad", 512, 2560, 2560, 1, 12.8, 16.1),
+    ("dgrad", 7567, 384, 5760, 1, 28.4, 34.5), ("dgrad", 4992, 1024, 3584, 1, 31.0, 38.4), ("dgrad", 12753, 512, 5888, 1, 63.1, 69.4),
+    ("dgrad", 738, 7680, 3712, 1, 32.9, 40.9), ("dgrad", 8035, 1280, 256, 1, 8.5, 10.2), ("dgrad", 21632, 384, 1664, 1, 22.6, 27.6),
+    ("dgrad", 14464, 640, 2048, 1, 27.2, 33.0), ("dgrad", 29316, 384, 5376, 1, 100.5, 117.0), ("dgrad", 12416, 1664, 128, 1, 12.3, 14.5),
+    ("dgrad", 310, 2688, 3200, 1, 13.2, 15.2), ("dgrad", 3328, 384, 3456, 1, 17.3, 18.8), ("dgrad", 1536, 3328, 1152, 1, 13.1, 15.3),
+    ("dgrad", 1920, 1920, 5248, 1, 66.9, 42.4), ("dgrad", 5760, 640, 6656, 1, 89.2, 49.8), ("dgrad", 2176, 3328, 7168, 1, 160.9, 100.2),
+    ("dgrad", 7168, 2560, 3712, 1, 97.4, 81.8), ("dgrad", 11779, 1536, 7424, 1, 195.1, 170.2), ("dgrad", 22016, 1280, 1280, 1, 53.9, 44.2),
+    ("dgrad", 169, 4224, 6272, 1, 23.6, 20.8), ("dgrad", 1922, 768, 5248, 1, 28.1, 23.9), ("dgrad", 738, 5248, 4992, 1, 34.7, 31.7),
+    ("dgrad", 24320, 5888, 256, 1, 78.4, 66.7), ("dgrad", 10439, 7552, 384, 1, 57.4, 48.0),
+    ("fwd", 26276, 128, 4608, 0, 51.6, 55.0), ("fwd", 8589, 256, 4992, 0, 23.6, 25.0), ("fwd", 7674, 768, 7936, 0, 57.3, 51.0),
+    ("fwd", 26775, 128, 768, 1, 12.3, 14.6), ("fwd", 9930, 128, 6144, 1, 27.4, 29.7), ("fwd", 20225, 768, 384, 1, 14.7, 16.5),
+    ("fwd", 11541, 768, 3328, 1, 48.2, 41.0), ("fwd", 15295, 896, 1408, 1, 33.4, 28.6), ("fwd", 3897, 896, 3456, 1, 19.9, 21.0),
+    ("dgrad", 20960, 896, 128, 0, 11.6, 14.1), ("dgrad", 5007, 7936, 256, 0, 22.3, 23.6), ("dgrad", 6193, 5248, 256, 0, 18.9, 20.3),
+    ("dgrad", 27860, 4096, 512, 0, 74.8, 67.2), ("dgrad", 10615, 896, 768, 0, 12.2, 13.1),
+    ("wgrad", 30720, 1408, 1664, 0, 95.2, 85.5), ("wgrad", 17716, 2688, 2944, 1, 200.2, 179.6), ("wgrad", 23680, 1920, 2304, 1, 150.9, 132.6),
+    ("wgrad", 6016, 2176, 2048, 1, 48.5, 42.0), ("wgrad", 24190, 384, 1152, 1, 21.7, 37.9), ("wgrad", 19455, 640, 1792, 1, 33.1, 48.4),
+    ("fwd", 303, 6016, 1408, 1, 12.6, 15.3), ("fwd", 2304, 7680, 896, 1, 29.6, 35.7), ("dgrad", 515, 2176, 8064, 0, 19.3, 29.7),
+    ("fwd", 1152, 5248, 1920, 0, 19.8, 29.8),
+]
+
+
 @pytest.fixture(scope="module")
 def lib():
     from train_gpt_b200 import build, _lib
@@ -42,15 +66,21 @@ def lib():
     return _lib.load()
 
 
-def _plan(lib, what, tokens, k, n, columns):
+def _args(what, tokens, k, n, columns):
+    """A linear's product as the library's callers lay it out."""
     from train_gpt_b200 import _lib
     major, mn = _lib.TG_MAJOR_K, _lib.TG_MAJOR_MN
     if what == "wgrad":
-        args = _lib.GemmArgs(M=k, N=n, K=tokens, lda=(k + 15) // 16 * 16, ldb=n, a_major=mn, b_major=mn, sb_gran_n=1, ldd=n)
-    elif what == "fwd":
-        args = _lib.GemmArgs(M=tokens, N=n, K=k, lda=k, ldb=n, a_major=major, b_major=mn, sb_gran_n=1 if columns else 128, ldd=n)
-    else:
-        args = _lib.GemmArgs(M=tokens, N=k, K=n, lda=n, ldb=n, a_major=major, b_major=major, sb_gran_n=1 if columns else 128, ldd=k)
+        return _lib.GemmArgs(M=k, N=n, K=tokens, lda=(k + 15) // 16 * 16, ldb=n, a_major=mn, b_major=mn, sb_gran_n=1 if columns else 128,
+                             sb_stride_n=1, ldd=n)
+    if what == "fwd":
+        return _lib.GemmArgs(M=tokens, N=n, K=k, lda=k, ldb=n, a_major=major, b_major=mn, sb_gran_n=1 if columns else 128, sb_stride_n=1, ldd=n)
+    return _lib.GemmArgs(M=tokens, N=k, K=n, lda=n, ldb=n, a_major=major, b_major=major, sb_gran_n=1 if columns else 128, sb_stride_n=n // 128, ldd=k)
+
+
+def _plan(lib, what, tokens, k, n, columns):
+    from train_gpt_b200 import _lib
+    args = _args(what, tokens, k, n, columns)
     width, ranges = ctypes.c_int(), ctypes.c_int()
     assert lib.tgh_gemm_plan(ctypes.byref(args), ctypes.byref(width), ctypes.byref(ranges)) == _lib.TG_OK
     return width.value, ranges.value
@@ -63,12 +93,19 @@ def test_takes_the_faster_width(lib, what, tokens, k, n, columns, wide_us, narro
     assert (narrow_us if width == 128 else wide_us) <= 1.04 * min(wide_us, narrow_us), width
 
 
+@pytest.mark.parametrize("what,tokens,k,n,columns,single_us,pair_us", PAIRS_MEASURED)
+def test_takes_the_faster_of_single_sms_and_pairs(lib, what, tokens, k, n, columns, single_us, pair_us):
+    kernel = ctypes.c_int()
+    assert lib.tgh_gemm_kernel(ctypes.byref(_args(what, tokens, k, n, columns)), ctypes.byref(kernel)) == 0
+    assert (pair_us if kernel.value == 2 else single_us) <= 1.04 * min(single_us, pair_us)
+
+
 @pytest.mark.parametrize("what,tokens,k,n,ranges", [("wgrad", 8192, 1024, 1024, 3), ("wgrad", 8192, 1024, 4096, 2), ("wgrad", 8192, 4096, 1024, 2),
                                                     ("wgrad", 8192, 1024, 3072, 1), ("wgrad", 32768, 1024, 1024, 3),
                                                     ("fwd", 8192, 1024, 4096, 1), ("dgrad", 1024, 128, 512, 1)])
 def test_a_training_steps_contraction_ranges(lib, what, tokens, k, n, ranges):
     """The number of ranges shows in the last bit of a weight gradient, so it does not change for whole blocks of tokens."""
-    assert _plan(lib, what, tokens, k, n, 0)[1] == ranges
+    assert _plan(lib, what, tokens, k, n, what == "wgrad")[1] == ranges
 
 
 def test_pairs_leave_reserved_sms_room_wherever_their_blocks_lie(lib):

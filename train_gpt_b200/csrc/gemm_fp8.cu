@@ -737,9 +737,12 @@ splitk_reduce_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, 
 // A pair of SMs with a 256 x 256 tile (gemm_ring.cu) moves a third less from the L2 per block and promotes with fewer instructions, but it
 // starts later and a wave of it is coarser.  Measured on 720 uncut problems of 130 to 32768 rows, in turn with the widths above: three
 // waves of pairs and more 1.04-1.12 times as fast with a scale per 128 columns, 1.05-1.4 with a scale per column (8192 x 2048 -> 8192 147
-// against 158 us and 176 against 230; weight gradient 2048 x 8192 of 8192 tokens 203 / 234), half a wave or less 0.66-0.76.  Where
-// column scales lie apart (the data gradient's, quantised along the other axis) the narrower kernels take half as long again per
-// block, once enough of them run at a time.  The rule takes the slower of the two by more than 2 % in none of the 720.
+// against 158 us and 176 against 230; weight gradient 2048 x 8192 of 8192 tokens 203 / 234), half a wave or less 0.66-0.76.  One
+// or two blocks are nothing to promote, and pairs lose there at any number of waves (20960 x 128 -> 896 11.6 / 14.1 us, 8192 x 256 -> 4992 23.6 / 25.0).
+// Cut problems, 150 of them: weight gradient 23680 x 1920 x 2304 in four ranges 151 / 133 us, forward 303 x 6016 -> 1408 in five 12.6 / 15.3.
+// Column scales that lie apart (apart_us), single SMs / pairs: 445 x 3456 -> 4736 13.0 / 21.0 us, 4992 x 3584 -> 1024 31.0 / 38.4, but cut in two
+// 2176 x 7168 -> 3328 161 / 100 (its kernel fetches each scale when it needs it, one sector for one number) and 22016 x 1280 -> 1280 53.9 / 44.2.  Of 550
+// problems, 330 of them such, the rule takes pairs where single SMs are more than 2 % faster in three (4 %).
 //
 // The tile width does not show in the result; the number of ranges does, in the last bit of float32 sums, and a training run
 // amplifies that over its steps.  So where the tokens are whole blocks of 128, as a training step's are, the number of
@@ -767,6 +770,17 @@ static int training_ranges(const tg_gemm_args* a, int wide) {
   return ranges;
 }
 
+// What a contraction block takes longer (or, in the ring, less long) than the figures of plan_gemm where the column scales of a block lie apart,
+// each in a sector with those of the same column's next blocks (the data gradient of a weight that was quantised along its columns): by the
+// number of blocks, that is, the distance between two columns' scales.
+static double apart_us(bool pair, int bn, bool cut, bool ring, int64_t nkb) {
+  const double far = double(std::max<int64_t>(nkb, 16) - 16);
+  if (pair) return std::min(0.005 * far, 0.16);
+  if (bn == 192 && cut) return std::min(std::max(0.04 * far - 0.32, 0.0), 0.6);
+  if (!ring) return 0.0;
+  return bn == 192 ? std::min(-0.04 + 0.004 * far, 0.11) : -0.04;
+}
+
 static GemmPlan plan_gemm(const tg_gemm_args* a) {
   const bool columns = a->sb_gran_n == 1;
   const int wide = a->N <= 128 ? 128 : columns ? 192 : 256;
@@ -775,7 +789,7 @@ static GemmPlan plan_gemm(const tg_gemm_args* a) {
   const int sms = gemm_sms();
   const bool whole = a->K % BK == 0 && (a->a_major == TG_MAJOR_MN || a->M % 128 == 0);      // (weight gradient: the tokens are K)
   const int fixed = whole ? training_ranges(a, wide) : 0;
-  double best = 0.0, best_blocks = 0.0;
+  double best = 0.0;
   for (const int bn : {wide, 128}) {
     const int64_t tiles = ((a->M + BM - 1) / BM) * ((a->N + bn - 1) / bn);
     for (int S = 1; S <= 8; ++S) {
@@ -790,7 +804,6 @@ static GemmPlan plan_gemm(const tg_gemm_args* a) {
       if (S > 1) us += 3.5 + double(4 * S + 2) * double(a->M) * double(a->N) / 8.0e6;
       if (best == 0.0 || us < best * 0.97) {
         best = us;
-        best_blocks = double(waves) * block * blocks;
         pl.bn = bn;
         pl.S = S;
       }
@@ -802,10 +815,14 @@ static GemmPlan plan_gemm(const tg_gemm_args* a) {
   if (pairs > 0 && a->M > 128 && a->N > 128) {
     const int64_t items = ((a->M + 255) / 256) * ((a->N + 255) / 256) * pl.S, waves = (items + pairs - 1) / pairs;
     const double blocks = double((nkb + pl.S - 1) / pl.S);
-    double us = 4.3 + double(waves) * pair_item_us(columns, blocks);
+    const bool apart = columns && a->sb_stride_n != 1;
+    double us = 4.3 + double(waves) * (pair_item_us(columns, blocks) + (apart ? apart_us(true, 256, false, true, nkb) * blocks : 0.0));
     if (pl.S > 1) us += 3.5 + double(4 * pl.S + 2) * double(a->M) * double(a->N) / 8.0e6;
-    if (columns && a->sb_stride_n != 1 && 2 * items > pairs) best += 0.5 * best_blocks;
-    pl.pair = us < best && (nkb >= 8 || waves >= 3);
+    if (apart) {
+      const int64_t tiles = ((a->M + BM - 1) / BM) * ((a->N + pl.bn - 1) / pl.bn) * pl.S;
+      best += double((tiles + sms - 1) / sms) * blocks * apart_us(false, pl.bn, pl.S > 1, blocks >= 12, nkb);
+    }
+    pl.pair = us < best && (nkb >= 8 || (waves >= 3 && nkb >= (apart ? 2 : 3)));
     if (pl.pair) pl.bn = 256;
     best = std::min(best, us);
   }
