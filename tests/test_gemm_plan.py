@@ -58,6 +58,15 @@ PAIRS_MEASURED = [
     ("fwd", 1152, 5248, 1920, 0, 19.8, 29.8),
 ]
 
+# The few-token kernel or the tiled ones: (tokens, K, N, scale per column, us of the few-token kernel, us of the tiled ones)
+FEW_MEASURED = [
+    (1, 2048, 256, 1, 5.0, 7.4), (16, 2560, 512, 0, 7.1, 8.1), (16, 3072, 512, 0, 7.3, 6.7), (16, 8192, 256, 0, 12.5, 7.5), (16, 16384, 512, 0, 9.0, 10.0),
+    (16, 32768, 256, 0, 12.2, 14.3), (32, 3584, 512, 0, 6.2, 7.4), (32, 512, 512, 0, 4.0, 3.8), (48, 1024, 4096, 0, 6.3, 5.7), (64, 2048, 512, 0, 5.8, 7.1),
+    (65, 2048, 2176, 0, 7.0, 7.8), (100, 1024, 4096, 0, 7.5, 5.8), (100, 1024, 4096, 1, 7.5, 6.2), (100, 4096, 4096, 0, 10.8, 10.1),
+    (100, 8192, 4096, 0, 14.4, 14.9), (100, 5504, 5120, 0, 13.2, 13.7), (128, 8192, 3072, 0, 13.1, 14.4), (128, 5504, 4096, 0, 12.6, 14.3),
+    (128, 4096, 6144, 0, 13.9, 13.5),
+]
+
 
 @pytest.fixture(scope="module")
 def lib():
@@ -91,6 +100,15 @@ def test_takes_the_faster_width(lib, what, tokens, k, n, columns, wide_us, narro
     width, ranges = _plan(lib, what, tokens, k, n, columns)
     assert width in (128, 192, 256) and ranges == 1
     assert (narrow_us if width == 128 else wide_us) <= 1.04 * min(wide_us, narrow_us), width
+
+
+@pytest.mark.parametrize("tokens,k,n,columns,few_us,tiled_us", FEW_MEASURED)
+def test_takes_the_few_token_kernel_where_it_is_faster(lib, tokens, k, n, columns, few_us, tiled_us):
+    from train_gpt_b200 import _lib
+    width, ranges = ctypes.c_int(), ctypes.c_int()
+    rc = lib.tgh_gemm_plan(ctypes.byref(_args("fwd", tokens, k, n, columns)), ctypes.byref(width), ctypes.byref(ranges))
+    assert rc in (_lib.TG_OK, _lib.TG_ERR_TOO_LARGE)
+    assert (tiled_us if rc == _lib.TG_OK else few_us) <= 1.03 * min(few_us, tiled_us)
 
 
 @pytest.mark.parametrize("what,tokens,k,n,columns,single_us,pair_us", PAIRS_MEASURED)

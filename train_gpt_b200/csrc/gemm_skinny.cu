@@ -28,14 +28,21 @@ namespace tg {
 // From 129 tokens on the tokens fill 128 MMA rows themselves, a token scale is a thread's own number instead of a column's,
 // and the tiled kernel is the faster one: 200 tokens, tiled / this kernel with 256 columns, a scale per 128 weight columns (per
 // column): 2048 x 8192 8.6 / 14.1 us (10.1 / 13.7), 4096 x 4096 12.0 / 16.2 (14.1 / 15.7), 8192 x 8192 25.0 / 40.4 (37.4 / 37.3).
-// Below, both sides with the weight from memory, this kernel / tiled (a scale per 128 weight columns; per column in brackets):
-//   100 tokens  512 x 512 5.4 / 4.0 (5.4 / 4.1), 1024 x 4096 7.5 / 5.8 (7.5 / 6.2), 2048 x 8192 9.7 / 8.3 (9.8 / 8.9), 4096 x 4096 10.8 / 10.1
-//               (10.9 / 11.0), 8192 x 8192 20.1 / 18.6 (20.3 / 21.6), 2048 x 2048 7.5 / 7.9 (7.6 / 8.4), 4096 x 1024 8.3 / 8.1 (8.3 / 9.1)
-//   48 tokens   512 x 512 4.8 / 3.9 (4.9 / 4.0), 640 x 7680 6.1 / 5.3 (6.1 / 5.6), 1024 x 1024 5.7 / 5.1 (5.8 / 5.4), 1024 x 4096 6.3 / 5.7
-//               (6.3 / 6.1), 2048 x 6144 7.9 / 8.0 (8.0 / 8.5), 4096 x 4096 8.9 / 9.1 (9.1 / 9.9), 8192 x 8192 15.9 / 17.6 (16.2 / 19.6)
-//   16 tokens   512 x 512 4.0 / 3.8 (4.1 / 3.9), 3072 x 512 7.9 / 6.7 (7.8 / 6.9), 1024 x 1024 4.7 / 5.0, 1024 x 4096 5.1 / 5.7, 8192 x 8192 13.4 / 16.9
-// So with more than 64 tokens and a scale per 128 columns the line is at the narrow weights, else at short contractions: the few-token
-// kernel's sums meet in a cluster or a second kernel, the tiled one's chain is then short.
+// Below, both sides with the weight from memory, this kernel / tiled, K x N, a scale per 128 weight columns unless said (with a scale per column
+// the tiled side takes up to a tenth longer, this one the same):
+//   1 to 32 tokens.  Weights of more than 512 columns stay here (16 tokens 1024 x 1024 4.7 / 5.0, 1024 x 4096 5.1 / 5.7, 8192 x 8192 13.4 / 16.9).
+//     Narrower ones are a few tiles, and the tiled kernel has them all in flight once it cuts the contraction three times or more, from K = 3072
+//     on: 16 x 2560 x 512 7.1 / 8.1, 3072 x 512 7.3 / 6.7, 4096 x 512 8.6 / 7.3, 8192 x 512 9.1 / 7.8, 8192 x 256 12.5 / 7.5; it makes eight ranges at most, so from
+//     4 M weights on it falls behind again: 12288 x 512 8.7 / 8.9, 16384 x 512 9.0 / 10.0, 32768 x 256 12.2 / 14.3.  One token against 2048 x 256 with a
+//     scale per column 5.0 / 7.4.  In between lies 32 x 3584 x 512 with 6.2 / 7.4.  512 x 512: 32 tokens 4.0 / 3.8, 8 tokens 3.6 / 3.7.
+//   33 to 64 tokens.  Short contractions are the tiled kernel's: 48 x 512 x 512 4.8 / 3.9, 640 x 7680 6.1 / 5.3, 1024 x 1024 5.7 / 5.1, 1024 x 4096 6.3 / 5.7; 2048 x 6144
+//     7.9 / 8.0, 8192 x 8192 15.9 / 17.6.  Narrow weights of long contractions stay here: 64 x 2048 x 512 5.8 / 7.1, though 48 x 4096 x 256 8.7 / 7.2.
+//   65 to 128 tokens.  With a scale per column only short contractions are tiled (100 x 1024 x 4096 7.5 / 6.2, 8192 x 8192 20.3 / 21.6, though 2048 x 8192
+//     9.8 / 8.9).  With one per 128 columns nearly all (100 x 1024 x 4096 7.5 / 5.8, 4096 x 4096 10.8 / 10.1, 8192 x 8192 20.1 / 18.6); not up to 2048 columns of
+//     1152 to 4608 (2048 x 2048 7.5 / 7.9), up to 2560 of about 2048 (65 x 2048 x 2176 7.0 / 7.8), nor 27 to 34 M weights (8192 x 4096 14.4 / 14.9, 5504 x
+//     5120 13.2 / 13.7), and with 128 tokens, whose contraction ranges are fixed, 20 to 34 M (8192 x 3072 13.1 / 14.4, 5504 x 4096 12.6 / 14.3; but 4096 x
+//     6144 13.9 / 13.5).
+// 1092 problems of these ranges: the kernel taken is more than 5 % slower than the other in 40 of them.
 constexpr int kSkinnyMaxTokens = 128;
 
 template <int BN_>
@@ -352,10 +359,17 @@ bool skinny_takes(const tg_gemm_args* a) {
       a->K > (1 << 22))
     return false;
   const bool columns = a->sb_gran_n == 1;
-  if (a->N <= 512 && (a->K <= 1024 || a->M <= 32)) return false;
-  if (a->M <= 32) return true;
+  const int64_t weights = a->K * a->N;
+  if (a->M <= 32) {
+    if (a->N > 512) return true;
+    if (a->K < 3072) return a->K > 512 || a->M <= 16;
+    return weights > 4 << 20 || (a->M > 20 && a->N > 448 && a->K > 3072 && a->K <= 4096);
+  }
+  if (a->N <= 512 && a->K <= 1024) return false;
   if (a->M <= 64) return a->K > (columns || a->N < 4096 ? 768 : 1024);
-  return a->K > 1024 && (columns || (a->N <= 2048 && a->K <= 4096));
+  if (a->K <= 1024 || columns) return a->K > 1024;
+  if (a->N <= 2048 ? a->K <= 4608 : a->N <= 2560 && a->K > 1536 && a->K < 3072) return true;
+  return weights > (a->M == 128 ? 19 << 20 : 26 << 20) && weights <= 32 << 20;
 }
 
 struct SkinnyPlan {
