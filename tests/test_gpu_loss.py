@@ -186,9 +186,13 @@ def test_loss_has_the_bits_of_the_mean_over_tokens(rows, vocab):
 
 
 # at the edges of the kernel that keeps a row's exponentials in tensor memory: just wide and large enough, one piece more than tensor memory
-# holds, the widest (and one column too wide), rows that start at every alignment; more rows than the GPU takes at a time
-@pytest.mark.parametrize("rows,vocab,cap", [(2200, 8193, 15.0), (560, 32769, 15.0), (549, 32775, 64.0), (340, 53247, 30.0), (339, 53249, 15.0),
-                                            (1500, 12301, 0.5)])
+# holds, the widest, rows that start at every alignment; more rows than the GPU takes at a time, a full last round and a short one.  The last four
+# are the other kernel's: a column too narrow and one too wide, rows too few, a last round too short.
+LARGE_RAGGED = [(2200, 8961, 15.0), (800, 32769, 15.0), (760, 32775, 64.0), (480, 53247, 30.0), (1500, 12301, 0.5), (1200, 33337, 15.0)]
+RAGGED = [(2200, 8959, 15.0), (480, 53249, 15.0), (440, 50257, 15.0), (620, 40001, 15.0)]
+
+
+@pytest.mark.parametrize("rows,vocab,cap", LARGE_RAGGED + RAGGED)
 def test_large_ragged_rows(rows, vocab, cap):
     from train_gpt_b200 import losses
     gen = torch.Generator("cuda").manual_seed(rows + vocab)
@@ -223,10 +227,10 @@ def test_large_ragged_rows(rows, vocab, cap):
 def test_large_ragged_rows_nan_and_small_scale():
     """A NaN spoils its own row alone; a scale whose product with 1 / sum is no normal number does not lose the gradient."""
     from train_gpt_b200 import losses
-    x = torch.randn(2000, 9001, device="cuda").mul(60).to(torch.bfloat16)
+    x = torch.randn(2100, 9001, device="cuda").mul(60).to(torch.bfloat16)
     x[7, 1234] = float("nan")
     x.requires_grad_(True)
-    t = torch.zeros(2000, dtype=torch.int64, device="cuda")
+    t = torch.zeros(2100, dtype=torch.int64, device="cuda")
     loss = losses.capped_cross_entropy(x, t, 64.0)
     loss.backward()
     assert bool(torch.isnan(loss)) and bool(torch.isnan(x.grad[7]).all()) and int(torch.isnan(x.grad).any(1).sum()) == 1

@@ -51,6 +51,8 @@ int tgh_dgamma_reduce(const tgh_dgamma_job* jobs, int n, int64_t rows, int64_t c
 
 /* Whether tgh_softcap_ce takes this problem (a row and its cap fit the one-pass kernel). */
 int tgh_softcap_ce_fits(float cap, int64_t rows, int64_t vocab);
+/* Whether it runs ragged rows (of 16-byte pieces) in groups of 512 threads with a row in tensor memory.  Needs no GPU. */
+int tgh_softcap_ce_in_groups(int64_t rows, int64_t vocab);
 /* Capped cross-entropy of each row AND the gradient of their mean from one read of the logits.
  *   logits    bf16 [rows, ld], row r starting at logits + r * ld (any alignment; the base 16-byte aligned)
  *   targets   int64 [rows], or int32 if !targets_64

@@ -515,13 +515,16 @@ __global__ void __launch_bounds__(WARP ? 256 : WHOLE ? kLossFwdThreads : kCeMaxT
 // The exponent's argument is z log2 e instead of (z - lse) log2 e: smaller, so its rounding costs the gradient less (the sum's order
 // and the last bits of the gradient are other ones than softcap_ce_kernel's).
 //
-// 8192 x 50257 406 -> 336 us (4.9 TB/s), 8192 x 25001 226 -> 179, 2048 x 50257 105 -> 93, 4096 x 9001 60 -> 51.  The rule: two rows per SM at a time
-// need rows to fill 296 of them, and the table's 64 KB are worth it from 18 M logits on (1024 x 9001 18.8 / 18.9 us, 512 x 25001 18.7 / 19.3,
-// 512 x 50257 32.2 / 31.0, 2048 x 9001 30.6 / 28.2); rows of up to 8192 columns leave too many of 512 threads without a piece in their last
-// pass (8192 x 4101 73.0 / 74.3, x 6001 77.1 / 79.1, x 5001 91.1 / 76.1).
+// 8192 x 50257 406 -> 336 us (4.9 TB/s), 8192 x 25001 226 -> 179, 2048 x 50257 105 -> 93, 4096 x 9001 60 -> 51.  The rule (softcap_ce_kernel / this one, with
+// a gradient; without one in brackets):
+//   columns   8201 leave a third pass nearly empty (3000 rows 39.4 / 40.8, 30.8 / 35.3), 9001 no longer (45.5 / 41.2, 35.6 / 35.6).
+//   rounds    two rows per SM at a time, 296 in all, and the table's 64 KB to begin with.  A last round of a few rows costs as much as a full one here,
+//             there a row alone on its SM is faster: 620 x 50257 38.8 / 42.5 (27.3 / 30.9), 920 x 25001 31.2 / 32.6 (22.6 / 25.6), 1248 x 20001 33.8 / 33.0 (25.2 / 26.8),
+//             1248 x 50257 68.5 / 67.7 (46.9 / 46.7), 1600 x 12301 33.2 / 31.0 (25.1 / 25.6).  So with six rounds and more, or five whose last is more than half
+//             full, from 18 M logits on; five with a shorter one from 40 M; fewer only with a last one more than half full and from 24 M
+//             (800 x 25001 27.5 / 26.9 (20.2 / 21.7), 592 x 50257 33.6 / 32.3 (24.0 / 23.6)).
 // ---------------------------------------------------------------------------------------
-constexpr int kCgMinCols = 8192;
-constexpr int64_t kCgMinLogits = 18'000'000;
+constexpr int kCgMinCols = 8960;
 constexpr int kCgThreads = 512, kCgGroups = 2;
 constexpr int kCgAhead = 4;                                  // pieces of a thread that are on their way to the L2
 constexpr int kCgTmemSlots = 8;                              // pieces of a thread in tensor memory
@@ -794,6 +797,15 @@ __global__ void __launch_bounds__(kMeanThreads) mean_kernel(const float* __restr
   }
 }
 
+// (`sms`: the row's rounds are counted for so many)
+static bool ce_in_groups(int64_t rows, int64_t vocab, int64_t sms) {
+  if (vocab < kCgMinCols || vocab > kCgMaxCols) return false;
+  const int64_t at_once = kCgGroups * sms, rounds = (rows + at_once - 1) / at_once, logits = rows * vocab;
+  const bool filled = 2 * (rows - (rounds - 1) * at_once) > at_once;
+  if (rounds >= 6 || (rounds == 5 && filled)) return logits >= 18'000'000;
+  return rounds == 5 ? logits >= 40'000'000 : filled && logits >= 24'000'000;
+}
+
 constexpr int kCeSmemMax = kCeSmemLimit;
 static int64_t ce_smem(int64_t vocab) {
   const int64_t row = (vocab + 14) / 8 * 16;
@@ -820,6 +832,8 @@ extern "C" int tgh_softcap_ce_fits(float cap, int64_t rows, int64_t vocab) {
   // the cap: exp(cap) and the table's exponents stay in range (see softcap_ce_kernel)
   return cap >= 0x1p-10f && cap <= 64.0f && rows <= INT32_MAX && vocab > 0 && vocab < (1 << 24) && ce_smem(vocab) <= kCeSmemMax;
 }
+
+extern "C" int tgh_softcap_ce_in_groups(int64_t rows, int64_t vocab) { return ce_in_groups(rows, vocab, sm_count()); }
 
 extern "C" int tgh_softcap_ce(const void* logits, const void* targets, int targets_64, float cap, void* dlogits, const float* gscale,
                               int only_if_scaled, float* nll, int64_t rows, int64_t vocab, int64_t ld, void* stream) {
@@ -853,7 +867,7 @@ extern "C" int tgh_softcap_ce(const void* logits, const void* targets, int targe
       const int64_t cap_blocks = int64_t(sm_count()) * std::min<int64_t>(per_sm_smem, 2);
       TG_CUDA_CHECK(launch_if_short(is_short, softcap_ce_kernel<false, true>, dim3(unsigned(std::min<int64_t>(rows, cap_blocks))), kLossFwdThreads,
                                     smem, st, a));
-    } else if (vocab > kCgMinCols && vocab <= kCgMaxCols && rows * vocab >= kCgMinLogits) {
+    } else if (ce_in_groups(rows, vocab, sm_count())) {
       const int slots = int(std::max<int64_t>(0, (vocab / 8 + kCgThreads - 1) / kCgThreads - kCgTmemSlots));
       const int blocks = int(std::min<int64_t>((rows + kCgGroups - 1) / kCgGroups, sm_count()));
       TG_CUDA_CHECK(launch_if_short(is_short, softcap_ce_groups_kernel, dim3(unsigned(blocks)), kCgThreads * kCgGroups,
