@@ -271,7 +271,7 @@ def test_every_split_of_a_row_over_warps(rows, cols, pure):
 
 # the largest tensors that take a block per row, and one row more, which takes warps: rows of one, two and four groups of pieces, a group
 # that is not full, the widest
-@pytest.mark.parametrize("rows,cols", [(1024, 1024), (2048, 1536), (1536, 2048), (910, 2304), (682, 3072), (409, 5120), (256, 8192), (291, 7168)])
+@pytest.mark.parametrize("rows,cols", [(1024, 1024), (2048, 1536), (1536, 2048), (910, 2304), (682, 3072), (444, 4608), (409, 5120), (256, 8192), (291, 7168), (296, 6144)])
 def test_block_per_row_has_the_bits_of_warps_per_row(rows, cols):
     from train_gpt_b200 import ops
     gen = torch.Generator("cuda").manual_seed(cols)

@@ -42,6 +42,9 @@ int tgh_gemm_two(const tg_gemm_args* a, const tg_gemm_args* b, void* stream);
 enum { TGH_TWO_APART = 0, TGH_TWO_WAVE = 1, TGH_TWO_PAIRS = 2 };
 int tgh_gemm_two_plan(const tg_gemm_args* a, const tg_gemm_args* b, int* rounds);
 
+/* Whether a norm's forward takes a thread block per row.  Needs no GPU. */
+int tgh_norm_few_rows(int64_t rows, int64_t cols);
+
 /* tg_rmsnorm_bwd (addend NULL) or tg_rmsnorm_bwd_add up to the partial sums of the weight's gradient, tg_rmsnorm_bwd_scratch_bytes(rows, cols)
  * of them, and the weight gradients of any number of norms of one size from those. */
 typedef struct { const void* partial; void* dgamma; } tgh_dgamma_job;

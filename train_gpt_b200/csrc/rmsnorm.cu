@@ -609,8 +609,13 @@ rmsnorm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 // Where the two meet (graph replays, microseconds with the quantiser, this kernel / the ones above): 1023 x 1024 3.0 / 3.8, 2047 x 1024 3.8 / 3.9
 // but without the quantiser 3.3 / 2.9; 1023 x 2048 3.8 / 5.2, 1447 x 2048 4.6 / 5.8, 2047 x 2048 5.9 / 6.0; 681 x 3072 3.6 / 4.3, 964 x 3072
 // 4.7 / 4.4; 511 x 4096 3.7 / 4.7, 723 x 4096 4.6 / 4.8 and 3.5 / 4.4; 255 x 8192 3.9 / 5.1, 361 x 8192 5.5 / 5.3; narrower rows fill warps of their own
-// (2895 x 512 4.0 / 3.0).
-static bool few_rows(int64_t rows, int64_t cols) { return rows * cols <= (cols < 1536 ? 1 << 20 : cols <= 2048 ? 3 << 20 : 1 << 21); }
+// (2895 x 512 4.0 / 3.0).  Beyond 4096 columns an SM holds three blocks or two, and a second round of them is the slower way: 444 x 4608 0.85 times as
+// long, 455 1.08; 296 x 6144 0.92, 341 x 6144 5.2 / 4.6.
+static bool few_rows(int64_t rows, int64_t cols) {
+  if (cols <= 4096) return rows * cols <= (cols < 1536 ? 1 << 20 : cols <= 2048 ? 3 << 20 : 1 << 21);
+  const int64_t threads = (cols / 8 + 31) / 32 * 32;
+  return rows <= 2048 / threads * sm_count() && rows * cols <= 1 << 21;
+}
 
 struct NormGeom {
   int nchunk, wpr;
@@ -870,6 +875,8 @@ extern "C" int tgh_rmsnorm_bwd_parts(const void* x, const void* gamma, const voi
                                      int64_t rows, int64_t cols, void* stream) {
   return rmsnorm_bwd_impl(x, gamma, g, addend, eps, dx, nullptr, partial, rows, cols, stream);
 }
+
+extern "C" int tgh_norm_few_rows(int64_t rows, int64_t cols) { return few_rows(rows, cols); }
 
 extern "C" int tgh_dgamma_reduce(const tgh_dgamma_job* jobs, int n, int64_t rows, int64_t cols, void* stream) {
   NormGeom g;
