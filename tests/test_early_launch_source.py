@@ -73,3 +73,37 @@ def test_no_load_takes_the_non_coherent_path():
         if f.endswith((".cu", ".cuh")):
             text = _strip(open(os.path.join(CSRC, f)).read())
             assert "ld.global.nc" not in text and "__ldg(" not in text, f
+
+
+def _bodies_with_start():
+    """(file, name, body) of the device functions whose kernels pass the trigger and the wait in as `start`."""
+    out = []
+    for f in sorted(os.listdir(CSRC)):
+        if not f.endswith((".cu", ".cuh")):
+            continue
+        text = _strip(open(os.path.join(CSRC, f)).read())
+        for m in re.finditer(r"__device__ __forceinline__ void (\w+)\(", text):
+            close_at = _balanced(text, m.end() - 1, "()")
+            if "START&&" in text[m.end():close_at]:
+                body_at = text.index("{", close_at)
+                out.append((f, m.group(1), text[body_at:_balanced(text, body_at, "{}") + 1]))
+    return out
+
+
+STARTED = _bodies_with_start()
+
+
+def test_finds_the_bodies_behind_the_kernels():
+    assert {b[1] for b in STARTED} == {"gemm_body", "ring_body"}
+    for f, name, _, body in KERNELS:            # and a kernel that hands its wait on does nothing else before it
+        if name in ("gemm_fp8_blockscaled_kernel", "gemm_two_kernel", "gemm_ring_kernel", "gemm_ring_two_kernel"):
+            assert re.search(r"\[\] \{\s*grid_trigger\(\);\s*grid_wait\(\);\s*\}", body), name
+
+
+@pytest.mark.parametrize("f,name,body", STARTED, ids=[b[1] for b in STARTED])
+def test_bodies_touch_no_memory_before_their_start(f, name, body):
+    """Scales, operands and results are read and written below `start()` only: no copy, no load through a pointer of the parameters."""
+    assert body.count("start();") == 1
+    before = body[:body.index("start();")]
+    for access in (r"tma_load", r"tma_store", r"cp_async", r"cp\.async", r"\bld_\w+\(", r"__ldc[gsav]\(", r"ld\.global", r"\.sa\b", r"\.sb\b", r"\.d\b", r"\bpromote"):
+        assert not re.search(access, before), (f, name, access)
