@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(kCgThreads * kCgGroups, 1) softcap_ce_groups_k
   float4* spill = reinterpret_cast<float4*>(s_cg + kTanhBytes) + group * smem_slots * (kCgSlotBytes / 16) + tid;
   const uint32_t tab = smem_u32(s_cg);
   const float gs = (p.gscale != nullptr ? *p.gscale : 1.0f) * (1.0f / float(p.rows));
-  const float2 l2e = make_float2(kLog2e, kLog2e), one = make_float2(1.f, 1.f), minus1 = make_float2(-1.f, -1.f), gs2 = make_float2(gs, gs);
+  const float2 l2e = make_float2(kLog2e, kLog2e), one = make_float2(1.f, 1.f), minus1 = make_float2(-1.f, -1.f);
   const __nv_bfloat162 c2 = __float2bfloat162_rn(sc.c);
   const int step = int(gridDim.x) * kCgGroups;
   int row = int(blockIdx.x) * kCgGroups + group;
@@ -709,23 +709,22 @@ __global__ void __launch_bounds__(kCgThreads * kCgGroups, 1) softcap_ce_groups_k
       // ---- the gradient: g, 1 / sum and gscale / rows multiplied
       if (p.d != nullptr) {
         __nv_bfloat16* dp = p.d + (now.base - p.logits);
-        // by the product of the last two where that is a normal number, else by gscale / rows and then by 1 / sum: the factors may be small,
-        // their product with g need not be
-        const float factor = __fmul_rn(inv, gs);
-        const bool one_product = !(fabsf(factor) < 1.2e-38f);
-        const float2 f2 = one_product ? make_float2(factor, factor) : make_float2(inv, inv);
+        // by the product of the last two.  Where that is no normal number (its product with g still may be one) gscale goes in 2^64 times as
+        // large and the result comes back by 2^-64, both exact: a gradient scaled by a power of two is the same gradient at any scale.
+        const bool direct = !(fabsf(__fmul_rn(inv, gs)) < 1.2e-38f);
+        const float factor = __fmul_rn(inv, direct ? gs : gs * 0x1p64f);
+        const float2 f2 = make_float2(factor, factor), down = make_float2(0x1p-64f, 0x1p-64f);
         auto second_pass = [&](float2 (&g)[4], int i) {
           uint4 o;
           uint32_t* op = &o.x;
-          if (!one_product) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) g[j] = __fmul2_rn(g[j], gs2);
+          for (int j = 0; j < 4; ++j) g[j] = __fmul2_rn(g[j], f2);
+          if (!direct) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) g[j] = __fmul2_rn(g[j], down);
           }
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 r = __fmul2_rn(g[j], f2);
-            op[j] = pack_bf16x2(r.x, r.y);
-          }
+          for (int j = 0; j < 4; ++j) op[j] = pack_bf16x2(g[j].x, g[j].y);
           if (i < now.last) *reinterpret_cast<uint4*>(dp + i * 8) = o;
         };
 #pragma unroll 2
