@@ -232,8 +232,9 @@ softcap_ce_bwd_kernel(const __nv_bfloat16* tanh_in, const int32_t* __restrict__ 
 // Ragged rows, which that kernel could only sum after a copy, skip the running maximum (|z| <= c <= 64: the sum neither
 // overflows nor loses its terms) and take as many threads as fill their last pass.
 //
-// One thread block per row (one warp for rows up to 2048 columns); a thread meets the same pieces in both passes,
-// so the only synchronisation is the reduction of the sum.
+// One thread block per row (one warp for rows up to 2048 columns); a thread meets the same pieces in both passes and has places of its own
+// for them, counted from the row's first whole piece, so the only synchronisation is the reduction of the sum.  (Counted from the row's first
+// boundary, a place changes hands where a ragged row is followed by an even one: a warp a row ahead overwrote what its neighbour was still to read.)
 // Bound by instruction issue and the ALU pipe (49 warp instructions per 64 logits, two of them ex2 in each pass), no longer by
 // memory.  8192 x 50257: 699 us for the two kernels, 2507 with the copies -> 415 us (DRAM floor 251); 8192 x 50304: 704 -> 462.
 // ---------------------------------------------------------------------------------------
@@ -379,7 +380,7 @@ __global__ void __launch_bounds__(WARP ? 256 : WHOLE ? kLossFwdThreads : kCeMaxT
         tp[j] = tanh_pair(wi[j], mag);
         z[j] = capped(tp[j]);
       }
-      if (!(WARP && WHOLE) || i < q.last) row_t[i] = to;
+      if (!(WARP && WHOLE) || i < q.last) row_t[i - q.first] = to;
       if constexpr (WHOLE) {
         if (!WARP || i < q.last) {
           const float mx = fmaxf(fmaxf(fmaxf(z[0].x, z[0].y), fmaxf(z[1].x, z[1].y)), fmaxf(fmaxf(z[2].x, z[2].y), fmaxf(z[3].x, z[3].y)));
@@ -410,7 +411,6 @@ __global__ void __launch_bounds__(WARP ? 256 : WHOLE ? kLossFwdThreads : kCeMaxT
         acc = __fadd2_rn(acc, __fadd2_rn(__fadd2_rn(e[0], e[1]), __fadd2_rn(e[2], e[3])));
       }
     }
-    const uint16_t* row_e = reinterpret_cast<const uint16_t*>(row_t);
     const int e_mine = WHOLE ? -1 : edge_of(q);
     uint32_t t_edge = 0u;
     if (!WHOLE && e_mine >= 0) {
@@ -466,11 +466,12 @@ __global__ void __launch_bounds__(WARP ? 256 : WHOLE ? kLossFwdThreads : kCeMaxT
     t = t < 0 ? 0 : (t >= p.vocab ? p.vocab - 1 : t);                 // clamped, as jnp.take_along_axis does
     const int at = int(t) + now.off, piece = at >> 3;                 // the target's place in the row's pieces
     const bool own = piece >= now.first && piece < now.last && (piece - now.first) % nt == tid;
+    const uint16_t* row_e = reinterpret_cast<const uint16_t*>(row_t - now.first);
     // ---- the gradient: gscale / rows * (exp(z - lse) - [target]) * (1 - t^2)
     if (p.d != nullptr) {
       __nv_bfloat16* dp = p.d + (now.base - p.logits);
       for (int i = now.first + tid; i < now.last; i += nt) {
-        const uint4 tw = row_t[i];
+        const uint4 tw = row_t[i - now.first];
         const uint32_t ti[4] = {tw.x, tw.y, tw.z, tw.w};
         uint4 o;
         uint32_t* op = &o.x;
