@@ -1,37 +1,37 @@
-"""The rule that picks the GEMM's tile width and contraction ranges, on the CPU, against times measured on a B200 with either width
-forced (microseconds of single launches in a graph): the width taken is at most 4 % slower than the other."""
+"""The rule that picks the GEMM's kernel, tile width and contraction ranges, on the CPU, against times measured on a B200 with each choice
+forced (microseconds of single launches in a graph): what is taken is at most 4 % slower than the fastest."""
 import ctypes
 
 import pytest
 
-# (what, tokens, K, N, scale per column, us with wide tiles, us with 128-column tiles)
+# (what, tokens, K, N, scale per column, us with wide tiles, us with 128-column tiles, us on pairs of SMs)
 MEASURED = [
-    ("wgrad", 16, 8192, 8192, 1, 28.8, 31.7),
-    ("wgrad", 64, 8192, 8192, 1, 29.0, 31.9),
-    ("wgrad", 256, 8192, 8192, 1, 37.4, 42.0),
-    ("wgrad", 512, 8192, 8192, 1, 57.8, 62.9),
-    ("wgrad", 16, 2048, 8192, 1, 10.9, 12.3),
-    ("wgrad", 128, 4096, 4096, 1, 10.7, 10.8),
-    ("wgrad", 64, 1024, 4096, 1, 5.8, 4.8),
-    ("wgrad", 256, 2048, 2048, 1, 6.4, 5.3),
-    ("wgrad", 384, 3072, 3072, 1, 10.5, 9.5),
-    ("fwd", 8192, 256, 8192, 0, 31.8, 38.5),
-    ("fwd", 32768, 256, 1024, 0, 18.2, 21.4),
-    ("fwd", 4096, 256, 4096, 0, 11.5, 12.5),
-    ("fwd", 32768, 128, 8192, 0, 107.1, 112.9),
-    ("fwd", 32768, 512, 4096, 0, 84.9, 106.4),
-    ("fwd", 4096, 128, 1024, 0, 4.9, 4.5),
-    ("fwd", 4096, 512, 1024, 0, 6.3, 6.2),
-    ("fwd", 200, 1024, 8192, 0, 7.5, 5.9),
-    ("fwd", 4096, 2048, 4096, 0, 33.4, 41.2),
-    ("fwd", 32768, 128, 8192, 1, 103.7, 116.9),
-    ("fwd", 8192, 256, 8192, 1, 37.6, 42.3),
-    ("fwd", 8192, 512, 8192, 1, 57.9, 62.9),
-    ("fwd", 4096, 512, 1024, 1, 8.7, 6.9),
-    ("fwd", 200, 2048, 8192, 1, 11.9, 9.8),
-    ("dgrad", 8192, 8192, 256, 0, 31.8, 38.6),
-    ("dgrad", 32768, 8192, 128, 1, 103.0, 117.0),
-    ("dgrad", 4096, 1024, 512, 1, 8.7, 6.9),
+    ("wgrad", 16, 8192, 8192, 1, 28.8, 31.7, 30.4),
+    ("wgrad", 64, 8192, 8192, 1, 29.0, 31.9, 30.7),
+    ("wgrad", 256, 8192, 8192, 1, 37.4, 42.0, 32.8),
+    ("wgrad", 512, 8192, 8192, 1, 57.8, 62.9, 47.7),
+    ("wgrad", 16, 2048, 8192, 1, 10.9, 12.3, 11.1),
+    ("wgrad", 128, 4096, 4096, 1, 10.7, 10.8, 11.1),
+    ("wgrad", 64, 1024, 4096, 1, 5.8, 4.8, 6.0),
+    ("wgrad", 256, 2048, 2048, 1, 6.4, 5.3, 6.6),
+    ("wgrad", 384, 3072, 3072, 1, 10.5, 9.5, 10.0),
+    ("fwd", 8192, 256, 8192, 0, 31.8, 38.5, 33.9),
+    ("fwd", 32768, 256, 1024, 0, 18.2, 21.4, 20.0),
+    ("fwd", 4096, 256, 4096, 0, 11.5, 12.5, 11.9),
+    ("fwd", 32768, 128, 8192, 0, 107.1, 112.9, 115.3),
+    ("fwd", 32768, 512, 4096, 0, 84.9, 106.4, 73.6),
+    ("fwd", 4096, 128, 1024, 0, 4.9, 4.5, 5.6),
+    ("fwd", 4096, 512, 1024, 0, 6.3, 6.2, 7.2),
+    ("fwd", 200, 1024, 8192, 0, 7.5, 5.9, 8.4),
+    ("fwd", 4096, 2048, 4096, 0, 33.4, 41.2, 33.1),
+    ("fwd", 32768, 128, 8192, 1, 103.7, 116.9, 107.6),
+    ("fwd", 8192, 256, 8192, 1, 37.6, 42.3, 32.9),
+    ("fwd", 8192, 512, 8192, 1, 57.9, 62.9, 47.3),
+    ("fwd", 4096, 512, 1024, 1, 8.7, 6.9, 7.9),
+    ("fwd", 200, 2048, 8192, 1, 11.9, 9.8, 14.0),
+    ("dgrad", 8192, 8192, 256, 0, 31.8, 38.6, 34.0),
+    ("dgrad", 32768, 8192, 128, 1, 103.0, 117.0, 107.5),
+    ("dgrad", 4096, 1024, 512, 1, 8.7, 6.9, 8.0),
 ]
 
 
@@ -54,6 +54,7 @@ PAIRS_MEASURED = [
     ("dgrad", 27860, 4096, 512, 0, 74.8, 67.2), ("dgrad", 10615, 896, 768, 0, 12.2, 13.1),
     ("wgrad", 30720, 1408, 1664, 0, 95.2, 85.5), ("wgrad", 17716, 2688, 2944, 1, 200.2, 179.6), ("wgrad", 23680, 1920, 2304, 1, 150.9, 132.6),
     ("wgrad", 6016, 2176, 2048, 1, 48.5, 42.0), ("wgrad", 24190, 384, 1152, 1, 21.7, 37.9), ("wgrad", 19455, 640, 1792, 1, 33.1, 48.4),
+    ("fwd", 8192, 128, 3072, 1, 13.6, 16.5), ("fwd", 8192, 256, 3072, 1, 16.4, 17.7), ("fwd", 8192, 256, 4096, 1, 21.8, 19.7), ("wgrad", 256, 4096, 4096, 1, 12.8, 12.1), ("wgrad", 256, 3584, 5632, 1, 14.6, 15.8), ("wgrad", 384, 5120, 5120, 1, 23.3, 20.2),
     ("fwd", 303, 6016, 1408, 1, 12.6, 15.3), ("fwd", 2304, 7680, 896, 1, 29.6, 35.7), ("dgrad", 515, 2176, 8064, 0, 19.3, 29.7),
     ("fwd", 1152, 5248, 1920, 0, 19.8, 29.8),
 ]
@@ -95,11 +96,18 @@ def _plan(lib, what, tokens, k, n, columns):
     return width.value, ranges.value
 
 
-@pytest.mark.parametrize("what,tokens,k,n,columns,wide_us,narrow_us", MEASURED)
-def test_takes_the_faster_width(lib, what, tokens, k, n, columns, wide_us, narrow_us):
+def _kernel(lib, what, tokens, k, n, columns):
+    kernel = ctypes.c_int()
+    assert lib.tgh_gemm_kernel(ctypes.byref(_args(what, tokens, k, n, columns)), ctypes.byref(kernel)) == 0
+    return kernel.value
+
+
+@pytest.mark.parametrize("what,tokens,k,n,columns,wide_us,narrow_us,pair_us", MEASURED)
+def test_takes_the_faster_width(lib, what, tokens, k, n, columns, wide_us, narrow_us, pair_us):
     width, ranges = _plan(lib, what, tokens, k, n, columns)
     assert width in (128, 192, 256) and ranges == 1
-    assert (narrow_us if width == 128 else wide_us) <= 1.04 * min(wide_us, narrow_us), width
+    on_pairs = _kernel(lib, what, tokens, k, n, columns) == 2
+    assert (pair_us if on_pairs else narrow_us if width == 128 else wide_us) <= 1.04 * min(wide_us, narrow_us, pair_us), (width, on_pairs)
 
 
 @pytest.mark.parametrize("tokens,k,n,columns,few_us,tiled_us", FEW_MEASURED)
@@ -113,9 +121,7 @@ def test_takes_the_few_token_kernel_where_it_is_faster(lib, tokens, k, n, column
 
 @pytest.mark.parametrize("what,tokens,k,n,columns,single_us,pair_us", PAIRS_MEASURED)
 def test_takes_the_faster_of_single_sms_and_pairs(lib, what, tokens, k, n, columns, single_us, pair_us):
-    kernel = ctypes.c_int()
-    assert lib.tgh_gemm_kernel(ctypes.byref(_args(what, tokens, k, n, columns)), ctypes.byref(kernel)) == 0
-    assert (pair_us if kernel.value == 2 else single_us) <= 1.04 * min(single_us, pair_us)
+    assert (pair_us if _kernel(lib, what, tokens, k, n, columns) == 2 else single_us) <= 1.04 * min(single_us, pair_us)
 
 
 @pytest.mark.parametrize("what,tokens,k,n,ranges", [("wgrad", 8192, 1024, 1024, 3), ("wgrad", 8192, 1024, 4096, 2), ("wgrad", 8192, 4096, 1024, 2),

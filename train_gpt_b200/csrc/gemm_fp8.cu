@@ -737,13 +737,14 @@ splitk_reduce_kernel(const float* __restrict__ ws, void* __restrict__ d, int M, 
 // A pair of SMs with a 256 x 256 tile (gemm_ring.cu) moves a third less from the L2 per block and promotes with fewer instructions, but it
 // starts later and a wave of it is coarser.  Measured on 720 uncut problems of 130 to 32768 rows, in turn with the widths above: three
 // waves of pairs and more 1.04-1.12 times as fast with a scale per 128 columns, 1.05-1.4 with a scale per column (8192 x 2048 -> 8192 147
-// against 158 us and 176 against 230; weight gradient 2048 x 8192 of 8192 tokens 203 / 234), half a wave or less 0.66-0.76.  One
-// or two blocks are nothing to promote, and pairs lose there (20960 x 128 -> 896 11.6 / 14.1 us, 8589 x 256 -> 4992 23.6 / 25.0) but
-// for one block in a few waves of 256-column tiles, where the two are within 2 % (17246 x 128 -> 896 10.8 / 10.9).
-// Cut problems, 150 of them: weight gradient 23680 x 1920 x 2304 in four ranges 151 / 133 us, forward 303 x 6016 -> 1408 in five 12.6 / 15.3.
+// against 158 us and 176 against 230; weight gradient 2048 x 8192 of 8192 tokens 203 / 234), half a wave or less 0.66-0.76.  A
+// contraction of one block is nothing to promote, and pairs lose there (20960 x 128 -> 896 11.6 / 14.1 us, with column scales 8192 x 128 -> 3072 13.6 / 16.5) but for
+// a few waves of 256-column tiles with a scale per 128, where the two are within 2 % (17246 x 128 -> 896 10.8 / 10.9).  Two blocks: with a scale per
+// 128 columns 8589 x 256 -> 4992 23.6 / 25.0; per column it depends on the last wave, as an item takes 2.1 us for its stores (8192 x 256 -> 3072 16.4 / 17.7, -> 4096
+// 21.8 / 19.7).  Cut problems, 150 of them: weight gradient 23680 x 1920 x 2304 in four ranges 151 / 133 us, forward 303 x 6016 -> 1408 in five 12.6 / 15.3.
 // Column scales that lie apart (apart_us), single SMs / pairs: 445 x 3456 -> 4736 13.0 / 21.0 us, 4992 x 3584 -> 1024 31.0 / 38.4, but cut in two
-// 2176 x 7168 -> 3328 161 / 100 (its kernel fetches each scale when it needs it, one sector for one number) and 22016 x 1280 -> 1280 53.9 / 44.2.  Of 550
-// problems, 330 of them such, the rule takes pairs where single SMs are more than 2 % faster in three (4 %).
+// 2176 x 7168 -> 3328 161 / 100 (its kernel fetches each scale when it needs it, one sector for one number) and 22016 x 1280 -> 1280 53.9 / 44.2.  Of 1100
+// problems, 660 of them such, the rule takes pairs where single SMs are more than 2 % faster in five (at most 6 %).
 //
 // The tile width does not show in the result; the number of ranges does, in the last bit of float32 sums, and a training run
 // amplifies that over its steps.  So where the tokens are whole blocks of 128, as a training step's are, the number of
@@ -817,14 +818,15 @@ static GemmPlan plan_gemm(const tg_gemm_args* a) {
     const int64_t items = ((a->M + 255) / 256) * ((a->N + 255) / 256) * pl.S, waves = (items + pairs - 1) / pairs;
     const double blocks = double((nkb + pl.S - 1) / pl.S);
     const bool apart = columns && a->sb_stride_n != 1;
-    double us = 4.3 + double(waves) * (pair_item_us(columns, blocks) + (apart ? apart_us(true, 256, false, true, nkb) * blocks : 0.0));
+    const double item = pair_item_us(columns, blocks) + (apart ? apart_us(true, 256, false, true, nkb) * blocks : 0.0);
+    double us = 4.3 + double(waves) * (columns ? std::max(item, 2.08) : item);        // (two blocks: the stores)
     if (pl.S > 1) us += 3.5 + double(4 * pl.S + 2) * double(a->M) * double(a->N) / 8.0e6;
     if (apart) {
       const int64_t tiles = ((a->M + BM - 1) / BM) * ((a->N + pl.bn - 1) / pl.bn) * pl.S;
       best += double((tiles + sms - 1) / sms) * blocks * apart_us(false, pl.bn, pl.S > 1, blocks >= 12, nkb);
     }
     const bool short_even = nkb == 1 && !columns && pl.bn == 256 && waves <= 5;
-    pl.pair = us < best && (nkb >= 8 || (waves >= 3 && (nkb >= (apart ? 2 : 3) || short_even)));
+    pl.pair = us < best && (nkb >= 8 || (waves >= 3 && (nkb >= 3 || (nkb == 2 && columns) || short_even)));
     if (pl.pair) pl.bn = 256;
     best = std::min(best, us);
   }
