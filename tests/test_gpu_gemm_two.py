@@ -22,7 +22,7 @@ def test_backward_has_the_bits_of_two_launches(tokens, k, n, tile, mode):
 # of data-gradient tiles that idle pairs take first.  The others stay apart.
 ON_PAIRS = [(8192, 2048, 2048, 1), (5000, 2048, 4224, 0), (24576, 1024, 1024, 6), (5000, 1024, 4096, 0), (24576, 1024, 3072, 9), (2048, 2048, 2048, 0),
             (700, 4096, 4096, 0), (12000, 768, 3072, 3), (4100, 640, 3200, 1)]
-PAIRS_APART = [(6145, 2048, 2176), (32768, 2048, 6144)]
+PAIRS_APART = [(6145, 2048, 2176), (32768, 2048, 6144), (8466, 384, 256), (512, 1024, 1920)]
 
 
 @pytest.mark.parametrize("tokens,k,n", [s[:3] for s in ON_PAIRS] + PAIRS_APART[:1])
