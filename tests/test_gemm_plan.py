@@ -124,6 +124,16 @@ def test_takes_the_faster_of_single_sms_and_pairs(lib, what, tokens, k, n, colum
     assert (pair_us if _kernel(lib, what, tokens, k, n, columns) == 2 else single_us) <= 1.04 * min(single_us, pair_us)
 
 
+# The scale ring on single SMs: (what, tokens, K, N, us without, us with)
+@pytest.mark.parametrize("what,tokens,k,n,plain_us,ring_us", [("wgrad", 12026, 384, 256, 10.36, 10.65), ("wgrad", 2944, 640, 384, 9.39, 9.64),
+                                                              ("wgrad", 12928, 256, 768, 11.8, 12.1), ("wgrad", 15047, 2176, 256, 20.0, 18.2),
+                                                              ("wgrad", 16896, 1792, 128, 15.2, 14.6), ("dgrad", 19200, 128, 6656, 65.5, 53.4),
+                                                              ("wgrad", 1920, 768, 384, 8.35, 7.92), ("dgrad", 244, 1152, 1792, 9.7, 7.7)])
+def test_takes_the_scale_ring_where_it_is_faster(lib, what, tokens, k, n, plain_us, ring_us):
+    kernel = _kernel(lib, what, tokens, k, n, 1)
+    assert kernel in (0, 1) and (ring_us if kernel == 1 else plain_us) <= 1.02 * min(plain_us, ring_us)
+
+
 @pytest.mark.parametrize("what,tokens,k,n,ranges", [("wgrad", 8192, 1024, 1024, 3), ("wgrad", 8192, 1024, 4096, 2), ("wgrad", 8192, 4096, 1024, 2),
                                                     ("wgrad", 8192, 1024, 3072, 1), ("wgrad", 32768, 1024, 1024, 3),
                                                     ("fwd", 8192, 1024, 4096, 1), ("dgrad", 1024, 128, 512, 1)])

@@ -832,8 +832,11 @@ static GemmPlan plan_gemm(const tg_gemm_args* a) {
   }
   pl.us = best;
   // Column scales through gemm_ring.cu's ring, where the contraction is long enough for its later start (the measurement is there).
+  // A range of a cut problem is worth it from 15 blocks on, as its float32 tile takes longer to leave (weight gradient of 12026 tokens, 384 x 256, 8 x
+  // 12 blocks 10.4 / 10.6 us, 15047 tokens 2176 x 256, 4 x 30 20.0 / 18.2), but where the scales lie apart (19200 x 6656 -> 128, 4 x 13 65.5 / 53.4).
   // Cut problems of 192-column tiles stay: their float32 tiles leave in three steps there (0.95-1.08 times as fast).
-  pl.ring = !pl.pair && columns && (nkb + pl.S - 1) / pl.S >= 12 && (pl.bn == 128 || (pl.bn == 192 && (pl.S == 1 && a->out_dtype == TG_OUT_BF16)));
+  const int64_t ring_from = pl.S > 1 && a->sb_stride_n == 1 ? 15 : 12;
+  pl.ring = !pl.pair && columns && (nkb + pl.S - 1) / pl.S >= ring_from && (pl.bn == 128 || (pl.bn == 192 && (pl.S == 1 && a->out_dtype == TG_OUT_BF16)));
   return pl;
 }
 
