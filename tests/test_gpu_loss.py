@@ -189,8 +189,8 @@ def test_loss_has_the_bits_of_the_mean_over_tokens(rows, vocab):
 # holds, the widest, rows that start at every alignment; more rows than the GPU takes at a time, a full last round and a short one.  The last four
 # are the other kernel's: a column too narrow and one too wide, rows too few, a last round too short.  Then that kernel where a block's rows start
 # at different alignments (three blocks per SM and one: 444 and 148 rows apart).
-LARGE_RAGGED = [(2200, 8961, 15.0), (800, 32769, 15.0), (760, 32775, 64.0), (480, 53247, 30.0), (1500, 12301, 0.5), (1200, 33337, 15.0)]
-RAGGED = [(2200, 8959, 15.0), (480, 53249, 15.0), (440, 50257, 15.0), (620, 40001, 15.0), (2200, 8193, 15.0), (2220, 8315, 15.0), (1000, 60001, 15.0)]
+LARGE_RAGGED = [(2200, 8705, 15.0), (800, 32769, 15.0), (760, 32775, 64.0), (480, 53247, 30.0), (1500, 12301, 0.5), (1200, 20003, 15.0)]
+RAGGED = [(2200, 8703, 15.0), (480, 53249, 15.0), (400, 50257, 15.0), (620, 40001, 15.0), (2200, 8193, 15.0), (2220, 8315, 15.0), (1000, 60001, 15.0)]
 
 
 @pytest.mark.parametrize("rows,vocab,cap", LARGE_RAGGED + RAGGED)

@@ -518,14 +518,15 @@ __global__ void __launch_bounds__(WARP ? 256 : WHOLE ? kLossFwdThreads : kCeMaxT
 //
 // 8192 x 50257 406 -> 336 us (4.9 TB/s), 8192 x 25001 226 -> 179, 2048 x 50257 105 -> 93, 4096 x 9001 60 -> 51.  The rule (softcap_ce_kernel / this one, with
 // a gradient; without one in brackets):
-//   columns   8201 leave a third pass nearly empty (3000 rows 39.4 / 40.8, 30.8 / 35.3), 9001 no longer (45.5 / 41.2, 35.6 / 35.6).
+//   columns   8201 leave a third pass nearly empty (3000 rows 39.4 / 40.8, 30.8 / 35.3), 8929 no longer (3952 rows 55.9 / 51.7, 44.2 / 43.4), 9001 (45.5 / 41.2, 35.6 / 35.6).
 //   rounds    two rows per SM at a time, 296 in all, and the table's 64 KB to begin with.  A last round of a few rows costs as much as a full one here,
-//             there a row alone on its SM is faster: 620 x 50257 38.8 / 42.5 (27.3 / 30.9), 920 x 25001 31.2 / 32.6 (22.6 / 25.6), 1248 x 20001 33.8 / 33.0 (25.2 / 26.8),
-//             1248 x 50257 68.5 / 67.7 (46.9 / 46.7), 1600 x 12301 33.2 / 31.0 (25.1 / 25.6).  So with six rounds and more, or five whose last is more than half
-//             full, from 18 M logits on; five with a shorter one from 40 M; fewer only with a last one more than half full and from 24 M
-//             (800 x 25001 27.5 / 26.9 (20.2 / 21.7), 592 x 50257 33.6 / 32.3 (24.0 / 23.6)).
+//             there a row alone on its SM is faster: 620 x 50257 38.8 / 42.5 (27.3 / 30.9), 700 x 32003 28.4 / 30.7, 920 x 25001 31.2 / 32.6 (22.6 / 25.6), but 722 x 34425
+//             36.8 / 32.6 (27.5 / 24.9), 1251 x 22492 38.6 / 35.5 (29.6 / 28.9), 1248 x 20001 33.8 / 33.0 (25.2 / 26.8), 1248 x 15441 28.1 / 28.7 (21.0 / 23.5), 1600 x 12301 33.2 / 31.0 (25.1 / 25.6).  So with six
+//             rounds and more, or a last one of more than two fifths, from 18 M logits on (1184 x 15441 25.6 / 25.3 (19.4 / 20.4)); five with a shorter one from 24 M.
+//             One rule for both, so that a loss has the same bits with and without a gradient; it goes by the gradient's time, and without one is up to 7 %
+//             slower than softcap_ce_kernel at the smallest of these (800 x 25001 20.2 / 21.7), faster from 30 M on.
 // ---------------------------------------------------------------------------------------
-constexpr int kCgMinCols = 8960;
+constexpr int kCgMinCols = 8704;
 constexpr int kCgThreads = 512, kCgGroups = 2;
 constexpr int kCgAhead = 4;                                  // pieces of a thread that are on their way to the L2
 constexpr int kCgTmemSlots = 8;                              // pieces of a thread in tensor memory
@@ -801,9 +802,9 @@ __global__ void __launch_bounds__(kMeanThreads) mean_kernel(const float* __restr
 static bool ce_in_groups(int64_t rows, int64_t vocab, int64_t sms) {
   if (vocab < kCgMinCols || vocab > kCgMaxCols) return false;
   const int64_t at_once = kCgGroups * sms, rounds = (rows + at_once - 1) / at_once, logits = rows * vocab;
-  const bool filled = 2 * (rows - (rounds - 1) * at_once) > at_once;
-  if (rounds >= 6 || (rounds == 5 && filled)) return logits >= 18'000'000;
-  return rounds == 5 ? logits >= 40'000'000 : filled && logits >= 24'000'000;
+  const bool filled = 5 * (rows - (rounds - 1) * at_once) > 2 * at_once;
+  if (rounds >= 6 || filled) return logits >= 18'000'000;
+  return rounds == 5 && logits >= 24'000'000;
 }
 
 constexpr int kCeSmemMax = kCeSmemLimit;
