@@ -1019,8 +1019,8 @@ static TwoPlan plan_two(const tg_gemm_args* a, const tg_gemm_args* b) {
   // Both on pairs of SMs, where one launch fills the last rounds (gemm_ring_two_kernel).  The modelled saving is 4 to 8 % too high (four
   // linears of 32768 tokens: 6-8 % modelled, -0.1 to 3 % measured in short runs, -1 to 2 % at the power cap); from a twelfth on large
   // problems gain (2-20 %, 700 x 4096 -> 4096 54.1 / 47.2 us with the quantisers).  Two short kernels launched early one after the other hide some
-  // of each other's ramps, which the model counts twice: below 2.1 us of modelled saving 8466 x 384 -> 256 had 15.7 apart / 17.4, 512 x 1024 -> 1920 13.2 / 13.9; of 89
-  // joint problems two with more still lose (211 x 3072 -> 2432 17.5 / 18.8).  A data gradient with a scale per
+  // of each other's ramps, which the model counts twice: below 2.1 us and 15 % of modelled saving 8466 x 384 -> 256 had 15.7 apart / 17.4, 512 x 1024 -> 1920 13.2 / 13.9
+  // (with 2 us but 20 %, 444 x 8064 -> 256 12.0 / 11.5); of 89 joint problems two with more still lose (211 x 3072 -> 2432 17.5 / 18.8).  A data gradient with a scale per
   // column stays apart: 12000 x 768 -> 3072 115 / 123 us, 4096 x 768 -> 3072 49.5 / 60, though 24576 x 1024 -> 1024 110 / 92.
   // (a is uncut: the callers hand both the same workspace, which only b may use in a joint launch.)
   auto wide = [](const tg_gemm_args* x) { return x->M > 128 && x->N > 128; };
@@ -1028,7 +1028,7 @@ static TwoPlan plan_two(const tg_gemm_args* a, const tg_gemm_args* b) {
     t.cut = cut_fits(b, t.b);
     if (t.cut || b->out_dtype == TG_OUT_BF16) {
       const double apart_us = t.a.us + t.b.us, together_us = pairs_together_us(b, t.cut ? t.b.S : 1, a, t.rounds);
-      if (together_us < (11.0 / 12.0) * apart_us && together_us < apart_us - 2.1) t.joint = TGH_TWO_PAIRS;
+      if (together_us < (11.0 / 12.0) * apart_us && (together_us < apart_us - 2.1 || together_us < 0.85 * apart_us)) t.joint = TGH_TWO_PAIRS;
     }
   }
   return t;

@@ -39,7 +39,7 @@ namespace tg {
 //     7.9 / 8.0, 8192 x 8192 15.9 / 17.6.  Narrow weights of long contractions stay here: 64 x 2048 x 512 5.8 / 7.1, though 48 x 4096 x 256 8.7 / 7.2.
 //   65 to 128 tokens.  With a scale per column only short contractions are tiled (100 x 1024 x 4096 7.5 / 6.2, 8192 x 8192 20.3 / 21.6, though 2048 x 8192
 //     9.8 / 8.9).  With one per 128 columns nearly all (100 x 1024 x 4096 7.5 / 5.8, 4096 x 4096 10.8 / 10.1, 8192 x 8192 20.1 / 18.6); not up to 2048 columns of
-//     1152 to 4608 (2048 x 2048 7.5 / 7.9), up to 2560 of about 2048 (65 x 2048 x 2176 7.0 / 7.8), nor 27 to 34 M weights (8192 x 4096 14.4 / 14.9, 5504 x
+//     1152 to 4608 (2048 x 2048 7.5 / 7.9), with fewer than 128 tokens up to 2560 of about 2048 (65 x 2048 x 2176 7.0 / 7.8), nor 27 to 34 M weights (8192 x 4096 14.4 / 14.9, 5504 x
 //     5120 13.2 / 13.7), and with 128 tokens, whose contraction ranges are fixed, 20 to 34 M (8192 x 3072 13.1 / 14.4, 5504 x 4096 12.6 / 14.3; but 4096 x
 //     6144 13.9 / 13.5).
 // 1092 problems of these ranges: the kernel taken is more than 5 % slower than the other in 40 of them.
@@ -368,7 +368,7 @@ bool skinny_takes(const tg_gemm_args* a) {
   if (a->N <= 512 && a->K <= 1024) return false;
   if (a->M <= 64) return a->K > (columns || a->N < 4096 ? 768 : 1024);
   if (a->K <= 1024 || columns) return a->K > 1024;
-  if (a->N <= 2048 ? a->K <= 4608 : a->N <= 2560 && a->K > 1536 && a->K < 3072) return true;
+  if (a->N <= 2048 ? a->K <= 4608 : a->N <= 2560 && a->K > 1536 && a->K < 3072 && a->M < 128) return true;
   return weights > (a->M == 128 ? 19 << 20 : 26 << 20) && weights <= 32 << 20;
 }
 
