@@ -712,21 +712,22 @@ __global__ void __launch_bounds__(kCgThreads * kCgGroups, 1) softcap_ce_groups_k
       if (p.d != nullptr) {
         __nv_bfloat16* dp = p.d + (now.base - p.logits);
         // by the product of the last two.  Where that is no normal number (its product with g still may be one) gscale goes in 2^64 times as
-        // large and the result comes back by 2^-64, both exact: a gradient scaled by a power of two is the same gradient at any scale.
+        // large and g 2^64 times as small, both exact where the result is no zero: a gradient scaled by a power of two has the same digits.
         const bool direct = !(fabsf(__fmul_rn(inv, gs)) < 1.2e-38f);
         const float factor = __fmul_rn(inv, direct ? gs : gs * 0x1p64f);
         const float2 f2 = make_float2(factor, factor), down = make_float2(0x1p-64f, 0x1p-64f);
         auto second_pass = [&](float2 (&g)[4], int i) {
           uint4 o;
           uint32_t* op = &o.x;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) g[j] = __fmul2_rn(g[j], f2);
           if (!direct) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) g[j] = __fmul2_rn(g[j], down);
           }
 #pragma unroll
-          for (int j = 0; j < 4; ++j) op[j] = pack_bf16x2(g[j].x, g[j].y);
+          for (int j = 0; j < 4; ++j) {
+            const float2 r = __fmul2_rn(g[j], f2);
+            op[j] = pack_bf16x2(r.x, r.y);
+          }
           if (i < now.last) *reinterpret_cast<uint4*>(dp + i * 8) = o;
         };
 #pragma unroll 2
